@@ -144,7 +144,8 @@ PX_API int32_t px_trimul_contract(const px_f16* a, const px_f16* b, px_f16* x, i
 #define PX_FAMILY_SELFTEST 9
 #define PX_FAMILY_PEER 10 /* px_peer_barrier: a rank did not arrive; detail bit r names the rank (mod 16) */
 #define PX_FAMILY_OPM 11
-#define PX_N_FAMILIES 12
+#define PX_FAMILY_SINGLE 12
+#define PX_N_FAMILIES 13
 PX_API int32_t px_device_error_flags(uint32_t* flags);
 PX_API int32_t px_device_error_detail(uint32_t* flags, uint32_t* detail);
 /* Limit of every bounded wait on the current device, in SM clock cycles (default 2^28, about 0.14 s); cycles <= 0
@@ -251,6 +252,21 @@ PX_API int32_t px_transition(const void* x_in, void* x_out, int32_t dtype, const
  * Replaces protenix/model/modules/transformer.py:185-188. */
 PX_API int32_t px_pair_bias_proj(const void* z, int32_t z_dtype, const float* ln_w, const float* ln_b, const px_w16* w,
                           float* out, int64_t rows, int32_t n_heads, float eps, void* stream);
+
+/* The single-representation branch of a block for c_s = 384, 16 heads x 24, transition x4 (fp32-grade products):
+ *   s1 = s + AttentionPairBias(s; pair_bias),  s_out = s1 + Transition(s1).
+ * Replaces AttentionPairBias.forward without s and the single transition, protenix/model/modules/transformer.py:40-254 and
+ * protenix/model/modules/pairformer.py:181-224.  px_single_prepare lays the fp32 weights (nn.Linear order) out once in a
+ * buffer of px_single_weights_bytes(); s and s_out [n][384] of s_dtype (may be the same), q_bias and LayerNorm vectors
+ * fp32 [384], pair_bias fp32 [16][n][n]. */
+PX_API int64_t px_single_weights_bytes(void);
+PX_API int64_t px_single_workspace_bytes(int64_t n);
+PX_API int32_t px_single_prepare(const float* w_q, const float* w_k, const float* w_v, const float* w_g, const float* w_o,
+                                 const float* w_a, const float* w_b, const float* w_out, void* prepared, void* stream);
+PX_API int32_t px_single_update(const void* s, void* s_out, int32_t s_dtype, const void* prepared, const float* ln_att_w,
+                                const float* ln_att_b, const float* q_bias, const float* ln_tr_w, const float* ln_tr_b,
+                                const float* pair_bias, void* workspace, int64_t workspace_bytes, int64_t n, float eps_att,
+                                float eps_tr, void* stream);
 
 /* ---- Recycling update of the pair representation ------------------------------------------
  * out[row] = z_init[row] + W LN(z[row]) for `rows` rows of 128 channels (W [128][128] in the format of z,

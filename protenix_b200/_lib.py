@@ -46,6 +46,10 @@ SIGNATURES = {
     "px_triangle_attention": (I32, [P, P, I32, P, P, P, P, P, P, P, P, P, P, I64, I64, I32, I32, F, F, P]),
     "px_transition": (I32, [P, P, I32, P, P, P, P, P, I64, I32, F, P]),
     "px_pair_bias_proj": (I32, [P, I32, P, P, P, P, I64, I32, F, P]),
+    "px_single_weights_bytes": (I64, []),
+    "px_single_workspace_bytes": (I64, [I64]),
+    "px_single_prepare": (I32, [P, P, P, P, P, P, P, P, P, P]),
+    "px_single_update": (I32, [P, P, I32, P, P, P, P, P, P, P, P, I64, I64, F, F, P]),
     "px_recycle_update": (I32, [P, P, P, I32, P, P, P, I64, F, P]),
     "px_scale_add_rowwise": (I32, [P, P, P, P, I64, I64, I64, I32, P]),
     "px_opm_outer": (I32, [P, P, P, I64, I64, I64, P]),

@@ -1,0 +1,564 @@
+// The single-representation branch of a Pairformer block (c_s = 384, 16 heads x 24) in fp32-grade arithmetic:
+//   s += W_o( softmax(q k^T / sqrt(24) + pair bias) v * sigmoid(W_g x) ),   x = LN(s)        (attention)
+//   s += W_out( silu(W_a y) * (W_b y) ),                                    y = LN(s)        (transition)
+//
+// The matrix products run on the 5th-generation tensor cores with every fp32 operand written as the sum of three bf16
+// values (8 + 8 + 8 significant bits) and the six partial products that reach 2^-24 accumulated in fp32: no operand
+// bit of an fp32 product is given up, and the range is that of fp32.  Six bf16 products cost 1/6 of the bf16 rate,
+// which is still five times that of the fp32 pipe.  Seven launches:
+//   split_rows        LayerNorm of s, written as three bf16 planes [3][N][384]
+//   split_gemm QKVG   [q | k | v | g] = x W^T, q scaled, sigmoid(g), fp32 [N][1536]
+//   single_attention  flash attention on the fp32 pipe (3.6 GFLOP at N = 1536), gated, written as three planes
+//   split_gemm RES    s1 = s + o W_o^T
+//   split_rows        LayerNorm of s1
+//   split_gemm SWIGLU h = silu(a) * b, a and b interleaved in the weight rows, written as three planes [3][N][1536]
+//   split_gemm RES    s2 = s1 + h W_out^T, the contraction split over a cluster of four CTAs
+// At N tokens each product has N/128 x (outputs/64) tiles: far too few to fill the chip at any N, so every launch is
+// bound by the latency of one tile (load, 24 MMAs per 64 inputs, epilogue); hence narrow 64-column tiles, no
+// persistence, and the split contraction where it is 1536 long.  Whole branch on an idle GPU: 64 us at N = 128 and 76 us at
+// N = 384, where library GEMMs and the composed attention took 290 us; 0.36 ms against 0.76 at N = 1536.
+#include "px_rowpipe.cuh"
+
+namespace px {
+
+constexpr int kSc = 384;                  // single channels
+constexpr int kSh = 16, kSd = 24;         // heads x head width
+constexpr int kSf = 4 * kSc;              // hidden width of the transition; also q | k | v | g
+constexpr int kSgBN = 64;                 // output columns of a tile
+constexpr int kSgABytes = 3 * 128 * 128;  // three planes of [128 rows][64 k] bf16
+constexpr int kSgWBytes = 3 * kSgBN * 128;
+constexpr int kSgStageBytes = kSgABytes + kSgWBytes;
+constexpr int kSgStages = 3;
+// Tensor memory: the leading products (plane 0 x plane 0) go round three accumulators, the corrections into three more.
+// The tensor core truncates when it adds to an accumulator, a bias that grows with the number of additions: one
+// accumulator for all 144 steps of K = 384 gave a relative error of 4.3e-6 on s; with these it is 2.6e-7 (fp32 GEMMs
+// of the library: 3.5e-7 to 4.8e-7).
+constexpr int kSgMain = 3;
+constexpr int kSgIssuers = 3;             // MMA-issuing warps, two of the six partial products each: an MMA of 64 columns
+                                          // takes 32 cycles, its issue about 100
+constexpr int kSgAcc = kSgMain + kSgIssuers;
+constexpr uint32_t kSgCols = 512;
+constexpr int kSgThreads = 32 * (1 + kSgIssuers + 4);
+constexpr int kSgSplit = 4;               // CTAs of a cluster that share a contraction of 1536
+
+enum { kSgQkvg = 0, kSgRes = 1, kSgSwiglu = 2 };
+
+struct SgBars {
+  uint64_t full[kSgStages], empty[kSgStages], acc_full;
+  uint32_t tmem_base;
+};
+
+// x = b0 + b1 + b2 with bf16 terms.
+__device__ __forceinline__ void split3(float x, bf16 (&b)[3]) {
+  b[0] = __float2bfloat16_rn(x);
+  const float r = x - __bfloat162float(b[0]);
+  b[1] = __float2bfloat16_rn(r);
+  b[2] = __float2bfloat16_rn(r - __bfloat162float(b[1]));
+}
+__device__ __forceinline__ void split3x2(float x, float y, uint32_t (&w)[3]) {
+  bf16 a[3], b[3];
+  split3(x, a);
+  split3(y, b);
+#pragma unroll
+  for (int p = 0; p < 3; ++p)
+    w[p] = (uint32_t)__bfloat16_as_ushort(a[p]) | ((uint32_t)__bfloat16_as_ushort(b[p]) << 16);
+}
+
+template <typename T>
+__device__ __forceinline__ float4 ld4(const T* p);
+template <>
+__device__ __forceinline__ float4 ld4<float>(const float* p) { return *reinterpret_cast<const float4*>(p); }
+template <>
+__device__ __forceinline__ float4 ld4<bf16>(const bf16* p) { return load4(p); }
+template <>
+__device__ __forceinline__ float4 ld4<__half>(const __half* p) {
+  const uint2 u = *reinterpret_cast<const uint2*>(p);
+  const float2 a = unpack_f16x2(u.x), b = unpack_f16x2(u.y);
+  return make_float4(a.x, a.y, b.x, b.y);
+}
+
+// LayerNorm of rows of 384, written as three bf16 planes; one warp per row, the row in registers.
+template <typename T>
+__global__ void __launch_bounds__(128) split_rows_kernel(const T* __restrict__ x, const float* __restrict__ gamma,
+                                                         const float* __restrict__ beta, bf16* __restrict__ out, int rows,
+                                                         float eps) {
+  const int row = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (row >= rows) return;
+  float4 v[3];
+  float s = 0.f;
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    v[i] = ld4<T>(x + (size_t)row * kSc + 128 * i + 4 * lane);
+    s += (v[i].x + v[i].y) + (v[i].z + v[i].w);
+  }
+  const float mean = warp_sum(s) * (1.0f / kSc);
+  float q = 0.f;
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    v[i].x -= mean, v[i].y -= mean, v[i].z -= mean, v[i].w -= mean;
+    q += (v[i].x * v[i].x + v[i].y * v[i].y) + (v[i].z * v[i].z + v[i].w * v[i].w);
+  }
+  const float rstd = rsqrtf(warp_sum(q) * (1.0f / kSc) + eps);
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    const int c = 128 * i + 4 * lane;
+    const float4 g = ld4<float>(gamma + c), b = ld4<float>(beta + c);
+    uint32_t lo[3], hi[3];
+    split3x2(fmaf(v[i].x * rstd, g.x, b.x), fmaf(v[i].y * rstd, g.y, b.y), lo);
+    split3x2(fmaf(v[i].z * rstd, g.z, b.z), fmaf(v[i].w * rstd, g.w, b.w), hi);
+#pragma unroll
+    for (int p = 0; p < 3; ++p)
+      *reinterpret_cast<uint2*>(out + ((size_t)p * rows + row) * kSc + c) = make_uint2(lo[p], hi[p]);
+  }
+}
+
+// fp32 weight rows -> three bf16 planes; source row r goes to row (r / blk) * stride + off + r % blk.
+__global__ void split_weight_kernel(const float* __restrict__ w, bf16* __restrict__ out, int rows, int k, int out_rows,
+                                    int blk, int stride, int off) {
+  const int r = blockIdx.x, dst = (r / blk) * stride + off + r % blk;
+  for (int c = threadIdx.x; c < k; c += blockDim.x) {
+    bf16 b[3];
+    split3(w[(size_t)r * k + c], b);
+#pragma unroll
+    for (int p = 0; p < 3; ++p) out[((size_t)p * out_rows + dst) * k + c] = b[p];
+  }
+}
+
+struct SgArgs {
+  const float* bias;      // QKVG: bias of q [384]
+  float* out_f;           // QKVG: [rows][1536]
+  bf16* out_planes;       // SWIGLU: [3][rows][1536]
+  const void* res;        // RES: residual and output [rows][384] of type T
+  void* out;
+  int rows, chunks;       // chunks of 64 inputs per CTA
+  float scale;            // QKVG: factor of q
+};
+
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.aligned;\n barrier.cluster.wait.aligned;\n" ::: "memory");
+}
+
+// One 128 x 64 tile of a split product per cluster (of gridDim.z CTAs, each with its share of the contraction).
+// Warp 0: TMA producer (three planes of A and of W per 64 inputs), warps 1..3: MMA issuers, warps 4..7: epilogue.
+template <int kMode, typename T>
+__global__ void __launch_bounds__(kSgThreads, 1)
+split_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w, const SgArgs g) {
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  unsigned char* ring = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  SgBars& bars = *reinterpret_cast<SgBars*>(ring + kSgStages * kSgStageBytes);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int n0 = blockIdx.x * kSgBN, m0 = blockIdx.y * 128, kc0 = blockIdx.z * g.chunks;
+
+  const bool skip = cta_skip_after_error();      // an earlier bounded wait gave up: do no work, but meet the barriers
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < kSgStages; ++s) {
+      mbar_init(&bars.full[s], 1);
+      mbar_init(&bars.empty[s], kSgIssuers);
+    }
+    mbar_init(&bars.acc_full, kSgIssuers);
+    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+  }
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(&bars.tmem_base)),
+                 "r"(kSgCols)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = bars.tmem_base;
+  float v[kSgBN];                                // epilogue: this thread's row of the tile
+  bool ok = !skip;
+
+  if (warp == 0) {
+    if (lane == 0 && ok) {
+      for (int i = 0; i < g.chunks; ++i) {
+        const int s = i % kSgStages;
+        if (!mbar_wait(&bars.empty[s], ((i / kSgStages) & 1) ^ 1, 1u)) break;
+        mbar_expect_tx(&bars.full[s], kSgStageBytes);
+        const uint32_t dst = smem_u32(ring + s * kSgStageBytes);
+        tma_load_3d(dst, &map_a, &bars.full[s], (kc0 + i) * 64, m0, 0);
+        tma_load_3d(dst + kSgABytes, &map_w, &bars.full[s], (kc0 + i) * 64, n0, 0);
+      }
+    }
+  } else if (warp <= kSgIssuers) {
+    if (lane == 0 && ok) {
+      // planes (i, j) with i + j <= 2, the terms above 2^-24 of the product: (0,0) (0,1) | (1,0) (1,1) | (0,2) (2,0)
+      const int w_ = warp - 1;
+      const int ai0 = w_ == 1 ? 1 : 0, aj0 = w_ == 2 ? 2 : 0, ai1 = w_, aj1 = w_ == 2 ? 0 : 1;
+      constexpr uint32_t idesc = umma_idesc_bf16(128, kSgBN);
+      const uint32_t corr = tmem_base + kSgBN * (kSgMain + w_);
+      bool done = true;
+      for (int i = 0; i < g.chunks; ++i) {
+        const int s = i % kSgStages;
+        done = mbar_wait(&bars.full[s], (i / kSgStages) & 1, 2u);
+        if (!done) break;
+        tc_fence_after();
+        const uint32_t a = smem_u32(ring + s * kSgStageBytes), w = a + kSgABytes;
+        const uint64_t da0 = umma_desc_sw128(a + ai0 * (128 * 128)), dw0 = umma_desc_sw128(w + aj0 * (kSgBN * 128));
+        const uint64_t da1 = umma_desc_sw128(a + ai1 * (128 * 128)), dw1 = umma_desc_sw128(w + aj1 * (kSgBN * 128));
+#pragma unroll
+        for (int ks = 0; ks < 4; ++ks) {
+          const int step = 4 * i + ks;
+          if (w_ == 0)
+            umma_bf16(tmem_base + kSgBN * (step % kSgMain), da0 + 2 * ks, dw0 + 2 * ks, idesc, step >= kSgMain);
+          else
+            umma_bf16(corr, da0 + 2 * ks, dw0 + 2 * ks, idesc, step > 0);
+          umma_bf16(corr, da1 + 2 * ks, dw1 + 2 * ks, idesc, step > 0 || w_ > 0);
+        }
+        umma_commit(&bars.empty[s]);
+      }
+      if (done) umma_commit(&bars.acc_full);
+    }
+  } else {
+    const int q = warp & 3, r = 32 * q + lane;     // tensor-memory lane = row of the tile
+    ok = ok && mbar_wait(&bars.acc_full, 0, 4u);
+    ok = __all_sync(0xffffffffu, ok);
+    if (ok) {
+      tc_fence_after();
+      const uint32_t t = tmem_base + ((uint32_t)(32 * q) << 16);
+      constexpr int kLast = (kSgAcc - 1) * kSgBN;  // corrections first
+      tmem_ld32(t + kLast, *reinterpret_cast<uint32_t(*)[32]>(&v[0]));
+      tmem_ld32(t + kLast + 32, *reinterpret_cast<uint32_t(*)[32]>(&v[32]));
+#pragma unroll
+      for (int p = 2 * (kSgAcc - 1) - 1; p >= 0; --p) {
+        uint32_t x[32];
+        tmem_ld32(t + (p >> 1) * kSgBN + 32 * (p & 1), x);
+        tmem_wait_ld();
+#pragma unroll
+        for (int e = 0; e < 32; ++e) v[32 * (p & 1) + e] += __uint_as_float(x[e]);
+      }
+      const int row = m0 + r;
+      if (kMode == kSgQkvg) {
+        const int part = n0 / kSc;                 // q, k, v or g: a tile of 64 lies in one of them
+        if (part == 0) {
+#pragma unroll
+          for (int e = 0; e < kSgBN; ++e) v[e] = (v[e] + __ldg(g.bias + n0 + e)) * g.scale;
+        } else if (part == 3) {
+#pragma unroll
+          for (int e = 0; e < kSgBN; ++e) v[e] = 1.0f / (1.0f + expf(-v[e]));
+        }
+        if (row < g.rows) {
+          float4* dst = reinterpret_cast<float4*>(g.out_f + (size_t)row * kSf + n0);
+#pragma unroll
+          for (int e = 0; e < kSgBN / 4; ++e) dst[e] = make_float4(v[4 * e], v[4 * e + 1], v[4 * e + 2], v[4 * e + 3]);
+        }
+      } else if (kMode == kSgSwiglu) {
+        if (row < g.rows) {                        // columns 0..31: a, 32..63: b of hidden units n0/2 ..
+#pragma unroll
+          for (int e = 0; e < 32; e += 8) {
+            uint32_t w[4][3];
+#pragma unroll
+            for (int p = 0; p < 4; ++p) {
+              const float a0 = v[e + 2 * p], a1 = v[e + 2 * p + 1];
+              const float h0 = a0 / (1.0f + expf(-a0)) * v[32 + e + 2 * p];
+              const float h1 = a1 / (1.0f + expf(-a1)) * v[32 + e + 2 * p + 1];
+              split3x2(h0, h1, w[p]);
+            }
+#pragma unroll
+            for (int p = 0; p < 3; ++p)
+              *reinterpret_cast<uint4*>(g.out_planes + ((size_t)p * g.rows + row) * kSf + n0 / 2 + e) =
+                  make_uint4(w[0][p], w[1][p], w[2][p], w[3][p]);
+          }
+        }
+      } else {
+        // partial sums to shared memory (the ring is idle: every product of this CTA is complete)
+        float4* stg = reinterpret_cast<float4*>(ring) + r * (kSgBN / 4);
+#pragma unroll
+        for (int e = 0; e < kSgBN / 4; ++e)
+          stg[e ^ (r & 15)] = make_float4(v[4 * e], v[4 * e + 1], v[4 * e + 2], v[4 * e + 3]);
+      }
+    }
+  }
+  if (kMode == kSgRes) {
+    __syncwarp();
+    cluster_sync();                                // every CTA's partial tile is in its shared memory
+    if (warp > kSgIssuers && ok) {
+      // each CTA sums and writes its share of the rows; a thread takes 16 bytes of a row at a time
+      const int split = gridDim.z, per = 128 / split, tid = threadIdx.x - 32 * (1 + kSgIssuers);
+      for (int i = tid; i < per * (kSgBN / 4); i += 128) {
+        const int r = blockIdx.z * per + i / (kSgBN / 4), c = i % (kSgBN / 4), row = m0 + r;
+        const uint32_t src = smem_u32(ring) + (r * (kSgBN / 4) + (c ^ (r & 15))) * 16;
+        float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int p = 0; p < split; ++p) {
+          uint32_t peer;
+          float4 x;
+          asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(peer) : "r"(src), "r"(p));
+          asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];\n"
+                       : "=f"(x.x), "=f"(x.y), "=f"(x.z), "=f"(x.w)
+                       : "r"(peer)
+                       : "memory");
+          sum.x += x.x, sum.y += x.y, sum.z += x.z, sum.w += x.w;
+        }
+        if (row < g.rows) {
+          // the update is rounded to the type of s before it is added, as the module's composition does
+          const size_t at = (size_t)row * kSc + n0 + 4 * c;
+          const float4 z = ld4<T>(reinterpret_cast<const T*>(g.res) + at);
+          T* o = reinterpret_cast<T*>(g.out) + at;
+          o[0] = T(z.x + float(T(sum.x))), o[1] = T(z.y + float(T(sum.y)));
+          o[2] = T(z.z + float(T(sum.z))), o[3] = T(z.w + float(T(sum.w)));
+        }
+      }
+    }
+    __syncwarp();
+    cluster_sync();                                // nobody leaves while a peer may still read its shared memory
+  }
+  tc_fence_before();
+  cta_teardown_sync();
+  if (warp == 0) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem_base), "r"(kSgCols) : "memory");
+  }
+}
+
+// Attention of one head and 32 queries over tiles of 64 keys, online softmax, fp32 throughout.  qkvg [n][1536] (q
+// scaled, g already a sigmoid), bias [16][n][n]; out: gated result as three planes [3][n][384].
+// Two groups of 128 threads take every other key tile and merge at the end (one group per CTA left an SM with five
+// warps at N = 384: 23 us).  A thread owns 4 queries x 4 keys of the logits; of the product with the values 4 queries
+// x 3 channels over half the keys of a tile.
+constexpr int kSaQ = 32, kSaK = 64, kSaLd = kSaK + 4, kSaGroups = 2;
+
+struct SaTile {
+  float k[kSd][kSaLd], v[kSd][kSaLd], p[kSaQ][kSaLd];
+};
+
+__global__ void __launch_bounds__(128 * kSaGroups, 2)
+single_attention_kernel(const float* __restrict__ qkvg, const float* __restrict__ bias, bf16* __restrict__ out, int n) {
+  extern __shared__ __align__(16) unsigned char sa_raw[];
+  float(*qs)[kSaQ] = reinterpret_cast<float(*)[kSaQ]>(sa_raw);
+  const int grp = threadIdx.x >> 7, tid = threadIdx.x & 127, ty = tid >> 4, tx = tid & 15;
+  SaTile& t = reinterpret_cast<SaTile*>(sa_raw + kSd * kSaQ * 4)[grp];
+  const int h = blockIdx.y, q0 = blockIdx.x * kSaQ;
+  const float* base = qkvg + h * kSd;
+  for (int i = threadIdx.x; i < kSaQ * (kSd / 4); i += 128 * kSaGroups) {
+    const int r = i & 31, d4 = i >> 5;
+    const float4 x = (q0 + r < n) ? ld4<float>(base + (size_t)(q0 + r) * kSf + 4 * d4) : make_float4(0.f, 0.f, 0.f, 0.f);
+    qs[4 * d4][r] = x.x, qs[4 * d4 + 1][r] = x.y, qs[4 * d4 + 2][r] = x.z, qs[4 * d4 + 3][r] = x.w;
+  }
+  float4 kr[3], vr[3];
+  auto load_kv = [&](int k0) {
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+      const int i = tid + 128 * j, k = k0 + (i & 63), d4 = i >> 6;
+      kr[j] = vr[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (k < n) {
+        const float* row = base + (size_t)k * kSf + 4 * d4;
+        kr[j] = ld4<float>(row + kSc);
+        vr[j] = ld4<float>(row + 2 * kSc);
+      }
+    }
+  };
+  const int khalf = tx >> 3, dg = 3 * (tx & 7);
+  float m[4], l[4], o[4][3];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    m[i] = -INFINITY, l[i] = 0.f;
+    o[i][0] = o[i][1] = o[i][2] = 0.f;
+  }
+  load_kv(kSaK * grp);
+  __syncthreads();
+  for (int k0 = kSaK * grp; k0 < n; k0 += kSaK * kSaGroups) {
+    named_barrier(1 + grp, 128);                   // the previous tile has been used
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+      const int i = tid + 128 * j, k = i & 63, d = 4 * (i >> 6);
+      t.k[d][k] = kr[j].x, t.k[d + 1][k] = kr[j].y, t.k[d + 2][k] = kr[j].z, t.k[d + 3][k] = kr[j].w;
+      t.v[d][k] = vr[j].x, t.v[d + 1][k] = vr[j].y, t.v[d + 2][k] = vr[j].z, t.v[d + 3][k] = vr[j].w;
+    }
+    float s[4][4];
+    const int kc = k0 + 4 * tx;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {                  // the pair bias starts the sum
+      const int qi = q0 + 4 * ty + i;
+      const float* b = bias + ((size_t)h * n + (qi < n ? qi : 0)) * n + kc;
+      if ((n & 3) == 0 && kc < n) {
+        const float4 b4 = __ldg(reinterpret_cast<const float4*>(b));
+        s[i][0] = b4.x, s[i][1] = b4.y, s[i][2] = b4.z, s[i][3] = b4.w;
+      } else {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) s[i][e] = kc + e < n ? __ldg(b + e) : -INFINITY;
+      }
+    }
+    named_barrier(1 + grp, 128);
+    if (k0 + kSaK * kSaGroups < n) load_kv(k0 + kSaK * kSaGroups);
+#pragma unroll
+    for (int d = 0; d < kSd; ++d) {
+      const float4 a = *reinterpret_cast<const float4*>(&qs[d][4 * ty]), b = *reinterpret_cast<const float4*>(&t.k[d][4 * tx]);
+      const float av[4] = {a.x, a.y, a.z, a.w}, bv[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) s[i][e] = fmaf(av[i], bv[e], s[i][e]);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      float mx = fmaxf(fmaxf(s[i][0], s[i][1]), fmaxf(s[i][2], s[i][3]));
+#pragma unroll
+      for (int x = 8; x > 0; x >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, x));
+      const float mn = fmaxf(m[i], mx), alpha = expf(m[i] - mn);
+      m[i] = mn;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) s[i][e] = expf(s[i][e] - mn);
+      l[i] = l[i] * alpha + ((s[i][0] + s[i][1]) + (s[i][2] + s[i][3]));
+      o[i][0] *= alpha, o[i][1] *= alpha, o[i][2] *= alpha;
+      *reinterpret_cast<float4*>(&t.p[4 * ty + i][4 * tx]) = make_float4(s[i][0], s[i][1], s[i][2], s[i][3]);
+    }
+    __syncwarp();                                  // the 16 threads of four queries sit in one warp
+#pragma unroll
+    for (int k = 0; k < kSaK / 2; k += 4) {
+      float4 p[4], w[3];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) p[i] = *reinterpret_cast<const float4*>(&t.p[4 * ty + i][32 * khalf + k]);
+#pragma unroll
+      for (int e = 0; e < 3; ++e) w[e] = *reinterpret_cast<const float4*>(&t.v[dg + e][32 * khalf + k]);
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int e = 0; e < 3; ++e)
+          o[i][e] = fmaf(p[i].x, w[e].x, fmaf(p[i].y, w[e].y, fmaf(p[i].z, w[e].z, fmaf(p[i].w, w[e].w, o[i][e]))));
+    }
+    __syncwarp();
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+#pragma unroll
+    for (int x = 8; x > 0; x >>= 1) l[i] += __shfl_xor_sync(0xffffffffu, l[i], x);
+#pragma unroll
+    for (int e = 0; e < 3; ++e) o[i][e] += __shfl_xor_sync(0xffffffffu, o[i][e], 8);
+  }
+  // group 1 hands its (m, l, o) to group 0 through its tile memory
+  float* part = &reinterpret_cast<SaTile*>(sa_raw + kSd * kSaQ * 4)[1].p[0][0];
+  __syncthreads();
+  if (grp == 1) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      float* r = part + (4 * ty + i) * (kSd + 2);
+      if (tx == 0) r[kSd] = m[i], r[kSd + 1] = l[i];
+      if (khalf == 0) r[dg] = o[i][0], r[dg + 1] = o[i][1], r[dg + 2] = o[i][2];
+    }
+  }
+  __syncthreads();
+  if (grp != 0 || khalf != 0) return;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int qi = q0 + 4 * ty + i;
+    if (qi >= n) continue;
+    const float* r = part + (4 * ty + i) * (kSd + 2);
+    const float mn = fmaxf(m[i], r[kSd]), a0 = expf(m[i] - mn), a1 = expf(r[kSd] - mn);   // m[0] is finite, m[1] may not be
+    const float inv = 1.0f / (l[i] * a0 + r[kSd + 1] * a1);
+#pragma unroll
+    for (int e = 0; e < 3; ++e) {
+      bf16 b[3];
+      split3((o[i][e] * a0 + r[dg + e] * a1) * inv * __ldg(base + (size_t)qi * kSf + 3 * kSc + dg + e), b);
+#pragma unroll
+      for (int p = 0; p < 3; ++p) out[((size_t)p * n + qi) * kSc + h * kSd + dg + e] = b[p];
+    }
+  }
+}
+
+PX_DEFINE_FAMILY_HOOKS(single)
+
+// Prepared weights: planes of [q|k|v|g] (1536 x 384), W_o (384 x 384), [a|b] interleaved (3072 x 384), W_out (384 x 1536)
+constexpr int64_t kSwQkvg = 0, kSwO = kSwQkvg + 3ll * kSf * kSc, kSwAb = kSwO + 3ll * kSc * kSc,
+                  kSwOut = kSwAb + 3ll * 2 * kSf * kSc, kSwEnd = kSwOut + 3ll * kSc * kSf;
+
+// planes [3][rows][k] bf16, box [3][box_rows][64]
+static bool make_plane_map(CUtensorMap* map, const bf16* base, int64_t rows, int64_t k, uint32_t box_rows) {
+  return make_map_3d(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, base, (uint64_t)k, (uint64_t)rows, 3, (uint64_t)k * 2,
+                     (uint64_t)rows * k * 2, 64, box_rows, CU_TENSOR_MAP_SWIZZLE_128B, 3);
+}
+
+template <int kMode, typename T>
+static bool launch_split_gemm(const bf16* a, const bf16* w, int64_t w_rows, int64_t k, int split, SgArgs g, cudaStream_t st) {
+  CUtensorMap ma, mw;
+  if (!make_plane_map(&ma, a, g.rows, k, 128) || !make_plane_map(&mw, w, w_rows, k, kSgBN)) return false;
+  constexpr size_t smem = (size_t)kSgStages * kSgStageBytes + sizeof(SgBars) + 1024;
+  static_assert(smem <= 232448, "shared memory budget");
+  if (cudaFuncSetAttribute(split_gemm_tc_kernel<kMode, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+    return false;
+  g.chunks = (int)(k / 64 / split);
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = 1, at[0].val.clusterDim.y = 1, at[0].val.clusterDim.z = (unsigned)split;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(w_rows / kSgBN), (unsigned)((g.rows + 127) / 128), (unsigned)split);
+  cfg.blockDim = dim3(kSgThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = at;
+  cfg.numAttrs = split > 1 ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, split_gemm_tc_kernel<kMode, T>, ma, mw, g) == cudaSuccess;
+}
+
+template <typename T>
+static int32_t run_single(const void* s, void* s_out, const bf16* w, const float* const ln[4], const float* q_bias,
+                          const float* bias, unsigned char* ws, int n, float eps_att, float eps_tr, cudaStream_t st) {
+  bf16* xp = (bf16*)ws;                                    // [3][n][384]: LN(s), the attention's result, LN(s1)
+  float* qkvg = (float*)(ws + (size_t)3 * n * kSc * 2);    // [n][1536]; later the hidden planes [3][n][1536]
+  bf16* hp = (bf16*)qkvg;
+  const unsigned lnb = (unsigned)((n + 3) / 4);
+  SgArgs g = {};
+  g.rows = n;
+  split_rows_kernel<T><<<lnb, 128, 0, st>>>((const T*)s, ln[0], ln[1], xp, n, eps_att);
+  g.bias = q_bias, g.out_f = qkvg, g.scale = 1.0f / sqrtf((float)kSd);
+  if (!launch_split_gemm<kSgQkvg, T>(xp, w + kSwQkvg, kSf, kSc, 1, g, st)) return PX_ERR_LAUNCH;
+  constexpr int sa_smem = kSd * kSaQ * 4 + kSaGroups * (int)sizeof(SaTile);
+  if (cudaFuncSetAttribute(single_attention_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, sa_smem) != cudaSuccess)
+    return PX_ERR_LAUNCH;
+  single_attention_kernel<<<dim3((unsigned)((n + kSaQ - 1) / kSaQ), kSh), 128 * kSaGroups, sa_smem, st>>>(qkvg, bias, xp, n);
+  g.res = s, g.out = s_out;
+  if (!launch_split_gemm<kSgRes, T>(xp, w + kSwO, kSc, kSc, 2, g, st)) return PX_ERR_LAUNCH;
+  split_rows_kernel<T><<<lnb, 128, 0, st>>>((const T*)s_out, ln[2], ln[3], xp, n, eps_tr);
+  g.out_planes = hp;
+  if (!launch_split_gemm<kSgSwiglu, T>(xp, w + kSwAb, 2 * kSf, kSc, 1, g, st)) return PX_ERR_LAUNCH;
+  g.res = s_out, g.out = s_out;
+  if (!launch_split_gemm<kSgRes, T>(hp, w + kSwOut, kSc, kSf, kSgSplit, g, st)) return PX_ERR_LAUNCH;
+  return cudaGetLastError() == cudaSuccess ? PX_OK : PX_ERR_LAUNCH;
+}
+
+}  // namespace px
+
+using namespace px;
+
+extern "C" int64_t px_single_weights_bytes(void) { return kSwEnd * 2; }
+
+extern "C" int64_t px_single_workspace_bytes(int64_t n) { return n <= 0 ? 0 : (3ll * kSc * 2 + 3ll * kSf * 2) * n; }
+
+extern "C" int32_t px_single_prepare(const float* w_q, const float* w_k, const float* w_v, const float* w_g, const float* w_o,
+                                     const float* w_a, const float* w_b, const float* w_out, void* prepared, void* stream) {
+  if (!w_q || !w_k || !w_v || !w_g || !w_o || !w_a || !w_b || !w_out || !prepared || ((uintptr_t)prepared & 15))
+    return PX_ERR_BAD_ARG;
+  cudaStream_t st = (cudaStream_t)stream;
+  bf16* p = (bf16*)prepared;
+  const float* qkvg[4] = {w_q, w_k, w_v, w_g};
+  for (int i = 0; i < 4; ++i)
+    split_weight_kernel<<<kSc, 128, 0, st>>>(qkvg[i], p + kSwQkvg, kSc, kSc, kSf, kSc, kSc, i * kSc);
+  split_weight_kernel<<<kSc, 128, 0, st>>>(w_o, p + kSwO, kSc, kSc, kSc, kSc, kSc, 0);
+  split_weight_kernel<<<kSf, 128, 0, st>>>(w_a, p + kSwAb, kSf, kSc, 2 * kSf, 32, 64, 0);
+  split_weight_kernel<<<kSf, 128, 0, st>>>(w_b, p + kSwAb, kSf, kSc, 2 * kSf, 32, 64, 32);
+  split_weight_kernel<<<kSc, 256, 0, st>>>(w_out, p + kSwOut, kSc, kSf, kSc, kSc, kSc, 0);
+  return cudaGetLastError() == cudaSuccess ? PX_OK : PX_ERR_LAUNCH;
+}
+
+extern "C" int32_t px_single_update(const void* s, void* s_out, int32_t s_dtype, const void* prepared, const float* ln_att_w,
+                                    const float* ln_att_b, const float* q_bias, const float* ln_tr_w, const float* ln_tr_b,
+                                    const float* pair_bias, void* workspace, int64_t workspace_bytes, int64_t n,
+                                    float eps_att, float eps_tr, void* stream) {
+  if (!s || !s_out || !prepared || !ln_att_w || !ln_att_b || !q_bias || !ln_tr_w || !ln_tr_b || !pair_bias || !workspace ||
+      n <= 0 || n > 32768)
+    return PX_ERR_BAD_ARG;
+  if (((uintptr_t)s | (uintptr_t)s_out | (uintptr_t)prepared | (uintptr_t)ln_att_w | (uintptr_t)ln_att_b | (uintptr_t)ln_tr_w |
+       (uintptr_t)ln_tr_b | (uintptr_t)pair_bias | (uintptr_t)workspace) & 15)
+    return PX_ERR_BAD_ARG;
+  if (workspace_bytes < px_single_workspace_bytes(n)) return PX_ERR_WORKSPACE;
+  const float* const ln[4] = {ln_att_w, ln_att_b, ln_tr_w, ln_tr_b};
+  cudaStream_t st = (cudaStream_t)stream;
+  unsigned char* ws = (unsigned char*)workspace;
+  switch (s_dtype) {
+    case PX_F32: return run_single<float>(s, s_out, (const bf16*)prepared, ln, q_bias, pair_bias, ws, (int)n, eps_att, eps_tr, st);
+    case PX_BF16: return run_single<bf16>(s, s_out, (const bf16*)prepared, ln, q_bias, pair_bias, ws, (int)n, eps_att, eps_tr, st);
+    case PX_F16: return run_single<__half>(s, s_out, (const bf16*)prepared, ln, q_bias, pair_bias, ws, (int)n, eps_att, eps_tr, st);
+    default: return PX_ERR_UNSUPPORTED;
+  }
+}

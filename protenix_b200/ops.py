@@ -133,7 +133,7 @@ def _launch(name: str, fn, *args) -> None:
 
 KERNEL_FAMILIES = ("trimul_contract", "triatt_flash", "transition", "trimul_in_proj", "trimul_out", "triatt_in_proj",
                    "triatt_out", "pair_bias_proj", "recycle_update", "selftest", "peer_barrier",
-                   "outer_product_mean")   # bit order of px_device_error_flags
+                   "outer_product_mean", "single_update")   # bit order of px_device_error_flags
 
 
 def device_error_flags(device=None, raise_on_error: bool = True) -> int:
@@ -410,6 +410,44 @@ def pair_bias_proj(z: torch.Tensor, ln_w, ln_b: Optional[torch.Tensor], w: torch
     rows, rows_dt = _rows_of(z, zn, eps)
     _launch("px_pair_bias_proj", _lib.load().px_pair_bias_proj, _ptr(rows), rows_dt, _ptr(ln_w), _ptr(ln_b),
             _ptr(w), _ptr(out), n * n, heads, float(eps), _stream(z))
+    return out
+
+
+C_S, N_HEAD_SINGLE = 384, 16     # the single-representation branch px_single_update is built for
+
+
+def single_weights(w_q, w_k, w_v, w_g, w_o, w_a, w_b, w_out) -> torch.Tensor:
+    """The fp32 matrices of the single-representation branch in the layout of ``px_single_update``."""
+    ws = [w.detach().float().contiguous() for w in (w_q, w_k, w_v, w_g, w_o, w_a, w_b, w_out)]
+    for w, shape in zip(ws, [(C_S, C_S)] * 5 + [(4 * C_S, C_S)] * 2 + [(C_S, 4 * C_S)]):
+        _need_cuda(w, "single weights")
+        if tuple(w.shape) != shape:
+            raise RuntimeError(f"single-representation weight must be {shape}, got {tuple(w.shape)}")
+    lib = _lib.load()
+    out = torch.empty(int(lib.px_single_weights_bytes()), dtype=torch.uint8, device=ws[0].device)
+    _launch("px_single_prepare", lib.px_single_prepare, *[_ptr(w) for w in ws], _ptr(out), _stream(out))
+    return out
+
+
+def single_update(s: torch.Tensor, prepared: torch.Tensor, ln_att_w, ln_att_b, q_bias, ln_tr_w, ln_tr_b,
+                  pair_bias: torch.Tensor, eps_att: float = 1e-5, eps_tr: float = 1e-5) -> torch.Tensor:
+    """s + AttentionPairBias(s) followed by the single transition, for s [..., N, 384] with one row per token."""
+    _need_cuda(s, "s")
+    _need_cuda(pair_bias, "pair_bias")
+    n = s.shape[-2]
+    if s.dtype not in _DTYPE or s.shape[-1] != C_S or s.numel() != n * C_S:
+        raise RuntimeError(f"s must be [N, {C_S}] in float32 / bfloat16 / float16, got {s.dtype} {tuple(s.shape)}")
+    if pair_bias.dtype != torch.float32 or tuple(pair_bias.shape) != (N_HEAD_SINGLE, n, n):
+        raise RuntimeError(f"pair_bias must be float32 [{N_HEAD_SINGLE}, N, N]")
+    for v in (ln_att_w, ln_att_b, q_bias, ln_tr_w, ln_tr_b):
+        _check_v(v, C_S, "single-representation vector")
+    lib = _lib.load()
+    nbytes = lib.px_single_workspace_bytes(n)
+    ws = workspace(s.device, nbytes)
+    out = torch.empty_like(s)
+    _launch("px_single_update", lib.px_single_update, _ptr(s), _ptr(out), _DTYPE[s.dtype], _ptr(prepared), _ptr(ln_att_w),
+            _ptr(ln_att_b), _ptr(q_bias), _ptr(ln_tr_w), _ptr(ln_tr_b), _ptr(pair_bias), _ptr(ws), nbytes, n, float(eps_att),
+            float(eps_tr), _stream(s))
     return out
 
 

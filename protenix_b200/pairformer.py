@@ -23,6 +23,7 @@ from .primitives import Transition
 from .transformer import AttentionPairBias
 from .triangular import (TriangleAttention, TriangleMultiplicationIncoming, TriangleMultiplicationOutgoing,
                          _pair_input)
+from .weights import prepared_of
 
 
 class PairformerBlock(nn.Module):
@@ -58,6 +59,16 @@ class PairformerBlock(nn.Module):
     def single_path(self, s: torch.Tensor, bias: torch.Tensor) -> torch.Tensor:
         """The single-representation update, given the pair bias of the block's final z.  It needs nothing else from
         z, and the pair path never reads s: a stack can run it beside the pair path of the next block."""
+        att, tr = self.attention_pair_bias, self.single_transition
+        if (self.c_s, att.n_heads, tr.n) == (ops.C_S, ops.N_HEAD_SINGLE, 4) and s.numel() == s.shape[-2] * self.c_s:
+            a = att.attention
+            ws = (a.linear_q.weight, a.linear_k.weight, a.linear_v.weight, a.linear_g.weight, a.linear_o.weight,
+                  tr.linear_no_bias_a.weight, tr.linear_no_bias_b.weight, tr.linear_no_bias.weight)
+            prepared = prepared_of(ws, "single", lambda: ops.single_weights(*ws))
+            f = lambda p: p.detach().float()
+            return ops.single_update(s.contiguous(), prepared, f(att.layernorm_a.weight), f(att.layernorm_a.bias),
+                                     f(a.linear_q.bias), f(tr.layernorm1.weight), f(tr.layernorm1.bias), bias,
+                                     att.layernorm_a.eps, tr.layernorm1.eps)
         s = s + self.attention_pair_bias(a=s, s=None, z=None, bias=bias)
         return s + self.single_transition(s)
 
