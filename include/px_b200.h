@@ -99,6 +99,14 @@ PX_API int32_t px_layer_norm_fwd(const void* x, const void* gamma, const void* b
 PX_API int32_t px_layer_norm_bwd(const void* dy, const void* x, const float* mean, const float* invvar, const void* gamma,
                           void* dx, void* dgamma, void* dbeta, float* scratch, int64_t rows, int64_t cols,
                           int32_t dtype, void* stream);
+/* The same two with the scale and offset (and their gradients) either of type `dtype` or, with params = PX_F32, the fp32
+ * parameters of a 16-bit x: rounded to the type of x inside, as a cast before (and after) the call would. */
+PX_API int32_t px_layer_norm_fwd_params(const void* x, const void* gamma, const void* beta, void* y, float* mean,
+                                        float* invvar, int64_t rows, int64_t cols, float eps, int32_t dtype, int32_t params,
+                                        void* stream);
+PX_API int32_t px_layer_norm_bwd_params(const void* dy, const void* x, const float* mean, const float* invvar,
+                                        const void* gamma, void* dx, void* dgamma, void* dbeta, float* scratch, int64_t rows,
+                                        int64_t cols, int32_t dtype, int32_t params, void* stream);
 
 /* ---- Standardised copy of fp32 rows --------------------------------------------------------
  * zn[row] = fp16((z[row] - mean) * rsqrt(var + eps)) over `rows` rows of 128 channels: LayerNorm without scale and
