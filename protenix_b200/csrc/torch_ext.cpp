@@ -1,0 +1,722 @@
+// The host path of the package in native code: what a forward pass does between two kernel launches.
+//
+// The kernels of one Pairformer block at N = 128 take some 200 us; launched one by one from Python, with the checks, the
+// weight look-ups and a foreign-function call for each, a block cost the host 700 us and a LayerNorm of the single
+// representation 18 us for a 3 us kernel.  Here a module keeps a `Params` object: the places of its parameters (the
+// module's own `_parameters` dictionaries), what was seen there last, and the forms the kernels want (fp32 vectors,
+// 16-bit matrices, the split planes of the single branch), renewed when a parameter, its storage, its version or a
+// submodule has changed.  A call checks its tensors, looks the parameters over (some tens of pointer comparisons) and
+// issues the launches through the C ABI of px_b200.h, whose functions are taken from the library handle that the Python
+// side has loaded.  Workspaces come from the caching allocator on each call.
+#include <ATen/ATen.h>
+#include <ATen/cuda/CUDAContext.h>
+#include <ATen/cuda/CUDAEvent.h>
+#include <ATen/ops/dropout.h>
+#include <ATen/ops/empty.h>
+#include <ATen/ops/empty_like.h>
+#include <ATen/ops/ones.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+#include <dlfcn.h>
+#include <torch/csrc/autograd/custom_function.h>
+#include <torch/csrc/autograd/python_variable.h>
+#include <torch/csrc/utils/pybind.h>
+
+#include <atomic>
+#include <mutex>
+#include <stdexcept>
+#include <string>
+#include <tuple>
+#include <vector>
+
+#include "../../include/px_b200.h"
+
+namespace py = pybind11;
+using at::Tensor;
+typedef c10::optional<Tensor> OptTensor;
+
+namespace {
+
+constexpr int64_t kCz = 128, kCs = 384, kHeadsSingle = 16, kHeads = 4, kHeadDim = 32;
+
+[[noreturn]] void fail(const std::string& what) { throw std::runtime_error(what); }
+
+// ---- the C ABI, by the handle of the loaded library ------------------------------------------------------------------
+#define PX_FUNCTIONS(X)                                                                                                  \
+  X(px_status_string) X(px_ld) X(px_ld_mask) X(px_layer_norm_fwd_params) X(px_layer_norm_bwd_params)                     \
+  X(px_scale_add_rowwise) X(px_standardise_rows) X(px_trimul_in_proj) X(px_trimul_contract) X(px_trimul_out)             \
+  X(px_trimul_workspace_bytes) X(px_triatt_in_proj) X(px_triatt_flash) X(px_triatt_flash_scratch_bytes) X(px_triatt_out) \
+  X(px_triatt_workspace_bytes) X(px_transition) X(px_pair_bias_proj) X(px_single_weights_bytes)                          \
+  X(px_single_workspace_bytes) X(px_single_prepare) X(px_single_update)
+struct Abi {
+#define X(f) decltype(&::f) f = nullptr;
+  PX_FUNCTIONS(X)
+#undef X
+} abi;
+
+void bind_library(uintptr_t handle) {
+#define X(f)                                                                   \
+  abi.f = reinterpret_cast<decltype(abi.f)>(dlsym((void*)handle, #f));         \
+  if (!abi.f) fail(std::string("the kernel library lacks ") + #f);
+  PX_FUNCTIONS(X)
+#undef X
+}
+
+// ---- launches: counted, and timed with event pairs while a timer is on -----------------------------------------------
+std::atomic<int64_t> g_launches{0};
+std::atomic<bool> g_timing{false};
+std::mutex g_timer_mutex;
+struct Timed {
+  const char* name;
+  at::cuda::CUDAEvent start{cudaEventDefault}, stop{cudaEventDefault};
+};
+std::vector<Timed> g_timed;
+
+template <typename F>
+void launch(const char* name, cudaStream_t st, F f) {
+  int32_t status;
+  if (g_timing.load(std::memory_order_relaxed)) {
+    Timed t;
+    t.name = name;
+    const auto stream = c10::cuda::getStreamFromExternal(st, c10::cuda::current_device());
+    t.start.record(stream);
+    status = f();
+    t.stop.record(stream);
+    std::lock_guard<std::mutex> lock(g_timer_mutex);
+    g_timed.push_back(std::move(t));
+  } else {
+    status = f();
+  }
+  ++g_launches;
+  if (status != PX_OK)
+    fail(std::string(name) + " failed: " + abi.px_status_string(status) + " (status " + std::to_string(status) + ")");
+}
+
+std::vector<std::pair<std::string, double>> timer_collect() {
+  std::lock_guard<std::mutex> lock(g_timer_mutex);
+  std::vector<std::pair<std::string, double>> out;
+  for (auto& t : g_timed) {
+    t.stop.synchronize();
+    out.emplace_back(t.name, (double)t.start.elapsed_time(t.stop));
+  }
+  g_timed.clear();
+  return out;
+}
+
+// ---- tensors ----------------------------------------------------------------------------------------------------------
+void need_cuda(const Tensor& t, const char* name) {
+  if (!t.is_cuda()) fail(std::string(name) + " must be a CUDA tensor: this package has no CPU path");
+}
+int dtype_code(const Tensor& t, const char* name) {
+  switch (t.scalar_type()) {
+    case at::kFloat: return PX_F32;
+    case at::kBFloat16: return PX_BF16;
+    case at::kHalf: return PX_F16;
+    default: fail(std::string(name) + " must be float32, bfloat16 or float16");
+  }
+}
+Tensor bytes_like(const Tensor& t, int64_t n) { return at::empty({n}, t.options().dtype(at::kByte)); }
+
+// [N, N, 128] or [1, N, N, 128] -> contiguous [N, N, 128]; batch says whether there was a leading 1.
+Tensor pair_tensor(const Tensor& z, bool& batch) {
+  if (!z.is_cuda()) fail("pair tensor must live on a CUDA device: this package has no CPU path");
+  batch = z.dim() == 4;
+  if (batch && z.size(0) != 1) fail("leading batch dimensions other than 1 are not supported");
+  const Tensor t = batch ? z.select(0, 0) : z;
+  if (t.dim() != 3) fail("expected [N, N, C] or [1, N, N, C]");
+  if (t.size(0) != t.size(1) || t.size(2) != kCz) fail("pair tensor must have shape [N, N, 128]");
+  if (t.scalar_type() != at::kFloat && t.scalar_type() != at::kBFloat16) fail("pair tensor must be float32 or bfloat16");
+  return t.contiguous();
+}
+Tensor pair_mask(const OptTensor& mask, const Tensor& z) {
+  if (!mask.has_value() || !mask->defined()) return Tensor();
+  Tensor m = mask->dim() == 3 ? mask->select(0, 0) : *mask;
+  if (m.device() != z.device() || m.scalar_type() != at::kFloat) m = m.to(z.device(), at::kFloat);
+  if (m.dim() != 2 || m.size(0) != z.size(0) || m.size(1) != z.size(0)) fail("mask must be [N, N]");
+  return m.contiguous();
+}
+const float* fptr(const Tensor& t) { return t.defined() ? (const float*)t.data_ptr() : nullptr; }
+
+// ---- parameters of a module -----------------------------------------------------------------------------------------
+// What a parameter becomes: 'f' an fp32 vector, 'z' a matrix in the format of the pair tensor's rows (bf16 rows: bf16, fp32
+// rows: fp16), 'h' an fp16 matrix, 's' one of the eight matrices of the single branch (laid out together).
+struct Prepared {
+  std::vector<Tensor> t[2];          // by format of z: 0 fp32, 1 bf16
+  std::vector<const void*> p[2];
+  std::vector<float> scalars;
+  at::cuda::CUDAEvent ready[2];
+  cudaStream_t made_on[2] = {nullptr, nullptr};
+  bool have[2] = {false, false};
+};
+
+class Params {
+ public:
+  // checks: (dict, name) of submodules; params: (dict, name, kind, shape); scalars: (dict, name)
+  Params(const py::list& checks, const py::list& params, const py::list& scalars) {
+    for (const auto& c : checks) {
+      const auto t = c.cast<py::tuple>();
+      checks_.push_back({t[0].cast<py::dict>(), t[1].cast<py::object>(), py::none()});
+    }
+    for (const auto& c : params) {
+      const auto t = c.cast<py::tuple>();
+      params_.push_back({t[0].cast<py::dict>(), t[1].cast<py::object>(), py::none()});
+      kind_.push_back(t[2].cast<std::string>()[0]);
+      shape_.push_back(t[3].cast<std::vector<int64_t>>());
+    }
+    for (const auto& c : scalars) {
+      const auto t = c.cast<py::tuple>();
+      scalars_.push_back({t[0].cast<py::dict>(), t[1].cast<py::object>(), py::none()});
+    }
+    for (auto& s : checks_) s.seen = py::reinterpret_borrow<py::object>(find(s));
+  }
+
+  // False when a submodule has been replaced: the object has to be made again from the module.
+  bool current() const {
+    for (const auto& s : checks_)
+      if (find(s) != s.seen.ptr()) return false;
+    return true;
+  }
+
+  // The kernels' forms of the parameters for z of format zf; needs the GIL.
+  std::shared_ptr<const Prepared> get(int zf, const at::Device& dev) {
+    bool same = prepared_ != nullptr;
+    seen_.resize(params_.size());
+    for (size_t i = 0; i < params_.size(); ++i) {
+      PyObject* o = find(params_[i]);
+      Seen now;
+      if (o != Py_None) {
+        if (!THPVariable_Check(o)) fail("a module parameter is not a tensor");
+        const Tensor& t = THPVariable_Unpack(o);
+        now = {o, t.data_ptr(), (uint32_t)t._version(), t.scalar_type()};
+      }
+      if (!(now == seen_[i])) {
+        same = false;
+        seen_[i] = now;
+      }
+    }
+    if (!same) {
+      prepared_ = std::make_shared<Prepared>();
+      params_hold_.clear();
+      for (auto& s : params_) params_hold_.push_back(py::reinterpret_borrow<py::object>(find(s)));
+    }
+    for (size_t i = 0; i < scalars_.size(); ++i) {
+      const float v = (float)PyFloat_AsDouble(find(scalars_[i]));
+      if (prepared_->scalars.size() <= i) prepared_->scalars.push_back(v);
+      if (prepared_->scalars[i] != v) {        // another value than the one calls in flight may hold
+        auto next = std::make_shared<Prepared>();
+        next->scalars = prepared_->scalars;
+        next->scalars[i] = v;
+        prepared_ = next;
+      }
+    }
+    if (!prepared_->have[zf]) make(*prepared_, zf, dev);
+    const cudaStream_t st = at::cuda::getCurrentCUDAStream(dev.index());
+    if (prepared_->made_on[zf] != st && !prepared_->ready[zf].query()) prepared_->ready[zf].block(at::cuda::getCurrentCUDAStream(dev.index()));
+    return prepared_;
+  }
+
+ private:
+  struct Slot {
+    py::dict dict;
+    py::object key, seen;
+  };
+  struct Seen {
+    PyObject* object = nullptr;
+    void* data = nullptr;
+    uint32_t version = 0;
+    at::ScalarType type = at::kFloat;
+    bool operator==(const Seen& o) const {
+      return object == o.object && data == o.data && version == o.version && type == o.type;
+    }
+  };
+  static PyObject* find(const Slot& s) {
+    PyObject* o = PyDict_GetItem(s.dict.ptr(), s.key.ptr());
+    return o ? o : Py_None;
+  }
+
+  void make(Prepared& p, int zf, const at::Device& dev) {
+    at::NoGradGuard no_grad;
+    std::vector<Tensor> singles;
+    p.t[zf].clear();
+    p.p[zf].clear();
+    for (size_t i = 0; i < params_.size(); ++i) {
+      PyObject* o = find(params_[i]);
+      Tensor t;
+      if (o != Py_None) {
+        t = THPVariable_Unpack(o).detach();
+        need_cuda(t, "parameters");
+        if (t.device() != dev) fail("parameters and inputs must be on the same device");
+        if (!t.sizes().equals(shape_[i]) || !t.is_floating_point())
+          fail("a parameter must be a floating-point tensor of the shape the kernels are built for");
+        const auto want = kind_[i] == 'f' || kind_[i] == 's' ? at::kFloat
+                          : kind_[i] == 'z' && zf == 1       ? at::kBFloat16
+                                                             : at::kHalf;
+        t = t.to(want).contiguous();
+        if (kind_[i] == 's') singles.push_back(t);
+        if (((uintptr_t)t.data_ptr() & 15) != 0) t = t.clone();
+      }
+      p.t[zf].push_back(t);
+      p.p[zf].push_back(t.defined() ? t.data_ptr() : nullptr);
+    }
+    if (!singles.empty()) {
+      const Tensor out = bytes_like(singles[0], abi.px_single_weights_bytes());
+      const float* w[8];
+      for (int i = 0; i < 8; ++i) w[i] = (const float*)singles[i].data_ptr();
+      const cudaStream_t st = at::cuda::getCurrentCUDAStream(dev.index());
+      launch("px_single_prepare", st, [&] {
+        return abi.px_single_prepare(w[0], w[1], w[2], w[3], w[4], w[5], w[6], w[7], out.data_ptr(), st);
+      });
+      for (size_t i = 0; i < params_.size(); ++i)      // the planes replace the matrices
+        if (kind_[i] == 's') p.t[zf][i] = Tensor(), p.p[zf][i] = nullptr;
+      p.t[zf].push_back(out);
+      p.p[zf].push_back(out.data_ptr());
+    }
+    p.made_on[zf] = at::cuda::getCurrentCUDAStream(dev.index());
+    p.ready[zf].record(at::cuda::getCurrentCUDAStream(dev.index()));
+    p.have[zf] = true;
+  }
+
+  std::vector<Slot> checks_, params_, scalars_;
+  std::vector<char> kind_;
+  std::vector<std::vector<int64_t>> shape_;
+  std::vector<Seen> seen_;
+  std::vector<py::object> params_hold_;      // the parameter objects seen last: their addresses cannot be reused
+  std::shared_ptr<Prepared> prepared_;
+};
+typedef std::shared_ptr<const Prepared> Ready;
+
+int64_t al(int64_t n) { return (n + 255) / 256 * 256; }
+int zformat(const Tensor& z) { return z.scalar_type() == at::kBFloat16 ? 1 : 0; }
+
+// ---- the pair updates ------------------------------------------------------------------------------------------------
+struct PairCall {
+  int64_t n;
+  int zf, dt;                    // format index and dtype code of z
+  const float* mask;
+  unsigned char* ws;             // shared by the updates, which run one after the other
+  cudaStream_t st;
+};
+int64_t pair_workspace(int64_t n) { return std::max(abi.px_trimul_workspace_bytes(n), abi.px_triatt_workspace_bytes(n)); }
+
+void standardise(const PairCall& c, const void* z, void* zn, float eps) {
+  launch("px_standardise_rows", c.st, [&] { return abi.px_standardise_rows((const float*)z, (px_f16*)zn, c.n * c.n, eps, c.st); });
+}
+
+// zn: the standardised copy of an fp32 z_in, if the caller has it
+void tri_mul(const PairCall& c, const Prepared& pr, const void* z_in, void* z_out, bool incoming, bool add, const void* zn) {
+  const auto& p = pr.p[c.zf];
+  const float eps = pr.scalars[0];
+  const int64_t n = c.n, ld = abi.px_ld(n), per = kCz * n * ld * 2;
+  px_f16 *a = (px_f16*)c.ws, *b = (px_f16*)(c.ws + per), *x = (px_f16*)(c.ws + 2 * per);
+  const void* rows = z_in;
+  int rows_dt = c.dt;
+  if (c.dt == PX_F32) {          // the projection and the output stage normalise the same z: one standardised copy
+    if (!zn) {
+      zn = c.ws + 3 * per;
+      standardise(c, z_in, (void*)zn, eps);
+    }
+    rows = zn, rows_dt = PX_F16;
+  }
+  auto f = [&](int i) { return (const float*)p[i]; };
+  auto w = [&](int i) { return (const px_w16*)p[i]; };
+  launch("px_trimul_in_proj", c.st, [&] {
+    return abi.px_trimul_in_proj(rows, rows_dt, c.mask, f(0), f(1), w(4), w(5), w(6), w(7), a, b, n, n, ld, incoming, eps, c.st);
+  });
+  launch("px_trimul_contract", c.st, [&] { return abi.px_trimul_contract(a, b, x, kCz, n, ld, c.st); });
+  launch("px_trimul_out", c.st, [&] {
+    return abi.px_trimul_out(x, z_in, (const px_f16*)zn, z_out, c.dt, f(0), f(1), f(2), f(3), w(8), w(9), n, n, ld, add, eps, c.st);
+  });
+}
+
+void tri_att(const PairCall& c, const Prepared& pr, const void* z_in, void* z_out, bool ending, bool add) {
+  const auto& p = pr.p[c.zf];
+  const float eps = pr.scalars[0], inf = pr.scalars[1];
+  const int64_t n = c.n, ldm = abi.px_ld_mask(n);
+  const int64_t qkv = al(n * kHeads * abi.px_ld(n) * kHeadDim * 2);   // v is [n][4][32][ld(n)], q and k fit as well
+  px_f16 *q = (px_f16*)c.ws, *k = (px_f16*)(c.ws + qkv), *v = (px_f16*)(c.ws + 2 * qkv), *o = (px_f16*)(c.ws + 3 * qkv);
+  unsigned char* bias = (unsigned char*)o + al(n * n * kCz * 2);
+  unsigned char* mbias = bias + al(kHeads * n * ldm * 4);
+  unsigned char* flags = mbias + al(n * ldm * 4);
+  const void *zn = nullptr, *rows = z_in;
+  int rows_dt = c.dt;
+  if (c.dt == PX_F32) {
+    zn = flags + al(abi.px_triatt_flash_scratch_bytes(n, n));
+    standardise(c, z_in, (void*)zn, eps);
+    rows = zn, rows_dt = PX_F16;
+  }
+  auto f = [&](int i) { return (const float*)p[i]; };
+  auto w = [&](int i) { return (const px_w16*)p[i]; };
+  launch("px_triatt_in_proj", c.st, [&] {
+    return abi.px_triatt_in_proj(rows, rows_dt, c.mask, f(0), f(1), w(3), w(4), w(5), w(2), q, k, v, (float*)bias, (float*)mbias, n, n,
+                                 ldm, ending, eps, inf, c.st);
+  });
+  launch("px_triatt_flash", c.st, [&] {
+    return abi.px_triatt_flash(q, k, v, (const float*)bias, (const float*)mbias, o, flags, n, n, ldm, c.st);
+  });
+  launch("px_triatt_out", c.st, [&] {
+    return abi.px_triatt_out(o, z_in, (const px_f16*)zn, z_out, c.dt, f(0), f(1), w(6), w(7), n, n, ending, add, eps, c.st);
+  });
+}
+
+void transition_rows(cudaStream_t st, const Prepared& pr, int zf, int dt, const void* x_in, void* x_out, int64_t rows, bool add) {
+  const auto& p = pr.p[zf];
+  launch("px_transition", st, [&] {
+    return abi.px_transition(x_in, x_out, dt, (const float*)p[0], (const float*)p[1], (const px_f16*)p[2], (const px_f16*)p[3],
+                             (const px_f16*)p[4], rows, add, pr.scalars[0], st);
+  });
+}
+
+Tensor tri_mul_forward(Params& params, const Tensor& z, const OptTensor& mask, bool incoming, bool inplace_add) {
+  bool batch;
+  const Tensor zc = pair_tensor(z, batch);
+  c10::cuda::CUDAGuard guard(zc.device());
+  at::NoGradGuard no_grad;
+  const Tensor m = pair_mask(mask, zc);
+  const Ready pr = params.get(zformat(zc), zc.device());
+  py::gil_scoped_release release;
+  const Tensor out = inplace_add && zc.data_ptr() == z.data_ptr() ? zc : at::empty_like(zc);
+  const Tensor ws = bytes_like(zc, abi.px_trimul_workspace_bytes(zc.size(0)));
+  const PairCall c{zc.size(0), zformat(zc), dtype_code(zc, "z"), fptr(m), (unsigned char*)ws.data_ptr(), at::cuda::getCurrentCUDAStream()};
+  tri_mul(c, *pr, zc.data_ptr(), out.data_ptr(), incoming, inplace_add, nullptr);
+  return batch ? out.unsqueeze(0) : out;
+}
+
+Tensor tri_att_forward(Params& params, const Tensor& z, const OptTensor& mask, bool ending) {
+  bool batch;
+  const Tensor zc = pair_tensor(z, batch);
+  c10::cuda::CUDAGuard guard(zc.device());
+  at::NoGradGuard no_grad;
+  const Tensor m = pair_mask(mask, zc);
+  const Ready pr = params.get(zformat(zc), zc.device());
+  py::gil_scoped_release release;
+  const Tensor out = at::empty_like(zc);
+  const Tensor ws = bytes_like(zc, abi.px_triatt_workspace_bytes(zc.size(0)));
+  const PairCall c{zc.size(0), zformat(zc), dtype_code(zc, "z"), fptr(m), (unsigned char*)ws.data_ptr(), at::cuda::getCurrentCUDAStream()};
+  tri_att(c, *pr, zc.data_ptr(), out.data_ptr(), ending, false);
+  return batch ? out.unsqueeze(0) : out;
+}
+
+Tensor transition_forward(Params& params, const Tensor& x) {
+  need_cuda(x, "x");
+  if (x.dim() < 1 || x.size(-1) != kCz) fail("transition kernel handles [..., 128] rows");
+  c10::cuda::CUDAGuard guard(x.device());
+  at::NoGradGuard no_grad;
+  const Tensor xc = x.contiguous();
+  const Ready pr = params.get(zformat(xc), xc.device());
+  py::gil_scoped_release release;
+  const Tensor out = at::empty_like(xc);
+  transition_rows(at::cuda::getCurrentCUDAStream(), *pr, zformat(xc), dtype_code(xc, "x"), xc.data_ptr(), out.data_ptr(),
+                  xc.numel() / kCz, false);
+  return out;
+}
+
+// ---- blocks ----------------------------------------------------------------------------------------------------------
+struct Block {
+  std::shared_ptr<Params> mul_out, mul_in, att_start, att_end, transition, pair_bias, single;   // the last two: s branch
+  bool current() const {
+    for (const auto& p : {mul_out, mul_in, att_start, att_end, transition, pair_bias, single})
+      if (p && !p->current()) return false;
+    return true;
+  }
+};
+struct BlockReady {
+  Ready mul_out, mul_in, att_start, att_end, transition, pair_bias, single;
+};
+
+// s_in -> s_out given the block's pair bias
+void single_update(cudaStream_t st, const Prepared& pr, int zf, const Tensor& s_in, const Tensor& s_out, const Tensor& bias,
+                   const Tensor& ws) {
+  const auto& p = pr.p[zf];
+  launch("px_single_update", st, [&] {
+    return abi.px_single_update(s_in.data_ptr(), s_out.data_ptr(), dtype_code(s_in, "s"), p.back(), (const float*)p[0],
+                                (const float*)p[1], (const float*)p[2], (const float*)p[3], (const float*)p[4],
+                                (const float*)bias.data_ptr(), ws.data_ptr(), ws.numel(), s_in.numel() / kCs, pr.scalars[0],
+                                pr.scalars[1], st);
+  });
+}
+
+c10::cuda::CUDAStream side_stream(c10::DeviceIndex dev) {
+  static std::mutex mutex;
+  static std::vector<c10::optional<c10::cuda::CUDAStream>> streams;
+  std::lock_guard<std::mutex> lock(mutex);
+  if ((size_t)dev >= streams.size()) streams.resize(dev + 1);
+  if (!streams[dev]) streams[dev] = c10::cuda::getStreamFromPool(false, dev);
+  return *streams[dev];
+}
+
+// The blocks one after the other.  The pair path never reads s, and the single branch takes nothing from z but the pair
+// bias of the block's final z: the single branch of block b runs on a side stream beside the pair path of block b + 1
+// (two pair-bias buffers take turns).  A single block has nothing to run beside and stays on the caller's stream.
+// Everything is allocated on the caller's stream, which waits for the side stream before this returns.
+std::tuple<OptTensor, Tensor> stack_forward(const std::vector<std::shared_ptr<Block>>& blocks, const OptTensor& s_in,
+                                            const Tensor& z, const OptTensor& mask, bool inplace) {
+  bool batch;
+  const Tensor zi = pair_tensor(z, batch);
+  c10::cuda::CUDAGuard guard(zi.device());
+  at::NoGradGuard no_grad;
+  const Tensor m = pair_mask(mask, zi);
+  const int zf = zformat(zi);
+  const int64_t n = zi.size(0);
+  Tensor s = s_in.has_value() ? *s_in : Tensor();
+  bool singles = false;
+  std::vector<BlockReady> ready;
+  for (const auto& b : blocks) {
+    const auto dev = zi.device();
+    BlockReady r{b->mul_out->get(zf, dev), b->mul_in->get(zf, dev), b->att_start->get(zf, dev), b->att_end->get(zf, dev),
+                 b->transition->get(zf, dev), nullptr, nullptr};
+    if (b->single && s.defined()) {
+      r.pair_bias = b->pair_bias->get(zf, dev), r.single = b->single->get(zf, dev);
+      singles = true;
+    }
+    ready.push_back(r);
+  }
+  if (singles) {
+    need_cuda(s, "s");
+    if (s.dim() < 2 || s.size(-1) != kCs || s.size(-2) != n || s.numel() != n * kCs) fail("s must be [N, 384]");
+    dtype_code(s, "s");
+    s = s.contiguous();
+  }
+  py::gil_scoped_release release;
+  // z is copied only if there is no block to write it anew: the first update reads z and writes the result's tensor
+  const bool own = inplace || zi.data_ptr() != z.data_ptr();
+  const Tensor zc = own ? zi : blocks.empty() ? zi.clone() : at::empty_like(zi);
+  const Tensor ws = bytes_like(zc, pair_workspace(n));
+  const auto main = at::cuda::getCurrentCUDAStream();
+  const PairCall c{n, zf, dtype_code(zc, "z"), fptr(m), (unsigned char*)ws.data_ptr(), main};
+  const bool fp32 = c.dt == PX_F32;
+  const auto side = singles && blocks.size() > 1 ? side_stream(zc.device().index()) : main;
+  const bool aside = side != main;
+  Tensor zn, bias[2], sb[2], sws;
+  at::cuda::CUDAEvent bias_ready[2], side_done[2];
+  if (singles) {
+    if (fp32) zn = at::empty(zc.sizes(), zc.options().dtype(at::kHalf));
+    for (int i = 0; i < (aside ? 2 : 1); ++i) bias[i] = at::empty({kHeadsSingle, n, n}, zc.options().dtype(at::kFloat));
+    for (int i = 0; i < (blocks.size() > 1 ? 2 : 1); ++i) sb[i] = at::empty_like(s);
+    sws = bytes_like(zc, abi.px_single_workspace_bytes(n));
+    if (aside) {
+      side_done[0].record(main);
+      side_done[0].block(side);
+    }
+  }
+  struct Join {                     // the caller's stream goes on when the side stream is through, after an error too
+    bool on;
+    c10::cuda::CUDAStream side, main;
+    ~Join() {
+      if (!on) return;
+      at::cuda::CUDAEvent e;
+      e.record(side);
+      e.block(main);
+    }
+  } join{aside, side, main};
+  const void* zn_valid = nullptr;   // zn holds the standardised rows of the current z, made with zn_eps
+  float zn_eps = 0.f;
+  int64_t k = 0;                    // single updates so far
+  for (size_t b = 0; b < ready.size(); ++b) {
+    const BlockReady& r = ready[b];
+    const void* first_zn = zn_valid && zn_eps == r.mul_out->scalars[0] ? zn_valid : nullptr;
+    zn_valid = nullptr;
+    tri_mul(c, *r.mul_out, b == 0 ? zi.data_ptr() : zc.data_ptr(), zc.data_ptr(), false, true, first_zn);
+    tri_mul(c, *r.mul_in, zc.data_ptr(), zc.data_ptr(), true, true, nullptr);
+    tri_att(c, *r.att_start, zc.data_ptr(), zc.data_ptr(), false, true);
+    tri_att(c, *r.att_end, zc.data_ptr(), zc.data_ptr(), true, true);
+    transition_rows(c.st, *r.transition, zf, c.dt, zc.data_ptr(), zc.data_ptr(), n * n, true);
+    if (!r.single) continue;
+    const int turn = aside ? k & 1 : 0;
+    const void* rows = zc.data_ptr();
+    if (fp32) {                     // the copy made for the pair bias also serves the next block's first update
+      zn_eps = r.pair_bias->scalars[0];
+      standardise(c, zc.data_ptr(), zn.data_ptr(), zn_eps);
+      rows = zn_valid = zn.data_ptr();
+    }
+    if (aside && k >= 2) side_done[turn].block(main);       // the single branch two blocks ago has read this buffer
+    const auto& p = r.pair_bias->p[zf];
+    launch("px_pair_bias_proj", c.st, [&] {
+      return abi.px_pair_bias_proj(rows, fp32 ? PX_F16 : PX_BF16, (const float*)p[0], (const float*)p[1], (const px_w16*)p[2],
+                                   (float*)bias[turn].data_ptr(), n * n, kHeadsSingle, r.pair_bias->scalars[0], c.st);
+    });
+    if (aside) {
+      bias_ready[turn].record(main);
+      bias_ready[turn].block(side);
+    }
+    single_update(side, *r.single, zf, s, sb[k & 1], bias[turn], sws);
+    s = sb[k & 1];
+    if (aside) side_done[turn].record(side);
+    ++k;
+  }
+  return {s.defined() ? OptTensor(s) : OptTensor(), batch ? zc.unsqueeze(0) : zc};
+}
+
+// ---- LayerNorm -------------------------------------------------------------------------------------------------------
+struct LnParams {
+  Tensor w, b;
+  int code;        // dtype code of both
+};
+// The parameters as the kernels take them: of the type of x, or fp32 (rounded to the type of x inside).
+LnParams ln_params(const Tensor& x, const OptTensor& weight, const OptTensor& bias) {
+  LnParams r;
+  auto fit = [&](const OptTensor& p, const char* name) -> Tensor {
+    if (!p.has_value() || !p->defined()) return Tensor();
+    need_cuda(*p, name);
+    if (p->numel() != x.size(-1)) fail(std::string(name) + " must have as many elements as the last axis");
+    return p->detach();
+  };
+  r.w = fit(weight, "weight");
+  r.b = fit(bias, "bias");
+  const Tensor& any = r.w.defined() ? r.w : r.b;
+  auto type = any.defined() && any.scalar_type() == at::kFloat && (!r.b.defined() || r.b.scalar_type() == at::kFloat)
+                  ? at::kFloat
+                  : x.scalar_type();
+  for (Tensor* t : {&r.w, &r.b})
+    if (t->defined()) *t = (t->scalar_type() == type ? *t : t->to(type)).contiguous();
+  r.code = type == at::kFloat ? PX_F32 : dtype_code(x, "input");
+  return r;
+}
+void ln_check(const Tensor& x, int64_t width) {
+  need_cuda(x, "input");
+  if (x.dim() < 1 || x.size(-1) != width) {
+    std::string s;
+    for (int64_t d : x.sizes()) s += (s.empty() ? "" : ", ") + std::to_string(d);
+    fail("Expected input with last dimension " + std::to_string(width) + ", got (" + s + ")");
+  }
+  dtype_code(x, "input");
+}
+Tensor ln_forward(const Tensor& x, const LnParams& p, double eps, Tensor* mean, Tensor* invvar) {
+  c10::cuda::CUDAGuard guard(x.device());
+  const Tensor y = at::empty_like(x);
+  const int64_t cols = x.size(-1), rows = cols ? x.numel() / cols : 0;
+  if (mean) {
+    *mean = at::empty({rows}, x.options().dtype(at::kFloat));
+    *invvar = at::empty({rows}, x.options().dtype(at::kFloat));
+  }
+  const cudaStream_t st = at::cuda::getCurrentCUDAStream();
+  launch("px_layer_norm_fwd", st, [&] {
+    return abi.px_layer_norm_fwd_params(x.data_ptr(), p.w.defined() ? p.w.data_ptr() : nullptr, p.b.defined() ? p.b.data_ptr() : nullptr,
+                                        y.data_ptr(), mean ? (float*)mean->data_ptr() : nullptr,
+                                        mean ? (float*)invvar->data_ptr() : nullptr, rows, cols, (float)eps, dtype_code(x, "input"),
+                                        p.code, st);
+  });
+  return y;
+}
+
+// y = LayerNorm(x); keeps x and the fp32 row statistics for the backward.
+struct LayerNormFunction : torch::autograd::Function<LayerNormFunction> {
+  static Tensor forward(torch::autograd::AutogradContext* ctx, const Tensor& x, const OptTensor& weight, const OptTensor& bias,
+                        double eps) {
+    const Tensor xc = x.contiguous();
+    const LnParams p = ln_params(xc, weight, bias);
+    Tensor mean, invvar;
+    const Tensor y = ln_forward(xc, p, eps, &mean, &invvar);
+    ctx->save_for_backward({xc, p.w, mean, invvar});
+    ctx->saved_data["code"] = (int64_t)p.code;
+    ctx->saved_data["w_type"] = (int64_t)(weight.has_value() && weight->defined() ? weight->scalar_type() : at::kFloat);
+    ctx->saved_data["b_type"] = (int64_t)(bias.has_value() && bias->defined() ? bias->scalar_type() : at::kFloat);
+    ctx->saved_data["want_w"] = weight.has_value() && weight->defined() && weight->requires_grad();
+    ctx->saved_data["want_b"] = bias.has_value() && bias->defined() && bias->requires_grad();
+    ctx->saved_data["want_x"] = x.requires_grad();
+    return y;
+  }
+  static torch::autograd::variable_list backward(torch::autograd::AutogradContext* ctx, torch::autograd::variable_list grads) {
+    const auto saved = ctx->get_saved_variables();
+    const Tensor &x = saved[0], &w = saved[1], &mean = saved[2], &invvar = saved[3];
+    c10::cuda::CUDAGuard guard(x.device());
+    const Tensor dy = grads[0].contiguous();
+    const int code = (int)ctx->saved_data["code"].toInt();
+    const bool want_w = ctx->saved_data["want_w"].toBool(), want_b = ctx->saved_data["want_b"].toBool();
+    const int64_t cols = x.size(-1), rows = cols ? x.numel() / cols : 0;
+    const auto grad_type = code == PX_F32 ? at::kFloat : x.scalar_type();
+    const Tensor dx = at::empty_like(x);
+    Tensor dw, db, scratch;
+    if (want_w) dw = at::empty({cols}, x.options().dtype(grad_type));
+    if (want_b) db = at::empty({cols}, x.options().dtype(grad_type));
+    if (want_w || want_b) scratch = at::empty({2 * cols}, x.options().dtype(at::kFloat));
+    const cudaStream_t st = at::cuda::getCurrentCUDAStream();
+    launch("px_layer_norm_bwd", st, [&] {
+      return abi.px_layer_norm_bwd_params(dy.data_ptr(), x.data_ptr(), (const float*)mean.data_ptr(), (const float*)invvar.data_ptr(),
+                                          w.defined() ? w.data_ptr() : nullptr, dx.data_ptr(), want_w ? dw.data_ptr() : nullptr,
+                                          want_b ? db.data_ptr() : nullptr, scratch.defined() ? (float*)scratch.data_ptr() : nullptr,
+                                          rows, cols, dtype_code(x, "x"), code, st);
+    });
+    auto as = [](const Tensor& t, int64_t type) { return t.defined() ? t.to((at::ScalarType)type) : t; };
+    return {ctx->saved_data["want_x"].toBool() ? dx : Tensor(), as(dw, ctx->saved_data["w_type"].toInt()),
+            as(db, ctx->saved_data["b_type"].toInt()), Tensor()};
+  }
+};
+
+Tensor layer_norm(const Tensor& x, const OptTensor& weight, const OptTensor& bias, int64_t width, double eps) {
+  ln_check(x, width);
+  auto wants = [](const OptTensor& t) { return t.has_value() && t->defined() && t->requires_grad(); };
+  if (at::GradMode::is_enabled() && (x.requires_grad() || wants(weight) || wants(bias)))
+    return LayerNormFunction::apply(x, weight, bias, eps);
+  const Tensor xc = x.contiguous();
+  return ln_forward(xc, ln_params(xc, weight, bias), eps, nullptr, nullptr);
+}
+
+// ---- residual + row-shared dropout -----------------------------------------------------------------------------------
+// residual + x * mask with mask [..., 1, C, D] shared over axis -3 (residual undefined: x * mask)
+Tensor scale_add(const Tensor& residual, const Tensor& x_, const Tensor& mask) {
+  c10::cuda::CUDAGuard guard(x_.device());
+  const Tensor x = x_.contiguous(), r = residual.defined() ? residual.contiguous() : residual;
+  const Tensor out = at::empty_like(x);
+  const int64_t rows = x.size(-3), cd = x.size(-2) * x.size(-1), batches = rows * cd ? x.numel() / (rows * cd) : 0;
+  const cudaStream_t st = at::cuda::getCurrentCUDAStream();
+  launch("px_scale_add_rowwise", st, [&] {
+    return abi.px_scale_add_rowwise(r.defined() ? r.data_ptr() : nullptr, x.data_ptr(), mask.data_ptr(), out.data_ptr(), batches, rows,
+                                    cd, dtype_code(x, "x"), st);
+  });
+  return out;
+}
+
+struct DropoutAddFunction : torch::autograd::Function<DropoutAddFunction> {
+  static Tensor forward(torch::autograd::AutogradContext* ctx, const Tensor& residual, const Tensor& x, const Tensor& mask) {
+    ctx->save_for_backward({mask});
+    ctx->saved_data["want_r"] = residual.requires_grad();
+    ctx->saved_data["want_x"] = x.requires_grad();
+    return scale_add(residual, x, mask);
+  }
+  static torch::autograd::variable_list backward(torch::autograd::AutogradContext* ctx, torch::autograd::variable_list grads) {
+    const auto saved = ctx->get_saved_variables();
+    return {ctx->saved_data["want_r"].toBool() ? grads[0] : Tensor(),
+            ctx->saved_data["want_x"].toBool() ? scale_add(Tensor(), grads[0], saved[0]) : Tensor(), Tensor()};
+  }
+};
+
+Tensor dropout_add(const Tensor& residual, const Tensor& x, double p) {
+  need_cuda(x, "x");
+  if (x.dim() < 3) fail("x must be [..., R, C, D]");
+  dtype_code(x, "x");
+  if (!residual.is_cuda() || residual.sizes() != x.sizes() || residual.scalar_type() != x.scalar_type()) fail("residual must match x");
+  auto shape = x.sizes().vec();
+  shape[shape.size() - 3] = 1;
+  // drawn as a dropout of ones: the same generator calls, so that a seed gives the same mask
+  const Tensor mask = at::dropout(at::ones(shape, x.options().requires_grad(false)), p, true);
+  return DropoutAddFunction::apply(residual, x, mask);
+}
+
+}  // namespace
+
+PYBIND11_MODULE(_C, m) {
+  m.def("bind_library", &bind_library);
+  m.def("layer_norm", &layer_norm);
+  m.def("dropout_add", &dropout_add);
+  py::class_<Params, std::shared_ptr<Params>>(m, "Params")
+      .def(py::init<py::list, py::list, py::list>())
+      .def("current", &Params::current)
+      // kept in a module's __dict__: a copy or an unpickled module makes its own
+      .def("__deepcopy__", [](const Params&, py::dict) { return py::none(); })
+      .def("__reduce__", [](const Params&) { return py::make_tuple(py::type::of(py::none()), py::tuple()); });
+  py::class_<Block, std::shared_ptr<Block>>(m, "Block")
+      .def(py::init([](std::vector<std::shared_ptr<Params>> p) {
+        if (p.size() != 7) fail("a block has seven parameter groups");
+        return std::make_shared<Block>(Block{p[0], p[1], p[2], p[3], p[4], p[5], p[6]});
+      }))
+      .def("current", &Block::current)
+      .def("__deepcopy__", [](const Block&, py::dict) { return py::none(); })
+      .def("__reduce__", [](const Block&) { return py::make_tuple(py::type::of(py::none()), py::tuple()); });
+  m.def("tri_mul_forward", &tri_mul_forward);
+  m.def("tri_att_forward", &tri_att_forward);
+  m.def("transition_forward", &transition_forward);
+  m.def("stack_forward", &stack_forward);
+  m.def("launches", [](bool reset) { return reset ? g_launches.exchange(0) : g_launches.load(); });
+  m.def("timer", [](bool on) { g_timing = on; });
+  m.def("timer_collect", &timer_collect);
+}

@@ -8,20 +8,7 @@ run in one kernel (``px_scale_add_rowwise``), forward and backward.  CUDA tensor
 """
 import torch
 
-from . import ops
-
-
-class _DropoutAddRowwise(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, residual, x, mask):
-        ctx.save_for_backward(mask)
-        return ops.scale_add_rowwise(residual, x, mask)
-
-    @staticmethod
-    def backward(ctx, grad):
-        (mask,) = ctx.saved_tensors
-        gx = ops.scale_add_rowwise(None, grad.contiguous(), mask) if ctx.needs_input_grad[1] else None
-        return (grad if ctx.needs_input_grad[0] else None), gx, None
+from . import native
 
 
 def dropout_add_rowwise(residual: torch.Tensor, x: torch.Tensor, p_drop: float, training: bool) -> torch.Tensor:
@@ -29,7 +16,4 @@ def dropout_add_rowwise(residual: torch.Tensor, x: torch.Tensor, p_drop: float, 
         return residual + x
     if not x.is_cuda:
         raise RuntimeError("dropout_add_rowwise (training): CUDA tensors only, this package has no CPU path")
-    shape = list(x.shape)
-    shape[-3] = 1
-    mask = torch.nn.functional.dropout(x.new_ones(shape), p=p_drop, training=True)
-    return _DropoutAddRowwise.apply(residual, x, mask)
+    return native.load().dropout_add(residual, x, p_drop)

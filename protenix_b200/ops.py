@@ -11,7 +11,7 @@ from typing import Dict, Optional, Tuple
 
 import torch
 
-from . import _lib
+from . import _lib, native
 from ._lib import PX_BF16, PX_F16, PX_F32
 from .weights import w16_of
 
@@ -20,6 +20,7 @@ C_Z = 128
 X_SCALE = 1.0 / 64      # PX_TRIMUL_X_SCALE: the contraction stores x scaled so that it stays inside the fp16 range
 N_HEAD_PAIR = 4
 D_HEAD_PAIR = 32
+C_S, N_HEAD_SINGLE = 384, 16     # the single-representation branch px_single_update is built for
 
 
 def _ptr(t: Optional[torch.Tensor]) -> Optional[int]:
@@ -89,13 +90,15 @@ class StageTimer:
 
     def __init__(self) -> None:
         self.events = []          # (name, start, stop)
+        self.native = []          # (name, milliseconds) of the launches of the native host path
 
     def summary(self) -> Dict[str, Tuple[int, float]]:
         """name -> (launches, total milliseconds); call after a device synchronize."""
         out: Dict[str, Tuple[int, float]] = {}
-        for name, a, b in self.events:
+        self.native += native.load().timer_collect()
+        for name, ms in [(name, a.elapsed_time(b)) for name, a, b in self.events] + self.native:
             c, t = out.get(name, (0, 0.0))
-            out[name] = (c + 1, t + a.elapsed_time(b))
+            out[name] = (c + 1, t + ms)
         return out
 
 
@@ -106,12 +109,13 @@ launch_count = 0     # kernels of this library launched since import (or since r
 def set_stage_timer(t: Optional[StageTimer]) -> None:
     global _timer
     _timer = t
+    native.load().timer(t is not None)
 
 
 def reset_launch_count() -> int:
     global launch_count
     n, launch_count = launch_count, 0
-    return n
+    return n + native.load().launches(True)
 
 
 def _launch(name: str, fn, *args) -> None:
@@ -203,53 +207,6 @@ def layer_norm(x: torch.Tensor, weight: Optional[torch.Tensor], bias: Optional[t
     _launch("px_layer_norm_fwd", _lib.load().px_layer_norm_fwd, _ptr(x), _ptr(weight), _ptr(bias), _ptr(y),
             _ptr(mean), _ptr(invvar), rows, cols, float(eps), _DTYPE[x.dtype], _stream(x))
     return (y, mean, invvar) if return_stats else y
-
-
-def layer_norm_bwd(dy: torch.Tensor, x: torch.Tensor, mean: torch.Tensor, invvar: torch.Tensor,
-                   weight: Optional[torch.Tensor], want_weight: bool, want_bias: bool):
-    """Gradients of layer_norm: (dx, dweight or None, dbias or None) from the upstream gradient dy, the input x and the
-    fp32 statistics the forward returned."""
-    _need_cuda(dy, "dy")
-    _need_cuda(x, "x")
-    if dy.shape != x.shape or dy.dtype != x.dtype or x.dtype not in _DTYPE:
-        raise RuntimeError("dy must match x (float32 / bfloat16 / float16)")
-    cols = x.shape[-1]
-    rows = x.numel() // cols if cols else 0
-    if mean.numel() != rows or invvar.numel() != rows or mean.dtype != torch.float32 or invvar.dtype != torch.float32:
-        raise RuntimeError("mean and invvar must be the float32 [rows] statistics of the forward")
-    if weight is not None and (weight.dtype != x.dtype or weight.numel() != cols):
-        raise RuntimeError(f"weight must be {x.dtype} with {cols} elements")
-    dy, x = dy.contiguous(), x.contiguous()
-    dx = torch.empty_like(x)
-    dw = torch.empty(cols, dtype=x.dtype, device=x.device) if want_weight else None
-    db = torch.empty(cols, dtype=x.dtype, device=x.device) if want_bias else None
-    scratch = torch.empty(2 * cols, dtype=torch.float32, device=x.device) if (want_weight or want_bias) else None
-    _launch("px_layer_norm_bwd", _lib.load().px_layer_norm_bwd, _ptr(dy), _ptr(x), _ptr(mean), _ptr(invvar), _ptr(weight),
-            _ptr(dx), _ptr(dw), _ptr(db), _ptr(scratch), rows, cols, _DTYPE[x.dtype], _stream(x))
-    return dx, dw, db
-
-
-def scale_add_rowwise(residual: Optional[torch.Tensor], x: torch.Tensor, mask: torch.Tensor) -> torch.Tensor:
-    """residual + x * mask with mask [..., 1, C, D] shared over axis -3 of x [..., R, C, D] (residual None: x * mask)."""
-    _need_cuda(x, "x")
-    _need_cuda(mask, "mask")
-    if x.dim() < 3 or x.dtype not in _DTYPE or mask.dtype != x.dtype:
-        raise RuntimeError("x must be [..., R, C, D] in float32 / bfloat16 / float16 and the mask of the same type")
-    want = list(x.shape)
-    want[-3] = 1
-    if list(mask.shape) != want:
-        raise RuntimeError(f"mask must have shape {want}")
-    if residual is not None and (residual.shape != x.shape or residual.dtype != x.dtype or not residual.is_cuda):
-        raise RuntimeError("residual must match x")
-    x = x.contiguous()
-    residual = None if residual is None else residual.contiguous()
-    mask = mask.contiguous()
-    out = torch.empty_like(x)
-    rows, cd = x.shape[-3], x.shape[-2] * x.shape[-1]
-    batches = x.numel() // (rows * cd) if rows * cd else 0
-    _launch("px_scale_add_rowwise", _lib.load().px_scale_add_rowwise, _ptr(residual), _ptr(x), _ptr(mask), _ptr(out),
-            batches, rows, cd, _DTYPE[x.dtype], _stream(x))
-    return out
 
 
 def standardise_rows(z: torch.Tensor, eps: float = 1e-5, out: Optional[torch.Tensor] = None) -> torch.Tensor:
@@ -410,44 +367,6 @@ def pair_bias_proj(z: torch.Tensor, ln_w, ln_b: Optional[torch.Tensor], w: torch
     rows, rows_dt = _rows_of(z, zn, eps)
     _launch("px_pair_bias_proj", _lib.load().px_pair_bias_proj, _ptr(rows), rows_dt, _ptr(ln_w), _ptr(ln_b),
             _ptr(w), _ptr(out), n * n, heads, float(eps), _stream(z))
-    return out
-
-
-C_S, N_HEAD_SINGLE = 384, 16     # the single-representation branch px_single_update is built for
-
-
-def single_weights(w_q, w_k, w_v, w_g, w_o, w_a, w_b, w_out) -> torch.Tensor:
-    """The fp32 matrices of the single-representation branch in the layout of ``px_single_update``."""
-    ws = [w.detach().float().contiguous() for w in (w_q, w_k, w_v, w_g, w_o, w_a, w_b, w_out)]
-    for w, shape in zip(ws, [(C_S, C_S)] * 5 + [(4 * C_S, C_S)] * 2 + [(C_S, 4 * C_S)]):
-        _need_cuda(w, "single weights")
-        if tuple(w.shape) != shape:
-            raise RuntimeError(f"single-representation weight must be {shape}, got {tuple(w.shape)}")
-    lib = _lib.load()
-    out = torch.empty(int(lib.px_single_weights_bytes()), dtype=torch.uint8, device=ws[0].device)
-    _launch("px_single_prepare", lib.px_single_prepare, *[_ptr(w) for w in ws], _ptr(out), _stream(out))
-    return out
-
-
-def single_update(s: torch.Tensor, prepared: torch.Tensor, ln_att_w, ln_att_b, q_bias, ln_tr_w, ln_tr_b,
-                  pair_bias: torch.Tensor, eps_att: float = 1e-5, eps_tr: float = 1e-5) -> torch.Tensor:
-    """s + AttentionPairBias(s) followed by the single transition, for s [..., N, 384] with one row per token."""
-    _need_cuda(s, "s")
-    _need_cuda(pair_bias, "pair_bias")
-    n = s.shape[-2]
-    if s.dtype not in _DTYPE or s.shape[-1] != C_S or s.numel() != n * C_S:
-        raise RuntimeError(f"s must be [N, {C_S}] in float32 / bfloat16 / float16, got {s.dtype} {tuple(s.shape)}")
-    if pair_bias.dtype != torch.float32 or tuple(pair_bias.shape) != (N_HEAD_SINGLE, n, n):
-        raise RuntimeError(f"pair_bias must be float32 [{N_HEAD_SINGLE}, N, N]")
-    for v in (ln_att_w, ln_att_b, q_bias, ln_tr_w, ln_tr_b):
-        _check_v(v, C_S, "single-representation vector")
-    lib = _lib.load()
-    nbytes = lib.px_single_workspace_bytes(n)
-    ws = workspace(s.device, nbytes)
-    out = torch.empty_like(s)
-    _launch("px_single_update", lib.px_single_update, _ptr(s), _ptr(out), _DTYPE[s.dtype], _ptr(prepared), _ptr(ln_att_w),
-            _ptr(ln_att_b), _ptr(q_bias), _ptr(ln_tr_w), _ptr(ln_tr_b), _ptr(pair_bias), _ptr(ws), nbytes, n, float(eps_att),
-            float(eps_tr), _stream(s))
     return out
 
 

@@ -4,8 +4,8 @@ Constructor arguments, forward signature, return values and ``state_dict`` keys 
 protenix/model/modules/pairformer.py:42-340.  A block is eight kernel families on the pair
 tensor (triangle multiplication out/in: projection, contraction, output stage; triangle
 attention start/end: projection, flash attention, output stage; transition) plus the small
-single-representation branch.  z is updated in place on a private copy (or on the caller's
-tensor with ``inplace_safe=True``); the two transposed copies of z the reference makes around
+single-representation branch, issued by the native host path.  z is updated in place on a private
+tensor (or on the caller's with ``inplace_safe=True``); the two transposed copies of z the reference makes around
 the ending-node attention do not exist here -- the ending-node kernels index z transposed.
 
 Inference only: dropout is the identity (eval mode), gradients are not produced.
@@ -18,12 +18,10 @@ from typing import Optional, Tuple
 import torch
 import torch.nn as nn
 
-from . import ops
+from . import native, ops
 from .primitives import Transition
 from .transformer import AttentionPairBias
-from .triangular import (TriangleAttention, TriangleMultiplicationIncoming, TriangleMultiplicationOutgoing,
-                         _pair_input)
-from .weights import prepared_of
+from .triangular import TriangleAttention, TriangleMultiplicationIncoming, TriangleMultiplicationOutgoing
 
 
 class PairformerBlock(nn.Module):
@@ -47,28 +45,41 @@ class PairformerBlock(nn.Module):
                                                          c_a=c_s, c_z=c_z)
             self.single_transition = Transition(c_in=c_s, n=4)
 
-    def pair_path_(self, zc: torch.Tensor, mask: Optional[torch.Tensor], zn: Optional[torch.Tensor] = None) -> None:
-        """The five pair updates of the block, in place.  ``zn``: the standardised fp16 copy of an fp32 zc as passed
-        in, when the caller has it (the first triangle update then skips its standardising pass)."""
-        self.tri_mul_out.apply_(zc, mask, zn=zn)
-        self.tri_mul_in.apply_(zc, mask)
-        self.tri_att_start.apply_(zc, mask, ending=False)
-        self.tri_att_end.apply_(zc, mask, ending=True)
-        self.pair_transition.forward_residual_(zc)
+    # the single-representation branch: vectors, then the eight matrices in the order of px_single_prepare
+    _V, _A, _T = (ops.C_S,), "attention_pair_bias", "single_transition"
+    NATIVE_SINGLE = ([(f"{_A}.layernorm_a.weight", "f", _V), (f"{_A}.layernorm_a.bias", "f", _V),
+                      (f"{_A}.attention.linear_q.bias", "f", _V), (f"{_T}.layernorm1.weight", "f", _V),
+                      (f"{_T}.layernorm1.bias", "f", _V)]
+                     + [(f"attention_pair_bias.attention.linear_{x}.weight", "s", (ops.C_S, ops.C_S)) for x in "qkvgo"]
+                     + [(f"single_transition.linear_no_bias_{x}.weight", "s", (4 * ops.C_S, ops.C_S)) for x in "ab"]
+                     + [(f"{_T}.linear_no_bias.weight", "s", (ops.C_S, 4 * ops.C_S))],
+                     [f"{_A}.layernorm_a.eps", f"{_T}.layernorm1.eps"])
+
+    def _native(self):
+        """The native view of this block's parameters."""
+        return native.kept(self, self._make_native)
+
+    def _make_native(self):
+        for m in (self.tri_mul_out, self.tri_mul_in, self.tri_att_start, self.tri_att_end):
+            m._check_shape()
+        if (self.pair_transition.c_in, self.pair_transition.n) != (ops.C_Z, 4):
+            raise RuntimeError(f"the pair transition kernel is specialised for c_z = {ops.C_Z}, factor 4")
+        parts = [native.params(self, *native.under(name, *getattr(self, name).NATIVE))
+                 for name in ("tri_mul_out", "tri_mul_in", "tri_att_start", "tri_att_end", "pair_transition")]
+        if self._single_kernel():
+            parts += [native.params(self, *native.under("attention_pair_bias", *self.attention_pair_bias.NATIVE)),
+                      native.params(self, *self.NATIVE_SINGLE)]
+        else:
+            parts += [None, None]
+        return native.load().Block(parts)
+
+    def _single_kernel(self) -> bool:
+        """Whether the single branch has the dimensions px_single_update is built for."""
+        return self.c_s == ops.C_S and self.n_heads == ops.N_HEAD_SINGLE
 
     def single_path(self, s: torch.Tensor, bias: torch.Tensor) -> torch.Tensor:
-        """The single-representation update, given the pair bias of the block's final z.  It needs nothing else from
-        z, and the pair path never reads s: a stack can run it beside the pair path of the next block."""
-        att, tr = self.attention_pair_bias, self.single_transition
-        if (self.c_s, att.n_heads, tr.n) == (ops.C_S, ops.N_HEAD_SINGLE, 4) and s.numel() == s.shape[-2] * self.c_s:
-            a = att.attention
-            ws = (a.linear_q.weight, a.linear_k.weight, a.linear_v.weight, a.linear_g.weight, a.linear_o.weight,
-                  tr.linear_no_bias_a.weight, tr.linear_no_bias_b.weight, tr.linear_no_bias.weight)
-            prepared = prepared_of(ws, "single", lambda: ops.single_weights(*ws))
-            f = lambda p: p.detach().float()
-            return ops.single_update(s.contiguous(), prepared, f(att.layernorm_a.weight), f(att.layernorm_a.bias),
-                                     f(a.linear_q.bias), f(tr.layernorm1.weight), f(tr.layernorm1.bias), bias,
-                                     att.layernorm_a.eps, tr.layernorm1.eps)
+        """The single-representation update, given the pair bias of the block's final z (it needs nothing else from z), as a
+        composition: for other widths and batches than the kernels take."""
         s = s + self.attention_pair_bias(a=s, s=None, z=None, bias=bias)
         return s + self.single_transition(s)
 
@@ -77,15 +88,23 @@ class PairformerBlock(nn.Module):
                 triangle_multiplicative: str = "torch", triangle_attention: str = "torch",
                 inplace_safe: bool = False, chunk_size: Optional[int] = None
                 ) -> Tuple[Optional[torch.Tensor], torch.Tensor]:
-        if self.training and self.p_drop > 0:
+        return _run_blocks([self], s, z, pair_mask, inplace_safe)
+
+
+def _run_blocks(blocks, s: Optional[torch.Tensor], z: torch.Tensor, pair_mask: Optional[torch.Tensor], inplace_safe: bool
+                ) -> Tuple[Optional[torch.Tensor], torch.Tensor]:
+    for block in blocks:
+        if block.training and block.p_drop > 0:
             raise RuntimeError("PairformerBlock: training-mode dropout is not implemented; call .eval()")
-        zc, mask, batch = _pair_input(z, pair_mask)
-        if not inplace_safe and zc.data_ptr() == z.data_ptr():
-            zc = zc.clone()
-        self.pair_path_(zc, mask)
-        if self.c_s > 0:
-            s = self.single_path(s, self.attention_pair_bias.pair_bias(zc))
-        return s, (zc[None] if batch else zc)
+    run = native.load().stack_forward
+    if s is None or all(b.c_s == 0 or (b._single_kernel() and s.numel() == s.shape[-2] * b.c_s) for b in blocks):
+        return run([b._native() for b in blocks], s, z, pair_mask, inplace_safe)
+    for block in blocks:
+        _, z = run([block._native()], None, z, pair_mask, inplace_safe)
+        if block.c_s > 0:
+            s = block.single_path(s, block.attention_pair_bias.pair_bias(z))
+        inplace_safe = True             # every later block works on the copy the first one made
+    return s, z
 
 
 class PairformerStack(nn.Module):
@@ -105,45 +124,7 @@ class PairformerStack(nn.Module):
                 triangle_multiplicative: str = "torch", triangle_attention: str = "torch",
                 inplace_safe: bool = False, chunk_size: Optional[int] = None
                 ) -> Tuple[torch.Tensor, torch.Tensor]:
-        zc, mask, batch = _pair_input(z, pair_mask)
-        if not inplace_safe and zc.data_ptr() == z.data_ptr():
-            zc = zc.clone()
-        # The pair path does not depend on s, and the single path takes only the pair bias from z: the single path of
-        # block b runs on a side stream beside the pair path of block b + 1.
-        main = torch.cuda.current_stream(zc.device)
-        side = _side_stream(zc.device)
-        side.wait_stream(main)
-        # fp32 z: the standardised copy made for a block's pair bias (its final z) also serves the first triangle
-        # update of the next block, which normalises the same rows with the same eps
-        zn_buf = torch.empty_like(zc, dtype=torch.float16) if zc.dtype == torch.float32 and s is not None else None
-        zn, zn_eps = None, None
-        for block in self.blocks:
-            if block.training and block.p_drop > 0:
-                raise RuntimeError("PairformerBlock: training-mode dropout is not implemented; call .eval()")
-            block.pair_path_(zc, mask, zn if zn is not None and zn_eps == block.tri_mul_out.layer_norm_in.eps else None)
-            zn = None
-            if block.c_s > 0 and s is not None:
-                if zn_buf is not None:
-                    zn = ops.standardise_rows(zc, block.attention_pair_bias.layernorm_z.eps, out=zn_buf)
-                    zn_eps = block.attention_pair_bias.layernorm_z.eps
-                bias = block.attention_pair_bias.pair_bias(zc, zn)   # reads the block's final z, on the main stream
-                bias.record_stream(side)
-                side.wait_stream(main)
-                with torch.cuda.stream(side):
-                    s = block.single_path(s, bias)
-        main.wait_stream(side)
-        if s is not None:
-            s.record_stream(main)
+        s, z = _run_blocks(list(self.blocks), s, z, pair_mask, inplace_safe)
         if os.environ.get("PX_CHECK_DEVICE_ERRORS", "0") == "1":    # synchronises: off unless asked for
-            ops.device_error_flags(zc.device)
-        return s, (zc[None] if batch else zc)
-
-
-_SIDE_STREAMS = {}
-
-
-def _side_stream(device: torch.device) -> "torch.cuda.Stream":
-    key = (device.type, device.index if device.index is not None else torch.cuda.current_device())
-    if key not in _SIDE_STREAMS:
-        _SIDE_STREAMS[key] = torch.cuda.Stream(device=device)
-    return _SIDE_STREAMS[key]
+            ops.device_error_flags(z.device)
+        return s, z

@@ -16,7 +16,7 @@ import torch
 import torch.nn as nn
 import torch.nn.functional as F
 
-from . import ops
+from . import native, ops
 from .layer_norm import LayerNorm
 
 _TRUNC_STD = 0.87962566103423978  # std of a unit normal truncated to [-2, 2]
@@ -65,6 +65,11 @@ LinearNoBias = partial(Linear, bias=False)
 class Transition(nn.Module):
     """x -> W_o(silu(W_a LN(x)) * (W_b LN(x))); returns the update (no residual)."""
 
+    _V = (ops.C_Z,)
+    NATIVE = ([("layernorm1.weight", "f", _V), ("layernorm1.bias", "f", _V), ("linear_no_bias_a.weight", "h", (4 * ops.C_Z, ops.C_Z)),
+               ("linear_no_bias_b.weight", "h", (4 * ops.C_Z, ops.C_Z)), ("linear_no_bias.weight", "h", (ops.C_Z, 4 * ops.C_Z))],
+              ["layernorm1.eps"])
+
     def __init__(self, c_in: int, n: int) -> None:
         super().__init__()
         self.n = n
@@ -91,8 +96,7 @@ class Transition(nn.Module):
         if not x.is_cuda:
             raise RuntimeError("Transition: CUDA tensors only (no CPU path)")
         if self._fused_ok(x):
-            xc = x.contiguous()
-            return ops.transition(xc, torch.empty_like(xc), *self._weights(), add_residual=False)
+            return native.load().transition_forward(native.kept(self, lambda: native.params(self, *self.NATIVE)), x)
         # small widths (single representation, c_in = 384): LayerNorm kernel + library GEMMs, fp32 arithmetic whatever
         # the storage type of x and of the parameters
         y = self.layernorm1(x.float().contiguous())

@@ -39,6 +39,16 @@ import torch.nn.functional as F
 from . import ops
 
 
+_SIDE_STREAMS: Dict[Tuple[str, int], "torch.cuda.Stream"] = {}
+
+
+def _side_stream(device: torch.device) -> "torch.cuda.Stream":
+    key = (device.type, device.index if device.index is not None else torch.cuda.current_device())
+    if key not in _SIDE_STREAMS:
+        _SIDE_STREAMS[key] = torch.cuda.Stream(device=device)
+    return _SIDE_STREAMS[key]
+
+
 # ----------------------------------------------------------------------------------------------
 class CudaStages:
     """Stage interface backed by the C-ABI kernels."""
@@ -498,8 +508,6 @@ class ShardedPairformer:
         px = self._peer_for(z_loc)
         main = side = None
         if z_loc.is_cuda and isinstance(self.stages, CudaStages):
-            from .pairformer import _side_stream
-
             main, side = torch.cuda.current_stream(z_loc.device), _side_stream(z_loc.device)
             side.wait_stream(main)
         mask_loc = mask_t_loc = mask_cols = None

@@ -37,6 +37,9 @@ class _SingleAttention(nn.Module):
 
 
 class AttentionPairBias(nn.Module):
+    NATIVE = ([("layernorm_z.weight", "f", (ops.C_Z,)), ("layernorm_z.bias", "f", (ops.C_Z,)),
+               ("linear_nobias_z.weight", "z", (ops.N_HEAD_SINGLE, ops.C_Z))], ["layernorm_z.eps"])   # the pair bias
+
     def __init__(self, has_s: bool = True, create_offset_ln_z: bool = False, n_heads: int = 16, c_a: int = 768,
                  c_s: int = 384, c_z: int = 128, biasinit: float = -2.0, cross_attention_mode: bool = False) -> None:
         super().__init__()

@@ -16,7 +16,7 @@ from typing import List, Optional
 import torch
 import torch.nn as nn
 
-from . import ops
+from . import native, ops
 from .layer_norm import LayerNorm
 from .primitives import trunc_normal_init_
 
@@ -85,6 +85,12 @@ class BaseTriangleMultiplicativeUpdate(nn.Module):
 class TriangleMultiplicativeUpdate(BaseTriangleMultiplicativeUpdate):
     """Algorithms 11 / 12.  ``forward`` returns the update, or z + update with ``_add_with_inplace``."""
 
+    _V, _M = (ops.C_Z,), (ops.C_Z, ops.C_Z)
+    NATIVE = ([("layer_norm_in.weight", "f", _V), ("layer_norm_in.bias", "f", _V), ("layer_norm_out.weight", "f", _V),
+               ("layer_norm_out.bias", "f", _V), ("linear_a_p.weight", "z", _M), ("linear_a_g.weight", "z", _M),
+               ("linear_b_p.weight", "z", _M), ("linear_b_g.weight", "z", _M), ("linear_z.weight", "h", _M),
+               ("linear_g.weight", "z", _M)], ["layer_norm_in.eps"])
+
     def __init__(self, c_z: int, c_hidden: int, _outgoing: bool = True) -> None:
         super().__init__(c_z=c_z, c_hidden=c_hidden, _outgoing=_outgoing)
         self.linear_a_p = OpenfoldLinear(c_z, c_hidden, bias=False)
@@ -92,11 +98,14 @@ class TriangleMultiplicativeUpdate(BaseTriangleMultiplicativeUpdate):
         self.linear_b_p = OpenfoldLinear(c_z, c_hidden, bias=False)
         self.linear_b_g = OpenfoldLinear(c_z, c_hidden, bias=False, init="gating")
 
-    def _kernel_args(self):
+    def _check_shape(self) -> None:
         if self.c_z != ops.C_Z or self.c_hidden != ops.C_Z:
             raise RuntimeError(
                 f"TriangleMultiplication kernels are specialised for c_z = c_hidden = {ops.C_Z}; "
                 f"got c_z={self.c_z}, c_hidden={self.c_hidden} (no fallback path)")
+
+    def _kernel_args(self):
+        self._check_shape()
         f = lambda p: p.detach().float()
         return (f(self.layer_norm_in.weight), f(self.layer_norm_in.bias), f(self.layer_norm_out.weight),
                 f(self.layer_norm_out.bias), self.linear_a_p.weight, self.linear_a_g.weight,
@@ -113,12 +122,9 @@ class TriangleMultiplicativeUpdate(BaseTriangleMultiplicativeUpdate):
     def forward(self, z: torch.Tensor, mask: Optional[torch.Tensor] = None, inplace_safe: bool = False,
                 _add_with_inplace: bool = False, _inplace_chunk_size: Optional[int] = 256,
                 triangle_multiplicative: str = "torch") -> torch.Tensor:
-        zc, mask, batch = _pair_input(z, mask)
-        add = bool(inplace_safe and _add_with_inplace)
-        out = zc if (add and zc.data_ptr() == z.data_ptr()) else torch.empty_like(zc)
-        ops.triangle_multiplication(zc, out, mask, *self._kernel_args(), incoming=not self._outgoing,
-                                    add_residual=add, eps=self.layer_norm_in.eps)
-        return out[None] if batch else out
+        self._check_shape()
+        params = native.kept(self, lambda: native.params(self, *self.NATIVE))
+        return native.load().tri_mul_forward(params, z, mask, not self._outgoing, bool(inplace_safe and _add_with_inplace))
 
 
 class TriangleMultiplicationOutgoing(TriangleMultiplicativeUpdate):
@@ -150,6 +156,11 @@ class Attention(nn.Module):
 class TriangleAttention(nn.Module):
     """Algorithms 13 / 14.  ``forward`` returns the update (no residual), like the reference."""
 
+    _V, _M = (ops.C_Z,), (ops.C_Z, ops.C_Z)
+    NATIVE = ([("layer_norm.weight", "f", _V), ("layer_norm.bias", "f", _V), ("linear.weight", "z", (ops.N_HEAD_PAIR, ops.C_Z)),
+               ("mha.linear_q.weight", "z", _M), ("mha.linear_k.weight", "z", _M), ("mha.linear_v.weight", "z", _M),
+               ("mha.linear_g.weight", "z", _M), ("mha.linear_o.weight", "h", _M)], ["layer_norm.eps", "inf"])
+
     def __init__(self, c_in: int, c_hidden: int, no_heads: int, starting: bool = True, inf: float = 1e9) -> None:
         super().__init__()
         self.c_in = c_in
@@ -161,11 +172,14 @@ class TriangleAttention(nn.Module):
         self.linear = OpenfoldLinear(c_in, no_heads, bias=False)
         self.mha = Attention(c_in, c_in, c_in, c_hidden, no_heads)
 
-    def _kernel_args(self):
+    def _check_shape(self) -> None:
         if (self.c_in, self.c_hidden, self.no_heads) != (ops.C_Z, ops.D_HEAD_PAIR, ops.N_HEAD_PAIR):
             raise RuntimeError(
                 f"TriangleAttention kernels are specialised for c_in={ops.C_Z}, {ops.N_HEAD_PAIR} heads x "
                 f"{ops.D_HEAD_PAIR}; got c_in={self.c_in}, {self.no_heads} heads x {self.c_hidden} (no fallback path)")
+
+    def _kernel_args(self):
+        self._check_shape()
         m = self.mha
         return (self.layer_norm.weight.detach().float(), self.layer_norm.bias.detach().float(),
                 self.linear.weight, m.linear_q.weight, m.linear_k.weight,
@@ -182,11 +196,9 @@ class TriangleAttention(nn.Module):
 
     def forward(self, x: torch.Tensor, mask: Optional[torch.Tensor] = None, chunk_size: Optional[int] = None,
                 triangle_attention: str = "torch", inplace_safe: bool = False) -> torch.Tensor:
-        xc, mask, batch = _pair_input(x, mask)
-        out = torch.empty_like(xc)
-        ops.triangle_attention(xc, out, mask, *self._kernel_args(), ending=not self.starting, add_residual=False,
-                               eps=self.layer_norm.eps, inf=self.inf)
-        return out[None] if batch else out
+        self._check_shape()
+        params = native.kept(self, lambda: native.params(self, *self.NATIVE))
+        return native.load().tri_att_forward(params, x, mask, not self.starting)
 
 
 TriangleAttentionStartingNode = TriangleAttention

@@ -30,21 +30,6 @@ def w16_of(p: torch.Tensor, fmt: torch.dtype) -> torch.Tensor:
     return w
 
 
-_prepared: Dict[Tuple[int, str], Tuple[Tuple, torch.Tensor, "weakref.ref"]] = {}
-
-
-def prepared_of(params, tag: str, make) -> torch.Tensor:
-    """``make()``, kept until any of the parameters ``params`` changes (the first one owns the entry)."""
-    key = tuple((id(p), p.data_ptr(), p._version, p.dtype) for p in params)
-    ck = (id(params[0]), tag)
-    ent = _prepared.get(ck)
-    if ent is not None and ent[0] == key and ent[2]() is params[0]:
-        return ent[1]
-    out = make()
-    _prepared[ck] = (key, out, weakref.ref(params[0], lambda _r, ck=ck: _prepared.pop(ck, None)))
-    return out
-
-
 def bf16_of(p: torch.Tensor) -> torch.Tensor:
     return w16_of(p, torch.bfloat16)
 
@@ -55,4 +40,3 @@ def f16_of(p: torch.Tensor) -> torch.Tensor:
 
 def clear() -> None:
     _cache.clear()
-    _prepared.clear()
