@@ -261,6 +261,42 @@ PX_API int32_t px_transition(const void* x_in, void* x_out, int32_t dtype, const
 PX_API int32_t px_pair_bias_proj(const void* z, int32_t z_dtype, const float* ln_w, const float* ln_b, const px_w16* w,
                           float* out, int64_t rows, int32_t n_heads, float eps, void* stream);
 
+/* ---- Folded weights ---------------------------------------------------------------------------
+ * The LayerNorm'd projections fold gamma, beta and constant factors into their weights.  A caller that keeps its weights
+ * folds them once (px_*_fold, into px_*_folded_bytes() bytes of device memory) and passes the result to the *_folded form
+ * of the stage, which then differs from the form above only in where the weights come from.  rows_dtype: PX_BF16 (rows of a
+ * bf16 z) or PX_F16 (standardised rows of an fp32 z); the weights are given as to the stage.  The folded form may read
+ * `folded` before earlier work of the stream is complete: it must have been written before that work was issued, or the
+ * stream synchronised after px_*_fold. */
+PX_API int64_t px_trimul_in_folded_bytes(void);
+PX_API int32_t px_trimul_in_fold(const float* ln_w, const float* ln_b, const px_w16* w_ap, const px_w16* w_ag, const px_w16* w_bp,
+                                 const px_w16* w_bg, int32_t rows_dtype, void* folded, void* stream);
+PX_API int32_t px_trimul_in_proj_folded(const void* z, int32_t z_dtype, const float* mask, const void* folded, px_f16* a,
+                                        px_f16* b, int64_t n_u, int64_t n_t, int64_t ld, int32_t incoming, float eps, void* stream);
+PX_API int64_t px_trimul_out_folded_bytes(void);
+PX_API int32_t px_trimul_out_fold(const float* ln_in_w, const float* ln_in_b, const float* ln_out_w, const float* ln_out_b,
+                                  const px_f16* w_z, const px_w16* w_g, int32_t rows_dtype, void* folded, void* stream);
+PX_API int32_t px_trimul_out_folded(const px_f16* x, const void* z_in, const px_f16* zn, void* z_out, int32_t z_dtype,
+                                    const void* folded, int64_t n_i, int64_t n_j, int64_t ld, int32_t add_residual, float eps,
+                                    void* stream);
+PX_API int64_t px_triatt_in_folded_bytes(void);
+PX_API int32_t px_triatt_in_fold(const float* ln_w, const float* ln_b, const px_w16* w_q, const px_w16* w_k, const px_w16* w_v,
+                                 const px_w16* w_bias, int32_t rows_dtype, void* folded, void* stream);
+PX_API int32_t px_triatt_in_proj_folded(const void* z, int32_t z_dtype, const float* mask, const void* folded, px_f16* q, px_f16* k,
+                                        px_f16* v, float* bias, float* mask_bias, int64_t n_u, int64_t n_t, int64_t ldm,
+                                        int32_t ending, float eps, float inf, void* stream);
+PX_API int64_t px_triatt_out_folded_bytes(void);
+PX_API int32_t px_triatt_out_fold(const float* ln_w, const float* ln_b, const px_w16* w_g, const px_f16* w_o, int32_t rows_dtype,
+                                  void* folded, void* stream);
+PX_API int32_t px_triatt_out_folded(const px_f16* o, const void* z_in, const px_f16* zn, void* z_out, int32_t z_dtype,
+                                    const void* folded, int64_t n_u, int64_t n_t, int32_t ending, int32_t add_residual, float eps,
+                                    void* stream);
+PX_API int64_t px_pair_bias_folded_bytes(void);
+PX_API int32_t px_pair_bias_fold(const float* ln_w, const float* ln_b, const px_w16* w, int32_t n_heads, int32_t rows_dtype,
+                                 void* folded, void* stream);
+PX_API int32_t px_pair_bias_proj_folded(const void* z, int32_t z_dtype, const void* folded, float* out, int64_t rows,
+                                        int32_t n_heads, float eps, void* stream);
+
 /* The single-representation branch of a block for c_s = 384, 16 heads x 24, transition x4 (fp32-grade products):
  *   s1 = s + AttentionPairBias(s; pair_bias),  s_out = s1 + Transition(s1).
  * Replaces AttentionPairBias.forward without s and the single transition, protenix/model/modules/transformer.py:40-254 and

@@ -48,6 +48,21 @@ SIGNATURES = {
     "px_triangle_attention": (I32, [P, P, I32, P, P, P, P, P, P, P, P, P, P, I64, I64, I32, I32, F, F, P]),
     "px_transition": (I32, [P, P, I32, P, P, P, P, P, I64, I32, F, P]),
     "px_pair_bias_proj": (I32, [P, I32, P, P, P, P, I64, I32, F, P]),
+    "px_trimul_in_folded_bytes": (I64, []),
+    "px_trimul_in_fold": (I32, [P, P, P, P, P, P, I32, P, P]),
+    "px_trimul_in_proj_folded": (I32, [P, I32, P, P, P, P, I64, I64, I64, I32, F, P]),
+    "px_trimul_out_folded_bytes": (I64, []),
+    "px_trimul_out_fold": (I32, [P, P, P, P, P, P, I32, P, P]),
+    "px_trimul_out_folded": (I32, [P, P, P, P, I32, P, I64, I64, I64, I32, F, P]),
+    "px_triatt_in_folded_bytes": (I64, []),
+    "px_triatt_in_fold": (I32, [P, P, P, P, P, P, I32, P, P]),
+    "px_triatt_in_proj_folded": (I32, [P, I32, P, P, P, P, P, P, P, I64, I64, I64, I32, F, F, P]),
+    "px_triatt_out_folded_bytes": (I64, []),
+    "px_triatt_out_fold": (I32, [P, P, P, P, I32, P, P]),
+    "px_triatt_out_folded": (I32, [P, P, P, P, I32, P, I64, I64, I32, I32, F, P]),
+    "px_pair_bias_folded_bytes": (I64, []),
+    "px_pair_bias_fold": (I32, [P, P, P, I32, I32, P, P]),
+    "px_pair_bias_proj_folded": (I32, [P, I32, P, P, I64, I32, F, P]),
     "px_single_weights_bytes": (I64, []),
     "px_single_workspace_bytes": (I64, [I64]),
     "px_single_prepare": (I32, [P, P, P, P, P, P, P, P, P, P]),

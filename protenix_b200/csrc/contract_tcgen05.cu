@@ -42,7 +42,7 @@ trimul_contract_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nk = (ld_k + kTcBK - 1) / kTcBK;      // ld_k: extent of the contraction index; ld: row stride of x
 
-  if (cta_skip_after_error()) return;   // an earlier bounded wait gave up: do not start new work
+  const bool skip = cta_begin();         // an earlier bounded wait gave up: do not start new work
   if (threadIdx.x == 0) {
     for (int s = 0; s < kTcStages; ++s) {
       mbar_init(&bars.full[s], 1);
@@ -60,9 +60,7 @@ trimul_contract_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
   }
-  asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-  __syncthreads();
-  asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+  if (!cta_ready(skip, warp == 0, bars.tmem_base, kTcCols)) return;
   const uint32_t tmem_base = bars.tmem_base;
 
   auto tile_coords = [&](int tile, int& c, int& i0, int& j0) {
@@ -188,6 +186,8 @@ static int sm_count_contract() {
   return sms;
 }
 
+static SmemLimit contract_limit;
+
 extern "C" int32_t px_trimul_contract(const px_bf16* a, const px_bf16* b, px_bf16* x, int64_t channels, int64_t n,
                                       int64_t ld, void* stream) {
   if (!a || !b || !x || channels <= 0 || channels > 65535 || n <= 0 || n > 32768 || ld != px_ld(n))
@@ -198,16 +198,14 @@ extern "C" int32_t px_trimul_contract(const px_bf16* a, const px_bf16* b, px_bf1
     return PX_ERR_LAUNCH;
   const int tiles_i = (int)((n + kTcBM - 1) / kTcBM), tiles_j = (int)((n + kTcBN - 1) / kTcBN);
   const int total = tiles_i * tiles_j * (int)channels;
-  int dev = 0, sms = 148;
-  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int sms = sm_count_contract();
   const int grid = total < sms ? total : sms;
   const size_t smem = (size_t)kTcStages * kTcStageBytes + sizeof(TcBarriers) + 1024;
-  if (cudaFuncSetAttribute(trimul_contract_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-      cudaSuccess)
-    return PX_ERR_LAUNCH;
-  trimul_contract_tc_kernel<<<grid, 192, smem, (cudaStream_t)stream>>>(ma, mb, (bf16*)x, (int)n, (int)ld, (int)ld,
-                                                                       tiles_i, tiles_j, total);
-  return cudaGetLastError() == cudaSuccess ? PX_OK : PX_ERR_LAUNCH;
+  if (!contract_limit.set(trimul_contract_tc_kernel, smem)) return PX_ERR_LAUNCH;
+  return launch_pdl(trimul_contract_tc_kernel, dim3(grid), 192, smem, (cudaStream_t)stream, ma, mb, (bf16*)x, (int)n, (int)ld,
+                    (int)ld, tiles_i, tiles_j, total)
+             ? PX_OK
+             : PX_ERR_LAUNCH;
 }
 
 // The same kernel for the outer product of the MSA module: one "channel", a_t [rows_a][ld_k] against
@@ -228,11 +226,10 @@ extern "C" int32_t px_opm_outer(const px_f16* a_t, const px_f16* b_t, px_f16* x,
   const int sms = sm_count_contract();
   const int grid = total < sms ? total : sms;
   const size_t smem = (size_t)kTcStages * kTcStageBytes + sizeof(TcBarriers) + 1024;
-  if (cudaFuncSetAttribute(trimul_contract_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-      cudaSuccess)
-    return PX_ERR_LAUNCH;
-  trimul_contract_tc_kernel<<<grid, 192, smem, (cudaStream_t)stream>>>(ma, mb, (bf16*)x, (int)rows_a, (int)ld_k,
-                                                                       (int)rows_b, tiles_i, tiles_j, total);
-  return cudaGetLastError() == cudaSuccess ? PX_OK : PX_ERR_LAUNCH;
+  if (!contract_limit.set(trimul_contract_tc_kernel, smem)) return PX_ERR_LAUNCH;
+  return launch_pdl(trimul_contract_tc_kernel, dim3(grid), 192, smem, (cudaStream_t)stream, ma, mb, (bf16*)x, (int)rows_a, (int)ld_k,
+                    (int)rows_b, tiles_i, tiles_j, total)
+             ? PX_OK
+             : PX_ERR_LAUNCH;
 }
 

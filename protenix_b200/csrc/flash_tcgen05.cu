@@ -110,7 +110,7 @@ triatt_flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int q0 = blockIdx.x * 128, h = blockIdx.y, u0 = blockIdx.z * kFRows;
 
-  if (cta_skip_after_error()) return;   // an earlier bounded wait gave up: do not start new work
+  const bool skip = cta_begin();         // an earlier bounded wait gave up: do not start new work
   if (threadIdx.x == 0) {
     for (int b = 0; b < 2; ++b) {
       mbar_init(&bars.bias_full[b], 1);
@@ -132,9 +132,7 @@ triatt_flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
   }
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
+  if (!cta_ready(skip, warp == 4 * kFGroups, bars.tmem_base, kFCols)) return;
   const uint32_t tmem_base = bars.tmem_base;
 
   if (warp >= 4 * kFGroups) {
@@ -388,6 +386,7 @@ triatt_flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
 __global__ void flash_tile_flags_kernel(const float* __restrict__ mb, unsigned long long* __restrict__ flags, int ldm,
                                         int nkt) {
   __shared__ unsigned long long word;
+  pdl_wait();
   const int u = blockIdx.x, w = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) word = 0ull;
   __syncthreads();
@@ -441,14 +440,15 @@ extern "C" int32_t px_triatt_flash(const px_f16* q, const px_f16* k, const px_f1
     return PX_ERR_LAUNCH;
   cudaStream_t st = (cudaStream_t)stream;
   if ((uintptr_t)scratch & 7) return PX_ERR_BAD_ARG;
-  flash_tile_flags_kernel<<<dim3((unsigned)n_u, (unsigned)((nkt + 63) / 64)), 128, 0, st>>>(
-      mask_bias, (unsigned long long*)scratch, (int)ldm, nkt);
-  const size_t smem = FlashLayout::total + 1024;
-  if (cudaFuncSetAttribute(triatt_flash_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-      cudaSuccess)
+  if (!launch_pdl(flash_tile_flags_kernel, dim3((unsigned)n_u, (unsigned)((nkt + 63) / 64)), 128, 0, st, mask_bias,
+                  (unsigned long long*)scratch, (int)ldm, nkt))
     return PX_ERR_LAUNCH;
+  const size_t smem = FlashLayout::total + 1024;
+  static SmemLimit limit;
+  if (!limit.set(triatt_flash_tc_kernel, smem)) return PX_ERR_LAUNCH;
   dim3 grid((unsigned)((n + 127) / 128), kFH, (unsigned)((n_u + kFRows - 1) / kFRows));
-  triatt_flash_tc_kernel<<<grid, kFThreads, smem, st>>>(mq, mk, mv, mbias, mask_bias, (const unsigned long long*)scratch, (bf16*)o,
-                                                  (int)n_u, (int)n, (int)ldm, nkt);
-  return cudaGetLastError() == cudaSuccess ? PX_OK : PX_ERR_LAUNCH;
+  return launch_pdl(triatt_flash_tc_kernel, grid, kFThreads, smem, st, mq, mk, mv, mbias, mask_bias,
+                    (const unsigned long long*)scratch, (bf16*)o, (int)n_u, (int)n, (int)ldm, nkt)
+             ? PX_OK
+             : PX_ERR_LAUNCH;
 }

@@ -53,7 +53,7 @@ opm_out_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
   OpBars& bars = *reinterpret_cast<OpBars*>(sm + OpLayout::bars);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
-  if (cta_skip_after_error()) return;   // an earlier bounded wait gave up: do not start new work
+  const bool skip = cta_begin();         // an earlier bounded wait gave up: do not start new work
   if (threadIdx.x == 0) {
     for (int s = 0; s < kOpStages; ++s) {
       mbar_init(&bars.full[s], 1);
@@ -71,9 +71,7 @@ opm_out_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
   }
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
+  if (!cta_ready(skip, warp == 0, bars.tmem_base, kOpCols)) return;
   const uint32_t tmem_base = bars.tmem_base;
 
   if (warp == 0) {
@@ -210,14 +208,15 @@ static int32_t launch_opm_out(const px_f16* x, const px_f16* w_out, const float*
                    kOpCc))
     return PX_ERR_LAUNCH;
   const size_t smem = OpLayout::total + 1024;
-  if (cudaFuncSetAttribute(opm_out_tc_kernel<Tz>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-    return PX_ERR_LAUNCH;
+  static SmemLimit limit;
+  if (!limit.set(opm_out_tc_kernel<Tz>, smem)) return PX_ERR_LAUNCH;
   const int64_t tiles_j = (n + 127) / 128, total = tiles_j * n_i;
   if (total > 0x7fffffff) return PX_ERR_UNSUPPORTED;
   const int grid = (int)(total < sm_count() ? total : sm_count());
-  opm_out_tc_kernel<Tz><<<grid, 192, smem, st>>>(mx, mw, bias, inv_norm, (const Tz*)z_in, (Tz*)z_out, (int)n, add_residual,
-                                                 (int)tiles_j, (int)total);
-  return cudaGetLastError() == cudaSuccess ? PX_OK : PX_ERR_LAUNCH;
+  return launch_pdl(opm_out_tc_kernel<Tz>, dim3(grid), 192, smem, st, mx, mw, bias, inv_norm, (const Tz*)z_in, (Tz*)z_out, (int)n,
+                    (int)add_residual, tiles_j, total)
+             ? PX_OK
+             : PX_ERR_LAUNCH;
 }
 
 }  // namespace px

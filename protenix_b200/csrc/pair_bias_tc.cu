@@ -20,7 +20,7 @@ constexpr uint32_t kPbColGram = 32;            // tensor memory: projection (16 
 
 struct PbBars {
   TileBars tile;
-  uint64_t acc_full, acc_free;
+  uint64_t acc_full, acc_free, w_full;
   uint32_t tmem_base;
 };
 struct PbLayout {
@@ -37,12 +37,28 @@ static_assert(PbLayout::a % 1024 == 0, "tile ring must keep the swizzle alignmen
 
 static __device__ float g_zero_beta[128];      // stands in for a LayerNorm without bias
 
+// The resident weights: 16 rows (the heads that exist, then zeros) and their correction panel.
+template <bool kF16>
+struct PbWeights {
+  const float *ln_w, *ln_b;
+  const bf16* w;
+  int n_heads;
+  static constexpr int kBytes = PbLayout::a;
+  __device__ __forceinline__ void fold(unsigned char* sm, int, int warp, int warps, int lane, int tid, int threads) const {
+    fold_weight_rows<kF16, kF16>(sm + PbLayout::w, sm + PbLayout::wx, 0, kPbWPanel, w, 0, n_heads, ln_w, ln_b ? ln_b : g_zero_beta, 1.0f,
+                                 warp, warps, lane);
+    for (int i = tid; i < (16 - n_heads) * 16; i += threads)
+      *reinterpret_cast<uint4*>(sm + PbLayout::w + operand_piece_offset(n_heads + i / 16, i % 16, kPbWPanel)) = make_uint4(0u, 0u, 0u, 0u);
+    for (int i = PbLayout::wx + n_heads * 32 + tid * 16; i < kBytes; i += threads * 16)
+      *reinterpret_cast<uint4*>(sm + i) = make_uint4(0u, 0u, 0u, 0u);
+  }
+};
+
 // kF16: the rows are the standardised fp16 copy of an fp32 pair tensor (fp16 weights); otherwise bf16 rows of z.
 template <bool kF16>
 __global__ void __launch_bounds__(kPbThreads, 1)
-pair_bias_tc_kernel(const __grid_constant__ CUtensorMap map_z, const float* __restrict__ ln_w,
-                    const float* __restrict__ ln_b, const bf16* __restrict__ w, float* __restrict__ out, long long rows,
-                    int n_heads, float eps, int n_tiles) {
+pair_bias_tc_kernel(const __grid_constant__ CUtensorMap map_z, const PbWeights<kF16> weights,
+                    const unsigned char* __restrict__ folded, float* __restrict__ out, long long rows, int n_heads, float eps, int n_tiles) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* sm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   PbBars& bars = *reinterpret_cast<PbBars*>(sm + PbLayout::bars);
@@ -59,9 +75,10 @@ pair_bias_tc_kernel(const __grid_constant__ CUtensorMap map_z, const float* __re
   ctx.n_t = (int)rows;
   ctx.swap = 0;
 
-  if (cta_skip_after_error()) return;   // an earlier bounded wait gave up: do not start new work
+  const bool skip = cta_begin();         // an earlier bounded wait gave up: do not start new work
   if (threadIdx.x == 0) {
     tile_bars_init(bars.tile, 1, kF16);
+    mbar_init(&bars.w_full, 1);
     mbar_init(&bars.acc_full, 1);
     mbar_init(&bars.acc_free, 4);
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
@@ -72,22 +89,13 @@ pair_bias_tc_kernel(const __grid_constant__ CUtensorMap map_z, const float* __re
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
   }
-  {
-    fold_weight_rows<kF16, kF16>(sm + PbLayout::w, sm + PbLayout::wx, 0, kPbWPanel, w, 0, n_heads, ln_w, ln_b ? ln_b : g_zero_beta, 1.0f,
-                     warp, kPbWarps, lane);
-    // operand and correction rows of the heads that do not exist
-    for (int i = threadIdx.x; i < (16 - n_heads) * 18; i += kPbThreads) {
-      const int r = n_heads + i / 18, piece = i % 18;
-      unsigned char* dst = piece < 16 ? sm + PbLayout::w + operand_piece_offset(r, piece, kPbWPanel)
-                                      : sm + PbLayout::wx + r * 32 + (piece - 16) * 16;
-      *reinterpret_cast<uint4*>(dst) = make_uint4(0u, 0u, 0u, 0u);
-    }
-    tile_write_ones<kF16>(ctx.tiles, threadIdx.x, kPbThreads);
-    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-  }
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
+  tile_write_ones<kF16>(ctx.tiles, threadIdx.x, kPbThreads);
+  asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+  if (!cta_ready(skip, warp == 8, bars.tmem_base, 256u, [&] {
+        if (folded && threadIdx.x == 0) folded_load(sm, folded, PbWeights<kF16>::kBytes, &bars.w_full);
+      }))
+    return;
+  fold_here(weights, folded, sm, 0, &bars.w_full);
   const uint32_t tmem_base = bars.tmem_base;
 
   if (warp >= 8) {
@@ -96,7 +104,7 @@ pair_bias_tc_kernel(const __grid_constant__ CUtensorMap map_z, const float* __re
         tile_producer_loop(ctx, &map_z);
       } else if (warp == 9) {
         tile_product_loop(ctx, tmem_base, smem_u32(sm + PbLayout::w), kPbWPanel, smem_u32(sm + PbLayout::wx),
-                          umma_idesc_16(128, 16, kF16, kF16), &bars.acc_full, &bars.acc_free);
+                          umma_idesc_16(128, 16, kF16, kF16), &bars.w_full, &bars.acc_full, &bars.acc_free);
       } else if (warp == 10) {
         if (!kF16) tile_gram_loop<kF16>(ctx, tmem_base + kPbColGram);   // standardised rows: nothing to measure
       }
@@ -142,25 +150,50 @@ pair_bias_tc_kernel(const __grid_constant__ CUtensorMap map_z, const float* __re
 PX_DEFINE_FAMILY_HOOKS(pair_bias)
 
 template <bool kF16>
-static int32_t launch_pair_bias(const void* z, const float* ln_w, const float* ln_b, const px_bf16* w, float* out,
-                                int64_t rows, int32_t n_heads, float eps, cudaStream_t st) {
+static int32_t launch_pair_bias(const void* z, const PbWeights<kF16>& weights, const void* folded, float* out, int64_t rows,
+                                int32_t n_heads, float eps, cudaStream_t st) {
   CUtensorMap mz;
   if (!make_map_3d(&mz, kF16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, z, 128, (uint64_t)rows, 1,
                    256, (uint64_t)rows * 256, 64, 128, CU_TENSOR_MAP_SWIZZLE_128B, 1))
     return PX_ERR_LAUNCH;
   const size_t smem = PbLayout::total + 1024;
-  if (cudaFuncSetAttribute(pair_bias_tc_kernel<kF16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-    return PX_ERR_LAUNCH;
+  static SmemLimit limit;
+  if (!limit.set(pair_bias_tc_kernel<kF16>, smem)) return PX_ERR_LAUNCH;
   const int64_t n_tiles = (rows + 127) / 128;
   const int grid = (int)(n_tiles < sm_count() ? n_tiles : sm_count());
-  pair_bias_tc_kernel<kF16><<<grid, kPbThreads, smem, st>>>(mz, ln_w, ln_b, (const bf16*)w, out, (long long)rows,
-                                                          n_heads, eps, (int)n_tiles);
-  return cudaGetLastError() == cudaSuccess ? PX_OK : PX_ERR_LAUNCH;
+  return launch_pdl(pair_bias_tc_kernel<kF16>, dim3(grid), kPbThreads, smem, st, mz, weights, (const unsigned char*)folded, out,
+                    (long long)rows, (int)n_heads, eps, (int)n_tiles)
+             ? PX_OK
+             : PX_ERR_LAUNCH;
 }
 
 }  // namespace px
 
 using namespace px;
+
+extern "C" int64_t px_pair_bias_folded_bytes(void) { return PbWeights<true>::kBytes; }
+
+extern "C" int32_t px_pair_bias_fold(const float* ln_w, const float* ln_b, const px_w16* w, int32_t n_heads, int32_t rows_dtype,
+                                     void* folded, void* stream) {
+  if (!ln_w || !w || !folded || (((uintptr_t)w | (uintptr_t)ln_w | (uintptr_t)ln_b | (uintptr_t)folded) & 15)) return PX_ERR_BAD_ARG;
+  if (n_heads <= 0 || n_heads > 16 || (rows_dtype != PX_F16 && rows_dtype != PX_BF16)) return PX_ERR_UNSUPPORTED;
+  cudaStream_t st = (cudaStream_t)stream;
+  return (rows_dtype == PX_F16 ? launch_fold(PbWeights<true>{ln_w, ln_b, (const bf16*)w, n_heads}, 1, folded, st)
+                               : launch_fold(PbWeights<false>{ln_w, ln_b, (const bf16*)w, n_heads}, 1, folded, st))
+             ? PX_OK
+             : PX_ERR_LAUNCH;
+}
+
+extern "C" int32_t px_pair_bias_proj_folded(const void* z, int32_t z_dtype, const void* folded, float* out, int64_t rows,
+                                            int32_t n_heads, float eps, void* stream) {
+  if (!z || !folded || !out || rows < 0 || (((uintptr_t)z | (uintptr_t)folded) & 15)) return PX_ERR_BAD_ARG;
+  if (n_heads <= 0 || n_heads > 16 || rows > 0x3fffffff) return PX_ERR_UNSUPPORTED;
+  if (rows == 0) return PX_OK;
+  cudaStream_t st = (cudaStream_t)stream;
+  if (z_dtype == PX_F16) return launch_pair_bias<true>(z, PbWeights<true>{}, folded, out, rows, n_heads, eps, st);
+  if (z_dtype == PX_BF16) return launch_pair_bias<false>(z, PbWeights<false>{}, folded, out, rows, n_heads, eps, st);
+  return PX_ERR_UNSUPPORTED;
+}
 
 extern "C" int32_t px_pair_bias_proj(const void* z, int32_t z_dtype, const float* ln_w, const float* ln_b,
                                      const px_bf16* w, float* out, int64_t rows, int32_t n_heads, float eps,
@@ -170,7 +203,10 @@ extern "C" int32_t px_pair_bias_proj(const void* z, int32_t z_dtype, const float
   if (((uintptr_t)z | (uintptr_t)w | (uintptr_t)ln_w | (uintptr_t)ln_b) & 15) return PX_ERR_BAD_ARG;
   if (rows == 0) return PX_OK;
   if (rows > 0x3fffffff) return PX_ERR_UNSUPPORTED;
-  if (z_dtype == PX_F16) return launch_pair_bias<true>(z, ln_w, ln_b, w, out, rows, n_heads, eps, (cudaStream_t)stream);
-  if (z_dtype == PX_BF16) return launch_pair_bias<false>(z, ln_w, ln_b, w, out, rows, n_heads, eps, (cudaStream_t)stream);
+  cudaStream_t st = (cudaStream_t)stream;
+  if (z_dtype == PX_F16)
+    return launch_pair_bias<true>(z, PbWeights<true>{ln_w, ln_b, (const bf16*)w, n_heads}, nullptr, out, rows, n_heads, eps, st);
+  if (z_dtype == PX_BF16)
+    return launch_pair_bias<false>(z, PbWeights<false>{ln_w, ln_b, (const bf16*)w, n_heads}, nullptr, out, rows, n_heads, eps, st);
   return PX_ERR_UNSUPPORTED;
 }

@@ -104,6 +104,46 @@ __device__ __forceinline__ void fold_weight_rows(unsigned char* dst, unsigned ch
   }
 }
 
+// Folded weights.  Folding 256 rows takes a CTA 5 to 6 us (global loads, two warp sums a row), a third of a row kernel at
+// N = 128, and it is the same work on every launch.  A caller that keeps the weights folds them once (`fold_kernel` writes the
+// image of the operands as they lie in shared memory, for each variant of CTA); the row kernels then fetch the image with one
+// bulk copy that overlaps the end of the kernel before them.  Without an image the CTA folds the weights itself.
+__device__ __forceinline__ void folded_load(unsigned char* dst, const unsigned char* image, uint32_t bytes, uint64_t* bar) {
+  mbar_expect_tx(bar, bytes);
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(smem_u32(dst)),
+               "l"(image), "r"(bytes), "r"(smem_u32(bar))
+               : "memory");
+}
+constexpr int kFoldThreads = 768;
+// One CTA per variant: weights.fold(sm, variant, warp, warps, lane, tid, threads) writes W::kBytes bytes at sm.
+template <typename W>
+__global__ void __launch_bounds__(kFoldThreads, 1) fold_kernel(const W weights, unsigned char* __restrict__ image) {
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  unsigned char* sm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  weights.fold(sm, blockIdx.x, threadIdx.x >> 5, kFoldThreads / 32, threadIdx.x & 31, threadIdx.x, kFoldThreads);
+  __syncthreads();
+  for (int i = threadIdx.x; i < W::kBytes / 16; i += kFoldThreads)
+    reinterpret_cast<uint4*>(image + (size_t)blockIdx.x * W::kBytes)[i] = reinterpret_cast<const uint4*>(sm)[i];
+}
+template <typename W>
+static bool launch_fold(const W& weights, int variants, void* image, cudaStream_t st) {
+  static SmemLimit limit;
+  if (!limit.set(fold_kernel<W>, W::kBytes + 1024)) return false;
+  fold_kernel<W><<<variants, kFoldThreads, W::kBytes + 1024, st>>>(weights, (unsigned char*)image);
+  return cudaGetLastError() == cudaSuccess;
+}
+// In a row kernel, after cta_ready: folds the weights here unless their image is on its way.  `full` is what the issuing threads
+// wait for before their first product.
+template <typename W>
+__device__ __forceinline__ void fold_here(const W& weights, const unsigned char* image, unsigned char* sm, int variant,
+                                          uint64_t* full) {
+  if (image) return;
+  weights.fold(sm, variant, threadIdx.x >> 5, blockDim.x >> 5, threadIdx.x & 31, threadIdx.x, blockDim.x);
+  asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+  __syncthreads();
+  if (threadIdx.x == 0) mbar_arrive(full);
+}
+
 // The register of a 32-entry array that belongs to this lane (arr[lane] without local memory).
 __device__ __forceinline__ float select_own(const uint32_t (&arr)[32], int lane) {
   uint32_t v = 0;
@@ -316,8 +356,10 @@ __device__ __forceinline__ void tile_stats_loop(const TileCtx& c, float eps, uin
 // hand the accumulator back and forth with the epilogue warps: arrays of n_acc barriers, tile k uses accumulator
 // k % n_acc at d_tmem + (k % n_acc) * acc_cols (n_acc = 1 or 2).
 __device__ __forceinline__ void tile_product_loop(const TileCtx& c, uint32_t d_tmem, uint32_t w_addr, int w_panel,
-                                                  uint32_t wx_addr, uint32_t idesc, uint64_t* acc_full,
-                                                  uint64_t* acc_free, int n_acc = 1, uint32_t acc_cols = 0) {
+                                                  uint32_t wx_addr, uint32_t idesc, uint64_t* w_full,
+                                                  uint64_t* acc_full, uint64_t* acc_free, int n_acc = 1,
+                                                  uint32_t acc_cols = 0) {
+  if (!mbar_wait(w_full, 0, 4u)) return;         // the resident weights
   const uint64_t wx_desc = umma_desc_sw32(wx_addr);
   // the correction step multiplies bf16 head/tail pairs whatever the format of the main operands; M and N as `idesc`
   const uint32_t idesc_corr = idesc | (1u << 7) | (1u << 10);

@@ -14,9 +14,29 @@ static __device__ long long g_wait_limit = 1ll << 28;
 // True once any bounded wait of this translation unit's kernels has given up (until the host reads the word).
 __device__ __forceinline__ bool tc_error_seen() { return *reinterpret_cast<volatile unsigned int*>(&g_tc_error) != 0; }
 
-// Called by every thread at the top of a kernel: after a wait has run out, CTAs that start later skip their work
-// (the decision is uniform over the CTA), so a failure holds the GPU for one wait limit, not one per CTA.
-__device__ __forceinline__ bool cta_skip_after_error() { return __syncthreads_or(tc_error_seen()) != 0; }
+// Called by every thread at the top of a kernel: whether a wait has run out before.  The answer is not needed before
+// cta_ready, so the read of the flag overlaps the set-up.
+__device__ __forceinline__ bool cta_begin() { return tc_error_seen(); }
+__device__ __forceinline__ void tc_fence_before();
+__device__ __forceinline__ void tc_fence_after();
+// The barrier after the set-up, and the wait for the kernels before this one.  False (for every thread of the CTA): a wait ran
+// out earlier and the CTA shall do no work, so that a failure holds the GPU for one wait limit and not one per CTA; its tensor
+// memory is given back here by the warp that allocated it.
+// before_wait(): work that needs nothing of earlier kernels (loads of the resident weights).
+struct Nothing {
+  __device__ __forceinline__ void operator()() const {}
+};
+template <typename F = Nothing>
+__device__ __forceinline__ bool cta_ready(bool skip, bool alloc_warp, const uint32_t& tmem_base, uint32_t cols, F before_wait = F()) {
+  tc_fence_before();
+  const bool stop = __syncthreads_or(skip) != 0;
+  tc_fence_after();
+  if (!stop) before_wait();
+  pdl_wait();
+  if (stop && alloc_warp)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem_base), "r"(cols) : "memory");
+  return !stop;
+}
 
 // Called by every thread at the end of a kernel, in place of the closing __syncthreads(): when a wait ran out, copies
 // may still be in flight towards this CTA's shared memory, so the CTA lingers before it frees anything.

@@ -25,7 +25,7 @@ constexpr uint32_t kRcColGram = 128;           // tensor memory: projection (128
 
 struct RcBars {
   TileBars tile;
-  uint64_t acc_full, acc_free, res_full[kTileStages], res_empty[kTileStages];
+  uint64_t w_full, acc_full, acc_free, res_full[kTileStages], res_empty[kTileStages];
   uint32_t tmem_base;
 };
 struct RcLayout {
@@ -67,9 +67,10 @@ recycle_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_consta
   ctx.n_t = (int)rows;
   ctx.swap = 0;
 
-  if (cta_skip_after_error()) return;   // an earlier bounded wait gave up: do not start new work
+  const bool skip = cta_begin();         // an earlier bounded wait gave up: do not start new work
   if (threadIdx.x == 0) {
     tile_bars_init(bars.tile, 1, kF16);
+    mbar_init(&bars.w_full, 1);
     mbar_init(&bars.acc_full, 1);
     mbar_init(&bars.acc_free, 8);
     for (int s = 0; s < kTileStages; ++s) {
@@ -84,13 +85,14 @@ recycle_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_consta
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
   }
-  fold_weight_rows<kF16, kF16>(sm + RcLayout::w, sm + RcLayout::wx, 0, kPanelBytes, w, 0, 128, ln_w, ln_b ? ln_b : g_rc_zero_beta, 1.0f,
-                   warp, kRcWarps, lane);
   tile_write_ones<kF16>(ctx.tiles, threadIdx.x, kRcThreads);
   asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-  tc_fence_before();
+  if (!cta_ready(skip, warp == 12, bars.tmem_base, 512u)) return;
+  fold_weight_rows<kF16, kF16>(sm + RcLayout::w, sm + RcLayout::wx, 0, kPanelBytes, w, 0, 128, ln_w, ln_b ? ln_b : g_rc_zero_beta, 1.0f,
+                   warp, kRcWarps, lane);
+  asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
   __syncthreads();
-  tc_fence_after();
+  if (threadIdx.x == 0) mbar_arrive(&bars.w_full);
   const uint32_t tmem_base = bars.tmem_base;
 
   if (warp >= 12) {
@@ -113,7 +115,7 @@ recycle_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_consta
         }
       } else if (warp == 13) {
         tile_product_loop(ctx, tmem_base, smem_u32(sm + RcLayout::w), kPanelBytes, smem_u32(sm + RcLayout::wx),
-                          umma_idesc_16(128, 128, kF16, kF16), &bars.acc_full, &bars.acc_free);
+                          umma_idesc_16(128, 128, kF16, kF16), &bars.w_full, &bars.acc_full, &bars.acc_free);
       } else if (warp == 14) {
         if (!kF16) tile_gram_loop<kF16>(ctx, tmem_base + kRcColGram);   // standardised rows: nothing to measure
       }
@@ -234,13 +236,14 @@ static int32_t launch_recycle(const void* z, const void* z_init, void* out, cons
     memset(&mo, 0, sizeof(mo));
   }
   const size_t smem = RcLayout::total + 1024;
-  if (cudaFuncSetAttribute(recycle_tc_kernel<Tz>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-    return PX_ERR_LAUNCH;
+  static SmemLimit limit;
+  if (!limit.set(recycle_tc_kernel<Tz>, smem)) return PX_ERR_LAUNCH;
   const int64_t n_tiles = (rows + 127) / 128;
   const int grid = (int)(n_tiles < sm_count() ? n_tiles : sm_count());
-  recycle_tc_kernel<Tz><<<grid, kRcThreads, smem, st>>>(mz, mi, mo, (const Tz*)z_init, (Tz*)out, ln_w, ln_b,
-                                                        (const bf16*)w, (long long)rows, eps, (int)n_tiles);
-  return cudaGetLastError() == cudaSuccess ? PX_OK : PX_ERR_LAUNCH;
+  return launch_pdl(recycle_tc_kernel<Tz>, dim3(grid), kRcThreads, smem, st, mz, mi, mo, (const Tz*)z_init, (Tz*)out, ln_w, ln_b,
+                    (const bf16*)w, (long long)rows, eps, (int)n_tiles)
+             ? PX_OK
+             : PX_ERR_LAUNCH;
 }
 
 }  // namespace px

@@ -4,14 +4,14 @@
 // the same mbar_wait the tensor-core kernels use; the wait gives up after the configured limit, records its code,
 // and the kernel returns through the same teardown helper.  Nothing faults and the context stays usable: the host
 // reads the flag with px_device_error_flags.  A second launch while the flag is still set returns at once
-// (cta_skip_after_error), which the out word shows.
+// (cta_begin), which the out word shows.
 #include "px_tcgen05.cuh"
 
 namespace px {
 
 __global__ void selftest_wait_kernel(unsigned int* out) {
   __shared__ uint64_t bar;
-  if (cta_skip_after_error()) {
+  if (__syncthreads_or(cta_begin())) {
     if (threadIdx.x == 0) out[0] = 2u;   // skipped: an earlier failure is still recorded
     return;
   }

@@ -82,6 +82,7 @@ template <typename T>
 __global__ void __launch_bounds__(128) split_rows_kernel(const T* __restrict__ x, const float* __restrict__ gamma,
                                                          const float* __restrict__ beta, bf16* __restrict__ out, int rows,
                                                          float eps) {
+  pdl_wait();
   const int row = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (row >= rows) return;
   float4 v[3];
@@ -149,7 +150,7 @@ split_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n0 = blockIdx.x * kSgBN, m0 = blockIdx.y * 128, kc0 = blockIdx.z * g.chunks;
 
-  const bool skip = cta_skip_after_error();      // an earlier bounded wait gave up: do no work, but meet the barriers
+  const bool stop = cta_begin();                 // an earlier bounded wait gave up: do no work, but meet the barriers
   if (threadIdx.x == 0) {
     for (int s = 0; s < kSgStages; ++s) {
       mbar_init(&bars.full[s], 1);
@@ -165,8 +166,9 @@ split_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
   }
   tc_fence_before();
-  __syncthreads();
+  const bool skip = __syncthreads_or(stop) != 0;
   tc_fence_after();
+  pdl_wait();
   const uint32_t tmem_base = bars.tmem_base;
   float v[kSgBN];                                // epilogue: this thread's row of the tile
   bool ok = !skip;
@@ -326,6 +328,7 @@ struct SaTile {
 __global__ void __launch_bounds__(128 * kSaGroups, 2)
 single_attention_kernel(const float* __restrict__ qkvg, const float* __restrict__ bias, bf16* __restrict__ out, int n) {
   extern __shared__ __align__(16) unsigned char sa_raw[];
+  pdl_wait();
   float(*qs)[kSaQ] = reinterpret_cast<float(*)[kSaQ]>(sa_raw);
   const int grp = threadIdx.x >> 7, tid = threadIdx.x & 127, ty = tid >> 4, tx = tid & 15;
   SaTile& t = reinterpret_cast<SaTile*>(sa_raw + kSd * kSaQ * 4)[grp];
@@ -475,19 +478,21 @@ static bool launch_split_gemm(const bf16* a, const bf16* w, int64_t w_rows, int6
   if (!make_plane_map(&ma, a, g.rows, k, 128) || !make_plane_map(&mw, w, w_rows, k, kSgBN)) return false;
   constexpr size_t smem = (size_t)kSgStages * kSgStageBytes + sizeof(SgBars) + 1024;
   static_assert(smem <= 232448, "shared memory budget");
-  if (cudaFuncSetAttribute(split_gemm_tc_kernel<kMode, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-    return false;
+  static SmemLimit limit;
+  if (!limit.set(split_gemm_tc_kernel<kMode, T>, smem)) return false;
   g.chunks = (int)(k / 64 / split);
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = 1, at[0].val.clusterDim.y = 1, at[0].val.clusterDim.z = (unsigned)split;
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  at[1].id = cudaLaunchAttributeClusterDimension;
+  at[1].val.clusterDim.x = 1, at[1].val.clusterDim.y = 1, at[1].val.clusterDim.z = (unsigned)split;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(w_rows / kSgBN), (unsigned)((g.rows + 127) / 128), (unsigned)split);
   cfg.blockDim = dim3(kSgThreads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
   cfg.attrs = at;
-  cfg.numAttrs = split > 1 ? 1 : 0;
+  cfg.numAttrs = split > 1 ? 2 : 1;
   return cudaLaunchKernelEx(&cfg, split_gemm_tc_kernel<kMode, T>, ma, mw, g) == cudaSuccess;
 }
 
@@ -500,16 +505,17 @@ static int32_t run_single(const void* s, void* s_out, const bf16* w, const float
   const unsigned lnb = (unsigned)((n + 3) / 4);
   SgArgs g = {};
   g.rows = n;
-  split_rows_kernel<T><<<lnb, 128, 0, st>>>((const T*)s, ln[0], ln[1], xp, n, eps_att);
+  if (!launch_pdl(split_rows_kernel<T>, dim3(lnb), 128, 0, st, (const T*)s, ln[0], ln[1], xp, n, eps_att)) return PX_ERR_LAUNCH;
   g.bias = q_bias, g.out_f = qkvg, g.scale = 1.0f / sqrtf((float)kSd);
   if (!launch_split_gemm<kSgQkvg, T>(xp, w + kSwQkvg, kSf, kSc, 1, g, st)) return PX_ERR_LAUNCH;
   constexpr int sa_smem = kSd * kSaQ * 4 + kSaGroups * (int)sizeof(SaTile);
-  if (cudaFuncSetAttribute(single_attention_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, sa_smem) != cudaSuccess)
+  static SmemLimit limit;
+  if (!limit.set(single_attention_kernel, sa_smem) ||
+      !launch_pdl(single_attention_kernel, dim3((unsigned)((n + kSaQ - 1) / kSaQ), kSh), 128 * kSaGroups, sa_smem, st, qkvg, bias, xp, n))
     return PX_ERR_LAUNCH;
-  single_attention_kernel<<<dim3((unsigned)((n + kSaQ - 1) / kSaQ), kSh), 128 * kSaGroups, sa_smem, st>>>(qkvg, bias, xp, n);
   g.res = s, g.out = s_out;
   if (!launch_split_gemm<kSgRes, T>(xp, w + kSwO, kSc, kSc, 2, g, st)) return PX_ERR_LAUNCH;
-  split_rows_kernel<T><<<lnb, 128, 0, st>>>((const T*)s_out, ln[2], ln[3], xp, n, eps_tr);
+  if (!launch_pdl(split_rows_kernel<T>, dim3(lnb), 128, 0, st, (const T*)s_out, ln[2], ln[3], xp, n, eps_tr)) return PX_ERR_LAUNCH;
   g.out_planes = hp;
   if (!launch_split_gemm<kSgSwiglu, T>(xp, w + kSwAb, 2 * kSf, kSc, 1, g, st)) return PX_ERR_LAUNCH;
   g.res = s_out, g.out = s_out;

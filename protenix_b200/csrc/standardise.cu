@@ -18,6 +18,7 @@ constexpr int kStdRowsPerBatch = 8;
 
 __global__ void __launch_bounds__(256) standardise_rows_kernel(const float* __restrict__ z, __half* __restrict__ zn,
                                                                long long rows, float eps) {
+  pdl_wait();
   const int lane = threadIdx.x & 31;
   const long long warp = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const long long nwarps = (long long)gridDim.x * (blockDim.x >> 5);
@@ -92,6 +93,8 @@ extern "C" int32_t px_standardise_rows(const float* z, px_f16* zn, int64_t rows,
   const long long batches = (rows + px::kStdRowsPerBatch - 1) / px::kStdRowsPerBatch;
   long long grid = (batches + 7) / 8;                    // eight warps per CTA
   if (grid > 8ll * sms) grid = 8ll * sms;                // a multiple of the SM count, eight CTAs resident per SM
-  px::standardise_rows_kernel<<<(unsigned)grid, 256, 0, (cudaStream_t)stream>>>(z, (__half*)zn, (long long)rows, eps);
-  return cudaGetLastError() == cudaSuccess ? PX_OK : PX_ERR_LAUNCH;
+  return px::launch_pdl(px::standardise_rows_kernel, dim3((unsigned)grid), 256, 0, (cudaStream_t)stream, z, (__half*)zn,
+                        (long long)rows, eps)
+             ? PX_OK
+             : PX_ERR_LAUNCH;
 }

@@ -44,9 +44,12 @@ constexpr int64_t kCz = 128, kCs = 384, kHeadsSingle = 16, kHeads = 4, kHeadDim 
 // ---- the C ABI, by the handle of the loaded library ------------------------------------------------------------------
 #define PX_FUNCTIONS(X)                                                                                                  \
   X(px_status_string) X(px_ld) X(px_ld_mask) X(px_layer_norm_fwd_params) X(px_layer_norm_bwd_params)                     \
-  X(px_scale_add_rowwise) X(px_standardise_rows) X(px_trimul_in_proj) X(px_trimul_contract) X(px_trimul_out)             \
-  X(px_trimul_workspace_bytes) X(px_triatt_in_proj) X(px_triatt_flash) X(px_triatt_flash_scratch_bytes) X(px_triatt_out) \
-  X(px_triatt_workspace_bytes) X(px_transition) X(px_pair_bias_proj) X(px_single_weights_bytes)                          \
+  X(px_scale_add_rowwise) X(px_standardise_rows) X(px_trimul_in_folded_bytes) X(px_trimul_in_fold)                       \
+  X(px_trimul_in_proj_folded) X(px_trimul_contract) X(px_trimul_out_folded_bytes) X(px_trimul_out_fold)                  \
+  X(px_trimul_out_folded) X(px_trimul_workspace_bytes) X(px_triatt_in_folded_bytes) X(px_triatt_in_fold)                 \
+  X(px_triatt_in_proj_folded) X(px_triatt_flash) X(px_triatt_flash_scratch_bytes) X(px_triatt_out_folded_bytes)          \
+  X(px_triatt_out_fold) X(px_triatt_out_folded) X(px_triatt_workspace_bytes) X(px_transition)                            \
+  X(px_pair_bias_folded_bytes) X(px_pair_bias_fold) X(px_pair_bias_proj_folded) X(px_single_weights_bytes)               \
   X(px_single_workspace_bytes) X(px_single_prepare) X(px_single_update)
 struct Abi {
 #define X(f) decltype(&::f) f = nullptr;
@@ -139,7 +142,9 @@ const float* fptr(const Tensor& t) { return t.defined() ? (const float*)t.data_p
 
 // ---- parameters of a module -----------------------------------------------------------------------------------------
 // What a parameter becomes: 'f' an fp32 vector, 'z' a matrix in the format of the pair tensor's rows (bf16 rows: bf16, fp32
-// rows: fp16), 'h' an fp16 matrix, 's' one of the eight matrices of the single branch (laid out together).
+// rows: fp16), 'h' an fp16 matrix, 's' an fp32 matrix.  What the group becomes then: kMul, kAtt and kBias the folded weights
+// of their row kernels (in, out), kSingle the laid-out matrices of the single branch behind its vectors, kPlain nothing more.
+enum Group { kPlain, kMul, kAtt, kBias, kSingle };
 struct Prepared {
   std::vector<Tensor> t[2];          // by format of z: 0 fp32, 1 bf16
   std::vector<const void*> p[2];
@@ -152,7 +157,12 @@ struct Prepared {
 class Params {
  public:
   // checks: (dict, name) of submodules; params: (dict, name, kind, shape); scalars: (dict, name)
-  Params(const py::list& checks, const py::list& params, const py::list& scalars) {
+  Params(const std::string& group, const py::list& checks, const py::list& params, const py::list& scalars) {
+    const char* names[] = {"plain", "mul", "att", "bias", "single"};
+    int g = 0;
+    while (g < 5 && group != names[g]) ++g;
+    if (g == 5) fail("unknown parameter group " + group);
+    group_ = (Group)g;
     for (const auto& c : checks) {
       const auto t = c.cast<py::tuple>();
       checks_.push_back({t[0].cast<py::dict>(), t[1].cast<py::object>(), py::none()});
@@ -236,46 +246,74 @@ class Params {
 
   void make(Prepared& p, int zf, const at::Device& dev) {
     at::NoGradGuard no_grad;
-    std::vector<Tensor> singles;
-    p.t[zf].clear();
-    p.p[zf].clear();
+    std::vector<Tensor> t;
     for (size_t i = 0; i < params_.size(); ++i) {
       PyObject* o = find(params_[i]);
-      Tensor t;
+      Tensor v;
       if (o != Py_None) {
-        t = THPVariable_Unpack(o).detach();
-        need_cuda(t, "parameters");
-        if (t.device() != dev) fail("parameters and inputs must be on the same device");
-        if (!t.sizes().equals(shape_[i]) || !t.is_floating_point())
+        v = THPVariable_Unpack(o).detach();
+        need_cuda(v, "parameters");
+        if (v.device() != dev) fail("parameters and inputs must be on the same device");
+        if (!v.sizes().equals(shape_[i]) || !v.is_floating_point())
           fail("a parameter must be a floating-point tensor of the shape the kernels are built for");
         const auto want = kind_[i] == 'f' || kind_[i] == 's' ? at::kFloat
                           : kind_[i] == 'z' && zf == 1       ? at::kBFloat16
                                                              : at::kHalf;
-        t = t.to(want).contiguous();
-        if (kind_[i] == 's') singles.push_back(t);
-        if (((uintptr_t)t.data_ptr() & 15) != 0) t = t.clone();
+        v = v.to(want).contiguous();
+        if (((uintptr_t)v.data_ptr() & 15) != 0) v = v.clone();
       }
-      p.t[zf].push_back(t);
-      p.p[zf].push_back(t.defined() ? t.data_ptr() : nullptr);
+      t.push_back(v);
     }
-    if (!singles.empty()) {
-      const Tensor out = bytes_like(singles[0], abi.px_single_weights_bytes());
-      const float* w[8];
-      for (int i = 0; i < 8; ++i) w[i] = (const float*)singles[i].data_ptr();
-      const cudaStream_t st = at::cuda::getCurrentCUDAStream(dev.index());
-      launch("px_single_prepare", st, [&] {
-        return abi.px_single_prepare(w[0], w[1], w[2], w[3], w[4], w[5], w[6], w[7], out.data_ptr(), st);
+    const auto stream = at::cuda::getCurrentCUDAStream(dev.index());
+    const cudaStream_t st = stream;
+    const int rows = zf == 1 ? PX_BF16 : PX_F16;
+    const auto byte = at::TensorOptions().device(dev).dtype(at::kByte);
+    auto f = [&](int i) { return t[i].defined() ? (const float*)t[i].data_ptr() : nullptr; };
+    auto w = [&](int i) { return (const px_w16*)t[i].data_ptr(); };
+    if (group_ == kMul) {
+      const Tensor in = at::empty({abi.px_trimul_in_folded_bytes()}, byte), out = at::empty({abi.px_trimul_out_folded_bytes()}, byte);
+      launch("px_trimul_in_fold", st, [&] {
+        return abi.px_trimul_in_fold(f(0), f(1), w(4), w(5), w(6), w(7), rows, in.data_ptr(), st);
       });
-      for (size_t i = 0; i < params_.size(); ++i)      // the planes replace the matrices
-        if (kind_[i] == 's') p.t[zf][i] = Tensor(), p.p[zf][i] = nullptr;
-      p.t[zf].push_back(out);
-      p.p[zf].push_back(out.data_ptr());
+      launch("px_trimul_out_fold", st, [&] {
+        return abi.px_trimul_out_fold(f(0), f(1), f(2), f(3), w(8), w(9), rows, out.data_ptr(), st);
+      });
+      t = {in, out};
+    } else if (group_ == kAtt) {
+      const Tensor in = at::empty({abi.px_triatt_in_folded_bytes()}, byte), out = at::empty({abi.px_triatt_out_folded_bytes()}, byte);
+      launch("px_triatt_in_fold", st, [&] {
+        return abi.px_triatt_in_fold(f(0), f(1), w(3), w(4), w(5), w(2), rows, in.data_ptr(), st);
+      });
+      launch("px_triatt_out_fold", st, [&] { return abi.px_triatt_out_fold(f(0), f(1), w(6), w(7), rows, out.data_ptr(), st); });
+      t = {in, out};
+    } else if (group_ == kBias) {
+      const Tensor out = at::empty({abi.px_pair_bias_folded_bytes()}, byte);
+      launch("px_pair_bias_fold", st, [&] {
+        return abi.px_pair_bias_fold(f(0), f(1), w(2), (int32_t)shape_[2][0], rows, out.data_ptr(), st);
+      });
+      t = {out};
+    } else if (group_ == kSingle) {
+      const Tensor out = at::empty({abi.px_single_weights_bytes()}, byte);
+      launch("px_single_prepare", st, [&] {
+        return abi.px_single_prepare(f(5), f(6), f(7), f(8), f(9), f(10), f(11), f(12), out.data_ptr(), st);
+      });
+      t.resize(5);
+      t.push_back(out);
     }
+    p.t[zf] = t;
+    p.p[zf].clear();
+    for (const Tensor& v : t) p.p[zf].push_back(v.defined() ? v.data_ptr() : nullptr);
+    // The row kernels fetch folded weights before the kernels in front of them are complete (programmatic launch): once per
+    // change of the weights, the host waits for the fold.
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    cudaStreamIsCapturing(st, &capturing);
+    if (capturing == cudaStreamCaptureStatusNone) cudaStreamSynchronize(st);
     p.made_on[zf] = at::cuda::getCurrentCUDAStream(dev.index());
     p.ready[zf].record(at::cuda::getCurrentCUDAStream(dev.index()));
     p.have[zf] = true;
   }
 
+  Group group_;
   std::vector<Slot> checks_, params_, scalars_;
   std::vector<char> kind_;
   std::vector<std::vector<int64_t>> shape_;
@@ -317,14 +355,12 @@ void tri_mul(const PairCall& c, const Prepared& pr, const void* z_in, void* z_ou
     }
     rows = zn, rows_dt = PX_F16;
   }
-  auto f = [&](int i) { return (const float*)p[i]; };
-  auto w = [&](int i) { return (const px_w16*)p[i]; };
   launch("px_trimul_in_proj", c.st, [&] {
-    return abi.px_trimul_in_proj(rows, rows_dt, c.mask, f(0), f(1), w(4), w(5), w(6), w(7), a, b, n, n, ld, incoming, eps, c.st);
+    return abi.px_trimul_in_proj_folded(rows, rows_dt, c.mask, p[0], a, b, n, n, ld, incoming, eps, c.st);
   });
   launch("px_trimul_contract", c.st, [&] { return abi.px_trimul_contract(a, b, x, kCz, n, ld, c.st); });
   launch("px_trimul_out", c.st, [&] {
-    return abi.px_trimul_out(x, z_in, (const px_f16*)zn, z_out, c.dt, f(0), f(1), f(2), f(3), w(8), w(9), n, n, ld, add, eps, c.st);
+    return abi.px_trimul_out_folded(x, z_in, (const px_f16*)zn, z_out, c.dt, p[1], n, n, ld, add, eps, c.st);
   });
 }
 
@@ -344,17 +380,15 @@ void tri_att(const PairCall& c, const Prepared& pr, const void* z_in, void* z_ou
     standardise(c, z_in, (void*)zn, eps);
     rows = zn, rows_dt = PX_F16;
   }
-  auto f = [&](int i) { return (const float*)p[i]; };
-  auto w = [&](int i) { return (const px_w16*)p[i]; };
   launch("px_triatt_in_proj", c.st, [&] {
-    return abi.px_triatt_in_proj(rows, rows_dt, c.mask, f(0), f(1), w(3), w(4), w(5), w(2), q, k, v, (float*)bias, (float*)mbias, n, n,
-                                 ldm, ending, eps, inf, c.st);
+    return abi.px_triatt_in_proj_folded(rows, rows_dt, c.mask, p[0], q, k, v, (float*)bias, (float*)mbias, n, n, ldm, ending, eps, inf,
+                                        c.st);
   });
   launch("px_triatt_flash", c.st, [&] {
     return abi.px_triatt_flash(q, k, v, (const float*)bias, (const float*)mbias, o, flags, n, n, ldm, c.st);
   });
   launch("px_triatt_out", c.st, [&] {
-    return abi.px_triatt_out(o, z_in, (const px_f16*)zn, z_out, c.dt, f(0), f(1), w(6), w(7), n, n, ending, add, eps, c.st);
+    return abi.px_triatt_out_folded(o, z_in, (const px_f16*)zn, z_out, c.dt, p[1], n, n, ending, add, eps, c.st);
   });
 }
 
@@ -531,8 +565,8 @@ std::tuple<OptTensor, Tensor> stack_forward(const std::vector<std::shared_ptr<Bl
     if (aside && k >= 2) side_done[turn].block(main);       // the single branch two blocks ago has read this buffer
     const auto& p = r.pair_bias->p[zf];
     launch("px_pair_bias_proj", c.st, [&] {
-      return abi.px_pair_bias_proj(rows, fp32 ? PX_F16 : PX_BF16, (const float*)p[0], (const float*)p[1], (const px_w16*)p[2],
-                                   (float*)bias[turn].data_ptr(), n * n, kHeadsSingle, r.pair_bias->scalars[0], c.st);
+      return abi.px_pair_bias_proj_folded(rows, fp32 ? PX_F16 : PX_BF16, p[0], (float*)bias[turn].data_ptr(), n * n, kHeadsSingle,
+                                          r.pair_bias->scalars[0], c.st);
     });
     if (aside) {
       bias_ready[turn].record(main);
@@ -699,7 +733,7 @@ PYBIND11_MODULE(_C, m) {
   m.def("layer_norm", &layer_norm);
   m.def("dropout_add", &dropout_add);
   py::class_<Params, std::shared_ptr<Params>>(m, "Params")
-      .def(py::init<py::list, py::list, py::list>())
+      .def(py::init<std::string, py::list, py::list, py::list>())
       .def("current", &Params::current)
       // kept in a module's __dict__: a copy or an unpickled module makes its own
       .def("__deepcopy__", [](const Params&, py::dict) { return py::none(); })

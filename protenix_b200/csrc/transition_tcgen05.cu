@@ -78,7 +78,7 @@ transition_tc_kernel(const __grid_constant__ CUtensorMap map_wa, const __grid_co
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int first_tile = blockIdx.x, tile_step = gridDim.x;
 
-  if (cta_skip_after_error()) return;   // an earlier bounded wait gave up: do not start new work
+  const bool skip = cta_begin();         // an earlier bounded wait gave up: do not start new work
   if (threadIdx.x == 0) {
     for (int b = 0; b < 2; ++b) {
       mbar_init(&bars.a_full[b], 4);
@@ -101,9 +101,7 @@ transition_tc_kernel(const __grid_constant__ CUtensorMap map_wa, const __grid_co
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
   }
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
+  if (!cta_ready(skip, warp == 16, bars.tmem_base, 512u)) return;
   const uint32_t tmem_base = bars.tmem_base;
 
   if (warp >= 16) {
@@ -383,14 +381,14 @@ static int32_t launch_transition(const void* x_in, void* x_out, const float* ln_
                    CU_TENSOR_MAP_SWIZZLE_128B))
     return PX_ERR_LAUNCH;
   const size_t smem = TransLayout::total + 1024;
-  if (cudaFuncSetAttribute(transition_tc_kernel<Tz>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-      cudaSuccess)
-    return PX_ERR_LAUNCH;
+  static SmemLimit limit;
+  if (!limit.set(transition_tc_kernel<Tz>, smem)) return PX_ERR_LAUNCH;
   const int64_t n_tiles = (rows + 127) / 128;
   const int grid = (int)(n_tiles < sm_count() ? n_tiles : sm_count());
-  transition_tc_kernel<Tz><<<grid, kTrThreads, smem, st>>>(ma, mb, mo, (const Tz*)x_in, (Tz*)x_out, ln_w, ln_b,
-                                                           (long long)rows, (int)n_tiles, add_residual, eps);
-  return cudaGetLastError() == cudaSuccess ? PX_OK : PX_ERR_LAUNCH;
+  return launch_pdl(transition_tc_kernel<Tz>, dim3(grid), kTrThreads, smem, st, ma, mb, mo, (const Tz*)x_in, (Tz*)x_out, ln_w, ln_b,
+                    (long long)rows, (int)n_tiles, (int)add_residual, eps)
+             ? PX_OK
+             : PX_ERR_LAUNCH;
 }
 
 }  // namespace px

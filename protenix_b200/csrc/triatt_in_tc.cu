@@ -33,6 +33,7 @@ constexpr uint32_t kAiColGram = 256;           // tensor memory: q|k (128) | v|b
 struct AiBars {
   TileBars tile;
   uint64_t acc_full[2][2], acc_free[2][2];   // [product][accumulator]
+  uint64_t w_full;
   uint32_t tmem_base;
 };
 struct AiLayout {
@@ -50,13 +51,32 @@ struct AiLayout {
 static_assert(AiLayout::total + 1024 <= 232448, "shared memory budget");
 static_assert(AiLayout::a % 1024 == 0, "tile ring must keep the swizzle alignment");
 
+// The resident weights of a CTA (variant: which pair of heads): q carries the softmax scale, the bias rows log2(e).
+template <bool kF16>
+struct AiWeights {
+  const float *ln_w, *ln_b;
+  const bf16 *q, *k, *v, *bias;
+  static constexpr int kBytes = AiLayout::a;
+  __device__ __forceinline__ void fold(unsigned char* sm, int hpair, int warp, int warps, int lane, int tid, int threads) const {
+    unsigned char *w0 = sm + AiLayout::w0, *w1 = sm + AiLayout::w1, *wx0 = sm + AiLayout::wx0, *wx1 = sm + AiLayout::wx1;
+    const float qscale = kLog2e * rsqrtf((float)kAiD);
+    fold_weight_rows<kF16, kF16>(w0, wx0, 0, kPanelBytes, q, 64 * hpair, 64, ln_w, ln_b, qscale, warp, warps, lane);
+    fold_weight_rows<kF16, kF16>(w0, wx0, 64, kPanelBytes, k, 64 * hpair, 64, ln_w, ln_b, 1.0f, warp, warps, lane);
+    fold_weight_rows<kF16, kF16>(w1, wx1, 0, kAiW1Panel, v, 64 * hpair, 64, ln_w, ln_b, 1.0f, warp, warps, lane);
+    fold_weight_rows<kF16, kF16>(w1, wx1, 64, kAiW1Panel, bias, 2 * hpair, 2, ln_w, ln_b, kLog2e, warp, warps, lane);
+    // rows 66..79 of the second operand and rows 66..127 of its correction panel are padding
+    for (int i = tid; i < 14 * 16; i += threads)
+      *reinterpret_cast<uint4*>(w1 + operand_piece_offset(66 + i / 16, i % 16, kAiW1Panel)) = make_uint4(0u, 0u, 0u, 0u);
+    for (int i = tid; i < 62 * 2; i += threads) *reinterpret_cast<uint4*>(wx1 + 66 * 32 + i * 16) = make_uint4(0u, 0u, 0u, 0u);
+  }
+};
+
 // kF16: the rows are the standardised fp16 copy of an fp32 pair tensor (fp16 weights); otherwise bf16 rows of z.
 template <bool kF16>
 __global__ void __launch_bounds__(kAiThreads, 1)
 triatt_in_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_constant__ CUtensorMap map_v,
-                    const float* __restrict__ mask, const float* __restrict__ ln_w,
-                    const float* __restrict__ ln_b, const bf16* __restrict__ w_q, const bf16* __restrict__ w_k,
-                    const bf16* __restrict__ w_v, const bf16* __restrict__ w_bias, bf16* __restrict__ q_out,
+                    const float* __restrict__ mask,
+                    const AiWeights<kF16> weights, const unsigned char* __restrict__ folded, bf16* __restrict__ q_out,
                     bf16* __restrict__ k_out, float* __restrict__ bias_out, float* __restrict__ mb_out, int n_u, int n,
                     int ldm, int swap, float eps, float inf, int tiles_t, int n_tiles) {
   constexpr int kAiAcc = kF16 ? 2 : 1;   // accumulators per product: the products of tile k+1 run beside the epilogue of k
@@ -77,9 +97,10 @@ triatt_in_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_cons
   ctx.n_t = n;
   ctx.swap = swap;
 
-  if (cta_skip_after_error()) return;   // an earlier bounded wait gave up: do not start new work
+  const bool skip = cta_begin();         // an earlier bounded wait gave up: do not start new work
   if (threadIdx.x == 0) {
     tile_bars_init(bars.tile, 2, kF16);
+    mbar_init(&bars.w_full, 1);
     for (int b = 0; b < 4; ++b) {
       mbar_init(&bars.acc_full[b >> 1][b & 1], 1);
       mbar_init(&bars.acc_free[b >> 1][b & 1], 8);
@@ -92,30 +113,14 @@ triatt_in_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_cons
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
   }
-  {
-    // weights -> resident operands (q carries the softmax scale, the bias rows log2(e))
-    const float qscale = kLog2e * rsqrtf((float)kAiD);
-    fold_weight_rows<kF16, kF16>(sm + AiLayout::w0, sm + AiLayout::wx0, 0, kPanelBytes, w_q, 64 * hpair, 64, ln_w, ln_b, qscale, warp,
-                     kAiWarps, lane);
-    fold_weight_rows<kF16, kF16>(sm + AiLayout::w0, sm + AiLayout::wx0, 64, kPanelBytes, w_k, 64 * hpair, 64, ln_w, ln_b, 1.0f, warp,
-                     kAiWarps, lane);
-    fold_weight_rows<kF16, kF16>(sm + AiLayout::w1, sm + AiLayout::wx1, 0, kAiW1Panel, w_v, 64 * hpair, 64, ln_w, ln_b, 1.0f, warp,
-                     kAiWarps, lane);
-    fold_weight_rows<kF16, kF16>(sm + AiLayout::w1, sm + AiLayout::wx1, 64, kAiW1Panel, w_bias, 2 * hpair, 2, ln_w, ln_b, kLog2e, warp,
-                     kAiWarps, lane);
-    // rows 66..79 of the second operand (and of its correction panel) are padding
-    for (int i = threadIdx.x; i < 14 * 18; i += kAiThreads) {
-      const int r = 66 + i / 18, piece = i % 18;
-      unsigned char* dst = piece < 16 ? sm + AiLayout::w1 + operand_piece_offset(r, piece, kAiW1Panel)
-                                      : sm + AiLayout::wx1 + r * 32 + (piece - 16) * 16;
-      *reinterpret_cast<uint4*>(dst) = make_uint4(0u, 0u, 0u, 0u);
-    }
-    tile_write_ones<kF16>(ctx.tiles, threadIdx.x, kAiThreads);
-    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-  }
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
+  tile_write_ones<kF16>(ctx.tiles, threadIdx.x, kAiThreads);
+  asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+  if (!cta_ready(skip, warp == 20, bars.tmem_base, 512u, [&] {
+        if (folded && threadIdx.x == 0)
+          folded_load(sm, folded + hpair * AiWeights<kF16>::kBytes, AiWeights<kF16>::kBytes, &bars.w_full);
+      }))
+    return;
+  fold_here(weights, folded, sm, hpair, &bars.w_full);
   const uint32_t tmem_base = bars.tmem_base;
 
   if (warp >= 20) {
@@ -126,10 +131,10 @@ triatt_in_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_cons
         if (!kF16) tile_gram_loop<kF16>(ctx, tmem_base + kAiColGram);   // standardised rows: nothing to measure
       } else if (warp == 21) {
         tile_product_loop(ctx, tmem_base, smem_u32(sm + AiLayout::w0), kPanelBytes, smem_u32(sm + AiLayout::wx0),
-                          umma_idesc_16(128, 128, kF16, kF16), bars.acc_full[0], bars.acc_free[0], kAiAcc, 256);
+                          umma_idesc_16(128, 128, kF16, kF16), &bars.w_full, bars.acc_full[0], bars.acc_free[0], kAiAcc, 256);
       } else {
         tile_product_loop(ctx, tmem_base + 128, smem_u32(sm + AiLayout::w1), kAiW1Panel, smem_u32(sm + AiLayout::wx1),
-                          umma_idesc_16(128, 80, kF16, kF16), bars.acc_full[1], bars.acc_free[1], kAiAcc, 256);
+                          umma_idesc_16(128, 80, kF16, kF16), &bars.w_full, bars.acc_full[1], bars.acc_free[1], kAiAcc, 256);
       }
     }
   } else if (warp >= 16) {
@@ -238,8 +243,7 @@ triatt_in_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_cons
 PX_DEFINE_FAMILY_HOOKS(triatt_in)
 
 template <bool kF16>
-static int32_t launch_triatt_in(const void* z, const float* mask, const float* ln_w, const float* ln_b,
-                                const px_bf16* w_q, const px_bf16* w_k, const px_bf16* w_v, const px_bf16* w_bias,
+static int32_t launch_triatt_in(const void* z, const float* mask, const AiWeights<kF16>& weights, const void* folded,
                                 px_f16* q, px_f16* k, px_f16* v, float* bias, float* mask_bias, int64_t n_u,
                                 int64_t n, int64_t ldm, int32_t ending, float eps, float inf, cudaStream_t st) {
   CUtensorMap mz, mv;
@@ -256,38 +260,75 @@ static int32_t launch_triatt_in(const void* z, const float* mask, const float* l
                    64, CU_TENSOR_MAP_SWIZZLE_NONE, 1))
     return PX_ERR_LAUNCH;
   const size_t smem = AiLayout::total + 1024;
-  if (cudaFuncSetAttribute(triatt_in_tc_kernel<kF16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-    return PX_ERR_LAUNCH;
+  static SmemLimit limit;
+  if (!limit.set(triatt_in_tc_kernel<kF16>, smem)) return PX_ERR_LAUNCH;
   const int64_t tiles_t = (n + 127) / 128, n_tiles = tiles_t * n_u;   // 128-wide tiles cover the pad columns up to ldm
   if (n_tiles > 0x7fffffff) return PX_ERR_UNSUPPORTED;
   const int pairs = (int)(n_tiles < sm_count() / 2 ? n_tiles : sm_count() / 2);
-  triatt_in_tc_kernel<kF16><<<2 * pairs, kAiThreads, smem, st>>>(mz, mv, mask, ln_w, ln_b, (const bf16*)w_q,
-                                                               (const bf16*)w_k, (const bf16*)w_v, (const bf16*)w_bias,
-                                                               (bf16*)q, (bf16*)k, bias, mask_bias, (int)n_u, (int)n,
-                                                               (int)ldm, ending, eps, inf, (int)tiles_t, (int)n_tiles);
-  return cudaGetLastError() == cudaSuccess ? PX_OK : PX_ERR_LAUNCH;
+  return launch_pdl(triatt_in_tc_kernel<kF16>, dim3(2 * pairs), kAiThreads, smem, st, mz, mv, mask, weights, (const unsigned char*)folded,
+                    (bf16*)q, (bf16*)k, bias, mask_bias, (int)n_u, (int)n, (int)ldm, (int)ending, eps, inf, (int)tiles_t,
+                    (int)n_tiles)
+             ? PX_OK
+             : PX_ERR_LAUNCH;
+}
+
+static bool triatt_in_args_ok(const void* z, const void* q, const void* k, const void* v, const float* bias, const float* mask_bias,
+                              int64_t n_u, int64_t n_t, int64_t ldm) {
+  return z && q && k && v && bias && mask_bias && n_u > 0 && n_t > 0 && n_u <= 32768 && n_t <= 32768 && ldm == px_ld_mask(n_t) &&
+         !(((uintptr_t)z | (uintptr_t)q | (uintptr_t)k | (uintptr_t)v) & 15);
+}
+template <bool kF16>
+static AiWeights<kF16> ai_weights(const float* ln_w, const float* ln_b, const px_w16* q, const px_w16* k, const px_w16* v,
+                                  const px_w16* bias) {
+  return {ln_w, ln_b, (const bf16*)q, (const bf16*)k, (const bf16*)v, (const bf16*)bias};
+}
+static bool ai_weights_ok(const float* ln_w, const float* ln_b, const px_w16* q, const px_w16* k, const px_w16* v, const px_w16* bias) {
+  return ln_w && ln_b && q && k && v && bias &&
+         !(((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)bias | (uintptr_t)ln_w | (uintptr_t)ln_b) & 15);
 }
 
 }  // namespace px
 
 using namespace px;
 
+extern "C" int64_t px_triatt_in_folded_bytes(void) { return 2 * AiWeights<true>::kBytes; }
+
+extern "C" int32_t px_triatt_in_fold(const float* ln_w, const float* ln_b, const px_w16* w_q, const px_w16* w_k, const px_w16* w_v,
+                                     const px_w16* w_bias, int32_t rows_dtype, void* folded, void* stream) {
+  if (!ai_weights_ok(ln_w, ln_b, w_q, w_k, w_v, w_bias) || !folded || ((uintptr_t)folded & 15)) return PX_ERR_BAD_ARG;
+  if (rows_dtype != PX_F16 && rows_dtype != PX_BF16) return PX_ERR_UNSUPPORTED;
+  cudaStream_t st = (cudaStream_t)stream;
+  return (rows_dtype == PX_F16 ? launch_fold(ai_weights<true>(ln_w, ln_b, w_q, w_k, w_v, w_bias), 2, folded, st)
+                               : launch_fold(ai_weights<false>(ln_w, ln_b, w_q, w_k, w_v, w_bias), 2, folded, st))
+             ? PX_OK
+             : PX_ERR_LAUNCH;
+}
+
+extern "C" int32_t px_triatt_in_proj_folded(const void* z, int32_t z_dtype, const float* mask, const void* folded, px_f16* q,
+                                            px_f16* k, px_f16* v, float* bias, float* mask_bias, int64_t n_u, int64_t n_t,
+                                            int64_t ldm, int32_t ending, float eps, float inf, void* stream) {
+  if (!triatt_in_args_ok(z, q, k, v, bias, mask_bias, n_u, n_t, ldm) || !folded || ((uintptr_t)folded & 15)) return PX_ERR_BAD_ARG;
+  cudaStream_t st = (cudaStream_t)stream;
+  if (z_dtype == PX_F16)
+    return launch_triatt_in<true>(z, mask, AiWeights<true>{}, folded, q, k, v, bias, mask_bias, n_u, n_t, ldm, ending, eps, inf, st);
+  if (z_dtype == PX_BF16)
+    return launch_triatt_in<false>(z, mask, AiWeights<false>{}, folded, q, k, v, bias, mask_bias, n_u, n_t, ldm, ending, eps, inf, st);
+  return PX_ERR_UNSUPPORTED;
+}
+
 extern "C" int32_t px_triatt_in_proj(const void* z, int32_t z_dtype, const float* mask, const float* ln_w,
                                      const float* ln_b, const px_bf16* w_q, const px_bf16* w_k, const px_bf16* w_v,
                                      const px_bf16* w_bias, px_f16* q, px_f16* k, px_f16* v, float* bias,
                                      float* mask_bias, int64_t n_u, int64_t n_t, int64_t ldm, int32_t ending,
                                      float eps, float inf, void* stream) {
-  if (!z || !ln_w || !ln_b || !w_q || !w_k || !w_v || !w_bias || !q || !k || !v || !bias || !mask_bias)
+  if (!triatt_in_args_ok(z, q, k, v, bias, mask_bias, n_u, n_t, ldm) || !ai_weights_ok(ln_w, ln_b, w_q, w_k, w_v, w_bias))
     return PX_ERR_BAD_ARG;
-  if (n_u <= 0 || n_t <= 0 || n_u > 32768 || n_t > 32768 || ldm != px_ld_mask(n_t)) return PX_ERR_BAD_ARG;
-  if (((uintptr_t)z | (uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)w_q | (uintptr_t)w_k | (uintptr_t)w_v |
-       (uintptr_t)w_bias | (uintptr_t)ln_w | (uintptr_t)ln_b) & 15)
-    return PX_ERR_BAD_ARG;
+  cudaStream_t st = (cudaStream_t)stream;
   if (z_dtype == PX_F16)   // standardised rows of an fp32 pair tensor (px_standardise_rows)
-    return launch_triatt_in<true>(z, mask, ln_w, ln_b, w_q, w_k, w_v, w_bias, q, k, v, bias, mask_bias, n_u, n_t, ldm,
-                                   ending, eps, inf, (cudaStream_t)stream);
+    return launch_triatt_in<true>(z, mask, ai_weights<true>(ln_w, ln_b, w_q, w_k, w_v, w_bias), nullptr, q, k, v, bias, mask_bias, n_u,
+                                  n_t, ldm, ending, eps, inf, st);
   if (z_dtype == PX_BF16)
-    return launch_triatt_in<false>(z, mask, ln_w, ln_b, w_q, w_k, w_v, w_bias, q, k, v, bias, mask_bias, n_u, n_t, ldm,
-                                  ending, eps, inf, (cudaStream_t)stream);
+    return launch_triatt_in<false>(z, mask, ai_weights<false>(ln_w, ln_b, w_q, w_k, w_v, w_bias), nullptr, q, k, v, bias, mask_bias, n_u,
+                                   n_t, ldm, ending, eps, inf, st);
   return PX_ERR_UNSUPPORTED;
 }

@@ -36,7 +36,7 @@ constexpr uint32_t kAoColG = 0, kAoColA2 = 128, kAoColOut = 192, kAoColGram = 32
 
 struct AoBars {
   TileBars tile;
-  uint64_t g_full, g_free, a2_ready, a2_free, out_full, out_free;
+  uint64_t g_full, g_free, a2_ready, a2_free, out_full, out_free, w_full;
   uint32_t tmem_base;
 };
 struct AoLayout {
@@ -53,12 +53,24 @@ struct AoLayout {
 static_assert(AoLayout::total + 1024 <= 232448, "shared memory budget");
 static_assert(AoLayout::a % 1024 == 0 && AoLayout::o % 1024 == 0, "tiles must keep the swizzle alignment");
 
+// The resident weights: gate (the 1/2 of sigmoid(x) = 1/2 + 1/2 tanh(x/2) folded in), output, correction panel of the gate.
+template <bool kF16>
+struct AoWeights {
+  const float *ln_w, *ln_b;
+  const bf16 *w_g, *w_o;
+  static constexpr int kBytes = AoLayout::a;
+  __device__ __forceinline__ void fold(unsigned char* sm, int, int warp, int warps, int lane, int, int) const {
+    fold_weight_rows<kF16, kF16>(sm + AoLayout::wg, sm + AoLayout::wx, 0, kPanelBytes, w_g, 0, 128, ln_w, ln_b, 0.5f, warp, warps, lane);
+    // the output weights multiply the fp16 rows o * sigmoid(g) and arrive as fp16
+    fold_weight_rows<true, true>(sm + AoLayout::wo, nullptr, 0, kPanelBytes, w_o, 0, 128, nullptr, nullptr, 1.0f, warp, warps, lane);
+  }
+};
+
 template <int kMode>
 __global__ void __launch_bounds__(kAoThreads, 1)
 triatt_out_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_constant__ CUtensorMap map_o,
                      const __grid_constant__ CUtensorMap map_out, const void* __restrict__ z_in, void* __restrict__ z_out,
-                     const float* __restrict__ ln_w, const float* __restrict__ ln_b, const bf16* __restrict__ w_g,
-                     const bf16* __restrict__ w_o, int n_u, int n, int swap, int add_residual, float eps, int tiles_t,
+                     const AoWeights<kMode != 0> weights, const unsigned char* __restrict__ folded, int n_u, int n, int swap, int add_residual, float eps, int tiles_t,
                      int n_tiles) {
   constexpr bool kTma = kMode != 1;                      // 16-bit output: packed over the o tile, leaves through TMA
   constexpr bool kF16 = kMode != 0;                      // the z tile is a standardised fp16 copy; o, W_o always fp16
@@ -78,10 +90,11 @@ triatt_out_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_con
   ctx.n_t = n;
   ctx.swap = swap;
 
-  if (cta_skip_after_error()) return;   // an earlier bounded wait gave up: do not start new work
+  const bool skip = cta_begin();         // an earlier bounded wait gave up: do not start new work
   if (threadIdx.x == 0) {
     // a stage is read by the statistics product, the gate product and the output warps
     tile_bars_init(bars.tile, 2, kF16);
+    mbar_init(&bars.w_full, 1);
     mbar_init(&bars.g_full, 1);
     mbar_init(&bars.g_free, 8);
     mbar_init(&bars.a2_ready, 8);
@@ -96,19 +109,13 @@ triatt_out_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_con
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
   }
-  {
-    // the gate rows carry the 1/2 of sigmoid(x) = 1/2 + 1/2 tanh(x/2)
-    fold_weight_rows<kF16, kF16>(sm + AoLayout::wg, sm + AoLayout::wx, 0, kPanelBytes, w_g, 0, 128, ln_w, ln_b, 0.5f, warp,
-                                 kAoWarps, lane);
-    // the output weights multiply the fp16 rows o * sigmoid(g) and arrive as fp16
-    fold_weight_rows<true, true>(sm + AoLayout::wo, nullptr, 0, kPanelBytes, w_o, 0, 128, nullptr, nullptr, 1.0f, warp,
-                                 kAoWarps, lane);
-    tile_write_ones<kF16>(ctx.tiles, threadIdx.x, kAoThreads);
-    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-  }
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
+  tile_write_ones<kF16>(ctx.tiles, threadIdx.x, kAoThreads);
+  asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+  if (!cta_ready(skip, warp == 20, bars.tmem_base, 512u, [&] {
+        if (folded && threadIdx.x == 0) folded_load(sm, folded, AoWeights<kF16>::kBytes, &bars.w_full);
+      }))
+    return;
+  fold_here(weights, folded, sm, 0, &bars.w_full);
   const uint32_t tmem_base = bars.tmem_base;
 
   if (warp >= 20) {
@@ -131,13 +138,14 @@ triatt_out_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_con
         if (!kF16) tile_gram_loop<kF16>(ctx, tmem_base + kAoColGram);   // standardised rows: nothing to measure
       } else if (warp == 21) {
         tile_product_loop(ctx, tmem_base + kAoColG, smem_u32(sm + AoLayout::wg), kPanelBytes, smem_u32(sm + AoLayout::wx),
-                          umma_idesc_16(128, 128, kF16, kF16), &bars.g_full, &bars.g_free);
+                          umma_idesc_16(128, 128, kF16, kF16), &bars.w_full, &bars.g_full, &bars.g_free);
       } else {
         // ---------------------------------------------------------------- output product, A operand in tensor memory
         constexpr uint32_t idesc = umma_idesc_f16(128, 128);
         const uint32_t wo_addr = smem_u32(sm + AoLayout::wo);
         int k = 0;
-        for (int tile = ctx.first_tile; tile < n_tiles; tile += ctx.tile_step, ++k) {
+        const bool have_w = mbar_wait(&bars.w_full, 0, 4u);      // the resident weights
+        for (int tile = ctx.first_tile; tile < n_tiles && have_w; tile += ctx.tile_step, ++k) {
           if (!mbar_wait(&bars.a2_ready, k & 1, 4u) || !mbar_wait(&bars.out_free, (k & 1) ^ 1, 8u)) break;
           tc_fence_after();
 #pragma unroll
@@ -310,8 +318,8 @@ triatt_out_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_con
 PX_DEFINE_FAMILY_HOOKS(triatt_out)
 
 template <int kMode>
-static int32_t launch_triatt_out(const px_f16* o, const void* z_in, const px_f16* zn, void* z_out, const float* ln_w, const float* ln_b,
-                                 const px_bf16* w_g, const px_bf16* w_o, int64_t n_u, int64_t n, int32_t ending,
+static int32_t launch_triatt_out(const px_f16* o, const void* z_in, const px_f16* zn, void* z_out,
+                                 const AoWeights<kMode != 0>& weights, const void* folded, int64_t n_u, int64_t n, int32_t ending,
                                  int32_t add_residual, float eps, cudaStream_t st) {
   CUtensorMap mz, mo, mout;
   // operand rows: bf16 z itself, or the standardised fp16 copy of an fp32 z; pair element (u, t) is row u*n + t, or
@@ -336,39 +344,65 @@ static int32_t launch_triatt_out(const px_f16* o, const void* z_in, const px_f16
                    128, CU_TENSOR_MAP_SWIZZLE_128B, 1))
     return PX_ERR_LAUNCH;
   const size_t smem = AoLayout::total + 1024;
-  if (cudaFuncSetAttribute(triatt_out_tc_kernel<kMode>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-    return PX_ERR_LAUNCH;
+  static SmemLimit limit;
+  if (!limit.set(triatt_out_tc_kernel<kMode>, smem)) return PX_ERR_LAUNCH;
   const int64_t tiles_t = (n + 127) / 128, n_tiles = tiles_t * n_u;
   if (n_tiles > 0x7fffffff) return PX_ERR_UNSUPPORTED;
   const int grid = (int)(n_tiles < sm_count() ? n_tiles : sm_count());
-  triatt_out_tc_kernel<kMode><<<grid, kAoThreads, smem, st>>>(mz, mo, mout, z_in, z_out, ln_w, ln_b,
-                                                           (const bf16*)w_g, (const bf16*)w_o, (int)n_u, (int)n, ending,
-                                                           add_residual, eps, (int)tiles_t, (int)n_tiles);
-  return cudaGetLastError() == cudaSuccess ? PX_OK : PX_ERR_LAUNCH;
+  return launch_pdl(triatt_out_tc_kernel<kMode>, dim3(grid), kAoThreads, smem, st, mz, mo, mout, z_in, z_out, weights,
+                    (const unsigned char*)folded, (int)n_u, (int)n, (int)ending, (int)add_residual, eps, (int)tiles_t, (int)n_tiles)
+             ? PX_OK
+             : PX_ERR_LAUNCH;
+}
+
+// The three forms by the type of z; w: the raw weights (ignored when they come folded).
+static int32_t triatt_out_any(const px_f16* o, const void* z_in, const px_f16* zn, void* z_out, int32_t z_dtype, const AoWeights<true>& w,
+                              const void* folded, int64_t n_u, int64_t n_t, int32_t ending, int32_t add_residual, float eps,
+                              cudaStream_t st) {
+  if (!o || !z_in || !z_out || n_u <= 0 || n_t <= 0 || n_u > 32768 || n_t > 32768) return PX_ERR_BAD_ARG;
+  if (z_dtype == PX_F32 && (!zn || ((uintptr_t)zn & 15))) return PX_ERR_BAD_ARG;
+  if (((uintptr_t)o | (uintptr_t)z_in | (uintptr_t)z_out) & 15) return PX_ERR_BAD_ARG;
+  if (z_dtype == PX_F16)   // z_in: standardised fp16 rows; z_out: the update in fp16 (no residual to add)
+    return add_residual ? PX_ERR_BAD_ARG
+                        : launch_triatt_out<2>(o, z_in, nullptr, z_out, w, folded, n_u, n_t, ending, 0, eps, st);
+  if (z_dtype == PX_F32) return launch_triatt_out<1>(o, z_in, zn, z_out, w, folded, n_u, n_t, ending, add_residual, eps, st);
+  if (z_dtype == PX_BF16)
+    return launch_triatt_out<0>(o, z_in, nullptr, z_out, AoWeights<false>{w.ln_w, w.ln_b, w.w_g, w.w_o}, folded, n_u, n_t, ending,
+                                add_residual, eps, st);
+  return PX_ERR_UNSUPPORTED;
+}
+static bool ao_weights_ok(const float* ln_w, const float* ln_b, const px_w16* w_g, const px_f16* w_o) {
+  return ln_w && ln_b && w_g && w_o && !(((uintptr_t)w_g | (uintptr_t)w_o | (uintptr_t)ln_w | (uintptr_t)ln_b) & 15);
 }
 
 }  // namespace px
 
 using namespace px;
 
+extern "C" int64_t px_triatt_out_folded_bytes(void) { return AoWeights<true>::kBytes; }
+
+extern "C" int32_t px_triatt_out_fold(const float* ln_w, const float* ln_b, const px_w16* w_g, const px_f16* w_o, int32_t rows_dtype,
+                                      void* folded, void* stream) {
+  if (!ao_weights_ok(ln_w, ln_b, w_g, w_o) || !folded || ((uintptr_t)folded & 15)) return PX_ERR_BAD_ARG;
+  if (rows_dtype != PX_F16 && rows_dtype != PX_BF16) return PX_ERR_UNSUPPORTED;
+  cudaStream_t st = (cudaStream_t)stream;
+  return (rows_dtype == PX_F16 ? launch_fold(AoWeights<true>{ln_w, ln_b, (const bf16*)w_g, (const bf16*)w_o}, 1, folded, st)
+                               : launch_fold(AoWeights<false>{ln_w, ln_b, (const bf16*)w_g, (const bf16*)w_o}, 1, folded, st))
+             ? PX_OK
+             : PX_ERR_LAUNCH;
+}
+
+extern "C" int32_t px_triatt_out_folded(const px_f16* o, const void* z_in, const px_f16* zn, void* z_out, int32_t z_dtype,
+                                        const void* folded, int64_t n_u, int64_t n_t, int32_t ending, int32_t add_residual, float eps,
+                                        void* stream) {
+  if (!folded || ((uintptr_t)folded & 15)) return PX_ERR_BAD_ARG;
+  return triatt_out_any(o, z_in, zn, z_out, z_dtype, AoWeights<true>{}, folded, n_u, n_t, ending, add_residual, eps, (cudaStream_t)stream);
+}
+
 extern "C" int32_t px_triatt_out(const px_f16* o, const void* z_in, const px_f16* zn, void* z_out, int32_t z_dtype,
                                  const float* ln_w, const float* ln_b, const px_w16* w_g, const px_f16* w_o, int64_t n_u,
                                  int64_t n_t, int32_t ending, int32_t add_residual, float eps, void* stream) {
-  if (!o || !z_in || !z_out || !ln_w || !ln_b || !w_g || !w_o || n_u <= 0 || n_t <= 0 || n_u > 32768 || n_t > 32768)
-    return PX_ERR_BAD_ARG;
-  if (z_dtype == PX_F32 && (!zn || ((uintptr_t)zn & 15))) return PX_ERR_BAD_ARG;
-  if (((uintptr_t)o | (uintptr_t)z_in | (uintptr_t)z_out | (uintptr_t)w_g | (uintptr_t)w_o | (uintptr_t)ln_w |
-       (uintptr_t)ln_b) & 15)
-    return PX_ERR_BAD_ARG;
-  if (z_dtype == PX_F16)   // z_in: standardised fp16 rows; z_out: the update in fp16 (no residual to add)
-    return add_residual ? PX_ERR_BAD_ARG
-                        : launch_triatt_out<2>(o, z_in, nullptr, z_out, ln_w, ln_b, w_g, w_o, n_u, n_t, ending, 0, eps,
-                                               (cudaStream_t)stream);
-  if (z_dtype == PX_F32)
-    return launch_triatt_out<1>(o, z_in, zn, z_out, ln_w, ln_b, w_g, w_o, n_u, n_t, ending, add_residual, eps,
-                                    (cudaStream_t)stream);
-  if (z_dtype == PX_BF16)
-    return launch_triatt_out<0>(o, z_in, nullptr, z_out, ln_w, ln_b, w_g, w_o, n_u, n_t, ending, add_residual, eps,
-                                   (cudaStream_t)stream);
-  return PX_ERR_UNSUPPORTED;
+  if (!ao_weights_ok(ln_w, ln_b, w_g, w_o)) return PX_ERR_BAD_ARG;
+  return triatt_out_any(o, z_in, zn, z_out, z_dtype, AoWeights<true>{ln_w, ln_b, (const bf16*)w_g, (const bf16*)w_o}, nullptr, n_u, n_t,
+                        ending, add_residual, eps, (cudaStream_t)stream);
 }

@@ -38,6 +38,7 @@ constexpr uint32_t kTiColGram = 256;           // tensor memory: out a | out b |
 struct TiBars {
   TileBars tile;
   uint64_t acc_full[2][2], acc_free[2][2];   // [output][accumulator]
+  uint64_t w_full;
   uint32_t tmem_base;
 };
 struct TiLayout {
@@ -52,14 +53,29 @@ struct TiLayout {
 };
 static_assert(TiLayout::total + 1024 <= 232448, "shared memory budget");
 
+// The resident weights of a CTA (variant: which 64 channels), [projection 64 | gate 64] per output with the correction panels
+// behind; the gate rows carry the 1/2 of sigmoid(x) = 1/2 + 1/2 tanh(x/2).
+template <bool kF16>
+struct TiWeights {
+  const float *ln_w, *ln_b;
+  const bf16 *ap, *ag, *bp, *bg;
+  static constexpr int kBytes = TiLayout::a;
+  __device__ __forceinline__ void fold(unsigned char* sm, int variant, int warp, int warps, int lane, int, int) const {
+    const int chan0 = 64 * variant;
+    unsigned char *w0 = sm + TiLayout::w, *x0 = sm + TiLayout::wx;
+    fold_weight_rows<kF16, kF16>(w0, x0, 0, kPanelBytes, ap, chan0, 64, ln_w, ln_b, 1.0f, warp, warps, lane);
+    fold_weight_rows<kF16, kF16>(w0, x0, 64, kPanelBytes, ag, chan0, 64, ln_w, ln_b, 0.5f, warp, warps, lane);
+    fold_weight_rows<kF16, kF16>(w0 + kOperandBytes, x0 + kTiWExtra, 0, kPanelBytes, bp, chan0, 64, ln_w, ln_b, 1.0f, warp, warps, lane);
+    fold_weight_rows<kF16, kF16>(w0 + kOperandBytes, x0 + kTiWExtra, 64, kPanelBytes, bg, chan0, 64, ln_w, ln_b, 0.5f, warp, warps, lane);
+  }
+};
+
 // kF16: the rows are the standardised fp16 copy of an fp32 pair tensor (fp16 weights); otherwise bf16 rows of z.
 template <bool kF16>
 __global__ void __launch_bounds__(kTiThreads, 1)
 trimul_in_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_constant__ CUtensorMap map_a,
                     const __grid_constant__ CUtensorMap map_b, const float* __restrict__ mask,
-                    const float* __restrict__ ln_w, const float* __restrict__ ln_b, const bf16* __restrict__ w_ap,
-                    const bf16* __restrict__ w_ag, const bf16* __restrict__ w_bp, const bf16* __restrict__ w_bg,
-                    int n_u, int n_t, int swap, float eps, int tiles_t, int n_tiles) {
+                    const TiWeights<kF16> weights, const unsigned char* __restrict__ folded, int n_u, int n_t, int swap, float eps, int tiles_t, int n_tiles) {
   constexpr int kTiAcc = kF16 ? 2 : 1;   // accumulators per output: the products of tile k+1 run beside the epilogue of k
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* sm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -78,9 +94,10 @@ trimul_in_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_cons
   ctx.n_t = n_t;
   ctx.swap = swap;
 
-  if (cta_skip_after_error()) return;   // an earlier bounded wait gave up: do not start new work
+  const bool skip = cta_begin();         // an earlier bounded wait gave up: do not start new work
   if (threadIdx.x == 0) {
     tile_bars_init(bars.tile, 2, kF16);
+    mbar_init(&bars.w_full, 1);
     for (int b = 0; b < 4; ++b) {
       mbar_init(&bars.acc_full[b >> 1][b & 1], 1);
       mbar_init(&bars.acc_free[b >> 1][b & 1], 8);
@@ -93,20 +110,14 @@ trimul_in_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_cons
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
   }
-  {
-    // weights -> resident operands; the gate rows carry the 1/2 of sigmoid(x) = 1/2 + 1/2 tanh(x/2)
-    unsigned char* w0 = sm + TiLayout::w;
-    unsigned char* x0 = sm + TiLayout::wx;
-    fold_weight_rows<kF16, kF16>(w0, x0, 0, kPanelBytes, w_ap, chan0, 64, ln_w, ln_b, 1.0f, warp, kTiWarps, lane);
-    fold_weight_rows<kF16, kF16>(w0, x0, 64, kPanelBytes, w_ag, chan0, 64, ln_w, ln_b, 0.5f, warp, kTiWarps, lane);
-    fold_weight_rows<kF16, kF16>(w0 + kOperandBytes, x0 + kTiWExtra, 0, kPanelBytes, w_bp, chan0, 64, ln_w, ln_b, 1.0f, warp, kTiWarps, lane);
-    fold_weight_rows<kF16, kF16>(w0 + kOperandBytes, x0 + kTiWExtra, 64, kPanelBytes, w_bg, chan0, 64, ln_w, ln_b, 0.5f, warp, kTiWarps, lane);
-    tile_write_ones<kF16>(ctx.tiles, threadIdx.x, kTiThreads);
-    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-  }
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
+  tile_write_ones<kF16>(ctx.tiles, threadIdx.x, kTiThreads);
+  asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+  if (!cta_ready(skip, warp == 20, bars.tmem_base, 512u, [&] {
+        if (folded && threadIdx.x == 0)
+          folded_load(sm, folded + (blockIdx.x & 1) * TiWeights<kF16>::kBytes, TiWeights<kF16>::kBytes, &bars.w_full);
+      }))
+    return;
+  fold_here(weights, folded, sm, blockIdx.x & 1, &bars.w_full);
   const uint32_t tmem_base = bars.tmem_base;
 
   if (warp >= 20) {
@@ -118,7 +129,7 @@ trimul_in_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_cons
       } else {
         const int ph = warp - 21;                          // MMA issuer of output ph
         tile_product_loop(ctx, tmem_base + 128 * ph, smem_u32(sm + TiLayout::w) + ph * kOperandBytes, kPanelBytes,
-                          smem_u32(sm + TiLayout::wx) + ph * kTiWExtra, umma_idesc_16(128, 128, kF16, kF16), bars.acc_full[ph],
+                          smem_u32(sm + TiLayout::wx) + ph * kTiWExtra, umma_idesc_16(128, 128, kF16, kF16), &bars.w_full, bars.acc_full[ph],
                           bars.acc_free[ph], kTiAcc, 256);
       }
     }
@@ -192,10 +203,8 @@ trimul_in_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_cons
 PX_DEFINE_FAMILY_HOOKS(trimul_in)
 
 template <bool kF16>
-static int32_t launch_trimul_in(const void* z, const float* mask, const float* ln_w, const float* ln_b,
-                                const px_w16* w_ap, const px_w16* w_ag, const px_w16* w_bp, const px_w16* w_bg,
-                                px_f16* a, px_f16* b, int64_t n_u, int64_t n_t, int64_t ld, int32_t incoming, float eps,
-                                cudaStream_t st) {
+static int32_t launch_trimul_in(const void* z, const float* mask, const TiWeights<kF16>& weights, const void* folded, px_f16* a,
+                                px_f16* b, int64_t n_u, int64_t n_t, int64_t ld, int32_t incoming, float eps, cudaStream_t st) {
   CUtensorMap mz, ma, mb;
   const CUtensorMapDataType zt = kF16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
   // pair element (u, t) is row u*n_t + t of z, or row t*n_u + u when the two indices are exchanged
@@ -211,36 +220,69 @@ static int32_t launch_trimul_in(const void* z, const float* mask, const float* l
                    (uint64_t)n_u * ld * 2, 128, 1, CU_TENSOR_MAP_SWIZZLE_NONE, 64))
     return PX_ERR_LAUNCH;
   const size_t smem = TiLayout::total + 1024;
-  if (cudaFuncSetAttribute(trimul_in_tc_kernel<kF16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-    return PX_ERR_LAUNCH;
+  static SmemLimit limit;
+  if (!limit.set(trimul_in_tc_kernel<kF16>, smem)) return PX_ERR_LAUNCH;
   const int64_t tiles_t = (ld + 127) / 128, n_tiles = tiles_t * n_u;
   if (n_tiles > 0x7fffffff) return PX_ERR_UNSUPPORTED;
   const int pairs = (int)(n_tiles < sm_count() / 2 ? n_tiles : sm_count() / 2);
-  trimul_in_tc_kernel<kF16><<<2 * pairs, kTiThreads, smem, st>>>(mz, ma, mb, mask, ln_w, ln_b, (const bf16*)w_ap,
-                                                                 (const bf16*)w_ag, (const bf16*)w_bp, (const bf16*)w_bg,
-                                                                 (int)n_u, (int)n_t, incoming, eps, (int)tiles_t,
-                                                                 (int)n_tiles);
-  return cudaGetLastError() == cudaSuccess ? PX_OK : PX_ERR_LAUNCH;
+  return launch_pdl(trimul_in_tc_kernel<kF16>, dim3(2 * pairs), kTiThreads, smem, st, mz, ma, mb, mask, weights,
+                    (const unsigned char*)folded, (int)n_u, (int)n_t, (int)incoming, eps, (int)tiles_t, (int)n_tiles)
+             ? PX_OK
+             : PX_ERR_LAUNCH;
+}
+
+static bool trimul_in_shapes_ok(const void* z, const px_f16* a, const px_f16* b, int64_t n_u, int64_t n_t, int64_t ld) {
+  return z && a && b && n_u > 0 && n_t > 0 && n_u <= 32768 && n_t <= 32768 && ld == px_ld(n_t) &&
+         !(((uintptr_t)z | (uintptr_t)a | (uintptr_t)b) & 15);
+}
+template <bool kF16>
+static TiWeights<kF16> ti_weights(const float* ln_w, const float* ln_b, const px_w16* ap, const px_w16* ag, const px_w16* bp,
+                                  const px_w16* bg) {
+  return {ln_w, ln_b, (const bf16*)ap, (const bf16*)ag, (const bf16*)bp, (const bf16*)bg};
+}
+static bool ti_weights_ok(const float* ln_w, const float* ln_b, const px_w16* ap, const px_w16* ag, const px_w16* bp,
+                          const px_w16* bg) {
+  return ln_w && ln_b && ap && ag && bp && bg &&
+         !(((uintptr_t)ap | (uintptr_t)ag | (uintptr_t)bp | (uintptr_t)bg | (uintptr_t)ln_w | (uintptr_t)ln_b) & 15);
 }
 
 }  // namespace px
 
 using namespace px;
 
+extern "C" int64_t px_trimul_in_folded_bytes(void) { return 2 * TiWeights<true>::kBytes; }
+
+extern "C" int32_t px_trimul_in_fold(const float* ln_w, const float* ln_b, const px_w16* w_ap, const px_w16* w_ag,
+                                     const px_w16* w_bp, const px_w16* w_bg, int32_t rows_dtype, void* folded, void* stream) {
+  if (!ti_weights_ok(ln_w, ln_b, w_ap, w_ag, w_bp, w_bg) || !folded || ((uintptr_t)folded & 15)) return PX_ERR_BAD_ARG;
+  if (rows_dtype != PX_F16 && rows_dtype != PX_BF16) return PX_ERR_UNSUPPORTED;
+  return (rows_dtype == PX_F16 ? launch_fold(ti_weights<true>(ln_w, ln_b, w_ap, w_ag, w_bp, w_bg), 2, folded, (cudaStream_t)stream)
+                               : launch_fold(ti_weights<false>(ln_w, ln_b, w_ap, w_ag, w_bp, w_bg), 2, folded, (cudaStream_t)stream))
+             ? PX_OK
+             : PX_ERR_LAUNCH;
+}
+
+extern "C" int32_t px_trimul_in_proj_folded(const void* z, int32_t z_dtype, const float* mask, const void* folded, px_f16* a,
+                                            px_f16* b, int64_t n_u, int64_t n_t, int64_t ld, int32_t incoming, float eps,
+                                            void* stream) {
+  if (!trimul_in_shapes_ok(z, a, b, n_u, n_t, ld) || !folded || ((uintptr_t)folded & 15)) return PX_ERR_BAD_ARG;
+  if (z_dtype == PX_F16)
+    return launch_trimul_in<true>(z, mask, TiWeights<true>{}, folded, a, b, n_u, n_t, ld, incoming, eps, (cudaStream_t)stream);
+  if (z_dtype == PX_BF16)
+    return launch_trimul_in<false>(z, mask, TiWeights<false>{}, folded, a, b, n_u, n_t, ld, incoming, eps, (cudaStream_t)stream);
+  return PX_ERR_UNSUPPORTED;
+}
+
 extern "C" int32_t px_trimul_in_proj(const void* z, int32_t z_dtype, const float* mask, const float* ln_w,
                                      const float* ln_b, const px_w16* w_ap, const px_w16* w_ag,
                                      const px_w16* w_bp, const px_w16* w_bg, px_f16* a, px_f16* b, int64_t n_u,
                                      int64_t n_t, int64_t ld, int32_t incoming, float eps, void* stream) {
-  if (!z || !ln_w || !ln_b || !w_ap || !w_ag || !w_bp || !w_bg || !a || !b) return PX_ERR_BAD_ARG;
-  if (n_u <= 0 || n_t <= 0 || n_u > 32768 || n_t > 32768 || ld != px_ld(n_t)) return PX_ERR_BAD_ARG;
-  if (((uintptr_t)z | (uintptr_t)a | (uintptr_t)b | (uintptr_t)w_ap | (uintptr_t)w_ag | (uintptr_t)w_bp |
-       (uintptr_t)w_bg | (uintptr_t)ln_w | (uintptr_t)ln_b) & 15)
-    return PX_ERR_BAD_ARG;
+  if (!trimul_in_shapes_ok(z, a, b, n_u, n_t, ld) || !ti_weights_ok(ln_w, ln_b, w_ap, w_ag, w_bp, w_bg)) return PX_ERR_BAD_ARG;
   if (z_dtype == PX_F16)   // standardised rows of an fp32 pair tensor (px_standardise_rows)
-    return launch_trimul_in<true>(z, mask, ln_w, ln_b, w_ap, w_ag, w_bp, w_bg, a, b, n_u, n_t, ld, incoming, eps,
-                                  (cudaStream_t)stream);
+    return launch_trimul_in<true>(z, mask, ti_weights<true>(ln_w, ln_b, w_ap, w_ag, w_bp, w_bg), nullptr, a, b, n_u, n_t, ld,
+                                  incoming, eps, (cudaStream_t)stream);
   if (z_dtype == PX_BF16)
-    return launch_trimul_in<false>(z, mask, ln_w, ln_b, w_ap, w_ag, w_bp, w_bg, a, b, n_u, n_t, ld, incoming, eps,
-                                   (cudaStream_t)stream);
+    return launch_trimul_in<false>(z, mask, ti_weights<false>(ln_w, ln_b, w_ap, w_ag, w_bp, w_bg), nullptr, a, b, n_u, n_t, ld,
+                                   incoming, eps, (cudaStream_t)stream);
   return PX_ERR_UNSUPPORTED;
 }

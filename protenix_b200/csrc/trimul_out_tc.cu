@@ -38,7 +38,7 @@ constexpr uint32_t kToColG = 0, kToColP = 144, kToColGram = 288;
 
 struct ToBars {
   uint64_t raw_full[kToStages], a_ready[kToStages], a_empty[kToStages];
-  uint64_t gram_full, gram_free, main_full, acc_full, acc_free;
+  uint64_t gram_full, gram_free, main_full, acc_full, acc_free, w_full;
   uint32_t tmem_base;
 };
 struct ToLayout {
@@ -56,13 +56,36 @@ struct ToLayout {
 static_assert(ToLayout::zt % 1024 == 0 && ToLayout::xt % 1024 == 0, "tiles must keep the swizzle alignment");
 static_assert(ToLayout::total + 1024 <= 232448, "shared memory budget");
 
+// The resident weights: gate | projection, each with 16 rows of ones behind it, and their correction panels.  The gate rows carry
+// the 1/2 of sigmoid(x) = 1/2 + 1/2 tanh(x/2); the z statistics use k 0..7 of the correction step, the x statistics k 8..15.
+template <bool kF16>
+struct ToWeights {
+  const float *ln_in_w, *ln_in_b, *ln_out_w, *ln_out_b;
+  const bf16 *w_z, *w_g;
+  static constexpr int kBytes = ToLayout::zt;
+  __device__ __forceinline__ void fold(unsigned char* sm, int, int warp, int warps, int lane, int tid, int threads) const {
+    fold_weight_rows<kF16, kF16>(sm + ToLayout::wg, sm + ToLayout::wxg, 0, kToWPanel, w_g, 0, 128, ln_in_w, ln_in_b, 0.5f, warp, warps,
+                                 lane, 0);
+    fold_weight_rows<true, true>(sm + ToLayout::wz, sm + ToLayout::wxz, 0, kToWPanel, w_z, 0, 128, ln_out_w, ln_out_b, 1.0f, warp, warps,
+                                 lane, 1);
+    for (int i = tid; i < 2 * 2 * 16 * 8; i += threads) {   // rows of ones behind both weights
+      const int panel = i >> 7, piece = i & 127;
+      const uint32_t one = ones16x2(panel >= 2 || kF16);     // panels 0, 1: gate weights, 2, 3: projection
+      *reinterpret_cast<uint4*>(sm + ToLayout::wg + panel * kToWPanel + 128 * 128 + piece * 16) = make_uint4(one, one, one, one);
+    }
+    for (int i = tid; i < 2 * 16 * 2; i += threads)          // ... which take no correction
+      *reinterpret_cast<uint4*>(sm + ToLayout::wxg + (i >> 5) * kToWExtra + 128 * 32 + (i & 31) * 16) = make_uint4(0u, 0u, 0u, 0u);
+    for (int i = 2 * (kToWBytes + kToWExtra) + tid * 16; i < kBytes; i += threads * 16)   // padding up to the tiles
+      *reinterpret_cast<uint4*>(sm + i) = make_uint4(0u, 0u, 0u, 0u);
+  }
+};
+
 template <typename Tz>
 __global__ void __launch_bounds__(kToThreads, 1)
 trimul_out_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_constant__ CUtensorMap map_x,
                      const __grid_constant__ CUtensorMap map_out, const Tz* __restrict__ z_in, Tz* __restrict__ z_out,
-                     const float* __restrict__ ln_in_w, const float* __restrict__ ln_in_b,
-                     const float* __restrict__ ln_out_w, const float* __restrict__ ln_out_b, const bf16* __restrict__ w_z,
-                     const bf16* __restrict__ w_g, int n_i, int n, int add_residual, float eps, int tiles_j, int n_tiles) {
+                     const ToWeights<sizeof(Tz) != 2> weights, const unsigned char* __restrict__ folded,
+                     int n_i, int n, int add_residual, float eps, int tiles_j, int n_tiles) {
   constexpr bool kTma = sizeof(Tz) == 2;               // bf16: residual from the z tile, output through TMA
   constexpr bool kF16 = !kTma;                           // operand format of the z side; the x side is always fp16
   extern __shared__ __align__(1024) unsigned char smem_raw[];
@@ -70,13 +93,14 @@ trimul_out_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_con
   ToBars& bars = *reinterpret_cast<ToBars*>(sm + ToLayout::bars);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
-  if (cta_skip_after_error()) return;   // an earlier bounded wait gave up: do not start new work
+  const bool skip = cta_begin();         // an earlier bounded wait gave up: do not start new work
   if (threadIdx.x == 0) {
     for (int s = 0; s < kToStages; ++s) {
       mbar_init(&bars.raw_full[s], 1);
       mbar_init(&bars.a_ready[s], 4);
       mbar_init(&bars.a_empty[s], 4);                      // three issuing threads and the store of the output rows
     }
+    mbar_init(&bars.w_full, 1);
     mbar_init(&bars.gram_full, 1);
     mbar_init(&bars.gram_free, 4);
     mbar_init(&bars.main_full, 2);
@@ -90,27 +114,14 @@ trimul_out_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_con
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
   }
-  {
-    // weights -> resident operands; the gate rows carry the 1/2 of sigmoid(x) = 1/2 + 1/2 tanh(x/2).  The z
-    // statistics use k 0..7 of the correction step, the x statistics k 8..15.
-    fold_weight_rows<kF16, kF16>(sm + ToLayout::wg, sm + ToLayout::wxg, 0, kToWPanel, w_g, 0, 128, ln_in_w, ln_in_b, 0.5f, warp, kToWarps,
-                     lane, 0);
-    fold_weight_rows<true, true>(sm + ToLayout::wz, sm + ToLayout::wxz, 0, kToWPanel, w_z, 0, 128, ln_out_w, ln_out_b, 1.0f, warp, kToWarps,
-                     lane, 1);
-    for (int i = threadIdx.x; i < 2 * 2 * 16 * 8; i += kToThreads) {   // rows of ones behind both weights
-      const int panel = i >> 7, piece = i & 127;
-      const uint32_t one = ones16x2(panel >= 2 || kF16);     // panels 0, 1: gate weights, 2, 3: projection
-      *reinterpret_cast<uint4*>(sm + ToLayout::wg + panel * kToWPanel + 128 * 128 + piece * 16) = make_uint4(one, one, one, one);
-    }
-    for (int i = threadIdx.x; i < 2 * 16 * 2; i += kToThreads)         // ... which take no correction
-      *reinterpret_cast<uint4*>(sm + ToLayout::wxg + (i >> 5) * kToWExtra + 128 * 32 + (i & 31) * 16) = make_uint4(0u, 0u, 0u, 0u);
-    for (int i = threadIdx.x; i < kToStages * 128 * 2; i += kToThreads)  // tile-side panels start out finite
-      *reinterpret_cast<uint4*>(sm + ToLayout::ax + i * 16) = make_uint4(0u, 0u, 0u, 0u);
-    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-  }
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
+  for (int i = threadIdx.x; i < kToStages * 128 * 2; i += kToThreads)  // tile-side panels start out finite
+    *reinterpret_cast<uint4*>(sm + ToLayout::ax + i * 16) = make_uint4(0u, 0u, 0u, 0u);
+  asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+  if (!cta_ready(skip, warp == 20, bars.tmem_base, 512u, [&] {
+        if (folded && threadIdx.x == 0) folded_load(sm, folded, ToWeights<kF16>::kBytes, &bars.w_full);
+      }))
+    return;
+  fold_here(weights, folded, sm, 0, &bars.w_full);
   const uint32_t tmem_base = bars.tmem_base;
   const int first_tile = blockIdx.x, tile_step = gridDim.x;
 
@@ -167,7 +178,8 @@ trimul_out_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_con
         const uint32_t w_addr = smem_u32(sm + (proj ? ToLayout::wz : ToLayout::wg));
         const uint64_t wx_desc = umma_desc_sw32(smem_u32(sm + (proj ? ToLayout::wxz : ToLayout::wxg)));
         int k = 0;
-        for (int tile = first_tile; tile < n_tiles; tile += tile_step, ++k) {
+        const bool have_w = mbar_wait(&bars.w_full, 0, 4u);      // the resident weights
+        for (int tile = first_tile; tile < n_tiles && have_w; tile += tile_step, ++k) {
           const int s = k % kToStages, m = k / kToStages;
           if (!mbar_wait(&bars.raw_full[s], m & 1, 4u) || !mbar_wait(&bars.acc_free, (k & 1) ^ 1, 8u)) break;
           tc_fence_after();
@@ -334,8 +346,8 @@ trimul_out_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_con
 PX_DEFINE_FAMILY_HOOKS(trimul_out)
 
 template <typename Tz>
-static int32_t launch_trimul_out(const px_f16* x, const void* z_in, const px_f16* zn, void* z_out, const float* ln_in_w, const float* ln_in_b,
-                                 const float* ln_out_w, const float* ln_out_b, const px_bf16* w_z, const px_bf16* w_g,
+static int32_t launch_trimul_out(const px_f16* x, const void* z_in, const px_f16* zn, void* z_out,
+                                 const ToWeights<sizeof(Tz) != 2>& weights, const void* folded,
                                  int64_t n_i, int64_t n, int64_t ld, int32_t add_residual, float eps, cudaStream_t st) {
   CUtensorMap mz, mx, mout;
   // operand rows: bf16 z itself, or the standardised fp16 copy of an fp32 z
@@ -355,36 +367,74 @@ static int32_t launch_trimul_out(const px_f16* x, const void* z_in, const px_f16
                    (uint64_t)n_i * ld * 2, 64, 1, CU_TENSOR_MAP_SWIZZLE_128B, 128))
     return PX_ERR_LAUNCH;
   const size_t smem = ToLayout::total + 1024;
-  if (cudaFuncSetAttribute(trimul_out_tc_kernel<Tz>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-    return PX_ERR_LAUNCH;
+  static SmemLimit limit;
+  if (!limit.set(trimul_out_tc_kernel<Tz>, smem)) return PX_ERR_LAUNCH;
   const int64_t tiles_j = (n + 127) / 128, n_tiles = tiles_j * n_i;
   if (n_tiles > 0x7fffffff) return PX_ERR_UNSUPPORTED;
   const int grid = (int)(n_tiles < sm_count() ? n_tiles : sm_count());
-  trimul_out_tc_kernel<Tz><<<grid, kToThreads, smem, st>>>(mz, mx, mout, (const Tz*)z_in, (Tz*)z_out, ln_in_w, ln_in_b,
-                                                           ln_out_w, ln_out_b, (const bf16*)w_z, (const bf16*)w_g, (int)n_i,
-                                                           (int)n, add_residual, eps, (int)tiles_j, (int)n_tiles);
-  return cudaGetLastError() == cudaSuccess ? PX_OK : PX_ERR_LAUNCH;
+  return launch_pdl(trimul_out_tc_kernel<Tz>, dim3(grid), kToThreads, smem, st, mz, mx, mout, (const Tz*)z_in, (Tz*)z_out, weights,
+                    (const unsigned char*)folded, (int)n_i, (int)n, (int)add_residual, eps, (int)tiles_j, (int)n_tiles)
+             ? PX_OK
+             : PX_ERR_LAUNCH;
+}
+
+static bool trimul_out_args_ok(const px_f16* x, const void* z_in, const px_f16* zn, const void* z_out, int32_t z_dtype, int64_t n_i,
+                               int64_t n_j, int64_t ld) {
+  return x && z_in && z_out && !(z_dtype == PX_F32 && (!zn || ((uintptr_t)zn & 15))) && n_i > 0 && n_j > 0 && n_i <= 32768 &&
+         n_j <= 32768 && ld == px_ld(n_j) && !(((uintptr_t)x | (uintptr_t)z_in | (uintptr_t)z_out) & 15);
+}
+template <bool kF16>
+static ToWeights<kF16> to_weights(const float* ln_in_w, const float* ln_in_b, const float* ln_out_w, const float* ln_out_b,
+                                  const px_f16* w_z, const px_w16* w_g) {
+  return {ln_in_w, ln_in_b, ln_out_w, ln_out_b, (const bf16*)w_z, (const bf16*)w_g};
+}
+static bool to_weights_ok(const float* ln_in_w, const float* ln_in_b, const float* ln_out_w, const float* ln_out_b,
+                          const px_f16* w_z, const px_w16* w_g) {
+  return ln_in_w && ln_in_b && ln_out_w && ln_out_b && w_z && w_g &&
+         !(((uintptr_t)w_z | (uintptr_t)w_g | (uintptr_t)ln_in_w | (uintptr_t)ln_in_b | (uintptr_t)ln_out_w | (uintptr_t)ln_out_b) & 15);
 }
 
 }  // namespace px
 
 using namespace px;
 
+extern "C" int64_t px_trimul_out_folded_bytes(void) { return ToWeights<true>::kBytes; }
+
+extern "C" int32_t px_trimul_out_fold(const float* ln_in_w, const float* ln_in_b, const float* ln_out_w, const float* ln_out_b,
+                                      const px_f16* w_z, const px_w16* w_g, int32_t rows_dtype, void* folded, void* stream) {
+  if (!to_weights_ok(ln_in_w, ln_in_b, ln_out_w, ln_out_b, w_z, w_g) || !folded || ((uintptr_t)folded & 15)) return PX_ERR_BAD_ARG;
+  if (rows_dtype != PX_F16 && rows_dtype != PX_BF16) return PX_ERR_UNSUPPORTED;
+  cudaStream_t st = (cudaStream_t)stream;
+  return (rows_dtype == PX_F16 ? launch_fold(to_weights<true>(ln_in_w, ln_in_b, ln_out_w, ln_out_b, w_z, w_g), 1, folded, st)
+                               : launch_fold(to_weights<false>(ln_in_w, ln_in_b, ln_out_w, ln_out_b, w_z, w_g), 1, folded, st))
+             ? PX_OK
+             : PX_ERR_LAUNCH;
+}
+
+extern "C" int32_t px_trimul_out_folded(const px_f16* x, const void* z_in, const px_f16* zn, void* z_out, int32_t z_dtype,
+                                        const void* folded, int64_t n_i, int64_t n_j, int64_t ld, int32_t add_residual, float eps,
+                                        void* stream) {
+  if (!trimul_out_args_ok(x, z_in, zn, z_out, z_dtype, n_i, n_j, ld) || !folded || ((uintptr_t)folded & 15)) return PX_ERR_BAD_ARG;
+  cudaStream_t st = (cudaStream_t)stream;
+  if (z_dtype == PX_F32)
+    return launch_trimul_out<float>(x, z_in, zn, z_out, ToWeights<true>{}, folded, n_i, n_j, ld, add_residual, eps, st);
+  if (z_dtype == PX_BF16)
+    return launch_trimul_out<bf16>(x, z_in, nullptr, z_out, ToWeights<false>{}, folded, n_i, n_j, ld, add_residual, eps, st);
+  return PX_ERR_UNSUPPORTED;
+}
+
 extern "C" int32_t px_trimul_out(const px_f16* x, const void* z_in, const px_f16* zn, void* z_out, int32_t z_dtype,
                                  const float* ln_in_w, const float* ln_in_b, const float* ln_out_w,
                                  const float* ln_out_b, const px_f16* w_z, const px_w16* w_g, int64_t n_i,
                                  int64_t n_j, int64_t ld, int32_t add_residual, float eps, void* stream) {
-  if (!x || !z_in || !z_out || !ln_in_w || !ln_in_b || !ln_out_w || !ln_out_b || !w_z || !w_g) return PX_ERR_BAD_ARG;
-  if (z_dtype == PX_F32 && (!zn || ((uintptr_t)zn & 15))) return PX_ERR_BAD_ARG;
-  if (n_i <= 0 || n_j <= 0 || n_i > 32768 || n_j > 32768 || ld != px_ld(n_j)) return PX_ERR_BAD_ARG;
-  if (((uintptr_t)x | (uintptr_t)z_in | (uintptr_t)z_out | (uintptr_t)w_z | (uintptr_t)w_g | (uintptr_t)ln_in_w |
-       (uintptr_t)ln_in_b | (uintptr_t)ln_out_w | (uintptr_t)ln_out_b) & 15)
+  if (!to_weights_ok(ln_in_w, ln_in_b, ln_out_w, ln_out_b, w_z, w_g) || !trimul_out_args_ok(x, z_in, zn, z_out, z_dtype, n_i, n_j, ld))
     return PX_ERR_BAD_ARG;
+  cudaStream_t st = (cudaStream_t)stream;
   if (z_dtype == PX_F32)
-    return launch_trimul_out<float>(x, z_in, zn, z_out, ln_in_w, ln_in_b, ln_out_w, ln_out_b, w_z, w_g, n_i, n_j, ld,
-                                    add_residual, eps, (cudaStream_t)stream);
+    return launch_trimul_out<float>(x, z_in, zn, z_out, to_weights<true>(ln_in_w, ln_in_b, ln_out_w, ln_out_b, w_z, w_g), nullptr, n_i,
+                                    n_j, ld, add_residual, eps, st);
   if (z_dtype == PX_BF16)
-    return launch_trimul_out<bf16>(x, z_in, nullptr, z_out, ln_in_w, ln_in_b, ln_out_w, ln_out_b, w_z, w_g, n_i, n_j, ld,
-                                   add_residual, eps, (cudaStream_t)stream);
+    return launch_trimul_out<bf16>(x, z_in, nullptr, z_out, to_weights<false>(ln_in_w, ln_in_b, ln_out_w, ln_out_b, w_z, w_g), nullptr,
+                                   n_i, n_j, ld, add_residual, eps, st);
   return PX_ERR_UNSUPPORTED;
 }

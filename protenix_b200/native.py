@@ -24,8 +24,8 @@ def load():
     return _ext
 
 
-def params(root, spec: Sequence[Tuple[str, str, Tuple[int, ...]]], scalars: Sequence[str]):
-    """A ``Params`` object over ``root``: spec lists (path of a parameter, kind, shape), scalars the paths of plain
+def params(root, group: str, spec: Sequence[Tuple[str, str, Tuple[int, ...]]], scalars: Sequence[str]):
+    """A ``Params`` object of a ``group`` over ``root``: spec lists (path of a parameter, kind, shape), scalars the paths of plain
     attributes.  The path's last part is the name, the parts before it submodules, which are checked for identity."""
     checks, places = [], []
 
@@ -41,7 +41,7 @@ def params(root, spec: Sequence[Tuple[str, str, Tuple[int, ...]]], scalars: Sequ
         module, name = owner(path)
         places.append((module._parameters, name, kind, list(shape)))
     attributes = [(module.__dict__, name) for module, name in map(owner, scalars)]
-    return load().Params(list(dict(((id(d), n), (d, n)) for d, n in checks).values()), places, attributes)
+    return load().Params(group, list(dict(((id(d), n), (d, n)) for d, n in checks).values()), places, attributes)
 
 
 def kept(module, make, name: str = "_px_params"):
@@ -53,6 +53,6 @@ def kept(module, make, name: str = "_px_params"):
     return held
 
 
-def under(prefix: str, spec, scalars):
-    """The same spec seen from a parent module."""
-    return [(f"{prefix}.{p}", k, s) for p, k, s in spec], [f"{prefix}.{p}" for p in scalars]
+def under(prefix: str, group: str, spec, scalars):
+    """The same description seen from a parent module."""
+    return group, [(f"{prefix}.{p}", k, s) for p, k, s in spec], [f"{prefix}.{p}" for p in scalars]

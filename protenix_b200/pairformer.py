@@ -47,7 +47,7 @@ class PairformerBlock(nn.Module):
 
     # the single-representation branch: vectors, then the eight matrices in the order of px_single_prepare
     _V, _A, _T = (ops.C_S,), "attention_pair_bias", "single_transition"
-    NATIVE_SINGLE = ([(f"{_A}.layernorm_a.weight", "f", _V), (f"{_A}.layernorm_a.bias", "f", _V),
+    NATIVE_SINGLE = ("single", [(f"{_A}.layernorm_a.weight", "f", _V), (f"{_A}.layernorm_a.bias", "f", _V),
                       (f"{_A}.attention.linear_q.bias", "f", _V), (f"{_T}.layernorm1.weight", "f", _V),
                       (f"{_T}.layernorm1.bias", "f", _V)]
                      + [(f"attention_pair_bias.attention.linear_{x}.weight", "s", (ops.C_S, ops.C_S)) for x in "qkvgo"]

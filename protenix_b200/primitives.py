@@ -66,7 +66,7 @@ class Transition(nn.Module):
     """x -> W_o(silu(W_a LN(x)) * (W_b LN(x))); returns the update (no residual)."""
 
     _V = (ops.C_Z,)
-    NATIVE = ([("layernorm1.weight", "f", _V), ("layernorm1.bias", "f", _V), ("linear_no_bias_a.weight", "h", (4 * ops.C_Z, ops.C_Z)),
+    NATIVE = ("plain", [("layernorm1.weight", "f", _V), ("layernorm1.bias", "f", _V), ("linear_no_bias_a.weight", "h", (4 * ops.C_Z, ops.C_Z)),
                ("linear_no_bias_b.weight", "h", (4 * ops.C_Z, ops.C_Z)), ("linear_no_bias.weight", "h", (ops.C_Z, 4 * ops.C_Z))],
               ["layernorm1.eps"])
 

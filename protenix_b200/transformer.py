@@ -37,7 +37,7 @@ class _SingleAttention(nn.Module):
 
 
 class AttentionPairBias(nn.Module):
-    NATIVE = ([("layernorm_z.weight", "f", (ops.C_Z,)), ("layernorm_z.bias", "f", (ops.C_Z,)),
+    NATIVE = ("bias", [("layernorm_z.weight", "f", (ops.C_Z,)), ("layernorm_z.bias", "f", (ops.C_Z,)),
                ("linear_nobias_z.weight", "z", (ops.N_HEAD_SINGLE, ops.C_Z))], ["layernorm_z.eps"])   # the pair bias
 
     def __init__(self, has_s: bool = True, create_offset_ln_z: bool = False, n_heads: int = 16, c_a: int = 768,

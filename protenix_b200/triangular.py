@@ -86,7 +86,7 @@ class TriangleMultiplicativeUpdate(BaseTriangleMultiplicativeUpdate):
     """Algorithms 11 / 12.  ``forward`` returns the update, or z + update with ``_add_with_inplace``."""
 
     _V, _M = (ops.C_Z,), (ops.C_Z, ops.C_Z)
-    NATIVE = ([("layer_norm_in.weight", "f", _V), ("layer_norm_in.bias", "f", _V), ("layer_norm_out.weight", "f", _V),
+    NATIVE = ("mul", [("layer_norm_in.weight", "f", _V), ("layer_norm_in.bias", "f", _V), ("layer_norm_out.weight", "f", _V),
                ("layer_norm_out.bias", "f", _V), ("linear_a_p.weight", "z", _M), ("linear_a_g.weight", "z", _M),
                ("linear_b_p.weight", "z", _M), ("linear_b_g.weight", "z", _M), ("linear_z.weight", "h", _M),
                ("linear_g.weight", "z", _M)], ["layer_norm_in.eps"])
@@ -157,7 +157,7 @@ class TriangleAttention(nn.Module):
     """Algorithms 13 / 14.  ``forward`` returns the update (no residual), like the reference."""
 
     _V, _M = (ops.C_Z,), (ops.C_Z, ops.C_Z)
-    NATIVE = ([("layer_norm.weight", "f", _V), ("layer_norm.bias", "f", _V), ("linear.weight", "z", (ops.N_HEAD_PAIR, ops.C_Z)),
+    NATIVE = ("att", [("layer_norm.weight", "f", _V), ("layer_norm.bias", "f", _V), ("linear.weight", "z", (ops.N_HEAD_PAIR, ops.C_Z)),
                ("mha.linear_q.weight", "z", _M), ("mha.linear_k.weight", "z", _M), ("mha.linear_v.weight", "z", _M),
                ("mha.linear_g.weight", "z", _M), ("mha.linear_o.weight", "h", _M)], ["layer_norm.eps", "inf"])
 
