@@ -17,7 +17,7 @@
 // bound by the latency of one tile (load, 24 MMAs per 64 inputs, epilogue); hence narrow 64-column tiles, no
 // persistence, and the split contraction where it is 1536 long.  Whole branch on an idle GPU: 64 us at N = 128 and 76 us at
 // N = 384, where library GEMMs and the composed attention took 290 us; 0.36 ms against 0.76 at N = 1536.
-#include "px_rowpipe.cuh"
+#include "px_split.cuh"
 
 namespace px {
 
@@ -47,35 +47,6 @@ struct SgBars {
   uint64_t full[kSgStages], empty[kSgStages], acc_full;
   uint32_t tmem_base;
 };
-
-// x = b0 + b1 + b2 with bf16 terms.
-__device__ __forceinline__ void split3(float x, bf16 (&b)[3]) {
-  b[0] = __float2bfloat16_rn(x);
-  const float r = x - __bfloat162float(b[0]);
-  b[1] = __float2bfloat16_rn(r);
-  b[2] = __float2bfloat16_rn(r - __bfloat162float(b[1]));
-}
-__device__ __forceinline__ void split3x2(float x, float y, uint32_t (&w)[3]) {
-  bf16 a[3], b[3];
-  split3(x, a);
-  split3(y, b);
-#pragma unroll
-  for (int p = 0; p < 3; ++p)
-    w[p] = (uint32_t)__bfloat16_as_ushort(a[p]) | ((uint32_t)__bfloat16_as_ushort(b[p]) << 16);
-}
-
-template <typename T>
-__device__ __forceinline__ float4 ld4(const T* p);
-template <>
-__device__ __forceinline__ float4 ld4<float>(const float* p) { return *reinterpret_cast<const float4*>(p); }
-template <>
-__device__ __forceinline__ float4 ld4<bf16>(const bf16* p) { return load4(p); }
-template <>
-__device__ __forceinline__ float4 ld4<__half>(const __half* p) {
-  const uint2 u = *reinterpret_cast<const uint2*>(p);
-  const float2 a = unpack_f16x2(u.x), b = unpack_f16x2(u.y);
-  return make_float4(a.x, a.y, b.x, b.y);
-}
 
 // LayerNorm of rows of 384, written as three bf16 planes; one warp per row, the row in registers.
 template <typename T>
@@ -110,18 +81,6 @@ __global__ void __launch_bounds__(128) split_rows_kernel(const T* __restrict__ x
 #pragma unroll
     for (int p = 0; p < 3; ++p)
       *reinterpret_cast<uint2*>(out + ((size_t)p * rows + row) * kSc + c) = make_uint2(lo[p], hi[p]);
-  }
-}
-
-// fp32 weight rows -> three bf16 planes; source row r goes to row (r / blk) * stride + off + r % blk.
-__global__ void split_weight_kernel(const float* __restrict__ w, bf16* __restrict__ out, int rows, int k, int out_rows,
-                                    int blk, int stride, int off) {
-  const int r = blockIdx.x, dst = (r / blk) * stride + off + r % blk;
-  for (int c = threadIdx.x; c < k; c += blockDim.x) {
-    bf16 b[3];
-    split3(w[(size_t)r * k + c], b);
-#pragma unroll
-    for (int p = 0; p < 3; ++p) out[((size_t)p * out_rows + dst) * k + c] = b[p];
   }
 }
 
@@ -465,12 +424,6 @@ PX_DEFINE_FAMILY_HOOKS(single)
 // Prepared weights: planes of [q|k|v|g] (1536 x 384), W_o (384 x 384), [a|b] interleaved (3072 x 384), W_out (384 x 1536)
 constexpr int64_t kSwQkvg = 0, kSwO = kSwQkvg + 3ll * kSf * kSc, kSwAb = kSwO + 3ll * kSc * kSc,
                   kSwOut = kSwAb + 3ll * 2 * kSf * kSc, kSwEnd = kSwOut + 3ll * kSc * kSf;
-
-// planes [3][rows][k] bf16, box [3][box_rows][64]
-static bool make_plane_map(CUtensorMap* map, const bf16* base, int64_t rows, int64_t k, uint32_t box_rows) {
-  return make_map_3d(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, base, (uint64_t)k, (uint64_t)rows, 3, (uint64_t)k * 2,
-                     (uint64_t)rows * k * 2, 64, box_rows, CU_TENSOR_MAP_SWIZZLE_128B, 3);
-}
 
 template <int kMode, typename T>
 static bool launch_split_gemm(const bf16* a, const bf16* w, int64_t w_rows, int64_t k, int split, SgArgs g, cudaStream_t st) {

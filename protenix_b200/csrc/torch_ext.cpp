@@ -11,10 +11,14 @@
 #include <ATen/ATen.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <ATen/cuda/CUDAEvent.h>
+#include <ATen/ops/bmm.h>
 #include <ATen/ops/dropout.h>
 #include <ATen/ops/empty.h>
 #include <ATen/ops/empty_like.h>
+#include <ATen/ops/full.h>
+#include <ATen/ops/mm.h>
 #include <ATen/ops/ones.h>
+#include <ATen/ops/softmax.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <dlfcn.h>
@@ -50,7 +54,9 @@ constexpr int64_t kCz = 128, kCs = 384, kHeadsSingle = 16, kHeads = 4, kHeadDim 
   X(px_triatt_in_proj_folded) X(px_triatt_flash) X(px_triatt_flash_scratch_bytes) X(px_triatt_out_folded_bytes)          \
   X(px_triatt_out_fold) X(px_triatt_out_folded) X(px_triatt_workspace_bytes) X(px_transition)                            \
   X(px_pair_bias_folded_bytes) X(px_pair_bias_fold) X(px_pair_bias_proj_folded) X(px_single_weights_bytes)               \
-  X(px_single_workspace_bytes) X(px_single_prepare) X(px_single_update)
+  X(px_single_workspace_bytes) X(px_single_prepare) X(px_single_update) X(px_opm_outer) X(px_opm_out)                    \
+  X(px_msa_opm_prep) X(px_msa_values) X(px_msa_gate_out) X(px_msa_transition_weights_bytes)                              \
+  X(px_msa_transition_prepare) X(px_msa_transition)
 struct Abi {
 #define X(f) decltype(&::f) f = nullptr;
   PX_FUNCTIONS(X)
@@ -143,8 +149,9 @@ const float* fptr(const Tensor& t) { return t.defined() ? (const float*)t.data_p
 // ---- parameters of a module -----------------------------------------------------------------------------------------
 // What a parameter becomes: 'f' an fp32 vector, 'z' a matrix in the format of the pair tensor's rows (bf16 rows: bf16, fp32
 // rows: fp16), 'h' an fp16 matrix, 's' an fp32 matrix.  What the group becomes then: kMul, kAtt and kBias the folded weights
-// of their row kernels (in, out), kSingle the laid-out matrices of the single branch behind its vectors, kPlain nothing more.
-enum Group { kPlain, kMul, kAtt, kBias, kSingle };
+// of their row kernels (in, out), kSingle and kMsa the laid-out matrices of the single branch and of the MSA transition behind what comes before them,
+// kPlain nothing more.
+enum Group { kPlain, kMul, kAtt, kBias, kSingle, kMsa };
 struct Prepared {
   std::vector<Tensor> t[2];          // by format of z: 0 fp32, 1 bf16
   std::vector<const void*> p[2];
@@ -158,10 +165,10 @@ class Params {
  public:
   // checks: (dict, name) of submodules; params: (dict, name, kind, shape); scalars: (dict, name)
   Params(const std::string& group, const py::list& checks, const py::list& params, const py::list& scalars) {
-    const char* names[] = {"plain", "mul", "att", "bias", "single"};
+    const char* names[] = {"plain", "mul", "att", "bias", "single", "msa"};
     int g = 0;
-    while (g < 5 && group != names[g]) ++g;
-    if (g == 5) fail("unknown parameter group " + group);
+    while (g < 6 && group != names[g]) ++g;
+    if (g == 6) fail("unknown parameter group " + group);
     group_ = (Group)g;
     for (const auto& c : checks) {
       const auto t = c.cast<py::tuple>();
@@ -298,6 +305,11 @@ class Params {
         return abi.px_single_prepare(f(5), f(6), f(7), f(8), f(9), f(10), f(11), f(12), out.data_ptr(), st);
       });
       t.resize(5);
+      t.push_back(out);
+    } else if (group_ == kMsa) {
+      const Tensor out = at::empty({abi.px_msa_transition_weights_bytes()}, byte);
+      launch("px_msa_transition_prepare", st, [&] { return abi.px_msa_transition_prepare(f(7), f(8), f(9), out.data_ptr(), st); });
+      t.resize(7);
       t.push_back(out);
     }
     p.t[zf] = t;
@@ -580,6 +592,96 @@ std::tuple<OptTensor, Tensor> stack_forward(const std::vector<std::shared_ptr<Bl
   return {s.defined() ? OptTensor(s) : OptTensor(), batch ? zc.unsqueeze(0) : zc};
 }
 
+// ---- MSA module ------------------------------------------------------------------------------------------------------
+// z_out = [z_in +] OuterProductMean(m) for m [S, N, 64] fp32; x_bytes bounds the outer products formed at a time.
+Tensor opm_forward(Params& params, const Tensor& m, const OptTensor& mask, const OptTensor& z_in, const Tensor& z_out, int64_t x_bytes) {
+  need_cuda(m, "m");
+  c10::cuda::CUDAGuard guard(m.device());
+  at::NoGradGuard no_grad;
+  const int64_t s_rows = m.size(0), n = m.size(1), ld = (s_rows + 7) / 8 * 8;
+  if (m.dim() != 3 || m.size(2) != 64 || m.scalar_type() != at::kFloat || !m.is_contiguous()) fail("m must be a contiguous float32 [S, N, 64] tensor");
+  if (n > 32768 || n < 1 || s_rows < 1) fail("outer_product_mean supports 1 <= N <= 32768 tokens");
+  const bool residual = z_in.has_value() && z_in->defined();
+  for (const Tensor& z : {z_out, residual ? *z_in : z_out})
+    if (z.dim() != 3 || z.size(0) != n || z.size(1) != n || z.size(2) != kCz || !z.is_contiguous() || z.scalar_type() != z_out.scalar_type())
+      fail("z must be contiguous [N, N, 128] with N = m.shape[1]");
+  Tensor mk;
+  if (mask.has_value() && mask->defined()) {
+    need_cuda(*mask, "msa_mask");
+    if (mask->dim() != 2 || mask->size(0) != s_rows || mask->size(1) != n) fail("msa_mask must be [N_seq, N_res]");
+    mk = mask->to(at::kFloat).contiguous();
+  }
+  const Ready pr = params.get(0, m.device());
+  py::gil_scoped_release release;
+  const auto& p = pr->p[0];
+  const float eps = pr->scalars[0], ln_eps = pr->scalars[1];
+  const auto opt = m.options();
+  const Tensor ab = at::empty({2, n * 32, ld}, opt.dtype(at::kHalf));
+  px_f16 *a = (px_f16*)ab.data_ptr(), *b = a + n * 32 * ld;
+  const Tensor inv = mk.defined() ? at::mm(mk.t(), mk).add_(eps).reciprocal_() : at::full({n, n}, 1.0f / ((float)s_rows + eps), opt);
+  const int64_t n_blk = std::max<int64_t>(1, std::min(n, x_bytes / (2048 * n)));   // rows i of x = [32 n_i][32 N] fp16
+  const Tensor x = at::empty({n_blk * 32, n * 32}, opt.dtype(at::kHalf));
+  const cudaStream_t st = at::cuda::getCurrentCUDAStream();
+  launch("px_msa_opm_prep", st, [&] {
+    return abi.px_msa_opm_prep((const float*)m.data_ptr(), fptr(mk), (const float*)p[0], (const float*)p[1], (const float*)p[2],
+                               (const float*)p[3], a, b, s_rows, n, ld, ln_eps, st);
+  });
+  const int64_t row = z_out.element_size() * n * kCz;
+  for (int64_t i0 = 0; i0 < n; i0 += n_blk) {
+    const int64_t ni = std::min(n_blk, n - i0);
+    launch("px_opm_outer", st, [&] { return abi.px_opm_outer(a + i0 * 32 * ld, b, (px_f16*)x.data_ptr(), ni * 32, n * 32, ld, st); });
+    launch("px_opm_out", st, [&] {
+      return abi.px_opm_out((const px_f16*)x.data_ptr(), (const px_f16*)p[4], (const float*)p[5], (const float*)inv.data_ptr() + i0 * n,
+                            residual ? (const char*)z_in->data_ptr() + i0 * row : nullptr, (char*)z_out.data_ptr() + i0 * row,
+                            dtype_code(z_out, "z"), ni, n, residual, st);
+    });
+  }
+  return z_out;
+}
+
+// m += PairWeightedAveraging(m, z), m += Transition(m) in place over chunks of sequences: m [S, N, 64] fp32, 8 heads x 8.
+void msa_stack_forward(Params& params, Params& bias_params, const Tensor& m, const Tensor& z_, int64_t chunk) {
+  need_cuda(m, "m");
+  bool batch;
+  const Tensor z = pair_tensor(z_, batch);
+  c10::cuda::CUDAGuard guard(m.device());
+  at::NoGradGuard no_grad;
+  const int64_t s_all = m.size(0), n = m.size(1), heads = 8;
+  if (m.dim() != 3 || m.size(2) != 64 || n != z.size(0) || m.scalar_type() != at::kFloat || !m.is_contiguous())
+    fail("m must be a contiguous float32 [S, N, 64] tensor with z [N, N, 128]");
+  const int zf = zformat(z);
+  const Ready pr = params.get(0, m.device()), br = bias_params.get(zf, m.device());
+  py::gil_scoped_release release;
+  const auto& p = pr->p[0];
+  const cudaStream_t st = at::cuda::getCurrentCUDAStream();
+  const auto opt = m.options();
+  Tensor w = at::empty({heads, n, n}, opt), zn;
+  const void* rows = z.data_ptr();
+  if (zf == 0) {
+    zn = at::empty(z.sizes(), opt.dtype(at::kHalf));
+    launch("px_standardise_rows", st, [&] {
+      return abi.px_standardise_rows((const float*)z.data_ptr(), (px_f16*)zn.data_ptr(), n * n, br->scalars[0], st);
+    });
+    rows = zn.data_ptr();
+  }
+  launch("px_pair_bias_proj", st, [&] {
+    return abi.px_pair_bias_proj_folded(rows, zf ? PX_BF16 : PX_F16, br->p[zf][0], (float*)w.data_ptr(), n * n, (int32_t)heads, br->scalars[0], st);
+  });
+  w = at::softmax(w, -1);
+  auto f = [&](int i) { return (const float*)p[i]; };
+  for (int64_t s0 = 0; s0 < s_all; s0 += chunk) {
+    const int64_t s = std::min(chunk, s_all - s0);
+    float* part = (float*)m.data_ptr() + s0 * n * 64;
+    const Tensor v = at::empty({heads, n, s * 8}, opt);
+    launch("px_msa_values", st, [&] { return abi.px_msa_values(part, f(0), f(1), f(2), (float*)v.data_ptr(), s, n, pr->scalars[0], st); });
+    const Tensor wv = at::bmm(w, v);                 // one [N x N] . [N x 8 S] product per head, fp32
+    launch("px_msa_gate_out", st, [&] {
+      return abi.px_msa_gate_out(part, (const float*)wv.data_ptr(), f(0), f(1), f(3), f(4), s, n, pr->scalars[0], st);
+    });
+    launch("px_msa_transition", st, [&] { return abi.px_msa_transition(part, p[7], f(5), f(6), s * n, pr->scalars[1], st); });
+  }
+}
+
 // ---- LayerNorm -------------------------------------------------------------------------------------------------------
 struct LnParams {
   Tensor w, b;
@@ -750,6 +852,8 @@ PYBIND11_MODULE(_C, m) {
   m.def("tri_att_forward", &tri_att_forward);
   m.def("transition_forward", &transition_forward);
   m.def("stack_forward", &stack_forward);
+  m.def("opm_forward", &opm_forward);
+  m.def("msa_stack_forward", &msa_stack_forward);
   m.def("launches", [](bool reset) { return reset ? g_launches.exchange(0) : g_launches.load(); });
   m.def("timer", [](bool on) { g_timing = on; });
   m.def("timer_collect", &timer_collect);

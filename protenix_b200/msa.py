@@ -15,12 +15,16 @@ from typing import Optional
 import torch
 import torch.nn as nn
 
-from . import ops
+from . import native, ops
 from .layer_norm import LayerNorm
 from .triangular import OpenfoldLinear
 
 
 class OuterProductMean(nn.Module):
+    NATIVE = ("plain", [("layer_norm.weight", "f", (64,)), ("layer_norm.bias", "f", (64,)), ("linear_1.weight", "s", (32, 64)),
+                        ("linear_2.weight", "s", (32, 64)), ("linear_out.weight", "h", (128, 1024)), ("linear_out.bias", "f", (128,))],
+              ["eps", "layer_norm.eps"])
+
     def __init__(self, c_m: int, c_z: int, c_hidden: int, eps: float = 1e-3) -> None:
         super().__init__()
         self.c_m, self.c_z, self.c_hidden, self.eps = c_m, c_z, c_hidden, eps
@@ -31,6 +35,9 @@ class OuterProductMean(nn.Module):
 
     def _run(self, m: torch.Tensor, mask: Optional[torch.Tensor], z_in: Optional[torch.Tensor],
              z_out: torch.Tensor) -> torch.Tensor:
+        if m.dtype == torch.float32 and (self.c_m, self.c_z, self.c_hidden) == (64, ops.C_Z, 32):
+            params = native.kept(self, lambda: native.params(self, *self.NATIVE))
+            return native.load().opm_forward(params, m, mask, z_in, z_out, ops.OPM_X_BYTES)
         ln_b = self.layer_norm.bias
         return ops.outer_product_mean(z_in, z_out, m, mask, self.layer_norm.weight, ln_b, self.linear_1.weight,
                                       self.linear_2.weight, self.linear_out.weight, self.linear_out.bias,
@@ -113,6 +120,16 @@ class MSAPairWeightedAveraging(nn.Module):
 class MSAStack(nn.Module):
     """Mirror of protenix/model/modules/pairformer.py:425-572 (eval path: ``inference_forward``)."""
 
+    _A, _V, _M = "msa_pair_weighted_averaging", (64,), (64, 64)
+    NATIVE = ("msa", [(f"{_A}.layernorm_m.weight", "f", _V), (f"{_A}.layernorm_m.bias", "f", _V),
+                      (f"{_A}.linear_no_bias_mv.weight", "s", _M), (f"{_A}.linear_no_bias_mg.weight", "s", _M),
+                      (f"{_A}.linear_no_bias_out.weight", "s", _M), ("transition_m.layernorm1.weight", "f", _V),
+                      ("transition_m.layernorm1.bias", "f", _V), ("transition_m.linear_no_bias_a.weight", "s", (256, 64)),
+                      ("transition_m.linear_no_bias_b.weight", "s", (256, 64)), ("transition_m.linear_no_bias.weight", "s", (64, 256))],
+              [f"{_A}.layernorm_m.eps", "transition_m.layernorm1.eps"])
+    NATIVE_BIAS = ("bias", [(f"{_A}.layernorm_z.weight", "f", (ops.C_Z,)), (f"{_A}.layernorm_z.bias", "f", (ops.C_Z,)),
+                            (f"{_A}.linear_no_bias_z.weight", "z", (8, ops.C_Z))], [f"{_A}.layernorm_z.eps"])
+
     def __init__(self, c_m: int = 64, c_z: int = 128, c: int = 8, dropout: float = 0.15,
                  msa_chunk_size: Optional[int] = 2048, msa_max_size: Optional[int] = 16384) -> None:
         super().__init__()
@@ -129,7 +146,14 @@ class MSAStack(nn.Module):
         """m += PairWeightedAveraging(m, z); m += Transition(m), in place over chunks of MSA rows."""
         if self.training and self.p_drop > 0:
             raise RuntimeError("MSAStack: training-mode dropout is not implemented; call .eval()")
-        w = self.msa_pair_weighted_averaging.pair_weights(z)      # the same for every chunk
+        att = self.msa_pair_weighted_averaging
+        if m.dtype == torch.float32 and m.is_contiguous() and self.transition_m.n == 4 and \
+                (att.c_m, att.c, att.n_heads, att.c_z) == (64, 8, 8, ops.C_Z):
+            params = native.kept(self, lambda: native.params(self, *self.NATIVE))
+            bias = native.kept(self, lambda: native.params(self, *self.NATIVE_BIAS), "_px_bias_params")
+            native.load().msa_stack_forward(params, bias, m, z, self.msa_chunk_size or m.shape[0])
+            return m
+        w = att.pair_weights(z)                                   # the same for every chunk
         chunk = self.msa_chunk_size or m.shape[0]
         for start in range(0, m.shape[0], chunk):
             part = m[start:start + chunk]

@@ -1,0 +1,64 @@
+"""The MSA embedding's kernels (values, gated output, transition, outer-product operands) through MSAStack and OuterProductMean:
+no further from the modules' composition in fp64 than the same composition in fp32."""
+import pytest
+import torch
+from torch.nn import functional as F
+
+import protenix_b200 as px
+from protenix_b200 import ops
+from protenix_b200.init_utils import randomize_parameters_
+from protenix_b200.msa import MSAStack
+
+pytestmark = pytest.mark.gpu
+
+
+def _stack(mod, m, w, dt):
+    att, tr, g = mod.msa_pair_weighted_averaging, mod.transition_m, (lambda p: p.detach().to(dt))
+    m, w = m.to(dt), w.to(dt)
+    s, n, _ = m.shape
+    x = F.layer_norm(m, (64,), g(att.layernorm_m.weight), g(att.layernorm_m.bias), att.layernorm_m.eps)
+    v = F.linear(x, g(att.linear_no_bias_mv.weight)).view(s, n, 8, 8)
+    o = torch.sigmoid(F.linear(x, g(att.linear_no_bias_mg.weight))) * torch.einsum("hij,sjhc->sihc", w, v).reshape(s, n, 64)
+    m = m + F.linear(o, g(att.linear_no_bias_out.weight))
+    y = F.layer_norm(m, (64,), g(tr.layernorm1.weight), g(tr.layernorm1.bias), tr.layernorm1.eps)
+    h = F.silu(F.linear(y, g(tr.linear_no_bias_a.weight))) * F.linear(y, g(tr.linear_no_bias_b.weight))
+    return m + F.linear(h, g(tr.linear_no_bias.weight))
+
+
+@pytest.mark.parametrize("s,n,chunk", [(1, 1, 2048), (3, 17, 2048), (64, 33, 2048), (127, 40, 2048), (129, 24, 100), (130, 130, 64)])
+def test_msa_stack(s, n, chunk):
+    torch.manual_seed(s * n)
+    mod = randomize_parameters_(MSAStack(msa_chunk_size=chunk), 3).cuda().eval()
+    m, z = 2 * torch.randn(s, n, 64, device="cuda") + 0.5, torch.randn(n, n, 128, device="cuda")
+    relf = lambda a, b: float((a.double() - b).norm() / b.norm())
+    with torch.no_grad():
+        w = mod.msa_pair_weighted_averaging.pair_weights(z)
+        want = _stack(mod, m, w, torch.float64)
+        single = relf(_stack(mod, m, w, torch.float32), want)
+        got = mod(m.clone(), z)
+        ops.device_error_flags()
+        assert relf(got, want) < 2 * single + 1e-7, (relf(got, want), single)
+        assert torch.equal(got, mod(m.clone(), z))
+
+
+@pytest.mark.parametrize("s,n,masked", [(1, 1, False), (7, 5, True), (128, 9, True), (129, 3, False), (136, 20, True)])
+def test_outer_product_operands(s, n, masked):
+    """px_msa_opm_prep: values, zero padding and both halves of the projection."""
+    torch.manual_seed(s)
+    mod = randomize_parameters_(px.OuterProductMean(64, 128, 32), 5).cuda()
+    m = torch.randn(s, n, 64, device="cuda")
+    mask = (torch.rand(s, n, device="cuda") > 0.3).float() if masked else None
+    ld = (s + 7) // 8 * 8
+    a, b = (torch.full((n * 32, ld), 7.0, dtype=torch.float16, device="cuda") for _ in range(2))
+    from protenix_b200 import _lib
+
+    ln = mod.layer_norm
+    p = lambda t: None if t is None else t.data_ptr()
+    _lib.check(_lib.load().px_msa_opm_prep(p(m), p(mask), p(ln.weight), p(ln.bias), p(mod.linear_1.weight), p(mod.linear_2.weight),
+                                           p(a), p(b), s, n, ld, ln.eps, torch.cuda.current_stream().cuda_stream), "px_msa_opm_prep")
+    x = F.layer_norm(m.double(), (64,), ln.weight.detach().double(), ln.bias.detach().double(), ln.eps)
+    for got, lin in ((a, mod.linear_1), (b, mod.linear_2)):
+        want = F.linear(x, lin.weight.detach().double()) * (1.0 if mask is None else mask.double()[..., None])
+        want = want.permute(1, 2, 0).reshape(n * 32, s)
+        assert (got[:, s:] == 0).all()
+        assert float((got[:, :s].double() - want).abs().max()) < 6e-4 * max(1.0, float(want.abs().max()))
