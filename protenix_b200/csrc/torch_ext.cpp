@@ -684,27 +684,23 @@ void msa_stack_forward(Params& params, Params& bias_params, const Tensor& m, con
 
 // ---- LayerNorm -------------------------------------------------------------------------------------------------------
 struct LnParams {
-  Tensor w, b;
+  Tensor w, b;     // as the kernels take them: of the type of x, or fp32 (rounded to the type of x inside)
   int code;        // dtype code of both
 };
-// The parameters as the kernels take them: of the type of x, or fp32 (rounded to the type of x inside).
+bool has(const OptTensor& t) { return t.has_value() && t->defined(); }
 LnParams ln_params(const Tensor& x, const OptTensor& weight, const OptTensor& bias) {
   LnParams r;
-  auto fit = [&](const OptTensor& p, const char* name) -> Tensor {
-    if (!p.has_value() || !p->defined()) return Tensor();
+  const bool fp32 = (!has(weight) || weight->scalar_type() == at::kFloat) && (!has(bias) || bias->scalar_type() == at::kFloat);
+  const auto type = fp32 ? at::kFloat : x.scalar_type();
+  auto fit = [&](const OptTensor& p, const char* name, Tensor& to) {
+    if (!has(p)) return;
     need_cuda(*p, name);
     if (p->numel() != x.size(-1)) fail(std::string(name) + " must have as many elements as the last axis");
-    return p->detach();
+    to = p->scalar_type() == type && p->is_contiguous() ? *p : p->detach().to(type).contiguous();
   };
-  r.w = fit(weight, "weight");
-  r.b = fit(bias, "bias");
-  const Tensor& any = r.w.defined() ? r.w : r.b;
-  auto type = any.defined() && any.scalar_type() == at::kFloat && (!r.b.defined() || r.b.scalar_type() == at::kFloat)
-                  ? at::kFloat
-                  : x.scalar_type();
-  for (Tensor* t : {&r.w, &r.b})
-    if (t->defined()) *t = (t->scalar_type() == type ? *t : t->to(type)).contiguous();
-  r.code = type == at::kFloat ? PX_F32 : dtype_code(x, "input");
+  fit(weight, "weight", r.w);
+  fit(bias, "bias", r.b);
+  r.code = fp32 ? PX_F32 : dtype_code(x, "input");
   return r;
 }
 void ln_check(const Tensor& x, int64_t width) {
@@ -743,12 +739,11 @@ struct LayerNormFunction : torch::autograd::Function<LayerNormFunction> {
     Tensor mean, invvar;
     const Tensor y = ln_forward(xc, p, eps, &mean, &invvar);
     ctx->save_for_backward({xc, p.w, mean, invvar});
-    ctx->saved_data["code"] = (int64_t)p.code;
-    ctx->saved_data["w_type"] = (int64_t)(weight.has_value() && weight->defined() ? weight->scalar_type() : at::kFloat);
-    ctx->saved_data["b_type"] = (int64_t)(bias.has_value() && bias->defined() ? bias->scalar_type() : at::kFloat);
-    ctx->saved_data["want_w"] = weight.has_value() && weight->defined() && weight->requires_grad();
-    ctx->saved_data["want_b"] = bias.has_value() && bias->defined() && bias->requires_grad();
-    ctx->saved_data["want_x"] = x.requires_grad();
+    const int64_t w_type = (int64_t)(has(weight) ? weight->scalar_type() : at::kFloat);
+    const int64_t b_type = (int64_t)(has(bias) ? bias->scalar_type() : at::kFloat);
+    // one entry: dtype code, types of the parameters, which gradients are wanted
+    ctx->saved_data["f"] = (int64_t)p.code | w_type << 8 | b_type << 16 | (int64_t)(has(weight) && weight->requires_grad()) << 24 |
+                           (int64_t)(has(bias) && bias->requires_grad()) << 25 | (int64_t)x.requires_grad() << 26;
     return y;
   }
   static torch::autograd::variable_list backward(torch::autograd::AutogradContext* ctx, torch::autograd::variable_list grads) {
@@ -756,8 +751,9 @@ struct LayerNormFunction : torch::autograd::Function<LayerNormFunction> {
     const Tensor &x = saved[0], &w = saved[1], &mean = saved[2], &invvar = saved[3];
     c10::cuda::CUDAGuard guard(x.device());
     const Tensor dy = grads[0].contiguous();
-    const int code = (int)ctx->saved_data["code"].toInt();
-    const bool want_w = ctx->saved_data["want_w"].toBool(), want_b = ctx->saved_data["want_b"].toBool();
+    const int64_t flags = ctx->saved_data["f"].toInt();
+    const int code = (int)(flags & 255);
+    const bool want_w = flags >> 24 & 1, want_b = flags >> 25 & 1;
     const int64_t cols = x.size(-1), rows = cols ? x.numel() / cols : 0;
     const auto grad_type = code == PX_F32 ? at::kFloat : x.scalar_type();
     const Tensor dx = at::empty_like(x);
@@ -772,15 +768,17 @@ struct LayerNormFunction : torch::autograd::Function<LayerNormFunction> {
                                           want_b ? db.data_ptr() : nullptr, scratch.defined() ? (float*)scratch.data_ptr() : nullptr,
                                           rows, cols, dtype_code(x, "x"), code, st);
     });
-    auto as = [](const Tensor& t, int64_t type) { return t.defined() ? t.to((at::ScalarType)type) : t; };
-    return {ctx->saved_data["want_x"].toBool() ? dx : Tensor(), as(dw, ctx->saved_data["w_type"].toInt()),
-            as(db, ctx->saved_data["b_type"].toInt()), Tensor()};
+    auto as = [&](const Tensor& t, int shift) {
+      const auto type = (at::ScalarType)(flags >> shift & 255);
+      return !t.defined() || t.scalar_type() == type ? t : t.to(type);
+    };
+    return {flags >> 26 & 1 ? dx : Tensor(), as(dw, 8), as(db, 16), Tensor()};
   }
 };
 
 Tensor layer_norm(const Tensor& x, const OptTensor& weight, const OptTensor& bias, int64_t width, double eps) {
   ln_check(x, width);
-  auto wants = [](const OptTensor& t) { return t.has_value() && t->defined() && t->requires_grad(); };
+  auto wants = [](const OptTensor& t) { return has(t) && t->requires_grad(); };
   if (at::GradMode::is_enabled() && (x.requires_grad() || wants(weight) || wants(bias)))
     return LayerNormFunction::apply(x, weight, bias, eps);
   const Tensor xc = x.contiguous();
@@ -805,14 +803,13 @@ Tensor scale_add(const Tensor& residual, const Tensor& x_, const Tensor& mask) {
 struct DropoutAddFunction : torch::autograd::Function<DropoutAddFunction> {
   static Tensor forward(torch::autograd::AutogradContext* ctx, const Tensor& residual, const Tensor& x, const Tensor& mask) {
     ctx->save_for_backward({mask});
-    ctx->saved_data["want_r"] = residual.requires_grad();
-    ctx->saved_data["want_x"] = x.requires_grad();
+    ctx->saved_data["f"] = (int64_t)residual.requires_grad() | (int64_t)x.requires_grad() << 1;
     return scale_add(residual, x, mask);
   }
   static torch::autograd::variable_list backward(torch::autograd::AutogradContext* ctx, torch::autograd::variable_list grads) {
     const auto saved = ctx->get_saved_variables();
-    return {ctx->saved_data["want_r"].toBool() ? grads[0] : Tensor(),
-            ctx->saved_data["want_x"].toBool() ? scale_add(Tensor(), grads[0], saved[0]) : Tensor(), Tensor()};
+    const int64_t flags = ctx->saved_data["f"].toInt();
+    return {flags & 1 ? grads[0] : Tensor(), flags & 2 ? scale_add(Tensor(), grads[0], saved[0]) : Tensor(), Tensor()};
   }
 };
 
@@ -823,8 +820,13 @@ Tensor dropout_add(const Tensor& residual, const Tensor& x, double p) {
   if (!residual.is_cuda() || residual.sizes() != x.sizes() || residual.scalar_type() != x.scalar_type()) fail("residual must match x");
   auto shape = x.sizes().vec();
   shape[shape.size() - 3] = 1;
-  // drawn as a dropout of ones: the same generator calls, so that a seed gives the same mask
-  const Tensor mask = at::dropout(at::ones(shape, x.options().requires_grad(false)), p, true);
+  Tensor mask;
+  {
+    // drawn as a dropout of ones: the same generator calls, so that a seed gives the same mask
+    at::AutoDispatchBelowAutograd below;
+    mask = at::dropout(at::ones(shape, x.options()), p, true);
+  }
+  if (!at::GradMode::is_enabled() || !(residual.requires_grad() || x.requires_grad())) return scale_add(residual, x, mask);
   return DropoutAddFunction::apply(residual, x, mask);
 }
 

@@ -17,6 +17,13 @@ from torch.nn.parameter import Parameter
 from . import native
 
 
+def _layer_norm(*args):
+    """The native op; the first call puts it in this function's place."""
+    global _layer_norm
+    _layer_norm = native.load().layer_norm
+    return _layer_norm(*args)
+
+
 class FusedLayerNorm(torch.nn.Module):
     def __init__(self, normalized_shape: Union[int, list, torch.Size], create_scale: bool = True,
                  create_offset: bool = True, eps: float = 1e-5) -> None:
@@ -27,6 +34,7 @@ class FusedLayerNorm(torch.nn.Module):
         if len(self.normalized_shape) != 1:
             raise RuntimeError("FusedLayerNorm normalises over the last axis only")
         self.eps = eps
+        self._width = int(normalized_shape[0])
         self.register_parameter("weight", Parameter(torch.ones(*normalized_shape)) if create_scale else None)
         self.register_parameter("bias", Parameter(torch.zeros(*normalized_shape)) if create_offset else None)
 
@@ -38,7 +46,7 @@ class FusedLayerNorm(torch.nn.Module):
 
     def forward(self, input: torch.Tensor) -> torch.Tensor:
         p = self._parameters
-        return native.load().layer_norm(input, p["weight"], p["bias"], self.normalized_shape[0], self.eps)
+        return _layer_norm(input, p["weight"], p["bias"], self._width, self.eps)
 
 
 def LayerNorm(c_in: int, create_scale: bool = True, create_offset: bool = True, eps: float = 1e-5) -> torch.nn.Module:
