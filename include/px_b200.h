@@ -325,14 +325,17 @@ PX_API int32_t px_pair_bias_proj_folded(const void* z, int32_t z_dtype, const vo
  * Replaces AttentionPairBias.forward without s and the single transition, protenix/model/modules/transformer.py:40-254 and
  * protenix/model/modules/pairformer.py:181-224.  px_single_prepare lays the fp32 weights (nn.Linear order) out once in a
  * buffer of px_single_weights_bytes(); s and s_out [n][384] of s_dtype (may be the same), q_bias and LayerNorm vectors
- * fp32 [384], pair_bias fp32 [16][n][n]. */
+ * fp32 [384], pair_bias fp32 [16][n][n].  px_single_project does what needs s alone (q, k, v and gate, left in the workspace of
+ * px_single_workspace_bytes(n)), px_single_finish the rest from that workspace. */
 PX_API int64_t px_single_weights_bytes(void);
 PX_API int64_t px_single_workspace_bytes(int64_t n);
 PX_API int32_t px_single_prepare(const float* w_q, const float* w_k, const float* w_v, const float* w_g, const float* w_o,
                                  const float* w_a, const float* w_b, const float* w_out, void* prepared, void* stream);
-PX_API int32_t px_single_update(const void* s, void* s_out, int32_t s_dtype, const void* prepared, const float* ln_att_w,
-                                const float* ln_att_b, const float* q_bias, const float* ln_tr_w, const float* ln_tr_b,
-                                const float* pair_bias, void* workspace, int64_t workspace_bytes, int64_t n, float eps_att,
+PX_API int32_t px_single_project(const void* s, int32_t s_dtype, const void* prepared, const float* ln_att_w,
+                                 const float* ln_att_b, const float* q_bias, void* workspace, int64_t workspace_bytes, int64_t n,
+                                 float eps_att, void* stream);
+PX_API int32_t px_single_finish(const void* s, void* s_out, int32_t s_dtype, const void* prepared, const float* ln_tr_w,
+                                const float* ln_tr_b, const float* pair_bias, void* workspace, int64_t workspace_bytes, int64_t n,
                                 float eps_tr, void* stream);
 
 /* ---- Recycling update of the pair representation ------------------------------------------

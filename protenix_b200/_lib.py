@@ -72,7 +72,8 @@ SIGNATURES = {
     "px_single_weights_bytes": (I64, []),
     "px_single_workspace_bytes": (I64, [I64]),
     "px_single_prepare": (I32, [P, P, P, P, P, P, P, P, P, P]),
-    "px_single_update": (I32, [P, P, I32, P, P, P, P, P, P, P, P, I64, I64, F, F, P]),
+    "px_single_project": (I32, [P, I32, P, P, P, P, P, I64, I64, F, P]),
+    "px_single_finish": (I32, [P, P, I32, P, P, P, P, P, I64, I64, F, P]),
     "px_recycle_update": (I32, [P, P, P, I32, P, P, P, I64, F, P]),
     "px_scale_add_rowwise": (I32, [P, P, P, P, I64, I64, I64, I32, P]),
     "px_opm_outer": (I32, [P, P, P, I64, I64, I64, P]),

@@ -17,6 +17,8 @@
 // bound by the latency of one tile (load, 24 MMAs per 64 inputs, epilogue); hence narrow 64-column tiles, no
 // persistence, and the split contraction where it is 1536 long.  Whole branch on an idle GPU: 64 us at N = 128 and 76 us at
 // N = 384, where library GEMMs and the composed attention took 290 us; 0.36 ms against 0.76 at N = 1536.
+#include <initializer_list>
+
 #include "px_split.cuh"
 
 namespace px {
@@ -449,31 +451,52 @@ static bool launch_split_gemm(const bf16* a, const bf16* w, int64_t w_rows, int6
   return cudaLaunchKernelEx(&cfg, split_gemm_tc_kernel<kMode, T>, ma, mw, g) == cudaSuccess;
 }
 
+// The two parts of the branch: what needs s alone, and what needs the pair bias.
+struct SingleWs {
+  bf16* xp;        // [3][n][384]: LN(s), the attention's result, LN(s1)
+  float* qkvg;     // [n][1536]; later the hidden planes [3][n][1536]
+};
+static SingleWs single_ws(void* ws, int n) { return {(bf16*)ws, (float*)((unsigned char*)ws + (size_t)3 * n * kSc * 2)}; }
+
 template <typename T>
-static int32_t run_single(const void* s, void* s_out, const bf16* w, const float* const ln[4], const float* q_bias,
-                          const float* bias, unsigned char* ws, int n, float eps_att, float eps_tr, cudaStream_t st) {
-  bf16* xp = (bf16*)ws;                                    // [3][n][384]: LN(s), the attention's result, LN(s1)
-  float* qkvg = (float*)(ws + (size_t)3 * n * kSc * 2);    // [n][1536]; later the hidden planes [3][n][1536]
-  bf16* hp = (bf16*)qkvg;
-  const unsigned lnb = (unsigned)((n + 3) / 4);
+static int32_t single_project(const void* s, const bf16* w, const float* ln_w, const float* ln_b, const float* q_bias, void* ws, int n,
+                              float eps, cudaStream_t st) {
+  const SingleWs b = single_ws(ws, n);
   SgArgs g = {};
   g.rows = n;
-  if (!launch_pdl(split_rows_kernel<T>, dim3(lnb), 128, 0, st, (const T*)s, ln[0], ln[1], xp, n, eps_att)) return PX_ERR_LAUNCH;
-  g.bias = q_bias, g.out_f = qkvg, g.scale = 1.0f / sqrtf((float)kSd);
-  if (!launch_split_gemm<kSgQkvg, T>(xp, w + kSwQkvg, kSf, kSc, 1, g, st)) return PX_ERR_LAUNCH;
+  if (!launch_pdl(split_rows_kernel<T>, dim3((unsigned)((n + 3) / 4)), 128, 0, st, (const T*)s, ln_w, ln_b, b.xp, n, eps)) return PX_ERR_LAUNCH;
+  g.bias = q_bias, g.out_f = b.qkvg, g.scale = 1.0f / sqrtf((float)kSd);
+  return launch_split_gemm<kSgQkvg, T>(b.xp, w + kSwQkvg, kSf, kSc, 1, g, st) ? PX_OK : PX_ERR_LAUNCH;
+}
+
+template <typename T>
+static int32_t single_finish(const void* s, void* s_out, const bf16* w, const float* ln_w, const float* ln_b, const float* bias, void* ws,
+                             int n, float eps, cudaStream_t st) {
+  const SingleWs b = single_ws(ws, n);
+  SgArgs g = {};
+  g.rows = n;
   constexpr int sa_smem = kSd * kSaQ * 4 + kSaGroups * (int)sizeof(SaTile);
   static SmemLimit limit;
   if (!limit.set(single_attention_kernel, sa_smem) ||
-      !launch_pdl(single_attention_kernel, dim3((unsigned)((n + kSaQ - 1) / kSaQ), kSh), 128 * kSaGroups, sa_smem, st, qkvg, bias, xp, n))
+      !launch_pdl(single_attention_kernel, dim3((unsigned)((n + kSaQ - 1) / kSaQ), kSh), 128 * kSaGroups, sa_smem, st, b.qkvg, bias, b.xp, n))
     return PX_ERR_LAUNCH;
   g.res = s, g.out = s_out;
-  if (!launch_split_gemm<kSgRes, T>(xp, w + kSwO, kSc, kSc, 2, g, st)) return PX_ERR_LAUNCH;
-  if (!launch_pdl(split_rows_kernel<T>, dim3(lnb), 128, 0, st, (const T*)s_out, ln[2], ln[3], xp, n, eps_tr)) return PX_ERR_LAUNCH;
-  g.out_planes = hp;
-  if (!launch_split_gemm<kSgSwiglu, T>(xp, w + kSwAb, 2 * kSf, kSc, 1, g, st)) return PX_ERR_LAUNCH;
+  if (!launch_split_gemm<kSgRes, T>(b.xp, w + kSwO, kSc, kSc, 2, g, st)) return PX_ERR_LAUNCH;
+  if (!launch_pdl(split_rows_kernel<T>, dim3((unsigned)((n + 3) / 4)), 128, 0, st, (const T*)s_out, ln_w, ln_b, b.xp, n, eps))
+    return PX_ERR_LAUNCH;
+  g.out_planes = (bf16*)b.qkvg;
+  if (!launch_split_gemm<kSgSwiglu, T>(b.xp, w + kSwAb, 2 * kSf, kSc, 1, g, st)) return PX_ERR_LAUNCH;
   g.res = s_out, g.out = s_out;
-  if (!launch_split_gemm<kSgRes, T>(hp, w + kSwOut, kSc, kSf, kSgSplit, g, st)) return PX_ERR_LAUNCH;
-  return cudaGetLastError() == cudaSuccess ? PX_OK : PX_ERR_LAUNCH;
+  return launch_split_gemm<kSgRes, T>((bf16*)b.qkvg, w + kSwOut, kSc, kSf, kSgSplit, g, st) ? PX_OK : PX_ERR_LAUNCH;
+}
+
+static bool single_args_ok(int64_t n, std::initializer_list<const void*> pointers) {
+  uintptr_t bits = 0;
+  for (const void* p : pointers) {
+    if (!p) return false;
+    bits |= (uintptr_t)p;
+  }
+  return n > 0 && n <= 32768 && !(bits & 15);
 }
 
 }  // namespace px
@@ -500,24 +523,32 @@ extern "C" int32_t px_single_prepare(const float* w_q, const float* w_k, const f
   return cudaGetLastError() == cudaSuccess ? PX_OK : PX_ERR_LAUNCH;
 }
 
-extern "C" int32_t px_single_update(const void* s, void* s_out, int32_t s_dtype, const void* prepared, const float* ln_att_w,
-                                    const float* ln_att_b, const float* q_bias, const float* ln_tr_w, const float* ln_tr_b,
-                                    const float* pair_bias, void* workspace, int64_t workspace_bytes, int64_t n,
-                                    float eps_att, float eps_tr, void* stream) {
-  if (!s || !s_out || !prepared || !ln_att_w || !ln_att_b || !q_bias || !ln_tr_w || !ln_tr_b || !pair_bias || !workspace ||
-      n <= 0 || n > 32768)
-    return PX_ERR_BAD_ARG;
-  if (((uintptr_t)s | (uintptr_t)s_out | (uintptr_t)prepared | (uintptr_t)ln_att_w | (uintptr_t)ln_att_b | (uintptr_t)ln_tr_w |
-       (uintptr_t)ln_tr_b | (uintptr_t)pair_bias | (uintptr_t)workspace) & 15)
-    return PX_ERR_BAD_ARG;
+extern "C" int32_t px_single_project(const void* s, int32_t s_dtype, const void* prepared, const float* ln_att_w,
+                                     const float* ln_att_b, const float* q_bias, void* workspace, int64_t workspace_bytes, int64_t n,
+                                     float eps_att, void* stream) {
+  if (!single_args_ok(n, {s, prepared, ln_att_w, ln_att_b, q_bias, workspace})) return PX_ERR_BAD_ARG;
   if (workspace_bytes < px_single_workspace_bytes(n)) return PX_ERR_WORKSPACE;
-  const float* const ln[4] = {ln_att_w, ln_att_b, ln_tr_w, ln_tr_b};
   cudaStream_t st = (cudaStream_t)stream;
-  unsigned char* ws = (unsigned char*)workspace;
+  const bf16* w = (const bf16*)prepared;
   switch (s_dtype) {
-    case PX_F32: return run_single<float>(s, s_out, (const bf16*)prepared, ln, q_bias, pair_bias, ws, (int)n, eps_att, eps_tr, st);
-    case PX_BF16: return run_single<bf16>(s, s_out, (const bf16*)prepared, ln, q_bias, pair_bias, ws, (int)n, eps_att, eps_tr, st);
-    case PX_F16: return run_single<__half>(s, s_out, (const bf16*)prepared, ln, q_bias, pair_bias, ws, (int)n, eps_att, eps_tr, st);
+    case PX_F32: return single_project<float>(s, w, ln_att_w, ln_att_b, q_bias, workspace, (int)n, eps_att, st);
+    case PX_BF16: return single_project<bf16>(s, w, ln_att_w, ln_att_b, q_bias, workspace, (int)n, eps_att, st);
+    case PX_F16: return single_project<__half>(s, w, ln_att_w, ln_att_b, q_bias, workspace, (int)n, eps_att, st);
+    default: return PX_ERR_UNSUPPORTED;
+  }
+}
+
+extern "C" int32_t px_single_finish(const void* s, void* s_out, int32_t s_dtype, const void* prepared, const float* ln_tr_w,
+                                    const float* ln_tr_b, const float* pair_bias, void* workspace, int64_t workspace_bytes, int64_t n,
+                                    float eps_tr, void* stream) {
+  if (!single_args_ok(n, {s, s_out, prepared, ln_tr_w, ln_tr_b, pair_bias, workspace})) return PX_ERR_BAD_ARG;
+  if (workspace_bytes < px_single_workspace_bytes(n)) return PX_ERR_WORKSPACE;
+  cudaStream_t st = (cudaStream_t)stream;
+  const bf16* w = (const bf16*)prepared;
+  switch (s_dtype) {
+    case PX_F32: return single_finish<float>(s, s_out, w, ln_tr_w, ln_tr_b, pair_bias, workspace, (int)n, eps_tr, st);
+    case PX_BF16: return single_finish<bf16>(s, s_out, w, ln_tr_w, ln_tr_b, pair_bias, workspace, (int)n, eps_tr, st);
+    case PX_F16: return single_finish<__half>(s, s_out, w, ln_tr_w, ln_tr_b, pair_bias, workspace, (int)n, eps_tr, st);
     default: return PX_ERR_UNSUPPORTED;
   }
 }

@@ -54,8 +54,8 @@ constexpr int64_t kCz = 128, kCs = 384, kHeadsSingle = 16, kHeads = 4, kHeadDim 
   X(px_triatt_in_proj_folded) X(px_triatt_flash) X(px_triatt_flash_scratch_bytes) X(px_triatt_out_folded_bytes)          \
   X(px_triatt_out_fold) X(px_triatt_out_folded) X(px_triatt_workspace_bytes) X(px_transition)                            \
   X(px_pair_bias_folded_bytes) X(px_pair_bias_fold) X(px_pair_bias_proj_folded) X(px_single_weights_bytes)               \
-  X(px_single_workspace_bytes) X(px_single_prepare) X(px_single_update) X(px_opm_outer) X(px_opm_out)                    \
-  X(px_msa_opm_prep) X(px_msa_values) X(px_msa_gate_out) X(px_msa_transition_weights_bytes)                              \
+  X(px_single_workspace_bytes) X(px_single_prepare) X(px_single_project) X(px_single_finish) X(px_opm_outer)             \
+  X(px_opm_out) X(px_msa_opm_prep) X(px_msa_values) X(px_msa_gate_out) X(px_msa_transition_weights_bytes)                              \
   X(px_msa_transition_prepare) X(px_msa_transition)
 struct Abi {
 #define X(f) decltype(&::f) f = nullptr;
@@ -346,37 +346,40 @@ struct PairCall {
   unsigned char* ws;             // shared by the updates, which run one after the other
   cudaStream_t st;
 };
+// as laid out by tri_mul and tri_att, and behind that the standardised rows
 int64_t pair_workspace(int64_t n) { return std::max(abi.px_trimul_workspace_bytes(n), abi.px_triatt_workspace_bytes(n)); }
 
-void standardise(const PairCall& c, const void* z, void* zn, float eps) {
-  launch("px_standardise_rows", c.st, [&] { return abi.px_standardise_rows((const float*)z, (px_f16*)zn, c.n * c.n, eps, c.st); });
-}
+// The standardised copy of the rows of z that the updates of an fp32 z read: where it lies, and whether it holds the current z,
+// made with which eps.
+struct Rows {
+  px_f16* zn = nullptr;
+  bool valid = false;
+  float eps = 0.f;
+  void need(const PairCall& c, const void* z, float want) {
+    if (valid && eps == want) return;
+    launch("px_standardise_rows", c.st, [&] { return abi.px_standardise_rows((const float*)z, zn, c.n * c.n, want, c.st); });
+    valid = true, eps = want;
+  }
+};
 
-// zn: the standardised copy of an fp32 z_in, if the caller has it
-void tri_mul(const PairCall& c, const Prepared& pr, const void* z_in, void* z_out, bool incoming, bool add, const void* zn) {
+void tri_mul(const PairCall& c, const Prepared& pr, const void* z_in, void* z_out, bool incoming, bool add, Rows& rows) {
   const auto& p = pr.p[c.zf];
   const float eps = pr.scalars[0];
   const int64_t n = c.n, ld = abi.px_ld(n), per = kCz * n * ld * 2;
   px_f16 *a = (px_f16*)c.ws, *b = (px_f16*)(c.ws + per), *x = (px_f16*)(c.ws + 2 * per);
-  const void* rows = z_in;
-  int rows_dt = c.dt;
-  if (c.dt == PX_F32) {          // the projection and the output stage normalise the same z: one standardised copy
-    if (!zn) {
-      zn = c.ws + 3 * per;
-      standardise(c, z_in, (void*)zn, eps);
-    }
-    rows = zn, rows_dt = PX_F16;
-  }
+  const bool fp32 = c.dt == PX_F32;      // the projection and the output stage normalise the same z: one standardised copy
+  if (fp32) rows.need(c, z_in, eps);
   launch("px_trimul_in_proj", c.st, [&] {
-    return abi.px_trimul_in_proj_folded(rows, rows_dt, c.mask, p[0], a, b, n, n, ld, incoming, eps, c.st);
+    return abi.px_trimul_in_proj_folded(fp32 ? rows.zn : z_in, fp32 ? PX_F16 : c.dt, c.mask, p[0], a, b, n, n, ld, incoming, eps, c.st);
   });
   launch("px_trimul_contract", c.st, [&] { return abi.px_trimul_contract(a, b, x, kCz, n, ld, c.st); });
+  rows.valid = false;
   launch("px_trimul_out", c.st, [&] {
-    return abi.px_trimul_out_folded(x, z_in, (const px_f16*)zn, z_out, c.dt, p[1], n, n, ld, add, eps, c.st);
+    return abi.px_trimul_out_folded(x, z_in, rows.zn, z_out, c.dt, p[1], n, n, ld, add, eps, c.st);
   });
 }
 
-void tri_att(const PairCall& c, const Prepared& pr, const void* z_in, void* z_out, bool ending, bool add) {
+void tri_att(const PairCall& c, const Prepared& pr, const void* z_in, void* z_out, bool ending, bool add, Rows& rows) {
   const auto& p = pr.p[c.zf];
   const float eps = pr.scalars[0], inf = pr.scalars[1];
   const int64_t n = c.n, ldm = abi.px_ld_mask(n);
@@ -385,22 +388,18 @@ void tri_att(const PairCall& c, const Prepared& pr, const void* z_in, void* z_ou
   unsigned char* bias = (unsigned char*)o + al(n * n * kCz * 2);
   unsigned char* mbias = bias + al(kHeads * n * ldm * 4);
   unsigned char* flags = mbias + al(n * ldm * 4);
-  const void *zn = nullptr, *rows = z_in;
-  int rows_dt = c.dt;
-  if (c.dt == PX_F32) {
-    zn = flags + al(abi.px_triatt_flash_scratch_bytes(n, n));
-    standardise(c, z_in, (void*)zn, eps);
-    rows = zn, rows_dt = PX_F16;
-  }
+  const bool fp32 = c.dt == PX_F32;
+  if (fp32) rows.need(c, z_in, eps);
   launch("px_triatt_in_proj", c.st, [&] {
-    return abi.px_triatt_in_proj_folded(rows, rows_dt, c.mask, p[0], q, k, v, (float*)bias, (float*)mbias, n, n, ldm, ending, eps, inf,
-                                        c.st);
+    return abi.px_triatt_in_proj_folded(fp32 ? rows.zn : z_in, fp32 ? PX_F16 : c.dt, c.mask, p[0], q, k, v, (float*)bias, (float*)mbias, n,
+                                        n, ldm, ending, eps, inf, c.st);
   });
   launch("px_triatt_flash", c.st, [&] {
     return abi.px_triatt_flash(q, k, v, (const float*)bias, (const float*)mbias, o, flags, n, n, ldm, c.st);
   });
+  rows.valid = false;
   launch("px_triatt_out", c.st, [&] {
-    return abi.px_triatt_out_folded(o, z_in, (const px_f16*)zn, z_out, c.dt, p[1], n, n, ending, add, eps, c.st);
+    return abi.px_triatt_out_folded(o, z_in, rows.zn, z_out, c.dt, p[1], n, n, ending, add, eps, c.st);
   });
 }
 
@@ -410,6 +409,13 @@ void transition_rows(cudaStream_t st, const Prepared& pr, int zf, int dt, const 
     return abi.px_transition(x_in, x_out, dt, (const float*)p[0], (const float*)p[1], (const px_f16*)p[2], (const px_f16*)p[3],
                              (const px_f16*)p[4], rows, add, pr.scalars[0], st);
   });
+}
+
+// The standardised rows at the end of a workspace of the size that the library asks for.
+Rows own_rows(const PairCall& c, const Tensor& ws) {
+  Rows r;
+  if (c.dt == PX_F32) r.zn = (px_f16*)(c.ws + ws.numel() - al(c.n * c.n * kCz * 2));
+  return r;
 }
 
 Tensor tri_mul_forward(Params& params, const Tensor& z, const OptTensor& mask, bool incoming, bool inplace_add) {
@@ -423,7 +429,8 @@ Tensor tri_mul_forward(Params& params, const Tensor& z, const OptTensor& mask, b
   const Tensor out = inplace_add && zc.data_ptr() == z.data_ptr() ? zc : at::empty_like(zc);
   const Tensor ws = bytes_like(zc, abi.px_trimul_workspace_bytes(zc.size(0)));
   const PairCall c{zc.size(0), zformat(zc), dtype_code(zc, "z"), fptr(m), (unsigned char*)ws.data_ptr(), at::cuda::getCurrentCUDAStream()};
-  tri_mul(c, *pr, zc.data_ptr(), out.data_ptr(), incoming, inplace_add, nullptr);
+  Rows rows = own_rows(c, ws);
+  tri_mul(c, *pr, zc.data_ptr(), out.data_ptr(), incoming, inplace_add, rows);
   return batch ? out.unsqueeze(0) : out;
 }
 
@@ -438,7 +445,8 @@ Tensor tri_att_forward(Params& params, const Tensor& z, const OptTensor& mask, b
   const Tensor out = at::empty_like(zc);
   const Tensor ws = bytes_like(zc, abi.px_triatt_workspace_bytes(zc.size(0)));
   const PairCall c{zc.size(0), zformat(zc), dtype_code(zc, "z"), fptr(m), (unsigned char*)ws.data_ptr(), at::cuda::getCurrentCUDAStream()};
-  tri_att(c, *pr, zc.data_ptr(), out.data_ptr(), ending, false);
+  Rows rows = own_rows(c, ws);
+  tri_att(c, *pr, zc.data_ptr(), out.data_ptr(), ending, false, rows);
   return batch ? out.unsqueeze(0) : out;
 }
 
@@ -469,14 +477,20 @@ struct BlockReady {
   Ready mul_out, mul_in, att_start, att_end, transition, pair_bias, single;
 };
 
-// s_in -> s_out given the block's pair bias
-void single_update(cudaStream_t st, const Prepared& pr, int zf, const Tensor& s_in, const Tensor& s_out, const Tensor& bias,
+// The single branch: what needs s alone, then s_in -> s_out given the block's pair bias.
+void single_project(cudaStream_t st, const Prepared& pr, int zf, const Tensor& s, const Tensor& ws) {
+  const auto& p = pr.p[zf];
+  launch("px_single_update", st, [&] {
+    return abi.px_single_project(s.data_ptr(), dtype_code(s, "s"), p.back(), (const float*)p[0], (const float*)p[1], (const float*)p[2],
+                                 ws.data_ptr(), ws.numel(), s.numel() / kCs, pr.scalars[0], st);
+  });
+}
+void single_finish(cudaStream_t st, const Prepared& pr, int zf, const Tensor& s_in, const Tensor& s_out, const Tensor& bias,
                    const Tensor& ws) {
   const auto& p = pr.p[zf];
   launch("px_single_update", st, [&] {
-    return abi.px_single_update(s_in.data_ptr(), s_out.data_ptr(), dtype_code(s_in, "s"), p.back(), (const float*)p[0],
-                                (const float*)p[1], (const float*)p[2], (const float*)p[3], (const float*)p[4],
-                                (const float*)bias.data_ptr(), ws.data_ptr(), ws.numel(), s_in.numel() / kCs, pr.scalars[0],
+    return abi.px_single_finish(s_in.data_ptr(), s_out.data_ptr(), dtype_code(s_in, "s"), p.back(), (const float*)p[3],
+                                (const float*)p[4], (const float*)bias.data_ptr(), ws.data_ptr(), ws.numel(), s_in.numel() / kCs,
                                 pr.scalars[1], st);
   });
 }
@@ -491,9 +505,14 @@ c10::cuda::CUDAStream side_stream(c10::DeviceIndex dev) {
 }
 
 // The blocks one after the other.  The pair path never reads s, and the single branch takes nothing from z but the pair
-// bias of the block's final z: the single branch of block b runs on a side stream beside the pair path of block b + 1
-// (two pair-bias buffers take turns).  A single block has nothing to run beside and stays on the caller's stream.
+// bias of the block's final z: the branch of a block can run on a side stream beside the pair path of the next block (two
+// pair-bias buffers take turns), and its projections, which need no bias, already beside that of its own block.  What runs
+// beside takes SMs from persistent kernels whose tiles are dealt out in advance, so it pays only where they leave some or the
+// branch is a large part of a block.  Four blocks, us per block, in order | beside, projections with the rest | beside,
+// projections first: N = 128: 225 | 189 | 186, 200: 405 | 377 | 372, 300: 733 | 695 | 704, 437: 1364 | 1324 | 1332,
+// 640: 2747 | 2742 | 2727, 1024: 8140 | 8195 | 8181; one block alone: 224 | - | 216 at N = 128, no difference from N = 200 on.
 // Everything is allocated on the caller's stream, which waits for the side stream before this returns.
+constexpr int64_t kBesideBelow = 768, kProjectFirstUpTo = 256;
 std::tuple<OptTensor, Tensor> stack_forward(const std::vector<std::shared_ptr<Block>>& blocks, const OptTensor& s_in,
                                             const Tensor& z, const OptTensor& mask, bool inplace) {
   bool batch;
@@ -530,13 +549,14 @@ std::tuple<OptTensor, Tensor> stack_forward(const std::vector<std::shared_ptr<Bl
   const auto main = at::cuda::getCurrentCUDAStream();
   const PairCall c{n, zf, dtype_code(zc, "z"), fptr(m), (unsigned char*)ws.data_ptr(), main};
   const bool fp32 = c.dt == PX_F32;
-  const auto side = singles && blocks.size() > 1 ? side_stream(zc.device().index()) : main;
-  const bool aside = side != main;
-  Tensor zn, bias[2], sb[2], sws;
-  at::cuda::CUDAEvent bias_ready[2], side_done[2];
+  Rows rows = own_rows(c, ws);
+  const bool first = n <= kProjectFirstUpTo;       // projections of s beside the pair path of their own block
+  const bool aside = singles && (blocks.size() > 1 ? n < kBesideBelow : first);
+  const auto side = aside ? side_stream(zc.device().index()) : main;
+  Tensor bias[2], sb[2], sws;
+  at::cuda::CUDAEvent bias_ready[2], side_done[2];   // bias_ready: what the rest of the branch waits for on its stream
   if (singles) {
-    if (fp32) zn = at::empty(zc.sizes(), zc.options().dtype(at::kHalf));
-    for (int i = 0; i < (aside ? 2 : 1); ++i) bias[i] = at::empty({kHeadsSingle, n, n}, zc.options().dtype(at::kFloat));
+    for (int i = 0; i < (blocks.size() > 1 ? 2 : 1); ++i) bias[i] = at::empty({kHeadsSingle, n, n}, zc.options().dtype(at::kFloat));
     for (int i = 0; i < (blocks.size() > 1 ? 2 : 1); ++i) sb[i] = at::empty_like(s);
     sws = bytes_like(zc, abi.px_single_workspace_bytes(n));
     if (aside) {
@@ -554,39 +574,38 @@ std::tuple<OptTensor, Tensor> stack_forward(const std::vector<std::shared_ptr<Bl
       e.block(main);
     }
   } join{aside, side, main};
-  const void* zn_valid = nullptr;   // zn holds the standardised rows of the current z, made with zn_eps
-  float zn_eps = 0.f;
-  int64_t k = 0;                    // single updates so far
+  int64_t k = 0, last = -1;         // single updates so far; the last block that has one
+  for (size_t b = 0; b < ready.size(); ++b)
+    if (ready[b].single) last = b;
   for (size_t b = 0; b < ready.size(); ++b) {
     const BlockReady& r = ready[b];
-    const void* first_zn = zn_valid && zn_eps == r.mul_out->scalars[0] ? zn_valid : nullptr;
-    zn_valid = nullptr;
-    tri_mul(c, *r.mul_out, b == 0 ? zi.data_ptr() : zc.data_ptr(), zc.data_ptr(), false, true, first_zn);
-    tri_mul(c, *r.mul_in, zc.data_ptr(), zc.data_ptr(), true, true, nullptr);
-    tri_att(c, *r.att_start, zc.data_ptr(), zc.data_ptr(), false, true);
-    tri_att(c, *r.att_end, zc.data_ptr(), zc.data_ptr(), true, true);
-    transition_rows(c.st, *r.transition, zf, c.dt, zc.data_ptr(), zc.data_ptr(), n * n, true);
+    if (r.single && first) single_project(side, *r.single, zf, s, sws);
+    void* const z = zc.data_ptr();
+    tri_mul(c, *r.mul_out, b == 0 ? zi.data_ptr() : z, z, false, true, rows);
+    tri_mul(c, *r.mul_in, z, z, true, true, rows);
+    tri_att(c, *r.att_start, z, z, false, true, rows);
+    tri_att(c, *r.att_end, z, z, true, true, rows);
+    rows.valid = false;
+    transition_rows(c.st, *r.transition, zf, c.dt, z, z, n * n, true);
     if (!r.single) continue;
-    const int turn = aside ? k & 1 : 0;
-    const void* rows = zc.data_ptr();
-    if (fp32) {                     // the copy made for the pair bias also serves the next block's first update
-      zn_eps = r.pair_bias->scalars[0];
-      standardise(c, zc.data_ptr(), zn.data_ptr(), zn_eps);
-      rows = zn_valid = zn.data_ptr();
-    }
+    const int turn = k & 1;
+    // the copy for the pair bias also serves the next block's first update
+    if (fp32) rows.need(c, z, r.pair_bias->scalars[0]);
     if (aside && k >= 2) side_done[turn].block(main);       // the single branch two blocks ago has read this buffer
     const auto& p = r.pair_bias->p[zf];
     launch("px_pair_bias_proj", c.st, [&] {
-      return abi.px_pair_bias_proj_folded(rows, fp32 ? PX_F16 : PX_BF16, p[0], (float*)bias[turn].data_ptr(), n * n, kHeadsSingle,
+      return abi.px_pair_bias_proj_folded(fp32 ? rows.zn : z, fp32 ? PX_F16 : PX_BF16, p[0], (float*)bias[turn].data_ptr(), n * n, kHeadsSingle,
                                           r.pair_bias->scalars[0], c.st);
     });
+    const auto rest = (int64_t)b == last ? main : side;     // the last block's rest has nothing to run beside
     if (aside) {
-      bias_ready[turn].record(main);
-      bias_ready[turn].block(side);
+      bias_ready[turn].record(rest == main ? side : main);
+      bias_ready[turn].block(rest);
     }
-    single_update(side, *r.single, zf, s, sb[k & 1], bias[turn], sws);
-    s = sb[k & 1];
-    if (aside) side_done[turn].record(side);
+    if (!first) single_project(rest, *r.single, zf, s, sws);
+    single_finish(rest, *r.single, zf, s, sb[turn], bias[turn], sws);
+    if (aside) side_done[turn].record(rest);
+    s = sb[turn];
     ++k;
   }
   return {s.defined() ? OptTensor(s) : OptTensor(), batch ? zc.unsqueeze(0) : zc};

@@ -20,7 +20,7 @@ C_Z = 128
 X_SCALE = 1.0 / 64      # PX_TRIMUL_X_SCALE: the contraction stores x scaled so that it stays inside the fp16 range
 N_HEAD_PAIR = 4
 D_HEAD_PAIR = 32
-C_S, N_HEAD_SINGLE = 384, 16     # the single-representation branch px_single_update is built for
+C_S, N_HEAD_SINGLE = 384, 16     # the single-representation branch that the kernels are built for
 
 
 def _ptr(t: Optional[torch.Tensor]) -> Optional[int]:

@@ -74,7 +74,7 @@ class PairformerBlock(nn.Module):
         return native.load().Block(parts)
 
     def _single_kernel(self) -> bool:
-        """Whether the single branch has the dimensions px_single_update is built for."""
+        """Whether the single branch has the dimensions its kernels are built for."""
         return self.c_s == ops.C_S and self.n_heads == ops.N_HEAD_SINGLE
 
     def single_path(self, s: torch.Tensor, bias: torch.Tensor) -> torch.Tensor:

@@ -1,4 +1,4 @@
-"""The single-representation branch (px_single_update) against the torch composition of the same modules in fp64, and no
+"""The single-representation branch (px_single_project, px_single_finish) against the torch composition of the same modules in fp64, and no
 further from it than the composition in fp32."""
 import pytest
 import torch
