@@ -20,7 +20,8 @@ constexpr int kMtC = 64, kMtHid = 256, kMtChunks = kMtHid / 64;
 constexpr int kMtABytes = 3 * 128 * 128;       // [3 planes][128 rows][64 k]
 constexpr int kMtW1Bytes = 3 * 128 * 128;      // [3][a 64 | b 64 rows][64 k]
 constexpr int kMtW2Bytes = 3 * 64 * 128;       // [3][64 outputs][64 hidden]
-constexpr int kMtWarps = 20, kMtThreads = 32 * kMtWarps;
+constexpr int kMtGate = 16;                    // SwiGLU warps
+constexpr int kMtWarps = kMtGate + 12, kMtThreads = 32 * kMtWarps;
 
 struct MtBars {
   uint64_t a_full[2], a_free[2], w1_full[2], w1_empty[2], w2_full, w2_empty, h_full[2], h_free[2], p_ready[2], out_full[2], out_free[2];
@@ -57,7 +58,7 @@ msa_transition_tc_kernel(const __grid_constant__ CUtensorMap map_w1, const __gri
       mbar_init(&bars.w1_empty[b], 1);
       mbar_init(&bars.h_full[b], 1);
       mbar_init(&bars.h_free[b], 1);
-      mbar_init(&bars.p_ready[b], 8);
+      mbar_init(&bars.p_ready[b], kMtGate);
       mbar_init(&bars.out_full[b], 1);
       mbar_init(&bars.out_free[b], 4);
     }
@@ -65,19 +66,19 @@ msa_transition_tc_kernel(const __grid_constant__ CUtensorMap map_w1, const __gri
     mbar_init(&bars.w2_empty, 1);
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
-  if (warp == 16) {
+  if (warp == kMtGate + 8) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(&bars.tmem_base)),
                  "r"(512u)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
   }
-  if (!cta_ready(skip, warp == 16, bars.tmem_base, 512u)) return;
+  if (!cta_ready(skip, warp == kMtGate + 8, bars.tmem_base, 512u)) return;
   const uint32_t tmem_base = bars.tmem_base;
 
-  if (warp >= 16) {
+  if (warp >= kMtGate + 8) {
     if (lane != 0) {
       // nothing: the control threads are lane 0 of their warps
-    } else if (warp == 16) {
+    } else if (warp == kMtGate + 8) {
       int j = 0;
       bool ok = true;
       for (int tile = first_tile; tile < n_tiles && ok; tile += tile_step) {
@@ -88,7 +89,7 @@ msa_transition_tc_kernel(const __grid_constant__ CUtensorMap map_w1, const __gri
           tma_load_3d(smem_u32(sm + MtLayout::w1 + (j & 1) * kMtW1Bytes), &map_w1, &bars.w1_full[j & 1], 0, 128 * c, 0);
         }
       }
-    } else if (warp == 19) {
+    } else if (warp == kMtGate + 11) {
       int j = 0;
       bool ok = true;
       for (int tile = first_tile; tile < n_tiles && ok; tile += tile_step) {
@@ -99,7 +100,7 @@ msa_transition_tc_kernel(const __grid_constant__ CUtensorMap map_w1, const __gri
           tma_load_3d(smem_u32(sm + MtLayout::w2), &map_w2, &bars.w2_full, 64 * c, 0, 0);
         }
       }
-    } else if (warp == 17) {
+    } else if (warp == kMtGate + 9) {
       // ---------------------------------------------------------------- first product: H = A [W_a; W_b]_c^T
       constexpr uint32_t idesc = umma_idesc_bf16(128, 128);
       int j = 0, k = 0;
@@ -153,9 +154,9 @@ msa_transition_tc_kernel(const __grid_constant__ CUtensorMap map_w1, const __gri
         if (ok) umma_commit(&bars.out_full[ob]);
       }
     }
-  } else if (warp >= 12) {
+  } else if (warp >= kMtGate + 4) {
     // ------------------------------------------------------------------ output rows: residual + store
-    const int qw = warp - 12;
+    const int qw = warp - kMtGate - 4;
     const uint32_t lane_addr = tmem_base + ((uint32_t)(32 * qw) << 16);
     unsigned char* stg = sm + MtLayout::stg + qw * 2048;     // rows of 64 bytes, 16-byte pieces swizzled by row pair
     const int rsub = lane >> 2, piece = lane & 3;
@@ -204,27 +205,33 @@ msa_transition_tc_kernel(const __grid_constant__ CUtensorMap map_w1, const __gri
         __syncwarp();
       }
     }
-  } else if (warp >= 8) {
+  } else if (warp >= kMtGate) {
     // ------------------------------------------------------------------ LayerNorm -> split, swizzled A operand
-    const int qw = warp - 8, li = lane & 15, sub = lane >> 4;
+    const int qw = warp - kMtGate, li = lane & 15, sub = lane >> 4;
     const float4 g4 = ln_w ? *reinterpret_cast<const float4*>(ln_w + 4 * li) : make_float4(1.f, 1.f, 1.f, 1.f);
     const float4 b4 = ln_b ? *reinterpret_cast<const float4*>(ln_b + 4 * li) : make_float4(0.f, 0.f, 0.f, 0.f);
     int k = 0;
     for (int tile = first_tile; tile < n_tiles; tile += tile_step, ++k) {
       const int ab = k & 1;
       const long long row0 = (long long)tile * 128 + 32 * qw;
-      float4 v[16];                                          // the warp's 32 rows, two at a time
+      float4 v[8];                                           // half of the warp's 32 rows, two rows a load
+      auto request = [&](int j1) {
 #pragma unroll
-      for (int j = 0; j < 16; ++j) {
-        const long long row = row0 + 2 * j + sub;
-        v[j] = row < rows ? *reinterpret_cast<const float4*>(m + (size_t)row * kMtC + 4 * li) : make_float4(0.f, 0.f, 0.f, 0.f);
-      }
+        for (int j = 0; j < 8; ++j) {
+          const long long row = row0 + 2 * (j1 + j) + sub;
+          v[j] = row < rows ? *reinterpret_cast<const float4*>(m + (size_t)row * kMtC + 4 * li) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+      };
+      request(0);
       bool ok = mbar_wait(&bars.a_free[ab], ((k >> 1) & 1) ^ 1, 16u);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
       unsigned char* sa = sm + MtLayout::a + ab * kMtABytes;
+#pragma unroll 1
+      for (int j1 = 0; j1 < 16; j1 += 8) {
+        if (j1) request(j1);
 #pragma unroll
-      for (int j0 = 0; j0 < 16; j0 += 4) {
+      for (int j0 = 0; j0 < 8; j0 += 4) {
         float s[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) s[j] = (v[j0 + j].x + v[j0 + j].y) + (v[j0 + j].z + v[j0 + j].w);
@@ -247,7 +254,7 @@ msa_transition_tc_kernel(const __grid_constant__ CUtensorMap map_w1, const __gri
         for (int j = 0; j < 4; ++j) {
           const float4 x = v[j0 + j];
           const float rstd = rsqrtf(s[j] * (1.0f / kMtC) + eps);
-          const int r = 32 * qw + 2 * (j0 + j) + sub;
+          const int r = 32 * qw + 2 * (j1 + j0 + j) + sub;
           uint32_t lo[3], hi[3];
           split3x2(fmaf(x.x * rstd, g4.x, b4.x), fmaf(x.y * rstd, g4.y, b4.y), lo);
           split3x2(fmaf(x.z * rstd, g4.z, b4.z), fmaf(x.w * rstd, g4.w, b4.w), hi);
@@ -256,13 +263,14 @@ msa_transition_tc_kernel(const __grid_constant__ CUtensorMap map_w1, const __gri
             *reinterpret_cast<uint2*>(sa + p * (128 * 128) + r * 128 + (((li >> 1) ^ (r & 7)) << 4) + (li & 1) * 8) = make_uint2(lo[p], hi[p]);
         }
       }
+      }
       asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
       __syncwarp();
       if (lane == 0) mbar_arrive(&bars.a_full[ab]);
     }
   } else {
     // ------------------------------------------------------------------ SwiGLU in registers
-    const int half = warp >> 2, qw = warp & 3;
+    const int part = warp >> 2, qw = warp & 3;               // 16 of the chunk's 64 columns, lane quarter
     const uint32_t lane_addr = tmem_base + ((uint32_t)(32 * qw) << 16);
     int j = 0;
     bool ok = true;
@@ -271,29 +279,25 @@ msa_transition_tc_kernel(const __grid_constant__ CUtensorMap map_w1, const __gri
         const int hb = j & 1;
         const uint32_t t_h = lane_addr + 128 * hb;
         ok = mbar_wait(&bars.h_full[hb], (j >> 1) & 1, 64u);
-        ok = named_barrier_all(2, 256, ok);                  // all eight warps go on, or none
+        ok = named_barrier_all(2, 32 * kMtGate, ok);         // all of these warps go on, or none
         if (!ok) break;
         tc_fence_after();
-        uint32_t w[3][16];
+        uint32_t w[3][8], a[16], b[16];
+        tmem_ld16(t_h + 16 * part, a);
+        tmem_ld16(t_h + 64 + 16 * part, b);
+        tmem_wait_ld();
 #pragma unroll
-        for (int hh = 0; hh < 2; ++hh) {
-          uint32_t a[16], b[16];
-          tmem_ld16(t_h + 32 * half + 16 * hh, a);
-          tmem_ld16(t_h + 64 + 32 * half + 16 * hh, b);
-          tmem_wait_ld();
-#pragma unroll
-          for (int e = 0; e < 8; ++e) {
-            const float a0 = __uint_as_float(a[2 * e]), a1 = __uint_as_float(a[2 * e + 1]);
-            const float h0 = a0 / (1.0f + expf(-a0)) * __uint_as_float(b[2 * e]);
-            const float h1 = a1 / (1.0f + expf(-a1)) * __uint_as_float(b[2 * e + 1]);
-            uint32_t p[3];
-            split3x2(h0, h1, p);
-            w[0][8 * hh + e] = p[0], w[1][8 * hh + e] = p[1], w[2][8 * hh + e] = p[2];
-          }
+        for (int e = 0; e < 8; ++e) {
+          const float a0 = __uint_as_float(a[2 * e]), a1 = __uint_as_float(a[2 * e + 1]);
+          const float h0 = a0 / (1.0f + expf(-a0)) * __uint_as_float(b[2 * e]);
+          const float h1 = a1 / (1.0f + expf(-a1)) * __uint_as_float(b[2 * e + 1]);
+          uint32_t p[3];
+          split3x2(h0, h1, p);
+          w[0][e] = p[0], w[1][e] = p[1], w[2][e] = p[2];
         }
-        named_barrier(2, 256);                               // everybody has read H: h goes over its first 96 columns
+        named_barrier(2, 32 * kMtGate);                      // everybody has read H: h goes over its first 96 columns
 #pragma unroll
-        for (int p = 0; p < 3; ++p) tmem_st16(t_h + 32 * p + 16 * half, w[p]);
+        for (int p = 0; p < 3; ++p) tmem_st8(t_h + 32 * p + 8 * part, w[p]);
         tmem_wait_st();
         tc_fence_before();
         __syncwarp();
@@ -304,7 +308,7 @@ msa_transition_tc_kernel(const __grid_constant__ CUtensorMap map_w1, const __gri
 
   tc_fence_before();
   cta_teardown_sync();
-  if (warp == 16) {
+  if (warp == kMtGate + 8) {
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem_base), "r"(512u) : "memory");
   }

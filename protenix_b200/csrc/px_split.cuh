@@ -12,13 +12,14 @@ __device__ __forceinline__ void split3(float x, bf16 (&b)[3]) {
   b[1] = __float2bfloat16_rn(r);
   b[2] = __float2bfloat16_rn(r - __bfloat162float(b[1]));
 }
+// Two values at a time, one conversion instruction a plane for both: w[p] = plane p of (x, y).
 __device__ __forceinline__ void split3x2(float x, float y, uint32_t (&w)[3]) {
-  bf16 a[3], b[3];
-  split3(x, a);
-  split3(y, b);
-#pragma unroll
-  for (int p = 0; p < 3; ++p)
-    w[p] = (uint32_t)__bfloat16_as_ushort(a[p]) | ((uint32_t)__bfloat16_as_ushort(b[p]) << 16);
+  w[0] = pack_bf16x2(x, y);
+  const float2 a = unpack_bf16x2(w[0]);
+  x -= a.x, y -= a.y;
+  w[1] = pack_bf16x2(x, y);
+  const float2 b = unpack_bf16x2(w[1]);
+  w[2] = pack_bf16x2(x - b.x, y - b.y);
 }
 
 template <typename T>
