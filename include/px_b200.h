@@ -154,7 +154,8 @@ PX_API int32_t px_trimul_contract(const px_f16* a, const px_f16* b, px_f16* x, i
 #define PX_FAMILY_OPM 11
 #define PX_FAMILY_SINGLE 12
 #define PX_FAMILY_MSA_TRANSITION 13
-#define PX_N_FAMILIES 14
+#define PX_FAMILY_MSA_AVERAGE 14
+#define PX_N_FAMILIES 15
 PX_API int32_t px_device_error_flags(uint32_t* flags);
 PX_API int32_t px_device_error_detail(uint32_t* flags, uint32_t* detail);
 /* Limit of every bounded wait on the current device, in SM clock cycles (default 2^28, about 0.14 s); cycles <= 0
@@ -266,8 +267,10 @@ PX_API int32_t px_pair_bias_proj(const void* z, int32_t z_dtype, const float* ln
  * Row-wise steps on m [S][N][64] fp32, LayerNorm vectors fp32 [64] or NULL, weights fp32 in nn.Linear order.
  * px_msa_opm_prep: a_t, b_t [32 N rows (i, c)][ld = S rounded up to 8] fp16, zero behind S, = mask * (LN(m) W^T) for W_1 and
  * W_2 [32][64]; mask fp32 [S][N] or NULL: the operands of px_opm_outer.
- * px_msa_values: v [8][N][S][8] = LN(m) W^T, W [64][64], 8 heads x 8 channels.
- * px_msa_gate_out: m += W_out(sigmoid(LN(m) W_g^T) * wv), wv laid out as v.
+ * px_msa_values: v [8][3][N][S][8] bf16 = LN(m) W^T, W [64][64], 8 heads x 8 channels, as three planes whose sum is the value.
+ * px_msa_weights: softmax over the last axis of logits fp32 [8][N][N], as planes w [8][3][N][ld = N rounded up to 8], zero behind N.
+ * px_msa_average: wv [8][N][S][8] fp32 = sum_j w[h][i][j] v[h][j], fp32-grade products of the two.
+ * px_msa_gate_out: m += W_out(sigmoid(LN(m) W_g^T) * wv).
  * px_msa_transition: m += W_out(silu(W_a LN(m)) * (W_b LN(m))) over `rows` rows, hidden width 256, fp32-grade products;
  * px_msa_transition_prepare lays the weights [256][64], [256][64], [64][256] out in px_msa_transition_weights_bytes().
  * Replace OuterProductMean's projections (protenix/model/triangular/layers.py:697-767), MSAPairWeightedAveraging and the
@@ -275,8 +278,10 @@ PX_API int32_t px_pair_bias_proj(const void* z, int32_t z_dtype, const float* ln
 PX_API int32_t px_msa_opm_prep(const float* m, const float* mask, const float* ln_w, const float* ln_b, const float* w_1,
                                const float* w_2, px_f16* a_t, px_f16* b_t, int64_t s_rows, int64_t n, int64_t ld, float eps,
                                void* stream);
-PX_API int32_t px_msa_values(const float* m, const float* ln_w, const float* ln_b, const float* w, float* v, int64_t s_rows,
+PX_API int32_t px_msa_values(const float* m, const float* ln_w, const float* ln_b, const float* w, px_bf16* v, int64_t s_rows,
                              int64_t n, float eps, void* stream);
+PX_API int32_t px_msa_weights(const float* logits, px_bf16* w, int64_t n, int64_t ld, void* stream);
+PX_API int32_t px_msa_average(const px_bf16* w, const px_bf16* v, float* wv, int64_t s_rows, int64_t n, int64_t ld, void* stream);
 PX_API int32_t px_msa_gate_out(float* m, const float* wv, const float* ln_w, const float* ln_b, const float* w_g,
                                const float* w_out, int64_t s_rows, int64_t n, float eps, void* stream);
 PX_API int64_t px_msa_transition_weights_bytes(void);

@@ -65,6 +65,8 @@ SIGNATURES = {
     "px_pair_bias_proj_folded": (I32, [P, I32, P, P, I64, I32, F, P]),
     "px_msa_opm_prep": (I32, [P, P, P, P, P, P, P, P, I64, I64, I64, F, P]),
     "px_msa_values": (I32, [P, P, P, P, P, I64, I64, F, P]),
+    "px_msa_weights": (I32, [P, P, I64, I64, P]),
+    "px_msa_average": (I32, [P, P, P, I64, I64, I64, P]),
     "px_msa_gate_out": (I32, [P, P, P, P, P, P, I64, I64, F, P]),
     "px_msa_transition_weights_bytes": (I64, []),
     "px_msa_transition_prepare": (I32, [P, P, P, P, P]),

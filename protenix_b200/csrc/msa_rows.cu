@@ -1,7 +1,7 @@
 // Row-wise steps of the MSA stack on an fp32 MSA embedding m [S][N][64] (c_m = 64), each one pass over m:
 //   msa_opm_prep    a_t, b_t [(i, c)][s] fp16 = mask * LN(m) W_1^T, LN(m) W_2^T (32 columns each): the operands of px_opm_outer
-//   msa_values      v [8 heads][j][8 s + c] = LN(m) W_mv^T: the right-hand side of the pair-weighted average, one GEMM per head
-//   msa_gate_out    m += W_out( sigmoid(LN(m) W_mg^T) * wv ), wv [8][i][8 s + c] as that GEMM leaves it
+//   msa_values      v [8 heads][3][j][8 s + c] = LN(m) W_mv^T as three bf16 planes: the right-hand side of the pair-weighted average
+//   msa_gate_out    m += W_out( sigmoid(LN(m) W_mg^T) * wv ), wv [8][i][8 s + c] as the average leaves it (msa_average_tc.cu)
 // Each is LayerNorm and one or two 64 x 64 products per row (8192 FLOP against 256 bytes read), in fp32 on the FMA pipe as before;
 // what they replace were library GEMMs with the LayerNorm, the mask, the gate, the residual and the permutations as separate
 // passes over tensors of m's size (100 MB at S = 1024, N = 384).
@@ -9,8 +9,8 @@
 // CTA = one token and 128 sequences, 256 threads.  The rows (256 bytes each, N * 256 apart) go through the LayerNorm into shared
 // memory, 16 lanes a row; a thread then owns 8 rows x 4 columns of the product (per 4 inputs: 8 broadcast and 4 contiguous
 // 16-byte reads against 128 FMAs).  With the token fixed, the transposed results are runs of 128 sequences: 256 bytes of
-// fp16 per (i, c), 4 KB of fp32 per head.
-#include "px_common.cuh"
+// fp16 per (i, c), 2 KB per head and plane.
+#include "px_split.cuh"
 
 namespace px {
 
@@ -128,7 +128,7 @@ msa_opm_prep_kernel(const float* __restrict__ m, const float* __restrict__ mask,
 
 __global__ void __launch_bounds__(kMrThreads, 3)
 msa_values_kernel(const float* __restrict__ m, const float* __restrict__ gamma, const float* __restrict__ beta,
-                  const float* __restrict__ w, float* __restrict__ v, int n, int s_rows, float eps) {
+                  const float* __restrict__ w, bf16* __restrict__ v, int n, int s_rows, float eps) {
   extern __shared__ __align__(16) unsigned char mr_raw[];
   MrSmem& sm = *reinterpret_cast<MrSmem*>(mr_raw);
   pdl_wait();
@@ -138,12 +138,27 @@ msa_values_kernel(const float* __restrict__ m, const float* __restrict__ gamma, 
   __syncthreads();
   float acc[8][4];
   product(sm, acc, ty, tx);
+  __syncthreads();                                   // x and w have been read
+  // [plane][head][128 sequences][8 channels], heads 2080 bytes apart
+  unsigned char* t = mr_raw;
+  constexpr int kHead = kMrRows * 16 + 32;
+  static_assert(24 * kHead <= (int)sizeof(MrSmem), "staging");
   const int h = tx >> 1, c = 4 * (tx & 1);           // columns 4 tx.. = head tx / 2, channels 4 (tx & 1)..
 #pragma unroll
   for (int a = 0; a < 8; ++a) {
-    const int s = s0 + ty + 16 * a;
-    if (s < s_rows)
-      *reinterpret_cast<float4*>(v + (((size_t)h * n + i) * s_rows + s) * 8 + c) = make_float4(acc[a][0], acc[a][1], acc[a][2], acc[a][3]);
+    uint32_t lo[3], hi[3];
+    split3x2(acc[a][0], acc[a][1], lo);
+    split3x2(acc[a][2], acc[a][3], hi);
+#pragma unroll
+    for (int p = 0; p < 3; ++p)
+      *reinterpret_cast<uint2*>(t + (p * 8 + h) * kHead + (ty + 16 * a) * 16 + 2 * c) = make_uint2(lo[p], hi[p]);
+  }
+  __syncthreads();
+  for (int j = threadIdx.x; j < 24 * kMrRows; j += kMrThreads) {
+    const int ph = j / kMrRows, s = j % kMrRows;     // ph = 8 plane + head
+    if (s0 + s < s_rows)
+      *reinterpret_cast<uint4*>(v + ((((size_t)(ph & 7) * 3 + (ph >> 3)) * n + i) * s_rows + s0 + s) * 8) =
+          *reinterpret_cast<const uint4*>(t + ph * kHead + s * 16);
   }
 }
 
@@ -208,13 +223,13 @@ extern "C" int32_t px_msa_opm_prep(const float* m, const float* mask, const floa
              : PX_ERR_LAUNCH;
 }
 
-extern "C" int32_t px_msa_values(const float* m, const float* ln_w, const float* ln_b, const float* w, float* v, int64_t s_rows,
+extern "C" int32_t px_msa_values(const float* m, const float* ln_w, const float* ln_b, const float* w, px_bf16* v, int64_t s_rows,
                                  int64_t n, float eps, void* stream) {
   if (!mr_ok(m, s_rows, n) || !w || !v || (((uintptr_t)ln_w | (uintptr_t)ln_b | (uintptr_t)w | (uintptr_t)v) & 15)) return PX_ERR_BAD_ARG;
   static SmemLimit limit;
   return limit.set(msa_values_kernel, sizeof(MrSmem)) &&
-                 launch_pdl(msa_values_kernel, mr_grid(s_rows, n), kMrThreads, sizeof(MrSmem), (cudaStream_t)stream, m, ln_w, ln_b, w, v,
-                            (int)n, (int)s_rows, eps)
+                 launch_pdl(msa_values_kernel, mr_grid(s_rows, n), kMrThreads, sizeof(MrSmem), (cudaStream_t)stream, m, ln_w, ln_b, w,
+                            (bf16*)v, (int)n, (int)s_rows, eps)
              ? PX_OK
              : PX_ERR_LAUNCH;
 }

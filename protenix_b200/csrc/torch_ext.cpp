@@ -11,14 +11,12 @@
 #include <ATen/ATen.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <ATen/cuda/CUDAEvent.h>
-#include <ATen/ops/bmm.h>
 #include <ATen/ops/dropout.h>
 #include <ATen/ops/empty.h>
 #include <ATen/ops/empty_like.h>
 #include <ATen/ops/full.h>
 #include <ATen/ops/mm.h>
 #include <ATen/ops/ones.h>
-#include <ATen/ops/softmax.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <dlfcn.h>
@@ -55,8 +53,8 @@ constexpr int64_t kCz = 128, kCs = 384, kHeadsSingle = 16, kHeads = 4, kHeadDim 
   X(px_triatt_out_fold) X(px_triatt_out_folded) X(px_triatt_workspace_bytes) X(px_transition)                            \
   X(px_pair_bias_folded_bytes) X(px_pair_bias_fold) X(px_pair_bias_proj_folded) X(px_single_weights_bytes)               \
   X(px_single_workspace_bytes) X(px_single_prepare) X(px_single_project) X(px_single_finish) X(px_opm_outer)             \
-  X(px_opm_out) X(px_msa_opm_prep) X(px_msa_values) X(px_msa_gate_out) X(px_msa_transition_weights_bytes)                              \
-  X(px_msa_transition_prepare) X(px_msa_transition)
+  X(px_opm_out) X(px_msa_opm_prep) X(px_msa_values) X(px_msa_weights) X(px_msa_average) X(px_msa_gate_out)               \
+  X(px_msa_transition_weights_bytes) X(px_msa_transition_prepare) X(px_msa_transition)
 struct Abi {
 #define X(f) decltype(&::f) f = nullptr;
   PX_FUNCTIONS(X)
@@ -674,7 +672,9 @@ void msa_stack_forward(Params& params, Params& bias_params, const Tensor& m, con
   const auto& p = pr->p[0];
   const cudaStream_t st = at::cuda::getCurrentCUDAStream();
   const auto opt = m.options();
-  Tensor w = at::empty({heads, n, n}, opt), zn;
+  const int64_t ld = (n + 7) / 8 * 8;
+  const Tensor logits = at::empty({heads, n, n}, opt), w = at::empty({heads, 3, n, ld}, opt.dtype(at::kBFloat16));
+  Tensor zn;
   const void* rows = z.data_ptr();
   if (zf == 0) {
     zn = at::empty(z.sizes(), opt.dtype(at::kHalf));
@@ -684,16 +684,18 @@ void msa_stack_forward(Params& params, Params& bias_params, const Tensor& m, con
     rows = zn.data_ptr();
   }
   launch("px_pair_bias_proj", st, [&] {
-    return abi.px_pair_bias_proj_folded(rows, zf ? PX_BF16 : PX_F16, br->p[zf][0], (float*)w.data_ptr(), n * n, (int32_t)heads, br->scalars[0], st);
+    return abi.px_pair_bias_proj_folded(rows, zf ? PX_BF16 : PX_F16, br->p[zf][0], (float*)logits.data_ptr(), n * n, (int32_t)heads, br->scalars[0], st);
   });
-  w = at::softmax(w, -1);
+  launch("px_msa_weights", st, [&] { return abi.px_msa_weights((const float*)logits.data_ptr(), (px_bf16*)w.data_ptr(), n, ld, st); });
   auto f = [&](int i) { return (const float*)p[i]; };
   for (int64_t s0 = 0; s0 < s_all; s0 += chunk) {
     const int64_t s = std::min(chunk, s_all - s0);
     float* part = (float*)m.data_ptr() + s0 * n * 64;
-    const Tensor v = at::empty({heads, n, s * 8}, opt);
-    launch("px_msa_values", st, [&] { return abi.px_msa_values(part, f(0), f(1), f(2), (float*)v.data_ptr(), s, n, pr->scalars[0], st); });
-    const Tensor wv = at::bmm(w, v);                 // one [N x N] . [N x 8 S] product per head, fp32
+    const Tensor v = at::empty({heads, 3, n, s * 8}, opt.dtype(at::kBFloat16)), wv = at::empty({heads, n, s * 8}, opt);
+    launch("px_msa_values", st, [&] { return abi.px_msa_values(part, f(0), f(1), f(2), (px_bf16*)v.data_ptr(), s, n, pr->scalars[0], st); });
+    launch("px_msa_average", st, [&] {
+      return abi.px_msa_average((const px_bf16*)w.data_ptr(), (const px_bf16*)v.data_ptr(), (float*)wv.data_ptr(), s, n, ld, st);
+    });
     launch("px_msa_gate_out", st, [&] {
       return abi.px_msa_gate_out(part, (const float*)wv.data_ptr(), f(0), f(1), f(3), f(4), s, n, pr->scalars[0], st);
     });

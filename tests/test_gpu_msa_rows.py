@@ -62,3 +62,27 @@ def test_outer_product_operands(s, n, masked):
         want = want.permute(1, 2, 0).reshape(n * 32, s)
         assert (got[:, s:] == 0).all()
         assert float((got[:, :s].double() - want).abs().max()) < 6e-4 * max(1.0, float(want.abs().max()))
+
+
+@pytest.mark.parametrize("s,n", [(1, 1), (16, 64), (17, 65), (33, 129), (16, 200)])
+def test_weighted_average(s, n):
+    """px_msa_weights and px_msa_average at the edges of their tiles (128 rows, 64 keys, 16 sequences)."""
+    from protenix_b200 import _lib
+
+    torch.manual_seed(n)
+    ld, lib, st = (n + 7) // 8 * 8, _lib.load(), torch.cuda.current_stream().cuda_stream
+    logits, v = 3 * torch.randn(8, n, n, device="cuda"), torch.randn(8, n, s * 8, device="cuda")
+    planes, rest = [], v.clone()
+    for _ in range(3):
+        planes.append(rest.bfloat16())
+        rest -= planes[-1].float()
+    vp = torch.stack(planes, 1).contiguous()
+    wp = torch.empty(8, 3, n, ld, dtype=torch.bfloat16, device="cuda")
+    got = torch.full((8, n, s * 8), float("nan"), device="cuda")
+    _lib.check(lib.px_msa_weights(logits.data_ptr(), wp.data_ptr(), n, ld, st), "px_msa_weights")
+    _lib.check(lib.px_msa_average(wp.data_ptr(), vp.data_ptr(), got.data_ptr(), s, n, ld, st), "px_msa_average")
+    ops.device_error_flags()
+    want = torch.softmax(logits.double(), -1) @ v.double()
+    relf = lambda a: float((a.double() - want).norm() / want.norm())
+    assert (wp[..., n:] == 0).all()
+    assert relf(got) < 2 * relf(torch.softmax(logits, -1) @ v) + 1e-7
