@@ -155,7 +155,8 @@ PX_API int32_t px_trimul_contract(const px_f16* a, const px_f16* b, px_f16* x, i
 #define PX_FAMILY_SINGLE 12
 #define PX_FAMILY_MSA_TRANSITION 13
 #define PX_FAMILY_MSA_AVERAGE 14
-#define PX_N_FAMILIES 15
+#define PX_FAMILY_MSA_ROWS 15
+#define PX_N_FAMILIES 16
 PX_API int32_t px_device_error_flags(uint32_t* flags);
 PX_API int32_t px_device_error_detail(uint32_t* flags, uint32_t* detail);
 /* Limit of every bounded wait on the current device, in SM clock cycles (default 2^28, about 0.14 s); cycles <= 0
@@ -264,7 +265,8 @@ PX_API int32_t px_pair_bias_proj(const void* z, int32_t z_dtype, const float* ln
                           float* out, int64_t rows, int32_t n_heads, float eps, void* stream);
 
 /* ---- MSA embedding ------------------------------------------------------------------------------
- * Row-wise steps on m [S][N][64] fp32, LayerNorm vectors fp32 [64] or NULL, weights fp32 in nn.Linear order.
+ * Row-wise steps on m [S][N][64] fp32, LayerNorm vectors fp32 [64] or NULL, fp32-grade products.  px_msa_rows_prepare lays a
+ * fp32 weight [64][64] (or, with w_b, two of [32][64] one after the other) out in px_msa_rows_weights_bytes().
  * px_msa_opm_prep: a_t, b_t [32 N rows (i, c)][ld = S rounded up to 8] fp16, zero behind S, = mask * (LN(m) W^T) for W_1 and
  * W_2 [32][64]; mask fp32 [S][N] or NULL: the operands of px_opm_outer.
  * px_msa_values: v [8][3][N][S][8] bf16 = LN(m) W^T, W [64][64], 8 heads x 8 channels, as three planes whose sum is the value.
@@ -275,15 +277,16 @@ PX_API int32_t px_pair_bias_proj(const void* z, int32_t z_dtype, const float* ln
  * px_msa_transition_prepare lays the weights [256][64], [256][64], [64][256] out in px_msa_transition_weights_bytes().
  * Replace OuterProductMean's projections (protenix/model/triangular/layers.py:697-767), MSAPairWeightedAveraging and the
  * transition of MSAStack (protenix/model/modules/pairformer.py:343-572). */
-PX_API int32_t px_msa_opm_prep(const float* m, const float* mask, const float* ln_w, const float* ln_b, const float* w_1,
-                               const float* w_2, px_f16* a_t, px_f16* b_t, int64_t s_rows, int64_t n, int64_t ld, float eps,
-                               void* stream);
-PX_API int32_t px_msa_values(const float* m, const float* ln_w, const float* ln_b, const float* w, px_bf16* v, int64_t s_rows,
+PX_API int64_t px_msa_rows_weights_bytes(void);
+PX_API int32_t px_msa_rows_prepare(const float* w_a, const float* w_b, void* prepared, void* stream);
+PX_API int32_t px_msa_opm_prep(const float* m, const float* mask, const float* ln_w, const float* ln_b, const void* prepared,
+                               px_f16* a_t, px_f16* b_t, int64_t s_rows, int64_t n, int64_t ld, float eps, void* stream);
+PX_API int32_t px_msa_values(const float* m, const float* ln_w, const float* ln_b, const void* prepared, px_bf16* v, int64_t s_rows,
                              int64_t n, float eps, void* stream);
 PX_API int32_t px_msa_weights(const float* logits, px_bf16* w, int64_t n, int64_t ld, void* stream);
 PX_API int32_t px_msa_average(const px_bf16* w, const px_bf16* v, float* wv, int64_t s_rows, int64_t n, int64_t ld, void* stream);
-PX_API int32_t px_msa_gate_out(float* m, const float* wv, const float* ln_w, const float* ln_b, const float* w_g,
-                               const float* w_out, int64_t s_rows, int64_t n, float eps, void* stream);
+PX_API int32_t px_msa_gate_out(float* m, const float* wv, const float* ln_w, const float* ln_b, const void* prepared_g,
+                               const void* prepared_out, int64_t s_rows, int64_t n, float eps, void* stream);
 PX_API int64_t px_msa_transition_weights_bytes(void);
 PX_API int32_t px_msa_transition_prepare(const float* w_a, const float* w_b, const float* w_out, void* prepared, void* stream);
 PX_API int32_t px_msa_transition(float* m, const void* prepared, const float* ln_w, const float* ln_b, int64_t rows, float eps,

@@ -54,7 +54,7 @@ constexpr int64_t kCz = 128, kCs = 384, kHeadsSingle = 16, kHeads = 4, kHeadDim 
   X(px_pair_bias_folded_bytes) X(px_pair_bias_fold) X(px_pair_bias_proj_folded) X(px_single_weights_bytes)               \
   X(px_single_workspace_bytes) X(px_single_prepare) X(px_single_project) X(px_single_finish) X(px_opm_outer)             \
   X(px_opm_out) X(px_msa_opm_prep) X(px_msa_values) X(px_msa_weights) X(px_msa_average) X(px_msa_gate_out)               \
-  X(px_msa_transition_weights_bytes) X(px_msa_transition_prepare) X(px_msa_transition)
+  X(px_msa_rows_weights_bytes) X(px_msa_rows_prepare) X(px_msa_transition_weights_bytes) X(px_msa_transition_prepare) X(px_msa_transition)
 struct Abi {
 #define X(f) decltype(&::f) f = nullptr;
   PX_FUNCTIONS(X)
@@ -147,9 +147,10 @@ const float* fptr(const Tensor& t) { return t.defined() ? (const float*)t.data_p
 // ---- parameters of a module -----------------------------------------------------------------------------------------
 // What a parameter becomes: 'f' an fp32 vector, 'z' a matrix in the format of the pair tensor's rows (bf16 rows: bf16, fp32
 // rows: fp16), 'h' an fp16 matrix, 's' an fp32 matrix.  What the group becomes then: kMul, kAtt and kBias the folded weights
-// of their row kernels (in, out), kSingle and kMsa the laid-out matrices of the single branch and of the MSA transition behind what comes before them,
+// of their row kernels (in, out), kSingle and kMsa the laid-out matrices of the single branch and of the MSA stack behind what comes before them, kOpm the
+// outer product's two projections laid out as one,
 // kPlain nothing more.
-enum Group { kPlain, kMul, kAtt, kBias, kSingle, kMsa };
+enum Group { kPlain, kMul, kAtt, kBias, kSingle, kMsa, kOpm };
 struct Prepared {
   std::vector<Tensor> t[2];          // by format of z: 0 fp32, 1 bf16
   std::vector<const void*> p[2];
@@ -163,10 +164,10 @@ class Params {
  public:
   // checks: (dict, name) of submodules; params: (dict, name, kind, shape); scalars: (dict, name)
   Params(const std::string& group, const py::list& checks, const py::list& params, const py::list& scalars) {
-    const char* names[] = {"plain", "mul", "att", "bias", "single", "msa"};
+    const char* names[] = {"plain", "mul", "att", "bias", "single", "msa", "opm"};
     int g = 0;
-    while (g < 6 && group != names[g]) ++g;
-    if (g == 6) fail("unknown parameter group " + group);
+    while (g < 7 && group != names[g]) ++g;
+    if (g == 7) fail("unknown parameter group " + group);
     group_ = (Group)g;
     for (const auto& c : checks) {
       const auto t = c.cast<py::tuple>();
@@ -275,6 +276,13 @@ class Params {
     const auto byte = at::TensorOptions().device(dev).dtype(at::kByte);
     auto f = [&](int i) { return t[i].defined() ? (const float*)t[i].data_ptr() : nullptr; };
     auto w = [&](int i) { return (const px_w16*)t[i].data_ptr(); };
+    auto msa_rows = [&](const Tensor& a, const Tensor& b) {          // b: the second half of the outputs
+      const Tensor out = at::empty({abi.px_msa_rows_weights_bytes()}, byte);
+      launch("px_msa_rows_prepare", st, [&] {
+        return abi.px_msa_rows_prepare((const float*)a.data_ptr(), b.defined() ? (const float*)b.data_ptr() : nullptr, out.data_ptr(), st);
+      });
+      return out;
+    };
     if (group_ == kMul) {
       const Tensor in = at::empty({abi.px_trimul_in_folded_bytes()}, byte), out = at::empty({abi.px_trimul_out_folded_bytes()}, byte);
       launch("px_trimul_in_fold", st, [&] {
@@ -309,6 +317,9 @@ class Params {
       launch("px_msa_transition_prepare", st, [&] { return abi.px_msa_transition_prepare(f(7), f(8), f(9), out.data_ptr(), st); });
       t.resize(7);
       t.push_back(out);
+      for (int i = 2; i < 5; ++i) t[i] = msa_rows(t[i], Tensor());
+    } else if (group_ == kOpm) {
+      t[2] = msa_rows(t[2], t[3]);
     }
     p.t[zf] = t;
     p.p[zf].clear();
@@ -640,8 +651,7 @@ Tensor opm_forward(Params& params, const Tensor& m, const OptTensor& mask, const
   const Tensor x = at::empty({n_blk * 32, n * 32}, opt.dtype(at::kHalf));
   const cudaStream_t st = at::cuda::getCurrentCUDAStream();
   launch("px_msa_opm_prep", st, [&] {
-    return abi.px_msa_opm_prep((const float*)m.data_ptr(), fptr(mk), (const float*)p[0], (const float*)p[1], (const float*)p[2],
-                               (const float*)p[3], a, b, s_rows, n, ld, ln_eps, st);
+    return abi.px_msa_opm_prep((const float*)m.data_ptr(), fptr(mk), (const float*)p[0], (const float*)p[1], p[2], a, b, s_rows, n, ld, ln_eps, st);
   });
   const int64_t row = z_out.element_size() * n * kCz;
   for (int64_t i0 = 0; i0 < n; i0 += n_blk) {
@@ -692,12 +702,12 @@ void msa_stack_forward(Params& params, Params& bias_params, const Tensor& m, con
     const int64_t s = std::min(chunk, s_all - s0);
     float* part = (float*)m.data_ptr() + s0 * n * 64;
     const Tensor v = at::empty({heads, 3, n, s * 8}, opt.dtype(at::kBFloat16)), wv = at::empty({heads, n, s * 8}, opt);
-    launch("px_msa_values", st, [&] { return abi.px_msa_values(part, f(0), f(1), f(2), (px_bf16*)v.data_ptr(), s, n, pr->scalars[0], st); });
+    launch("px_msa_values", st, [&] { return abi.px_msa_values(part, f(0), f(1), p[2], (px_bf16*)v.data_ptr(), s, n, pr->scalars[0], st); });
     launch("px_msa_average", st, [&] {
       return abi.px_msa_average((const px_bf16*)w.data_ptr(), (const px_bf16*)v.data_ptr(), (float*)wv.data_ptr(), s, n, ld, st);
     });
     launch("px_msa_gate_out", st, [&] {
-      return abi.px_msa_gate_out(part, (const float*)wv.data_ptr(), f(0), f(1), f(3), f(4), s, n, pr->scalars[0], st);
+      return abi.px_msa_gate_out(part, (const float*)wv.data_ptr(), f(0), f(1), p[3], p[4], s, n, pr->scalars[0], st);
     });
     launch("px_msa_transition", st, [&] { return abi.px_msa_transition(part, p[7], f(5), f(6), s * n, pr->scalars[1], st); });
   }

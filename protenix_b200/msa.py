@@ -21,7 +21,7 @@ from .triangular import OpenfoldLinear
 
 
 class OuterProductMean(nn.Module):
-    NATIVE = ("plain", [("layer_norm.weight", "f", (64,)), ("layer_norm.bias", "f", (64,)), ("linear_1.weight", "s", (32, 64)),
+    NATIVE = ("opm", [("layer_norm.weight", "f", (64,)), ("layer_norm.bias", "f", (64,)), ("linear_1.weight", "s", (32, 64)),
                         ("linear_2.weight", "s", (32, 64)), ("linear_out.weight", "h", (128, 1024)), ("linear_out.bias", "f", (128,))],
               ["eps", "layer_norm.eps"])
 

@@ -137,7 +137,7 @@ def _launch(name: str, fn, *args) -> None:
 
 KERNEL_FAMILIES = ("trimul_contract", "triatt_flash", "transition", "trimul_in_proj", "trimul_out", "triatt_in_proj",
                    "triatt_out", "pair_bias_proj", "recycle_update", "selftest", "peer_barrier",
-                   "outer_product_mean", "single_update", "msa_transition", "msa_average")   # bit order of px_device_error_flags
+                   "outer_product_mean", "single_update", "msa_transition", "msa_average", "msa_rows")   # bit order of px_device_error_flags
 
 
 def device_error_flags(device=None, raise_on_error: bool = True) -> int:

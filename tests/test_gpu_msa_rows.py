@@ -54,8 +54,10 @@ def test_outer_product_operands(s, n, masked):
 
     ln = mod.layer_norm
     p = lambda t: None if t is None else t.data_ptr()
-    _lib.check(_lib.load().px_msa_opm_prep(p(m), p(mask), p(ln.weight), p(ln.bias), p(mod.linear_1.weight), p(mod.linear_2.weight),
-                                           p(a), p(b), s, n, ld, ln.eps, torch.cuda.current_stream().cuda_stream), "px_msa_opm_prep")
+    lib, st = _lib.load(), torch.cuda.current_stream().cuda_stream
+    w = torch.empty(lib.px_msa_rows_weights_bytes(), dtype=torch.uint8, device="cuda")
+    _lib.check(lib.px_msa_rows_prepare(p(mod.linear_1.weight), p(mod.linear_2.weight), p(w), st), "px_msa_rows_prepare")
+    _lib.check(lib.px_msa_opm_prep(p(m), p(mask), p(ln.weight), p(ln.bias), p(w), p(a), p(b), s, n, ld, ln.eps, st), "px_msa_opm_prep")
     x = F.layer_norm(m.double(), (64,), ln.weight.detach().double(), ln.bias.detach().double(), ln.eps)
     for got, lin in ((a, mod.linear_1), (b, mod.linear_2)):
         want = F.linear(x, lin.weight.detach().double()) * (1.0 if mask is None else mask.double()[..., None])
