@@ -222,15 +222,12 @@ PX_API int32_t px_triatt_in_proj(const void* z, int32_t z_dtype, const float* ma
                           int64_t ldm, int32_t ending, float eps, float inf, void* stream);
 /* Stage 2: o[u][t][h*32+d] = softmax_k(q.k + bias[h][t][k] + mask_bias[u][k]) v on the tcgen05
  * tensor cores: TMA-fed, logits and probabilities live in tensor memory only, online softmax in
- * base 2.  v is the transposed layout [u][h][32][ld(n)] written by stage 1; `scratch` needs
- * px_triatt_flash_scratch_bytes(n_u, n) bytes (per-tile mask flags).  All pointers 16-byte aligned.
+ * base 2.  v is the transposed layout [u][h][32][ld(n)] written by stage 1.  All pointers 16-byte aligned.
  * Replaces the back-ends selected in protenix/model/triangular/layers.py:441-469 (_attention
  * :276-296, the Triton kernel protenix/model/tri_attention/forward.py:22-188, DS4Sci and
  * cuEquivariance calls). */
 PX_API int32_t px_triatt_flash(const px_f16* q, const px_f16* k, const px_f16* v, const float* bias,
-                        const float* mask_bias, px_f16* o, void* scratch, int64_t n_u, int64_t n, int64_t ldm,
-                        void* stream);
-PX_API int64_t px_triatt_flash_scratch_bytes(int64_t n_u, int64_t n);
+                        const float* mask_bias, px_f16* o, int64_t n_u, int64_t n, int64_t ldm, void* stream);
 /* Stage 3: z_out(u,t) = [z_in(u,t) +] W_o (o[u][t] * sigmoid(W_g LN(z_in(u,t)))), where (u,t)
  * addresses z[u][t] (starting) or z[t][u] (ending).  z_out may alias z_in.  zn: the standardised copy of z_in
  * (same layout) when z_dtype is PX_F32 (NULL otherwise).  z_dtype PX_F16: z_in is itself the standardised fp16 copy

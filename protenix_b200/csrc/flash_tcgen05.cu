@@ -102,7 +102,7 @@ __device__ __forceinline__ void exp2_poly2(float x0, float x1, float& p0, float&
 __global__ void __launch_bounds__(kFThreads, 1)
 triatt_flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                        const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_b,
-                       const float* __restrict__ mb, const unsigned long long* __restrict__ tile_masked,
+                       const float* __restrict__ mb,
                        bf16* __restrict__ o, int n_u, int n, int ldm, int nkt) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* sm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -211,8 +211,7 @@ triatt_flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     const uint32_t t_p = tmem_base + lane_addr + kFColP + (kFKT / 2) * g;
     const uint32_t t_o = tmem_base + lane_addr + kFColO + kFON * kFRpg * g;
     const int ug = u0 + kFRpg * g;                  // first row of this group
-    const int words = (nkt + 63) / 64;              // mask-flag words per row: one bit per 64-key tile
-    unsigned long long flag_word[kFRpg];
+    unsigned long long flag_word[kFRpg];            // bit kt & 63: some key of tile kt has a mask bias other than zero
     float m_ref[kFRpg], l_sum[kFRpg];             // reference maximum and denominator of this thread's query per row
 #pragma unroll
     for (int r = 0; r < kFRpg; ++r) {
@@ -223,9 +222,32 @@ triatt_flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     bool ok = true;
     for (int kt = 0; kt < nkt && ok; ++kt) {
       if ((kt & 63) == 0) {
+        for (int r = 0; r < kFRpg; ++r) flag_word[r] = 0;
+        // A load covers two tiles (ldm is a multiple of 128), eight are in flight beside the first TMA loads and products (two
+        // in flight: 6.17 ms at N = 1536, against 5.88).  As a kernel of its own this cost a launch: 16.6 us together at
+        // N = 128 against 12.6, 143 against 136 at N = 384.
+        const int left = min(nkt - kt, 64);
+#pragma unroll 1
+        for (int t0 = 0; t0 < left; t0 += 8) {
+          float4 m4[kFRpg][4];
 #pragma unroll
-        for (int r = 0; r < kFRpg; ++r)
-          flag_word[r] = (ug + r < n_u) ? __ldg(tile_masked + (size_t)(ug + r) * words + (kt >> 6)) : ~0ull;
+          for (int r = 0; r < kFRpg; ++r)
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+              m4[r][j] = t0 + 2 * j < left ? __ldg(reinterpret_cast<const float4*>(mb + (size_t)((ug + r < n_u) ? ug + r : 0) * ldm +
+                                                                                   (kt + t0 + 2 * j) * kFKT) + lane)
+                                           : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+          for (int r = 0; r < kFRpg; ++r) {
+            unsigned bits = 0;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              const unsigned b = __ballot_sync(0xffffffffu, m4[r][j].x != 0.f || m4[r][j].y != 0.f || m4[r][j].z != 0.f || m4[r][j].w != 0.f);
+              bits |= (((b & 0xffffu) ? 1u : 0u) | ((b >> 16) ? 2u : 0u)) << (2 * j);
+            }
+            flag_word[r] |= (unsigned long long)bits << t0;
+          }
+        }
       }
       ok = mbar_wait(&bars.bias_full[kt & 1], (kt >> 1) & 1, 64u);
       ok = __all_sync(0xffffffffu, ok);
@@ -381,26 +403,6 @@ triatt_flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
   }
 }
 
-// Bit (kt & 63) of flags[u][kt >> 6] is set when any key of the 64-key tile kt carries a non-zero mask bias
-// for row u.  One CTA per (u, word); each warp handles tiles warp, warp + 4, ...
-__global__ void flash_tile_flags_kernel(const float* __restrict__ mb, unsigned long long* __restrict__ flags, int ldm,
-                                        int nkt) {
-  __shared__ unsigned long long word;
-  pdl_wait();
-  const int u = blockIdx.x, w = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (threadIdx.x == 0) word = 0ull;
-  __syncthreads();
-  for (int t = warp; t < 64; t += 4) {
-    const int kt = 64 * w + t;
-    if (kt >= nkt) break;
-    const float* p = mb + (size_t)u * ldm + kt * kFKT;
-    const bool any = __any_sync(0xffffffffu, p[lane] != 0.0f || p[lane + 32] != 0.0f);
-    if (any && lane == 0) atomicOr(&word, 1ull << t);
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) flags[(size_t)u * gridDim.y + w] = word;
-}
-
 PX_DEFINE_FAMILY_HOOKS(flash)
 
 }  // namespace px
@@ -409,15 +411,10 @@ using namespace px;
 
 extern "C" int64_t px_ld_mask(int64_t n) { return (n + 127) / 128 * 128; }
 
-extern "C" int64_t px_triatt_flash_scratch_bytes(int64_t n_u, int64_t n) {
-  if (n_u <= 0 || n <= 0) return 0;
-  return (n_u * ((((n + kFKT - 1) / kFKT) + 63) / 64) * 8 + 255) / 256 * 256;
-}
-
 extern "C" int32_t px_triatt_flash(const px_f16* q, const px_f16* k, const px_f16* v, const float* bias,
-                                   const float* mask_bias, px_f16* o, void* scratch, int64_t n_u, int64_t n,
+                                   const float* mask_bias, px_f16* o, int64_t n_u, int64_t n,
                                    int64_t ldm, void* stream) {
-  if (!q || !k || !v || !bias || !mask_bias || !o || !scratch || n_u <= 0 || n <= 0 || n_u > 32768 || n > 32768 ||
+  if (!q || !k || !v || !bias || !mask_bias || !o || n_u <= 0 || n <= 0 || n_u > 32768 || n > 32768 ||
       ldm != px_ld_mask(n))
     return PX_ERR_BAD_ARG;
   if (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)bias | (uintptr_t)mask_bias | (uintptr_t)o) & 15)
@@ -439,16 +436,11 @@ extern "C" int32_t px_triatt_flash(const px_f16* q, const px_f16* k, const px_f1
                    (uint64_t)n * ldm * 4, 32, 128, CU_TENSOR_MAP_SWIZZLE_128B))
     return PX_ERR_LAUNCH;
   cudaStream_t st = (cudaStream_t)stream;
-  if ((uintptr_t)scratch & 7) return PX_ERR_BAD_ARG;
-  if (!launch_pdl(flash_tile_flags_kernel, dim3((unsigned)n_u, (unsigned)((nkt + 63) / 64)), 128, 0, st, mask_bias,
-                  (unsigned long long*)scratch, (int)ldm, nkt))
-    return PX_ERR_LAUNCH;
   const size_t smem = FlashLayout::total + 1024;
   static SmemLimit limit;
   if (!limit.set(triatt_flash_tc_kernel, smem)) return PX_ERR_LAUNCH;
   dim3 grid((unsigned)((n + 127) / 128), kFH, (unsigned)((n_u + kFRows - 1) / kFRows));
-  return launch_pdl(triatt_flash_tc_kernel, grid, kFThreads, smem, st, mq, mk, mv, mbias, mask_bias,
-                    (const unsigned long long*)scratch, (bf16*)o, (int)n_u, (int)n, (int)ldm, nkt)
+  return launch_pdl(triatt_flash_tc_kernel, grid, kFThreads, smem, st, mq, mk, mv, mbias, mask_bias, (bf16*)o, (int)n_u, (int)n, (int)ldm, nkt)
              ? PX_OK
              : PX_ERR_LAUNCH;
 }

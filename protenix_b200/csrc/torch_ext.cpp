@@ -49,7 +49,7 @@ constexpr int64_t kCz = 128, kCs = 384, kHeadsSingle = 16, kHeads = 4, kHeadDim 
   X(px_scale_add_rowwise) X(px_standardise_rows) X(px_trimul_in_folded_bytes) X(px_trimul_in_fold)                       \
   X(px_trimul_in_proj_folded) X(px_trimul_contract) X(px_trimul_out_folded_bytes) X(px_trimul_out_fold)                  \
   X(px_trimul_out_folded) X(px_trimul_workspace_bytes) X(px_triatt_in_folded_bytes) X(px_triatt_in_fold)                 \
-  X(px_triatt_in_proj_folded) X(px_triatt_flash) X(px_triatt_flash_scratch_bytes) X(px_triatt_out_folded_bytes)          \
+  X(px_triatt_in_proj_folded) X(px_triatt_flash) X(px_triatt_out_folded_bytes)                                           \
   X(px_triatt_out_fold) X(px_triatt_out_folded) X(px_triatt_workspace_bytes) X(px_transition)                            \
   X(px_pair_bias_folded_bytes) X(px_pair_bias_fold) X(px_pair_bias_proj_folded) X(px_single_weights_bytes)               \
   X(px_single_workspace_bytes) X(px_single_prepare) X(px_single_project) X(px_single_finish) X(px_opm_outer)             \
@@ -396,7 +396,6 @@ void tri_att(const PairCall& c, const Prepared& pr, const void* z_in, void* z_ou
   px_f16 *q = (px_f16*)c.ws, *k = (px_f16*)(c.ws + qkv), *v = (px_f16*)(c.ws + 2 * qkv), *o = (px_f16*)(c.ws + 3 * qkv);
   unsigned char* bias = (unsigned char*)o + al(n * n * kCz * 2);
   unsigned char* mbias = bias + al(kHeads * n * ldm * 4);
-  unsigned char* flags = mbias + al(n * ldm * 4);
   const bool fp32 = c.dt == PX_F32;
   if (fp32) rows.need(c, z_in, eps);
   launch("px_triatt_in_proj", c.st, [&] {
@@ -404,7 +403,7 @@ void tri_att(const PairCall& c, const Prepared& pr, const void* z_in, void* z_ou
                                         n, ldm, ending, eps, inf, c.st);
   });
   launch("px_triatt_flash", c.st, [&] {
-    return abi.px_triatt_flash(q, k, v, (const float*)bias, (const float*)mbias, o, flags, n, n, ldm, c.st);
+    return abi.px_triatt_flash(q, k, v, (const float*)bias, (const float*)mbias, o, n, n, ldm, c.st);
   });
   rows.valid = false;
   launch("px_triatt_out", c.st, [&] {

@@ -27,7 +27,7 @@ extern "C" int64_t px_triatt_workspace_bytes(int64_t n) {
   const int64_t ld = px_ld_mask(n);
   return (int64_t)(3 * align256(att_qkv_elems(n) * 2) + align256((size_t)n * n * kC * 2) +
                    align256((size_t)kH * n * ld * 4) + align256((size_t)n * ld * 4) +
-                   align256((size_t)px_triatt_flash_scratch_bytes(n, n)) + align256((size_t)n * n * kC * 2));
+                   align256((size_t)n * n * kC * 2));
 }
 
 extern "C" int32_t px_triangle_attention(const void* z_in, void* z_out, int32_t z_dtype, const float* mask,
@@ -52,8 +52,6 @@ extern "C" int32_t px_triangle_attention(const void* z_in, void* z_out, int32_t 
   p += align256((size_t)kH * n * ld * 4);
   float* mbias = (float*)p;
   p += align256((size_t)n * ld * 4);
-  void* flags = (void*)p;
-  p += align256((size_t)px_triatt_flash_scratch_bytes(n, n));
   px_f16* zn = (px_f16*)p;
   const void* rows = z_in;                 // the rows the tensor core multiplies: bf16 z itself, or ...
   int32_t rows_dtype = z_dtype, s;
@@ -66,7 +64,7 @@ extern "C" int32_t px_triangle_attention(const void* z_in, void* z_out, int32_t 
   s = px_triatt_in_proj(rows, rows_dtype, mask, ln_w, ln_b, w_q, w_k, w_v, w_bias, q, k, v, bias, mbias, n, n, ld, ending,
                         eps, inf, stream);
   if (s != PX_OK) return s;
-  s = px_triatt_flash(q, k, v, bias, mbias, o, flags, n, n, ld, stream);
+  s = px_triatt_flash(q, k, v, bias, mbias, o, n, n, ld, stream);
   if (s != PX_OK) return s;
   return px_triatt_out(o, z_in, zn, z_out, z_dtype, ln_w, ln_b, w_g, w_o, n, n, ending, add_residual, eps, stream);
 }

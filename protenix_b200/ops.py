@@ -119,8 +119,7 @@ def reset_launch_count() -> int:
 
 
 def _launch(name: str, fn, *args) -> None:
-    """Call one C-ABI launcher, optionally bracketed by CUDA events (one kernel per launcher, except
-    ``px_triatt_flash``, which runs its small tile-flag kernel first: its stage time covers both)."""
+    """Call one C-ABI launcher, optionally bracketed by CUDA events."""
     global launch_count
     if _timer is not None:
         a = torch.cuda.Event(enable_timing=True)
@@ -318,19 +317,18 @@ def triangle_attention(z_in: torch.Tensor, z_out: torch.Tensor, mask: Optional[t
     k, v, o = q + qkv, q + 2 * qkv, q + 3 * qkv
     bias = o + al(n * n * C_Z * 2)
     mbias = bias + al(N_HEAD_PAIR * n * ldn * 4)
-    flags = mbias + al(n * ldn * 4)
     dt, st, eps = _pair_dtype(z_in), _stream(z_in), float(eps)
     rows, rows_dt = _ptr(z_in), dt
     zn = _zn_arg(z_in, zn)
     if dt == PX_F32:            # the projection and the output stage normalise the same z: one standardised copy
         if zn is None:
-            zn = flags + al(lib.px_triatt_flash_scratch_bytes(n, n))
+            zn = mbias + al(n * ldn * 4)
             _launch("px_standardise_rows", lib.px_standardise_rows, _ptr(z_in), zn, n * n, eps, st)
         rows, rows_dt = zn, PX_F16
     _launch("px_triatt_in_proj", lib.px_triatt_in_proj, rows, rows_dt, _ptr(mask), _ptr(ln_w), _ptr(ln_b),
             _ptr(w_q), _ptr(w_k), _ptr(w_v), _ptr(w_bias), q, k, v, bias, mbias, n, n, ldn, int(ending), eps,
             float(inf), st)
-    _launch("px_triatt_flash", lib.px_triatt_flash, q, k, v, bias, mbias, o, flags, n, n, ldn, st)
+    _launch("px_triatt_flash", lib.px_triatt_flash, q, k, v, bias, mbias, o, n, n, ldn, st)
     _launch("px_triatt_out", lib.px_triatt_out, o, _ptr(z_in), zn, _ptr(z_out), dt, _ptr(ln_w), _ptr(ln_b), _ptr(w_g),
             _ptr(w_o), n, n, int(ending), int(add_residual), eps, st)
     return z_out
@@ -547,9 +545,8 @@ def triatt_flash(q, k, v, bias_full: torch.Tensor, mb) -> torch.Tensor:
         raise RuntimeError("q, k, v must be float16, the pair bias and mask_bias float32")
     o = torch.empty(n_u, n, C_Z, dtype=torch.float16, device=q.device)
     lib = _lib.load()
-    scratch = torch.empty(int(lib.px_triatt_flash_scratch_bytes(n_u, n)), dtype=torch.uint8, device=q.device)
     _launch("px_triatt_flash", lib.px_triatt_flash, _ptr(q), _ptr(k), _ptr(v), _ptr(bias_full), _ptr(mb), _ptr(o),
-            _ptr(scratch), n_u, n, ldm, _stream(q))
+            n_u, n, ldm, _stream(q))
     return o
 
 
