@@ -264,6 +264,8 @@ PX_API int32_t px_pair_bias_proj(const void* z, int32_t z_dtype, const float* ln
 /* ---- MSA embedding ------------------------------------------------------------------------------
  * Row-wise steps on m [S][N][64] fp32, LayerNorm vectors fp32 [64] or NULL, fp32-grade products.  px_msa_rows_prepare lays a
  * fp32 weight [64][64] (or, with w_b, two of [32][64] one after the other) out in px_msa_rows_weights_bytes().
+ * px_msa_embed: m[s][i] = W x + s_proj[i] with x = one_hot(msa[index[s]][i]) | has_deletion | deletion_value, W [64][34], s_proj
+ * [N][64], for s_rows selected sequences (index within the MSA's rows; a class outside 0..31 gives NaN).
  * px_msa_opm_prep: a_t, b_t [32 N rows (i, c)][ld = S rounded up to 8] fp16, zero behind S, = mask * (LN(m) W^T) for W_1 and
  * W_2 [32][64]; mask fp32 [S][N] or NULL: the operands of px_opm_outer.
  * px_msa_values: v [8][3][N][S][8] bf16 = LN(m) W^T, W [64][64], 8 heads x 8 channels, as three planes whose sum is the value.
@@ -274,6 +276,8 @@ PX_API int32_t px_pair_bias_proj(const void* z, int32_t z_dtype, const float* ln
  * px_msa_transition_prepare lays the weights [256][64], [256][64], [64][256] out in px_msa_transition_weights_bytes().
  * Replace OuterProductMean's projections (protenix/model/triangular/layers.py:697-767), MSAPairWeightedAveraging and the
  * transition of MSAStack (protenix/model/modules/pairformer.py:343-572). */
+PX_API int32_t px_msa_embed(const int64_t* msa, const float* has_deletion, const float* deletion_value, const int64_t* index,
+                            const float* w, const float* s_proj, float* m, int64_t s_rows, int64_t n, void* stream);
 PX_API int64_t px_msa_rows_weights_bytes(void);
 PX_API int32_t px_msa_rows_prepare(const float* w_a, const float* w_b, void* prepared, void* stream);
 PX_API int32_t px_msa_opm_prep(const float* m, const float* mask, const float* ln_w, const float* ln_b, const void* prepared,

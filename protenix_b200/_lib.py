@@ -62,6 +62,7 @@ SIGNATURES = {
     "px_pair_bias_folded_bytes": (I64, []),
     "px_pair_bias_fold": (I32, [P, P, P, I32, I32, P, P]),
     "px_pair_bias_proj_folded": (I32, [P, I32, P, P, I64, I32, F, P]),
+    "px_msa_embed": (I32, [P, P, P, P, P, P, P, I64, I64, P]),
     "px_msa_rows_weights_bytes": (I64, []),
     "px_msa_rows_prepare": (I32, [P, P, P, P]),
     "px_msa_opm_prep": (I32, [P, P, P, P, P, P, P, I64, I64, I64, F, P]),

@@ -12,7 +12,7 @@ LIB = os.path.join(HERE, "libpx_b200.so")
 EXT_SRC = os.path.join(CSRC, "torch_ext.cpp")       # the native host path: C++ only, built against torch's headers
 EXT = os.path.join(HERE, "_C.so")
 SOURCES = ["api.cu", "layer_norm.cu", "trimul.cu", "trimul_in_tc.cu", "trimul_out_tc.cu", "contract_tcgen05.cu", "flash_tcgen05.cu", "triatt.cu", "triatt_in_tc.cu", "triatt_out_tc.cu", "pair_bias_tc.cu", "recycle_tc.cu", "transition_tcgen05.cu", "peer.cu", "selftest.cu", "standardise.cu", "opm_tc.cu", "dropout_add.cu", "single_tc.cu", "msa_rows_tc.cu", "msa_transition_tc.cu",
-           "msa_average_tc.cu"]
+           "msa_average_tc.cu", "msa_embed.cu"]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-std=c++17", "-lineinfo",
     "--expt-relaxed-constexpr", "-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=hidden",

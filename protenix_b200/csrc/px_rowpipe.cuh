@@ -431,17 +431,4 @@ __device__ __forceinline__ void rows_out_store(unsigned char* stg, const float (
   __syncwarp();
 }
 
-// Number of SMs of the current device (cached per device ordinal).
-static inline int sm_count() {
-  static int cached[64] = {};
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
-  if (!cached[dev]) {
-    int n = 0;
-    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
-    cached[dev] = n;
-  }
-  return cached[dev];
-}
-
 }  // namespace px

@@ -5,7 +5,7 @@ signature, ``state_dict`` keys).  The work that scales with N^2 -- the outer pro
 (2 * 1024 * S FLOP per pair element) and the 1024 -> 128 output projection with bias, normalisation and the
 residual -- runs in the tcgen05 kernels behind ``px_opm_outer`` / ``px_opm_out``.  What scales with S * N (the
 LayerNorm of the MSA embedding, the two c_m -> 32 projections, the mask and the normalisation counts: a thousandth of
-the FLOPs) is prepared here with the LayerNorm kernel and library GEMMs.  CUDA only; c_hidden = 32 and c_z = 128 are
+the FLOPs) is one pass of ``px_msa_opm_prep``.  CUDA only; c_hidden = 32 and c_z = 128 are
 the compiled shapes; the outer products are formed for blocks of token rows so that their buffer stays within 2 GiB.
 """
 from __future__ import annotations
@@ -75,11 +75,17 @@ class OuterProductMean(nn.Module):
         m, mask, _ = self._msa_input(m, mask)
         return self._run(m, mask, z, z)
 
+    @torch.no_grad()
+    def add_to(self, z: torch.Tensor, m: torch.Tensor, mask: Optional[torch.Tensor] = None) -> torch.Tensor:
+        """z + OuterProductMean(m) as a new tensor, z as in ``apply_``."""
+        m, mask, _ = self._msa_input(m, mask)
+        return self._run(m, mask, z, torch.empty_like(z))
+
 
 class MSAPairWeightedAveraging(nn.Module):
     """Mirror of protenix/model/modules/pairformer.py:343-422.  The pair bias Linear(LayerNorm(z)) (n_heads values per
-    pair element, the only N^2-sized step) runs in ``px_pair_bias_proj``; the rest is S*N-sized work on the LayerNorm
-    kernel and library GEMMs."""
+    pair element) runs in ``px_pair_bias_proj``; the MSAStack below runs the rest in its kernels, and this composition on
+    the LayerNorm kernel and library GEMMs serves the module alone and other widths."""
 
     def __init__(self, c_m: int = 64, c: int = 32, c_z: int = 128, n_heads: int = 8) -> None:
         super().__init__()
@@ -183,16 +189,17 @@ class MSABlock(nn.Module):
     def forward(self, m: torch.Tensor, z: torch.Tensor, pair_mask, triangle_multiplicative: str = "torch",
                 triangle_attention: str = "torch", inplace_safe: bool = False, chunk_size: Optional[int] = None):
         """(m, z) -> (m or None, z).  m [S, N, c_m], z [N, N, c_z] (a leading batch of 1 is accepted for z).  m is
-        updated in place, as the reference's eval path does; z is copied first unless ``inplace_safe``."""
+        updated in place, as the reference's eval path does; z is left as it is unless ``inplace_safe``."""
         batch = z.dim() == 4
         zc = z[0] if batch else z
         if not zc.is_cuda or not m.is_cuda:
             raise RuntimeError("MSABlock: CUDA tensors only (no CPU path)")
         zc = zc.contiguous()
-        if not inplace_safe and zc.data_ptr() == z.data_ptr():
-            zc = zc.clone()
         mm = m[0] if m.dim() == 4 else m
-        self.outer_product_mean_msa.apply_(zc, mm)
+        if inplace_safe or zc.data_ptr() != z.data_ptr():
+            self.outer_product_mean_msa.apply_(zc, mm)
+        else:                           # the first update reads the caller's z and writes the block's own
+            zc = self.outer_product_mean_msa.add_to(zc, mm)
         if not self.is_last_block:
             mm = self.msa_stack(mm, zc)
         _, zc = self.pair_stack(None, zc, pair_mask, inplace_safe=True)
@@ -239,6 +246,20 @@ class MSAModule(nn.Module):
                      pair_dropout=pair_dropout, msa_chunk_size=self.msa_chunk_size, msa_max_size=self.msa_max_size,
                      hidden_scale_up=hidden_scale_up) for i in range(n_blocks))
 
+    def _embed(self, feat, idx: torch.Tensor, s_inputs: torch.Tensor) -> torch.Tensor:
+        """m for the sampled rows of the features (msa, has_deletion, deletion_value)."""
+        msa, w = feat[0], self.linear_no_bias_m.weight
+        s = self.linear_no_bias_s(s_inputs.float())
+        if (msa.is_cuda and msa.dim() == 2 and msa.dtype == torch.int64 and w.dtype == torch.float32 and self.c_m == 64
+                and self.linear_no_bias_m.precision is None and s.dtype == torch.float32 and s.shape == (msa.shape[1], 64)
+                and s.device == msa.device and all(f.device == msa.device and f.shape == msa.shape for f in feat)):
+            return ops.msa_embed(*feat, idx, w, s)
+        feat = [torch.index_select(f, -2, idx) for f in feat]
+        onehot = torch.zeros(*feat[0].shape, 32, dtype=torch.float32, device=msa.device)
+        onehot.scatter_(feat[0].dim(), feat[0].unsqueeze(-1), 1)
+        sample = torch.cat([onehot] + [f.reshape(*onehot.shape[:-1], 1).float() for f in feat[1:]], dim=-1)
+        return self.linear_no_bias_m(sample) + s
+
     @torch.no_grad()
     def forward(self, input_feature_dict: dict, z: torch.Tensor, s_inputs: torch.Tensor, pair_mask: torch.Tensor,
                 triangle_multiplicative: str = "torch", triangle_attention: str = "torch",
@@ -253,12 +274,7 @@ class MSAModule(nn.Module):
         idx = sample_msa_indices(msa.shape[-2], msa.device, self.msa_configs["test_lowerb"], self.msa_configs["strategy"])
         if self.msa_configs["test_cutoff"] > 0:
             idx = idx[:self.msa_configs["test_cutoff"]]
-        feat = {k: torch.index_select(input_feature_dict[k], -2, idx) for k in self.input_feature}
-        onehot = torch.zeros(*feat["msa"].shape, 32, dtype=torch.float32, device=msa.device)
-        onehot.scatter_(feat["msa"].dim(), feat["msa"].unsqueeze(-1), 1)
-        sample = torch.cat([onehot, feat["has_deletion"].reshape(*onehot.shape[:-1], 1).float(),
-                            feat["deletion_value"].reshape(*onehot.shape[:-1], 1).float()], dim=-1)
-        m = self.linear_no_bias_m(sample) + self.linear_no_bias_s(s_inputs.float())
+        m = self._embed([input_feature_dict[k] for k in self.input_feature], idx, s_inputs)
         if m.dim() == 4:
             m = m[0]
         m = m.contiguous()

@@ -221,6 +221,19 @@ def standardise_rows(z: torch.Tensor, eps: float = 1e-5, out: Optional[torch.Ten
     return out
 
 
+def msa_embed(msa, has_deletion, deletion_value, index, w, s_proj) -> torch.Tensor:
+    """m [S', N, 64] = Linear(one_hot(msa) | has_deletion | deletion_value) + s_proj over the rows ``index`` of the features [S, N]."""
+    f32 = lambda t: t.detach().to(torch.float32).contiguous()
+    msa, index = msa.contiguous(), index.contiguous()
+    hd, dv, w, s_proj = f32(has_deletion), f32(deletion_value), f32(w), f32(s_proj)
+    for t, nm in ((msa, "msa"), (hd, "has_deletion"), (dv, "deletion_value"), (index, "index"), (w, "w"), (s_proj, "s_proj")):
+        _need_cuda(t, nm)
+    m = torch.empty(index.numel(), msa.shape[1], 64, dtype=torch.float32, device=msa.device)
+    _launch("px_msa_embed", _lib.load().px_msa_embed, _ptr(msa), _ptr(hd), _ptr(dv), _ptr(index), _ptr(w), _ptr(s_proj), _ptr(m),
+            index.numel(), msa.shape[1], _stream(m))
+    return m
+
+
 def add_update_rows(z: torch.Tensor, upd: torch.Tensor) -> torch.Tensor:
     """z += upd in place for an fp32 tensor [..., 128] and an fp16 update of the same shape."""
     _need_cuda(z, "z")

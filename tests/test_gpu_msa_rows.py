@@ -88,3 +88,15 @@ def test_weighted_average(s, n):
     relf = lambda a: float((a.double() - want).norm() / want.norm())
     assert (wp[..., n:] == 0).all()
     assert relf(got) < 2 * relf(torch.softmax(logits, -1) @ v) + 1e-7
+
+
+@pytest.mark.parametrize("s,n", [(1, 1), (5, 17), (40, 33)])
+def test_embedding(s, n):
+    """px_msa_embed against the linear layer over the concatenated features, for a permuted part of the sequences."""
+    torch.manual_seed(s)
+    msa = torch.randint(0, 32, (s, n), device="cuda")
+    hd, dv = (torch.rand(s, n, device="cuda") for _ in range(2))
+    w, sp = torch.randn(64, 34, device="cuda"), torch.randn(n, 64, device="cuda")
+    idx = torch.randperm(s, device="cuda")[:max(1, s // 2)]
+    x = torch.cat([F.one_hot(msa, 32).double(), hd[..., None].double(), dv[..., None].double()], -1)[idx]
+    torch.testing.assert_close(ops.msa_embed(msa, hd, dv, idx, w, sp).double(), x @ w.double().t() + sp.double(), rtol=1e-6, atol=2e-6)
