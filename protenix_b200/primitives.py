@@ -4,7 +4,8 @@ Mirrors protenix/model/modules/primitives.py:33-101 (``Linear`` / ``LinearNoBias
 :166-230 (``Transition``): same constructor arguments, parameter names and initialisers
 (truncated-normal fan-in scaling; the reference draws from scipy's truncnorm, here torch's
 ``trunc_normal_`` gives the same distribution).  The pair transition (c_in = 128, n = 4) runs
-as one fused kernel; the single-representation transition is a few tiny GEMMs left to torch.
+as one fused kernel; a block's single transition runs in the single-branch kernels, other widths as a composition on
+library GEMMs.
 """
 from __future__ import annotations
 

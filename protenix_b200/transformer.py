@@ -3,8 +3,8 @@
 Parameter names follow protenix/model/modules/transformer.py:40-254 and
 protenix/model/modules/primitives.py:680-760.  The O(N^2 c_z) part -- LayerNorm(z) and the
 128 -> n_heads projection that produces the bias -- runs in ``px_pair_bias_proj``; what is
-left is attention over an [N, c_a] matrix (about 0.2 % of a block's FLOPs), computed in fp32
-with torch's scaled-dot-product attention.
+left is attention over an [N, c_a] matrix (about 0.2 % of a block's FLOPs), computed here in fp32
+with torch's scaled-dot-product attention; a block of the base dimensions runs it in the single-branch kernels instead.
 """
 from __future__ import annotations
 
