@@ -32,7 +32,7 @@
 // fp16, the denominators sum the fp32 values.  Every mbarrier wait is bounded.
 #include <math_constants.h>
 
-#include "px_tcgen05.cuh"
+#include "px_rowpipe.cuh"
 
 namespace px {
 
@@ -102,8 +102,8 @@ __device__ __forceinline__ void exp2_poly2(float x0, float x1, float& p0, float&
 __global__ void __launch_bounds__(kFThreads, 1)
 triatt_flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                        const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_b,
-                       const float* __restrict__ mb,
-                       bf16* __restrict__ o, int n_u, int n, int ldm, int nkt) {
+                       const __grid_constant__ CUtensorMap map_o, const float* __restrict__ mb,
+                       int n_u, int n, int ldm, int nkt) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* sm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   FlashBars& bars = *reinterpret_cast<FlashBars*>(sm + FlashLayout::bars);
@@ -372,26 +372,33 @@ triatt_flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     ok = __all_sync(0xffffffffu, ok);
     if (ok) {
       tc_fence_after();
-      const int qi = q0 + row;
+      // the rows leave by TMA from the place of their queries, which every product has read: a warp's 32 queries of one row are
+      // 2 KB there (64-byte swizzle).  Written by their threads, 16 bytes at 256-byte distances, they took 4 % of the kernel at
+      // N = 384 (135 us against 129) and 1.6 % at N = 1536 (5.89 ms against 5.79).
 #pragma unroll
       for (int r = 0; r < kFRpg; ++r) {
         uint32_t a[32];
         tmem_ld32(t_o + kFON * r, a);
         tmem_wait_ld();
-        if (ug + r < n_u && qi < n) {
-          const float inv = 1.0f / l_sum[r];
-          bf16* dst = o + ((size_t)(ug + r) * n + qi) * kC + h * kFD;
+        unsigned char* tile = sm + FlashLayout::q + (g * kFRpg + r) * kFQBytes;
+        const float inv = 1.0f / l_sum[r];
 #pragma unroll
-          for (int v = 0; v < 4; ++v) {
-            uint4 pk;
-            pk.x = pack_f16x2(__uint_as_float(a[8 * v + 0]) * inv, __uint_as_float(a[8 * v + 1]) * inv);
-            pk.y = pack_f16x2(__uint_as_float(a[8 * v + 2]) * inv, __uint_as_float(a[8 * v + 3]) * inv);
-            pk.z = pack_f16x2(__uint_as_float(a[8 * v + 4]) * inv, __uint_as_float(a[8 * v + 5]) * inv);
-            pk.w = pack_f16x2(__uint_as_float(a[8 * v + 6]) * inv, __uint_as_float(a[8 * v + 7]) * inv);
-            *reinterpret_cast<uint4*>(dst + 8 * v) = pk;
-          }
+        for (int v = 0; v < 4; ++v) {
+          uint4 pk;
+          pk.x = pack_f16x2(__uint_as_float(a[8 * v + 0]) * inv, __uint_as_float(a[8 * v + 1]) * inv);
+          pk.y = pack_f16x2(__uint_as_float(a[8 * v + 2]) * inv, __uint_as_float(a[8 * v + 3]) * inv);
+          pk.z = pack_f16x2(__uint_as_float(a[8 * v + 4]) * inv, __uint_as_float(a[8 * v + 5]) * inv);
+          pk.w = pack_f16x2(__uint_as_float(a[8 * v + 6]) * inv, __uint_as_float(a[8 * v + 7]) * inv);
+          *reinterpret_cast<uint4*>(tile + row * 64 + ((v ^ ((row >> 1) & 3)) << 4)) = pk;
+        }
+        asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+        __syncwarp();
+        if (lane == 0 && ug + r < n_u && q0 + 32 * qw < n) {
+          tma_store_3d(&map_o, smem_u32(tile + 32 * qw * 64), h * kFD, q0 + 32 * qw, ug + r);
+          tma_store_commit();
         }
       }
+      if (lane == 0) tma_store_wait<0>();
     }
   }
 
@@ -421,7 +428,7 @@ extern "C" int32_t px_triatt_flash(const px_f16* q, const px_f16* k, const px_f1
     return PX_ERR_BAD_ARG;
   const int64_t ldt = px_ld(n);
   const int nkt = (int)((n + kFKT - 1) / kFKT);
-  CUtensorMap mq, mk, mv, mbias;
+  CUtensorMap mq, mk, mv, mbias, mo;
   const uint64_t uh = (uint64_t)n_u * kFH;
   // q, k: [n_u*4][n][32] fp16, box [1][128][32], 64-byte swizzle
   if (!make_map_3d(&mq, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, q, kFD, (uint64_t)n, uh, kFD * 2, (uint64_t)n * kFD * 2, kFD,
@@ -433,14 +440,17 @@ extern "C" int32_t px_triatt_flash(const px_f16* q, const px_f16* k, const px_f1
                    (uint64_t)kFD * ldt * 2, 64, kFD, CU_TENSOR_MAP_SWIZZLE_128B) ||
       // pair bias: [4][n q][n k, row stride ldm] fp32, box [1][128][32], 128-byte swizzle
       !make_map_3d(&mbias, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, bias, (uint64_t)n, (uint64_t)n, kFH, (uint64_t)ldm * 4,
-                   (uint64_t)n * ldm * 4, 32, 128, CU_TENSOR_MAP_SWIZZLE_128B))
+                   (uint64_t)n * ldm * 4, 32, 128, CU_TENSOR_MAP_SWIZZLE_128B) ||
+      // o: [n_u][n][128] fp16, box [1][32][32], 64-byte swizzle
+      !make_map_3d(&mo, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, o, kC, (uint64_t)n, (uint64_t)n_u, kC * 2, (uint64_t)n * kC * 2, kFD, 32,
+                   CU_TENSOR_MAP_SWIZZLE_64B))
     return PX_ERR_LAUNCH;
   cudaStream_t st = (cudaStream_t)stream;
   const size_t smem = FlashLayout::total + 1024;
   static SmemLimit limit;
   if (!limit.set(triatt_flash_tc_kernel, smem)) return PX_ERR_LAUNCH;
   dim3 grid((unsigned)((n + 127) / 128), kFH, (unsigned)((n_u + kFRows - 1) / kFRows));
-  return launch_pdl(triatt_flash_tc_kernel, grid, kFThreads, smem, st, mq, mk, mv, mbias, mask_bias, (bf16*)o, (int)n_u, (int)n, (int)ldm, nkt)
+  return launch_pdl(triatt_flash_tc_kernel, grid, kFThreads, smem, st, mq, mk, mv, mbias, mo, mask_bias, (int)n_u, (int)n, (int)ldm, nkt)
              ? PX_OK
              : PX_ERR_LAUNCH;
 }
