@@ -335,7 +335,8 @@ PX_API int32_t px_pair_bias_proj_folded(const void* z, int32_t z_dtype, const vo
  * protenix/model/modules/pairformer.py:181-224.  px_single_prepare lays the fp32 weights (nn.Linear order) out once in a
  * buffer of px_single_weights_bytes(); s and s_out [n][384] of s_dtype (may be the same), q_bias and LayerNorm vectors
  * fp32 [384], pair_bias fp32 [16][n][n].  px_single_project does what needs s alone (q, k, v and gate, left in the workspace of
- * px_single_workspace_bytes(n)), px_single_finish the rest from that workspace. */
+ * px_single_workspace_bytes(n)), px_single_finish the rest from that workspace.  Both may read `prepared` before earlier work of the
+ * stream is complete: synchronise the stream after px_single_prepare. */
 PX_API int64_t px_single_weights_bytes(void);
 PX_API int64_t px_single_workspace_bytes(int64_t n);
 PX_API int32_t px_single_prepare(const float* w_q, const float* w_k, const float* w_v, const float* w_g, const float* w_o,

@@ -129,6 +129,15 @@ split_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
   tc_fence_before();
   const bool skip = __syncthreads_or(stop) != 0;
   tc_fence_after();
+  // the weights of the first stages do not wait for the kernel before this one
+  const int early = g.chunks < kSgStages ? g.chunks : kSgStages;
+  if (threadIdx.x == 0 && !skip) {
+    for (int i = 0; i < early; ++i) {
+      mbar_expect_tx(&bars.full[i], kSgStageBytes);
+      tma_load_3d(smem_u32(ring + i * kSgStageBytes) + kSgABytes, &map_w, &bars.full[i], (kc0 + i) * 64, n0, 0);
+    }
+  }
+  __syncwarp();
   pdl_wait();
   const uint32_t tmem_base = bars.tmem_base;
   float v[kSgBN];                                // epilogue: this thread's row of the tile
@@ -139,10 +148,12 @@ split_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
       for (int i = 0; i < g.chunks; ++i) {
         const int s = i % kSgStages;
         if (!mbar_wait(&bars.empty[s], ((i / kSgStages) & 1) ^ 1, 1u)) break;
-        mbar_expect_tx(&bars.full[s], kSgStageBytes);
         const uint32_t dst = smem_u32(ring + s * kSgStageBytes);
+        if (i >= early) {
+          mbar_expect_tx(&bars.full[s], kSgStageBytes);
+          tma_load_3d(dst + kSgABytes, &map_w, &bars.full[s], (kc0 + i) * 64, n0, 0);
+        }
         tma_load_3d(dst, &map_a, &bars.full[s], (kc0 + i) * 64, m0, 0);
-        tma_load_3d(dst + kSgABytes, &map_w, &bars.full[s], (kc0 + i) * 64, n0, 0);
       }
     }
   } else if (warp <= kSgIssuers) {
