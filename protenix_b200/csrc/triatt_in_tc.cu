@@ -9,7 +9,8 @@
 // work in pairs on the same tiles; CTA parity picks two of the four heads.
 //
 //   warps 0..7    epilogue of q | k: a thread owns one pair element and both heads of q (warps 0..3) or k (4..7):
-//                 64-byte runs per head, coalesced across the warp.
+//                 a warp's 32 rows of a head, 2 KB, are staged (64-byte swizzle) and leave by TMA.  Written by their threads in
+//                 pieces of 16 bytes, half a sector each, they took the kernel from 32 to 42 us at N = 384 and from 119 to 144 at N = 768.
 //   warps 8..15   epilogue of v | bias: v goes through a [64 d][128 t] staging tile and a TMA store (the transpose),
 //                 the two bias values of the row are written directly.
 //   warps 16..19  one thread per row: statistics, correction row, scale pair, mask bias.
@@ -44,7 +45,8 @@ struct AiLayout {
   static constexpr int a = wx1 + 128 * 32;                      // row-tile ring
   static constexpr int ax = a + kTileStages * kTileBytes;
   static constexpr int out = ax + kTileSlots * kTileExtra;      // v staging
-  static constexpr int scale = out + kAiStageOut;               // float2 (rstd, rstd or 0 beyond n) per row and slot
+  static constexpr int qk = out + kAiStageOut;                  // q, k staging: 8 warps x 2 heads x [32 t][32] fp16
+  static constexpr int scale = qk + 8 * 2 * 2048;               // float2 (rstd, rstd or 0 beyond n) per row and slot
   static constexpr int bars = scale + kTileSlots * 128 * 8;
   static constexpr int total = bars + (int)sizeof(AiBars);
 };
@@ -75,9 +77,9 @@ struct AiWeights {
 template <bool kF16>
 __global__ void __launch_bounds__(kAiThreads, 1)
 triatt_in_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_constant__ CUtensorMap map_v,
-                    const float* __restrict__ mask,
-                    const AiWeights<kF16> weights, const unsigned char* __restrict__ folded, bf16* __restrict__ q_out,
-                    bf16* __restrict__ k_out, float* __restrict__ bias_out, float* __restrict__ mb_out, int n_u, int n,
+                    const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k, const float* __restrict__ mask,
+                    const AiWeights<kF16> weights, const unsigned char* __restrict__ folded,
+                    float* __restrict__ bias_out, float* __restrict__ mb_out, int n_u, int n,
                     int ldm, int swap, float eps, float inf, int tiles_t, int n_tiles) {
   constexpr int kAiAcc = kF16 ? 2 : 1;   // accumulators per product: the products of tile k+1 run beside the epilogue of k
   extern __shared__ __align__(1024) unsigned char smem_raw[];
@@ -154,10 +156,10 @@ triatt_in_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_cons
     const int which = warp >> 2, qw = warp & 3;          // 0: q, 1: k
     const int row = 32 * qw + lane;
     const uint32_t t_acc = tmem_base + ((uint32_t)(32 * qw) << 16) + 64 * which;
-    bf16* out = which ? k_out : q_out;
+    unsigned char* stage = sm + AiLayout::qk + warp * 4096;
     int k = 0;
     for (int tile = ctx.first_tile; tile < n_tiles; tile += ctx.tile_step, ++k) {
-      const int u = tile / tiles_t, t = (tile % tiles_t) * 128 + row;
+      const int u = tile / tiles_t, tw = (tile % tiles_t) * 128 + 32 * qw;   // the warp's first row
       const int ab = kAiAcc == 2 ? (k & 1) : 0, an = kAiAcc == 2 ? (k >> 1) : k;
       bool ok = mbar_wait(&bars.acc_full[0][ab], an & 1, 32u);
       ok = __all_sync(0xffffffffu, ok);
@@ -171,23 +173,27 @@ triatt_in_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_cons
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&bars.acc_free[0][ab]);  // this warp has read its part of the accumulator
-      if (t < n) {
-        auto emit = [&](const uint32_t(&v)[32], int head) {
-          uint4* dst = reinterpret_cast<uint4*>(out + (((size_t)u * kAiH + head) * n + t) * kAiD);
+      if (lane == 0) tma_store_wait_read<0>();            // the stores of the tile before have read the staging area
+      __syncwarp();
 #pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            uint4 o;
-            o.x = pack_f16x2(rstd * __uint_as_float(v[8 * j + 0]), rstd * __uint_as_float(v[8 * j + 1]));
-            o.y = pack_f16x2(rstd * __uint_as_float(v[8 * j + 2]), rstd * __uint_as_float(v[8 * j + 3]));
-            o.z = pack_f16x2(rstd * __uint_as_float(v[8 * j + 4]), rstd * __uint_as_float(v[8 * j + 5]));
-            o.w = pack_f16x2(rstd * __uint_as_float(v[8 * j + 6]), rstd * __uint_as_float(v[8 * j + 7]));
-            dst[j] = o;
-          }
-        };
-        emit(h0, 2 * hpair);
-        emit(h1, 2 * hpair + 1);
+      for (int j = 0; j < 8; ++j) {
+        const uint32_t(&v)[32] = j < 4 ? h0 : h1;
+        const int e = 8 * (j & 3);
+        *reinterpret_cast<uint4*>(stage + (j >> 2) * 2048 + lane * 64 + (((j & 3) ^ ((lane >> 1) & 3)) << 4)) =
+            make_uint4(pack_f16x2(rstd * __uint_as_float(v[e]), rstd * __uint_as_float(v[e + 1])),
+                       pack_f16x2(rstd * __uint_as_float(v[e + 2]), rstd * __uint_as_float(v[e + 3])),
+                       pack_f16x2(rstd * __uint_as_float(v[e + 4]), rstd * __uint_as_float(v[e + 5])),
+                       pack_f16x2(rstd * __uint_as_float(v[e + 6]), rstd * __uint_as_float(v[e + 7])));
+      }
+      asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+      __syncwarp();
+      if (lane == 0 && tw < n) {
+        for (int e = 0; e < 2; ++e)
+          tma_store_3d(which ? &map_k : &map_q, smem_u32(stage + e * 2048), 0, tw, u * kAiH + 2 * hpair + e);
+        tma_store_commit();
       }
     }
+    if (lane == 0) tma_store_wait<0>();
   } else {
     // ------------------------------------------------------------------ epilogue of v | bias
     const int half = (warp >> 2) & 1, qw = warp & 3;
@@ -246,7 +252,7 @@ template <bool kF16>
 static int32_t launch_triatt_in(const void* z, const float* mask, const AiWeights<kF16>& weights, const void* folded,
                                 px_f16* q, px_f16* k, px_f16* v, float* bias, float* mask_bias, int64_t n_u,
                                 int64_t n, int64_t ldm, int32_t ending, float eps, float inf, cudaStream_t st) {
-  CUtensorMap mz, mv;
+  CUtensorMap mz, mv, mq, mk;
   const CUtensorMapDataType zt = kF16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
   // pair element (u, t) is row u*n + t of z, or row t*n_u + u when the two indices are exchanged
   const bool ok = ending ? make_map_3d(&mz, zt, z, 128, (uint64_t)n_u, (uint64_t)n, 256, (uint64_t)n_u * 256, 64, 1,
@@ -259,14 +265,19 @@ static int32_t launch_triatt_in(const void* z, const float* mask, const AiWeight
   if (!make_map_3d(&mv, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, v, ldt, (uint64_t)n_u * 128, 1, ldt * 2, ldt * 2 * n_u * 128, 128,
                    64, CU_TENSOR_MAP_SWIZZLE_NONE, 1))
     return PX_ERR_LAUNCH;
+  // q, k: [n_u * 4][n][32], a store writes [32 t][32]
+  for (int i = 0; i < 2; ++i)
+    if (!make_map_3d(i ? &mk : &mq, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, i ? k : q, kAiD, (uint64_t)n, (uint64_t)n_u * kAiH, kAiD * 2,
+                     (uint64_t)n * kAiD * 2, kAiD, 32, CU_TENSOR_MAP_SWIZZLE_64B))
+      return PX_ERR_LAUNCH;
   const size_t smem = AiLayout::total + 1024;
   static SmemLimit limit;
   if (!limit.set(triatt_in_tc_kernel<kF16>, smem)) return PX_ERR_LAUNCH;
   const int64_t tiles_t = (n + 127) / 128, n_tiles = tiles_t * n_u;   // 128-wide tiles cover the pad columns up to ldm
   if (n_tiles > 0x7fffffff) return PX_ERR_UNSUPPORTED;
   const int pairs = (int)(n_tiles < sm_count() / 2 ? n_tiles : sm_count() / 2);
-  return launch_pdl(triatt_in_tc_kernel<kF16>, dim3(2 * pairs), kAiThreads, smem, st, mz, mv, mask, weights, (const unsigned char*)folded,
-                    (bf16*)q, (bf16*)k, bias, mask_bias, (int)n_u, (int)n, (int)ldm, (int)ending, eps, inf, (int)tiles_t,
+  return launch_pdl(triatt_in_tc_kernel<kF16>, dim3(2 * pairs), kAiThreads, smem, st, mz, mv, mq, mk, mask, weights,
+                    (const unsigned char*)folded, bias, mask_bias, (int)n_u, (int)n, (int)ldm, (int)ending, eps, inf, (int)tiles_t,
                     (int)n_tiles)
              ? PX_OK
              : PX_ERR_LAUNCH;
