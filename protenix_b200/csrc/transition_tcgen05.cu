@@ -12,7 +12,8 @@
 //                 H buffer as the A operand of the second product.  The two H buffers alternate.
 //   warps 8..11   LayerNorm: lanes across channels (coalesced), eight rows in flight per warp; the normalised rows
 //                 are written as the K-major, 128-byte-swizzled A operand of the first product (two buffers).
-//   warps 12..15  output: accumulator -> shared staging -> + residual -> coalesced stores (two accumulators).
+//   warps 12..15  output: accumulator -> shared staging -> + residual -> coalesced stores (two accumulators); fp32 rows, unless
+//                 their residual lies in another tensor, leave by TMA, added in L2.
 //   warp 16       TMA producer of the weight chunks: rows 64c..64c+63 of W_a and W_b and columns 64c..64c+63 of
 //                 W_o, 48 KB, 3-stage ring (the weights are re-read from L2 for every tile: 384 KB per 128 rows).
 //   warps 17, 18  MMA issuers: H = A [W_a;W_b]_c^T (M=128, N=128, K=128) and OUT += h W_o,c^T (M=128, N=128, K=64, h
@@ -66,10 +67,10 @@ struct Raw4<float> {
   __device__ __forceinline__ float4 get() const { return v; }
 };
 
-template <typename Tz>
+template <typename Tz, bool kBulk>
 __global__ void __launch_bounds__(kTrThreads, 1)
 transition_tc_kernel(const __grid_constant__ CUtensorMap map_wa, const __grid_constant__ CUtensorMap map_wb,
-                     const __grid_constant__ CUtensorMap map_wo, const Tz* __restrict__ x_in, Tz* __restrict__ x_out,
+                     const __grid_constant__ CUtensorMap map_wo, const __grid_constant__ CUtensorMap map_out, const Tz* __restrict__ x_in, Tz* __restrict__ x_out,
                      const float* __restrict__ ln_w, const float* __restrict__ ln_b, long long rows, int n_tiles,
                      int add_residual, float eps) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
@@ -183,6 +184,35 @@ transition_tc_kernel(const __grid_constant__ CUtensorMap map_wa, const __grid_co
     const int srow = 32 * qw + lane;
     const int rsub = lane >> 3, piece = lane & 7;          // reader: row within a group of 4, 16-byte piece
     int k = 0;
+    if constexpr (kBulk) {
+      // fp32 rows stored, or added in L2 where x_out is x: nothing is read here but the accumulator
+      for (int tile = first_tile; tile < n_tiles; tile += tile_step, ++k) {
+        const int ob = k & 1;
+        bool ok = mbar_wait(&bars.out_full[ob], (k >> 1) & 1, 32u);
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) break;
+        tc_fence_after();
+        const long long first = (long long)tile * 128 + 32 * qw;
+#pragma unroll 1
+        for (int q = 0; q < 4; ++q) {
+          uint32_t r[32];
+          float v[32];
+          tmem_ld32(lane_addr + 256 + 128 * ob + 32 * q, r);
+          tmem_wait_ld();
+          if (q == 3) {                                      // this warp has read its part of the accumulator
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&bars.out_free[ob]);
+          }
+#pragma unroll
+          for (int e = 0; e < 32; ++e) v[e] = 2.0f * __uint_as_float(r[e]);      // the second product is of h / 2
+          if (lane == 0) tma_store_wait_read<0>();           // the block before has left the staging area
+          __syncwarp();
+          rows_bulk_out(stg + qw * 4096, v, &map_out, add_residual != 0, 32 * q, (int)first, 0, first < rows, lane);
+        }
+      }
+      if (lane == 0) tma_store_wait<0>();
+    } else {
     for (int tile = first_tile; tile < n_tiles; tile += tile_step, ++k) {
       const int ob = k & 1;
       const long long row0 = (long long)tile * 128;
@@ -236,6 +266,7 @@ transition_tc_kernel(const __grid_constant__ CUtensorMap map_wa, const __grid_co
         }
         __syncwarp();
       }
+    }
     }
   } else if (warp >= 8) {
     // ------------------------------------------------------------------ LayerNorm -> swizzled A operand
@@ -367,11 +398,12 @@ transition_tc_kernel(const __grid_constant__ CUtensorMap map_wa, const __grid_co
 
 PX_DEFINE_FAMILY_HOOKS(transition)
 
-template <typename Tz>
+// kBulk (fp32 rows): the output goes through TMA, which covers everything but a residual from another tensor.
+template <typename Tz, bool kBulk>
 static int32_t launch_transition(const void* x_in, void* x_out, const float* ln_w, const float* ln_b, const px_bf16* w_a,
                                  const px_bf16* w_b, const px_bf16* w_o, int64_t rows, int32_t add_residual, float eps,
                                  cudaStream_t st) {
-  CUtensorMap ma, mb, mo;
+  CUtensorMap ma, mb, mo, mx = {};
   // W_a, W_b: [512 rows][128 k] fp16, box [64 rows][64 k]; W_o: [128 rows][512 k], box [128 rows][64 k]
   if (!make_map_3d(&ma, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, w_a, 128, 512, 1, 256, 512 * 256, 64, 64,
                    CU_TENSOR_MAP_SWIZZLE_128B) ||
@@ -380,12 +412,15 @@ static int32_t launch_transition(const void* x_in, void* x_out, const float* ln_
       !make_map_3d(&mo, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, w_o, 512, 128, 1, 1024, 128 * 1024, 64, 128,
                    CU_TENSOR_MAP_SWIZZLE_128B))
     return PX_ERR_LAUNCH;
+  if (kBulk && !make_map_3d(&mx, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, x_out, 128, (uint64_t)rows, 1, 512, (uint64_t)rows * 512, 32, 32,
+                            CU_TENSOR_MAP_SWIZZLE_128B))
+    return PX_ERR_LAUNCH;
   const size_t smem = TransLayout::total + 1024;
   static SmemLimit limit;
-  if (!limit.set(transition_tc_kernel<Tz>, smem)) return PX_ERR_LAUNCH;
+  if (!limit.set(transition_tc_kernel<Tz, kBulk>, smem)) return PX_ERR_LAUNCH;
   const int64_t n_tiles = (rows + 127) / 128;
   const int grid = (int)(n_tiles < sm_count() ? n_tiles : sm_count());
-  return launch_pdl(transition_tc_kernel<Tz>, dim3(grid), kTrThreads, smem, st, ma, mb, mo, (const Tz*)x_in, (Tz*)x_out, ln_w, ln_b,
+  return launch_pdl(transition_tc_kernel<Tz, kBulk>, dim3(grid), kTrThreads, smem, st, ma, mb, mo, mx, (const Tz*)x_in, (Tz*)x_out, ln_w, ln_b,
                     (long long)rows, (int)n_tiles, (int)add_residual, eps)
              ? PX_OK
              : PX_ERR_LAUNCH;
@@ -403,8 +438,9 @@ extern "C" int32_t px_transition(const void* x_in, void* x_out, int32_t dtype, c
   if (rows == 0) return PX_OK;
   if ((rows + 127) / 128 > 0x7fffffff) return PX_ERR_UNSUPPORTED;
   if (dtype == PX_F32)
-    return launch_transition<float>(x_in, x_out, ln_w, ln_b, w_a, w_b, w_o, rows, add_residual, eps, (cudaStream_t)stream);
+    return (rows <= 0x7fffffff && !(add_residual && x_in != x_out) ? launch_transition<float, true> : launch_transition<float, false>)(
+        x_in, x_out, ln_w, ln_b, w_a, w_b, w_o, rows, add_residual, eps, (cudaStream_t)stream);
   if (dtype == PX_BF16)
-    return launch_transition<bf16>(x_in, x_out, ln_w, ln_b, w_a, w_b, w_o, rows, add_residual, eps, (cudaStream_t)stream);
+    return launch_transition<bf16, false>(x_in, x_out, ln_w, ln_b, w_a, w_b, w_o, rows, add_residual, eps, (cudaStream_t)stream);
   return PX_ERR_UNSUPPORTED;
 }

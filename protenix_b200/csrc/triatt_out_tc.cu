@@ -1,9 +1,10 @@
 // Triangle attention, stage 3 on the 5th-generation tensor cores:
 //   z_out(u,t) = [z_in(u,t) +] W_o ( o[u][t] * sigmoid(W_g LN(z_in(u,t))) ),
 //   (u,t) = z[u][t] (starting node) or z[t][u] (ending node); z_out may alias z_in.
-// Three forms (kMode): 0 = z stored as bf16 (rows multiplied as stored, output through shared memory and TMA);
+// The forms (kMode): 0 = z stored as bf16 (rows multiplied as stored, output through shared memory and TMA);
 // 1 = z stored as fp32 (the rows arrive as their standardised fp16 copy, residual and output fp32, coalesced through
-// a staging area); 2 = only the standardised fp16 rows are at hand and the update itself is wanted, in fp16, without
+// a staging area), where the residual is another tensor than the output; 3 = the same where it is the output or
+// there is none: the rows leave by TMA, added to z in L2; 2 = only the standardised fp16 rows are at hand and the update itself is wanted, in fp16, without
 // residual (the row-sharded path computes the ending-node update where the columns live and adds it where the rows
 // live, so that 16-bit tensors cross NVLink in both directions).
 //
@@ -17,7 +18,7 @@
 //                 swizzled tile (fp16), o * sigmoid(g) packed to fp16 into tensor memory.
 //   warps 8..15   output: accumulator + residual (the raw z tile still in shared memory), packed to bf16 over the
 //                 o tile in place, which then leaves through a TMA store; the store addresses z[u][t] or z[t][u],
-//                 so the ending node costs nothing extra.  fp32 rows are written with plain stores instead.
+//                 so the ending node costs nothing extra.  fp32 rows by form.
 //   warps 16..19  one thread per row: statistics, correction row, the row's rstd.
 //   warp 20       TMA producer (z and o tiles); warp 21 MMA issuer of the gate product, warp 22 of the output
 //                 product (A operand in tensor memory), warp 23 of the statistics product.
@@ -72,7 +73,8 @@ triatt_out_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_con
                      const __grid_constant__ CUtensorMap map_out, const void* __restrict__ z_in, void* __restrict__ z_out,
                      const AoWeights<kMode != 0> weights, const unsigned char* __restrict__ folded, int n_u, int n, int swap, int add_residual, float eps, int tiles_t,
                      int n_tiles) {
-  constexpr bool kTma = kMode != 1;                      // 16-bit output: packed over the o tile, leaves through TMA
+  constexpr bool kTma = kMode == 0 || kMode == 2;        // 16-bit output: packed over the o tile, leaves through TMA
+  constexpr bool kBulk = kMode == 3;                     // fp32 output: staged, stored or added by TMA
   constexpr bool kF16 = kMode != 0;                      // the z tile is a standardised fp16 copy; o, W_o always fp16
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* sm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -223,7 +225,7 @@ triatt_out_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_con
       const long long row_stride = swap ? n_u : 1;
       const int valid = n - (t0 + 32 * qw) < 32 ? (n - (t0 + 32 * qw) > 0 ? n - (t0 + 32 * qw) : 0) : 32;
       RowsOutReq rq;
-      if (!kTma) {
+      if (!kTma && !kBulk) {
         rows_out_request(rq, reinterpret_cast<const float*>(z_in), first_row, row_stride, valid, 64 * half, lane,
                          add_residual != 0);
         if (add_residual && lane < valid)
@@ -276,6 +278,15 @@ triatt_out_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_con
             }
             *reinterpret_cast<uint4*>(otile + operand_piece_offset(row, piece)) = make_uint4(w[0], w[1], w[2], w[3]);
           }
+        } else if (kBulk) {
+          // fp32 rows: the first block staged in the o tile, the second in the z tile (not its rows of ones), which the gate
+          // warps and the tensor core have finished reading (8 warps x 4 KB each)
+          float v[32];
+#pragma unroll
+          for (int e = 0; e < 32; ++e) v[e] = __uint_as_float(acc[e]);
+          unsigned char* stg = hh == 0 ? otile + (warp & 7) * 4096 : ctx.tiles + s * kTileBytes + half * kTilePanel + qw * 4096;
+          const int tw = t0 + 32 * qw;
+          rows_bulk_out(stg, v, &map_out, add_residual != 0, 64 * half + 32 * hh, swap ? u : tw, swap ? tw : u, tw < n, lane);
         } else {
           // fp32 rows: coalesced through a warp-private staging area inside the o tile, which the gate warps and
           // the tensor core have finished reading (8 warps x 4 KB)
@@ -300,11 +311,12 @@ triatt_out_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_con
           mbar_arrive(&bars.tile.a_empty[s]);
         }
       } else {
+        if (kBulk && lane == 0) tma_store_wait_read<0>();
         named_barrier(1, 256);
         if (leader) mbar_arrive(&bars.tile.a_empty[s]);
       }
     }
-    if (kTma && leader) tma_store_wait<0>();
+    if (kTma ? leader : kBulk && lane == 0) tma_store_wait<0>();
   }
 
   tc_fence_before();
@@ -325,13 +337,19 @@ static int32_t launch_triatt_out(const px_f16* o, const void* z_in, const px_f16
   // operand rows: bf16 z itself, or the standardised fp16 copy of an fp32 z; pair element (u, t) is row u*n + t, or
   // row t*n_u + u when the two indices are exchanged
   const CUtensorMapDataType zt = kMode == 0 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
-  const void* zrows = kMode == 1 ? (const void*)zn : z_in;
+  const void* zrows = kMode == 1 || kMode == 3 ? (const void*)zn : z_in;
   if (!(ending ? make_map_3d(&mz, zt, zrows, 128, (uint64_t)n_u, (uint64_t)n, 256, (uint64_t)n_u * 256, 64, 1,
                              CU_TENSOR_MAP_SWIZZLE_128B, 128)
                : make_map_3d(&mz, zt, zrows, 128, (uint64_t)n, (uint64_t)n_u, 256, (uint64_t)n * 256, 64, 128,
                              CU_TENSOR_MAP_SWIZZLE_128B, 1)))
     return PX_ERR_LAUNCH;
-  if (kMode != 1) {
+  if (kMode == 3) {
+    if (!(ending ? make_map_3d(&mout, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, z_out, 128, (uint64_t)n_u, (uint64_t)n, 512, (uint64_t)n_u * 512, 32,
+                               1, CU_TENSOR_MAP_SWIZZLE_128B, 32)
+                 : make_map_3d(&mout, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, z_out, 128, (uint64_t)n, (uint64_t)n_u, 512, (uint64_t)n * 512, 32,
+                               32, CU_TENSOR_MAP_SWIZZLE_128B, 1)))
+      return PX_ERR_LAUNCH;
+  } else if (kMode != 1) {
     if (!(ending ? make_map_3d(&mout, zt, z_out, 128, (uint64_t)n_u, (uint64_t)n, 256, (uint64_t)n_u * 256, 64, 1,
                                CU_TENSOR_MAP_SWIZZLE_128B, 128)
                  : make_map_3d(&mout, zt, z_out, 128, (uint64_t)n, (uint64_t)n_u, 256, (uint64_t)n * 256, 64, 128,
@@ -365,7 +383,9 @@ static int32_t triatt_out_any(const px_f16* o, const void* z_in, const px_f16* z
   if (z_dtype == PX_F16)   // z_in: standardised fp16 rows; z_out: the update in fp16 (no residual to add)
     return add_residual ? PX_ERR_BAD_ARG
                         : launch_triatt_out<2>(o, z_in, nullptr, z_out, w, folded, n_u, n_t, ending, 0, eps, st);
-  if (z_dtype == PX_F32) return launch_triatt_out<1>(o, z_in, zn, z_out, w, folded, n_u, n_t, ending, add_residual, eps, st);
+  if (z_dtype == PX_F32)
+    return (add_residual && z_in != z_out ? launch_triatt_out<1> : launch_triatt_out<3>)(o, z_in, zn, z_out, w, folded, n_u, n_t, ending,
+                                                                                       add_residual, eps, st);
   if (z_dtype == PX_BF16)
     return launch_triatt_out<0>(o, z_in, nullptr, z_out, AoWeights<false>{w.ln_w, w.ln_b, w.w_g, w.w_o}, folded, n_u, n_t, ending,
                                 add_residual, eps, st);

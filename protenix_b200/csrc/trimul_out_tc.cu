@@ -15,7 +15,8 @@
 //
 //   warps 0..15   epilogue: a thread owns one pair element and 32 channels: p * sigmoid(g) + residual (the raw z
 //                 tile in shared memory), packed to bf16 over the z tile in place, which leaves through a TMA store.
-//                 fp32 rows are written with plain stores instead.
+//                 fp32 rows are staged the same way and stored or added by TMA; where the residual lies in another tensor, it
+//                 is read and the rows are written with plain accesses.
 //   warps 16..19  one thread per row: both sets of statistics, the correction row, the scale pair.
 //   warp 20       TMA producer (z and x tiles); warps 21, 22 MMA issuers of the gate and of the projection product,
 //                 warp 23 of the two statistics products.
@@ -80,7 +81,7 @@ struct ToWeights {
   }
 };
 
-template <typename Tz>
+template <typename Tz, bool kBulk>
 __global__ void __launch_bounds__(kToThreads, 1)
 trimul_out_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_constant__ CUtensorMap map_x,
                      const __grid_constant__ CUtensorMap map_out, const Tz* __restrict__ z_in, Tz* __restrict__ z_out,
@@ -263,7 +264,7 @@ trimul_out_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_con
       const int s = k % kToStages;
       const int i = tile / tiles_j, j0 = (tile % tiles_j) * 128;
       RowsOutReq rq;
-      if (!kTma) {                                         // the residual values are requested before the wait
+      if (!kTma && !kBulk) {                               // the residual values are requested before the wait
         const int valid = n - (j0 + 32 * qw) < 32 ? (n - (j0 + 32 * qw) > 0 ? n - (j0 + 32 * qw) : 0) : 32;
         rows_out_request(rq, reinterpret_cast<const float*>(z_in), (long long)i * n + j0 + 32 * qw, 1, valid, 32 * part, lane,
                          add_residual != 0);
@@ -322,6 +323,13 @@ trimul_out_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_con
           tma_store_wait_read<0>();                          // the store has read the stage: hand it back
           mbar_arrive(&bars.a_empty[s]);
         }
+      } else if (kBulk) {
+        // fp32 rows: staged inside the stage's tiles, which the tensor core has finished reading (16 warps x 4 KB)
+        unsigned char* stg = sm + (warp < 8 ? ToLayout::zt : ToLayout::xt) + s * kOperandBytes + (warp & 7) * 4096;
+        rows_bulk_out(stg, v, &map_out, add_residual != 0, 32 * part, j0 + 32 * qw, i, j0 + 32 * qw < n, lane);
+        if (lane == 0) tma_store_wait_read<0>();
+        named_barrier(1, 512);
+        if (leader) mbar_arrive(&bars.a_empty[s]);
       } else {
         // fp32 rows: coalesced through a warp-private staging area inside the stage's tiles, which the tensor core
         // has finished reading (16 warps x 4 KB = the z tile and the x tile)
@@ -332,7 +340,7 @@ trimul_out_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_con
         if (leader) mbar_arrive(&bars.a_empty[s]);
       }
     }
-    if (kTma && leader) tma_store_wait<0>();
+    if (kTma ? leader : kBulk && lane == 0) tma_store_wait<0>();
   }
 
   tc_fence_before();
@@ -345,7 +353,8 @@ trimul_out_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_con
 
 PX_DEFINE_FAMILY_HOOKS(trimul_out)
 
-template <typename Tz>
+// kBulk (fp32 z): the output goes through TMA, which covers everything but a residual from another tensor.
+template <typename Tz, bool kBulk>
 static int32_t launch_trimul_out(const px_f16* x, const void* z_in, const px_f16* zn, void* z_out,
                                  const ToWeights<sizeof(Tz) != 2>& weights, const void* folded,
                                  int64_t n_i, int64_t n, int64_t ld, int32_t add_residual, float eps, cudaStream_t st) {
@@ -359,6 +368,10 @@ static int32_t launch_trimul_out(const px_f16* x, const void* z_in, const px_f16
     if (!make_map_3d(&mout, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, z_out, 128, (uint64_t)n, (uint64_t)n_i, 256, (uint64_t)n * 256,
                      64, 128, CU_TENSOR_MAP_SWIZZLE_128B, 1))
       return PX_ERR_LAUNCH;
+  } else if (kBulk) {
+    if (!make_map_3d(&mout, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, z_out, 128, (uint64_t)n, (uint64_t)n_i, 512, (uint64_t)n * 512, 32, 32,
+                     CU_TENSOR_MAP_SWIZZLE_128B, 1))
+      return PX_ERR_LAUNCH;
   } else {
     memset(&mout, 0, sizeof(mout));
   }
@@ -368,11 +381,11 @@ static int32_t launch_trimul_out(const px_f16* x, const void* z_in, const px_f16
     return PX_ERR_LAUNCH;
   const size_t smem = ToLayout::total + 1024;
   static SmemLimit limit;
-  if (!limit.set(trimul_out_tc_kernel<Tz>, smem)) return PX_ERR_LAUNCH;
+  if (!limit.set(trimul_out_tc_kernel<Tz, kBulk>, smem)) return PX_ERR_LAUNCH;
   const int64_t tiles_j = (n + 127) / 128, n_tiles = tiles_j * n_i;
   if (n_tiles > 0x7fffffff) return PX_ERR_UNSUPPORTED;
   const int grid = (int)(n_tiles < sm_count() ? n_tiles : sm_count());
-  return launch_pdl(trimul_out_tc_kernel<Tz>, dim3(grid), kToThreads, smem, st, mz, mx, mout, (const Tz*)z_in, (Tz*)z_out, weights,
+  return launch_pdl(trimul_out_tc_kernel<Tz, kBulk>, dim3(grid), kToThreads, smem, st, mz, mx, mout, (const Tz*)z_in, (Tz*)z_out, weights,
                     (const unsigned char*)folded, (int)n_i, (int)n, (int)add_residual, eps, (int)tiles_j, (int)n_tiles)
              ? PX_OK
              : PX_ERR_LAUNCH;
@@ -417,9 +430,9 @@ extern "C" int32_t px_trimul_out_folded(const px_f16* x, const void* z_in, const
   if (!trimul_out_args_ok(x, z_in, zn, z_out, z_dtype, n_i, n_j, ld) || !folded || ((uintptr_t)folded & 15)) return PX_ERR_BAD_ARG;
   cudaStream_t st = (cudaStream_t)stream;
   if (z_dtype == PX_F32)
-    return launch_trimul_out<float>(x, z_in, zn, z_out, ToWeights<true>{}, folded, n_i, n_j, ld, add_residual, eps, st);
+    return (add_residual && z_in != z_out ? launch_trimul_out<float, false> : launch_trimul_out<float, true>)(x, z_in, zn, z_out, ToWeights<true>{}, folded, n_i, n_j, ld, add_residual, eps, st);
   if (z_dtype == PX_BF16)
-    return launch_trimul_out<bf16>(x, z_in, nullptr, z_out, ToWeights<false>{}, folded, n_i, n_j, ld, add_residual, eps, st);
+    return launch_trimul_out<bf16, false>(x, z_in, nullptr, z_out, ToWeights<false>{}, folded, n_i, n_j, ld, add_residual, eps, st);
   return PX_ERR_UNSUPPORTED;
 }
 
@@ -431,10 +444,10 @@ extern "C" int32_t px_trimul_out(const px_f16* x, const void* z_in, const px_f16
     return PX_ERR_BAD_ARG;
   cudaStream_t st = (cudaStream_t)stream;
   if (z_dtype == PX_F32)
-    return launch_trimul_out<float>(x, z_in, zn, z_out, to_weights<true>(ln_in_w, ln_in_b, ln_out_w, ln_out_b, w_z, w_g), nullptr, n_i,
+    return (add_residual && z_in != z_out ? launch_trimul_out<float, false> : launch_trimul_out<float, true>)(x, z_in, zn, z_out, to_weights<true>(ln_in_w, ln_in_b, ln_out_w, ln_out_b, w_z, w_g), nullptr, n_i,
                                     n_j, ld, add_residual, eps, st);
   if (z_dtype == PX_BF16)
-    return launch_trimul_out<bf16>(x, z_in, nullptr, z_out, to_weights<false>(ln_in_w, ln_in_b, ln_out_w, ln_out_b, w_z, w_g), nullptr,
+    return launch_trimul_out<bf16, false>(x, z_in, nullptr, z_out, to_weights<false>(ln_in_w, ln_in_b, ln_out_w, ln_out_b, w_z, w_g), nullptr,
                                    n_i, n_j, ld, add_residual, eps, st);
   return PX_ERR_UNSUPPORTED;
 }
