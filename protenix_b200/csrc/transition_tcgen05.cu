@@ -185,7 +185,7 @@ transition_tc_kernel(const __grid_constant__ CUtensorMap map_wa, const __grid_co
     const int rsub = lane >> 3, piece = lane & 7;          // reader: row within a group of 4, 16-byte piece
     int k = 0;
     if constexpr (kBulk) {
-      // fp32 rows stored, or added in L2 where x_out is x: nothing is read here but the accumulator
+      // rows stored, or added in L2 where x_out is x: nothing is read here but the accumulator
       for (int tile = first_tile; tile < n_tiles; tile += tile_step, ++k) {
         const int ob = k & 1;
         bool ok = mbar_wait(&bars.out_full[ob], (k >> 1) & 1, 32u);
@@ -193,22 +193,54 @@ transition_tc_kernel(const __grid_constant__ CUtensorMap map_wa, const __grid_co
         if (!ok) break;
         tc_fence_after();
         const long long first = (long long)tile * 128 + 32 * qw;
+        if constexpr (sizeof(Tz) == 4) {
 #pragma unroll 1
-        for (int q = 0; q < 4; ++q) {
-          uint32_t r[32];
-          float v[32];
-          tmem_ld32(lane_addr + 256 + 128 * ob + 32 * q, r);
-          tmem_wait_ld();
-          if (q == 3) {                                      // this warp has read its part of the accumulator
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&bars.out_free[ob]);
-          }
+          for (int q = 0; q < 4; ++q) {
+            uint32_t r[32];
+            float v[32];
+            tmem_ld32(lane_addr + 256 + 128 * ob + 32 * q, r);
+            tmem_wait_ld();
+            if (q == 3) {                                      // this warp has read its part of the accumulator
+              tc_fence_before();
+              __syncwarp();
+              if (lane == 0) mbar_arrive(&bars.out_free[ob]);
+            }
 #pragma unroll
-          for (int e = 0; e < 32; ++e) v[e] = 2.0f * __uint_as_float(r[e]);      // the second product is of h / 2
-          if (lane == 0) tma_store_wait_read<0>();           // the block before has left the staging area
-          __syncwarp();
-          rows_bulk_out(stg + qw * 4096, v, &map_out, add_residual != 0, 32 * q, (int)first, 0, first < rows, lane);
+            for (int e = 0; e < 32; ++e) v[e] = 2.0f * __uint_as_float(r[e]);      // the second product is of h / 2
+            if (lane == 0) tma_store_wait_read<0>();           // the block before has left the staging area
+            __syncwarp();
+            rows_bulk_out(stg + qw * 4096, v, &map_out, add_residual != 0, 32 * q, (int)first, 0, first < rows, lane);
+          }
+        } else {
+#pragma unroll 1
+          for (int q = 0; q < 2; ++q) {                      // 64 channels: rows of 128 bytes
+            uint32_t w[32];
+#pragma unroll
+            for (int hh = 0; hh < 2; ++hh) {
+              uint32_t r[32];
+              tmem_ld32(lane_addr + 256 + 128 * ob + 64 * q + 32 * hh, r);
+              tmem_wait_ld();
+#pragma unroll
+              for (int e = 0; e < 16; ++e) w[16 * hh + e] = pack_bf16x2(2.0f * __uint_as_float(r[2 * e]), 2.0f * __uint_as_float(r[2 * e + 1]));
+            }
+            if (q == 1) {
+              tc_fence_before();
+              __syncwarp();
+              if (lane == 0) mbar_arrive(&bars.out_free[ob]);
+            }
+            if (lane == 0) tma_store_wait_read<0>();
+            __syncwarp();
+            unsigned char* row = stg + qw * 4096 + lane * 128;
+#pragma unroll
+            for (int c = 0; c < 8; ++c)
+              *reinterpret_cast<uint4*>(row + ((c ^ (lane & 7)) << 4)) = make_uint4(w[4 * c], w[4 * c + 1], w[4 * c + 2], w[4 * c + 3]);
+            asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+            __syncwarp();
+            if (lane == 0 && first < rows) {
+              tma_store_3d(&map_out, smem_u32(stg + qw * 4096), 64 * q, (int)first, 0);
+              tma_store_commit();
+            }
+          }
         }
       }
       if (lane == 0) tma_store_wait<0>();
@@ -398,7 +430,8 @@ transition_tc_kernel(const __grid_constant__ CUtensorMap map_wa, const __grid_co
 
 PX_DEFINE_FAMILY_HOOKS(transition)
 
-// kBulk (fp32 rows): the output goes through TMA, which covers everything but a residual from another tensor.
+// kBulk: the output goes through TMA, which covers what has no residual and, for fp32 rows, a residual that is the output itself
+// (added in 16 bits it would round twice).
 template <typename Tz, bool kBulk>
 static int32_t launch_transition(const void* x_in, void* x_out, const float* ln_w, const float* ln_b, const px_bf16* w_a,
                                  const px_bf16* w_b, const px_bf16* w_o, int64_t rows, int32_t add_residual, float eps,
@@ -412,8 +445,9 @@ static int32_t launch_transition(const void* x_in, void* x_out, const float* ln_
       !make_map_3d(&mo, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, w_o, 512, 128, 1, 1024, 128 * 1024, 64, 128,
                    CU_TENSOR_MAP_SWIZZLE_128B))
     return PX_ERR_LAUNCH;
-  if (kBulk && !make_map_3d(&mx, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, x_out, 128, (uint64_t)rows, 1, 512, (uint64_t)rows * 512, 32, 32,
-                            CU_TENSOR_MAP_SWIZZLE_128B))
+  constexpr uint64_t kRow = 128 * sizeof(Tz);
+  if (kBulk && !make_map_3d(&mx, sizeof(Tz) == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, x_out, 128,
+                            (uint64_t)rows, 1, kRow, (uint64_t)rows * kRow, 128 / sizeof(Tz), 32, CU_TENSOR_MAP_SWIZZLE_128B))
     return PX_ERR_LAUNCH;
   const size_t smem = TransLayout::total + 1024;
   static SmemLimit limit;
@@ -441,6 +475,7 @@ extern "C" int32_t px_transition(const void* x_in, void* x_out, int32_t dtype, c
     return (rows <= 0x7fffffff && !(add_residual && x_in != x_out) ? launch_transition<float, true> : launch_transition<float, false>)(
         x_in, x_out, ln_w, ln_b, w_a, w_b, w_o, rows, add_residual, eps, (cudaStream_t)stream);
   if (dtype == PX_BF16)
-    return launch_transition<bf16, false>(x_in, x_out, ln_w, ln_b, w_a, w_b, w_o, rows, add_residual, eps, (cudaStream_t)stream);
+    return (rows <= 0x7fffffff && !add_residual ? launch_transition<bf16, true> : launch_transition<bf16, false>)(
+        x_in, x_out, ln_w, ln_b, w_a, w_b, w_o, rows, add_residual, eps, (cudaStream_t)stream);
   return PX_ERR_UNSUPPORTED;
 }

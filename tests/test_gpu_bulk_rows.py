@@ -37,3 +37,19 @@ def test_stored_added_and_plain_rows_agree(n):
             ops.device_error_flags()
             assert torch.equal(added, plain), name
             assert torch.equal(z + update, plain), name
+
+
+@pytest.mark.parametrize("rows", [1, 31, 128, 129, 1000])
+def test_bf16_transition_without_residual(rows):
+    """bf16 rows stored by TMA against the plain accesses, which add the residual before they round."""
+    torch.manual_seed(rows)
+    x = torch.randn(rows, 128, device="cuda").bfloat16()
+    tr = randomize_parameters_(px.Transition(c_in=128, n=4), 5).cuda().eval()
+    update, zero, fp32 = torch.full_like(x, float("nan")), torch.empty_like(x), torch.empty(rows, 128, device="cuda")
+    with torch.no_grad():
+        ops.transition(x, update, *tr._weights(), add_residual=False)
+        ops.transition(x, zero, *tr._weights(), add_residual=True)
+        ops.transition(x.float(), fp32, *tr._weights(), add_residual=False)
+    ops.device_error_flags()
+    assert torch.equal(update, fp32.bfloat16())
+    assert torch.equal(zero, (x.float() + fp32).bfloat16())
