@@ -95,17 +95,6 @@ __device__ __forceinline__ float4 load4(const bf16* p) {
   float2 a = unpack_bf16x2(u.x), b = unpack_bf16x2(u.y);
   return make_float4(a.x, a.y, b.x, b.y);
 }
-__device__ __forceinline__ float2 load2(const float* p) { return *reinterpret_cast<const float2*>(p); }
-__device__ __forceinline__ float2 load2(const bf16* p) {
-  return unpack_bf16x2(*reinterpret_cast<const uint32_t*>(p));
-}
-__device__ __forceinline__ void store2(float* p, float a, float b) {
-  *reinterpret_cast<float2*>(p) = make_float2(a, b);
-}
-__device__ __forceinline__ void store2(bf16* p, float a, float b) {
-  *reinterpret_cast<uint32_t*>(p) = pack_bf16x2(a, b);
-}
-
 
 // Programmatic dependent launch: a kernel launched with launch_pdl may start while the one before it drains, and waits here,
 // before it touches anything that earlier kernels wrote or read, until those are complete.  Its launch, barrier set-up,

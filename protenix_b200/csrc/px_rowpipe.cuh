@@ -65,9 +65,6 @@ __device__ __forceinline__ void write_correction_row(unsigned char* panel, int r
   if (zero_other) *reinterpret_cast<uint4*>(panel + r * 32 + ((sw ^ 1) << 4)) = make_uint4(0u, 0u, 0u, 0u);
 }
 
-// Rounds to bf16 and stores two bytes.
-__device__ __forceinline__ void store_bf16_int(bf16* p, float v) { *p = __float2bfloat16_rn(v); }
-
 // 16-bit weight values -> fp32 (`kF16`: the weights are fp16, otherwise bf16).
 template <bool kF16>
 __device__ __forceinline__ float4 load4_w16(const uint16_t* p) {
