@@ -17,8 +17,10 @@
 #include <ATen/ops/full.h>
 #include <ATen/ops/mm.h>
 #include <ATen/ops/ones.h>
+#include <c10/cuda/CUDAException.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
+#include <c10/util/SmallVector.h>
 #include <dlfcn.h>
 #include <torch/csrc/autograd/custom_function.h>
 #include <torch/csrc/autograd/python_variable.h>
@@ -152,13 +154,75 @@ const float* fptr(const Tensor& t) { return t.defined() ? (const float*)t.data_p
 // kPlain nothing more.
 enum Group { kPlain, kMul, kAtt, kBias, kSingle, kMsa, kOpm };
 struct Prepared {
-  std::vector<Tensor> t[2];          // by format of z: 0 fp32, 1 bf16
+  std::vector<Tensor> t[2];          // by format of z: 0 fp32, 1 bf16; complete, and no aliases of the parameters
   std::vector<const void*> p[2];
   std::vector<float> scalars;
-  at::cuda::CUDAEvent ready[2];
-  cudaStream_t made_on[2] = {nullptr, nullptr};
   bool have[2] = {false, false};
 };
+typedef std::shared_ptr<const Prepared> Ready;
+
+// Where a call runs: the device, its current stream, and the graph that this stream is being captured into, if any.
+struct Use {
+  at::Device dev;
+  c10::cuda::CUDAStream stream;
+  cudaGraph_t graph = nullptr;
+  explicit Use(const at::Device& d) : dev(d), stream(at::cuda::getCurrentCUDAStream(d.index())) {
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    cudaGraph_t g = nullptr;
+    if (cudaStreamGetCaptureInfo(stream, &status, nullptr, &g, nullptr, nullptr) != cudaSuccess) {
+      cudaGetLastError();            // the legacy stream beside somebody else's capture: not being captured itself
+      return;
+    }
+    if (status == cudaStreamCaptureStatusActive) graph = g;
+  }
+};
+
+// A graph launches the kernels of its capture with the addresses of that time, however often the weights have been laid out
+// anew since: it holds the set it was captured with until it is destroyed.  The graph lets go of it on a thread of the driver that may
+// not call CUDA, so the set waits in a list and is freed by the next call that looks up weights (the list outlives the process'
+// other objects: it is never destroyed).
+class GraphHeld {
+ public:
+  static void keep(cudaGraph_t graph, const Ready& set) {
+    Ready* const box = new Ready(set);
+    cudaUserObject_t object;
+    if (cudaUserObjectCreate(&object, box, &GraphHeld::let_go, 1, cudaUserObjectNoDestructorSync) != cudaSuccess) {
+      cudaGetLastError();
+      delete box;
+      fail("the graph cannot hold the weights of its capture");
+    }
+    if (cudaGraphRetainUserObject(graph, object, 1, cudaGraphUserObjectMove) != cudaSuccess) {
+      cudaGetLastError();
+      cudaUserObjectRelease(object, 1);
+      fail("the graph cannot hold the weights of its capture");
+    }
+  }
+  static void free_released() {
+    if (!any_.load(std::memory_order_acquire)) return;
+    std::vector<Ready*> now;
+    {
+      std::lock_guard<std::mutex> lock(mutex_);
+      now.swap(list());
+      any_ = false;
+    }
+    for (Ready* r : now) delete r;
+  }
+
+ private:
+  static void CUDART_CB let_go(void* box) {
+    std::lock_guard<std::mutex> lock(mutex_);
+    list().push_back((Ready*)box);
+    any_.store(true, std::memory_order_release);
+  }
+  static std::vector<Ready*>& list() {
+    static auto* const l = new std::vector<Ready*>;
+    return *l;
+  }
+  static std::mutex mutex_;
+  static std::atomic<bool> any_;
+};
+std::mutex GraphHeld::mutex_;
+std::atomic<bool> GraphHeld::any_{false};
 
 class Params {
  public:
@@ -193,41 +257,38 @@ class Params {
     return true;
   }
 
-  // The kernels' forms of the parameters for z of format zf; needs the GIL.
-  std::shared_ptr<const Prepared> get(int zf, const at::Device& dev) {
+  // The kernels' forms of the parameters for z of format zf; needs the GIL.  What it returns is complete: the host has waited for
+  // it, so every stream may use it.  Inside a capture nothing can be laid out, since the graph's replays alone would write it.
+  Ready get(int zf, const Use& use) {
+    GraphHeld::free_released();
     bool same = prepared_ != nullptr;
-    seen_.resize(params_.size());
+    c10::SmallVector<Seen, 16> now(params_.size());
     for (size_t i = 0; i < params_.size(); ++i) {
       PyObject* o = find(params_[i]);
-      Seen now;
       if (o != Py_None) {
         if (!THPVariable_Check(o)) fail("a module parameter is not a tensor");
         const Tensor& t = THPVariable_Unpack(o);
-        now = {o, t.data_ptr(), (uint32_t)t._version(), t.scalar_type()};
+        now[i] = {o, t.data_ptr(), (uint32_t)t._version(), t.scalar_type()};
       }
-      if (!(now == seen_[i])) {
-        same = false;
-        seen_[i] = now;
-      }
+      same = same && now[i] == seen_[i];
     }
-    if (!same) {
+    c10::SmallVector<float, 4> scalars;
+    for (const auto& s : scalars_) {
+      scalars.push_back((float)PyFloat_AsDouble(find(s)));
+      same = same && prepared_->scalars[scalars.size() - 1] == scalars.back();
+    }
+    if (use.graph && !(same && prepared_->have[zf]))
+      fail("the weights are new to this module, or have changed, and cannot be laid out inside a graph capture: call the module once "
+           "with inputs of this type before capturing");
+    if (!same) {                     // calls in flight hold the set they were given
       prepared_ = std::make_shared<Prepared>();
+      prepared_->scalars.assign(scalars.begin(), scalars.end());
+      seen_.assign(now.begin(), now.end());
       params_hold_.clear();
       for (auto& s : params_) params_hold_.push_back(py::reinterpret_borrow<py::object>(find(s)));
     }
-    for (size_t i = 0; i < scalars_.size(); ++i) {
-      const float v = (float)PyFloat_AsDouble(find(scalars_[i]));
-      if (prepared_->scalars.size() <= i) prepared_->scalars.push_back(v);
-      if (prepared_->scalars[i] != v) {        // another value than the one calls in flight may hold
-        auto next = std::make_shared<Prepared>();
-        next->scalars = prepared_->scalars;
-        next->scalars[i] = v;
-        prepared_ = next;
-      }
-    }
-    if (!prepared_->have[zf]) make(*prepared_, zf, dev);
-    const cudaStream_t st = at::cuda::getCurrentCUDAStream(dev.index());
-    if (prepared_->made_on[zf] != st && !prepared_->ready[zf].query()) prepared_->ready[zf].block(at::cuda::getCurrentCUDAStream(dev.index()));
+    if (!prepared_->have[zf]) make(*prepared_, zf, use);
+    if (use.graph) GraphHeld::keep(use.graph, prepared_);
     return prepared_;
   }
 
@@ -250,8 +311,9 @@ class Params {
     return o ? o : Py_None;
   }
 
-  void make(Prepared& p, int zf, const at::Device& dev) {
+  void make(Prepared& p, int zf, const Use& use) {
     at::NoGradGuard no_grad;
+    const at::Device& dev = use.dev;
     std::vector<Tensor> t;
     for (size_t i = 0; i < params_.size(); ++i) {
       PyObject* o = find(params_[i]);
@@ -270,8 +332,7 @@ class Params {
       }
       t.push_back(v);
     }
-    const auto stream = at::cuda::getCurrentCUDAStream(dev.index());
-    const cudaStream_t st = stream;
+    const cudaStream_t st = use.stream;
     const int rows = zf == 1 ? PX_BF16 : PX_F16;
     const auto byte = at::TensorOptions().device(dev).dtype(at::kByte);
     auto f = [&](int i) { return t[i].defined() ? (const float*)t[i].data_ptr() : nullptr; };
@@ -321,16 +382,18 @@ class Params {
     } else if (group_ == kOpm) {
       t[2] = msa_rows(t[2], t[3]);
     }
+    for (Tensor& v : t)              // a set of its own: what a graph reads outlives the parameters, and the whole set changes at once
+      for (const auto& o : params_hold_)
+        if (v.defined() && !o.is_none() && v.is_alias_of(THPVariable_Unpack(o.ptr()))) {
+          v = v.clone();
+          break;
+        }
     p.t[zf] = t;
     p.p[zf].clear();
     for (const Tensor& v : t) p.p[zf].push_back(v.defined() ? v.data_ptr() : nullptr);
-    // The row kernels fetch folded weights before the kernels in front of them are complete (programmatic launch): once per
-    // change of the weights, the host waits for the fold.
-    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
-    cudaStreamIsCapturing(st, &capturing);
-    if (capturing == cudaStreamCaptureStatusNone) cudaStreamSynchronize(st);
-    p.made_on[zf] = at::cuda::getCurrentCUDAStream(dev.index());
-    p.ready[zf].record(at::cuda::getCurrentCUDAStream(dev.index()));
+    // The row kernels fetch folded weights before the kernels in front of them are complete (programmatic launch), and other
+    // streams use the set too: once per change of the weights, the host waits for it.
+    C10_CUDA_CHECK(cudaStreamSynchronize(st));
     p.have[zf] = true;
   }
 
@@ -342,7 +405,6 @@ class Params {
   std::vector<py::object> params_hold_;      // the parameter objects seen last: their addresses cannot be reused
   std::shared_ptr<Prepared> prepared_;
 };
-typedef std::shared_ptr<const Prepared> Ready;
 
 int64_t al(int64_t n) { return (n + 255) / 256 * 256; }
 int zformat(const Tensor& z) { return z.scalar_type() == at::kBFloat16 ? 1 : 0; }
@@ -432,7 +494,7 @@ Tensor tri_mul_forward(Params& params, const Tensor& z, const OptTensor& mask, b
   c10::cuda::CUDAGuard guard(zc.device());
   at::NoGradGuard no_grad;
   const Tensor m = pair_mask(mask, zc);
-  const Ready pr = params.get(zformat(zc), zc.device());
+  const Ready pr = params.get(zformat(zc), Use(zc.device()));
   py::gil_scoped_release release;
   const Tensor out = inplace_add && zc.data_ptr() == z.data_ptr() ? zc : at::empty_like(zc);
   const Tensor ws = bytes_like(zc, abi.px_trimul_workspace_bytes(zc.size(0)));
@@ -448,7 +510,7 @@ Tensor tri_att_forward(Params& params, const Tensor& z, const OptTensor& mask, b
   c10::cuda::CUDAGuard guard(zc.device());
   at::NoGradGuard no_grad;
   const Tensor m = pair_mask(mask, zc);
-  const Ready pr = params.get(zformat(zc), zc.device());
+  const Ready pr = params.get(zformat(zc), Use(zc.device()));
   py::gil_scoped_release release;
   const Tensor out = at::empty_like(zc);
   const Tensor ws = bytes_like(zc, abi.px_triatt_workspace_bytes(zc.size(0)));
@@ -464,7 +526,7 @@ Tensor transition_forward(Params& params, const Tensor& x) {
   c10::cuda::CUDAGuard guard(x.device());
   at::NoGradGuard no_grad;
   const Tensor xc = x.contiguous();
-  const Ready pr = params.get(zformat(xc), xc.device());
+  const Ready pr = params.get(zformat(xc), Use(xc.device()));
   py::gil_scoped_release release;
   const Tensor out = at::empty_like(xc);
   transition_rows(at::cuda::getCurrentCUDAStream(), *pr, zformat(xc), dtype_code(xc, "x"), xc.data_ptr(), out.data_ptr(),
@@ -503,13 +565,16 @@ void single_finish(cudaStream_t st, const Prepared& pr, int zf, const Tensor& s_
   });
 }
 
-c10::cuda::CUDAStream side_stream(c10::DeviceIndex dev) {
+// One side stream per device for plain calls and one for captures: work of another thread's plain call must not meet a stream that is
+// being captured.
+c10::cuda::CUDAStream side_stream(const Use& use) {
   static std::mutex mutex;
   static std::vector<c10::optional<c10::cuda::CUDAStream>> streams;
+  const size_t i = 2 * (size_t)use.dev.index() + (use.graph ? 1 : 0);
   std::lock_guard<std::mutex> lock(mutex);
-  if ((size_t)dev >= streams.size()) streams.resize(dev + 1);
-  if (!streams[dev]) streams[dev] = c10::cuda::getStreamFromPool(false, dev);
-  return *streams[dev];
+  if (i >= streams.size()) streams.resize(i + 1);
+  if (!streams[i]) streams[i] = c10::cuda::getStreamFromPool(false, use.dev.index());
+  return *streams[i];
 }
 
 // The blocks one after the other.  The pair path never reads s, and the single branch takes nothing from z but the pair
@@ -532,13 +597,13 @@ std::tuple<OptTensor, Tensor> stack_forward(const std::vector<std::shared_ptr<Bl
   const int64_t n = zi.size(0);
   Tensor s = s_in.has_value() ? *s_in : Tensor();
   bool singles = false;
+  const Use use(zi.device());
   std::vector<BlockReady> ready;
   for (const auto& b : blocks) {
-    const auto dev = zi.device();
-    BlockReady r{b->mul_out->get(zf, dev), b->mul_in->get(zf, dev), b->att_start->get(zf, dev), b->att_end->get(zf, dev),
-                 b->transition->get(zf, dev), nullptr, nullptr};
+    BlockReady r{b->mul_out->get(zf, use), b->mul_in->get(zf, use), b->att_start->get(zf, use), b->att_end->get(zf, use),
+                 b->transition->get(zf, use), nullptr, nullptr};
     if (b->single && s.defined()) {
-      r.pair_bias = b->pair_bias->get(zf, dev), r.single = b->single->get(zf, dev);
+      r.pair_bias = b->pair_bias->get(zf, use), r.single = b->single->get(zf, use);
       singles = true;
     }
     ready.push_back(r);
@@ -560,7 +625,7 @@ std::tuple<OptTensor, Tensor> stack_forward(const std::vector<std::shared_ptr<Bl
   Rows rows = own_rows(c, ws);
   const bool first = n <= kProjectFirstUpTo;       // projections of s beside the pair path of their own block
   const bool aside = singles && (blocks.size() > 1 ? n < kBesideBelow : first);
-  const auto side = aside ? side_stream(zc.device().index()) : main;
+  const auto side = aside ? side_stream(use) : main;
   Tensor bias[2], sb[2], sws;
   at::cuda::CUDAEvent bias_ready[2], side_done[2];   // bias_ready: what the rest of the branch waits for on its stream
   if (singles) {
@@ -638,7 +703,7 @@ Tensor opm_forward(Params& params, const Tensor& m, const OptTensor& mask, const
     if (mask->dim() != 2 || mask->size(0) != s_rows || mask->size(1) != n) fail("msa_mask must be [N_seq, N_res]");
     mk = mask->to(at::kFloat).contiguous();
   }
-  const Ready pr = params.get(0, m.device());
+  const Ready pr = params.get(0, Use(m.device()));
   py::gil_scoped_release release;
   const auto& p = pr->p[0];
   const float eps = pr->scalars[0], ln_eps = pr->scalars[1];
@@ -676,7 +741,8 @@ void msa_stack_forward(Params& params, Params& bias_params, const Tensor& m, con
   if (m.dim() != 3 || m.size(2) != 64 || n != z.size(0) || m.scalar_type() != at::kFloat || !m.is_contiguous())
     fail("m must be a contiguous float32 [S, N, 64] tensor with z [N, N, 128]");
   const int zf = zformat(z);
-  const Ready pr = params.get(0, m.device()), br = bias_params.get(zf, m.device());
+  const Use use(m.device());
+  const Ready pr = params.get(0, use), br = bias_params.get(zf, use);
   py::gil_scoped_release release;
   const auto& p = pr->p[0];
   const cudaStream_t st = at::cuda::getCurrentCUDAStream();

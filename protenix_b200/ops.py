@@ -163,8 +163,11 @@ _workspaces: Dict[Tuple[int, int], torch.Tensor] = {}
 
 
 def workspace(device: torch.device, nbytes: int) -> torch.Tensor:
-    """A per-(device, stream) scratch buffer, grown on demand and reused between calls."""
+    """A per-(device, stream) scratch buffer, grown on demand and reused between calls; inside a CUDA graph capture a
+    buffer of the graph's own."""
     dev = torch.device(device)
+    if torch.cuda.is_current_stream_capturing():
+        return torch.empty(int(nbytes), dtype=torch.uint8, device=dev)
     key = (dev.index if dev.index is not None else torch.cuda.current_device(),
            torch.cuda.current_stream(dev).cuda_stream)
     buf = _workspaces.get(key)

@@ -5,6 +5,7 @@ where it multiplies fp16 operands (rows of an fp32 pair tensor, which the kernel
 and every intermediate tensor).  The modules keep fp32 parameters with the reference's names so that its
 checkpoints load with ``strict=True``.  A cached copy is keyed on the parameter's storage pointer, device, in-place
 version counter and the wanted format, so ``load_state_dict``, ``.to()`` and optimiser steps all invalidate it.
+Inside a CUDA graph capture nothing is looked up or kept: the conversion becomes part of the graph.
 """
 from __future__ import annotations
 
@@ -20,6 +21,8 @@ def w16_of(p: torch.Tensor, fmt: torch.dtype) -> torch.Tensor:
     """``p`` as a contiguous tensor of the 16-bit format ``fmt`` (``torch.bfloat16`` or ``torch.float16``)."""
     if p.dtype == fmt and p.is_contiguous() and not p.requires_grad:
         return p
+    if p.is_cuda and torch.cuda.is_current_stream_capturing():
+        return p.detach().to(fmt).contiguous()       # written by the graph's replays, into the graph's own memory
     key = (p.data_ptr(), p._version, p.device, tuple(p.shape), p.dtype)
     ent = _cache.get((id(p), fmt))
     if ent is not None and ent[0] == key and ent[2]() is p:
