@@ -158,6 +158,7 @@ struct Prepared {
   std::vector<const void*> p[2];
   std::vector<float> scalars;
   bool have[2] = {false, false};
+  std::vector<cudaStream_t> streams[2];   // that calls have used it on: its memory is not given out again before they are through
 };
 typedef std::shared_ptr<const Prepared> Ready;
 
@@ -289,6 +290,7 @@ class Params {
     }
     if (!prepared_->have[zf]) make(*prepared_, zf, use);
     if (use.graph) GraphHeld::keep(use.graph, prepared_);
+    else used_on(*prepared_, zf, use.stream);
     return prepared_;
   }
 
@@ -309,6 +311,15 @@ class Params {
   static PyObject* find(const Slot& s) {
     PyObject* o = PyDict_GetItem(s.dict.ptr(), s.key.ptr());
     return o ? o : Py_None;
+  }
+
+  // The allocator knows the stream of make(); every other one is told to it once, and asked of when the set is freed.
+  static void used_on(Prepared& p, int zf, const c10::cuda::CUDAStream& stream) {
+    for (const cudaStream_t s : p.streams[zf])
+      if (s == stream.stream()) return;
+    for (const Tensor& t : p.t[zf])
+      if (t.defined()) t.record_stream(stream.unwrap());
+    p.streams[zf].push_back(stream.stream());
   }
 
   void make(Prepared& p, int zf, const Use& use) {
@@ -394,6 +405,7 @@ class Params {
     // The row kernels fetch folded weights before the kernels in front of them are complete (programmatic launch), and other
     // streams use the set too: once per change of the weights, the host waits for it.
     C10_CUDA_CHECK(cudaStreamSynchronize(st));
+    p.streams[zf] = {st};
     p.have[zf] = true;
   }
 

@@ -5,7 +5,8 @@ where it multiplies fp16 operands (rows of an fp32 pair tensor, which the kernel
 and every intermediate tensor).  The modules keep fp32 parameters with the reference's names so that its
 checkpoints load with ``strict=True``.  A cached copy is keyed on the parameter's storage pointer, device, in-place
 version counter and the wanted format, so ``load_state_dict``, ``.to()`` and optimiser steps all invalidate it.
-Inside a CUDA graph capture nothing is looked up or kept: the conversion becomes part of the graph.
+Inside a CUDA graph capture nothing is looked up or kept: the conversion becomes part of the graph.  A stream that uses a
+copy for the first time waits for its conversion, and the copy's memory is not given out again before that stream is through with it.
 """
 from __future__ import annotations
 
@@ -14,7 +15,27 @@ from typing import Dict, Tuple
 
 import torch
 
-_cache: Dict[Tuple[int, torch.dtype], Tuple[Tuple, torch.Tensor, "weakref.ref"]] = {}
+
+class _Copy:
+    """One kept copy: of which state of which parameter, and the streams that may use it without further ado."""
+
+    def __init__(self, key: Tuple, w: torch.Tensor, ref: "weakref.ref") -> None:
+        self.key, self.w, self.ref = key, w, ref
+        if w.is_cuda:
+            stream = torch.cuda.current_stream(w.device)
+            self.made, self.streams = stream.record_event(), {stream.cuda_stream}
+
+    def for_current_stream(self) -> torch.Tensor:
+        if self.w.is_cuda:
+            stream = torch.cuda.current_stream(self.w.device)
+            if stream.cuda_stream not in self.streams:
+                stream.wait_event(self.made)
+                self.w.record_stream(stream)
+                self.streams.add(stream.cuda_stream)
+        return self.w
+
+
+_cache: Dict[Tuple[int, torch.dtype], _Copy] = {}
 
 
 def w16_of(p: torch.Tensor, fmt: torch.dtype) -> torch.Tensor:
@@ -25,11 +46,11 @@ def w16_of(p: torch.Tensor, fmt: torch.dtype) -> torch.Tensor:
         return p.detach().to(fmt).contiguous()       # written by the graph's replays, into the graph's own memory
     key = (p.data_ptr(), p._version, p.device, tuple(p.shape), p.dtype)
     ent = _cache.get((id(p), fmt))
-    if ent is not None and ent[0] == key and ent[2]() is p:
-        return ent[1]
+    if ent is not None and ent.key == key and ent.ref() is p:
+        return ent.for_current_stream()
     w = p.detach().to(fmt).contiguous()
     ck = (id(p), fmt)
-    _cache[ck] = (key, w, weakref.ref(p, lambda _r, ck=ck: _cache.pop(ck, None)))
+    _cache[ck] = _Copy(key, w, weakref.ref(p, lambda _r, ck=ck: _cache.pop(ck, None)))
     return w
 
 
