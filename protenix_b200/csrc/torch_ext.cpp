@@ -227,8 +227,10 @@ std::atomic<bool> GraphHeld::any_{false};
 
 class Params {
  public:
-  // checks: (dict, name) of submodules; params: (dict, name, kind, shape); scalars: (dict, name)
-  Params(const std::string& group, const py::list& checks, const py::list& params, const py::list& scalars) {
+  // root: the module this is kept for; checks: (dict, name) of submodules; params: (dict, name, kind, shape, module);
+  // scalars: (dict, name).  Modules are held weakly: they hold this.
+  Params(const std::string& group, const py::object& root, const py::list& checks, const py::list& params, const py::list& scalars)
+      : root_(py::weakref(root)) {
     const char* names[] = {"plain", "mul", "att", "bias", "single", "msa", "opm"};
     int g = 0;
     while (g < 7 && group != names[g]) ++g;
@@ -236,23 +238,25 @@ class Params {
     group_ = (Group)g;
     for (const auto& c : checks) {
       const auto t = c.cast<py::tuple>();
-      checks_.push_back({t[0].cast<py::dict>(), t[1].cast<py::object>(), py::none()});
+      checks_.push_back({t[0].cast<py::dict>(), t[1].cast<py::object>(), py::none(), py::none()});
     }
     for (const auto& c : params) {
       const auto t = c.cast<py::tuple>();
-      params_.push_back({t[0].cast<py::dict>(), t[1].cast<py::object>(), py::none()});
+      params_.push_back({t[0].cast<py::dict>(), t[1].cast<py::object>(), py::none(), py::weakref(t[4])});
       kind_.push_back(t[2].cast<std::string>()[0]);
       shape_.push_back(t[3].cast<std::vector<int64_t>>());
     }
     for (const auto& c : scalars) {
       const auto t = c.cast<py::tuple>();
-      scalars_.push_back({t[0].cast<py::dict>(), t[1].cast<py::object>(), py::none()});
+      scalars_.push_back({t[0].cast<py::dict>(), t[1].cast<py::object>(), py::none(), py::none()});
     }
     for (auto& s : checks_) s.seen = py::reinterpret_borrow<py::object>(find(s));
   }
 
-  // False when a submodule has been replaced: the object has to be made again from the module.
-  bool current() const {
+  // False for another module than the one it was made for (a replica or a shallow copy of it, which took over its attributes), and
+  // when a submodule has been replaced: the object has to be made again from the module.
+  bool current(const py::handle& module) const {
+    if (PyWeakref_GetObject(root_.ptr()) != module.ptr()) return false;
     for (const auto& s : checks_)
       if (find(s) != s.seen.ptr()) return false;
     return true;
@@ -264,8 +268,9 @@ class Params {
     GraphHeld::free_released();
     bool same = prepared_ != nullptr;
     c10::SmallVector<Seen, 16> now(params_.size());
+    std::vector<py::object> elsewhere;       // keeps what is not a registered parameter, which may be computed on each look
     for (size_t i = 0; i < params_.size(); ++i) {
-      PyObject* o = find(params_[i]);
+      PyObject* o = parameter(params_[i], elsewhere);
       if (o != Py_None) {
         if (!THPVariable_Check(o)) fail("a module parameter is not a tensor");
         const Tensor& t = THPVariable_Unpack(o);
@@ -286,7 +291,7 @@ class Params {
       prepared_->scalars.assign(scalars.begin(), scalars.end());
       seen_.assign(now.begin(), now.end());
       params_hold_.clear();
-      for (auto& s : params_) params_hold_.push_back(py::reinterpret_borrow<py::object>(find(s)));
+      for (const Seen& n : now) params_hold_.push_back(py::reinterpret_borrow<py::object>(n.object ? n.object : Py_None));
     }
     if (!prepared_->have[zf]) make(*prepared_, zf, use);
     if (use.graph) GraphHeld::keep(use.graph, prepared_);
@@ -297,7 +302,7 @@ class Params {
  private:
   struct Slot {
     py::dict dict;
-    py::object key, seen;
+    py::object key, seen, owner;     // owner: weak reference to the module
   };
   struct Seen {
     PyObject* object = nullptr;
@@ -311,6 +316,14 @@ class Params {
   static PyObject* find(const Slot& s) {
     PyObject* o = PyDict_GetItem(s.dict.ptr(), s.key.ptr());
     return o ? o : Py_None;
+  }
+  // A parameter as the module's attribute gives it: registered (the usual case, looked up directly), or a plain attribute or a property
+  // (flattened, replicated and parametrised modules).
+  static PyObject* parameter(const Slot& s, std::vector<py::object>& elsewhere) {
+    if (PyObject* o = PyDict_GetItemWithError(s.dict.ptr(), s.key.ptr())) return o;
+    if (PyErr_Occurred()) throw py::error_already_set();
+    elsewhere.push_back(py::getattr(PyWeakref_GetObject(s.owner.ptr()), s.key));
+    return elsewhere.back().ptr();
   }
 
   // The allocator knows the stream of make(); every other one is told to it once, and asked of when the set is freed.
@@ -327,7 +340,7 @@ class Params {
     const at::Device& dev = use.dev;
     std::vector<Tensor> t;
     for (size_t i = 0; i < params_.size(); ++i) {
-      PyObject* o = find(params_[i]);
+      PyObject* o = params_hold_[i].ptr();
       Tensor v;
       if (o != Py_None) {
         v = THPVariable_Unpack(o).detach();
@@ -410,6 +423,7 @@ class Params {
   }
 
   Group group_;
+  py::object root_;                          // weak reference
   std::vector<Slot> checks_, params_, scalars_;
   std::vector<char> kind_;
   std::vector<std::vector<int64_t>> shape_;
@@ -549,9 +563,9 @@ Tensor transition_forward(Params& params, const Tensor& x) {
 // ---- blocks ----------------------------------------------------------------------------------------------------------
 struct Block {
   std::shared_ptr<Params> mul_out, mul_in, att_start, att_end, transition, pair_bias, single;   // the last two: s branch
-  bool current() const {
+  bool current(const py::handle& module) const {
     for (const auto& p : {mul_out, mul_in, att_start, att_end, transition, pair_bias, single})
-      if (p && !p->current()) return false;
+      if (p && !p->current(module)) return false;
     return true;
   }
 };
@@ -945,7 +959,7 @@ PYBIND11_MODULE(_C, m) {
   m.def("layer_norm", &layer_norm);
   m.def("dropout_add", &dropout_add);
   py::class_<Params, std::shared_ptr<Params>>(m, "Params")
-      .def(py::init<std::string, py::list, py::list, py::list>())
+      .def(py::init<std::string, py::object, py::list, py::list, py::list>())
       .def("current", &Params::current)
       // kept in a module's __dict__: a copy or an unpickled module makes its own
       .def("__deepcopy__", [](const Params&, py::dict) { return py::none(); })

@@ -45,8 +45,12 @@ class FusedLayerNorm(torch.nn.Module):
             torch.nn.init.zeros_(self.bias)
 
     def forward(self, input: torch.Tensor) -> torch.Tensor:
-        p = self._parameters
-        return _layer_norm(input, p["weight"], p["bias"], self._width, self.eps)
+        p = self._parameters            # the attributes by the short way
+        try:
+            weight, bias = p["weight"], p["bias"]
+        except KeyError:                # parametrised, flattened or replicated: a property or a plain attribute
+            weight, bias = self.weight, self.bias
+        return _layer_norm(input, weight, bias, self._width, self.eps)
 
 
 def LayerNorm(c_in: int, create_scale: bool = True, create_offset: bool = True, eps: float = 1e-5) -> torch.nn.Module:

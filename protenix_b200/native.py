@@ -39,15 +39,16 @@ def params(root, group: str, spec: Sequence[Tuple[str, str, Tuple[int, ...]]], s
 
     for path, kind, shape in spec:
         module, name = owner(path)
-        places.append((module._parameters, name, kind, list(shape)))
+        places.append((module._parameters, name, kind, list(shape), module))
     attributes = [(module.__dict__, name) for module, name in map(owner, scalars)]
-    return load().Params(group, list(dict(((id(d), n), (d, n)) for d, n in checks).values()), places, attributes)
+    return load().Params(group, root, list(dict(((id(d), n), (d, n)) for d, n in checks).values()), places, attributes)
 
 
 def kept(module, make, name: str = "_px_params"):
-    """``make()``, kept in the module's __dict__ until one of the submodules it looked through is replaced."""
+    """``make()``, kept in the module's __dict__ until one of the submodules it looked through is replaced.  A module that has
+    taken over the __dict__ of another one (a replica, a shallow copy) makes its own."""
     held = module.__dict__.get(name)
-    if held is None or not held.current():
+    if held is None or not held.current(module):
         held = make()
         module.__dict__[name] = held
     return held

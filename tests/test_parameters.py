@@ -1,0 +1,93 @@
+"""Where modules find their parameters: registered, or as plain attributes and properties (parametrised, flattened, replicated modules)."""
+import copy
+
+import pytest
+import torch
+from torch.nn.utils import parametrize
+
+import protenix_b200 as px
+from protenix_b200.init_utils import randomize_parameters_
+
+
+class Twice(torch.nn.Module):
+    def forward(self, w):
+        return 2 * w
+
+
+PLACES = ["tri_mul_out.layer_norm_in", "tri_mul_in.linear_a_p", "tri_att_start.mha.linear_q", "tri_att_end.layer_norm", "pair_transition.linear_no_bias",
+          "attention_pair_bias.layernorm_z", "attention_pair_bias.attention.linear_k", "single_transition.layernorm1"]
+
+
+def _flatten(module):
+    """The weight as a plain attribute, as wrappers that keep parameters in one flat buffer leave it."""
+    w = module._parameters.pop("weight")
+    module.weight = w.detach()
+
+
+def test_layer_norm_finds_parameters_that_are_not_registered():
+    """On the CPU the op is refused for that reason and no other."""
+    for change in (lambda m: parametrize.register_parametrization(m, "weight", Twice()), _flatten):
+        ln = px.LayerNorm(8)
+        change(ln)
+        with pytest.raises(RuntimeError, match="CUDA"):
+            ln(torch.randn(3, 8))
+
+
+@pytest.mark.gpu
+def test_layer_norm_with_a_parametrised_and_a_flattened_weight():
+    x, dy = torch.randn(33, 128, device="cuda"), torch.randn(33, 128, device="cuda")
+    plain = randomize_parameters_(px.LayerNorm(128), 1).cuda()
+    want = plain(x)
+    flat = copy.deepcopy(plain)
+    _flatten(flat)
+    assert torch.equal(flat(x), want)
+    double = copy.deepcopy(plain)
+    with torch.no_grad():
+        double.weight.mul_(2)
+    want = torch.autograd.grad(double(x), [double.weight, double.bias], dy)
+    parametrize.register_parametrization(plain, "weight", Twice())
+    got = torch.autograd.grad(plain(x), [plain.parametrizations.weight.original, plain.bias], dy)
+    assert torch.equal(got[0], 2 * want[0]) and torch.equal(got[1], want[1])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("warm", [False, True])
+def test_block_with_parametrised_and_flattened_weights(warm):
+    n = 40
+    s, z = torch.randn(n, 384, device="cuda"), torch.randn(n, n, 128, device="cuda")
+    plain, want, flat = (randomize_parameters_(px.PairformerBlock(), 3).cuda().eval() for _ in range(3))
+    first = want(s, z, None)
+    if warm:                                                      # the change comes after the parameters have been looked up
+        plain(s, z, None), flat(s, z, None)
+    for place in PLACES:
+        parametrize.register_parametrization(plain.get_submodule(place), "weight", Twice())
+        _flatten(flat.get_submodule(place))
+        with torch.no_grad():
+            want.get_submodule(place).weight.mul_(2)
+    assert all(torch.equal(a, b) for a, b in zip(flat(s, z, None), first))
+    for _ in range(2):
+        assert all(torch.equal(a, b) for a, b in zip(plain(s, z, None), want(s, z, None)))
+    with torch.no_grad():                                         # and the computed weights follow
+        plain.get_submodule(PLACES[2]).parametrizations.weight.original.mul_(0.5)
+        want.get_submodule(PLACES[2]).weight.mul_(0.5)
+    assert all(torch.equal(a, b) for a, b in zip(plain(s, z, None), want(s, z, None)))
+    del flat.get_submodule(PLACES[0]).weight
+    with pytest.raises(AttributeError):
+        flat(s, z, None)
+
+
+@pytest.mark.gpu
+def test_replicas_and_shallow_copies_look_up_their_own_parameters():
+    n = 40
+    z = torch.randn(n, n, 128, device="cuda")
+    for kind in (lambda: px.TriangleAttention(c_in=128, c_hidden=32, no_heads=4), lambda: px.PairformerBlock(c_s=0)):
+        call = lambda m: m(z) if isinstance(m, px.TriangleAttention) else m(None, z, None)[1]
+        mod, other = (randomize_parameters_(kind(), seed).cuda().eval() for seed in (3, 4))
+        want, new = call(mod), call(other)
+        with torch.no_grad():
+            replica = torch.nn.parallel.replicate(mod, [0])[0]
+            twin = copy.copy(mod)
+            twin._modules = dict(other._modules)
+            mod.load_state_dict({k: v.clone() for k, v in other.state_dict().items()}, assign=True)
+        assert torch.equal(call(replica), want)
+        assert torch.equal(call(twin), new) and torch.equal(call(mod), new)
