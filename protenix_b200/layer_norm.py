@@ -38,6 +38,10 @@ class FusedLayerNorm(torch.nn.Module):
         self.register_parameter("weight", Parameter(torch.ones(*normalized_shape)) if create_scale else None)
         self.register_parameter("bias", Parameter(torch.zeros(*normalized_shape)) if create_offset else None)
 
+    def __setstate__(self, state) -> None:
+        super().__setstate__(state)
+        self._width = int(self.normalized_shape[0])      # modules saved whole before it existed have none
+
     def reset_parameters(self) -> None:
         if self.weight is not None:
             torch.nn.init.ones_(self.weight)

@@ -1,5 +1,6 @@
 """Where modules find their parameters: registered, or as plain attributes and properties (parametrised, flattened, replicated modules)."""
 import copy
+import pickle
 
 import pytest
 import torch
@@ -31,6 +32,15 @@ def test_layer_norm_finds_parameters_that_are_not_registered():
         change(ln)
         with pytest.raises(RuntimeError, match="CUDA"):
             ln(torch.randn(3, 8))
+
+
+def test_layer_norm_saved_whole_without_its_width_loads():
+    """The attribute is younger than saved modules are."""
+    ln = px.LayerNorm(8)
+    del ln.__dict__["_width"]
+    for twin in (copy.deepcopy(ln), pickle.loads(pickle.dumps(ln))):
+        with pytest.raises(RuntimeError, match="CUDA"):           # the CPU is refused, and nothing before that fails
+            twin(torch.randn(3, 8))
 
 
 @pytest.mark.gpu
