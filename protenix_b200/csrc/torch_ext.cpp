@@ -228,7 +228,8 @@ std::atomic<bool> GraphHeld::any_{false};
 class Params {
  public:
   // root: the module this is kept for; checks: (dict, name) of submodules; params: (dict, name, kind, shape, module);
-  // scalars: (dict, name).  Modules are held weakly: they hold this.
+  // scalars: (module, name).  Modules and their __dict__ are held weakly or not at all: they hold this, and the garbage collector
+  // does not see through it.
   Params(const std::string& group, const py::object& root, const py::list& checks, const py::list& params, const py::list& scalars)
       : root_(py::weakref(root)) {
     const char* names[] = {"plain", "mul", "att", "bias", "single", "msa", "opm"};
@@ -248,7 +249,7 @@ class Params {
     }
     for (const auto& c : scalars) {
       const auto t = c.cast<py::tuple>();
-      scalars_.push_back({t[0].cast<py::dict>(), t[1].cast<py::object>(), py::none(), py::none()});
+      scalars_.push_back({py::dict(), t[1].cast<py::object>(), py::none(), py::weakref(t[0])});
     }
     for (auto& s : checks_) s.seen = py::reinterpret_borrow<py::object>(find(s));
   }
@@ -280,7 +281,7 @@ class Params {
     }
     c10::SmallVector<float, 4> scalars;
     for (const auto& s : scalars_) {
-      scalars.push_back((float)PyFloat_AsDouble(find(s)));
+      scalars.push_back(py::getattr(PyWeakref_GetObject(s.owner.ptr()), s.key).cast<float>());
       same = same && prepared_->scalars[scalars.size() - 1] == scalars.back();
     }
     if (use.graph && !(same && prepared_->have[zf]))

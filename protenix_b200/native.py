@@ -40,7 +40,7 @@ def params(root, group: str, spec: Sequence[Tuple[str, str, Tuple[int, ...]]], s
     for path, kind, shape in spec:
         module, name = owner(path)
         places.append((module._parameters, name, kind, list(shape), module))
-    attributes = [(module.__dict__, name) for module, name in map(owner, scalars)]
+    attributes = [owner(path) for path in scalars]
     return load().Params(group, root, list(dict(((id(d), n), (d, n)) for d, n in checks).values()), places, attributes)
 
 

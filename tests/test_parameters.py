@@ -1,6 +1,8 @@
 """Where modules find their parameters: registered, or as plain attributes and properties (parametrised, flattened, replicated modules)."""
 import copy
+import gc
 import pickle
+import weakref
 
 import pytest
 import torch
@@ -101,3 +103,23 @@ def test_replicas_and_shallow_copies_look_up_their_own_parameters():
             mod.load_state_dict({k: v.clone() for k, v in other.state_dict().items()}, assign=True)
         assert torch.equal(call(replica), want)
         assert torch.equal(call(twin), new) and torch.equal(call(mod), new)
+
+
+def test_kept_look_ups_do_not_keep_their_module_alive():
+    """What a module keeps refers to the module's own attributes; with the last reference to the module its parameters are gone."""
+    from protenix_b200 import native
+    from protenix_b200.msa import MSABlock
+
+    for make, names in ((lambda: px.TriangleAttention(c_in=128, c_hidden=32, no_heads=4), [""]),
+                        (lambda: px.OuterProductMean(c_m=64, c_z=128, c_hidden=32), [""]),
+                        (lambda: MSABlock(), ["outer_product_mean_msa", "pair_stack.tri_att_end"])):
+        mod = make()
+        for name in names:
+            m = mod.get_submodule(name)
+            native.kept(m, lambda: native.params(m, *m.NATIVE))
+        if isinstance(mod, MSABlock):
+            mod.pair_stack._native()
+        held = [weakref.ref(p) for p in mod.parameters()]
+        del mod, m
+        gc.collect()
+        assert not any(r() is not None for r in held)
