@@ -11,11 +11,13 @@ from .triangular import (OpenfoldLinear, TriangleAttention, TriangleAttentionEnd
                          TriangleAttentionStartingNode, TriangleMultiplicationIncoming,
                          TriangleMultiplicationOutgoing, TriangleMultiplicativeUpdate)
 from .fused_ops import dropout_add_rowwise
+from .weights import weights_changed
 
 __all__ = [
     "FusedLayerNorm", "LayerNorm", "PairformerBlock", "PairformerStack", "Linear", "LinearNoBias", "Transition",
     "AttentionPairBias", "OpenfoldLinear", "TriangleAttention", "TriangleAttentionEndingNode",
     "TriangleAttentionStartingNode", "TriangleMultiplicationIncoming", "TriangleMultiplicationOutgoing",
     "TriangleMultiplicativeUpdate", "dropout_add_rowwise", "RecyclingTrunk", "OuterProductMean",
+    "weights_changed",
 ]
 __version__ = "0.1.0"

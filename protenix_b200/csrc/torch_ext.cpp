@@ -5,7 +5,7 @@
 // representation 18 us for a 3 us kernel.  Here a module keeps a `Params` object: the places of its parameters (the
 // module's own `_parameters` dictionaries), what was seen there last, and the forms the kernels want (fp32 vectors,
 // 16-bit matrices, the split planes of the single branch), renewed when a parameter, its storage, its version or a
-// submodule has changed.  A call checks its tensors, looks the parameters over (some tens of pointer comparisons) and
+// submodule has changed (what is written past the version counter has to be announced: weights.py).  A call checks its tensors, looks the parameters over (some tens of pointer comparisons) and
 // issues the launches through the C ABI of px_b200.h, whose functions are taken from the library handle that the Python
 // side has loaded.  Workspaces come from the caching allocator on each call.
 #include <ATen/ATen.h>
@@ -275,7 +275,7 @@ class Params {
       if (o != Py_None) {
         if (!THPVariable_Check(o)) fail("a module parameter is not a tensor");
         const Tensor& t = THPVariable_Unpack(o);
-        now[i] = {o, t.data_ptr(), (uint32_t)t._version(), t.scalar_type()};
+        now[i] = {o, t.data_ptr(), t.storage().unsafeGetStorageImpl(), (uint32_t)t._version(), t.scalar_type()};
       }
       same = same && now[i] == seen_[i];
     }
@@ -292,7 +292,11 @@ class Params {
       prepared_->scalars.assign(scalars.begin(), scalars.end());
       seen_.assign(now.begin(), now.end());
       params_hold_.clear();
-      for (const Seen& n : now) params_hold_.push_back(py::reinterpret_borrow<py::object>(n.object ? n.object : Py_None));
+      storages_.clear();
+      for (const Seen& n : now) {
+        params_hold_.push_back(py::reinterpret_borrow<py::object>(n.object ? n.object : Py_None));
+        if (n.object) storages_.push_back(THPVariable_Unpack(n.object).storage().getWeakStorageImpl());
+      }
     }
     if (!prepared_->have[zf]) make(*prepared_, zf, use);
     if (use.graph) GraphHeld::keep(use.graph, prepared_);
@@ -308,10 +312,11 @@ class Params {
   struct Seen {
     PyObject* object = nullptr;
     void* data = nullptr;
+    const void* storage = nullptr;
     uint32_t version = 0;
     at::ScalarType type = at::kFloat;
     bool operator==(const Seen& o) const {
-      return object == o.object && data == o.data && version == o.version && type == o.type;
+      return object == o.object && data == o.data && storage == o.storage && version == o.version && type == o.type;
     }
   };
   static PyObject* find(const Slot& s) {
@@ -429,7 +434,10 @@ class Params {
   std::vector<char> kind_;
   std::vector<std::vector<int64_t>> shape_;
   std::vector<Seen> seen_;
-  std::vector<py::object> params_hold_;      // the parameter objects seen last: their addresses cannot be reused
+  // The parameter objects seen last, and their storages, these without the memory: the addresses of neither can be reused, so that
+  // another object or storage is told from them even where its memory lies where the old one's did.
+  std::vector<py::object> params_hold_;
+  std::vector<c10::weak_intrusive_ptr<c10::StorageImpl>> storages_;
   std::shared_ptr<Prepared> prepared_;
 };
 

@@ -123,3 +123,44 @@ def test_kept_look_ups_do_not_keep_their_module_alive():
         del mod, m
         gc.collect()
         assert not any(r() is not None for r in held)
+
+
+def test_wrapper_copies_follow_announced_writes_and_new_storages():
+    from protenix_b200 import weights
+
+    lin = px.OpenfoldLinear(8, 4, bias=False)
+    kept = weights.f16_of(lin.weight)
+    lin.weight.data.copy_(torch.ones(4, 8))                       # past the version counter
+    px.weights_changed(lin)
+    assert weights.f16_of(lin.weight) is not kept and bool((weights.f16_of(lin.weight) == 1).all())
+    memory = torch.zeros(64)                                      # two storages over the same memory, one after the other
+    over = lambda: torch.from_numpy(memory.numpy())[:32].view(4, 8)
+    lin.weight.data = over()
+    first, version = weights.f16_of(lin.weight), lin.weight._version
+    lin.weight.data = torch.empty(4, 8)
+    memory.fill_(3.0)
+    lin.weight.data = over()
+    assert lin.weight._version == version and lin.weight.data_ptr() == memory.data_ptr()
+    assert bool((weights.f16_of(lin.weight) == 3).all()) and bool((first == 0).all())
+
+
+@pytest.mark.gpu
+def test_modules_follow_announced_writes_and_new_storages():
+    n = 40
+    s, z = torch.randn(n, 384, device="cuda"), torch.randn(n, n, 128, device="cuda")
+    blk, other = (randomize_parameters_(px.PairformerBlock(), seed).cuda().eval() for seed in (3, 4))
+    first, want = blk(s, z, None), other(s, z, None)
+    new = other.state_dict()
+    for name, p in blk.named_parameters():                        # an average written over the weights, past the version counters
+        p.data.copy_(new[name])
+    assert all(torch.equal(a, b) for a, b in zip(blk(s, z, None), first))       # one set or the other, not a mixture
+    px.weights_changed(blk.tri_att_start)                         # announced for a part, kept by the block
+    px.weights_changed(blk)
+    assert all(torch.equal(a, b) for a, b in zip(blk(s, z, None), want))
+    old = {k: p.data.clone() for k, p in blk.named_parameters()}
+    for name, p in blk.named_parameters():                        # memory given back and taken again, most of it at the same addresses
+        p.data = torch.empty(0, device="cuda")
+        p.data = torch.empty_like(old[name]).normal_(0, 0.05)
+        new[name] = p.data.clone()
+    other.load_state_dict(new)
+    assert all(torch.equal(a, b) for a, b in zip(blk(s, z, None), other(s, z, None)))
