@@ -116,6 +116,11 @@ std::vector<std::pair<std::string, double>> timer_collect() {
 void need_cuda(const Tensor& t, const char* name) {
   if (!t.is_cuda()) fail(std::string(name) + " must be a CUDA tensor: this package has no CPU path");
 }
+// The kernels of a call run on one device, and an address of another one may not be mapped there.
+void need_on(const Tensor& t, const at::Device& dev, const char* name) {
+  need_cuda(t, name);
+  if (t.device() != dev) fail(std::string(name) + " must be on the device of the other tensors");
+}
 int dtype_code(const Tensor& t, const char* name) {
   switch (t.scalar_type()) {
     case at::kFloat: return PX_F32;
@@ -157,6 +162,7 @@ struct Prepared {
   std::vector<Tensor> t[2];          // by format of z: 0 fp32, 1 bf16; complete, and no aliases of the parameters
   std::vector<const void*> p[2];
   std::vector<float> scalars;
+  at::Device dev = at::kCPU;         // where the parameters are
   bool have[2] = {false, false};
   std::vector<cudaStream_t> streams[2];   // that calls have used it on: its memory is not given out again before they are through
 };
@@ -299,6 +305,7 @@ class Params {
       }
     }
     if (!prepared_->have[zf]) make(*prepared_, zf, use);
+    if (prepared_->dev != use.dev) fail("parameters and inputs must be on the same device");
     if (use.graph) GraphHeld::keep(use.graph, prepared_);
     else used_on(*prepared_, zf, use.stream);
     return prepared_;
@@ -425,6 +432,7 @@ class Params {
     // streams use the set too: once per change of the weights, the host waits for it.
     C10_CUDA_CHECK(cudaStreamSynchronize(st));
     p.streams[zf] = {st};
+    p.dev = dev;
     p.have[zf] = true;
   }
 
@@ -644,7 +652,7 @@ std::tuple<OptTensor, Tensor> stack_forward(const std::vector<std::shared_ptr<Bl
     ready.push_back(r);
   }
   if (singles) {
-    need_cuda(s, "s");
+    need_on(s, zi.device(), "s");
     if (s.dim() < 2 || s.size(-1) != kCs || s.size(-2) != n || s.numel() != n * kCs) fail("s must be [N, 384]");
     dtype_code(s, "s");
     s = s.contiguous();
@@ -729,12 +737,14 @@ Tensor opm_forward(Params& params, const Tensor& m, const OptTensor& mask, const
   if (m.dim() != 3 || m.size(2) != 64 || m.scalar_type() != at::kFloat || !m.is_contiguous()) fail("m must be a contiguous float32 [S, N, 64] tensor");
   if (n > 32768 || n < 1 || s_rows < 1) fail("outer_product_mean supports 1 <= N <= 32768 tokens");
   const bool residual = z_in.has_value() && z_in->defined();
-  for (const Tensor& z : {z_out, residual ? *z_in : z_out})
+  for (const Tensor& z : {z_out, residual ? *z_in : z_out}) {
+    need_on(z, m.device(), "z");
     if (z.dim() != 3 || z.size(0) != n || z.size(1) != n || z.size(2) != kCz || !z.is_contiguous() || z.scalar_type() != z_out.scalar_type())
       fail("z must be contiguous [N, N, 128] with N = m.shape[1]");
+  }
   Tensor mk;
   if (mask.has_value() && mask->defined()) {
-    need_cuda(*mask, "msa_mask");
+    need_on(*mask, m.device(), "msa_mask");
     if (mask->dim() != 2 || mask->size(0) != s_rows || mask->size(1) != n) fail("msa_mask must be [N_seq, N_res]");
     mk = mask->to(at::kFloat).contiguous();
   }
@@ -770,6 +780,7 @@ void msa_stack_forward(Params& params, Params& bias_params, const Tensor& m, con
   need_cuda(m, "m");
   bool batch;
   const Tensor z = pair_tensor(z_, batch);
+  need_on(z, m.device(), "z");
   c10::cuda::CUDAGuard guard(m.device());
   at::NoGradGuard no_grad;
   const int64_t s_all = m.size(0), n = m.size(1), heads = 8;
@@ -825,7 +836,7 @@ LnParams ln_params(const Tensor& x, const OptTensor& weight, const OptTensor& bi
   const auto type = fp32 ? at::kFloat : x.scalar_type();
   auto fit = [&](const OptTensor& p, const char* name, Tensor& to) {
     if (!has(p)) return;
-    need_cuda(*p, name);
+    need_on(*p, x.device(), name);
     if (p->numel() != x.size(-1)) fail(std::string(name) + " must have as many elements as the last axis");
     to = p->scalar_type() == type && p->is_contiguous() ? *p : p->detach().to(type).contiguous();
   };
@@ -948,7 +959,8 @@ Tensor dropout_add(const Tensor& residual, const Tensor& x, double p) {
   need_cuda(x, "x");
   if (x.dim() < 3) fail("x must be [..., R, C, D]");
   dtype_code(x, "x");
-  if (!residual.is_cuda() || residual.sizes() != x.sizes() || residual.scalar_type() != x.scalar_type()) fail("residual must match x");
+  need_on(residual, x.device(), "residual");
+  if (residual.sizes() != x.sizes() || residual.scalar_type() != x.scalar_type()) fail("residual must match x");
   auto shape = x.sizes().vec();
   shape[shape.size() - 3] = 1;
   Tensor mask;

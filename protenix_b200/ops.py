@@ -38,6 +38,12 @@ def _need_cuda(t: torch.Tensor, name: str) -> None:
         raise RuntimeError(f"{name} must be contiguous")
 
 
+def _one_device(*tensors: Optional[torch.Tensor]) -> None:
+    """The kernels of a call run on one device, and an address of another one may not be mapped there."""
+    if len({t.device for t in tensors if t is not None}) > 1:
+        raise RuntimeError("parameters and inputs must be on the same device")
+
+
 def _pair_dtype(z: torch.Tensor) -> int:
     if z.dtype not in (torch.float32, torch.bfloat16):
         raise RuntimeError(f"pair tensor must be float32 or bfloat16, got {z.dtype}")
@@ -194,6 +200,7 @@ def layer_norm(x: torch.Tensor, weight: Optional[torch.Tensor], bias: Optional[t
     _need_cuda(x, "input")
     if x.dtype not in _DTYPE:
         raise RuntimeError(f"layer_norm supports float32/bfloat16/float16, got {x.dtype}")
+    _one_device(x, weight, bias)
     cols = x.shape[-1]
     rows = x.numel() // cols if cols else 0
     for t, nm in ((weight, "weight"), (bias, "bias")):
@@ -217,6 +224,7 @@ def standardise_rows(z: torch.Tensor, eps: float = 1e-5, out: Optional[torch.Ten
     _need_cuda(z, "z")
     if z.dtype != torch.float32 or z.shape[-1] != C_Z:
         raise RuntimeError("standardise_rows takes a float32 tensor [..., 128]")
+    _one_device(z, out)
     if out is None:
         out = torch.empty(z.shape, dtype=torch.float16, device=z.device)
     rows = z.numel() // C_Z
@@ -231,6 +239,7 @@ def msa_embed(msa, has_deletion, deletion_value, index, w, s_proj) -> torch.Tens
     hd, dv, w, s_proj = f32(has_deletion), f32(deletion_value), f32(w), f32(s_proj)
     for t, nm in ((msa, "msa"), (hd, "has_deletion"), (dv, "deletion_value"), (index, "index"), (w, "w"), (s_proj, "s_proj")):
         _need_cuda(t, nm)
+    _one_device(msa, hd, dv, index, w, s_proj)
     m = torch.empty(index.numel(), msa.shape[1], 64, dtype=torch.float32, device=msa.device)
     _launch("px_msa_embed", _lib.load().px_msa_embed, _ptr(msa), _ptr(hd), _ptr(dv), _ptr(index), _ptr(w), _ptr(s_proj), _ptr(m),
             index.numel(), msa.shape[1], _stream(m))
@@ -241,6 +250,7 @@ def add_update_rows(z: torch.Tensor, upd: torch.Tensor) -> torch.Tensor:
     """z += upd in place for an fp32 tensor [..., 128] and an fp16 update of the same shape."""
     _need_cuda(z, "z")
     _need_cuda(upd, "upd")
+    _one_device(z, upd)
     if z.dtype != torch.float32 or upd.dtype != torch.float16 or z.shape != upd.shape or z.shape[-1] != C_Z:
         raise RuntimeError("add_update_rows takes a float32 tensor [..., 128] and a float16 update of the same shape")
     _launch("px_add_update_rows", _lib.load().px_add_update_rows, _ptr(z), _ptr(upd), z.numel() // C_Z, _stream(z))
@@ -282,6 +292,7 @@ def triangle_multiplication(z_in: torch.Tensor, z_out: torch.Tensor, mask: Optio
     n = _check_pair(z_in, "z_in")
     if _check_pair(z_out, "z_out") != n or z_out.dtype != z_in.dtype:
         raise RuntimeError("z_out must match z_in in shape and dtype")
+    _one_device(z_in, z_out, mask, ln_in_w, ln_in_b, ln_out_w, ln_out_b, w_ap, w_ag, w_bp, w_bg, w_z, w_g, zn)
     mask = _check_mask(mask, n)
     for v, nm in ((ln_in_w, "ln_in_w"), (ln_in_b, "ln_in_b"), (ln_out_w, "ln_out_w"), (ln_out_b, "ln_out_b")):
         _check_v(v, C_Z, nm)
@@ -317,6 +328,7 @@ def triangle_attention(z_in: torch.Tensor, z_out: torch.Tensor, mask: Optional[t
     n = _check_pair(z_in, "z_in")
     if _check_pair(z_out, "z_out") != n or z_out.dtype != z_in.dtype:
         raise RuntimeError("z_out must match z_in in shape and dtype")
+    _one_device(z_in, z_out, mask, ln_w, ln_b, w_bias, w_q, w_k, w_v, w_g, w_o, zn)
     mask = _check_mask(mask, n)
     _check_v(ln_w, C_Z, "ln_w")
     _check_v(ln_b, C_Z, "ln_b")
@@ -356,6 +368,7 @@ def transition(x_in: torch.Tensor, x_out: torch.Tensor, ln_w, ln_b, w_a, w_b, w_
     _need_cuda(x_out, "x_out")
     if x_in.shape[-1] != C_Z or x_out.shape != x_in.shape or x_out.dtype != x_in.dtype:
         raise RuntimeError(f"transition kernel handles [..., {C_Z}] rows with matching output")
+    _one_device(x_in, x_out, ln_w, ln_b, w_a, w_b, w_o)
     _check_v(ln_w, C_Z, "ln_w")
     _check_v(ln_b, C_Z, "ln_b")
     w_a = _w(w_a, F16, (4 * C_Z, C_Z), "w_a")
@@ -375,6 +388,7 @@ def pair_bias_proj(z: torch.Tensor, ln_w, ln_b: Optional[torch.Tensor], w: torch
     _check_v(ln_w, C_Z, "ln_w")
     if ln_b is not None:
         _check_v(ln_b, C_Z, "ln_b")
+    _one_device(z, ln_w, ln_b, w, zn)
     heads = w.shape[0]
     w = _w(w, _zfmt(z), (heads, C_Z), "w")
     out = torch.empty(heads, n, n, dtype=torch.float32, device=z.device)
@@ -393,6 +407,7 @@ def recycle_update(z: torch.Tensor, z_init: torch.Tensor, ln_w, ln_b: Optional[t
         raise RuntimeError("z and z_init must have the same shape [..., 128] and dtype")
     if not (z.is_contiguous() and z_init.is_contiguous()):
         raise RuntimeError("z and z_init must be contiguous")
+    _one_device(z, z_init, ln_w, ln_b, w, out)
     _check_v(ln_w, C_Z, "ln_w")
     if ln_b is not None:
         _check_v(ln_b, C_Z, "ln_b")
@@ -434,6 +449,7 @@ def outer_product_mean(z_in: Optional[torch.Tensor], z_out: torch.Tensor, m: tor
         raise RuntimeError("z must be [N, N, 128] with N = m.shape[1]")
     if not z_out.is_contiguous() or (z_in is not None and not z_in.is_contiguous()):
         raise RuntimeError("z must be contiguous")
+    _one_device(z_in, z_out, m, msa_mask, ln_w, ln_b, w_1, w_2, w_out, b_out)
     dev = m.device
     if msa_mask is None:
         mask = torch.ones(s_rows, n, dtype=torch.float32, device=dev)
@@ -483,6 +499,7 @@ def trimul_in_proj(z: torch.Tensor, mask: Optional[torch.Tensor], ln_w, ln_b, w_
     """a, b as [128][n_u][ld(n_t)] fp16.  z is [n_u][n_t][128]; with ``incoming`` it is [n_t][n_u][128]."""
     r, c = _slab(z)
     n_u, n_t = (c, r) if incoming else (r, c)
+    _one_device(z, mask, ln_w, ln_b, w_ap, w_ag, w_bp, w_bg, zn)
     lib = _lib.load()
     ldt = lib.px_ld(n_t)
     zf = _zfmt(z)
@@ -500,6 +517,7 @@ def trimul_contract(a: torch.Tensor, b: torch.Tensor) -> torch.Tensor:
     """x[c][i][j] = X_SCALE * sum_k a[c][i][k] b[c][j][k] for [C][n][ld] fp16 operands (pad columns zero)."""
     _need_cuda(a, "a")
     _need_cuda(b, "b")
+    _one_device(a, b)
     ch, n, ldn = a.shape
     if a.dtype != torch.float16 or b.shape != a.shape or b.dtype != a.dtype or ldn != ld(n):
         raise RuntimeError("contraction operands must be float16 [C][n][ld(n)] of equal shape")
@@ -511,6 +529,7 @@ def trimul_contract(a: torch.Tensor, b: torch.Tensor) -> torch.Tensor:
 def trimul_out(x: torch.Tensor, z: torch.Tensor, ln_in_w, ln_in_b, ln_out_w, ln_out_b, w_z, w_g,
                eps: float = 1e-5, zn: Optional[torch.Tensor] = None) -> torch.Tensor:
     """z[n_i][n_j] += W_z LN(x) * sigmoid(W_g LN(z)) in place; x is [128][n_i][ld(n_j)]."""
+    _one_device(x, z, ln_in_w, ln_in_b, ln_out_w, ln_out_b, w_z, w_g, zn)
     n_i, n_j = _slab(z)
     _need_cuda(x, "x")
     if x.dtype != torch.float16 or x.dim() != 3 or x.shape[0] != C_Z or x.shape[1] != n_i or x.shape[2] != ld(n_j):
@@ -531,6 +550,7 @@ def triatt_in_proj(z: torch.Tensor, mask: Optional[torch.Tensor], ln_w, ln_b, w_
     n_u, n_t = _slab(z)
     if ending:
         n_u, n_t = n_t, n_u
+    _one_device(z, mask, ln_w, ln_b, w_bias, w_q, w_k, w_v, zn)
     lib = _lib.load()
     ldm = lib.px_ld_mask(n_t)
     zf = _zfmt(z)
@@ -554,6 +574,7 @@ def triatt_flash(q, k, v, bias_full: torch.Tensor, mb) -> torch.Tensor:
     n_u, _, n, _ = q.shape
     for t, nm in ((q, "q"), (k, "k"), (v, "v"), (bias_full, "bias"), (mb, "mask_bias")):
         _need_cuda(t, nm)
+    _one_device(q, k, v, bias_full, mb)
     ldm = bias_full.shape[2]
     if tuple(bias_full.shape) != (N_HEAD_PAIR, n, ldm) or tuple(mb.shape) != (n_u, ldm):
         raise RuntimeError("pair bias must be [4][n][ldm] and mask_bias [n_u][ldm]")
@@ -574,6 +595,7 @@ def triatt_out(o: torch.Tensor, z: torch.Tensor, ln_w, ln_b, w_g, w_o, eps: floa
     n_u, n_t = _slab(z)
     if ending:
         n_u, n_t = n_t, n_u
+    _one_device(o, z, ln_w, ln_b, w_g, w_o, zn, update_out)
     _need_cuda(o, "o")
     if o.dtype != torch.float16 or tuple(o.shape) != (n_u, n_t, C_Z):
         raise RuntimeError("o must be float16 [n_u][n_t][128]")
@@ -597,6 +619,7 @@ def pair_bias_rows(z: torch.Tensor, ln_w, ln_b: Optional[torch.Tensor], w: torch
                    zn: Optional[torch.Tensor] = None) -> torch.Tensor:
     """bias[h, u, t] for a row slab z [n_u][n_t][128].  zn: the standardised copy of an fp32 slab, if at hand."""
     n_u, n_t = _slab(z)
+    _one_device(z, ln_w, ln_b, w, zn)
     heads = w.shape[0]
     w = _w(w, _zfmt(z), (heads, C_Z), "w")
     out = torch.empty(heads, n_u, n_t, dtype=torch.float32, device=z.device)
@@ -616,6 +639,7 @@ def transition_rows(x: torch.Tensor, ln_w, ln_b, w_a, w_b, w_o, eps: float = 1e-
         _need_cuda(out, "out")
         if out.shape != x.shape or out.dtype != x.dtype:
             raise RuntimeError("out must match x")
+    _one_device(x, out, ln_w, ln_b, w_a, w_b, w_o)
     w_a, w_b = _w(w_a, F16, (4 * C_Z, C_Z), "w_a"), _w(w_b, F16, (4 * C_Z, C_Z), "w_b")
     w_o = _w(w_o, F16, (C_Z, 4 * C_Z), "w_o")
     _launch("px_transition", _lib.load().px_transition, _ptr(x), _ptr(out), _pair_dtype(x), _ptr(ln_w), _ptr(ln_b),

@@ -164,3 +164,26 @@ def test_modules_follow_announced_writes_and_new_storages():
         new[name] = p.data.clone()
     other.load_state_dict(new)
     assert all(torch.equal(a, b) for a, b in zip(blk(s, z, None), other(s, z, None)))
+
+
+def test_wrappers_tell_devices_apart():
+    from protenix_b200 import ops
+
+    here, there = torch.empty(4), torch.empty(4, device="meta")
+    ops._one_device(here, None, here)
+    with pytest.raises(RuntimeError, match="same device"):
+        ops._one_device(here, None, there)
+
+
+@pytest.mark.gpu
+@pytest.mark.skipif(torch.cuda.device_count() < 2, reason="needs two GPUs")
+def test_inputs_of_another_gpu_than_the_weights_are_refused():
+    """On the host, before a launch: also after a call on the right GPU."""
+    z, s, far = torch.randn(40, 40, 128), torch.randn(40, 384), "cuda:1"
+    blk, ln = px.PairformerBlock().cuda().eval(), px.LayerNorm(128).cuda()
+    trunk = px.RecyclingTrunk(n_blocks=0).cuda().eval()
+    blk(s.cuda(), z.cuda(), None), ln(z.cuda()), trunk(s.cuda(), z.cuda())
+    for call in (lambda: blk(s.to(far), z.to(far), None), lambda: blk(s.to(far), z.cuda(), None), lambda: ln(z.to(far)),
+                 lambda: trunk(s.to(far), z.to(far)), lambda: px.dropout_add_rowwise(z.cuda(), z.to(far), 0.5, True)):
+        with pytest.raises(RuntimeError, match="same device|device of the other"):
+            call()
