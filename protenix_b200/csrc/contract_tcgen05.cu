@@ -5,8 +5,8 @@
 //
 // Bound by the operands' way from L2: a CTA of its own with a 128 x 256 tile takes 48 KB for every 512 cycles of products, 96 bytes a
 // cycle, where all SMs together get about 44 each.  So two CTAs on neighbouring SMs share a 256 x 256 tile (cta_group::2): each
-// loads its 128 rows of A and half of B's, 32 KB for the same products.  N = 437: 44.3 -> 39.7 us, 768: 114
-// -> 107, 1024: 256 -> 222, outer product of 384 tokens and 1024 sequences: 316 -> 254.  Results leave by TMA: 16-byte stores of
+// loads its 128 rows of A and half of B's, 32 KB for the same products.  N = 437: 49.3 -> 45.5 us, 768: 120 -> 107, 1024: 265
+// -> 235, outer product of 384 tokens and 1024 sequences: 266 -> 242; not everywhere, see pairs_pay.  Results leave by TMA: 16-byte stores of
 // rows, half a sector each, took 37.7 us in place of 27.0 at N = 384, 131 in place of 114 at N = 768.
 //
 // Persistent kernel, one CTA per SM, 192 threads (in brackets: what the leader of a pair does for both):
@@ -328,12 +328,18 @@ static int32_t launch_contract(const void* a, const void* b, void* x, int64_t ch
   return PX_ERR_LAUNCH;
 }
 
-// A pair works on 256 rows.  Where 128-row tiles would need an odd number, half a pair idles on the last: that costs more than the
-// pair saves up to five tiles (N = 384: 27.0 us single, 31.5 paired; 640: 77, 83) and less from nine on (1600: 1081, 1053).  Two tiles are short of work for
-// pairs (N = 200, beside another stream: 17.6 single, 19.1 paired).
-static bool pairs_pay(int64_t rows) {
-  const int64_t t = (rows + kTcBM - 1) / kTcBM;
-  return (t % 2 == 0 && t >= 4) || t >= 9;
+// A pair fetches a third less per product and takes longer to hand a tile over, so it pays where the way from L2 bounds the
+// tile: with a contraction long enough, the longer the better operand rows lie.  Rows of whole 128-byte lines come fastest, rows of whole
+// 32-byte sectors next, and others touch a sector more for every 128 bytes (us, single | paired; outer products of 300
+// tokens: 256 sequences 57.7 | 68.6, 448 78.6 | 80.3, 512 87.5 | 83.8, 1024 149 | 136; 240 0.97, 272 1.04 and 304 1.06 times as
+// fast in pairs; 136 70.0 | 70.5, 152 74.1 | 72.0, 500 134 | 110).  Few 128-row tiles leave half a pair idle on an odd last one (128 channels, N = 384: 31.1
+// | 37.2, 512: 45.5 | 47.5, 640: 84.5 | 88.4, 768: 120 | 107, 832: 182 | 177, 850: 284 | 239, 1152: 375 | 370, 1400: 1069
+// | 816; straddling rows, 390: 47.5 | 43.4, 520: 81.8 | 79.1, 344: 38.9 | 39.2), and with less than two tiles to an SM there is nothing to
+// hand over beside (outer products of 64 tokens, 1024 sequences: 16.5 | 17.4; 92, 400: 16.9 | 18.5; 100, 1000: 41.2 | 35.1).
+static bool pairs_pay(int64_t channels, int64_t rows_a, int64_t rows_b, int64_t ld_k) {
+  const int64_t t = (rows_a + kTcBM - 1) / kTcBM, tiles = channels * t * ((rows_b + kTcBN - 1) / kTcBN);
+  const bool lines = ld_k % 64 == 0, sectors = ld_k % 16 == 0;
+  return t >= (sectors ? 6 : 4) && ld_k >= (lines ? 448 : sectors ? 272 : 152) && tiles >= 2 * sm_count();
 }
 
 }  // namespace px
@@ -345,7 +351,7 @@ extern "C" int32_t px_trimul_contract(const px_bf16* a, const px_bf16* b, px_bf1
   if (!a || !b || !x || channels <= 0 || channels > 65535 || n <= 0 || n > 32768 || ld != px_ld(n))
     return PX_ERR_BAD_ARG;
   if (((uintptr_t)a | (uintptr_t)b | (uintptr_t)x) & 15) return PX_ERR_BAD_ARG;
-  return (pairs_pay(n) ? launch_contract<2> : launch_contract<1>)(a, b, x, channels, n, n, ld, ld, (cudaStream_t)stream);
+  return (pairs_pay(channels, n, n, ld) ? launch_contract<2> : launch_contract<1>)(a, b, x, channels, n, n, ld, ld, (cudaStream_t)stream);
 }
 
 // The same kernel for the outer product of the MSA module: one "channel", a_t [rows_a][ld_k] against
@@ -356,5 +362,5 @@ extern "C" int32_t px_opm_outer(const px_f16* a_t, const px_f16* b_t, px_f16* x,
       ld_k <= 0 || ld_k % 8 || ld_k > (1 << 20))
     return PX_ERR_BAD_ARG;
   if (((uintptr_t)a_t | (uintptr_t)b_t | (uintptr_t)x) & 15) return PX_ERR_BAD_ARG;
-  return (pairs_pay(rows_a) ? launch_contract<2> : launch_contract<1>)(a_t, b_t, x, 1, rows_a, rows_b, ld_k, rows_b, (cudaStream_t)stream);
+  return (pairs_pay(1, rows_a, rows_b, ld_k) ? launch_contract<2> : launch_contract<1>)(a_t, b_t, x, 1, rows_a, rows_b, ld_k, rows_b, (cudaStream_t)stream);
 }
