@@ -4,12 +4,12 @@
 // 393216 rows; 6 x that on the tensor core is 0.16 ms at its measured rate, and the rows (256 bytes in and out) 31 us.
 //
 // Persistent kernel, one CTA per SM, 128 rows per tile, three tiles in flight as in the pair transition:
-//   warps 0..7    SwiGLU of a 64-wide hidden chunk (lane quarter x half of the columns): h = silu(a) b, split, written back over
+//   warps 0..15   SwiGLU of a 64-wide hidden chunk (lane quarter x quarter of the columns): h = silu(a) b, split, written back over
 //                 the chunk's accumulator as the A operand of the second product (three planes of 32 columns)
-//   warps 8..11   LayerNorm: 16 lanes a row, split rows written as three swizzled planes (two buffers)
-//   warps 12..15  output: accumulators + residual, staged so that a warp's accesses cover 64 contiguous bytes of 8 rows
-//   warps 16, 19  TMA producers of the weight chunks ([W_a; W_b] two stages, W_out one; they come from L2 for every tile)
-//   warps 17, 18  MMA issuers of the first product (M=128, N=128) and of the second (M=128, N=64)
+//   warps 16..19  LayerNorm: 16 lanes a row, split rows written as three swizzled planes (two buffers)
+//   warps 20..23  output: accumulators + residual, staged so that a warp's accesses cover 64 contiguous bytes of 8 rows
+//   warps 24, 27  TMA producers of the weight chunks ([W_a; W_b] two stages, W_out one; they come from L2 for every tile)
+//   warps 25, 26  MMA issuers of the first product (M=128, N=128) and of the second (M=128, N=64)
 // The tensor core truncates on accumulation: the first product adds its corrections before its leading terms, the second has
 // an accumulator for each.  Tensor memory: H (2 x 128) | out, corrections (2 x 128).  Every wait is bounded.
 #include "px_split.cuh"
