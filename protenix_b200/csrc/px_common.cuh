@@ -53,10 +53,6 @@ template <>
 __device__ __forceinline__ float2 unpack16x2<false>(uint32_t u) {
   return unpack_bf16x2(u);
 }
-template <bool kF16>
-__device__ __forceinline__ uint16_t round16(float v) {
-  return kF16 ? __half_as_ushort(__float2half_rn(v)) : __bfloat16_as_ushort(__float2bfloat16_rn(v));
-}
 // (1, 1) as a pair of bf16 or of fp16
 __host__ __device__ constexpr uint32_t ones16x2(bool f16) { return f16 ? 0x3C003C00u : 0x3F803F80u; }
 

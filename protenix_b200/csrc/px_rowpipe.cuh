@@ -186,37 +186,6 @@ __device__ __forceinline__ void named_barrier(int id, int threads) {
   asm volatile("bar.sync %0, %1;\n" ::"r"(id), "r"(threads) : "memory");
 }
 
-// Mean and 1/std of one bf16 row already in the swizzled operand at `op` (row r), computed by two threads, each
-// over 64 channels (`half` = 0/1; the two threads are neighbouring lanes).  One pass: sums of (x - x0) and
-// (x - x0)^2 with the row's first element as pivot, which keeps the variance accurate when |mean| >> std.
-__device__ __forceinline__ void row_stats_from_operand(const unsigned char* op, int r, int half, float eps, float& mean,
-                                                       float& rstd) {
-  const float x0 = __uint_as_float(*reinterpret_cast<const uint32_t*>(op + operand_piece_offset(r, 0)) << 16);
-  float s0 = 0.f, s1 = 0.f, q0 = 0.f, q1 = 0.f;
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    // pieces 4*half..4*half+3 of both k panels: the 8 lanes of a quarter warp touch 8 distinct bank groups
-    const int p = ((i >> 2) << 3) + 4 * half + (i & 3);
-    const uint4 v = *reinterpret_cast<const uint4*>(op + operand_piece_offset(r, p));
-    const float2 a = unpack_bf16x2(v.x), b = unpack_bf16x2(v.y), c = unpack_bf16x2(v.z), d = unpack_bf16x2(v.w);
-    float e;
-    e = a.x - x0, s0 += e, q0 = fmaf(e, e, q0);
-    e = a.y - x0, s1 += e, q1 = fmaf(e, e, q1);
-    e = b.x - x0, s0 += e, q0 = fmaf(e, e, q0);
-    e = b.y - x0, s1 += e, q1 = fmaf(e, e, q1);
-    e = c.x - x0, s0 += e, q0 = fmaf(e, e, q0);
-    e = c.y - x0, s1 += e, q1 = fmaf(e, e, q1);
-    e = d.x - x0, s0 += e, q0 = fmaf(e, e, q0);
-    e = d.y - x0, s1 += e, q1 = fmaf(e, e, q1);
-  }
-  float s = s0 + s1, q = q0 + q1;
-  s += __shfl_xor_sync(0xffffffffu, s, 1);
-  q += __shfl_xor_sync(0xffffffffu, q, 1);
-  const float m = s * (1.0f / kC);
-  mean = x0 + m;
-  rstd = rsqrtf(fmaxf(q * (1.0f / kC) - m * m, 0.f) + eps);
-}
-
 // ---------------------------------------------------------------------------------------------------------------
 // Row tiles: the part of the pipeline that is the same for every kernel that consumes LayerNorm'd pair rows.
 // A tile is 128 pair elements (one u, 128 consecutive t); element (u, t) is row u*n_t + t of z, or row t*n_u + u when
