@@ -547,7 +547,7 @@ Tensor tri_mul_forward(Params& params, const Tensor& z, const OptTensor& mask, b
   return batch ? out.unsqueeze(0) : out;
 }
 
-Tensor tri_att_forward(Params& params, const Tensor& z, const OptTensor& mask, bool ending) {
+Tensor tri_att_forward(Params& params, const Tensor& z, const OptTensor& mask, bool ending, bool inplace_add) {
   bool batch;
   const Tensor zc = pair_tensor(z, batch);
   c10::cuda::CUDAGuard guard(zc.device());
@@ -555,15 +555,15 @@ Tensor tri_att_forward(Params& params, const Tensor& z, const OptTensor& mask, b
   const Tensor m = pair_mask(mask, zc);
   const Ready pr = params.get(zformat(zc), Use(zc.device()));
   py::gil_scoped_release release;
-  const Tensor out = at::empty_like(zc);
+  const Tensor out = inplace_add && zc.data_ptr() == z.data_ptr() ? zc : at::empty_like(zc);
   const Tensor ws = bytes_like(zc, abi.px_triatt_workspace_bytes(zc.size(0)));
   const PairCall c{zc.size(0), zformat(zc), dtype_code(zc, "z"), fptr(m), (unsigned char*)ws.data_ptr(), at::cuda::getCurrentCUDAStream()};
   Rows rows = own_rows(c, ws);
-  tri_att(c, *pr, zc.data_ptr(), out.data_ptr(), ending, false, rows);
+  tri_att(c, *pr, zc.data_ptr(), out.data_ptr(), ending, inplace_add, rows);
   return batch ? out.unsqueeze(0) : out;
 }
 
-Tensor transition_forward(Params& params, const Tensor& x) {
+Tensor transition_forward(Params& params, const Tensor& x, bool inplace_add) {
   need_cuda(x, "x");
   if (x.dim() < 1 || x.size(-1) != kCz) fail("transition kernel handles [..., 128] rows");
   c10::cuda::CUDAGuard guard(x.device());
@@ -571,9 +571,9 @@ Tensor transition_forward(Params& params, const Tensor& x) {
   const Tensor xc = x.contiguous();
   const Ready pr = params.get(zformat(xc), Use(xc.device()));
   py::gil_scoped_release release;
-  const Tensor out = at::empty_like(xc);
+  const Tensor out = inplace_add && xc.data_ptr() == x.data_ptr() ? xc : at::empty_like(xc);
   transition_rows(at::cuda::getCurrentCUDAStream(), *pr, zformat(xc), dtype_code(xc, "x"), xc.data_ptr(), out.data_ptr(),
-                  xc.numel() / kCz, false);
+                  xc.numel() / kCz, inplace_add);
   return out;
 }
 

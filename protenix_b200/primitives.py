@@ -89,15 +89,21 @@ class Transition(nn.Module):
                 self.linear_no_bias.weight)
 
     def forward_residual_(self, x: torch.Tensor) -> torch.Tensor:
-        """x += Transition(x) in place (pair path of the Pairformer block)."""
+        """x += Transition(x) in place on a contiguous fp32 or bf16 tensor of pair rows."""
+        if x.is_cuda and x.is_contiguous() and self._fused_ok(x):
+            return self._native_forward(x, True)
         ops.transition(x, x, *self._weights(), add_residual=True)
         return x
+
+    def _native_forward(self, x: torch.Tensor, inplace_add: bool) -> torch.Tensor:
+        params = native.kept(self, lambda: native.params(self, *self.NATIVE))
+        return native.load().transition_forward(params, x, inplace_add)
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         if not x.is_cuda:
             raise RuntimeError("Transition: CUDA tensors only (no CPU path)")
         if self._fused_ok(x):
-            return native.load().transition_forward(native.kept(self, lambda: native.params(self, *self.NATIVE)), x)
+            return self._native_forward(x, False)
         # small widths (single representation, c_in = 384): LayerNorm kernel + library GEMMs, fp32 arithmetic whatever
         # the storage type of x and of the parameters
         y = self.layernorm1(x.float().contiguous())

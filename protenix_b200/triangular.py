@@ -113,8 +113,10 @@ class TriangleMultiplicativeUpdate(BaseTriangleMultiplicativeUpdate):
                 self.linear_g.weight)
 
     def apply_(self, z: torch.Tensor, mask: Optional[torch.Tensor], zn: Optional[torch.Tensor] = None) -> torch.Tensor:
-        """z += update, in place, on a contiguous [N,N,128] tensor (used by the block).  ``zn``: the standardised
-        fp16 copy of an fp32 z, if the caller has it."""
+        """z += update, in place, on a contiguous [N,N,128] tensor.  ``zn``: the standardised fp16 copy of an fp32 z, if the
+        caller has it; the tensor wrappers take it."""
+        if zn is None and z.is_contiguous():
+            return self.forward(z, mask, inplace_safe=True, _add_with_inplace=True)
         ops.triangle_multiplication(z, z, mask, *self._kernel_args(), incoming=not self._outgoing,
                                     add_residual=True, eps=self.layer_norm_in.eps, zn=zn)
         return z
@@ -189,16 +191,21 @@ class TriangleAttention(nn.Module):
                zn: Optional[torch.Tensor] = None) -> torch.Tensor:
         """z += update in place; ``ending`` selects attention along columns of the *untransposed* z,
         which equals the reference's transpose / starting-node / transpose sequence
-        (protenix/model/modules/pairformer.py:160-168)."""
+        (protenix/model/modules/pairformer.py:160-168).  ``zn`` as for the triangle multiplication."""
+        if zn is None and z.is_contiguous():
+            return self._native_forward(z, mask, ending, True)
         ops.triangle_attention(z, z, mask, *self._kernel_args(), ending=ending, add_residual=True,
                                eps=self.layer_norm.eps, inf=self.inf, zn=zn)
         return z
 
     def forward(self, x: torch.Tensor, mask: Optional[torch.Tensor] = None, chunk_size: Optional[int] = None,
                 triangle_attention: str = "torch", inplace_safe: bool = False) -> torch.Tensor:
+        return self._native_forward(x, mask, not self.starting, False)
+
+    def _native_forward(self, x, mask, ending: bool, inplace_add: bool) -> torch.Tensor:
         self._check_shape()
         params = native.kept(self, lambda: native.params(self, *self.NATIVE))
-        return native.load().tri_att_forward(params, x, mask, not self.starting)
+        return native.load().tri_att_forward(params, x, mask, ending, inplace_add)
 
 
 TriangleAttentionStartingNode = TriangleAttention

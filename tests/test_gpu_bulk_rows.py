@@ -1,4 +1,6 @@
-"""fp32 rows that leave by TMA (added in place, or without a residual) against the plain accesses (residual in another tensor)."""
+"""The ways in which the output stages' rows leave give the same bits: added in place, stored without a residual, and with the residual of
+another tensor.  The triangle kernels write fp32 rows of the last kind with plain accesses, everything else leaves by TMA (the transition
+has its residual fetched by TMA into the staging area).  The modules' in-place forms and the tensor wrappers agree as well."""
 import pytest
 import torch
 
@@ -37,11 +39,15 @@ def test_stored_added_and_plain_rows_agree(n):
             ops.device_error_flags()
             assert torch.equal(added, plain), name
             assert torch.equal(z + update, plain), name
+            zm = z.clone()
+            same = (mul.apply_(zm, mask) if name == "mul" else tr.forward_residual_(zm) if name == "transition" else
+                    mod.apply_(zm, mask, ending=name == "end"))
+            assert same.data_ptr() == zm.data_ptr() and torch.equal(zm, plain), name
 
 
 @pytest.mark.parametrize("rows", [1, 31, 128, 129, 1000])
 def test_bf16_transition_without_residual(rows):
-    """bf16 rows stored by TMA against the plain accesses, which add the residual before they round."""
+    """bf16 rows: the update alone is the fp32 one rounded, and a residual is added before the rounding."""
     torch.manual_seed(rows)
     x = torch.randn(rows, 128, device="cuda").bfloat16()
     tr = randomize_parameters_(px.Transition(c_in=128, n=4), 5).cuda().eval()
