@@ -241,15 +241,16 @@ def kernel_algo(n: int, zbytes: int, n_msa: int = 1024) -> dict:
 # captures at N = 768 with an fp32 z summarised under profiles/ (<kernel>_N768.md).  For these kernels traffic grows
 # with N^2 (operands of the N^3 kernels are re-read from L2, not DRAM), so a launch at another N is scaled by N^2.
 NCU_TRAFFIC_PER_PAIR = {
-    "px_triatt_flash": 596.6e6 / 768 ** 2,
-    "px_transition": 551.6e6 / 768 ** 2,
-    "px_trimul_contract": 420.1e6 / 768 ** 2,
-    "px_trimul_in_proj": 399.0e6 / 768 ** 2,
-    "px_trimul_out": 877.6e6 / 768 ** 2,
-    "px_triatt_in_proj": 563.4e6 / 768 ** 2,
-    "px_triatt_out": 863.3e6 / 768 ** 2,
-    "px_standardise_rows": 399.8e6 / 768 ** 2,
-    "px_recycle_update": 728.3e6 / 768 ** 2,
+    "px_triatt_flash": 602.5e6 / 768 ** 2,
+    "px_transition": 547.0e6 / 768 ** 2,
+    "px_trimul_contract": 424.1e6 / 768 ** 2,
+    "px_trimul_in_proj": 395.8e6 / 768 ** 2,
+    "px_trimul_out": 856.9e6 / 768 ** 2,
+    "px_triatt_in_proj": 561.7e6 / 768 ** 2,
+    "px_triatt_out": 851.2e6 / 768 ** 2,
+    "px_standardise_rows": 398.5e6 / 768 ** 2,
+    "px_pair_bias_proj": 172.7e6 / 768 ** 2,
+    "px_recycle_update": 728.4e6 / 768 ** 2,
 }
 
 
@@ -457,8 +458,8 @@ def side_size_record(stack, sharded, dev, world: int, rank: int, zdt, args) -> d
         ms = float(tt.item())
         sub.close()
     return {"n_token": n, "blocks": nb, "ms_per_block": ms / nb, "token_pairs_per_s": n * n * nb / (ms * 1e-3),
-            "note": "z is 75 MB at this size (< L2): every step starts with a copy of z over the working tensor, and a "
-                    "block's intermediates (1.1 GB) exceed L2"}
+            "note": f"z is {n * n * 128 * z0.element_size() >> 20} MiB at this size, more than L2; every step starts with a copy of z "
+                    "over the working tensor"}
 
 
 def main() -> None:
