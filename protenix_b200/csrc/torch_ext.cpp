@@ -5,9 +5,10 @@
 // representation 18 us for a 3 us kernel.  Here a module keeps a `Params` object: the places of its parameters (the
 // module's own `_parameters` dictionaries), what was seen there last, and the forms the kernels want (fp32 vectors,
 // 16-bit matrices, the split planes of the single branch), renewed when a parameter, its storage, its version or a
-// submodule has changed (what is written past the version counter has to be announced: weights.py).  A call checks its tensors, looks the parameters over (some tens of pointer comparisons) and
-// issues the launches through the C ABI of px_b200.h, whose functions are taken from the library handle that the Python
-// side has loaded.  Workspaces come from the caching allocator on each call.
+// submodule has changed (what is written past the version counter has to be announced: weights.py).  A call checks its
+// tensors, looks the parameters over (some tens of pointer comparisons) and issues the launches through the C ABI of
+// px_b200.h, whose functions are taken from the library handle that the Python side has loaded.  Workspaces come from the
+// caching allocator on each call.
 #include <ATen/ATen.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <ATen/cuda/CUDAEvent.h>
@@ -26,6 +27,7 @@
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/utils/pybind.h>
 
+#include <algorithm>
 #include <atomic>
 #include <mutex>
 #include <stdexcept>
@@ -273,22 +275,20 @@ class Params {
   // it, so every stream may use it.  Inside a capture nothing can be laid out, since the graph's replays alone would write it.
   Ready get(int zf, const Use& use) {
     GraphHeld::free_released();
-    bool same = prepared_ != nullptr;
+    c10::SmallVector<py::object, 16> objects;      // held, since a computed one runs Python code, and other threads with it
+    for (const auto& s : params_) objects.push_back(parameter(s));
+    c10::SmallVector<float, 4> scalars;
+    for (const auto& s : scalars_) scalars.push_back(py::getattr(PyWeakref_GetObject(s.owner.ptr()), s.key).cast<float>());
+    bool same = prepared_ != nullptr && std::equal(scalars.begin(), scalars.end(), prepared_->scalars.begin());
     c10::SmallVector<Seen, 16> now(params_.size());
-    std::vector<py::object> elsewhere;       // keeps what is not a registered parameter, which may be computed on each look
     for (size_t i = 0; i < params_.size(); ++i) {
-      PyObject* o = parameter(params_[i], elsewhere);
+      PyObject* const o = objects[i].ptr();
       if (o != Py_None) {
         if (!THPVariable_Check(o)) fail("a module parameter is not a tensor");
         const Tensor& t = THPVariable_Unpack(o);
         now[i] = {o, t.data_ptr(), t.storage().unsafeGetStorageImpl(), (uint32_t)t._version(), t.scalar_type()};
       }
       same = same && now[i] == seen_[i];
-    }
-    c10::SmallVector<float, 4> scalars;
-    for (const auto& s : scalars_) {
-      scalars.push_back(py::getattr(PyWeakref_GetObject(s.owner.ptr()), s.key).cast<float>());
-      same = same && prepared_->scalars[scalars.size() - 1] == scalars.back();
     }
     if (use.graph && !(same && prepared_->have[zf]))
       fail("the weights are new to this module, or have changed, and cannot be laid out inside a graph capture: call the module once "
@@ -297,12 +297,10 @@ class Params {
       prepared_ = std::make_shared<Prepared>();
       prepared_->scalars.assign(scalars.begin(), scalars.end());
       seen_.assign(now.begin(), now.end());
-      params_hold_.clear();
+      params_hold_.assign(objects.begin(), objects.end());
       storages_.clear();
-      for (const Seen& n : now) {
-        params_hold_.push_back(py::reinterpret_borrow<py::object>(n.object ? n.object : Py_None));
+      for (const Seen& n : now)
         if (n.object) storages_.push_back(THPVariable_Unpack(n.object).storage().getWeakStorageImpl());
-      }
     }
     if (!prepared_->have[zf]) make(*prepared_, zf, use);
     if (prepared_->dev != use.dev) fail("parameters and inputs must be on the same device");
@@ -332,11 +330,10 @@ class Params {
   }
   // A parameter as the module's attribute gives it: registered (the usual case, looked up directly), or a plain attribute or a property
   // (flattened, replicated and parametrised modules).
-  static PyObject* parameter(const Slot& s, std::vector<py::object>& elsewhere) {
-    if (PyObject* o = PyDict_GetItemWithError(s.dict.ptr(), s.key.ptr())) return o;
+  static py::object parameter(const Slot& s) {
+    if (PyObject* o = PyDict_GetItemWithError(s.dict.ptr(), s.key.ptr())) return py::reinterpret_borrow<py::object>(o);
     if (PyErr_Occurred()) throw py::error_already_set();
-    elsewhere.push_back(py::getattr(PyWeakref_GetObject(s.owner.ptr()), s.key));
-    return elsewhere.back().ptr();
+    return py::getattr(PyWeakref_GetObject(s.owner.ptr()), s.key);
   }
 
   // The allocator knows the stream of make(); every other one is told to it once, and asked of when the set is freed.
