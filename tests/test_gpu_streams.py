@@ -1,4 +1,6 @@
 """Weights kept between calls, used and renewed on several streams."""
+import threading
+
 import pytest
 import torch
 
@@ -62,3 +64,32 @@ def test_16_bit_copies_across_streams():
     assert torch.equal(junk[0], p.detach().half())
     if not waiting:
         pytest.skip("the host took longer than the delay: nothing was in flight")
+
+
+def test_threads_share_a_module_while_its_weights_are_renewed():
+    """Several threads call one stack on streams of their own; one of them lays the (same) weights out anew again and again."""
+    n = 40
+    stack = randomize_parameters_(px.PairformerStack(n_blocks=2), 3).cuda().eval()
+    inputs = [(torch.randn(n, 384, device="cuda"), torch.randn(n, n, 128, device="cuda")) for _ in range(4)]
+    want = [stack(s, z, None) for s, z in inputs]
+    torch.cuda.synchronize()
+    wrong = []
+
+    def work(i):
+        stream = torch.cuda.Stream()
+        with torch.cuda.stream(stream):
+            for k in range(30):
+                if i == 0:
+                    px.weights_changed(stack)
+                got = stack(*inputs[i], None)
+                stream.synchronize()
+                if not all(torch.equal(a, b) for a, b in zip(got, want[i])):
+                    wrong.append((i, k))
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    ops.device_error_flags()
+    assert not wrong
