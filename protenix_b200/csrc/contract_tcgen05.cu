@@ -93,7 +93,7 @@ trimul_contract_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
   // operand ring first (1024-byte aligned for the 128-byte swizzle), staging and barriers after it
   unsigned char* ring = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   TcBarriers& bars = *reinterpret_cast<TcBarriers*>(ring + Shape::kBars);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const int nk = (ld_k + kTcBK - 1) / kTcBK;      // ld_k: extent of the contraction index; ld: row stride of x
   const uint32_t rank = kPair ? cluster_rank() : 0;
   const int first_tile = blockIdx.x / kCtas, tile_step = gridDim.x / kCtas;
@@ -150,7 +150,7 @@ trimul_contract_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
   if (stop) {
     // nothing
   } else if (warp == 0) {
-    if (lane == 0) {
+    if (elect_lane()) {
       uint32_t it = 0;
       bool ok = true;
       for (int tile = first_tile; tile < total_tiles && ok; tile += tile_step) {
@@ -176,7 +176,7 @@ trimul_contract_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
       }
     }
   } else if (warp == 1) {
-    if (lane == 0 && rank == 0) {
+    if (elect_lane() && rank == 0) {
       constexpr uint32_t idesc = umma_idesc_f16(kTcBM * kCtas, kTcBN);
       uint32_t it = 0, tcount = 0;
       bool ok = true;

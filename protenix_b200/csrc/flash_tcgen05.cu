@@ -107,7 +107,7 @@ triatt_flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* sm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   FlashBars& bars = *reinterpret_cast<FlashBars*>(sm + FlashLayout::bars);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const int q0 = blockIdx.x * 128, h = blockIdx.y, u0 = blockIdx.z * kFRows;
 
   const bool skip = cta_begin();         // an earlier bounded wait gave up: do not start new work
@@ -140,7 +140,7 @@ triatt_flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     asm volatile("setmaxnreg.dec.sync.aligned.u32 40;\n");   // registers go to the softmax warpgroups (with 24 the
                                                              // control threads spill: 6.02 ms against 5.91 at N=1536)
     const int g = warp - 4 * kFGroups;
-    if (g == kFGroups && lane == 0) {
+    if (g == kFGroups && elect_lane()) {
       // ---------------------------------------------------------------- pair-bias loader (all six rows share a tile)
       for (int kt = 0; kt < nkt; ++kt) {
         const int b = kt & 1;
@@ -150,7 +150,7 @@ triatt_flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
           tma_load_3d(smem_u32(sm + FlashLayout::bias + b * kFBiasBytes + c * (128 * 128)), &map_b, &bars.bias_full[b],
                       kt * kFKT + c * 32, q0, h);
       }
-    } else if (g < kFGroups && lane == 0) {
+    } else if (g < kFGroups && elect_lane()) {
       constexpr uint32_t idesc_s = umma_idesc_f16(128, kFKT), idesc_o = umma_idesc_f16(128, kFON);
       const int n_items = nkt * kFRpg;              // work item i = (key tile i / 3, row i % 3 of the group)
       const uint32_t q_addr = smem_u32(sm + FlashLayout::q + g * kFRpg * kFQBytes);

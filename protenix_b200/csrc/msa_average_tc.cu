@@ -67,7 +67,7 @@ msa_average_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* sm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   MvBars& bars = *reinterpret_cast<MvBars*>(sm + MvLayout::bars);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const int first_tile = blockIdx.x, tile_step = gridDim.x;
 
   const bool skip = cta_begin();
@@ -90,8 +90,8 @@ msa_average_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
   const uint32_t tmem_base = bars.tmem_base;
 
   if (warp >= 4) {
-    if (lane != 0) {
-      // nothing: the control threads are lane 0 of their warps
+    if (!elect_lane()) {
+      // nothing: one elected lane of each control warp works
     } else if (warp == 4) {
       int it = 0;
       bool ok = true;

@@ -70,7 +70,7 @@ msa_rows_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* sm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   MrBars& bars = *reinterpret_cast<MrBars*>(sm + MrLayout::bars);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const int first_tile = blockIdx.x, tile_step = gridDim.x;
 
   const bool skip = cta_begin();
@@ -99,8 +99,8 @@ msa_rows_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
 
   if (warp >= 20) {
     constexpr uint32_t idesc = umma_idesc_bf16(128, kMrC);
-    if (lane != 0 || (warp == 21 && kMode != kMrGate)) {
-      // nothing: the control threads are lane 0 of their warps
+    if (!elect_lane() || (warp == 21 && kMode != kMrGate)) {
+      // nothing: one elected lane of each control warp works
     } else if (warp == 20) {
       mbar_expect_tx(&bars.w_full, kMode == kMrGate ? 2 * kMrWBytes : kMrWBytes);
       tma_load_3d(smem_u32(sm + MrLayout::w), &map_w, &bars.w_full, 0, 0, 0);

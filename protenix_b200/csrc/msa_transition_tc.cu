@@ -46,7 +46,7 @@ msa_transition_tc_kernel(const __grid_constant__ CUtensorMap map_w1, const __gri
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* sm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   MtBars& bars = *reinterpret_cast<MtBars*>(sm + MtLayout::bars);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const int first_tile = blockIdx.x, tile_step = gridDim.x;
 
   const bool skip = cta_begin();
@@ -76,8 +76,8 @@ msa_transition_tc_kernel(const __grid_constant__ CUtensorMap map_w1, const __gri
   const uint32_t tmem_base = bars.tmem_base;
 
   if (warp >= kMtGate + 8) {
-    if (lane != 0) {
-      // nothing: the control threads are lane 0 of their warps
+    if (!elect_lane()) {
+      // nothing: one elected lane of each control warp works
     } else if (warp == kMtGate + 8) {
       int j = 0;
       bool ok = true;

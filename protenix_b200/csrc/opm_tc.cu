@@ -51,7 +51,7 @@ opm_out_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* sm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   OpBars& bars = *reinterpret_cast<OpBars*>(sm + OpLayout::bars);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
 
   const bool skip = cta_begin();         // an earlier bounded wait gave up: do not start new work
   if (threadIdx.x == 0) {
@@ -75,7 +75,7 @@ opm_out_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
   const uint32_t tmem_base = bars.tmem_base;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_lane()) {
       uint32_t it = 0;
       bool ok = true;
       for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
@@ -92,7 +92,7 @@ opm_out_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_lane()) {
       constexpr uint32_t idesc = umma_idesc_f16(128, 128);
       uint32_t it = 0, tcount = 0;
       bool ok = true;

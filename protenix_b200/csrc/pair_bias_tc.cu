@@ -62,7 +62,7 @@ pair_bias_tc_kernel(const __grid_constant__ CUtensorMap map_z, const PbWeights<k
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* sm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   PbBars& bars = *reinterpret_cast<PbBars*>(sm + PbLayout::bars);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   TileCtx ctx;
   ctx.tiles = sm + PbLayout::a;
   ctx.extras = sm + PbLayout::ax;
@@ -99,7 +99,7 @@ pair_bias_tc_kernel(const __grid_constant__ CUtensorMap map_z, const PbWeights<k
   const uint32_t tmem_base = bars.tmem_base;
 
   if (warp >= 8) {
-    if (lane == 0) {
+    if (elect_lane()) {
       if (warp == 8) {
         tile_producer_loop(ctx, &map_z);
       } else if (warp == 9) {

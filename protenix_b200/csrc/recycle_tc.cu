@@ -54,7 +54,7 @@ recycle_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_consta
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* sm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   RcBars& bars = *reinterpret_cast<RcBars*>(sm + RcLayout::bars);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   TileCtx ctx;
   ctx.tiles = sm + RcLayout::a;
   ctx.extras = sm + RcLayout::ax;
@@ -96,7 +96,7 @@ recycle_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_consta
   const uint32_t tmem_base = bars.tmem_base;
 
   if (warp >= 12) {
-    if (lane == 0) {
+    if (elect_lane()) {
       if (warp == 12) {
         // z tile into the operand ring and (bf16) the z_init tile into the output ring
         int k = 0;

@@ -108,7 +108,7 @@ split_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* ring = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   SgBars& bars = *reinterpret_cast<SgBars*>(ring + kSgStages * kSgStageBytes);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const int n0 = blockIdx.x * kSgBN, m0 = blockIdx.y * 128, kc0 = blockIdx.z * g.chunks;
 
   const bool stop = cta_begin();                 // an earlier bounded wait gave up: do no work, but meet the barriers
@@ -144,7 +144,7 @@ split_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
   bool ok = !skip;
 
   if (warp == 0) {
-    if (lane == 0 && ok) {
+    if (elect_lane() && ok) {
       for (int i = 0; i < g.chunks; ++i) {
         const int s = i % kSgStages;
         if (!mbar_wait(&bars.empty[s], ((i / kSgStages) & 1) ^ 1, 1u)) break;
@@ -157,7 +157,7 @@ split_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
       }
     }
   } else if (warp <= kSgIssuers) {
-    if (lane == 0 && ok) {
+    if (elect_lane() && ok) {
       // planes (i, j) with i + j <= 2, the terms above 2^-24 of the product: (0,0) (0,1) | (1,0) (1,1) | (0,2) (2,0)
       const int w_ = warp - 1;
       const int ai0 = w_ == 1 ? 1 : 0, aj0 = w_ == 2 ? 2 : 0, ai1 = w_, aj1 = w_ == 2 ? 0 : 1;

@@ -76,7 +76,7 @@ transition_tc_kernel(const __grid_constant__ CUtensorMap map_wa, const __grid_co
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* sm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   TransBars& bars = *reinterpret_cast<TransBars*>(sm + TransLayout::bars);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const int first_tile = blockIdx.x, tile_step = gridDim.x;
 
   const bool skip = cta_begin();         // an earlier bounded wait gave up: do not start new work
@@ -107,8 +107,8 @@ transition_tc_kernel(const __grid_constant__ CUtensorMap map_wa, const __grid_co
   const uint32_t tmem_base = bars.tmem_base;
 
   if (warp >= 16) {
-    if (lane != 0) {
-      // nothing: the control threads are lane 0 of their warps
+    if (!elect_lane()) {
+      // nothing: one elected lane of each control warp works
     } else if (warp == 16) {
       // ---------------------------------------------------------------- weight producer
       int j = 0;                                      // chunk counter over all tiles of this CTA

@@ -85,7 +85,7 @@ triatt_in_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_cons
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* sm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   AiBars& bars = *reinterpret_cast<AiBars*>(sm + AiLayout::bars);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const int hpair = blockIdx.x & 1;                      // this CTA's heads: 2*hpair, 2*hpair + 1
   TileCtx ctx;
   ctx.tiles = sm + AiLayout::a;
@@ -126,7 +126,7 @@ triatt_in_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_cons
   const uint32_t tmem_base = bars.tmem_base;
 
   if (warp >= 20) {
-    if (lane == 0) {
+    if (elect_lane()) {
       if (warp == 20) {
         tile_producer_loop(ctx, &map_z);
       } else if (warp == 23) {

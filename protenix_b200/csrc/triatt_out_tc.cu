@@ -79,7 +79,7 @@ triatt_out_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_con
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* sm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   AoBars& bars = *reinterpret_cast<AoBars*>(sm + AoLayout::bars);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   TileCtx ctx;
   ctx.tiles = sm + AoLayout::a;
   ctx.extras = sm + AoLayout::ax;
@@ -121,7 +121,7 @@ triatt_out_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_con
   const uint32_t tmem_base = bars.tmem_base;
 
   if (warp >= 20) {
-    if (lane == 0) {
+    if (elect_lane()) {
       if (warp == 20) {
         // ---------------------------------------------------------------- tile producer: z (bf16 rows) and o
         int k = 0;

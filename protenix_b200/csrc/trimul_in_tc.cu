@@ -80,7 +80,7 @@ trimul_in_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_cons
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* sm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   TiBars& bars = *reinterpret_cast<TiBars*>(sm + TiLayout::bars);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const int chan0 = 64 * (blockIdx.x & 1);               // this CTA's channels of a and b
   TileCtx ctx;
   ctx.tiles = sm + TiLayout::a;
@@ -121,7 +121,7 @@ trimul_in_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_cons
   const uint32_t tmem_base = bars.tmem_base;
 
   if (warp >= 20) {
-    if (lane == 0) {
+    if (elect_lane()) {
       if (warp == 20) {
         tile_producer_loop(ctx, &map_z);
       } else if (warp == 23) {

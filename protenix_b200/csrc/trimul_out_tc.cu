@@ -92,7 +92,7 @@ trimul_out_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_con
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* sm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   ToBars& bars = *reinterpret_cast<ToBars*>(sm + ToLayout::bars);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
 
   const bool skip = cta_begin();         // an earlier bounded wait gave up: do not start new work
   if (threadIdx.x == 0) {
@@ -127,7 +127,7 @@ trimul_out_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_con
   const int first_tile = blockIdx.x, tile_step = gridDim.x;
 
   if (warp >= 20) {
-    if (lane == 0) {
+    if (elect_lane()) {
       if (warp == 20) {
         // ---------------------------------------------------------------- tile producer: z (bf16 rows) and x
         int k = 0;
