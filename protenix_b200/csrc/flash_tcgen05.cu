@@ -6,25 +6,26 @@
 // fp16 keeps three more bits than bf16), the pair bias, the logits, the softmax and the accumulators fp32.
 //
 // One CTA = (head h, 128 queries, 6 attended rows u), 16 warps:
-//   warps 0..11   three softmax groups of four warps; group g owns rows u0+2g, u0+2g+1, each thread one query row.
-//                 The kernel is bound by the latency of a group's chain (wait S, load, add, reduce, exponentials,
-//                 store P), not by any one unit, so three groups are kept in flight per SM.  Per work item a thread
-//                 adds its 64 pair-bias values from the shared tile (the bias does not depend on u: all six rows
-//                 use the same tile), and keeps the softmax denominator of its row in a register.
-//   warps 12..14  one control thread per group (tcgen05 and TMA instructions cost ~100 cycles of issue each, so
-//                 one issuing thread for all groups would be the bottleneck).  It loads the group's Q tiles once
+//   warps 0..11   three softmax groups of four warps; group g owns rows u0+2g, u0+2g+1, each thread one query row and
+//                 the softmax denominator of it.  The pair bias does not depend on u: all six rows use the same tile.
+//   warps 12..14  one control warp per group, whose elected lane issues.  It loads the group's Q tiles once
 //                 and, per work item, a K tile [64 keys][32] (64-byte swizzle) and a transposed V tile
-//                 [32 d][64 keys] (128-byte swizzle) into the group's 4-stage ring; issues S = Q K^T (M=128, N=64,
-//                 K=32) into the group's S buffer in tensor memory; and, once the group has written P (fp16) into
-//                 its P buffer, issues O_u += P V with P as the TMEM-resident A operand (M=128, N=32, K=64).  S of
-//                 the next item is issued as soon as the group has pulled the current S into registers, so it is
-//                 ready when the group comes back.
-//   warp 15       one thread loads the pair-bias tiles [128 q][64 k] fp32 (two 128-byte-swizzled boxes, 2-deep ring).
+//                 [32 d][64 keys] (128-byte swizzle) into the group's 4-stage ring; copies the pair bias of the first 32
+//                 keys into the group's S buffer in tensor memory and adds Q K^T (M=128, N=64, K=32) to it; and, once the
+//                 group has written P (fp16) into its P buffer, issues O_u += P V with P as the TMEM-resident A operand
+//                 (M=128, N=32, K=64).  S of the next item is issued as soon as the group has pulled the current S into
+//                 registers, so it is ready when the group comes back.  The bias of the other 32 keys is added by the softmax
+//                 threads, which leave zeros in those columns for the next product.
+//   warp 15       loads the pair-bias tiles [128 q][64 k] fp32 (two 128-byte-swizzled boxes, 2-deep ring).
 // Tensor memory: S (3 x 64) | P (3 x 32, two fp16 per column) | O (6 x 32).
 //
-// Letting the tensor core add the bias (S += I B with an identity operand and the bias tile as an MN-major fp16
-// operand: eight more MMAs per item) was measured and lost: 7.8 ms against 6.3 ms at N=1536.  The 48 instructions
-// it takes off every softmax thread weigh less than the ten MMA issues it puts on the group's control thread.
+// What bounds it (per item of 128 queries x 64 keys, 800 cycles at N = 1536): nothing alone.  Tensor pipe 416 (a copy
+// of 8 columns takes 64 cycles, S 96, P V 64), special-function unit 384, issue slots 440, L2 29 bytes a cycle and SM at most
+// (with the arithmetic taken out 457 cycles are left, of L2 traffic).  Hence the bias split in halves: all 64 columns copied
+// make the tensor pipe 80 % busy and S late (N = 384 118.7 us against 110.4, N = 1536 level), none copied is 48 more
+// instructions of 400 per softmax thread (123.5, 5.61 ms against 5.06).  24 or 40 columns: as 32 within 1 %.  Writing the bias
+// into S from the softmax threads for the next item: 5.32 ms (a store and its wait are on the group's chain).  Four groups of
+// one row: 5.15 to 7.0 ms.  Exponentials without the cubic 5.52, every third pair 5.02, every second 5.26, a quartic 5.08.
 //
 // Softmax is online in base 2 with a lazy reference maximum: the reference only moves (and O_u is rescaled
 // through TMEM) when the tile maximum exceeds it by more than 8, so probabilities stay below 2^8.
@@ -41,6 +42,7 @@ constexpr int kFGroups = 3;               // softmax groups per CTA
 constexpr int kFRpg = 2;                  // attended rows per group
 constexpr int kFRows = kFGroups * kFRpg;  // attended rows per CTA
 constexpr int kFKT = 64;                  // keys per work item
+constexpr int kFCopied = 32;              // columns of S that are laid out with the pair bias before the product (a copy into tensor memory)
 constexpr int kFStages = 4;               // K/V ring of each group (work items = (key tile, row))
 constexpr int kFQBytes = 128 * 64;        // [128][32] fp16
 constexpr int kFKBytes = kFKT * 64;       // [64][32] fp16
@@ -54,6 +56,7 @@ constexpr int kFColS = 0, kFColP = kFGroups * kFKT, kFColO = kFColP + kFGroups *
 constexpr float kRescaleGap = 8.0f;
 constexpr int kFThreads = 32 * (4 * kFGroups + 4);
 static_assert(kFColO + kFRows * kFON <= 512, "tensor memory budget");
+static_assert(kFCopied == 32 && kFKT == 64, "the copied columns are one box of the bias tile, the others one store");
 
 struct FlashBars {
   uint64_t q_full[kFGroups], kv_full[kFGroups][kFStages], bias_full[2], bias_empty[2], s_full[kFGroups],
@@ -114,7 +117,7 @@ triatt_flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
   if (threadIdx.x == 0) {
     for (int b = 0; b < 2; ++b) {
       mbar_init(&bars.bias_full[b], 1);
-      mbar_init(&bars.bias_empty[b], 4 * kFGroups);
+      mbar_init(&bars.bias_empty[b], 5 * kFGroups);     // four softmax warps and the copies of each group
     }
     for (int g = 0; g < kFGroups; ++g) {
       mbar_init(&bars.q_full[g], 1);
@@ -136,74 +139,90 @@ triatt_flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
   const uint32_t tmem_base = bars.tmem_base;
 
   if (warp >= 4 * kFGroups) {
-    // ------------------------------------------------------------------ control thread of group g
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 40;\n");   // registers go to the softmax warpgroups (with 24 the
-                                                             // control threads spill: 6.02 ms against 5.91 at N=1536)
+    // ------------------------------------------------------------------ control warp of group g
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 32;\n");   // registers go to the softmax warpgroups
     const int g = warp - 4 * kFGroups;
-    if (g == kFGroups && elect_lane()) {
+    if (g == kFGroups) {
       // ---------------------------------------------------------------- pair-bias loader (all six rows share a tile)
       for (int kt = 0; kt < nkt; ++kt) {
         const int b = kt & 1;
-        if (!mbar_wait(&bars.bias_empty[b], ((kt >> 1) & 1) ^ 1, 1u)) break;
-        mbar_expect_tx(&bars.bias_full[b], kFBiasBytes);
-        for (int c = 0; c < kFKT / 32; ++c)
-          tma_load_3d(smem_u32(sm + FlashLayout::bias + b * kFBiasBytes + c * (128 * 128)), &map_b, &bars.bias_full[b],
-                      kt * kFKT + c * 32, q0, h);
+        if (!mbar_wait_warp(&bars.bias_empty[b], ((kt >> 1) & 1) ^ 1, 1u)) break;
+        if (elect_lane()) {
+          mbar_expect_tx(&bars.bias_full[b], kFBiasBytes);
+          for (int c = 0; c < kFKT / 32; ++c)
+            tma_load_3d(smem_u32(sm + FlashLayout::bias + b * kFBiasBytes + c * (128 * 128)), &map_b, &bars.bias_full[b],
+                        kt * kFKT + c * 32, q0, h);
+        }
+        __syncwarp();
       }
-    } else if (g < kFGroups && elect_lane()) {
+    } else {
       constexpr uint32_t idesc_s = umma_idesc_f16(128, kFKT), idesc_o = umma_idesc_f16(128, kFON);
-      const int n_items = nkt * kFRpg;              // work item i = (key tile i / 3, row i % 3 of the group)
+      const int n_items = nkt * kFRpg;              // work item i = (key tile i / 2, row i % 2 of the group)
       const uint32_t q_addr = smem_u32(sm + FlashLayout::q + g * kFRpg * kFQBytes);
       const uint32_t ring = smem_u32(sm + FlashLayout::kv + g * kFStages * kFStageBytes);
       const uint32_t d_s = tmem_base + kFColS + kFKT * g, d_p = tmem_base + kFColP + (kFKT / 2) * g;
       const uint32_t d_o = tmem_base + kFColO + kFON * kFRpg * g;
       const int uh0 = (u0 + g * kFRpg) * kFH + h;   // rows past n_u: coordinate beyond the tensor -> zero fill
-      bool ok = true;
-      auto load_kv = [&](int i) {                   // K and V tiles of item i into stage i % kFStages
+      auto load_kv = [&](int i) {                   // K and V tiles of item i into stage i % kFStages (one lane)
         const int s = i % kFStages, kt = i / kFRpg, uh = uh0 + (i % kFRpg) * kFH;
         mbar_expect_tx(&bars.kv_full[g][s], kFKBytes + kFVBox);
         tma_load_3d(ring + s * kFStageBytes, &map_k, &bars.kv_full[g][s], 0, kt * kFKT, uh);
         tma_load_3d(ring + s * kFStageBytes + kFKBytes, &map_v, &bars.kv_full[g][s], kt * kFKT, 0, uh);
       };
-      auto issue_s = [&](int i) {                   // S(i) = Q_r K^T
-        const int s = i % kFStages;
-        if (!mbar_wait(&bars.kv_full[g][s], (i / kFStages) & 1, 8u)) return false;
+      auto issue_s = [&](int i) {                   // S(i) = bias + Q_r K^T
+        const int s = i % kFStages, kt = i / kFRpg, r = i % kFRpg;
+        if (r == 0 && !mbar_wait_warp(&bars.bias_full[kt & 1], (kt >> 1) & 1, 64u)) return false;
+        if (!mbar_wait_warp(&bars.kv_full[g][s], (i / kFStages) & 1, 8u)) return false;
         tc_fence_after();
-        const uint64_t dq = umma_desc_sw64(q_addr + (i % kFRpg) * kFQBytes), dk = umma_desc_sw64(ring + s * kFStageBytes);
-        umma_bf16(d_s, dq, dk, idesc_s, 0u);
-        umma_bf16(d_s, dq + 2, dk + 2, idesc_s, 1u);
-        umma_commit(&bars.s_full[g]);
+        if (elect_lane()) {
+          const uint32_t tile = smem_u32(sm + FlashLayout::bias + (kt & 1) * kFBiasBytes);
+#pragma unroll
+          for (int c = 0; c < kFCopied / 8; ++c)    // 32 bytes (8 columns) of the 128-byte rows of the tile's first box
+            tmem_copy_128x256b(d_s + 8 * c, umma_desc_sw128(tile) + 2 * c);
+          const uint64_t dq = umma_desc_sw64(q_addr + r * kFQBytes), dk = umma_desc_sw64(ring + s * kFStageBytes);
+          umma_bf16(d_s, dq, dk, idesc_s, 1u);
+          umma_bf16(d_s, dq + 2, dk + 2, idesc_s, 1u);
+          umma_commit(&bars.s_full[g]);
+          if (r == kFRpg - 1) umma_commit(&bars.bias_empty[kt & 1]);   // this group is done with the bias tile
+        }
+        __syncwarp();
         return true;
       };
-      mbar_expect_tx(&bars.q_full[g], kFRpg * kFQBytes);
-      for (int r = 0; r < kFRpg; ++r) tma_load_3d(q_addr + r * kFQBytes, &map_q, &bars.q_full[g], 0, q0, uh0 + r * kFH);
-      for (int i = 0; i < kFStages - 1 && i < n_items; ++i) load_kv(i);   // first use of these stages
-      ok = ok && mbar_wait(&bars.q_full[g], 0, 4u);
-      ok = ok && issue_s(0);
+      if (elect_lane()) {
+        mbar_expect_tx(&bars.q_full[g], kFRpg * kFQBytes);
+        for (int r = 0; r < kFRpg; ++r) tma_load_3d(q_addr + r * kFQBytes, &map_q, &bars.q_full[g], 0, q0, uh0 + r * kFH);
+        for (int i = 0; i < kFStages - 1 && i < n_items; ++i) load_kv(i);   // first use of these stages
+      }
+      __syncwarp();
+      bool ok = mbar_wait_warp(&bars.q_full[g], 0, 4u) && mbar_wait_warp(&bars.s_free[g], 0, 2u) && issue_s(0);
       for (int i = 0; i < n_items && ok; ++i) {
         const int kt = i / kFRpg, r = i % kFRpg;
         if (i + 1 < n_items) {                      // next S as soon as the group holds the current one in registers
-          ok = mbar_wait(&bars.s_free[g], i & 1, 2u) && issue_s(i + 1);
+          ok = mbar_wait_warp(&bars.s_free[g], (i + 1) & 1, 2u) && issue_s(i + 1);
           if (!ok) break;
         }
         if (i + kFStages - 1 < n_items) {           // refill: that stage was last read by P.V of item i-1
-          if (i >= 1) ok = mbar_wait(&bars.pv_done[g], (i - 1) & 1, 32u);
+          if (i >= 1) ok = mbar_wait_warp(&bars.pv_done[g], (i - 1) & 1, 32u);
           if (!ok) break;
-          load_kv(i + kFStages - 1);
+          if (elect_lane()) load_kv(i + kFStages - 1);
+          __syncwarp();
         }
-        ok = mbar_wait(&bars.p_ready[g], i & 1, 16u);
+        ok = mbar_wait_warp(&bars.p_ready[g], i & 1, 16u);
         if (!ok) break;
         tc_fence_after();
-        const uint64_t dv = umma_desc_sw128(ring + (i % kFStages) * kFStageBytes + kFKBytes);
+        if (elect_lane()) {
+          const uint64_t dv = umma_desc_sw128(ring + (i % kFStages) * kFStageBytes + kFKBytes);
 #pragma unroll
-        for (int ks = 0; ks < kFKT / 16; ++ks)  // 16 keys per step: 8 TMEM columns of P, 32 bytes of the value rows
-          umma_bf16_ts(d_o + kFON * r, d_p + 8 * ks, dv + 2 * ks, idesc_o, (kt | ks) ? 1u : 0u);
-        umma_commit(&bars.pv_done[g]);
+          for (int ks = 0; ks < kFKT / 16; ++ks)    // 16 keys per step: 8 TMEM columns of P, 32 bytes of the value rows
+            umma_bf16_ts(d_o + kFON * r, d_p + 8 * ks, dv + 2 * ks, idesc_o, (kt | ks) ? 1u : 0u);
+          umma_commit(&bars.pv_done[g]);
+        }
+        __syncwarp();
       }
     }
   } else {
     // ------------------------------------------------------------------ softmax groups
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 152;\n");
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 160;\n");
     const int g = warp >> 2, qw = warp & 3;
     const int row = 32 * qw + lane;                 // query row inside the tile = TMEM lane
     const uint32_t lane_addr = (uint32_t)(32 * qw) << 16;
@@ -219,6 +238,18 @@ triatt_flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
       m_ref[r] = -CUDART_INF_F;
       l_sum[r] = 0.f;
     }
+    // the product adds to what S holds: the columns without the bias start from zero
+    auto clear_rest = [&] {
+      uint32_t zero[kFKT - kFCopied];
+#pragma unroll
+      for (int e = 0; e < kFKT - kFCopied; ++e) zero[e] = 0u;
+      tmem_st32(t_s + kFCopied, zero);
+      tmem_wait_st();
+    };
+    clear_rest();
+    tc_fence_before();
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&bars.s_free[g]);
     bool ok = true;
     for (int kt = 0; kt < nkt && ok; ++kt) {
       if ((kt & 63) == 0) {
@@ -249,16 +280,12 @@ triatt_flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
           }
         }
       }
-      ok = mbar_wait(&bars.bias_full[kt & 1], (kt >> 1) & 1, 64u);
-      ok = __all_sync(0xffffffffu, ok);
-      if (!ok) break;
-      const float* bias_tile = reinterpret_cast<const float*>(sm + FlashLayout::bias + (kt & 1) * kFBiasBytes);
 #pragma unroll
       for (int r = 0; r < kFRpg; ++r) {
         const int i = kt * kFRpg + r;               // this group's work item
+        // a wait that gave up is voted on once per item, below: what is computed till then goes nowhere
         ok = mbar_wait(&bars.s_full[g], i & 1, 128u);
-        ok = __all_sync(0xffffffffu, ok);
-        if (!ok) break;
+        __syncwarp();
         tc_fence_after();
         float s[kFKT];
         {
@@ -267,25 +294,19 @@ triatt_flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
           tmem_ld32(t_s, t0);
           tmem_ld32(t_s + 32, t1);
           tmem_wait_ld();
+          clear_rest();
         }
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(&bars.s_free[g]);  // S is in registers: the next S may be computed
-        // + pair bias: box c of the tile holds columns 32c..32c+31 of all 128 rows, 128-byte rows, 16-byte pieces
-        // swizzled by row
+        // + pair bias of the other columns: 128-byte rows, 16-byte pieces swizzled by row
+        if (r == 0) ok = mbar_wait(&bars.bias_full[kt & 1], (kt >> 1) & 1, 64u) && ok;
+        const float* brow = reinterpret_cast<const float*>(sm + FlashLayout::bias + (kt & 1) * kFBiasBytes) + row * 32;
 #pragma unroll
-        for (int c = 0; c < kFKT / 32; ++c) {
-          const float* brow = bias_tile + c * (128 * 32) + row * 32;
-#pragma unroll
-          for (int p = 0; p < 8; ++p) {
-            const float4 b4 = *reinterpret_cast<const float4*>(brow + ((p ^ (row & 7)) << 2));
-            add2(s[32 * c + 4 * p + 0], s[32 * c + 4 * p + 1], b4.x, b4.y);
-            add2(s[32 * c + 4 * p + 2], s[32 * c + 4 * p + 3], b4.z, b4.w);
-          }
-        }
-        if (r == kFRpg - 1) {
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&bars.bias_empty[kt & 1]);   // this warp is done with the bias tile
+        for (int c = kFCopied / 4; c < kFKT / 4; ++c) {
+          const float4 b4 = *reinterpret_cast<const float4*>(brow + (c >> 3) * (128 * 32) + (((c & 7) ^ (row & 7)) << 2));
+          add2(s[4 * c + 0], s[4 * c + 1], b4.x, b4.y);
+          add2(s[4 * c + 2], s[4 * c + 3], b4.z, b4.w);
         }
         if ((flag_word[r] >> (kt & 63)) & 1ull) {     // warp-uniform
           const int u = (ug + r < n_u) ? ug + r : 0;
@@ -307,17 +328,12 @@ triatt_flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
           mq[c] = fmaxf(mq[c], s[16 * c + 15]);
         }
         const float mt = fmaxf(fmaxf(mq[0], mq[1]), fmaxf(mq[2], mq[3]));
-        // Does the reference maximum have to move?  Rare after the first tiles (warp-uniform decision).
-        const bool first = (kt == 0);
-        const bool move = !first && __any_sync(0xffffffffu, mt > m_ref[r] + kRescaleGap);
-        float alpha = 1.0f;
-        if (first) {
-          m_ref[r] = mt;                              // first tile: the P.V product overwrites O
-        } else if (move) {
-          const float m_new = (mt > m_ref[r] + kRescaleGap) ? mt : m_ref[r];
-          alpha = fast_exp2(m_ref[r] - m_new);
-          m_ref[r] = m_new;
-        }
+        // Does the reference maximum have to move?  Rare after the first tiles.  The exponentials need only this thread's own answer;
+        // the warp's (tensor memory is rescaled by whole warps) is asked for beside them.
+        const bool up = mt > m_ref[r] + kRescaleGap;
+        const bool move = __any_sync(0xffffffffu, up) && kt > 0;     // first tile: the P.V product overwrites O
+        const float m_old = m_ref[r];
+        m_ref[r] = up ? mt : m_old;
         uint32_t w[kFKT / 2];
         float l0 = 0.f, l1 = 0.f;
         {
@@ -338,15 +354,14 @@ triatt_flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
             add2(l0, l1, p0, p1);
           }
         }
-        l_sum[r] = l_sum[r] * alpha + (l0 + l1);
         // P.V of the previous item must be through before O is rescaled or the P buffer overwritten
-        if (i >= 1) {
-          ok = mbar_wait(&bars.pv_done[g], (i - 1) & 1, 256u);
-          ok = __all_sync(0xffffffffu, ok);
-          if (!ok) break;
-          tc_fence_after();
-        }
+        if (i >= 1) ok = mbar_wait(&bars.pv_done[g], (i - 1) & 1, 256u) && ok;
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) break;
+        tc_fence_after();
         if (move) {
+          const float alpha = fast_exp2(m_old - m_ref[r]);
+          l_sum[r] *= alpha;
 #pragma unroll
           for (int c = 0; c < kFON / 16; ++c) {
             uint32_t a[16];
@@ -357,6 +372,7 @@ triatt_flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
             tmem_st16(t_o + kFON * r + 16 * c, a);
           }
         }
+        l_sum[r] += l0 + l1;
         {
           uint32_t(&w0)[32] = *reinterpret_cast<uint32_t(*)[32]>(&w[0]);
           tmem_st32(t_p, w0);
@@ -364,7 +380,12 @@ triatt_flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         tmem_wait_st();
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(&bars.p_ready[g]);
+        if (lane == 0) {
+          mbar_arrive(&bars.p_ready[g]);
+          // Done with the bias tile.  Only here, where every value read from it has been used: signalled right behind the loads, the
+          // next tile now and then overtook them (one row in 10^8 wrong; the copies delay loads from shared memory).
+          if (r == kFRpg - 1) mbar_arrive(&bars.bias_empty[kt & 1]);
+        }
       }
     }
     // ---- epilogue: o = O / denominator for this group's rows

@@ -1,0 +1,51 @@
+"""The triangle attention core alone (px_triatt_flash) against fp64 at the edges of its tiles: 64 keys a work item of which the pair
+bias of the first 32 reaches the logits by a copy into tensor memory and that of the others by addition, 128 queries and six rows a CTA."""
+import pytest
+import torch
+
+from protenix_b200 import ops
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("masked", [False, True])
+@pytest.mark.parametrize("n", [1, 7, 31, 32, 33, 63, 64, 65, 96, 127, 128, 129, 161, 193])
+def test_attention_core(n, masked):
+    g = torch.Generator("cuda").manual_seed(n)
+    draw = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    ldt, ldm = ops.ld(n), (n + 127) // 128 * 128
+    q, k = (0.3 * draw(n, 4, n, 32)).half(), draw(n, 4, n, 32).half()
+    v = torch.zeros(n, 4, 32, ldt, dtype=torch.half, device="cuda")
+    v[..., :n] = draw(n, 4, 32, n).half()
+    bias = torch.zeros(4, n, ldm, device="cuda")
+    bias[..., :n] = 4 * draw(4, n, n)                         # far beyond what 16 bits would carry to the tolerance below
+    bias[..., :n] += torch.linspace(-20, 20, n, device="cuda")[:, None]
+    mb = torch.full((n, ldm), -float("inf"), device="cuda")
+    mb[:, :n] = 0
+    if masked:
+        mb[:, :n][torch.rand(n, n, generator=g, device="cuda") < 0.3] = -1.44e9
+    o = ops.triatt_flash(q, k, v, bias, mb)
+    ops.device_error_flags()
+    # the logits as fp32 holds them: a masked key's is -1.44e9 whatever was added before
+    s = torch.einsum("uhqd,uhkd->uhqk", q.double(), k.double()) + bias[..., :n].double()
+    s = (s.float() + mb[:, None, None, :n]).double()
+    want = torch.einsum("uhqk,uhdk->uqhd", torch.softmax(s * 0.6931471805599453, -1), v[..., :n].double()).reshape(n, n, 128)
+    assert torch.isfinite(o).all()
+    rel = float((o.double() - want).norm() / want.norm())
+    # P and o are rounded to fp16 (2^-12 each on average half of it), exponentials to 7.5e-5
+    assert rel < 6e-4, rel
+
+
+def test_attention_core_is_the_same_every_time():
+    """Tiles handed back too early show as a wrong row in some of many runs."""
+    n = 600
+    g = torch.Generator("cuda").manual_seed(n)
+    draw = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    q, k, v = (0.3 * draw(n, 4, n, 32)).half(), draw(n, 4, n, 32).half(), draw(n, 4, 32, n).half()
+    ldm = (n + 127) // 128 * 128
+    bias, mb = torch.zeros(4, n, ldm, device="cuda"), torch.full((n, ldm), -float("inf"), device="cuda")
+    bias[..., :n] = 2 * draw(4, n, n)
+    mb[:, :n] = 0
+    first = ops.triatt_flash(q, k, v, bias, mb)
+    differs = sum((ops.triatt_flash(q, k, v, bias, mb) != first).any() for _ in range(300))
+    assert int(differs) == 0
