@@ -7,17 +7,22 @@
 // Persistent kernel, one CTA per SM, 128 rows per tile, three tiles in flight: while the tensor core works through
 // the eight 64-wide hidden chunks of one tile, the next tile is being normalised and the previous one written out.
 //
-//   warps 0..7    SwiGLU: a thread owns one row and half of the current hidden chunk: it pulls a|b out of tensor
-//                 memory, forms h = silu(a) * b, and writes h (fp16) back over the first 32 columns of the same
-//                 H buffer as the A operand of the second product.  The two H buffers alternate.
-//   warps 8..11   LayerNorm: lanes across channels (coalesced), eight rows in flight per warp; the normalised rows
+//   warps 0..7    SwiGLU, two groups of four warps that take the hidden chunks in turn, each with its own H buffer: a thread
+//                 owns one row, pulls a|b out of tensor memory in steps of 16, forms h = silu(a) * b, and writes h (fp16)
+//                 over a values it has read, as the A operand of the second product.  No thread needs another's values, so
+//                 the groups meet at no barrier and one group's chain of waits runs beside the other's arithmetic (all
+//                 eight warps on one chunk, two barriers each: 67 us against 61 at N = 384, 476..525 against 416..438 at N = 1024).
+//   warps 8..11   LayerNorm: eight lanes a row, eight rows in flight per warp; the normalised rows
 //                 are written as the K-major, 128-byte-swizzled A operand of the first product (two buffers).
 //   warps 12..15  output: accumulator -> shared staging (where the residual waits) -> TMA store or addition (two accumulators).
 //   warp 16       TMA producer of the weight chunks: rows 64c..64c+63 of W_a and W_b and columns 64c..64c+63 of
 //                 W_o, 48 KB, 3-stage ring (the weights are re-read from L2 for every tile: 384 KB per 128 rows).
 //   warps 17, 18  MMA issuers: H = A [W_a;W_b]_c^T (M=128, N=128, K=128) and OUT += h W_o,c^T (M=128, N=128, K=64, h
-//                 as the TMEM-resident A operand).  Two threads because a tcgen05.mma costs its issuing thread
-//                 about 100 cycles.
+//                 as the TMEM-resident A operand).  One warp for both, each first product right behind the second one that frees
+//                 its buffer, was slower (64.7 us against 61 at N = 384).
+// What bounds it: above some 700 tokens the power limit (1.6 GHz at N = 768; without the weight loads, the tanh, the
+// LayerNorm or the products it takes 90 to 100 % of its time), below it the chain p_ready -> second product (256 cycles of
+// the tensor pipe) -> first product (512) -> h, of which two run side by side.
 // Tensor memory: H_0 | H_1 | OUT_0 | OUT_1, 128 columns each.  Every mbarrier wait is bounded.
 #include "px_rowpipe.cuh"
 
@@ -41,29 +46,47 @@ struct TransLayout {
   static constexpr int a = 0;                                  // two normalised tiles
   static constexpr int w = a + 2 * kTrABytes;                  // weight ring
   static constexpr int stg = w + kTrStages * kTrStageBytes;    // output staging: [128 rows][32 fp32]
-  static constexpr int bars = stg + 128 * 128;
+  static constexpr int affine = stg + 128 * 128;               // gamma / 2 and beta / 2
+  static constexpr int bars = affine + 2 * kC * 4;
   static constexpr int total = bars + (int)sizeof(TransBars);
 };
 
-// Four consecutive channels as they are stored (8 or 16 bytes), so that loads can be kept in flight cheaply.
+// Sixteen channels of a row as they are stored: lane p of the row's eight holds 8p..8p+7 and 64+8p..64+8p+7, whatever the type, so
+// that both types are summed in one order.
 template <typename Tz>
-struct Raw4;
+struct Raw16;
 template <>
-struct Raw4<bf16> {
-  uint2 v;
-  __device__ __forceinline__ void load(const bf16* p) { v = *reinterpret_cast<const uint2*>(p); }
-  __device__ __forceinline__ void zero() { v = make_uint2(0u, 0u); }
-  __device__ __forceinline__ float4 get() const {
-    const float2 a = unpack_bf16x2(v.x), b = unpack_bf16x2(v.y);
-    return make_float4(a.x, a.y, b.x, b.y);
+struct Raw16<bf16> {
+  uint4 v[2];
+  __device__ __forceinline__ void load(const bf16* row, int p) {
+#pragma unroll
+    for (int i = 0; i < 2; ++i) v[i] = *reinterpret_cast<const uint4*>(row + 64 * i + 8 * p);
+  }
+  __device__ __forceinline__ void zero() { v[0] = v[1] = make_uint4(0u, 0u, 0u, 0u); }
+  __device__ __forceinline__ void get(float (&x)[16]) const {
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const uint32_t w[4] = {v[i].x, v[i].y, v[i].z, v[i].w};
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float2 f = unpack_bf16x2(w[e]);
+        x[8 * i + 2 * e] = f.x, x[8 * i + 2 * e + 1] = f.y;
+      }
+    }
   }
 };
 template <>
-struct Raw4<float> {
-  float4 v;
-  __device__ __forceinline__ void load(const float* p) { v = *reinterpret_cast<const float4*>(p); }
-  __device__ __forceinline__ void zero() { v = make_float4(0.f, 0.f, 0.f, 0.f); }
-  __device__ __forceinline__ float4 get() const { return v; }
+struct Raw16<float> {
+  float4 v[4];
+  __device__ __forceinline__ void load(const float* row, int p) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) v[i] = *reinterpret_cast<const float4*>(row + 64 * (i >> 1) + 8 * p + 4 * (i & 1));
+  }
+  __device__ __forceinline__ void zero() { v[0] = v[1] = v[2] = v[3] = make_float4(0.f, 0.f, 0.f, 0.f); }
+  __device__ __forceinline__ void get(float (&x)[16]) const {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) x[4 * i] = v[i].x, x[4 * i + 1] = v[i].y, x[4 * i + 2] = v[i].z, x[4 * i + 3] = v[i].w;
+  }
 };
 
 template <typename Tz>
@@ -86,7 +109,7 @@ transition_tc_kernel(const __grid_constant__ CUtensorMap map_wa, const __grid_co
       mbar_init(&bars.a_free[b], 1);
       mbar_init(&bars.h_full[b], 1);
       mbar_init(&bars.h_free[b], 1);
-      mbar_init(&bars.p_ready[b], 8);
+      mbar_init(&bars.p_ready[b], 4);
       mbar_init(&bars.out_full[b], 1);
       mbar_init(&bars.out_free[b], 4);
     }
@@ -107,24 +130,25 @@ transition_tc_kernel(const __grid_constant__ CUtensorMap map_wa, const __grid_co
   const uint32_t tmem_base = bars.tmem_base;
 
   if (warp >= 16) {
-    if (!elect_lane()) {
-      // nothing: one elected lane of each control warp works
-    } else if (warp == 16) {
+    if (warp == 16) {
       // ---------------------------------------------------------------- weight producer
       int j = 0;                                      // chunk counter over all tiles of this CTA
       bool ok = true;
       for (int tile = first_tile; tile < n_tiles && ok; tile += tile_step) {
         for (int c = 0; c < kTrChunks && ok; ++c, ++j) {
           const int s = j % kTrStages;
-          ok = mbar_wait(&bars.w_empty[s], ((j / kTrStages) & 1) ^ 1, 1u);
+          ok = mbar_wait_warp(&bars.w_empty[s], ((j / kTrStages) & 1) ^ 1, 1u);
           if (!ok) break;
-          mbar_expect_tx(&bars.w_full[s], kTrStageBytes);
-          const uint32_t base = smem_u32(sm + TransLayout::w + s * kTrStageBytes);
-          for (int p = 0; p < 2; ++p) {  // k panel p: rows 0..63 from W_a, rows 64..127 from W_b
-            tma_load_3d(base + p * 16384, &map_wa, &bars.w_full[s], 64 * p, 64 * c, 0);
-            tma_load_3d(base + p * 16384 + 8192, &map_wb, &bars.w_full[s], 64 * p, 64 * c, 0);
+          if (elect_lane()) {
+            mbar_expect_tx(&bars.w_full[s], kTrStageBytes);
+            const uint32_t base = smem_u32(sm + TransLayout::w + s * kTrStageBytes);
+            for (int p = 0; p < 2; ++p) {  // k panel p: rows 0..63 from W_a, rows 64..127 from W_b
+              tma_load_3d(base + p * 16384, &map_wa, &bars.w_full[s], 64 * p, 64 * c, 0);
+              tma_load_3d(base + p * 16384 + 8192, &map_wb, &bars.w_full[s], 64 * p, 64 * c, 0);
+            }
+            tma_load_3d(base + kTrW1Bytes, &map_wo, &bars.w_full[s], 64 * c, 0, 0);
           }
-          tma_load_3d(base + kTrW1Bytes, &map_wo, &bars.w_full[s], 64 * c, 0, 0);
+          __syncwarp();
         }
       }
     } else if (warp == 17) {
@@ -134,22 +158,25 @@ transition_tc_kernel(const __grid_constant__ CUtensorMap map_wa, const __grid_co
       bool ok = true;
       for (int tile = first_tile; tile < n_tiles && ok; tile += tile_step, ++k) {
         const int ab = k & 1;
-        ok = mbar_wait(&bars.a_full[ab], (k >> 1) & 1, 2u);
+        ok = mbar_wait_warp(&bars.a_full[ab], (k >> 1) & 1, 2u);
         const uint32_t a_addr = smem_u32(sm + TransLayout::a + ab * kTrABytes);
         for (int c = 0; c < kTrChunks && ok; ++c, ++j) {
           const int s = j % kTrStages, hb = j & 1;
-          ok = mbar_wait(&bars.w_full[s], (j / kTrStages) & 1, 4u) && mbar_wait(&bars.h_free[hb], ((j >> 1) & 1) ^ 1, 4u);
+          ok = mbar_wait_warp(&bars.w_full[s], (j / kTrStages) & 1, 4u) && mbar_wait_warp(&bars.h_free[hb], ((j >> 1) & 1) ^ 1, 4u);
           if (!ok) break;
           tc_fence_after();
-          const uint32_t wbase = smem_u32(sm + TransLayout::w + s * kTrStageBytes);
+          if (elect_lane()) {
+            const uint32_t wbase = smem_u32(sm + TransLayout::w + s * kTrStageBytes);
 #pragma unroll
-          for (int ks = 0; ks < 8; ++ks)
-            umma_bf16(tmem_base + 128 * hb, umma_desc_sw128(a_addr + (ks >> 2) * 16384) + 2 * (ks & 3),
-                      umma_desc_sw128(wbase + (ks >> 2) * 16384) + 2 * (ks & 3), idesc, ks ? 1u : 0u);
-          umma_commit(&bars.h_full[hb]);
-          umma_commit(&bars.w_empty[s]);                // this thread's share of the reads of the stage
+            for (int ks = 0; ks < 8; ++ks)
+              umma_bf16(tmem_base + 128 * hb, umma_desc_sw128(a_addr + (ks >> 2) * 16384) + 2 * (ks & 3),
+                        umma_desc_sw128(wbase + (ks >> 2) * 16384) + 2 * (ks & 3), idesc, ks ? 1u : 0u);
+            umma_commit(&bars.h_full[hb]);
+            umma_commit(&bars.w_empty[s]);              // this warp's share of the reads of the stage
+            if (c == kTrChunks - 1) umma_commit(&bars.a_free[ab]);   // the tile has been read for the last time
+          }
+          __syncwarp();
         }
-        if (ok) umma_commit(&bars.a_free[ab]);          // the tile has been read for the last time
       }
     } else if (warp == 18) {
       // ---------------------------------------------------------------- second product: OUT += h W_o,c^T
@@ -158,20 +185,23 @@ transition_tc_kernel(const __grid_constant__ CUtensorMap map_wa, const __grid_co
       bool ok = true;
       for (int tile = first_tile; tile < n_tiles && ok; tile += tile_step, ++k) {
         const int ob = k & 1;
-        ok = mbar_wait(&bars.out_free[ob], ((k >> 1) & 1) ^ 1, 8u);
+        ok = mbar_wait_warp(&bars.out_free[ob], ((k >> 1) & 1) ^ 1, 8u);
         for (int c = 0; c < kTrChunks && ok; ++c, ++j) {
           const int s = j % kTrStages, hb = j & 1;
-          ok = mbar_wait(&bars.w_full[s], (j / kTrStages) & 1, 4u) && mbar_wait(&bars.p_ready[hb], (j >> 1) & 1, 8u);
+          ok = mbar_wait_warp(&bars.w_full[s], (j / kTrStages) & 1, 4u) && mbar_wait_warp(&bars.p_ready[hb], (j >> 1) & 1, 8u);
           if (!ok) break;
           tc_fence_after();
-          const uint64_t dwo = umma_desc_sw128(smem_u32(sm + TransLayout::w + s * kTrStageBytes) + kTrW1Bytes);
+          if (elect_lane()) {
+            const uint64_t dwo = umma_desc_sw128(smem_u32(sm + TransLayout::w + s * kTrStageBytes) + kTrW1Bytes);
 #pragma unroll
-          for (int ks = 0; ks < 4; ++ks)
-            umma_bf16_ts(tmem_base + 256 + 128 * ob, tmem_base + 128 * hb + 8 * ks, dwo + 2 * ks, idesc, (c | ks) ? 1u : 0u);
-          umma_commit(&bars.h_free[hb]);
-          umma_commit(&bars.w_empty[s]);
+            for (int ks = 0; ks < 4; ++ks)
+              umma_bf16_ts(tmem_base + 256 + 128 * ob, tmem_base + 128 * hb + 8 * ks, dwo + 2 * ks, idesc, (c | ks) ? 1u : 0u);
+            umma_commit(&bars.h_free[hb]);
+            umma_commit(&bars.w_empty[s]);
+            if (c == kTrChunks - 1) umma_commit(&bars.out_full[ob]);
+          }
+          __syncwarp();
         }
-        if (ok) umma_commit(&bars.out_full[ob]);
       }
     }
   } else if (warp >= 12) {
@@ -263,27 +293,29 @@ transition_tc_kernel(const __grid_constant__ CUtensorMap map_wa, const __grid_co
     // The normalised rows enter the first product halved: a' = a / 2 is the argument of the gate's tanh, b' = b / 2,
     // and h' = a' b' (1 + tanh a') = silu(a) b / 2 is what the SwiGLU warps write; the output warps double the second
     // product.  Powers of two: nothing changes but two multiplications per hidden element that are no longer needed.
-    float4 g4 = *reinterpret_cast<const float4*>(ln_w + 4 * lane);
-    float4 b4 = *reinterpret_cast<const float4*>(ln_b + 4 * lane);
-    g4.x *= 0.5f, g4.y *= 0.5f, g4.z *= 0.5f, g4.w *= 0.5f;
-    b4.x *= 0.5f, b4.y *= 0.5f, b4.z *= 0.5f, b4.w *= 0.5f;
-    const int panel_off = (lane >> 4) * 16384 + (lane & 1) * 8, chunk = (lane & 15) >> 1;
+    float* const affine = reinterpret_cast<float*>(sm + TransLayout::affine);     // gamma / 2, then beta / 2
+    affine[threadIdx.x - 256] = 0.5f * ln_w[threadIdx.x - 256];
+    affine[kC + threadIdx.x - 256] = 0.5f * ln_b[threadIdx.x - 256];
+    named_barrier(1, 128);
+    // Eight lanes a row and four rows at a time, 16 channels a lane: three exchanges a sum for four rows.  With 32 lanes a row the exchanges were a third of the instructions of
+    // these four warps, and they were late: 61 us against 58 at N = 384, 15.2 against 13.6 for one tile, 434 against 399 at N = 1024.
+    const int piece = lane & 7, r0 = lane >> 3;
     int k = 0;
     for (int tile = first_tile; tile < n_tiles; tile += tile_step, ++k) {
       const int ab = k & 1;
-      const long long row0 = (long long)tile * 128;
+      const long long row0 = (long long)tile * 128 + 32 * qw + r0;
       bool ok = mbar_wait(&bars.a_free[ab], ((k >> 1) & 1) ^ 1, 16u);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
       unsigned char* sa = sm + TransLayout::a + ab * kTrABytes;
       // eight rows per batch; the next batch is requested (as stored) before this one is reduced
-      Raw4<Tz> raw[8];
+      Raw16<Tz> raw[2];
       auto request = [&](int rb) {
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const long long grow = row0 + 32 * qw + rb + j;
+        for (int j = 0; j < 2; ++j) {
+          const long long grow = row0 + rb + 4 * j;
           if (grow < rows) {
-            raw[j].load(x_in + (size_t)grow * kC + 4 * lane);
+            raw[j].load(x_in + (size_t)grow * kC, piece);
           } else {
             raw[j].zero();
           }
@@ -292,41 +324,54 @@ transition_tc_kernel(const __grid_constant__ CUtensorMap map_wa, const __grid_co
       request(0);
 #pragma unroll 1
       for (int rb = 0; rb < 32; rb += 8) {
-        float4 x[8];
+        float x[2][16], sum[2];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) x[j] = raw[j].get();
+        for (int j = 0; j < 2; ++j) raw[j].get(x[j]);
         if (rb + 8 < 32) request(rb + 8);
-        float sum[8];
+        auto reduce = [&] {
 #pragma unroll
-        for (int j = 0; j < 8; ++j) sum[j] = x[j].x + x[j].y + x[j].z + x[j].w;
+          for (int o = 4; o > 0; o >>= 1)
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1)
+            for (int j = 0; j < 2; ++j) sum[j] += __shfl_xor_sync(0xffffffffu, sum[j], o);
+        };
 #pragma unroll
-          for (int j = 0; j < 8; ++j) sum[j] += __shfl_xor_sync(0xffffffffu, sum[j], o);
+        for (int j = 0; j < 2; ++j) {
+          float p[4];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
+          for (int e = 0; e < 4; ++e) p[e] = (x[j][e] + x[j][4 + e]) + (x[j][8 + e] + x[j][12 + e]);
+          sum[j] = (p[0] + p[1]) + (p[2] + p[3]);
+        }
+        reduce();
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
           const float mean = sum[j] * (1.0f / kC);
-          x[j].x -= mean;
-          x[j].y -= mean;
-          x[j].z -= mean;
-          x[j].w -= mean;
-          sum[j] = x[j].x * x[j].x + x[j].y * x[j].y + x[j].z * x[j].z + x[j].w * x[j].w;
+          float p[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+          for (int e = 0; e < 16; ++e) {
+            x[j][e] -= mean;
+            p[e & 3] = fmaf(x[j][e], x[j][e], p[e & 3]);
+          }
+          sum[j] = (p[0] + p[1]) + (p[2] + p[3]);
+        }
+        reduce();
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          const float rstd = row0 + rb + 4 * j < rows ? rsqrtf(sum[j] * (1.0f / kC) + eps) : 0.f;
+#pragma unroll
+          for (int e = 0; e < 16; ++e) x[j][e] *= rstd;
         }
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1)
+        for (int i = 0; i < 2; ++i) {
+          const float4* g = reinterpret_cast<const float4*>(affine + 64 * i + 8 * piece);
+          const float4 g0 = g[0], g1 = g[1], b0 = g[kC / 4], b1 = g[kC / 4 + 1];
 #pragma unroll
-          for (int j = 0; j < 8; ++j) sum[j] += __shfl_xor_sync(0xffffffffu, sum[j], o);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const int r = 32 * qw + rb + j;                  // row inside the tile
-          const long long grow = row0 + r;
-          const float rstd = rsqrtf(sum[j] * (1.0f / kC) + eps);
-          uint2 o = make_uint2(0u, 0u);
-          if (grow < rows) {
-            o.x = pack_f16x2(x[j].x * rstd * g4.x + b4.x, x[j].y * rstd * g4.y + b4.y);
-            o.y = pack_f16x2(x[j].z * rstd * g4.z + b4.z, x[j].w * rstd * g4.w + b4.w);
+          for (int j = 0; j < 2; ++j) {
+            const int r = 32 * qw + r0 + rb + 4 * j;       // row inside the tile
+            const float* v = &x[j][8 * i];
+            *reinterpret_cast<uint4*>(sa + i * 16384 + r * 128 + ((piece ^ (r & 7)) << 4)) =
+                make_uint4(pack_f16x2(fmaf(v[0], g0.x, b0.x), fmaf(v[1], g0.y, b0.y)), pack_f16x2(fmaf(v[2], g0.z, b0.z), fmaf(v[3], g0.w, b0.w)),
+                           pack_f16x2(fmaf(v[4], g1.x, b1.x), fmaf(v[5], g1.y, b1.y)), pack_f16x2(fmaf(v[6], g1.z, b1.z), fmaf(v[7], g1.w, b1.w)));
           }
-          *reinterpret_cast<uint2*>(sa + panel_off + r * 128 + ((chunk ^ (r & 7)) << 4)) = o;
         }
       }
       asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
@@ -335,40 +380,38 @@ transition_tc_kernel(const __grid_constant__ CUtensorMap map_wa, const __grid_co
     }
   } else {
     // ------------------------------------------------------------------ SwiGLU in registers
-    // All eight warps work on the current hidden chunk (lane quarter x half of its 64 columns), so that the second
-    // product can start after half the time; the H buffers alternate from chunk to chunk.
-    const int half = warp >> 2, qw = warp & 3;
-    const uint32_t lane_addr = tmem_base + ((uint32_t)(32 * qw) << 16);
-    int j = 0;                                        // chunk counter over all tiles of this CTA
+    // Two groups of four warps, each on every other chunk and its H buffer.  A thread owns its row's 64 hidden values of the chunk,
+    // so nothing is exchanged between threads.  The 16 values of a step are h, packed into 8 columns over a values read before.
+    const int hb = warp >> 2, qw = warp & 3;
+    const uint32_t t_h = tmem_base + ((uint32_t)(32 * qw) << 16) + 128 * hb;
+    int n = 0;                                        // chunks of this group so far
     bool ok = true;
     for (int tile = first_tile; tile < n_tiles && ok; tile += tile_step) {
-      for (int c = 0; c < kTrChunks && ok; ++c, ++j) {
-        const int hb = j & 1;
-        const uint32_t t_h = lane_addr + 128 * hb;
-        ok = mbar_wait(&bars.h_full[hb], (j >> 1) & 1, 64u);
-        ok = named_barrier_all(2, 256, ok);                // all eight warps go on, or none
+      for (int c = hb; c < kTrChunks; c += 2, ++n) {
+        ok = mbar_wait_warp(&bars.h_full[hb], n & 1, 64u);
         if (!ok) break;
         tc_fence_after();
-        uint32_t w[16];
+        uint32_t a[2][16], b[2][16];
+        tmem_ld16(t_h, a[0]);
+        tmem_ld16(t_h + 64, b[0]);
 #pragma unroll
-        for (int hh = 0; hh < 2; ++hh) {
-          uint32_t a[16], b[16];
-          tmem_ld16(t_h + 32 * half + 16 * hh, a);
-          tmem_ld16(t_h + 64 + 32 * half + 16 * hh, b);
+        for (int p = 0; p < 4; ++p) {
           tmem_wait_ld();
+          if (p < 3) {
+            tmem_ld16(t_h + 16 * (p + 1), a[(p + 1) & 1]);
+            tmem_ld16(t_h + 64 + 16 * (p + 1), b[(p + 1) & 1]);
+          }
+          uint32_t w[8];
 #pragma unroll
           for (int e = 0; e < 8; ++e) {
             // silu(a) * b / 2 = a' b' (1 + tanh a') with a' = a / 2, b' = b / 2 as the accumulators hold them:
             // one special-function op, one multiplication and one fused multiply-add per element
-            const float a0 = __uint_as_float(a[2 * e]), a1 = __uint_as_float(a[2 * e + 1]);
-            const float h0 = a0 * __uint_as_float(b[2 * e]), h1 = a1 * __uint_as_float(b[2 * e + 1]);
-            w[8 * hh + e] = pack_f16x2(fmaf(h0, tanh_fast(a0), h0), fmaf(h1, tanh_fast(a1), h1));
+            const float a0 = __uint_as_float(a[p & 1][2 * e]), a1 = __uint_as_float(a[p & 1][2 * e + 1]);
+            const float h0 = a0 * __uint_as_float(b[p & 1][2 * e]), h1 = a1 * __uint_as_float(b[p & 1][2 * e + 1]);
+            w[e] = pack_f16x2(fmaf(h0, tanh_fast(a0), h0), fmaf(h1, tanh_fast(a1), h1));
           }
+          tmem_st8(t_h + 8 * p, w);
         }
-        // h overwrites the first 32 columns of H; all warps must have read their a before any of them writes:
-        // the a columns 0..31 of the half-0 warps are exactly where h lands
-        named_barrier(2, 256);
-        tmem_st16(t_h + 16 * half, w);
         tmem_wait_st();
         tc_fence_before();
         __syncwarp();
