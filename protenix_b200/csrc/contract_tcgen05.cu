@@ -99,6 +99,7 @@ trimul_contract_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
   const int first_tile = blockIdx.x / kCtas, tile_step = gridDim.x / kCtas;
 
   const bool skip = cta_begin();         // an earlier bounded wait gave up: do not start new work
+  if (threadIdx.x == 32) prefetch_maps(map_a, map_b, map_x);
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) {
       mbar_init(&bars.full[s], 1);
@@ -265,7 +266,7 @@ trimul_contract_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
           mbar_arrive(&bars.acc_empty[ab]);
       }
     }
-    if (lane == 0) tma_store_wait<0>();
+    if (lane == 0) tma_store_wait_read<0>();
   }
 
   // teardown: everybody meets, then the allocating warp frees the tensor memory

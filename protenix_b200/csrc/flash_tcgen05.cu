@@ -114,6 +114,7 @@ triatt_flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
   const int q0 = blockIdx.x * 128, h = blockIdx.y, u0 = blockIdx.z * kFRows;
 
   const bool skip = cta_begin();         // an earlier bounded wait gave up: do not start new work
+  if (threadIdx.x == 32) prefetch_maps(map_q, map_k, map_v, map_b, map_o);
   if (threadIdx.x == 0) {
     for (int b = 0; b < 2; ++b) {
       mbar_init(&bars.bias_full[b], 1);
@@ -419,7 +420,7 @@ triatt_flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
           tma_store_commit();
         }
       }
-      if (lane == 0) tma_store_wait<0>();
+      if (lane == 0) tma_store_wait_read<0>();
     }
   }
 

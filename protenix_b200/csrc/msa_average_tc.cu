@@ -71,6 +71,7 @@ msa_average_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
   const int first_tile = blockIdx.x, tile_step = gridDim.x;
 
   const bool skip = cta_begin();
+  if (threadIdx.x == 32) prefetch_maps(map_w, map_v);
   if (threadIdx.x == 0) {
     for (int s = 0; s < kMvStages; ++s) {
       mbar_init(&bars.full[s], 1);

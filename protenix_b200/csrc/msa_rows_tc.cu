@@ -74,6 +74,10 @@ msa_rows_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
   const int first_tile = blockIdx.x, tile_step = gridDim.x;
 
   const bool skip = cta_begin();
+  if (threadIdx.x == 32) {
+    prefetch_maps(map_w);
+    if (kMode == kMrGate) prefetch_maps(map_w2);
+  }
   if (threadIdx.x == 0) {
     for (int b = 0; b < 2; ++b) {
       mbar_init(&bars.a_full[b], 8);

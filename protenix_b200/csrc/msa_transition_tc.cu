@@ -50,6 +50,7 @@ msa_transition_tc_kernel(const __grid_constant__ CUtensorMap map_w1, const __gri
   const int first_tile = blockIdx.x, tile_step = gridDim.x;
 
   const bool skip = cta_begin();
+  if (threadIdx.x == 32) prefetch_maps(map_w1, map_w2);
   if (threadIdx.x == 0) {
     for (int b = 0; b < 2; ++b) {
       mbar_init(&bars.a_full[b], 4);

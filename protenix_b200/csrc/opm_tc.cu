@@ -54,6 +54,7 @@ opm_out_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
   const int warp = warp_index(), lane = threadIdx.x & 31;
 
   const bool skip = cta_begin();         // an earlier bounded wait gave up: do not start new work
+  if (threadIdx.x == 32) prefetch_maps(map_x, map_w);
   if (threadIdx.x == 0) {
     for (int s = 0; s < kOpStages; ++s) {
       mbar_init(&bars.full[s], 1);

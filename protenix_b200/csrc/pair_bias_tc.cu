@@ -76,6 +76,7 @@ pair_bias_tc_kernel(const __grid_constant__ CUtensorMap map_z, const PbWeights<k
   ctx.swap = 0;
 
   const bool skip = cta_begin();         // an earlier bounded wait gave up: do not start new work
+  if (threadIdx.x == 32) prefetch_maps(map_z);
   if (threadIdx.x == 0) {
     tile_bars_init(bars.tile, 1, kF16);
     mbar_init(&bars.w_full, 1);

@@ -162,14 +162,11 @@ __device__ __forceinline__ void tma_add_3d(const CUtensorMap* map, uint32_t src,
                : "memory");
 }
 __device__ __forceinline__ void tma_store_commit() { asm volatile("cp.async.bulk.commit_group;\n" ::: "memory"); }
-// Waits until at most N of this thread's store groups still read their shared-memory source.
+// Waits until at most N of this thread's store groups still read their shared-memory source.  Enough at the end of a kernel, too:
+// what shared memory held is on its way, and the grid is not complete before it has arrived.
 template <int N>
 __device__ __forceinline__ void tma_store_wait_read() {
   asm volatile("cp.async.bulk.wait_group.read %0;\n" ::"n"(N) : "memory");
-}
-template <int N>
-__device__ __forceinline__ void tma_store_wait() {
-  asm volatile("cp.async.bulk.wait_group %0;\n" ::"n"(N) : "memory");
 }
 // Barrier over `threads` threads that also returns whether `ok` held on all of them, so that a group can leave a
 // loop together after one of its waits ran out.

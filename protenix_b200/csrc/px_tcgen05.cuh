@@ -38,15 +38,17 @@ __device__ __forceinline__ bool cta_ready(bool skip, bool alloc_warp, const uint
   return !stop;
 }
 
-// Called by every thread at the end of a kernel, in place of the closing __syncthreads(): when a wait ran out, copies
-// may still be in flight towards this CTA's shared memory, so the CTA lingers before it frees anything.
-__device__ __forceinline__ void cta_teardown_sync() {
-  if (__syncthreads_or(tc_error_seen())) {
-    const long long t0 = clock64();
-    while (clock64() - t0 < 200000) {
-    }
-    __syncthreads();
-  }
+// Called by every thread at the end of a kernel, in place of the closing __syncthreads(): copies that a wait gave up on have
+// landed by now (see mbar_wait).
+__device__ __forceinline__ void cta_teardown_sync() { __syncthreads(); }
+
+// Asks for the descriptors of a kernel's TMA copies (one thread, before pdl_wait): the first copy through each would fetch it
+// from global memory, after the kernel before has ended.
+template <typename... Maps>
+__device__ __forceinline__ void prefetch_maps(const Maps&... maps) {
+  const CUtensorMap* list[] = {&maps...};
+#pragma unroll
+  for (const CUtensorMap* m : list) asm volatile("prefetch.tensormap [%0];\n" ::"l"(reinterpret_cast<uint64_t>(m)) : "memory");
 }
 
 // Index of this warp, in a form that the compiler knows to be the same for all its lanes.
@@ -70,7 +72,7 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(smem_u32(bar)) : "memory");
 }
-// Bounded wait for the phase with the given parity; false = gave up (error flag set).
+// Bounded wait for the phase with the given parity; false = gave up (error flag set, copies in flight have landed).
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, unsigned int code) {
   const uint32_t addr = smem_u32(bar);
   {
@@ -94,12 +96,18 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, unsign
         : "r"(addr), "r"(parity), "r"(1000000u)
         : "memory");
     if (done) return true;
-    if (tc_error_seen()) return false;   // another wait gave up: this one would only repeat its limit
+    if (tc_error_seen()) break;          // another wait gave up: this one would only repeat its limit
     if (clock64() - t0 > *reinterpret_cast<volatile long long*>(&g_wait_limit)) {
       atomicOr(&g_tc_error, code);
-      return false;
+      break;
     }
   }
+  // Copies may still be in flight towards this CTA's shared memory, so whoever gives up lingers before it goes on to the end of the
+  // kernel, where everything is freed.  (Looking at the flag there instead cost every launch a trip to L2.)
+  const long long t1 = clock64();
+  while (clock64() - t1 < 200000) {
+  }
+  return false;
 }
 
 // The same for a whole warp: all lanes wait and get one answer.

@@ -68,6 +68,10 @@ recycle_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_consta
   ctx.swap = 0;
 
   const bool skip = cta_begin();         // an earlier bounded wait gave up: do not start new work
+  if (threadIdx.x == 32) {
+    prefetch_maps(map_z);
+    if (kTma) prefetch_maps(map_init, map_out);
+  }
   if (threadIdx.x == 0) {
     tile_bars_init(bars.tile, 1, kF16);
     mbar_init(&bars.w_full, 1);
@@ -203,7 +207,7 @@ recycle_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_consta
         }
       }
     }
-    if (kTma && leader) tma_store_wait<0>();
+    if (kTma && leader) tma_store_wait_read<0>();
   }
 
   tc_fence_before();

@@ -112,6 +112,7 @@ split_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
   const int n0 = blockIdx.x * kSgBN, m0 = blockIdx.y * 128, kc0 = blockIdx.z * g.chunks;
 
   const bool stop = cta_begin();                 // an earlier bounded wait gave up: do no work, but meet the barriers
+  if (threadIdx.x == 32) prefetch_maps(map_a, map_w);
   if (threadIdx.x == 0) {
     for (int s = 0; s < kSgStages; ++s) {
       mbar_init(&bars.full[s], 1);

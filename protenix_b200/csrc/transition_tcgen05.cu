@@ -103,6 +103,7 @@ transition_tc_kernel(const __grid_constant__ CUtensorMap map_wa, const __grid_co
   const int first_tile = blockIdx.x, tile_step = gridDim.x;
 
   const bool skip = cta_begin();         // an earlier bounded wait gave up: do not start new work
+  if (threadIdx.x == 32) prefetch_maps(map_wa, map_wb, map_wo, map_out, map_res);
   if (threadIdx.x == 0) {
     for (int b = 0; b < 2; ++b) {
       mbar_init(&bars.a_full[b], 4);
@@ -286,7 +287,7 @@ transition_tc_kernel(const __grid_constant__ CUtensorMap map_wa, const __grid_co
         }
       }
     }
-    if (lane == 0) tma_store_wait<0>();
+    if (lane == 0) tma_store_wait_read<0>();
   } else if (warp >= 8) {
     // ------------------------------------------------------------------ LayerNorm -> swizzled A operand
     const int qw = warp - 8;

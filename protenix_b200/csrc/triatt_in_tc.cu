@@ -100,6 +100,7 @@ triatt_in_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_cons
   ctx.swap = swap;
 
   const bool skip = cta_begin();         // an earlier bounded wait gave up: do not start new work
+  if (threadIdx.x == 32) prefetch_maps(map_z, map_v, map_q, map_k);
   if (threadIdx.x == 0) {
     tile_bars_init(bars.tile, 2, kF16);
     mbar_init(&bars.w_full, 1);
@@ -193,7 +194,7 @@ triatt_in_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_cons
         tma_store_commit();
       }
     }
-    if (lane == 0) tma_store_wait<0>();
+    if (lane == 0) tma_store_wait_read<0>();
   } else {
     // ------------------------------------------------------------------ epilogue of v | bias
     const int half = (warp >> 2) & 1, qw = warp & 3;
@@ -235,7 +236,7 @@ triatt_in_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_cons
         tma_store_commit();
       }
     }
-    if (leader) tma_store_wait<0>();
+    if (leader) tma_store_wait_read<0>();
   }
 
   tc_fence_before();

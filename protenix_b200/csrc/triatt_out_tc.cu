@@ -93,6 +93,10 @@ triatt_out_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_con
   ctx.swap = swap;
 
   const bool skip = cta_begin();         // an earlier bounded wait gave up: do not start new work
+  if (threadIdx.x == 32) {
+    prefetch_maps(map_z, map_o);
+    if (kTma || kBulk) prefetch_maps(map_out);
+  }
   if (threadIdx.x == 0) {
     // a stage is read by the statistics product, the gate product and the output warps
     tile_bars_init(bars.tile, 2, kF16);
@@ -316,7 +320,7 @@ triatt_out_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_con
         if (leader) mbar_arrive(&bars.tile.a_empty[s]);
       }
     }
-    if (kTma ? leader : kBulk && lane == 0) tma_store_wait<0>();
+    if (kTma ? leader : kBulk && lane == 0) tma_store_wait_read<0>();
   }
 
   tc_fence_before();

@@ -95,6 +95,10 @@ trimul_out_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_con
   const int warp = warp_index(), lane = threadIdx.x & 31;
 
   const bool skip = cta_begin();         // an earlier bounded wait gave up: do not start new work
+  if (threadIdx.x == 32) {
+    prefetch_maps(map_z, map_x);
+    if (kTma || kBulk) prefetch_maps(map_out);
+  }
   if (threadIdx.x == 0) {
     for (int s = 0; s < kToStages; ++s) {
       mbar_init(&bars.raw_full[s], 1);
@@ -340,7 +344,7 @@ trimul_out_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_con
         if (leader) mbar_arrive(&bars.a_empty[s]);
       }
     }
-    if (kTma ? leader : kBulk && lane == 0) tma_store_wait<0>();
+    if (kTma ? leader : kBulk && lane == 0) tma_store_wait_read<0>();
   }
 
   tc_fence_before();
