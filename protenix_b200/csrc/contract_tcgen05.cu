@@ -91,7 +91,7 @@ trimul_contract_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
   constexpr int kStages = Shape::kStages;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   // operand ring first (1024-byte aligned for the 128-byte swizzle), staging and barriers after it
-  unsigned char* ring = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  unsigned char* ring = smem_aligned(smem_raw);
   TcBarriers& bars = *reinterpret_cast<TcBarriers*>(ring + Shape::kBars);
   const int warp = warp_index(), lane = threadIdx.x & 31;
   const int nk = (ld_k + kTcBK - 1) / kTcBK;      // ld_k: extent of the contraction index; ld: row stride of x

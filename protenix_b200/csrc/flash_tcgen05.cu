@@ -108,7 +108,7 @@ triatt_flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                        const __grid_constant__ CUtensorMap map_o, const float* __restrict__ mb,
                        int n_u, int n, int ldm, int nkt) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
-  unsigned char* sm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  unsigned char* sm = smem_aligned(smem_raw);
   FlashBars& bars = *reinterpret_cast<FlashBars*>(sm + FlashLayout::bars);
   const int warp = warp_index(), lane = threadIdx.x & 31;
   const int q0 = blockIdx.x * 128, h = blockIdx.y, u0 = blockIdx.z * kFRows;
@@ -383,8 +383,8 @@ triatt_flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         __syncwarp();
         if (lane == 0) {
           mbar_arrive(&bars.p_ready[g]);
-          // Done with the bias tile.  Only here, where every value read from it has been used: signalled right behind the loads, the
-          // next tile now and then overtook them (one row in 10^8 wrong; the copies delay loads from shared memory).
+          // Done with the bias tile.  Only here, where every value read from it has been used: signalled right behind the loads, while
+          // these were generic ones, the next tile now and then overtook them (one row in 10^8 wrong).
           if (r == kFRpg - 1) mbar_arrive(&bars.bias_empty[kt & 1]);
         }
       }

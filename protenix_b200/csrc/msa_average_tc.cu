@@ -65,7 +65,7 @@ __global__ void __launch_bounds__(kMvThreads, 1)
 msa_average_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_v, float* __restrict__ out,
                       int n, int cols, int tiles_m, int tiles_n, int n_tiles, int chunks) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
-  unsigned char* sm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  unsigned char* sm = smem_aligned(smem_raw);
   MvBars& bars = *reinterpret_cast<MvBars*>(sm + MvLayout::bars);
   const int warp = warp_index(), lane = threadIdx.x & 31;
   const int first_tile = blockIdx.x, tile_step = gridDim.x;

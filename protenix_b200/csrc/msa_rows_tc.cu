@@ -68,7 +68,7 @@ template <int kMode>
 __global__ void __launch_bounds__(kMrThreads, 1)
 msa_rows_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_w2, const MrArgs g) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
-  unsigned char* sm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  unsigned char* sm = smem_aligned(smem_raw);
   MrBars& bars = *reinterpret_cast<MrBars*>(sm + MrLayout::bars);
   const int warp = warp_index(), lane = threadIdx.x & 31;
   const int first_tile = blockIdx.x, tile_step = gridDim.x;

@@ -44,7 +44,7 @@ __global__ void __launch_bounds__(kMtThreads, 1)
 msa_transition_tc_kernel(const __grid_constant__ CUtensorMap map_w1, const __grid_constant__ CUtensorMap map_w2, float* m,
                          const float* __restrict__ ln_w, const float* __restrict__ ln_b, long long rows, int n_tiles, float eps) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
-  unsigned char* sm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  unsigned char* sm = smem_aligned(smem_raw);
   MtBars& bars = *reinterpret_cast<MtBars*>(sm + MtLayout::bars);
   const int warp = warp_index(), lane = threadIdx.x & 31;
   const int first_tile = blockIdx.x, tile_step = gridDim.x;

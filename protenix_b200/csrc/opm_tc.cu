@@ -49,7 +49,7 @@ opm_out_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
                   const float* __restrict__ bias, const float* __restrict__ inv_norm, const Tz* z_in,
                   Tz* z_out, int n, int add_residual, int tiles_j, int total_tiles) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
-  unsigned char* sm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  unsigned char* sm = smem_aligned(smem_raw);
   OpBars& bars = *reinterpret_cast<OpBars*>(sm + OpLayout::bars);
   const int warp = warp_index(), lane = threadIdx.x & 31;
 

@@ -20,6 +20,11 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
+// The first 1024-byte boundary of the dynamic shared memory.  As an offset from the array, so that the compiler still sees shared
+// memory behind every pointer made from it: rounded through an integer, all plain accesses were generic ones (slower, counted
+// with global memory, and not in order with the mbarrier operations behind them).
+__device__ __forceinline__ unsigned char* smem_aligned(unsigned char* raw) { return raw + ((0u - smem_u32(raw)) & 1023u); }
+
 __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
   __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
   return *reinterpret_cast<uint32_t*>(&v);

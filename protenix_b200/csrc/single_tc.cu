@@ -106,7 +106,7 @@ template <int kMode, typename T>
 __global__ void __launch_bounds__(kSgThreads, 1)
 split_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w, const SgArgs g) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
-  unsigned char* ring = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  unsigned char* ring = smem_aligned(smem_raw);
   SgBars& bars = *reinterpret_cast<SgBars*>(ring + kSgStages * kSgStageBytes);
   const int warp = warp_index(), lane = threadIdx.x & 31;
   const int n0 = blockIdx.x * kSgBN, m0 = blockIdx.y * 128, kc0 = blockIdx.z * g.chunks;

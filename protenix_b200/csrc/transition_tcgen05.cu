@@ -97,7 +97,7 @@ transition_tc_kernel(const __grid_constant__ CUtensorMap map_wa, const __grid_co
                      const float* __restrict__ ln_w, const float* __restrict__ ln_b, long long rows, int n_tiles,
                      int add_residual, int apart, float eps) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
-  unsigned char* sm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  unsigned char* sm = smem_aligned(smem_raw);
   TransBars& bars = *reinterpret_cast<TransBars*>(sm + TransLayout::bars);
   const int warp = warp_index(), lane = threadIdx.x & 31;
   const int first_tile = blockIdx.x, tile_step = gridDim.x;

@@ -90,7 +90,7 @@ trimul_out_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_con
   constexpr bool kTma = sizeof(Tz) == 2;               // bf16: residual from the z tile, output through TMA
   constexpr bool kF16 = !kTma;                           // operand format of the z side; the x side is always fp16
   extern __shared__ __align__(1024) unsigned char smem_raw[];
-  unsigned char* sm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  unsigned char* sm = smem_aligned(smem_raw);
   ToBars& bars = *reinterpret_cast<ToBars*>(sm + ToLayout::bars);
   const int warp = warp_index(), lane = threadIdx.x & 31;
 
