@@ -2,24 +2,23 @@
 //   out[h][row] = (W LN(z[row]))[h], h < n_heads <= 16, fp32, for every pair element (row) of z.
 //
 // Persistent kernel, one CTA per SM, 128 rows per tile, on the row-tile pipeline of px_rowpipe.cuh (TMA-fed raw rows,
-// LayerNorm folded into the resident 16 x 128 weight plus one correction K step, row statistics from a tensor-core
-// Gram product).  HBM-bound: 128*sizeof(Tz) bytes read and 4*n_heads written per row.
+// LayerNorm folded into the resident 16 x 128 weight plus one correction K step).  HBM-bound: 128*sizeof(Tz) bytes read and 4*n_heads written per row.
 //   warps 0..3  epilogue: a thread owns one row, reads its 16 accumulator columns and writes n_heads floats
 //               (coalesced across the warp for every head);
-//   warps 4..7  one thread per row: statistics, correction row, the row's rstd;
-//   warp 8      TMA producer; warp 9 MMA issuer of the projection (M=128, N=16), warp 10 of the statistics product.
+//   warps 4..7 (bf16 rows 4..11)  statistics, correction row, the row's rstd;
+//   then a TMA producer and the MMA issuer of the projection (M=128, N=16).
 // Every mbarrier wait is bounded.
 #include "px_rowpipe.cuh"
 
 namespace px {
 
-constexpr int kPbWarps = 12;
-constexpr int kPbThreads = 32 * kPbWarps;
+constexpr int kPbStages = 4;
+constexpr int pb_threads(bool f16) { return 32 * (4 + tile_stats_warps(f16) + 2); }
 constexpr int kPbWPanel = 16 * 128;            // [16 heads][64 k] bf16
-constexpr uint32_t kPbColGram = 32;            // tensor memory: projection (16 of 32 columns) | statistics (144)
+constexpr uint32_t kPbCols = 32;               // tensor memory: projection (16 of 32 columns)
 
 struct PbBars {
-  TileBars tile;
+  TileBars<kPbStages> tile;
   uint64_t acc_full, acc_free, w_full;
   uint32_t tmem_base;
 };
@@ -27,9 +26,9 @@ struct PbLayout {
   static constexpr int w = 0;                                   // [16][128 k] as two k panels
   static constexpr int wx = w + 2 * kPbWPanel;                  // correction panel [16][16 k]
   static constexpr int a = wx + 1024;                           // row-tile ring
-  static constexpr int ax = a + kTileStages * kTileBytes;
-  static constexpr int scale = ax + kTileSlots * kTileExtra;    // rstd per row and slot
-  static constexpr int bars = scale + kTileSlots * 128 * 4;
+  static constexpr int ax = a + kPbStages * kTileBytes;
+  static constexpr int scale = ax + tile_slots(kPbStages) * kTileExtra;    // rstd per row and slot
+  static constexpr int bars = scale + tile_slots(kPbStages) * 128 * 4;
   static constexpr int total = bars + (int)sizeof(PbBars);
 };
 static_assert(PbLayout::total + 1024 <= 232448, "shared memory budget");
@@ -56,14 +55,16 @@ struct PbWeights {
 
 // kF16: the rows are the standardised fp16 copy of an fp32 pair tensor (fp16 weights); otherwise bf16 rows of z.
 template <bool kF16>
-__global__ void __launch_bounds__(kPbThreads, 1)
+__global__ void __launch_bounds__(pb_threads(kF16), 1)
 pair_bias_tc_kernel(const __grid_constant__ CUtensorMap map_z, const PbWeights<kF16> weights,
                     const unsigned char* __restrict__ folded, float* __restrict__ out, long long rows, int n_heads, float eps, int n_tiles) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
-  unsigned char* sm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  unsigned char* sm = smem_aligned(smem_raw);
   PbBars& bars = *reinterpret_cast<PbBars*>(sm + PbLayout::bars);
   const int warp = warp_index(), lane = threadIdx.x & 31;
-  TileCtx ctx;
+  typedef TileCtx<kPbStages, kF16> Ctx;
+  constexpr int kCtl = 4 + tile_stats_warps(kF16);       // first control warp
+  Ctx ctx;
   ctx.tiles = sm + PbLayout::a;
   ctx.extras = sm + PbLayout::ax;
   ctx.bars = &bars.tile;
@@ -84,36 +85,30 @@ pair_bias_tc_kernel(const __grid_constant__ CUtensorMap map_z, const PbWeights<k
     mbar_init(&bars.acc_free, 4);
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
-  if (warp == 8) {
+  if (warp == kCtl) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(&bars.tmem_base)),
-                 "r"(256u)
+                 "r"(kPbCols)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
   }
-  tile_write_ones<kF16>(ctx.tiles, threadIdx.x, kPbThreads);
   asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-  if (!cta_ready(skip, warp == 8, bars.tmem_base, 256u, [&] {
+  if (!cta_ready(skip, warp == kCtl, bars.tmem_base, kPbCols, [&] {
         if (folded && threadIdx.x == 0) folded_load(sm, folded, PbWeights<kF16>::kBytes, &bars.w_full);
       }))
     return;
   fold_here(weights, folded, sm, 0, &bars.w_full);
   const uint32_t tmem_base = bars.tmem_base;
 
-  if (warp >= 8) {
-    if (elect_lane()) {
-      if (warp == 8) {
-        tile_producer_loop(ctx, &map_z);
-      } else if (warp == 9) {
-        tile_product_loop(ctx, tmem_base, smem_u32(sm + PbLayout::w), kPbWPanel, smem_u32(sm + PbLayout::wx),
-                          umma_idesc_16(128, 16, kF16, kF16), &bars.w_full, &bars.acc_full, &bars.acc_free);
-      } else if (warp == 10) {
-        if (!kF16) tile_gram_loop<kF16>(ctx, tmem_base + kPbColGram);   // standardised rows: nothing to measure
-      }
-    }
+  if (warp >= kCtl) {
+    if (warp == kCtl)
+      tile_producer_loop(ctx, &map_z);
+    else
+      tile_product_loop(ctx, tmem_base, smem_u32(sm + PbLayout::w), kPbWPanel, smem_u32(sm + PbLayout::wx),
+                        umma_idesc_16(128, 16, kF16, kF16), &bars.w_full, &bars.acc_full, &bars.acc_free);
   } else if (warp >= 4) {
     float* scale = reinterpret_cast<float*>(sm + PbLayout::scale);
-    tile_stats_loop<kF16>(ctx, eps, tmem_base + kPbColGram, warp - 4, lane,
-                        [&](int k, int u, int t, int r, float rstd) { scale[(k % kTileSlots) * 128 + r] = rstd; });
+    tile_stats_loop(ctx, eps, warp - 4, lane,
+                        [&](int k, int u, int t, int r, float rstd) { scale[(k % Ctx::kSlots) * 128 + r] = rstd; });
   } else {
     // ------------------------------------------------------------------ epilogue
     const int row = 32 * warp + lane;
@@ -125,7 +120,7 @@ pair_bias_tc_kernel(const __grid_constant__ CUtensorMap map_z, const PbWeights<k
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
       tc_fence_after();
-      const float rstd = reinterpret_cast<const float*>(sm + PbLayout::scale)[(k % kTileSlots) * 128 + row];
+      const float rstd = reinterpret_cast<const float*>(sm + PbLayout::scale)[(k % Ctx::kSlots) * 128 + row];
       uint32_t acc[16];
       tmem_ld16(t_acc, acc);
       tmem_wait_ld();
@@ -142,9 +137,9 @@ pair_bias_tc_kernel(const __grid_constant__ CUtensorMap map_z, const PbWeights<k
 
   tc_fence_before();
   cta_teardown_sync();
-  if (warp == 8) {
+  if (warp == kCtl) {
     tc_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem_base), "r"(256u) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem_base), "r"(kPbCols) : "memory");
   }
 }
 
@@ -162,7 +157,7 @@ static int32_t launch_pair_bias(const void* z, const PbWeights<kF16>& weights, c
   if (!limit.set(pair_bias_tc_kernel<kF16>, smem)) return PX_ERR_LAUNCH;
   const int64_t n_tiles = (rows + 127) / 128;
   const int grid = (int)(n_tiles < sm_count() ? n_tiles : sm_count());
-  return launch_pdl(pair_bias_tc_kernel<kF16>, dim3(grid), kPbThreads, smem, st, mz, weights, (const unsigned char*)folded, out,
+  return launch_pdl(pair_bias_tc_kernel<kF16>, dim3(grid), pb_threads(kF16), smem, st, mz, weights, (const unsigned char*)folded, out,
                     (long long)rows, (int)n_heads, eps, (int)n_tiles)
              ? PX_OK
              : PX_ERR_LAUNCH;

@@ -116,7 +116,7 @@ constexpr int kFoldThreads = 768;
 template <typename W>
 __global__ void __launch_bounds__(kFoldThreads, 1) fold_kernel(const W weights, unsigned char* __restrict__ image) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
-  unsigned char* sm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  unsigned char* sm = smem_aligned(smem_raw);
   weights.fold(sm, blockIdx.x, threadIdx.x >> 5, kFoldThreads / 32, threadIdx.x & 31, threadIdx.x, kFoldThreads);
   __syncthreads();
   for (int i = threadIdx.x; i < W::kBytes / 16; i += kFoldThreads)
@@ -186,174 +186,166 @@ __device__ __forceinline__ void named_barrier(int id, int threads) {
 // ---------------------------------------------------------------------------------------------------------------
 // Row tiles: the part of the pipeline that is the same for every kernel that consumes LayerNorm'd pair rows.
 // A tile is 128 pair elements (one u, 128 consecutive t); element (u, t) is row u*n_t + t of z, or row t*n_u + u when
-// the two indices are exchanged (`swap`).  A stage of the ring holds the tile as two k panels of 144 rows (the
-// last 16 rows are ones, see below) and the tile's correction panel.
+// the two indices are exchanged (`swap`).  A stage of the ring holds the tile as two k panels of 128 rows.
 //   * producer thread: TMA loads of the rows (bf16 rows of z, or the standardised fp16 copy of an fp32 z);
-//   * statistics issuer thread: Z Z^T | Z 1 (M=128, N=144) into tensor memory: the diagonal holds each row's sum
-//     of squares and columns 128..143 its plain sum;
-//   * statistics threads (one per row): variance = E[x^2] - mean^2 in fp32 (accurate while |mean| is not orders of
-//     magnitude above the deviation), correction row (-mean, std), and whatever the kernel wants per row.  For
-//     standardised rows the statistics are known: (0, 1).
+//   * statistics threads: mean and variance of the row as it lies in the stage (bf16 rows), correction row (-mean, std),
+//     and whatever the kernel wants per row.  For standardised rows the statistics are known: (0, 1).  A product Z Z^T
+//     with the sums of squares on its diagonal took 600 cycles of the tensor pipe a tile, and 144 columns of tensor memory that
+//     now hold a second set of accumulators for bf16 rows, too.
+// What bounds these kernels from N = 384 on is the way of a tile from memory, 2 us under load: three stages where they fit
+// (with the statistics as they are now; projections of the triangle multiplication, bf16 N = 768 132 -> 117 us, N = 437 55.3 -> 47.5;
+// fp16 N = 384 in a stack 36.4 -> 31.8; two stages and a second staging buffer 148 at N = 768 where three took 136).
 // ---------------------------------------------------------------------------------------------------------------
-constexpr int kTileStages = 2;
-constexpr int kTileSlots = 4;    // slots of everything written per tile by the statistics warps (scales, correction
-                                 // rows, the a_ready barrier): read after the stage is freed, by an epilogue that may
-                                 // run two tiles behind the products when the accumulators are double-buffered
-constexpr int kTilePanel = 144 * 128;          // [128 rows + 16 rows of ones][64 k] bf16
-constexpr int kTileBytes = 2 * kTilePanel;
+constexpr int kTileBytes = kOperandBytes;
 constexpr int kTileExtra = 128 * 32;           // [128 rows][16 k] correction panel
-constexpr uint32_t kGramCols = 144;
 
+// Slots of everything written per tile by the statistics warps (scales, correction rows, the a_ready barrier): read after the
+// stage is freed, by an epilogue that may run two tiles behind the products when the accumulators are double-buffered.  Slot
+// k % slots is rewritten for tile k + slots, whose stage is the one of tile k + 2, and handed out only after the products of
+// that tile, which are issued after the correction step of tile k and wait for the epilogue of tile k (at the latest) to have
+// read its scales and its accumulator.
+constexpr int tile_slots(int stages) { return stages + 2; }
+// The correction rows of standardised rows are all alike: one panel serves every tile.
+constexpr int tile_extras(int stages, bool standardised) { return standardised ? 1 : tile_slots(stages); }
+
+template <int kStages>
 struct TileBars {
   // raw_full: tile in shared memory; a_ready: statistics, correction rows and scales written;
   // a_empty: every MMA that reads the stage is complete (one commit per issuing thread)
-  uint64_t raw_full[kTileStages], a_ready[kTileSlots], a_empty[kTileStages], gram_full, gram_free;
+  uint64_t raw_full[kStages], a_ready[tile_slots(kStages)], a_empty[kStages];
 };
+// kStandardised: the rows are a standardised fp16 copy (otherwise bf16 rows of z).
+template <int kStages_, bool kStandardised_>
 struct TileCtx {
-  unsigned char* tiles;     // kTileStages x kTileBytes
-  unsigned char* extras;    // kTileSlots x kTileExtra (the correction step of a tile runs after its stage is freed)
-  TileBars* bars;
+  static constexpr int kStages = kStages_, kSlots = tile_slots(kStages_);
+  static constexpr bool kStandardised = kStandardised_;
+  unsigned char* tiles;     // kStages x kTileBytes
+  unsigned char* extras;    // tile_extras() x kTileExtra (the correction step of a tile runs after its stage is freed)
+  TileBars<kStages_>* bars;
   int first_tile, tile_step, n_tiles, tiles_t, n_u, n_t, swap;
+  __device__ __forceinline__ unsigned char* extra(int k) const { return extras + (kStandardised ? 0 : (k % kSlots) * kTileExtra); }
 };
 
-// readers: how many arrivals free a stage besides the statistics side, which adds one (the thread that issues the
-// statistics product) or, for standardised rows, four (the statistics warps, which only watch the tile arrive).
-__device__ __forceinline__ void tile_bars_init(TileBars& b, int readers, bool standardised) {
-  for (int s = 0; s < kTileStages; ++s) {
+// Statistics warps: a thread per row where there is nothing to measure, two for bf16 rows.
+constexpr int tile_stats_warps(bool standardised) { return standardised ? 4 : 8; }
+// readers: how many arrivals free a stage besides those of the statistics warps.
+template <int kStages>
+__device__ __forceinline__ void tile_bars_init(TileBars<kStages>& b, int readers, bool standardised) {
+  const int warps = tile_stats_warps(standardised);
+  for (int s = 0; s < kStages; ++s) {
     mbar_init(&b.raw_full[s], 1);
-    mbar_init(&b.a_empty[s], readers + (standardised ? 4 : 1));
+    mbar_init(&b.a_empty[s], readers + warps);
   }
-  for (int s = 0; s < kTileSlots; ++s) mbar_init(&b.a_ready[s], 4);
-  mbar_init(&b.gram_full, 1);
-  mbar_init(&b.gram_free, 4);
+  for (int s = 0; s < tile_slots(kStages); ++s) mbar_init(&b.a_ready[s], warps);
 }
 
-// The 16 rows of ones behind every tile panel (never overwritten: a tile load covers 128 rows).
-template <bool kF16>
-__device__ __forceinline__ void tile_write_ones(unsigned char* tiles, int tid, int nthreads) {
-  constexpr uint32_t one = ones16x2(kF16);
-  for (int i = tid; i < kTileStages * 2 * 16 * 8; i += nthreads) {
-    const int panel = i >> 7, piece = i & 127;
-    *reinterpret_cast<uint4*>(tiles + panel * kTilePanel + 128 * 128 + piece * 16) = make_uint4(one, one, one, one);
-  }
-}
-
-// One thread: TMA loads of the bf16 tiles.
-__device__ __forceinline__ void tile_producer_loop(const TileCtx& c, const CUtensorMap* map_z) {
+// One warp: TMA loads of the tiles.
+template <typename Ctx>
+__device__ __forceinline__ void tile_producer_loop(const Ctx& c, const CUtensorMap* map_z) {
   int k = 0;
   for (int tile = c.first_tile; tile < c.n_tiles; tile += c.tile_step, ++k) {
-    const int s = k % kTileStages, n = k / kTileStages;
-    if (!mbar_wait(&c.bars->a_empty[s], (n & 1) ^ 1, 1u)) break;
-    const int u = tile / c.tiles_t, t0 = (tile % c.tiles_t) * 128;
-    mbar_expect_tx(&c.bars->raw_full[s], kOperandBytes);
-    const uint32_t dst = smem_u32(c.tiles + s * kTileBytes);
-    for (int p = 0; p < 2; ++p)
-      tma_load_3d(dst + p * kTilePanel, map_z, &c.bars->raw_full[s], 64 * p, c.swap ? u : t0, c.swap ? t0 : u);
-  }
-}
-
-// One thread: the statistics product of every tile into tensor-memory columns [gram_col, gram_col + 144).
-template <bool kF16>
-__device__ __forceinline__ void tile_gram_loop(const TileCtx& c, uint32_t tmem_gram) {
-  constexpr uint32_t idesc_gram = umma_idesc_16(128, kGramCols, kF16, kF16);
-  int k = 0;
-  for (int tile = c.first_tile; tile < c.n_tiles; tile += c.tile_step, ++k) {
-    const int s = k % kTileStages, n = k / kTileStages;
-    if (!mbar_wait(&c.bars->raw_full[s], n & 1, 2u) || !mbar_wait(&c.bars->gram_free, (k & 1) ^ 1, 2u)) break;
-    tc_fence_after();
-    const uint32_t a_addr = smem_u32(c.tiles + s * kTileBytes);
-#pragma unroll
-    for (int ks = 0; ks < 8; ++ks) {
-      const uint64_t d = umma_desc_sw128(a_addr + (ks >> 2) * kTilePanel) + 2 * (ks & 3);
-      umma_bf16(tmem_gram, d, d, idesc_gram, ks ? 1u : 0u);
+    const int s = k % Ctx::kStages, n = k / Ctx::kStages;
+    if (!mbar_wait_warp(&c.bars->a_empty[s], (n & 1) ^ 1, 1u)) break;
+    if (elect_lane()) {
+      const int u = tile / c.tiles_t, t0 = (tile % c.tiles_t) * 128;
+      mbar_expect_tx(&c.bars->raw_full[s], kOperandBytes);
+      const uint32_t dst = smem_u32(c.tiles + s * kTileBytes);
+      for (int p = 0; p < 2; ++p)
+        tma_load_3d(dst + p * kPanelBytes, map_z, &c.bars->raw_full[s], 64 * p, c.swap ? u : t0, c.swap ? t0 : u);
     }
-    umma_commit(&c.bars->gram_full);
-    umma_commit(&c.bars->a_empty[s]);
+    __syncwarp();
   }
 }
 
-// Four warps, one thread per row (`qw` = warp's lane quarter, 0..3).  per_row(k, u, t, r, rstd) is called once per
+// The statistics warps (`sw` = 0..3, or 0..7 for bf16 rows).  per_row(k, u, t, r, rstd) is called once per
 // tile and row with the row's 1/std, before a_ready is signalled.  `kStandardised`: the rows are a standardised copy
-// (mean 0, deviation 1 by construction), so the correction row is (0, 1) and the factor is 1.
-template <bool kStandardised, typename PerRow>
-__device__ __forceinline__ void tile_stats_loop(const TileCtx& c, float eps, uint32_t tmem_gram, int qw, int lane,
-                                                PerRow per_row) {
-  const int r = 32 * qw + lane;
-  const uint32_t t_gram = tmem_gram + ((uint32_t)(32 * qw) << 16);
+// (mean 0, deviation 1 by construction), so the correction row is (0, 1), written once, and the factor is 1.
+// bf16 rows: two neighbouring lanes share a row, eight 16-byte pieces each (lane 1 begins at another piece, so that the two meet
+// different banks), and sum d and d^2 of d = x - x0 in fp32: about one of its values, nothing cancels however far the row lies from zero.
+template <typename Ctx, typename PerRow>
+__device__ __forceinline__ void tile_stats_loop(const Ctx& c, float eps, int sw, int lane, PerRow per_row) {
+  constexpr bool kStandardised = Ctx::kStandardised;
+  const int r = kStandardised ? 32 * sw + lane : 16 * sw + (lane >> 1), half = lane & 1;
   int k = 0;
-  bool ok = true;
   for (int tile = c.first_tile; tile < c.n_tiles; tile += c.tile_step, ++k) {
-    const int s = k % kTileStages;
+    const int s = k % Ctx::kStages;
     const int u = tile / c.tiles_t, t = (tile % c.tiles_t) * 128 + r;
     float mean = 0.f, std = 1.f, rstd = 1.f;
-    if (kStandardised) {
-      // nothing to measure (no statistics product runs in this mode): the arrival of the tile only paces this loop,
-      // so that the slots it writes are those of tiles in flight
-      ok = mbar_wait(&c.bars->raw_full[s], (k / kTileStages) & 1, 16u);
-      ok = __all_sync(0xffffffffu, ok);
-      if (!ok) break;
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&c.bars->a_empty[s]);   // seen: the stage may move on (no phase can be missed)
-    } else {
-      ok = mbar_wait(&c.bars->gram_full, k & 1, 16u);
-      ok = __all_sync(0xffffffffu, ok);
-      if (!ok) break;
-      tc_fence_after();
-      uint32_t diag[32], sums[16];
-      tmem_ld32(t_gram + 32 * qw, diag);
-      tmem_ld16(t_gram + 128, sums);
-      tmem_wait_ld();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&c.bars->gram_free);
-      mean = __uint_as_float(sums[0]) * (1.0f / kC);
-      const float var = fmaxf(select_own(diag, lane) * (1.0f / kC) - mean * mean, 0.f);
+    // for standardised rows the arrival of the tile only paces this loop, so that the slots it writes are those of tiles in flight
+    if (!mbar_wait_warp(&c.bars->raw_full[s], (k / Ctx::kStages) & 1, 16u)) break;
+    if (!kStandardised) {
+      const unsigned char* z = c.tiles + s * kTileBytes;
+      const float x0 = unpack_bf16x2(*reinterpret_cast<const uint32_t*>(z + operand_piece_offset(r, 0))).x;
+      float s0 = 0.f, s1 = 0.f, q0 = 0.f, q1 = 0.f;
+#pragma unroll
+      for (int p = 0; p < 8; ++p) {
+        const uint4 v = *reinterpret_cast<const uint4*>(z + operand_piece_offset(r, 8 * half + (p ^ (4 * half))));
+        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          float2 x = unpack_bf16x2(w[e]);
+          add2(x.x, x.y, -x0, -x0);
+          add2(s0, s1, x.x, x.y);
+          fma2(q0, q1, x.x, x.y, x.x, x.y, q0, q1);
+        }
+      }
+      float sum = s0 + s1, sq = q0 + q1;
+      sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+      sq += __shfl_xor_sync(0xffffffffu, sq, 1);
+      const float m = sum * (1.0f / kC), var = fmaxf(sq * (1.0f / kC) - m * m, 0.f);
+      mean = x0 + m;
       rstd = rsqrtf(var + eps);
       std = sqrtf(var + eps);
     }
     // rstd * (W'x - mean * s + std * t): the row side of the correction step holds (-mean, std)
-    write_correction_row(c.extras + (k % kTileSlots) * kTileExtra, r, -mean, std, false);
-    per_row(k, u, t, r, rstd);
+    if (kStandardised ? k == 0 : half == 0) write_correction_row(c.extra(k), r, -mean, std, false);
+    if (kStandardised || half == 0) per_row(k, u, t, r, rstd);
     asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
     __syncwarp();
-    if (lane == 0) mbar_arrive(&c.bars->a_ready[k % kTileSlots]);
+    if (lane == 0) {
+      mbar_arrive(&c.bars->a_ready[k % Ctx::kSlots]);
+      mbar_arrive(&c.bars->a_empty[s]);                 // after the last use of what was read from the stage
+    }
   }
 }
 
-// One thread: for every tile, 8 MMAs M=128 (rows) x N (weight rows of `w_addr`, two k panels of w_panel bytes) into
+// One warp: for every tile, 8 MMAs M=128 (rows) x N (weight rows of `w_addr`, two k panels of w_panel bytes) into
 // tensor-memory column d_tmem, then the correction step against the weight-side panel at wx_addr.  acc_full/acc_free
 // hand the accumulator back and forth with the epilogue warps: arrays of n_acc barriers, tile k uses accumulator
 // k % n_acc at d_tmem + (k % n_acc) * acc_cols (n_acc = 1 or 2).
-__device__ __forceinline__ void tile_product_loop(const TileCtx& c, uint32_t d_tmem, uint32_t w_addr, int w_panel,
+template <typename Ctx>
+__device__ __forceinline__ void tile_product_loop(const Ctx& c, uint32_t d_tmem, uint32_t w_addr, int w_panel,
                                                   uint32_t wx_addr, uint32_t idesc, uint64_t* w_full,
                                                   uint64_t* acc_full, uint64_t* acc_free, int n_acc = 1,
                                                   uint32_t acc_cols = 0) {
-  if (!mbar_wait(w_full, 0, 4u)) return;         // the resident weights
+  if (!mbar_wait_warp(w_full, 0, 4u)) return;    // the resident weights
   const uint64_t wx_desc = umma_desc_sw32(wx_addr);
   // the correction step multiplies bf16 head/tail pairs whatever the format of the main operands; M and N as `idesc`
   const uint32_t idesc_corr = idesc | (1u << 7) | (1u << 10);
   int k = 0;
   for (int tile = c.first_tile; tile < c.n_tiles; tile += c.tile_step, ++k) {
-    const int s = k % kTileStages, n = k / kTileStages;
+    const int s = k % Ctx::kStages, n = k / Ctx::kStages;
     const int ab = n_acc == 2 ? (k & 1) : 0, an = n_acc == 2 ? (k >> 1) : k;
     const uint32_t d = d_tmem + ab * acc_cols;
-    if (!mbar_wait(&c.bars->raw_full[s], n & 1, 4u) || !mbar_wait(&acc_free[ab], (an & 1) ^ 1, 8u)) break;
+    if (!mbar_wait_warp(&c.bars->raw_full[s], n & 1, 4u) || !mbar_wait_warp(&acc_free[ab], (an & 1) ^ 1, 8u)) break;
     tc_fence_after();
-    const uint32_t a_addr = smem_u32(c.tiles + s * kTileBytes);
+    if (elect_lane()) {
+      const uint32_t a_addr = smem_u32(c.tiles + s * kTileBytes);
 #pragma unroll
-    for (int ks = 0; ks < 8; ++ks)
-      umma_bf16(d, umma_desc_sw128(a_addr + (ks >> 2) * kTilePanel) + 2 * (ks & 3),
-                umma_desc_sw128(w_addr + (ks >> 2) * w_panel) + 2 * (ks & 3), idesc, ks ? 1u : 0u);
-    // This thread's reads of the stage end here: the producer may refill it while the statistics of the tile are
-    // still on their way.  The correction step reads the tile's slot of the correction ring; slot k % 4 (rows, scales
-    // and the a_ready barrier alike) is rewritten for tile k + 4, whose stage is handed out only after the products
-    // of tile k + 2, which this thread issues after the correction step below and which wait for the epilogue of
-    // tile k (at the latest) to have read its scales and its accumulator.
-    umma_commit(&c.bars->a_empty[s]);
-    if (!mbar_wait(&c.bars->a_ready[k % kTileSlots], (k / kTileSlots) & 1, 4u)) break;   // needs the statistics
+      for (int ks = 0; ks < 8; ++ks)
+        umma_bf16(d, umma_desc_sw128(a_addr + (ks >> 2) * kPanelBytes) + 2 * (ks & 3),
+                  umma_desc_sw128(w_addr + (ks >> 2) * w_panel) + 2 * (ks & 3), idesc, ks ? 1u : 0u);
+      // this warp's reads of the stage end here: the producer may refill it while the statistics of the tile are on their way
+      umma_commit(&c.bars->a_empty[s]);
+    }
+    __syncwarp();
+    if (!mbar_wait_warp(&c.bars->a_ready[k % Ctx::kSlots], (k / Ctx::kSlots) & 1, 4u)) break;   // needs the statistics
     tc_fence_after();
-    umma_bf16(d, umma_desc_sw32(smem_u32(c.extras + (k % kTileSlots) * kTileExtra)), wx_desc, idesc_corr, 1u);
-    umma_commit(&acc_full[ab]);
+    if (elect_lane()) {
+      umma_bf16(d, umma_desc_sw32(smem_u32(c.extra(k))), wx_desc, idesc_corr, 1u);
+      umma_commit(&acc_full[ab]);
+    }
+    __syncwarp();
   }
 }
 

@@ -3,14 +3,12 @@
 // (protenix/model/protenix.py:246: z = z_init + linear_no_bias_z_cycle(layernorm_z_cycle(z))).
 //
 // Persistent kernel, one CTA per SM, 128 rows per tile, on the row-tile pipeline of px_rowpipe.cuh (TMA-fed raw rows,
-// LayerNorm folded into the resident weight plus one correction K step, row statistics from a tensor-core Gram
-// product).  HBM-bound: per row 128*sizeof(Tz) bytes of z and of z_init are read and as many written.
+// LayerNorm folded into the resident weight plus one correction K step).  HBM-bound: per row 128*sizeof(Tz) bytes of z and of z_init are read and as many written.
 //   warps 0..7   output rows: a thread owns one row and 64 of its channels, adds rstd * accumulator to the z_init
 //                tile in shared memory (brought in by TMA, in place) and one thread stores the tile by TMA;
 //                fp32 rows read z_init from global memory and use plain stores;
-//   warps 8..11  one thread per row: statistics, correction row, the row's rstd;
-//   warp 12      TMA producer (z tiles and z_init tiles); warp 13 MMA issuer of the projection (M=128, N=128),
-//   warp 14      MMA issuer of the statistics product.
+//   warps 8..11  (bf16 rows 8..15) statistics, correction row, the row's rstd;
+//   then         a TMA producer (z tiles and z_init tiles) and the MMA issuer of the projection (M=128, N=128).
 // `out` may be the same buffer as `z` or as `z_init`: a tile is written only after all of its reads.
 // Every mbarrier wait is bounded.
 #include <cstring>
@@ -19,23 +17,23 @@
 
 namespace px {
 
-constexpr int kRcWarps = 15;
-constexpr int kRcThreads = 32 * kRcWarps;
-constexpr uint32_t kRcColGram = 128;           // tensor memory: projection (128 columns) | statistics (144)
+constexpr int kRcStages = 2;
+constexpr int rc_warps(bool f16) { return 8 + tile_stats_warps(f16) + 2; }
+constexpr uint32_t kRcCols = 128;              // tensor memory: projection
 
 struct RcBars {
-  TileBars tile;
-  uint64_t w_full, acc_full, acc_free, res_full[kTileStages], res_empty[kTileStages];
+  TileBars<kRcStages> tile;
+  uint64_t w_full, acc_full, acc_free, res_full[kRcStages], res_empty[kRcStages];
   uint32_t tmem_base;
 };
 struct RcLayout {
   static constexpr int w = 0;                                   // [128][128 k] as two k panels
   static constexpr int wx = w + kOperandBytes;                  // correction panel [128][16 k]
   static constexpr int a = wx + 128 * 32;                       // row-tile ring
-  static constexpr int ax = a + kTileStages * kTileBytes;
-  static constexpr int res = ax + kTileSlots * kTileExtra;      // z_init tiles, then the output tiles, in place
-  static constexpr int scale = res + kTileStages * kOperandBytes;  // rstd per row and slot
-  static constexpr int bars = scale + kTileSlots * 128 * 4;
+  static constexpr int ax = a + kRcStages * kTileBytes;
+  static constexpr int res = ax + tile_slots(kRcStages) * kTileExtra;      // z_init tiles, then the output tiles, in place
+  static constexpr int scale = res + kRcStages * kOperandBytes;  // rstd per row and slot
+  static constexpr int bars = scale + tile_slots(kRcStages) * 128 * 4;
   static constexpr int total = bars + (int)sizeof(RcBars);
 };
 static_assert(RcLayout::total + 1024 <= 232448, "shared memory budget");
@@ -44,7 +42,7 @@ static_assert(RcLayout::a % 1024 == 0 && RcLayout::res % 1024 == 0, "tiles must 
 static __device__ float g_rc_zero_beta[128];   // stands in for a LayerNorm without bias
 
 template <typename Tz>
-__global__ void __launch_bounds__(kRcThreads, 1)
+__global__ void __launch_bounds__(32 * rc_warps(sizeof(Tz) != 2), 1)
 recycle_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_constant__ CUtensorMap map_init,
                   const __grid_constant__ CUtensorMap map_out, const Tz* z_init, Tz* out,
                   const float* __restrict__ ln_w, const float* __restrict__ ln_b, const bf16* __restrict__ w,
@@ -52,10 +50,12 @@ recycle_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_consta
   constexpr bool kTma = sizeof(Tz) == 2;               // bf16: z_init and out go through shared memory and TMA
   constexpr bool kF16 = !kTma;                           // fp32: the rows of z arrive as a standardised fp16 copy
   extern __shared__ __align__(1024) unsigned char smem_raw[];
-  unsigned char* sm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  unsigned char* sm = smem_aligned(smem_raw);
   RcBars& bars = *reinterpret_cast<RcBars*>(sm + RcLayout::bars);
   const int warp = warp_index(), lane = threadIdx.x & 31;
-  TileCtx ctx;
+  typedef TileCtx<kRcStages, kF16> Ctx;
+  constexpr int kCtl = 8 + tile_stats_warps(kF16);       // first control warp
+  Ctx ctx;
   ctx.tiles = sm + RcLayout::a;
   ctx.extras = sm + RcLayout::ax;
   ctx.bars = &bars.tile;
@@ -77,57 +77,58 @@ recycle_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_consta
     mbar_init(&bars.w_full, 1);
     mbar_init(&bars.acc_full, 1);
     mbar_init(&bars.acc_free, 8);
-    for (int s = 0; s < kTileStages; ++s) {
+    for (int s = 0; s < kRcStages; ++s) {
       mbar_init(&bars.res_full[s], 1);
       mbar_init(&bars.res_empty[s], 1);
     }
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
-  if (warp == 12) {
+  if (warp == kCtl) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(&bars.tmem_base)),
-                 "r"(512u)
+                 "r"(kRcCols)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
   }
-  tile_write_ones<kF16>(ctx.tiles, threadIdx.x, kRcThreads);
   asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-  if (!cta_ready(skip, warp == 12, bars.tmem_base, 512u)) return;
+  if (!cta_ready(skip, warp == kCtl, bars.tmem_base, kRcCols)) return;
   fold_weight_rows<kF16, kF16>(sm + RcLayout::w, sm + RcLayout::wx, 0, kPanelBytes, w, 0, 128, ln_w, ln_b ? ln_b : g_rc_zero_beta, 1.0f,
-                   warp, kRcWarps, lane);
+                   warp, rc_warps(kF16), lane);
   asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
   __syncthreads();
   if (threadIdx.x == 0) mbar_arrive(&bars.w_full);
   const uint32_t tmem_base = bars.tmem_base;
 
-  if (warp >= 12) {
-    if (elect_lane()) {
-      if (warp == 12) {
-        // z tile into the operand ring and (bf16) the z_init tile into the output ring
-        int k = 0;
-        for (int tile = ctx.first_tile; tile < n_tiles; tile += ctx.tile_step, ++k) {
-          const int s = k % kTileStages, n = k / kTileStages;
-          if (!mbar_wait(&bars.tile.a_empty[s], (n & 1) ^ 1, 1u)) break;
+  if (warp >= kCtl) {
+    if (warp == kCtl) {
+      // z tile into the operand ring and (bf16) the z_init tile into the output ring
+      int k = 0;
+      for (int tile = ctx.first_tile; tile < n_tiles; tile += ctx.tile_step, ++k) {
+        const int s = k % kRcStages, n = k / kRcStages;
+        if (!mbar_wait_warp(&bars.tile.a_empty[s], (n & 1) ^ 1, 1u)) break;
+        if (elect_lane()) {
           mbar_expect_tx(&bars.tile.raw_full[s], kOperandBytes);
           const uint32_t dst = smem_u32(ctx.tiles + s * kTileBytes);
-          for (int p = 0; p < 2; ++p) tma_load_3d(dst + p * kTilePanel, &map_z, &bars.tile.raw_full[s], 64 * p, tile * 128, 0);
-          if (kTma) {
-            if (!mbar_wait(&bars.res_empty[s], (n & 1) ^ 1, 1u)) break;
+          for (int p = 0; p < 2; ++p) tma_load_3d(dst + p * kPanelBytes, &map_z, &bars.tile.raw_full[s], 64 * p, tile * 128, 0);
+        }
+        __syncwarp();
+        if (kTma) {
+          if (!mbar_wait_warp(&bars.res_empty[s], (n & 1) ^ 1, 1u)) break;
+          if (elect_lane()) {
             mbar_expect_tx(&bars.res_full[s], kOperandBytes);
             const uint32_t rdst = smem_u32(sm + RcLayout::res + s * kOperandBytes);
             for (int p = 0; p < 2; ++p) tma_load_3d(rdst + p * kPanelBytes, &map_init, &bars.res_full[s], 64 * p, tile * 128, 0);
           }
+          __syncwarp();
         }
-      } else if (warp == 13) {
-        tile_product_loop(ctx, tmem_base, smem_u32(sm + RcLayout::w), kPanelBytes, smem_u32(sm + RcLayout::wx),
-                          umma_idesc_16(128, 128, kF16, kF16), &bars.w_full, &bars.acc_full, &bars.acc_free);
-      } else if (warp == 14) {
-        if (!kF16) tile_gram_loop<kF16>(ctx, tmem_base + kRcColGram);   // standardised rows: nothing to measure
       }
+    } else {
+      tile_product_loop(ctx, tmem_base, smem_u32(sm + RcLayout::w), kPanelBytes, smem_u32(sm + RcLayout::wx),
+                        umma_idesc_16(128, 128, kF16, kF16), &bars.w_full, &bars.acc_full, &bars.acc_free);
     }
   } else if (warp >= 8) {
     float* scale = reinterpret_cast<float*>(sm + RcLayout::scale);
-    tile_stats_loop<kF16>(ctx, eps, tmem_base + kRcColGram, warp - 8, lane,
-                        [&](int k, int u, int t, int r, float rstd) { scale[(k % kTileSlots) * 128 + r] = rstd; });
+    tile_stats_loop(ctx, eps, warp - 8, lane,
+                        [&](int k, int u, int t, int r, float rstd) { scale[(k % Ctx::kSlots) * 128 + r] = rstd; });
   } else {
     // ------------------------------------------------------------------ output rows
     const int half = (warp >> 2) & 1, qw = warp & 3;
@@ -137,7 +138,7 @@ recycle_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_consta
     int k = 0;
     bool ok = true;
     for (int tile = ctx.first_tile; tile < n_tiles && ok; tile += ctx.tile_step, ++k) {
-      const int s = k % kTileStages, n = k / kTileStages;
+      const int s = k % kRcStages, n = k / kRcStages;
       // fp32 rows: this warp's 32 rows and their z_init values for the first 32 channels, requested before the wait
       const long long first_row = (long long)tile * 128 + 32 * qw;
       const int valid = rows - first_row < 32 ? (rows - first_row > 0 ? (int)(rows - first_row) : 0) : 32;
@@ -157,7 +158,7 @@ recycle_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_consta
       ok = named_barrier_all(1, 256, ok);                  // all eight warps go on, or none
       if (!ok) break;
       tc_fence_after();
-      const float rstd = reinterpret_cast<const float*>(sm + RcLayout::scale)[(k % kTileSlots) * 128 + row];
+      const float rstd = reinterpret_cast<const float*>(sm + RcLayout::scale)[(k % Ctx::kSlots) * 128 + row];
       unsigned char* rtile = sm + RcLayout::res + s * kOperandBytes;
 #pragma unroll
       for (int hh = 0; hh < 2; ++hh) {
@@ -212,9 +213,9 @@ recycle_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_consta
 
   tc_fence_before();
   cta_teardown_sync();
-  if (warp == 12) {
+  if (warp == kCtl) {
     tc_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem_base), "r"(512u) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem_base), "r"(kRcCols) : "memory");
   }
 }
 
@@ -244,7 +245,7 @@ static int32_t launch_recycle(const void* z, const void* z_init, void* out, cons
   if (!limit.set(recycle_tc_kernel<Tz>, smem)) return PX_ERR_LAUNCH;
   const int64_t n_tiles = (rows + 127) / 128;
   const int grid = (int)(n_tiles < sm_count() ? n_tiles : sm_count());
-  return launch_pdl(recycle_tc_kernel<Tz>, dim3(grid), kRcThreads, smem, st, mz, mi, mo, (const Tz*)z_init, (Tz*)out, ln_w, ln_b,
+  return launch_pdl(recycle_tc_kernel<Tz>, dim3(grid), 32 * rc_warps(sizeof(Tz) != 2), smem, st, mz, mi, mo, (const Tz*)z_init, (Tz*)out, ln_w, ln_b,
                     (const bf16*)w, (long long)rows, eps, (int)n_tiles)
              ? PX_OK
              : PX_ERR_LAUNCH;

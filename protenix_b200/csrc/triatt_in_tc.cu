@@ -5,7 +5,7 @@
 //   element (u, t) = z[u][t] (starting node) or z[t][u] (ending node).
 //
 // Persistent kernel, one CTA per SM, on the row-tile pipeline of px_rowpipe.cuh (TMA-fed raw rows, LayerNorm folded
-// into the resident weights plus one correction K step, row statistics from a tensor-core Gram product).  The CTAs
+// into the resident weights plus one correction K step).  The CTAs
 // work in pairs on the same tiles; CTA parity picks two of the four heads.
 //
 //   warps 0..7    epilogue of q | k: a thread owns one pair element and both heads of q (warps 0..3) or k (4..7):
@@ -13,9 +13,8 @@
 //                 pieces of 16 bytes, half a sector each, they took the kernel from 32 to 42 us at N = 384 and from 119 to 144 at N = 768.
 //   warps 8..15   epilogue of v | bias: v goes through a [64 d][128 t] staging tile and a TMA store (the transpose),
 //                 the two bias values of the row are written directly.
-//   warps 16..19  one thread per row: statistics, correction row, scale pair, mask bias.
-//   warp 20       TMA producer; warps 21, 22 MMA issuers of the two products (N = 128 and N = 80), warp 23 of the
-//                 statistics product.
+//   warps 16..19  (bf16 rows 16..23) statistics, correction row, scale pair, mask bias.
+//   then          a TMA producer and the MMA issuers of the two products (N = 128 and N = 80), each into two accumulators in turn.
 // Algorithmic HBM traffic per pair element: 256 + 4 read, 3*256 + 16 + 4 written.  Every wait is bounded.
 #include <math_constants.h>
 
@@ -25,42 +24,44 @@ namespace px {
 
 constexpr int kAiH = 4, kAiD = 32;
 constexpr int kAiW1Panel = 80 * 128;           // [v 64 | bias 16][64 k]
-constexpr int kAiStageOut = 64 * 256;          // [64 d][128 t] fp16
-constexpr int kAiWarps = 24;
-constexpr int kAiThreads = 32 * kAiWarps;
-constexpr uint32_t kAiColGram = 256;           // tensor memory: q|k (128) | v|bias (80) | - | statistics (144);
-                                               // standardised rows: a second set of accumulators at 256 instead
+constexpr int kAiStageOut = 32 * 256;          // [32 d][128 t] fp16: one head
+constexpr int ai_threads(bool f16) { return 32 * (16 + tile_stats_warps(f16) + 3); }
+constexpr int ai_stages(bool f16) { return f16 ? 3 : 2; }     // what shared memory holds: standardised rows need one correction panel
+// tensor memory: q|k (128) | v|bias (80) | -, twice
 
+template <bool kF16>
 struct AiBars {
-  TileBars tile;
+  TileBars<ai_stages(kF16)> tile;
   uint64_t acc_full[2][2], acc_free[2][2];   // [product][accumulator]
   uint64_t w_full;
   uint32_t tmem_base;
 };
+template <bool kF16>
 struct AiLayout {
+  static constexpr int kStages = ai_stages(kF16);
   static constexpr int w0 = 0;                                  // [q 64 | k 64][128 k]
   static constexpr int w1 = w0 + kOperandBytes;                 // [v 64 | bias 16][128 k]
   static constexpr int wx0 = w1 + 2 * kAiW1Panel;               // correction panels
   static constexpr int wx1 = wx0 + 128 * 32;
   static constexpr int a = wx1 + 128 * 32;                      // row-tile ring
-  static constexpr int ax = a + kTileStages * kTileBytes;
-  static constexpr int out = ax + kTileSlots * kTileExtra;      // v staging
-  static constexpr int qk = out + kAiStageOut;                  // q, k staging: 8 warps x 2 heads x [32 t][32] fp16
+  static constexpr int ax = a + kStages * kTileBytes;
+  static constexpr int out = ax + tile_extras(kStages, kF16) * kTileExtra;   // v staging, per head
+  static constexpr int qk = out + 2 * kAiStageOut;              // q, k staging: 8 warps x 2 heads x [32 t][32] fp16
   static constexpr int scale = qk + 8 * 2 * 2048;               // float2 (rstd, rstd or 0 beyond n) per row and slot
-  static constexpr int bars = scale + kTileSlots * 128 * 8;
-  static constexpr int total = bars + (int)sizeof(AiBars);
+  static constexpr int bars = scale + tile_slots(kStages) * 128 * 8;
+  static constexpr int total = bars + (int)sizeof(AiBars<kF16>);
 };
-static_assert(AiLayout::total + 1024 <= 232448, "shared memory budget");
-static_assert(AiLayout::a % 1024 == 0, "tile ring must keep the swizzle alignment");
+static_assert(AiLayout<true>::total + 1024 <= 232448 && AiLayout<false>::total + 1024 <= 232448, "shared memory budget");
+static_assert(AiLayout<true>::a % 1024 == 0, "tile ring must keep the swizzle alignment");
 
 // The resident weights of a CTA (variant: which pair of heads): q carries the softmax scale, the bias rows log2(e).
 template <bool kF16>
 struct AiWeights {
   const float *ln_w, *ln_b;
   const bf16 *q, *k, *v, *bias;
-  static constexpr int kBytes = AiLayout::a;
+  static constexpr int kBytes = AiLayout<kF16>::a;
   __device__ __forceinline__ void fold(unsigned char* sm, int hpair, int warp, int warps, int lane, int tid, int threads) const {
-    unsigned char *w0 = sm + AiLayout::w0, *w1 = sm + AiLayout::w1, *wx0 = sm + AiLayout::wx0, *wx1 = sm + AiLayout::wx1;
+    unsigned char *w0 = sm + AiLayout<kF16>::w0, *w1 = sm + AiLayout<kF16>::w1, *wx0 = sm + AiLayout<kF16>::wx0, *wx1 = sm + AiLayout<kF16>::wx1;
     const float qscale = kLog2e * rsqrtf((float)kAiD);
     fold_weight_rows<kF16, kF16>(w0, wx0, 0, kPanelBytes, q, 64 * hpair, 64, ln_w, ln_b, qscale, warp, warps, lane);
     fold_weight_rows<kF16, kF16>(w0, wx0, 64, kPanelBytes, k, 64 * hpair, 64, ln_w, ln_b, 1.0f, warp, warps, lane);
@@ -75,21 +76,22 @@ struct AiWeights {
 
 // kF16: the rows are the standardised fp16 copy of an fp32 pair tensor (fp16 weights); otherwise bf16 rows of z.
 template <bool kF16>
-__global__ void __launch_bounds__(kAiThreads, 1)
+__global__ void __launch_bounds__(ai_threads(kF16), 1)
 triatt_in_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_constant__ CUtensorMap map_v,
                     const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k, const float* __restrict__ mask,
                     const AiWeights<kF16> weights, const unsigned char* __restrict__ folded,
                     float* __restrict__ bias_out, float* __restrict__ mb_out, int n_u, int n,
                     int ldm, int swap, float eps, float inf, int tiles_t, int n_tiles) {
-  constexpr int kAiAcc = kF16 ? 2 : 1;   // accumulators per product: the products of tile k+1 run beside the epilogue of k
   extern __shared__ __align__(1024) unsigned char smem_raw[];
-  unsigned char* sm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-  AiBars& bars = *reinterpret_cast<AiBars*>(sm + AiLayout::bars);
+  unsigned char* sm = smem_aligned(smem_raw);
+  AiBars<kF16>& bars = *reinterpret_cast<AiBars<kF16>*>(sm + AiLayout<kF16>::bars);
   const int warp = warp_index(), lane = threadIdx.x & 31;
   const int hpair = blockIdx.x & 1;                      // this CTA's heads: 2*hpair, 2*hpair + 1
-  TileCtx ctx;
-  ctx.tiles = sm + AiLayout::a;
-  ctx.extras = sm + AiLayout::ax;
+  typedef TileCtx<ai_stages(kF16), kF16> Ctx;
+  constexpr int kCtl = 16 + tile_stats_warps(kF16);      // first control warp
+  Ctx ctx;
+  ctx.tiles = sm + AiLayout<kF16>::a;
+  ctx.extras = sm + AiLayout<kF16>::ax;
   ctx.bars = &bars.tile;
   ctx.first_tile = blockIdx.x >> 1;
   ctx.tile_step = gridDim.x >> 1;
@@ -110,15 +112,14 @@ triatt_in_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_cons
     }
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
-  if (warp == 20) {
+  if (warp == kCtl) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(&bars.tmem_base)),
                  "r"(512u)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
   }
-  tile_write_ones<kF16>(ctx.tiles, threadIdx.x, kAiThreads);
   asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-  if (!cta_ready(skip, warp == 20, bars.tmem_base, 512u, [&] {
+  if (!cta_ready(skip, warp == kCtl, bars.tmem_base, 512u, [&] {
         if (folded && threadIdx.x == 0)
           folded_load(sm, folded + hpair * AiWeights<kF16>::kBytes, AiWeights<kF16>::kBytes, &bars.w_full);
       }))
@@ -126,25 +127,21 @@ triatt_in_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_cons
   fold_here(weights, folded, sm, hpair, &bars.w_full);
   const uint32_t tmem_base = bars.tmem_base;
 
-  if (warp >= 20) {
-    if (elect_lane()) {
-      if (warp == 20) {
-        tile_producer_loop(ctx, &map_z);
-      } else if (warp == 23) {
-        if (!kF16) tile_gram_loop<kF16>(ctx, tmem_base + kAiColGram);   // standardised rows: nothing to measure
-      } else if (warp == 21) {
-        tile_product_loop(ctx, tmem_base, smem_u32(sm + AiLayout::w0), kPanelBytes, smem_u32(sm + AiLayout::wx0),
-                          umma_idesc_16(128, 128, kF16, kF16), &bars.w_full, bars.acc_full[0], bars.acc_free[0], kAiAcc, 256);
-      } else {
-        tile_product_loop(ctx, tmem_base + 128, smem_u32(sm + AiLayout::w1), kAiW1Panel, smem_u32(sm + AiLayout::wx1),
-                          umma_idesc_16(128, 80, kF16, kF16), &bars.w_full, bars.acc_full[1], bars.acc_free[1], kAiAcc, 256);
-      }
+  if (warp >= kCtl) {
+    if (warp == kCtl) {
+      tile_producer_loop(ctx, &map_z);
+    } else if (warp == kCtl + 1) {
+      tile_product_loop(ctx, tmem_base, smem_u32(sm + AiLayout<kF16>::w0), kPanelBytes, smem_u32(sm + AiLayout<kF16>::wx0),
+                        umma_idesc_16(128, 128, kF16, kF16), &bars.w_full, bars.acc_full[0], bars.acc_free[0], 2, 256);
+    } else {
+      tile_product_loop(ctx, tmem_base + 128, smem_u32(sm + AiLayout<kF16>::w1), kAiW1Panel, smem_u32(sm + AiLayout<kF16>::wx1),
+                        umma_idesc_16(128, 80, kF16, kF16), &bars.w_full, bars.acc_full[1], bars.acc_free[1], 2, 256);
     }
   } else if (warp >= 16) {
     // ------------------------------------------------------------------ row statistics, one thread per row
-    float2* scale = reinterpret_cast<float2*>(sm + AiLayout::scale);
-    tile_stats_loop<kF16>(ctx, eps, tmem_base + kAiColGram, warp - 16, lane, [&](int k, int u, int t, int r, float rstd) {
-      scale[(k % kTileSlots) * 128 + r] = make_float2(rstd, t < n ? rstd : 0.f);
+    float2* scale = reinterpret_cast<float2*>(sm + AiLayout<kF16>::scale);
+    tile_stats_loop(ctx, eps, warp - 16, lane, [&](int k, int u, int t, int r, float rstd) {
+      scale[(k % Ctx::kSlots) * 128 + r] = make_float2(rstd, t < n ? rstd : 0.f);
       if (hpair == 0 && t < ldm) {                       // mask bias, -inf in the pad columns [n, ldm)
         float mv = -CUDART_INF_F;
         if (t < n)
@@ -157,16 +154,16 @@ triatt_in_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_cons
     const int which = warp >> 2, qw = warp & 3;          // 0: q, 1: k
     const int row = 32 * qw + lane;
     const uint32_t t_acc = tmem_base + ((uint32_t)(32 * qw) << 16) + 64 * which;
-    unsigned char* stage = sm + AiLayout::qk + warp * 4096;
+    unsigned char* stage = sm + AiLayout<kF16>::qk + warp * 4096;
     int k = 0;
     for (int tile = ctx.first_tile; tile < n_tiles; tile += ctx.tile_step, ++k) {
       const int u = tile / tiles_t, tw = (tile % tiles_t) * 128 + 32 * qw;   // the warp's first row
-      const int ab = kAiAcc == 2 ? (k & 1) : 0, an = kAiAcc == 2 ? (k >> 1) : k;
+      const int ab = k & 1, an = k >> 1;
       bool ok = mbar_wait(&bars.acc_full[0][ab], an & 1, 32u);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
       tc_fence_after();
-      const float rstd = reinterpret_cast<const float2*>(sm + AiLayout::scale)[(k % kTileSlots) * 128 + row].x;
+      const float rstd = reinterpret_cast<const float2*>(sm + AiLayout<kF16>::scale)[(k % Ctx::kSlots) * 128 + row].x;
       uint32_t h0[32], h1[32];
       tmem_ld32(t_acc + 256 * ab, h0);
       tmem_ld32(t_acc + 256 * ab + 32, h1);
@@ -200,20 +197,21 @@ triatt_in_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_cons
     const int half = (warp >> 2) & 1, qw = warp & 3;
     const int row = 32 * qw + lane;
     const uint32_t t_acc = tmem_base + ((uint32_t)(32 * qw) << 16) + 128 + 32 * half;
-    const bool leader = (threadIdx.x & 255) == 0;
-    unsigned char* stage = sm + AiLayout::out + (32 * half) * 256 + row * 2;
+    const bool leader = (threadIdx.x & 127) == 0;        // of the four warps of a head
     int k = 0;
     bool ok = true;
     for (int tile = ctx.first_tile; tile < n_tiles && ok; tile += ctx.tile_step, ++k) {
       const int u = tile / tiles_t, t0 = (tile % tiles_t) * 128, t = t0 + row;
-      const int ab = kAiAcc == 2 ? (k & 1) : 0, an = kAiAcc == 2 ? (k >> 1) : k;
+      const int ab = k & 1, an = k >> 1;
+      unsigned char* const area = sm + AiLayout<kF16>::out + half * kAiStageOut;
+      unsigned char* const stage = area + row * 2;
       ok = mbar_wait(&bars.acc_full[1][ab], an & 1, 64u);
-      // the store that last read the staging buffer (one tile ago) must be through with it
+      // the store that last read the staging area (one tile ago) must be through with it
       if (leader) tma_store_wait_read<0>();
-      ok = named_barrier_all(1, 256, ok);                  // all eight warps go on, or none
+      ok = named_barrier_all(1 + half, 128, ok);           // all four warps go on, or none
       if (!ok) break;
       tc_fence_after();
-      const float2 sc = reinterpret_cast<const float2*>(sm + AiLayout::scale)[(k % kTileSlots) * 128 + row];
+      const float2 sc = reinterpret_cast<const float2*>(sm + AiLayout<kF16>::scale)[(k % Ctx::kSlots) * 128 + row];
       uint32_t v[32], b[16];
       tmem_ld32(t_acc + 256 * ab, v);
       if (half == 0) tmem_ld16(tmem_base + ((uint32_t)(32 * qw) << 16) + 256 * ab + 128 + 64, b);
@@ -230,9 +228,9 @@ triatt_in_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_cons
           bias_out[((size_t)(2 * hpair + e) * n_u + u) * ldm + t] = sc.y * __uint_as_float(b[e]);
       }
       asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-      named_barrier(1, 256);
+      named_barrier(1 + half, 128);
       if (leader) {
-        tma_store_3d(&map_v, smem_u32(sm + AiLayout::out), t0, u * 128 + 64 * hpair, 0);
+        tma_store_3d(&map_v, smem_u32(area), t0, u * 128 + 64 * hpair + 32 * half, 0);
         tma_store_commit();
       }
     }
@@ -241,7 +239,7 @@ triatt_in_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_cons
 
   tc_fence_before();
   cta_teardown_sync();
-  if (warp == 20) {
+  if (warp == kCtl) {
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem_base), "r"(512u) : "memory");
   }
@@ -261,23 +259,23 @@ static int32_t launch_triatt_in(const void* z, const float* mask, const AiWeight
                          : make_map_3d(&mz, zt, z, 128, (uint64_t)n, (uint64_t)n_u, 256, (uint64_t)n * 256, 64, 128,
                                        CU_TENSOR_MAP_SWIZZLE_128B, 1);
   if (!ok) return PX_ERR_LAUNCH;
-  // v is [n_u * 128 rows (u, head, d)][ldt]: a store writes [64 rows][128 t]
+  // v is [n_u * 128 rows (u, head, d)][ldt]: a store writes [32 rows][128 t]
   const uint64_t ldt = (uint64_t)px_ld(n);
   if (!make_map_3d(&mv, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, v, ldt, (uint64_t)n_u * 128, 1, ldt * 2, ldt * 2 * n_u * 128, 128,
-                   64, CU_TENSOR_MAP_SWIZZLE_NONE, 1))
+                   32, CU_TENSOR_MAP_SWIZZLE_NONE, 1))
     return PX_ERR_LAUNCH;
   // q, k: [n_u * 4][n][32], a store writes [32 t][32]
   for (int i = 0; i < 2; ++i)
     if (!make_map_3d(i ? &mk : &mq, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, i ? k : q, kAiD, (uint64_t)n, (uint64_t)n_u * kAiH, kAiD * 2,
                      (uint64_t)n * kAiD * 2, kAiD, 32, CU_TENSOR_MAP_SWIZZLE_64B))
       return PX_ERR_LAUNCH;
-  const size_t smem = AiLayout::total + 1024;
+  const size_t smem = AiLayout<kF16>::total + 1024;
   static SmemLimit limit;
   if (!limit.set(triatt_in_tc_kernel<kF16>, smem)) return PX_ERR_LAUNCH;
   const int64_t tiles_t = (n + 127) / 128, n_tiles = tiles_t * n_u;   // 128-wide tiles cover the pad columns up to ldm
   if (n_tiles > 0x7fffffff) return PX_ERR_UNSUPPORTED;
   const int pairs = (int)(n_tiles < sm_count() / 2 ? n_tiles : sm_count() / 2);
-  return launch_pdl(triatt_in_tc_kernel<kF16>, dim3(2 * pairs), kAiThreads, smem, st, mz, mv, mq, mk, mask, weights,
+  return launch_pdl(triatt_in_tc_kernel<kF16>, dim3(2 * pairs), ai_threads(kF16), smem, st, mz, mv, mq, mk, mask, weights,
                     (const unsigned char*)folded, bias, mask_bias, (int)n_u, (int)n, (int)ldm, (int)ending, eps, inf, (int)tiles_t,
                     (int)n_tiles)
              ? PX_OK

@@ -9,7 +9,7 @@
 // live, so that 16-bit tensors cross NVLink in both directions).
 //
 // Persistent kernel, one CTA per SM, on the row-tile pipeline of px_rowpipe.cuh (TMA-fed raw rows, LayerNorm folded
-// into the resident gate weights plus one correction K step, row statistics from a tensor-core Gram product).  A
+// into the resident gate weights plus one correction K step).  A
 // stage of the ring holds the z tile and the o tile of 128 pair elements.  Both products of a tile run on the
 // tensor core; the gated rows go from registers back into tensor memory as the A operand of the second product and
 // never touch shared memory.
@@ -19,11 +19,11 @@
 //   warps 8..15   output: accumulator + residual (the raw z tile still in shared memory), packed to bf16 over the
 //                 o tile in place, which then leaves through a TMA store; the store addresses z[u][t] or z[t][u],
 //                 so the ending node costs nothing extra.  fp32 rows by form.
-//   warps 16..19  one thread per row: statistics, correction row, the row's rstd.
-//   warp 20       TMA producer (z and o tiles); warp 21 MMA issuer of the gate product, warp 22 of the output
-//                 product (A operand in tensor memory), warp 23 of the statistics product.
-// Tensor memory: gate accumulator (128) | gated rows, two fp16 per column (64) | output accumulator (128) |
-// statistics (144).  Algorithmic HBM traffic per pair element: 256 + 128*sizeof(Tz) read, 128*sizeof(Tz) written.
+//   warps 16..19  (bf16 rows 16..23) statistics, correction row, the row's rstd.
+//   then          a TMA producer (z and o tiles), the MMA issuer of the gate product and that of the output
+//                 product (A operand in tensor memory).
+// Tensor memory: gate accumulator (128) | gated rows, two fp16 per column (64) | output accumulator (128).
+// Algorithmic HBM traffic per pair element: 256 + 128*sizeof(Tz) read, 128*sizeof(Tz) written.
 // Every mbarrier wait is bounded.
 #include <cstring>
 
@@ -31,12 +31,12 @@
 
 namespace px {
 
-constexpr int kAoWarps = 24;
-constexpr int kAoThreads = 32 * kAoWarps;
-constexpr uint32_t kAoColG = 0, kAoColA2 = 128, kAoColOut = 192, kAoColGram = 320;
+constexpr int kAoStages = 2;
+constexpr int ao_threads(bool f16) { return 32 * (16 + tile_stats_warps(f16) + 3); }
+constexpr uint32_t kAoColG = 0, kAoColA2 = 128, kAoColOut = 192;
 
 struct AoBars {
-  TileBars tile;
+  TileBars<kAoStages> tile;
   uint64_t g_full, g_free, a2_ready, a2_free, out_full, out_free, w_full;
   uint32_t tmem_base;
 };
@@ -45,10 +45,10 @@ struct AoLayout {
   static constexpr int wo = wg + kOperandBytes;                 // output weights
   static constexpr int wx = wo + kOperandBytes;                 // gate correction panel
   static constexpr int a = wx + 128 * 32;                       // z tiles
-  static constexpr int ax = a + kTileStages * kTileBytes;       // z correction panels
-  static constexpr int o = ax + kTileSlots * kTileExtra;        // o tiles (later the output rows)
-  static constexpr int scale = o + kTileStages * kOperandBytes; // rstd per row and slot
-  static constexpr int bars = scale + kTileSlots * 128 * 4;
+  static constexpr int ax = a + kAoStages * kTileBytes;       // z correction panels
+  static constexpr int o = ax + tile_slots(kAoStages) * kTileExtra;        // o tiles (later the output rows)
+  static constexpr int scale = o + kAoStages * kOperandBytes; // rstd per row and slot
+  static constexpr int bars = scale + tile_slots(kAoStages) * 128 * 4;
   static constexpr int total = bars + (int)sizeof(AoBars);
 };
 static_assert(AoLayout::total + 1024 <= 232448, "shared memory budget");
@@ -68,7 +68,7 @@ struct AoWeights {
 };
 
 template <int kMode>
-__global__ void __launch_bounds__(kAoThreads, 1)
+__global__ void __launch_bounds__(ao_threads(kMode != 0), 1)
 triatt_out_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_constant__ CUtensorMap map_o,
                      const __grid_constant__ CUtensorMap map_out, const void* __restrict__ z_in, void* __restrict__ z_out,
                      const AoWeights<kMode != 0> weights, const unsigned char* __restrict__ folded, int n_u, int n, int swap, int add_residual, float eps, int tiles_t,
@@ -77,10 +77,12 @@ triatt_out_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_con
   constexpr bool kBulk = kMode == 3;                     // fp32 output: staged, stored or added by TMA
   constexpr bool kF16 = kMode != 0;                      // the z tile is a standardised fp16 copy; o, W_o always fp16
   extern __shared__ __align__(1024) unsigned char smem_raw[];
-  unsigned char* sm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  unsigned char* sm = smem_aligned(smem_raw);
   AoBars& bars = *reinterpret_cast<AoBars*>(sm + AoLayout::bars);
   const int warp = warp_index(), lane = threadIdx.x & 31;
-  TileCtx ctx;
+  typedef TileCtx<kAoStages, kF16> Ctx;
+  constexpr int kCtl = 16 + tile_stats_warps(kF16);      // first control warp
+  Ctx ctx;
   ctx.tiles = sm + AoLayout::a;
   ctx.extras = sm + AoLayout::ax;
   ctx.bars = &bars.tile;
@@ -98,7 +100,7 @@ triatt_out_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_con
     if (kTma || kBulk) prefetch_maps(map_out);
   }
   if (threadIdx.x == 0) {
-    // a stage is read by the statistics product, the gate product and the output warps
+    // a stage is read by the gate product and the output warps
     tile_bars_init(bars.tile, 2, kF16);
     mbar_init(&bars.w_full, 1);
     mbar_init(&bars.g_full, 1);
@@ -109,51 +111,51 @@ triatt_out_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_con
     mbar_init(&bars.out_free, 8);
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
-  if (warp == 20) {
+  if (warp == kCtl) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(&bars.tmem_base)),
                  "r"(512u)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
   }
-  tile_write_ones<kF16>(ctx.tiles, threadIdx.x, kAoThreads);
   asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-  if (!cta_ready(skip, warp == 20, bars.tmem_base, 512u, [&] {
+  if (!cta_ready(skip, warp == kCtl, bars.tmem_base, 512u, [&] {
         if (folded && threadIdx.x == 0) folded_load(sm, folded, AoWeights<kF16>::kBytes, &bars.w_full);
       }))
     return;
   fold_here(weights, folded, sm, 0, &bars.w_full);
   const uint32_t tmem_base = bars.tmem_base;
 
-  if (warp >= 20) {
-    if (elect_lane()) {
-      if (warp == 20) {
-        // ---------------------------------------------------------------- tile producer: z (bf16 rows) and o
-        int k = 0;
-        for (int tile = ctx.first_tile; tile < n_tiles; tile += ctx.tile_step, ++k) {
-          const int s = k % kTileStages, m = k / kTileStages;
-          if (!mbar_wait(&bars.tile.a_empty[s], (m & 1) ^ 1, 1u)) break;
+  if (warp >= kCtl) {
+    if (warp == kCtl) {
+      // ---------------------------------------------------------------- tile producer: z (bf16 rows) and o
+      int k = 0;
+      for (int tile = ctx.first_tile; tile < n_tiles; tile += ctx.tile_step, ++k) {
+        const int s = k % kAoStages, m = k / kAoStages;
+        if (!mbar_wait_warp(&bars.tile.a_empty[s], (m & 1) ^ 1, 1u)) break;
+        if (elect_lane()) {
           const int u = tile / tiles_t, t0 = (tile % tiles_t) * 128;
           mbar_expect_tx(&bars.tile.raw_full[s], 2 * kOperandBytes);
           const uint32_t zdst = smem_u32(ctx.tiles + s * kTileBytes), odst = smem_u32(sm + AoLayout::o + s * kOperandBytes);
           for (int p = 0; p < 2; ++p) {
-            tma_load_3d(zdst + p * kTilePanel, &map_z, &bars.tile.raw_full[s], 64 * p, swap ? u : t0, swap ? t0 : u);
+            tma_load_3d(zdst + p * kPanelBytes, &map_z, &bars.tile.raw_full[s], 64 * p, swap ? u : t0, swap ? t0 : u);
             tma_load_3d(odst + p * kPanelBytes, &map_o, &bars.tile.raw_full[s], 64 * p, t0, u);
           }
         }
-      } else if (warp == 23) {
-        if (!kF16) tile_gram_loop<kF16>(ctx, tmem_base + kAoColGram);   // standardised rows: nothing to measure
-      } else if (warp == 21) {
-        tile_product_loop(ctx, tmem_base + kAoColG, smem_u32(sm + AoLayout::wg), kPanelBytes, smem_u32(sm + AoLayout::wx),
-                          umma_idesc_16(128, 128, kF16, kF16), &bars.w_full, &bars.g_full, &bars.g_free);
-      } else {
-        // ---------------------------------------------------------------- output product, A operand in tensor memory
-        constexpr uint32_t idesc = umma_idesc_f16(128, 128);
-        const uint32_t wo_addr = smem_u32(sm + AoLayout::wo);
-        int k = 0;
-        const bool have_w = mbar_wait(&bars.w_full, 0, 4u);      // the resident weights
-        for (int tile = ctx.first_tile; tile < n_tiles && have_w; tile += ctx.tile_step, ++k) {
-          if (!mbar_wait(&bars.a2_ready, k & 1, 4u) || !mbar_wait(&bars.out_free, (k & 1) ^ 1, 8u)) break;
-          tc_fence_after();
+        __syncwarp();
+      }
+    } else if (warp == kCtl + 1) {
+      tile_product_loop(ctx, tmem_base + kAoColG, smem_u32(sm + AoLayout::wg), kPanelBytes, smem_u32(sm + AoLayout::wx),
+                        umma_idesc_16(128, 128, kF16, kF16), &bars.w_full, &bars.g_full, &bars.g_free);
+    } else {
+      // ---------------------------------------------------------------- output product, A operand in tensor memory
+      constexpr uint32_t idesc = umma_idesc_f16(128, 128);
+      const uint32_t wo_addr = smem_u32(sm + AoLayout::wo);
+      int k = 0;
+      const bool have_w = mbar_wait_warp(&bars.w_full, 0, 4u);   // the resident weights
+      for (int tile = ctx.first_tile; tile < n_tiles && have_w; tile += ctx.tile_step, ++k) {
+        if (!mbar_wait_warp(&bars.a2_ready, k & 1, 4u) || !mbar_wait_warp(&bars.out_free, (k & 1) ^ 1, 8u)) break;
+        tc_fence_after();
+        if (elect_lane()) {
 #pragma unroll
           for (int ks = 0; ks < 8; ++ks)
             umma_bf16_ts(tmem_base + kAoColOut, tmem_base + kAoColA2 + 8 * ks,
@@ -161,13 +163,14 @@ triatt_out_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_con
           umma_commit(&bars.out_full);
           umma_commit(&bars.a2_free);
         }
+        __syncwarp();
       }
     }
   } else if (warp >= 16) {
     // ------------------------------------------------------------------ row statistics, one thread per row
     float* scale = reinterpret_cast<float*>(sm + AoLayout::scale);
-    tile_stats_loop<kF16>(ctx, eps, tmem_base + kAoColGram, warp - 16, lane,
-                        [&](int k, int u, int t, int r, float rstd) { scale[(k % kTileSlots) * 128 + r] = rstd; });
+    tile_stats_loop(ctx, eps, warp - 16, lane,
+                        [&](int k, int u, int t, int r, float rstd) { scale[(k % Ctx::kSlots) * 128 + r] = rstd; });
   } else if (warp < 8) {
     // ------------------------------------------------------------------ gate: o * sigmoid(g) -> tensor memory
     const int half = warp >> 2, qw = warp & 3;
@@ -175,12 +178,12 @@ triatt_out_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_con
     const uint32_t lane_addr = tmem_base + ((uint32_t)(32 * qw) << 16);
     int k = 0;
     for (int tile = ctx.first_tile; tile < n_tiles; tile += ctx.tile_step, ++k) {
-      const int s = k % kTileStages;
+      const int s = k % kAoStages;
       bool ok = mbar_wait(&bars.g_full, k & 1, 32u) && mbar_wait(&bars.a2_free, (k & 1) ^ 1, 32u);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
       tc_fence_after();
-      const float rstd = reinterpret_cast<const float*>(sm + AoLayout::scale)[(k % kTileSlots) * 128 + row];
+      const float rstd = reinterpret_cast<const float*>(sm + AoLayout::scale)[(k % Ctx::kSlots) * 128 + row];
       const unsigned char* otile = sm + AoLayout::o + s * kOperandBytes;
       uint32_t packed[32];
 #pragma unroll
@@ -221,7 +224,7 @@ triatt_out_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_con
     int k = 0;
     bool ok = true;
     for (int tile = ctx.first_tile; tile < n_tiles && ok; tile += ctx.tile_step, ++k) {
-      const int s = k % kTileStages;
+      const int s = k % kAoStages;
       const int u = tile / tiles_t, t0 = (tile % tiles_t) * 128;
       // fp32 rows: this warp's 32 rows (u, t0 + 32 qw + i) in units of 128-channel rows of z, and their residual
       // values for the first 32 channels, requested before the wait (the second block's lines are asked of L2)
@@ -268,7 +271,7 @@ triatt_out_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_con
             const int piece = 8 * half + 4 * hh + j;
             uint32_t w[4];
             if (add_residual) {
-              const uint4 zv = *reinterpret_cast<const uint4*>(ztile + operand_piece_offset(row, piece, kTilePanel));
+              const uint4 zv = *reinterpret_cast<const uint4*>(ztile + operand_piece_offset(row, piece, kPanelBytes));
               const uint32_t zw[4] = {zv.x, zv.y, zv.z, zv.w};
 #pragma unroll
               for (int e = 0; e < 4; ++e) {
@@ -283,12 +286,12 @@ triatt_out_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_con
             *reinterpret_cast<uint4*>(otile + operand_piece_offset(row, piece)) = make_uint4(w[0], w[1], w[2], w[3]);
           }
         } else if (kBulk) {
-          // fp32 rows: the first block staged in the o tile, the second in the z tile (not its rows of ones), which the gate
+          // fp32 rows: the first block staged in the o tile, the second in the z tile, which the gate
           // warps and the tensor core have finished reading (8 warps x 4 KB each)
           float v[32];
 #pragma unroll
           for (int e = 0; e < 32; ++e) v[e] = __uint_as_float(acc[e]);
-          unsigned char* stg = hh == 0 ? otile + (warp & 7) * 4096 : ctx.tiles + s * kTileBytes + half * kTilePanel + qw * 4096;
+          unsigned char* stg = hh == 0 ? otile + (warp & 7) * 4096 : ctx.tiles + s * kTileBytes + half * kPanelBytes + qw * 4096;
           const int tw = t0 + 32 * qw;
           rows_bulk_out(stg, v, &map_out, add_residual != 0, 64 * half + 32 * hh, swap ? u : tw, swap ? tw : u, tw < n, lane);
         } else {
@@ -325,7 +328,7 @@ triatt_out_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_con
 
   tc_fence_before();
   cta_teardown_sync();
-  if (warp == 20) {
+  if (warp == kCtl) {
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem_base), "r"(512u) : "memory");
   }
@@ -371,7 +374,7 @@ static int32_t launch_triatt_out(const px_f16* o, const void* z_in, const px_f16
   const int64_t tiles_t = (n + 127) / 128, n_tiles = tiles_t * n_u;
   if (n_tiles > 0x7fffffff) return PX_ERR_UNSUPPORTED;
   const int grid = (int)(n_tiles < sm_count() ? n_tiles : sm_count());
-  return launch_pdl(triatt_out_tc_kernel<kMode>, dim3(grid), kAoThreads, smem, st, mz, mo, mout, z_in, z_out, weights,
+  return launch_pdl(triatt_out_tc_kernel<kMode>, dim3(grid), ao_threads(kMode != 0), smem, st, mz, mo, mout, z_in, z_out, weights,
                     (const unsigned char*)folded, (int)n_u, (int)n, (int)ending, (int)add_residual, eps, (int)tiles_t, (int)n_tiles)
              ? PX_OK
              : PX_ERR_LAUNCH;

@@ -5,38 +5,32 @@
 //
 // Persistent kernel, one CTA per SM.  A tile is 128 pair elements (one u, 128 consecutive t); the CTAs work in
 // pairs on the same sequence of tiles, each CTA producing 64 of the 128 channels of a and of b (the second read of
-// a tile comes from L2).  Halving the weights a CTA keeps resident leaves shared memory for output staging and
-// tensor memory for the row statistics (px_rowpipe.cuh has the parts shared with the other row kernels):
+// a tile comes from L2).  Halving the weights a CTA keeps resident leaves shared memory for output staging
+// (px_rowpipe.cuh has the parts shared with the other row kernels):
 //   * The weights stay in shared memory for the whole kernel with gamma and the 1/2 of the sigmoid folded in;
 //     LayerNorm's mean and beta terms enter the product as one extra K step (see px_rowpipe.cuh).
-//   * The row statistics come from the tensor core as well: Z Z^T has the sums of squares on its diagonal, and 16
-//     rows of ones kept behind every tile in shared memory add the plain sums as columns 128..143 of that product.
-//     Variance = E[x^2] - mean^2 in fp32: accurate while |mean| is not orders of magnitude above the deviation.
 //   * The gated outputs are staged as [channel][t] in shared memory (two-byte stores, conflict-free) and leave
-//     through TMA stores, 256-byte runs per channel.
+//     through TMA stores, 256-byte runs per channel.  Four warps share a staging area of 32 channels.
 //
 //   warps 0..7    epilogue of output a: a thread owns one pair element (accumulator lane) and 32 of the CTA's 64
 //                 channels; warps 8..15 do the same for output b, concurrently.
-//   warps 16..19  one thread per row: reads the two statistics out of tensor memory, writes the correction row and
-//                 the row's scale pair.
-//   warp 20       TMA producer of the row tiles (bf16 rows of z, or standardised fp16 rows), two-stage ring.
-//   warps 21..23  MMA issuers (a tcgen05.mma costs its issuing thread 100 cycles and more, so the work is split):
-//                 warp 21 output a, warp 22 output b, each 8 MMAs M=128 (t) N=128 (projection | gate) K=16 plus the
-//                 correction step; warp 23 the statistics product (8 MMAs, N=144).
+//   warps 16..19  (bf16 rows 16..23) statistics, correction row, the row's scale pair.
+//   then          a TMA producer of the row tiles (bf16 rows of z, or standardised fp16 rows), three-stage ring, and
+//                 the MMA issuers of outputs a and b, each 8 MMAs M=128 (t) N=128 (projection | gate) K=16 plus the
+//                 correction step, into two accumulators in turn.
 // Algorithmic HBM traffic per pair element: 256 + 4 read, 512 written.  Every mbarrier wait is bounded.
 #include "px_rowpipe.cuh"
 
 namespace px {
 
+constexpr int kTiStages = 3;
 constexpr int kTiWExtra = 128 * 32;            // [128 rows][16 k] weight-side correction panel
-constexpr int kTiStageOut = 64 * 256;          // [64 channels][128 t] fp16
-constexpr int kTiWarps = 24;
-constexpr int kTiThreads = 32 * kTiWarps;
-constexpr uint32_t kTiColGram = 256;           // tensor memory: out a | out b | statistics (144 columns); standardised
-                                               // rows need no statistics product: a second pair of accumulators there
+constexpr int kTiStageOut = 32 * 256;          // [32 channels][128 t] fp16
+constexpr int ti_threads(bool f16) { return 32 * (16 + tile_stats_warps(f16) + 3); }
+// tensor memory: out a | out b, twice
 
 struct TiBars {
-  TileBars tile;
+  TileBars<kTiStages> tile;
   uint64_t acc_full[2][2], acc_free[2][2];   // [output][accumulator]
   uint64_t w_full;
   uint32_t tmem_base;
@@ -45,10 +39,10 @@ struct TiLayout {
   static constexpr int w = 0;                                   // per output: [projection 64 | gate 64][128 k]
   static constexpr int wx = w + 2 * kOperandBytes;              // per output: correction panel
   static constexpr int a = wx + 2 * kTiWExtra;                  // row-tile ring
-  static constexpr int ax = a + kTileStages * kTileBytes;       // row-tile correction panels
-  static constexpr int out = ax + kTileSlots * kTileExtra;      // output staging, one buffer per output
-  static constexpr int scale = out + 2 * kTiStageOut;           // float2 (rstd, rstd*mask/2) per row and slot
-  static constexpr int bars = scale + kTileSlots * 128 * 8;
+  static constexpr int ax = a + kTiStages * kTileBytes;       // row-tile correction panels
+  static constexpr int out = ax + tile_slots(kTiStages) * kTileExtra;   // output staging, per output and half of its channels
+  static constexpr int scale = out + 4 * kTiStageOut;           // float2 (rstd, rstd*mask/2) per row and slot
+  static constexpr int bars = scale + tile_slots(kTiStages) * 128 * 8;
   static constexpr int total = bars + (int)sizeof(TiBars);
 };
 static_assert(TiLayout::total + 1024 <= 232448, "shared memory budget");
@@ -72,17 +66,18 @@ struct TiWeights {
 
 // kF16: the rows are the standardised fp16 copy of an fp32 pair tensor (fp16 weights); otherwise bf16 rows of z.
 template <bool kF16>
-__global__ void __launch_bounds__(kTiThreads, 1)
+__global__ void __launch_bounds__(ti_threads(kF16), 1)
 trimul_in_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_constant__ CUtensorMap map_a,
                     const __grid_constant__ CUtensorMap map_b, const float* __restrict__ mask,
                     const TiWeights<kF16> weights, const unsigned char* __restrict__ folded, int n_u, int n_t, int swap, float eps, int tiles_t, int n_tiles) {
-  constexpr int kTiAcc = kF16 ? 2 : 1;   // accumulators per output: the products of tile k+1 run beside the epilogue of k
   extern __shared__ __align__(1024) unsigned char smem_raw[];
-  unsigned char* sm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  unsigned char* sm = smem_aligned(smem_raw);
   TiBars& bars = *reinterpret_cast<TiBars*>(sm + TiLayout::bars);
   const int warp = warp_index(), lane = threadIdx.x & 31;
+  constexpr int kCtl = 16 + tile_stats_warps(kF16);      // first control warp
   const int chan0 = 64 * (blockIdx.x & 1);               // this CTA's channels of a and b
-  TileCtx ctx;
+  typedef TileCtx<kTiStages, kF16> Ctx;
+  Ctx ctx;
   ctx.tiles = sm + TiLayout::a;
   ctx.extras = sm + TiLayout::ax;
   ctx.bars = &bars.tile;
@@ -105,15 +100,14 @@ trimul_in_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_cons
     }
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
-  if (warp == 20) {
+  if (warp == kCtl) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(&bars.tmem_base)),
                  "r"(512u)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
   }
-  tile_write_ones<kF16>(ctx.tiles, threadIdx.x, kTiThreads);
   asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-  if (!cta_ready(skip, warp == 20, bars.tmem_base, 512u, [&] {
+  if (!cta_ready(skip, warp == kCtl, bars.tmem_base, 512u, [&] {
         if (folded && threadIdx.x == 0)
           folded_load(sm, folded + (blockIdx.x & 1) * TiWeights<kF16>::kBytes, TiWeights<kF16>::kBytes, &bars.w_full);
       }))
@@ -121,48 +115,46 @@ trimul_in_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_cons
   fold_here(weights, folded, sm, blockIdx.x & 1, &bars.w_full);
   const uint32_t tmem_base = bars.tmem_base;
 
-  if (warp >= 20) {
-    if (elect_lane()) {
-      if (warp == 20) {
-        tile_producer_loop(ctx, &map_z);
-      } else if (warp == 23) {
-        if (!kF16) tile_gram_loop<kF16>(ctx, tmem_base + kTiColGram);   // standardised rows: nothing to measure
-      } else {
-        const int ph = warp - 21;                          // MMA issuer of output ph
-        tile_product_loop(ctx, tmem_base + 128 * ph, smem_u32(sm + TiLayout::w) + ph * kOperandBytes, kPanelBytes,
-                          smem_u32(sm + TiLayout::wx) + ph * kTiWExtra, umma_idesc_16(128, 128, kF16, kF16), &bars.w_full, bars.acc_full[ph],
-                          bars.acc_free[ph], kTiAcc, 256);
-      }
+  if (warp >= kCtl) {
+    if (warp == kCtl) {
+      tile_producer_loop(ctx, &map_z);
+    } else {
+      const int ph = warp - kCtl - 1;                            // MMA issuer of output ph
+      tile_product_loop(ctx, tmem_base + 128 * ph, smem_u32(sm + TiLayout::w) + ph * kOperandBytes, kPanelBytes,
+                        smem_u32(sm + TiLayout::wx) + ph * kTiWExtra, umma_idesc_16(128, 128, kF16, kF16), &bars.w_full, bars.acc_full[ph],
+                        bars.acc_free[ph], 2, 256);
     }
   } else if (warp >= 16) {
     // ------------------------------------------------------------------ row statistics, one thread per row
     float2* scale = reinterpret_cast<float2*>(sm + TiLayout::scale);
-    tile_stats_loop<kF16>(ctx, eps, tmem_base + kTiColGram, warp - 16, lane, [&](int k, int u, int t, int r, float rstd) {
+    tile_stats_loop(ctx, eps, warp - 16, lane, [&](int k, int u, int t, int r, float rstd) {
       float mk = 0.f;
       if (t < n_t) mk = mask ? __ldg(mask + (swap ? ((size_t)t * n_u + u) : ((size_t)u * n_t + t))) : 1.f;
-      scale[(k % kTileSlots) * 128 + r] = make_float2(rstd, 0.5f * rstd * mk);
+      scale[(k % Ctx::kSlots) * 128 + r] = make_float2(rstd, 0.5f * rstd * mk);
     });
   } else {
     // ------------------------------------------------------------------ epilogue of output ph
     const int ph = warp >> 3, half = (warp >> 2) & 1, qw = warp & 3;
     const int row = 32 * qw + lane;                      // this thread's pair element = accumulator lane
     const uint32_t t_acc = tmem_base + ((uint32_t)(32 * qw) << 16) + 128 * ph + 32 * half;
-    const bool leader = (threadIdx.x & 255) == 0;
+    const int group = 2 * ph + half;                     // four warps that share a staging area
+    const bool leader = (threadIdx.x & 127) == 0;
     const CUtensorMap* map_out = ph ? &map_b : &map_a;
-    unsigned char* stage = sm + TiLayout::out + ph * kTiStageOut + (32 * half) * 256 + row * 2;
     int k = 0;
     bool ok = true;
     for (int tile = ctx.first_tile; tile < n_tiles && ok; tile += ctx.tile_step, ++k) {
       const int u = tile / tiles_t, t0 = (tile % tiles_t) * 128;
-      const int ab = kTiAcc == 2 ? (k & 1) : 0, an = kTiAcc == 2 ? (k >> 1) : k;
+      const int ab = k & 1;
       const uint32_t t_buf = t_acc + 256 * ab;
-      ok = mbar_wait(&bars.acc_full[ph][ab], an & 1, 32u);
-      // the store that last read the staging buffer (one tile ago) must be through with it
+      unsigned char* const area = sm + TiLayout::out + group * kTiStageOut;
+      unsigned char* const stage = area + row * 2;
+      ok = mbar_wait(&bars.acc_full[ph][ab], (k >> 1) & 1, 32u);
+      // the store that last read the staging area (one tile ago) must be through with it
       if (leader) tma_store_wait_read<0>();
-      ok = named_barrier_all(1 + ph, 256, ok);             // all eight warps go on, or none
+      ok = named_barrier_all(1 + group, 128, ok);          // all four warps go on, or none
       if (!ok) break;
       tc_fence_after();
-      const float2 sc = reinterpret_cast<const float2*>(sm + TiLayout::scale)[(k % kTileSlots) * 128 + row];
+      const float2 sc = reinterpret_cast<const float2*>(sm + TiLayout::scale)[(k % Ctx::kSlots) * 128 + row];
       // mask * p * sigmoid(g) = h + h * tanh(g / 2) with h = mask * p / 2 (the halves are folded in)
       auto emit = [&](const uint32_t(&p)[16], const uint32_t(&g)[16], int hh) {
 #pragma unroll
@@ -184,9 +176,9 @@ trimul_in_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_cons
       emit(p0, g0, 0);
       emit(p1, g1, 1);
       asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-      named_barrier(1 + ph, 256);
+      named_barrier(1 + group, 128);
       if (leader) {
-        tma_store_3d(map_out, smem_u32(sm + TiLayout::out + ph * kTiStageOut), t0, u, chan0);
+        tma_store_3d(map_out, smem_u32(area), t0, u, chan0 + 32 * half);
         tma_store_commit();
       }
     }
@@ -195,7 +187,7 @@ trimul_in_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_cons
 
   tc_fence_before();
   cta_teardown_sync();
-  if (warp == 20) {
+  if (warp == kCtl) {
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem_base), "r"(512u) : "memory");
   }
@@ -214,11 +206,11 @@ static int32_t launch_trimul_in(const void* z, const float* mask, const TiWeight
                            : make_map_3d(&mz, zt, z, 128, (uint64_t)n_t, (uint64_t)n_u, 256, (uint64_t)n_t * 256, 64, 128,
                                          CU_TENSOR_MAP_SWIZZLE_128B, 1);
   if (!ok) return PX_ERR_LAUNCH;
-  // outputs [128 channels][n_u][ld]: a store writes [64 channels][one u][128 t]
+  // outputs [128 channels][n_u][ld]: a store writes [32 channels][one u][128 t]
   if (!make_map_3d(&ma, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, a, (uint64_t)ld, (uint64_t)n_u, 128, (uint64_t)ld * 2,
-                   (uint64_t)n_u * ld * 2, 128, 1, CU_TENSOR_MAP_SWIZZLE_NONE, 64) ||
+                   (uint64_t)n_u * ld * 2, 128, 1, CU_TENSOR_MAP_SWIZZLE_NONE, 32) ||
       !make_map_3d(&mb, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, b, (uint64_t)ld, (uint64_t)n_u, 128, (uint64_t)ld * 2,
-                   (uint64_t)n_u * ld * 2, 128, 1, CU_TENSOR_MAP_SWIZZLE_NONE, 64))
+                   (uint64_t)n_u * ld * 2, 128, 1, CU_TENSOR_MAP_SWIZZLE_NONE, 32))
     return PX_ERR_LAUNCH;
   const size_t smem = TiLayout::total + 1024;
   static SmemLimit limit;
@@ -226,7 +218,7 @@ static int32_t launch_trimul_in(const void* z, const float* mask, const TiWeight
   const int64_t tiles_t = (ld + 127) / 128, n_tiles = tiles_t * n_u;
   if (n_tiles > 0x7fffffff) return PX_ERR_UNSUPPORTED;
   const int pairs = (int)(n_tiles < sm_count() / 2 ? n_tiles : sm_count() / 2);
-  return launch_pdl(trimul_in_tc_kernel<kF16>, dim3(2 * pairs), kTiThreads, smem, st, mz, ma, mb, mask, weights,
+  return launch_pdl(trimul_in_tc_kernel<kF16>, dim3(2 * pairs), ti_threads(kF16), smem, st, mz, ma, mb, mask, weights,
                     (const unsigned char*)folded, (int)n_u, (int)n_t, (int)incoming, eps, (int)tiles_t, (int)n_tiles)
              ? PX_OK
              : PX_ERR_LAUNCH;
