@@ -131,13 +131,13 @@ trimul_out_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_con
   const int first_tile = blockIdx.x, tile_step = gridDim.x;
 
   if (warp >= 20) {
-    if (elect_lane()) {
-      if (warp == 20) {
-        // ---------------------------------------------------------------- tile producer: z (bf16 rows) and x
-        int k = 0;
-        for (int tile = first_tile; tile < n_tiles; tile += tile_step, ++k) {
-          const int s = k % kToStages, m = k / kToStages;
-          if (!mbar_wait(&bars.a_empty[s], (m & 1) ^ 1, 1u)) break;
+    if (warp == 20) {
+      // ---------------------------------------------------------------- tile producer: z (bf16 rows) and x
+      int k = 0;
+      for (int tile = first_tile; tile < n_tiles; tile += tile_step, ++k) {
+        const int s = k % kToStages, m = k / kToStages;
+        if (!mbar_wait_warp(&bars.a_empty[s], (m & 1) ^ 1, 1u)) break;
+        if (elect_lane()) {
           const int i = tile / tiles_j, j0 = (tile % tiles_j) * 128;
           mbar_expect_tx(&bars.raw_full[s], 2 * kOperandBytes);
           const uint32_t zdst = smem_u32(sm + ToLayout::zt + s * kOperandBytes), xdst = smem_u32(sm + ToLayout::xt + s * kOperandBytes);
@@ -145,28 +145,45 @@ trimul_out_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_con
             tma_load_3d(zdst + p * kPanelBytes, &map_z, &bars.raw_full[s], 64 * p, j0, i);
             tma_load_3d(xdst + p * kPanelBytes, &map_x, &bars.raw_full[s], j0 + 64 * p, i, 0);
           }
+          // The tile that takes this stage next is asked of L2 (a stage is held until its rows have left, so only two tiles are on
+          // their way): bf16 N = 768 122 -> 107 us, fp32 without a residual N = 1024 230 -> 203.  Not where rows are added in L2,
+          // which is then what is waited for: 552 -> 610 at N = 1536, 140 -> 151 at N = 768.
+          const int next = tile + 2 * tile_step;
+          if ((kTma || (kBulk && !add_residual)) && next < n_tiles) {
+            const int i2 = next / tiles_j, j2 = (next % tiles_j) * 128;
+            for (int p = 0; p < 2; ++p) {
+              tma_prefetch_3d(&map_z, 64 * p, j2, i2);
+              tma_prefetch_3d(&map_x, j2 + 64 * p, i2, 0);
+            }
+          }
         }
-      } else if (warp == 23) {
-        // ---------------------------------------------------------------- statistics products: Z Z^T, then X^T X
-        constexpr uint32_t idesc_z = umma_idesc_16(128, 128, kF16, kF16), idesc_x = umma_idesc_f16(128, 128, true, true);
-        int k = 0;
-        for (int tile = first_tile; tile < n_tiles; tile += tile_step, ++k) {
-          const int s = k % kToStages, m = k / kToStages;
-          // bf16 rows: two phases of the statistics accumulator per tile (z, then x); standardised rows have known
-          // statistics, so only x is measured and the phases alternate from tile to tile
-          if (!mbar_wait(&bars.raw_full[s], m & 1, 2u) || !mbar_wait(&bars.gram_free, kF16 ? ((k & 1) ^ 1) : 1u, 2u)) break;
-          tc_fence_after();
-          const uint32_t z_addr = smem_u32(sm + ToLayout::zt + s * kOperandBytes), x_addr = smem_u32(sm + ToLayout::xt + s * kOperandBytes);
-          if (!kF16) {
+        __syncwarp();
+      }
+    } else if (warp == 23) {
+      // ---------------------------------------------------------------- statistics products: Z Z^T, then X^T X
+      constexpr uint32_t idesc_z = umma_idesc_16(128, 128, kF16, kF16), idesc_x = umma_idesc_f16(128, 128, true, true);
+      int k = 0;
+      for (int tile = first_tile; tile < n_tiles; tile += tile_step, ++k) {
+        const int s = k % kToStages, m = k / kToStages;
+        // bf16 rows: two phases of the statistics accumulator per tile (z, then x); standardised rows have known
+        // statistics, so only x is measured and the phases alternate from tile to tile
+        if (!mbar_wait_warp(&bars.raw_full[s], m & 1, 2u) || !mbar_wait_warp(&bars.gram_free, kF16 ? ((k & 1) ^ 1) : 1u, 2u)) break;
+        tc_fence_after();
+        const uint32_t z_addr = smem_u32(sm + ToLayout::zt + s * kOperandBytes), x_addr = smem_u32(sm + ToLayout::xt + s * kOperandBytes);
+        if (!kF16) {
+          if (elect_lane()) {
 #pragma unroll
             for (int ks = 0; ks < 8; ++ks) {
               const uint64_t d = umma_desc_sw128(z_addr + (ks >> 2) * kPanelBytes) + 2 * (ks & 3);
               umma_bf16(tmem_base + kToColGram, d, d, idesc_z, ks ? 1u : 0u);
             }
             umma_commit(&bars.gram_full);
-            if (!mbar_wait(&bars.gram_free, 0u, 2u)) break;
-            tc_fence_after();
           }
+          __syncwarp();
+          if (!mbar_wait_warp(&bars.gram_free, 0u, 2u)) break;
+          tc_fence_after();
+        }
+        if (elect_lane()) {
 #pragma unroll
           for (int ks = 0; ks < 8; ++ks) {
             const uint64_t d = umma_desc_mn_sw128(x_addr + ks * 2048, kPanelBytes, 1024);
@@ -175,19 +192,22 @@ trimul_out_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_con
           umma_commit(&bars.gram_full);
           umma_commit(&bars.a_empty[s]);
         }
-      } else {
-        // ---------------------------------------------------------------- gate (warp 21) / projection (warp 22) product
-        const bool proj = warp == 22;
-        const uint32_t idesc = proj ? umma_idesc_f16(128, 144, true, false) : umma_idesc_16(128, 144, kF16, kF16);
-        const uint32_t d_tmem = tmem_base + (proj ? kToColP : kToColG);
-        const uint32_t w_addr = smem_u32(sm + (proj ? ToLayout::wz : ToLayout::wg));
-        const uint64_t wx_desc = umma_desc_sw32(smem_u32(sm + (proj ? ToLayout::wxz : ToLayout::wxg)));
-        int k = 0;
-        const bool have_w = mbar_wait(&bars.w_full, 0, 4u);      // the resident weights
-        for (int tile = first_tile; tile < n_tiles && have_w; tile += tile_step, ++k) {
-          const int s = k % kToStages, m = k / kToStages;
-          if (!mbar_wait(&bars.raw_full[s], m & 1, 4u) || !mbar_wait(&bars.acc_free, (k & 1) ^ 1, 8u)) break;
-          tc_fence_after();
+        __syncwarp();
+      }
+    } else {
+      // ---------------------------------------------------------------- gate (warp 21) / projection (warp 22) product
+      const bool proj = warp == 22;
+      const uint32_t idesc = proj ? umma_idesc_f16(128, 144, true, false) : umma_idesc_16(128, 144, kF16, kF16);
+      const uint32_t d_tmem = tmem_base + (proj ? kToColP : kToColG);
+      const uint32_t w_addr = smem_u32(sm + (proj ? ToLayout::wz : ToLayout::wg));
+      const uint64_t wx_desc = umma_desc_sw32(smem_u32(sm + (proj ? ToLayout::wxz : ToLayout::wxg)));
+      int k = 0;
+      const bool have_w = mbar_wait_warp(&bars.w_full, 0, 4u);   // the resident weights
+      for (int tile = first_tile; tile < n_tiles && have_w; tile += tile_step, ++k) {
+        const int s = k % kToStages, m = k / kToStages;
+        if (!mbar_wait_warp(&bars.raw_full[s], m & 1, 4u) || !mbar_wait_warp(&bars.acc_free, (k & 1) ^ 1, 8u)) break;
+        tc_fence_after();
+        if (elect_lane()) {
           const uint32_t a_addr = smem_u32(sm + (proj ? ToLayout::xt : ToLayout::zt) + s * kOperandBytes);
 #pragma unroll
           for (int ks = 0; ks < 8; ++ks) {
@@ -195,14 +215,18 @@ trimul_out_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_con
                                          : umma_desc_sw128(a_addr + (ks >> 2) * kPanelBytes) + 2 * (ks & 3);
             umma_bf16(d_tmem, a_desc, umma_desc_sw128(w_addr + (ks >> 2) * kToWPanel) + 2 * (ks & 3), idesc, ks ? 1u : 0u);
           }
-          umma_commit(&bars.main_full);                        // the sums (columns 128..143) are there
-          if (!mbar_wait(&bars.a_ready[s], m & 1, 4u)) break;  // the correction step needs the statistics
-          tc_fence_after();
+          umma_commit(&bars.main_full);                      // the sums (columns 128..143) are there
+        }
+        __syncwarp();
+        if (!mbar_wait_warp(&bars.a_ready[s], m & 1, 4u)) break;   // the correction step needs the statistics
+        tc_fence_after();
+        if (elect_lane()) {
           umma_bf16(d_tmem, umma_desc_sw32(smem_u32(sm + ToLayout::ax + s * 128 * 32)), wx_desc,
                     umma_idesc_bf16(128, 144, false, false), 1u);
           umma_commit(&bars.acc_full);
           umma_commit(&bars.a_empty[s]);
         }
+        __syncwarp();
       }
     }
   } else if (warp >= 16) {
