@@ -151,17 +151,17 @@ trimul_contract_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
   if (stop) {
     // nothing
   } else if (warp == 0) {
-    if (elect_lane()) {
-      uint32_t it = 0;
-      bool ok = true;
-      for (int tile = first_tile; tile < total_tiles && ok; tile += tile_step) {
-        int c, i0, j0;
-        tile_coords(tile, c, i0, j0);
-        for (int kt = 0; kt < nk && ok; ++kt, ++it) {
-          const int s = it % kStages;
-          const uint32_t ph = (it / kStages) & 1;
-          ok = mbar_wait(&bars.empty[s], ph ^ 1, 1u);
-          if (!ok) break;
+    uint32_t it = 0;
+    bool ok = true;
+    for (int tile = first_tile; tile < total_tiles && ok; tile += tile_step) {
+      int c, i0, j0;
+      tile_coords(tile, c, i0, j0);
+      for (int kt = 0; kt < nk && ok; ++kt, ++it) {
+        const int s = it % kStages;
+        const uint32_t ph = (it / kStages) & 1;
+        ok = mbar_wait_warp(&bars.empty[s], ph ^ 1, 1u);
+        if (!ok) break;
+        if (elect_lane()) {
           const uint32_t sa = smem_u32(ring + s * Shape::kStageBytes);
           if constexpr (kPair) {
             if (rank == 0) mbar_expect_tx(&bars.full[s], 2 * Shape::kStageBytes);
@@ -174,44 +174,50 @@ trimul_contract_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
             tma_load_3d(sa + kTcABytes, &map_b, &bars.full[s], kt * kTcBK, j0, c);
           }
         }
+        __syncwarp();
       }
     }
   } else if (warp == 1) {
-    if (elect_lane() && rank == 0) {
+    if (rank == 0) {
       constexpr uint32_t idesc = umma_idesc_f16(kTcBM * kCtas, kTcBN);
       uint32_t it = 0, tcount = 0;
       bool ok = true;
       for (int tile = first_tile; tile < total_tiles && ok; tile += tile_step, ++tcount) {
         const uint32_t ab = tcount & 1, aph = (tcount >> 1) & 1;
-        ok = mbar_wait(&bars.acc_empty[ab], aph ^ 1, 2u);
+        ok = mbar_wait_warp(&bars.acc_empty[ab], aph ^ 1, 2u);
         if (!ok) break;
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + ab * kTcBN;
         for (int kt = 0; kt < nk; ++kt, ++it) {
           const int s = it % kStages;
           const uint32_t ph = (it / kStages) & 1;
-          ok = mbar_wait(&bars.full[s], ph, 4u);
+          ok = mbar_wait_warp(&bars.full[s], ph, 4u);
           if (!ok) break;
           tc_fence_after();
-          const uint32_t sa = smem_u32(ring + s * Shape::kStageBytes);
-          const uint64_t da = umma_desc_sw128(sa), db = umma_desc_sw128(sa + kTcABytes);
+          if (elect_lane()) {
+            const uint32_t sa = smem_u32(ring + s * Shape::kStageBytes);
+            const uint64_t da = umma_desc_sw128(sa), db = umma_desc_sw128(sa + kTcABytes);
 #pragma unroll
-          for (int k = 0; k < kTcBK / 16; ++k) {  // 16 fp16 = 32 bytes = 2 units of the start-address field
+            for (int k = 0; k < kTcBK / 16; ++k) {  // 16 fp16 = 32 bytes = 2 units of the start-address field
+              if constexpr (kPair)
+                umma_pair(d_tmem, da + 2 * k, db + 2 * k, idesc, (kt | k) ? 1u : 0u);
+              else
+                umma_bf16(d_tmem, da + 2 * k, db + 2 * k, idesc, (kt | k) ? 1u : 0u);
+            }
             if constexpr (kPair)
-              umma_pair(d_tmem, da + 2 * k, db + 2 * k, idesc, (kt | k) ? 1u : 0u);
+              umma_commit_pair(&bars.empty[s]);
             else
-              umma_bf16(d_tmem, da + 2 * k, db + 2 * k, idesc, (kt | k) ? 1u : 0u);
+              umma_commit(&bars.empty[s]);
+            if (kt == nk - 1) {
+              if constexpr (kPair)
+                umma_commit_pair(&bars.acc_full[ab]);
+              else
+                umma_commit(&bars.acc_full[ab]);
+            }
           }
-          if constexpr (kPair)
-            umma_commit_pair(&bars.empty[s]);
-          else
-            umma_commit(&bars.empty[s]);
+          __syncwarp();
         }
         if (!ok) break;
-        if constexpr (kPair)
-          umma_commit_pair(&bars.acc_full[ab]);
-        else
-          umma_commit(&bars.acc_full[ab]);
       }
     }
   } else {
@@ -316,7 +322,7 @@ static int32_t launch_contract(const void* a, const void* b, void* x, int64_t ch
   at[1].id = cudaLaunchAttributeClusterDimension;
   at[1].val.clusterDim.x = kCtas, at[1].val.clusterDim.y = 1, at[1].val.clusterDim.z = 1;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)((total < room ? total : room) * kCtas));
+  cfg.gridDim = dim3((unsigned)(even_grid(total, room) * kCtas));
   cfg.blockDim = dim3(192);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;

@@ -348,7 +348,7 @@ static int32_t launch_msa_rows(const void* w, const void* w2, MrArgs g, int64_t 
   g.n = (int)n, g.s_rows = (int)s_rows, g.n_tiles = (int)n_tiles;      // at most 2^13 * 2^15 tiles
   const size_t smem = MrLayout::total + 1024;
   static SmemLimit limit;
-  const int grid = (int)(n_tiles < sm_count() ? n_tiles : sm_count());
+  const int grid = even_grid(n_tiles, sm_count());
   return limit.set(msa_rows_tc_kernel<kMode>, smem) &&
                  launch_pdl(msa_rows_tc_kernel<kMode>, dim3((unsigned)grid), kMrThreads, smem, st, mw, mw2, g)
              ? PX_OK

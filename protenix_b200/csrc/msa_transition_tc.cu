@@ -346,7 +346,7 @@ extern "C" int32_t px_msa_transition(float* m, const void* prepared, const float
   if (!make_plane_map(&m1, p, 2 * kMtHid, kMtC, 128) || !make_plane_map(&m2, p + kMtW1Elems, kMtC, kMtHid, 64)) return PX_ERR_LAUNCH;
   const size_t smem = MtLayout::total + 1024;
   static SmemLimit limit;
-  const int grid = (int)(n_tiles < sm_count() ? n_tiles : sm_count());
+  const int grid = even_grid(n_tiles, sm_count());
   return limit.set(msa_transition_tc_kernel, smem) &&
                  launch_pdl(msa_transition_tc_kernel, dim3(grid), kMtThreads, smem, (cudaStream_t)stream, m1, m2, m, ln_w, ln_b,
                             (long long)rows, (int)n_tiles, eps)

@@ -156,7 +156,7 @@ static int32_t launch_pair_bias(const void* z, const PbWeights<kF16>& weights, c
   static SmemLimit limit;
   if (!limit.set(pair_bias_tc_kernel<kF16>, smem)) return PX_ERR_LAUNCH;
   const int64_t n_tiles = (rows + 127) / 128;
-  const int grid = (int)(n_tiles < sm_count() ? n_tiles : sm_count());
+  const int grid = even_grid(n_tiles, sm_count());
   return launch_pdl(pair_bias_tc_kernel<kF16>, dim3(grid), pb_threads(kF16), smem, st, mz, weights, (const unsigned char*)folded, out,
                     (long long)rows, (int)n_heads, eps, (int)n_tiles)
              ? PX_OK

@@ -150,4 +150,12 @@ static inline int sm_count() {
   return cached[dev];
 }
 
+// CTAs (or pairs of them) of a persistent kernel that deals out `tiles` in turn: as few of the `room` that fit as end with the same
+// number of tiles each.  The others would only end a tile earlier, and they keep CTAs of another stream (the single branch) from
+// the SMs and ask L2 for more at once: pair path at N = 200 249 -> 246 us a block, with the single branch beside it 288 -> 285.
+static inline int even_grid(int64_t tiles, int64_t room) {
+  const int64_t rounds = (tiles + room - 1) / room;
+  return (int)((tiles + rounds - 1) / rounds);
+}
+
 }  // namespace px

@@ -244,7 +244,7 @@ static int32_t launch_recycle(const void* z, const void* z_init, void* out, cons
   static SmemLimit limit;
   if (!limit.set(recycle_tc_kernel<Tz>, smem)) return PX_ERR_LAUNCH;
   const int64_t n_tiles = (rows + 127) / 128;
-  const int grid = (int)(n_tiles < sm_count() ? n_tiles : sm_count());
+  const int grid = even_grid(n_tiles, sm_count());
   return launch_pdl(recycle_tc_kernel<Tz>, dim3(grid), 32 * rc_warps(sizeof(Tz) != 2), smem, st, mz, mi, mo, (const Tz*)z_init, (Tz*)out, ln_w, ln_b,
                     (const bf16*)w, (long long)rows, eps, (int)n_tiles)
              ? PX_OK

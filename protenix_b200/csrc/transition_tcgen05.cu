@@ -455,7 +455,7 @@ static int32_t launch_transition(const void* x_in, void* x_out, const float* ln_
   static SmemLimit limit;
   if (!limit.set(transition_tc_kernel<Tz>, smem)) return PX_ERR_LAUNCH;
   const int64_t n_tiles = (rows + 127) / 128;
-  const int grid = (int)(n_tiles < sm_count() ? n_tiles : sm_count());
+  const int grid = even_grid(n_tiles, sm_count());
   return launch_pdl(transition_tc_kernel<Tz>, dim3(grid), kTrThreads, smem, st, ma, mb, mo, mx, mr, (const Tz*)x_in, ln_w, ln_b,
                     (long long)rows, (int)n_tiles, (int)add_residual, (int)(sizeof(Tz) == 2 || x_in != x_out), eps)
              ? PX_OK
