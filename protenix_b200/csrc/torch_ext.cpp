@@ -490,7 +490,9 @@ void tri_mul(const PairCall& c, const Prepared& pr, const void* z_in, void* z_ou
   });
 }
 
-void tri_att(const PairCall& c, const Prepared& pr, const void* z_in, void* z_out, bool ending, bool add, Rows& rows) {
+// before_core(): called when everything in front of the attention core has been launched.
+template <typename F>
+void tri_att(const PairCall& c, const Prepared& pr, const void* z_in, void* z_out, bool ending, bool add, Rows& rows, F before_core) {
   const auto& p = pr.p[c.zf];
   const float eps = pr.scalars[0], inf = pr.scalars[1];
   const int64_t n = c.n, ldm = abi.px_ld_mask(n);
@@ -504,6 +506,7 @@ void tri_att(const PairCall& c, const Prepared& pr, const void* z_in, void* z_ou
     return abi.px_triatt_in_proj_folded(fp32 ? rows.zn : z_in, fp32 ? PX_F16 : c.dt, c.mask, p[0], q, k, v, (float*)bias, (float*)mbias, n,
                                         n, ldm, ending, eps, inf, c.st);
   });
+  before_core();
   launch("px_triatt_flash", c.st, [&] {
     return abi.px_triatt_flash(q, k, v, (const float*)bias, (const float*)mbias, o, n, n, ldm, c.st);
   });
@@ -556,7 +559,7 @@ Tensor tri_att_forward(Params& params, const Tensor& z, const OptTensor& mask, b
   const Tensor ws = bytes_like(zc, abi.px_triatt_workspace_bytes(zc.size(0)));
   const PairCall c{zc.size(0), zformat(zc), dtype_code(zc, "z"), fptr(m), (unsigned char*)ws.data_ptr(), at::cuda::getCurrentCUDAStream()};
   Rows rows = own_rows(c, ws);
-  tri_att(c, *pr, zc.data_ptr(), out.data_ptr(), ending, inplace_add, rows);
+  tri_att(c, *pr, zc.data_ptr(), out.data_ptr(), ending, inplace_add, rows, [] {});
   return batch ? out.unsqueeze(0) : out;
 }
 
@@ -618,14 +621,16 @@ c10::cuda::CUDAStream side_stream(const Use& use) {
 }
 
 // The blocks one after the other.  The pair path never reads s, and the single branch takes nothing from z but the pair
-// bias of the block's final z: the branch of a block can run on a side stream beside the pair path of the next block (two
-// pair-bias buffers take turns), and its projections, which need no bias, already beside that of its own block.  What runs
-// beside takes SMs from persistent kernels whose tiles are dealt out in advance, so it pays only where they leave some or the
-// branch is a large part of a block.  Four blocks, us per block, in order | beside, projections with the rest | beside,
-// projections first: N = 128: 225 | 189 | 186, 200: 405 | 377 | 372, 300: 733 | 695 | 704, 437: 1364 | 1324 | 1332,
-// 640: 2747 | 2742 | 2727, 1024: 8140 | 8195 | 8181; one block alone: 224 | - | 216 at N = 128, no difference from N = 200 on.
+// bias of the block's final z: the branch of a block runs on a side stream beside the pair path of the next block (two
+// pair-bias buffers take turns).  It is let go when the next block comes to its first attention core, whose CTAs are dealt out
+// as SMs come free; beside the row kernels, whose tiles are dealt out in advance, each of its kernels held up the tile of some
+// SM, and with it the whole kernel.  24 blocks, us per block, in order | beside from the block's start on | beside the attention core:
+// N = 24: 161 | 113 | 111, 64: 168 | 120 | 114, 128: - | 155 | 142, 200: - | 296 | 284, 256: 388 | 348 | 334, 384: - | 741 | 728,
+// 437: 1064 | 1044 | 1028, 640: 2305 | 2273 | 2242, 768: 3442 | - | 3419, 1024: 6838 | - | 6805, 1280: 11999 | - | 11973.  Its
+// transition only beside the second core: 145 at N = 128, 276 against 278 at 200, 720 against 719 at 384.
+// One block alone: its projections of s, which need no bias, beside its own pair path (224 | 216 at N = 128, no difference from 200 on).
 // Everything is allocated on the caller's stream, which waits for the side stream before this returns.
-constexpr int64_t kBesideBelow = 768, kProjectFirstUpTo = 256;
+constexpr int64_t kBesideBelow = 1281, kProjectFirstUpTo = 256;
 std::tuple<OptTensor, Tensor> stack_forward(const std::vector<std::shared_ptr<Block>>& blocks, const OptTensor& s_in,
                                             const Tensor& z, const OptTensor& mask, bool inplace) {
   bool batch;
@@ -663,11 +668,13 @@ std::tuple<OptTensor, Tensor> stack_forward(const std::vector<std::shared_ptr<Bl
   const PairCall c{n, zf, dtype_code(zc, "z"), fptr(m), (unsigned char*)ws.data_ptr(), main};
   const bool fp32 = c.dt == PX_F32;
   Rows rows = own_rows(c, ws);
-  const bool first = n <= kProjectFirstUpTo;       // projections of s beside the pair path of their own block
+  const bool first = n <= kProjectFirstUpTo;       // projections of s beside the pair path of the first block from its start on
   const bool aside = singles && (blocks.size() > 1 ? n < kBesideBelow : first);
   const auto side = aside ? side_stream(use) : main;
   Tensor bias[2], sb[2], sws;
-  at::cuda::CUDAEvent bias_ready[2], side_done[2];   // bias_ready: what the rest of the branch waits for on its stream
+  at::cuda::CUDAEvent gate, side_done[2];
+  int64_t waiting = -1;             // block whose bias is made and whose update is still to be issued
+  int waiting_turn = 0;
   if (singles) {
     for (int i = 0; i < (blocks.size() > 1 ? 2 : 1); ++i) bias[i] = at::empty({kHeadsSingle, n, n}, zc.options().dtype(at::kFloat));
     for (int i = 0; i < (blocks.size() > 1 ? 2 : 1); ++i) sb[i] = at::empty_like(s);
@@ -692,12 +699,23 @@ std::tuple<OptTensor, Tensor> stack_forward(const std::vector<std::shared_ptr<Bl
     if (ready[b].single) last = b;
   for (size_t b = 0; b < ready.size(); ++b) {
     const BlockReady& r = ready[b];
-    if (r.single && first) single_project(side, *r.single, zf, s, sws);
+    if (r.single && first && (b == 0 || !aside)) single_project(side, *r.single, zf, s, sws);
     void* const z = zc.data_ptr();
     tri_mul(c, *r.mul_out, b == 0 ? zi.data_ptr() : z, z, false, true, rows);
     tri_mul(c, *r.mul_in, z, z, true, true, rows);
-    tri_att(c, *r.att_start, z, z, false, true, rows);
-    tri_att(c, *r.att_end, z, z, true, true, rows);
+    tri_att(c, *r.att_start, z, z, false, true, rows, [&] {
+      if (!aside || (waiting < 0 && !r.single)) return;
+      gate.record(main);
+      gate.block(side);
+      if (waiting >= 0) {
+        single_finish(side, *ready[waiting].single, zf, s, sb[waiting_turn], bias[waiting_turn], sws);
+        side_done[waiting_turn].record(side);
+        s = sb[waiting_turn];
+        waiting = -1;
+      }
+      if (r.single && !(first && b == 0)) single_project(side, *r.single, zf, s, sws);
+    });
+    tri_att(c, *r.att_end, z, z, true, true, rows, [] {});
     rows.valid = false;
     transition_rows(c.st, *r.transition, zf, c.dt, z, z, n * n, true);
     if (!r.single) continue;
@@ -710,14 +728,18 @@ std::tuple<OptTensor, Tensor> stack_forward(const std::vector<std::shared_ptr<Bl
       return abi.px_pair_bias_proj_folded(fp32 ? rows.zn : z, fp32 ? PX_F16 : PX_BF16, p[0], (float*)bias[turn].data_ptr(), n * n, kHeadsSingle,
                                           r.pair_bias->scalars[0], c.st);
     });
-    const auto rest = (int64_t)b == last ? main : side;     // the last block's rest has nothing to run beside
-    if (aside) {
-      bias_ready[turn].record(rest == main ? side : main);
-      bias_ready[turn].block(rest);
+    if (aside && (int64_t)b != last) {
+      waiting = b, waiting_turn = turn;
+      ++k;
+      continue;
     }
-    if (!first) single_project(rest, *r.single, zf, s, sws);
-    single_finish(rest, *r.single, zf, s, sb[turn], bias[turn], sws);
-    if (aside) side_done[turn].record(rest);
+    if (aside) {                                   // the last block's rest has nothing to run beside
+      gate.record(side);
+      gate.block(main);
+    } else if (!first) {
+      single_project(main, *r.single, zf, s, sws);
+    }
+    single_finish(main, *r.single, zf, s, sb[turn], bias[turn], sws);
     s = sb[turn];
     ++k;
   }
