@@ -113,9 +113,9 @@ __global__ void __launch_bounds__(256) ln_fwd_cached(const T* __restrict__ x, co
 
 // Rows of exactly LANES x 16 bytes, LANES a power of two <= 32: a group of LANES lanes owns a row.  The rows in flight
 // stay packed as loaded and are converted once per pass (sum, squares, output): held as floats they took 100 registers
-// and a third of the warps (68 us on [768^2, 128] bf16; now 55 us, 0.86 of the copy rate).  Every CTA is resident; (2, 8)
-// measured 55, (4, 4) 62, (6, 2) 69.
-constexpr int kLnFwdOcc = 3, kLnFwdGroups = 4;           // CTAs per SM, row groups in flight per warp
+// and a third of the warps (68 us on [768^2, 128] bf16).  Every CTA is resident, and the rows of the next round are requested
+// before this one's are reduced: 53.6 us, 0.88 of the copy rate; without that, and three CTAs to an SM, 55.7; with it and three CTAs 64.0.
+constexpr int kLnFwdOcc = 2, kLnFwdGroups = 4;           // CTAs per SM, row groups in flight per warp
 template <typename T, int LANES, typename P>
 __global__ void __launch_bounds__(256, kLnFwdOcc) ln_fwd_rows16(const T* __restrict__ x, const P* __restrict__ gamma,
                                                                 const P* __restrict__ beta, T* __restrict__ y,
@@ -131,14 +131,21 @@ __global__ void __launch_bounds__(256, kLnFwdOcc) ln_fwd_rows16(const T* __restr
     g[e] = gamma ? param<T, P>(gamma[li * VEC + e]) : 1.f;
     b[e] = beta ? param<T, P>(beta[li * VEC + e]) : 0.f;
   }
+  uint4 next[kB];                                          // the rows of the next round, on their way while this one's are worked on
+  auto request = [&](int64_t r0) {
+#pragma unroll
+    for (int j = 0; j < kB; ++j) {
+      const int64_t row = r0 + j * kR + sub;
+      next[j] = row < rows ? __ldcs(reinterpret_cast<const uint4*>(x + row * kCols) + li) : make_uint4(0, 0, 0, 0);
+    }
+  };
+  request(warp0 * (kB * kR));
   for (int64_t r0 = warp0 * (kB * kR); r0 < rows; r0 += nwarps * (kB * kR)) {
     uint4 raw[kB];
     float acc[kB], mean[kB];
 #pragma unroll
-    for (int j = 0; j < kB; ++j) {
-      const int64_t row = r0 + j * kR + sub;
-      raw[j] = row < rows ? __ldcs(reinterpret_cast<const uint4*>(x + row * kCols) + li) : make_uint4(0, 0, 0, 0);
-    }
+    for (int j = 0; j < kB; ++j) raw[j] = next[j];
+    request(r0 + nwarps * (kB * kR));
 #pragma unroll
     for (int j = 0; j < kB; ++j) {
       const Vec<T, VEC> t = *reinterpret_cast<const Vec<T, VEC>*>(&raw[j]);
@@ -282,17 +289,17 @@ static cudaError_t dispatch(const void* x, const void* g, const void* b, void* y
 // groups, warps and CTAs are combined once at the end (shuffles, shared memory, one atomic per column and CTA into an
 // fp32 scratch, which a second kernel converts).  The row-by-row form below, with a shared-memory atomic per element,
 // took 234 us on [768^2, 128] bf16 where the three tensors take 69 us at the copy rate; it is left for wider rows.
-// CTAs per SM and row groups in flight per warp: 88 us with (2, 3) on [768^2, 128] bf16; (2, 2) 92, (2, 4) 97, (3, 2) 97,
-// (4, 1) 97.
+// Two CTAs to an SM and two (fp32 three) row groups a warp, the next round's requested before this one's are reduced: [768^2, 128]
+// bf16 85 us, fp32 147; without the early request and with three groups 91 and 153, with it and three groups 98 in bf16, two 155 in fp32.
 constexpr int kLnBwdOcc = 2;
-constexpr int ln_bwd_groups(int it) { return it == 1 ? 3 : it == 2 ? 2 : 1; }
+constexpr int ln_bwd_groups(int it, int bytes) { return it == 1 ? (bytes == 4 ? 3 : 2) : it == 2 ? 2 : 1; }
 template <typename T, typename P, int LANES, int IT>
 __global__ void __launch_bounds__(256, IT == 1 ? kLnBwdOcc : 1) ln_bwd_rows(const T* __restrict__ dy, const T* __restrict__ x,
                                                    const float* __restrict__ mean, const float* __restrict__ invvar,
                                                    const P* __restrict__ gamma, T* __restrict__ dx,
                                                    float* __restrict__ scratch, long long rows, int cols) {
   constexpr int VEC = 16 / (int)sizeof(T), kR = 32 / LANES;
-  constexpr int kB = ln_bwd_groups(IT);                  // row groups in flight per warp
+  constexpr int kB = ln_bwd_groups(IT, (int)sizeof(T));                  // row groups in flight per warp
   extern __shared__ float ln_bwd_sums[];                 // [8 warps][2][cols]
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, sub = lane / LANES, li = lane % LANES;
   const int nvec = cols / VEC;
@@ -307,23 +314,37 @@ __global__ void __launch_bounds__(256, IT == 1 ? kLnBwdOcc : 1) ln_bwd_rows(cons
       dg[i][e] = db[i][e] = 0.f;
     }
   const long long step = (long long)gridDim.x * 8 * kR * kB;
-  for (long long r0 = ((long long)blockIdx.x * 8 + warp) * (kR * kB); r0 < rows; r0 += step) {
-    uint4 rx[kB][IT], ry[kB][IT];
-    float mu[kB], rs[kB];
+  // the rows of the next round are on their way while this one's are worked on
+  uint4 nx[kB][IT], ny[kB][IT];
+  float nmu[kB], nrs[kB];
+  auto request = [&](long long r0) {
 #pragma unroll
     for (int j = 0; j < kB; ++j) {
       const long long row = r0 + j * kR + sub;
       const bool in = row < rows;
-      mu[j] = in ? __ldg(mean + row) : 0.f;
-      rs[j] = in ? __ldg(invvar + row) : 0.f;
+      nmu[j] = in ? __ldg(mean + row) : 0.f;
+      nrs[j] = in ? __ldg(invvar + row) : 0.f;
 #pragma unroll
       for (int i = 0; i < IT; ++i) {
         const int v = li + LANES * i;
         const bool have = in && v < nvec;                // absent values count as zero everywhere
-        rx[j][i] = have ? __ldcs(reinterpret_cast<const uint4*>(x + (size_t)row * cols) + v) : make_uint4(0, 0, 0, 0);
-        ry[j][i] = have ? __ldcs(reinterpret_cast<const uint4*>(dy + (size_t)row * cols) + v) : make_uint4(0, 0, 0, 0);
+        nx[j][i] = have ? __ldcs(reinterpret_cast<const uint4*>(x + (size_t)row * cols) + v) : make_uint4(0, 0, 0, 0);
+        ny[j][i] = have ? __ldcs(reinterpret_cast<const uint4*>(dy + (size_t)row * cols) + v) : make_uint4(0, 0, 0, 0);
       }
     }
+  };
+  const long long begin = ((long long)blockIdx.x * 8 + warp) * (kR * kB);
+  request(begin);
+  for (long long r0 = begin; r0 < rows; r0 += step) {
+    uint4 rx[kB][IT], ry[kB][IT];
+    float mu[kB], rs[kB];
+#pragma unroll
+    for (int j = 0; j < kB; ++j) {
+      mu[j] = nmu[j], rs[j] = nrs[j];
+#pragma unroll
+      for (int i = 0; i < IT; ++i) rx[j][i] = nx[j][i], ry[j][i] = ny[j][i];
+    }
+    request(r0 + step);
     float s1[kB], s2[kB];
 #pragma unroll
     for (int j = 0; j < kB; ++j) {
@@ -449,7 +470,7 @@ __global__ void ln_bwd_finish_kernel(const float* __restrict__ scratch, P* __res
 template <typename T, typename P, int LANES, int IT>
 static cudaError_t launch_bwd_rows(const void* dy, const void* x, const float* mean, const float* invvar, const void* gamma,
                                    void* dx, float* scratch, long long rows, int cols, int sms, cudaStream_t st) {
-  constexpr int kB = ln_bwd_groups(IT), kRows = 8 * (32 / LANES) * kB;
+  constexpr int kB = ln_bwd_groups(IT, (int)sizeof(T)), kRows = 8 * (32 / LANES) * kB;
   const size_t smem = scratch ? (size_t)16 * cols * sizeof(float) : 0;
   const long long want = (rows + kRows - 1) / kRows;
   const int grid = (int)(want < kLnBwdOcc * sms ? want : (long long)kLnBwdOcc * sms);   // resident CTAs: every extra one adds 2 * cols atomics
