@@ -111,7 +111,8 @@ triatt_flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
   unsigned char* sm = smem_aligned(smem_raw);
   FlashBars& bars = *reinterpret_cast<FlashBars*>(sm + FlashLayout::bars);
   const int warp = warp_index(), lane = threadIdx.x & 31;
-  const int q0 = blockIdx.x * 128, h = blockIdx.y, u0 = blockIdx.z * kFRows;
+  // the last rows first: their q, k and v were written last and may still lie in L2
+  const int q0 = blockIdx.x * 128, h = blockIdx.y, u0 = (gridDim.z - 1 - blockIdx.z) * kFRows;
 
   const bool skip = cta_begin();         // an earlier bounded wait gave up: do not start new work
   if (threadIdx.x == 32) prefetch_maps(map_q, map_k, map_v, map_b, map_o);

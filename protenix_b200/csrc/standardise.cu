@@ -23,7 +23,11 @@ __global__ void __launch_bounds__(256) standardise_rows_kernel(const float* __re
   const long long warp = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const long long nwarps = (long long)gridDim.x * (blockDim.x >> 5);
   constexpr int kB = kStdRowsPerBatch;
-  for (long long r0 = warp * kB; r0 < rows; r0 += nwarps * kB) {
+  // From the last row to the first: z's last rows were written last, and the rows that the next kernel begins with are then the ones
+  // written last here, so both find in L2 what is left there (with the order of rows in the attention core, which is turned round for the
+  // same reason: pair path, us per block, N = 384 674 -> 666, 512 1293 -> 1276, 640 2172 -> 2155, 1024 on level).
+  for (long long b = (rows + kB - 1) / kB - 1 - warp; b >= 0; b -= nwarps) {
+    const long long r0 = b * kB;
     float4 v[kB];
     float acc[kB];
 #pragma unroll
