@@ -14,7 +14,7 @@
 //   split_gemm SWIGLU h = silu(a) * b, a and b interleaved in the weight rows, written as three planes [3][N][1536]
 //   split_gemm RES    s2 = s1 + h W_out^T, the contraction split over a cluster of four CTAs
 // At N tokens each product has N/128 x (outputs/64) tiles: far too few to fill the chip at any N, so every launch is
-// bound by the latency of one tile (load, 24 MMAs per 64 inputs, epilogue); hence narrow 64-column tiles, no
+// bound by the latency of one tile (load, 16 MMAs per 64 inputs, epilogue); hence narrow 64-column tiles, no
 // persistence, and the split contraction where it is 1536 long.  Whole branch on an idle GPU: 64 us at N = 128 and 76 us at
 // N = 384, where library GEMMs and the composed attention took 290 us; 0.36 ms against 0.76 at N = 1536.
 #include <initializer_list>
@@ -31,16 +31,19 @@ constexpr int kSgABytes = 3 * 128 * 128;  // three planes of [128 rows][64 k] bf
 constexpr int kSgWBytes = 3 * kSgBN * 128;
 constexpr int kSgStageBytes = kSgABytes + kSgWBytes;
 constexpr int kSgStages = 3;
-// Tensor memory: the leading products (plane 0 x plane 0) go round three accumulators, the corrections into three more.
-// The tensor core truncates when it adds to an accumulator, a bias that grows with the number of additions: one
-// accumulator for all 144 steps of K = 384 gave a relative error of 4.3e-6 on s; with these it is 2.6e-7 (fp32 GEMMs
+// Tensor memory: the leading products (plane 0 x plane 0) go round four accumulators, the corrections of order 2^-8 and of order
+// 2^-16 have one each.  The tensor core truncates when it adds to an accumulator, a bias that grows with the number of additions: one
+// accumulator for all 144 steps of K = 384 gave a relative error of 4.3e-6 on s; with these it is 2.0e-7 (fp32 GEMMs
 // of the library: 3.5e-7 to 4.8e-7).
-constexpr int kSgMain = 3;
-constexpr int kSgIssuers = 3;             // MMA-issuing warps, two of the six partial products each: an MMA of 64 columns
-                                          // takes 32 cycles, its issue about 100
-constexpr int kSgAcc = kSgMain + kSgIssuers;
+// The planes of W lie behind one another, so that neighbouring partial products with one plane of A are one product of 128 columns:
+// A0 W0 (48 cycles of the tensor pipe a step), A0 [W1 W2] (64), A1 [W0 W1] (64), A2 W0 (48), where six products of 64 columns, read
+// from shared memory one by one, took 288: 0.4 to 0.8 us of 11 to 15 a kernel at N = 128, and the error was 2.4e-7.
+constexpr int kSgMain = 4;
+constexpr int kSgCorr = kSgBN * kSgMain;  // columns of the corrections: order 2^-8, then order 2^-16
+constexpr int kSgAcc = kSgMain + 2;
+constexpr int kSgEpilogue = 4;            // first of the epilogue's four warps
 constexpr uint32_t kSgCols = 512;
-constexpr int kSgThreads = 32 * (1 + kSgIssuers + 4);
+constexpr int kSgThreads = 32 * (kSgEpilogue + 4);
 constexpr int kSgSplit = 4;               // CTAs of a cluster that share a contraction of 1536
 
 enum { kSgQkvg = 0, kSgRes = 1, kSgSwiglu = 2 };
@@ -101,7 +104,7 @@ __device__ __forceinline__ void cluster_sync() {
 }
 
 // One 128 x 64 tile of a split product per cluster (of gridDim.z CTAs, each with its share of the contraction).
-// Warp 0: TMA producer (three planes of A and of W per 64 inputs), warps 1..3: MMA issuers, warps 4..7: epilogue.
+// Warp 0: TMA producer (three planes of A and of W per 64 inputs), warp 1: MMA issuer, warps 4..7: epilogue.
 template <int kMode, typename T>
 __global__ void __launch_bounds__(kSgThreads, 1)
 split_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w, const SgArgs g) {
@@ -116,9 +119,9 @@ split_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
   if (threadIdx.x == 0) {
     for (int s = 0; s < kSgStages; ++s) {
       mbar_init(&bars.full[s], 1);
-      mbar_init(&bars.empty[s], kSgIssuers);
+      mbar_init(&bars.empty[s], 1);
     }
-    mbar_init(&bars.acc_full, kSgIssuers);
+    mbar_init(&bars.acc_full, 1);
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
   if (warp == 0) {
@@ -145,10 +148,10 @@ split_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
   bool ok = !skip;
 
   if (warp == 0) {
-    if (elect_lane() && ok) {
-      for (int i = 0; i < g.chunks; ++i) {
-        const int s = i % kSgStages;
-        if (!mbar_wait(&bars.empty[s], ((i / kSgStages) & 1) ^ 1, 1u)) break;
+    for (int i = 0; i < g.chunks && ok; ++i) {
+      const int s = i % kSgStages;
+      if (!mbar_wait_warp(&bars.empty[s], ((i / kSgStages) & 1) ^ 1, 1u)) break;
+      if (elect_lane()) {
         const uint32_t dst = smem_u32(ring + s * kSgStageBytes);
         if (i >= early) {
           mbar_expect_tx(&bars.full[s], kSgStageBytes);
@@ -156,37 +159,34 @@ split_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
         }
         tma_load_3d(dst, &map_a, &bars.full[s], (kc0 + i) * 64, m0, 0);
       }
+      __syncwarp();
     }
-  } else if (warp <= kSgIssuers) {
-    if (elect_lane() && ok) {
-      // planes (i, j) with i + j <= 2, the terms above 2^-24 of the product: (0,0) (0,1) | (1,0) (1,1) | (0,2) (2,0)
-      const int w_ = warp - 1;
-      const int ai0 = w_ == 1 ? 1 : 0, aj0 = w_ == 2 ? 2 : 0, ai1 = w_, aj1 = w_ == 2 ? 0 : 1;
-      constexpr uint32_t idesc = umma_idesc_bf16(128, kSgBN);
-      const uint32_t corr = tmem_base + kSgBN * (kSgMain + w_);
-      bool done = true;
-      for (int i = 0; i < g.chunks; ++i) {
-        const int s = i % kSgStages;
-        done = mbar_wait(&bars.full[s], (i / kSgStages) & 1, 2u);
-        if (!done) break;
-        tc_fence_after();
+  } else if (warp == 1) {
+    constexpr uint32_t idesc1 = umma_idesc_bf16(128, kSgBN), idesc2 = umma_idesc_bf16(128, 2 * kSgBN);
+    bool done = ok;
+    for (int i = 0; i < g.chunks && done; ++i) {
+      const int s = i % kSgStages;
+      done = mbar_wait_warp(&bars.full[s], (i / kSgStages) & 1, 2u);
+      if (!done) break;
+      tc_fence_after();
+      if (elect_lane()) {
         const uint32_t a = smem_u32(ring + s * kSgStageBytes), w = a + kSgABytes;
-        const uint64_t da0 = umma_desc_sw128(a + ai0 * (128 * 128)), dw0 = umma_desc_sw128(w + aj0 * (kSgBN * 128));
-        const uint64_t da1 = umma_desc_sw128(a + ai1 * (128 * 128)), dw1 = umma_desc_sw128(w + aj1 * (kSgBN * 128));
+        const uint64_t a0 = umma_desc_sw128(a), a1 = umma_desc_sw128(a + 128 * 128), a2 = umma_desc_sw128(a + 2 * 128 * 128);
+        const uint64_t w0 = umma_desc_sw128(w), w1 = umma_desc_sw128(w + kSgBN * 128);
 #pragma unroll
-        for (int ks = 0; ks < 4; ++ks) {
+        for (int ks = 0; ks < 4; ++ks) {           // the terms above 2^-24 of the product: planes i + j <= 2
           const int step = 4 * i + ks;
-          if (w_ == 0)
-            umma_bf16(tmem_base + kSgBN * (step % kSgMain), da0 + 2 * ks, dw0 + 2 * ks, idesc, step >= kSgMain);
-          else
-            umma_bf16(corr, da0 + 2 * ks, dw0 + 2 * ks, idesc, step > 0);
-          umma_bf16(corr, da1 + 2 * ks, dw1 + 2 * ks, idesc, step > 0 || w_ > 0);
+          umma_bf16(tmem_base + kSgBN * ks, a0 + 2 * ks, w0 + 2 * ks, idesc1, i > 0);
+          umma_bf16(tmem_base + kSgCorr, a0 + 2 * ks, w1 + 2 * ks, idesc2, step > 0);
+          umma_bf16(tmem_base + kSgCorr, a1 + 2 * ks, w0 + 2 * ks, idesc2, 1u);
+          umma_bf16(tmem_base + kSgCorr + kSgBN, a2 + 2 * ks, w0 + 2 * ks, idesc1, 1u);
         }
         umma_commit(&bars.empty[s]);
+        if (i == g.chunks - 1) umma_commit(&bars.acc_full);
       }
-      if (done) umma_commit(&bars.acc_full);
+      __syncwarp();
     }
-  } else {
+  } else if (warp >= kSgEpilogue) {
     const int q = warp & 3, r = 32 * q + lane;     // tensor-memory lane = row of the tile
     ok = ok && mbar_wait(&bars.acc_full, 0, 4u);
     ok = __all_sync(0xffffffffu, ok);
@@ -249,9 +249,9 @@ split_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
   if (kMode == kSgRes) {
     __syncwarp();
     cluster_sync();                                // every CTA's partial tile is in its shared memory
-    if (warp > kSgIssuers && ok) {
+    if (warp >= kSgEpilogue && ok) {
       // each CTA sums and writes its share of the rows; a thread takes 16 bytes of a row at a time
-      const int split = gridDim.z, per = 128 / split, tid = threadIdx.x - 32 * (1 + kSgIssuers);
+      const int split = gridDim.z, per = 128 / split, tid = threadIdx.x - 32 * kSgEpilogue;
       for (int i = tid; i < per * (kSgBN / 4); i += 128) {
         const int r = blockIdx.z * per + i / (kSgBN / 4), c = i % (kSgBN / 4), row = m0 + r;
         const uint32_t src = smem_u32(ring) + (r * (kSgBN / 4) + (c ^ (r & 15))) * 16;
