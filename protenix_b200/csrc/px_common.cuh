@@ -58,8 +58,6 @@ template <>
 __device__ __forceinline__ float2 unpack16x2<false>(uint32_t u) {
   return unpack_bf16x2(u);
 }
-// (1, 1) as a pair of bf16 or of fp16
-__host__ __device__ constexpr uint32_t ones16x2(bool f16) { return f16 ? 0x3C003C00u : 0x3F803F80u; }
 
 // Packed fp32 arithmetic (sm_100): two elements per issue slot.  Pays where the issue slots are the scarce resource
 // (flash attention: -7 %); the SwiGLU of the transition kernel got 22 % slower with it and stays scalar.

@@ -141,14 +141,6 @@ __device__ __forceinline__ void fold_here(const W& weights, const unsigned char*
   if (threadIdx.x == 0) mbar_arrive(full);
 }
 
-// The register of a 32-entry array that belongs to this lane (arr[lane] without local memory).
-__device__ __forceinline__ float select_own(const uint32_t (&arr)[32], int lane) {
-  uint32_t v = 0;
-#pragma unroll
-  for (int e = 0; e < 32; ++e) v = (lane == e) ? arr[e] : v;
-  return __uint_as_float(v);
-}
-
 // TMA store of a 3-D box from shared memory (bulk async group of the calling thread).
 __device__ __forceinline__ void tma_store_3d(const CUtensorMap* map, uint32_t src, int x, int y, int z) {
   asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];\n"
@@ -257,11 +249,35 @@ __device__ __forceinline__ void tile_producer_loop(const Ctx& c, const CUtensorM
   }
 }
 
+// Mean and variance of row r of a bf16 tile.  Two neighbouring lanes share a row, eight 16-byte pieces each (lane 1 begins at another
+// piece, so that the two meet different banks), and sum d and d^2 of d = x - x0 in fp32: about one of its values, nothing cancels
+// however far the row lies from zero.
+__device__ __forceinline__ void bf16_row_stats(const unsigned char* tile, int r, int half, float& mean, float& var) {
+  const float x0 = unpack_bf16x2(*reinterpret_cast<const uint32_t*>(tile + operand_piece_offset(r, 0))).x;
+  float s0 = 0.f, s1 = 0.f, q0 = 0.f, q1 = 0.f;
+#pragma unroll
+  for (int p = 0; p < 8; ++p) {
+    const uint4 v = *reinterpret_cast<const uint4*>(tile + operand_piece_offset(r, 8 * half + (p ^ (4 * half))));
+    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      float2 x = unpack_bf16x2(w[e]);
+      add2(x.x, x.y, -x0, -x0);
+      add2(s0, s1, x.x, x.y);
+      fma2(q0, q1, x.x, x.y, x.x, x.y, q0, q1);
+    }
+  }
+  float sum = s0 + s1, sq = q0 + q1;
+  sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+  sq += __shfl_xor_sync(0xffffffffu, sq, 1);
+  const float m = sum * (1.0f / kC);
+  var = fmaxf(sq * (1.0f / kC) - m * m, 0.f);
+  mean = x0 + m;
+}
+
 // The statistics warps (`sw` = 0..3, or 0..7 for bf16 rows).  per_row(k, u, t, r, rstd) is called once per
 // tile and row with the row's 1/std, before a_ready is signalled.  `kStandardised`: the rows are a standardised copy
 // (mean 0, deviation 1 by construction), so the correction row is (0, 1), written once, and the factor is 1.
-// bf16 rows: two neighbouring lanes share a row, eight 16-byte pieces each (lane 1 begins at another piece, so that the two meet
-// different banks), and sum d and d^2 of d = x - x0 in fp32: about one of its values, nothing cancels however far the row lies from zero.
 template <typename Ctx, typename PerRow>
 __device__ __forceinline__ void tile_stats_loop(const Ctx& c, float eps, int sw, int lane, PerRow per_row) {
   constexpr bool kStandardised = Ctx::kStandardised;
@@ -274,26 +290,8 @@ __device__ __forceinline__ void tile_stats_loop(const Ctx& c, float eps, int sw,
     // for standardised rows the arrival of the tile only paces this loop, so that the slots it writes are those of tiles in flight
     if (!mbar_wait_warp(&c.bars->raw_full[s], (k / Ctx::kStages) & 1, 16u)) break;
     if (!kStandardised) {
-      const unsigned char* z = c.tiles + s * kTileBytes;
-      const float x0 = unpack_bf16x2(*reinterpret_cast<const uint32_t*>(z + operand_piece_offset(r, 0))).x;
-      float s0 = 0.f, s1 = 0.f, q0 = 0.f, q1 = 0.f;
-#pragma unroll
-      for (int p = 0; p < 8; ++p) {
-        const uint4 v = *reinterpret_cast<const uint4*>(z + operand_piece_offset(r, 8 * half + (p ^ (4 * half))));
-        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          float2 x = unpack_bf16x2(w[e]);
-          add2(x.x, x.y, -x0, -x0);
-          add2(s0, s1, x.x, x.y);
-          fma2(q0, q1, x.x, x.y, x.x, x.y, q0, q1);
-        }
-      }
-      float sum = s0 + s1, sq = q0 + q1;
-      sum += __shfl_xor_sync(0xffffffffu, sum, 1);
-      sq += __shfl_xor_sync(0xffffffffu, sq, 1);
-      const float m = sum * (1.0f / kC), var = fmaxf(sq * (1.0f / kC) - m * m, 0.f);
-      mean = x0 + m;
+      float var;
+      bf16_row_stats(c.tiles + s * kTileBytes, r, half, mean, var);
       rstd = rsqrtf(var + eps);
       std = sqrtf(var + eps);
     }

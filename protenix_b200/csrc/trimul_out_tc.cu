@@ -10,17 +10,18 @@
 //     fp32 z, its standardised fp16 copy `zn` (px_standardise_rows), whose statistics are known;
 //   * the x tile arrives by TMA exactly as it lies in memory, [128 channels][128 j], and is used as an MN-major
 //     operand: the tensor core reads it transposed;
-//   * the statistics of both come from Gram products (diagonal = sums of squares) and from 16 rows of ones kept
-//     behind each weight matrix (columns 128..143 of the two accumulators = plain sums).
+//   * the statistics of both are summed by threads from the tiles in shared memory (Gram products with the sums of squares on their
+//     diagonals and rows of ones behind the weights took 600 to 1200 cycles more of the tensor pipe a tile, and the statistics of a
+//     tile as long to come: bf16 N = 200 15.3 -> 14.5 us, 437 45.0 -> 42.7, 768 109 -> 105, 1536 435 -> 420; fp32 N = 128 8.5 -> 8.2,
+//     200 15.0 -> 14.5, 640 98.5 -> 96.5, from 768 on level).
 //
 //   warps 0..15   epilogue: a thread owns one pair element and 32 channels: p * sigmoid(g) + residual (the raw z
 //                 tile in shared memory), packed to bf16 over the z tile in place, which leaves through a TMA store.
 //                 fp32 rows are staged the same way and stored or added by TMA; where the residual lies in another tensor, it
 //                 is read and the rows are written with plain accesses.
-//   warps 16..19  one thread per row: both sets of statistics, the correction row, the scale pair.
-//   warp 20       TMA producer (z and x tiles); warps 21, 22 MMA issuers of the gate and of the projection product,
-//                 warp 23 of the two statistics products.
-// Tensor memory: gate accumulator (144) | projection accumulator (144) | statistics (128, z then x).
+//   warps 16..    statistics of 16 rows a warp at a time (8 warps, or 4 where the z side has none): correction rows, scales.
+//   then          TMA producer (z and x tiles); MMA issuers of the gate and of the projection product.
+// Tensor memory: one or two sets of gate accumulator (128) | projection accumulator (128).
 // Algorithmic HBM traffic per pair element: 256 + 128*sizeof(Tz) read, 128*sizeof(Tz) written.  Every wait is bounded.
 #include <cstring>
 
@@ -28,23 +29,24 @@
 
 namespace px {
 
-constexpr int kToWarps = 24;
-constexpr int kToThreads = 32 * kToWarps;
-constexpr int kToWPanel = 144 * 128;           // [128 weight rows + 16 rows of ones][64 k]
-constexpr int kToWBytes = 2 * kToWPanel;
-constexpr int kToWExtra = 144 * 32;
+__host__ __device__ constexpr int to_stats_warps(bool standardised) { return standardised ? 4 : 8; }
+__host__ __device__ constexpr int to_threads(bool standardised) { return 32 * (16 + to_stats_warps(standardised) + 3); }
+constexpr int kToWBytes = 2 * kPanelBytes;     // [128 weight rows][128 k]
+constexpr int kToWExtra = 128 * 32;
 constexpr int kToStages = 2;
 constexpr int kToSlots = kToStages + 1;
-constexpr uint32_t kToColG = 0, kToColP = 144, kToColGram = 288;
+constexpr uint32_t kToColG = 0, kToColP = 128, kToColSet = 256;
 
+// a_ready, the correction rows and the scales of a stage are written anew for the tile two later, whose load waits for a_empty, which the
+// epilogue hands back when it has used them all.
 struct ToBars {
   uint64_t raw_full[kToStages], a_ready[kToStages], a_empty[kToStages];
-  uint64_t gram_full, gram_free, main_full, acc_full, acc_free, w_full;
+  uint64_t acc_full[2], acc_free[2], w_full;
   uint32_t tmem_base;
 };
 struct ToLayout {
-  static constexpr int wg = 0;                                  // gate weights | ones
-  static constexpr int wz = wg + kToWBytes;                     // projection weights | ones
+  static constexpr int wg = 0;                                  // gate weights
+  static constexpr int wz = wg + kToWBytes;                     // projection weights
   static constexpr int wxg = wz + kToWBytes;                    // correction panels (k 0..7: z, k 8..15: x)
   static constexpr int wxz = wxg + kToWExtra;
   static constexpr int zt = wxz + kToWExtra;                    // z tiles (later the output rows)
@@ -57,38 +59,32 @@ struct ToLayout {
 static_assert(ToLayout::zt % 1024 == 0 && ToLayout::xt % 1024 == 0, "tiles must keep the swizzle alignment");
 static_assert(ToLayout::total + 1024 <= 232448, "shared memory budget");
 
-// The resident weights: gate | projection, each with 16 rows of ones behind it, and their correction panels.  The gate rows carry
+// The resident weights: gate | projection, and their correction panels.  The gate rows carry
 // the 1/2 of sigmoid(x) = 1/2 + 1/2 tanh(x/2); the z statistics use k 0..7 of the correction step, the x statistics k 8..15.
 template <bool kF16>
 struct ToWeights {
   const float *ln_in_w, *ln_in_b, *ln_out_w, *ln_out_b;
   const bf16 *w_z, *w_g;
   static constexpr int kBytes = ToLayout::zt;
-  __device__ __forceinline__ void fold(unsigned char* sm, int, int warp, int warps, int lane, int tid, int threads) const {
-    fold_weight_rows<kF16, kF16>(sm + ToLayout::wg, sm + ToLayout::wxg, 0, kToWPanel, w_g, 0, 128, ln_in_w, ln_in_b, 0.5f, warp, warps,
+  static_assert(kBytes == 2 * (kToWBytes + kToWExtra), "no padding in the image");
+  __device__ __forceinline__ void fold(unsigned char* sm, int, int warp, int warps, int lane, int, int) const {
+    fold_weight_rows<kF16, kF16>(sm + ToLayout::wg, sm + ToLayout::wxg, 0, kPanelBytes, w_g, 0, 128, ln_in_w, ln_in_b, 0.5f, warp, warps,
                                  lane, 0);
-    fold_weight_rows<true, true>(sm + ToLayout::wz, sm + ToLayout::wxz, 0, kToWPanel, w_z, 0, 128, ln_out_w, ln_out_b, 1.0f, warp, warps,
+    fold_weight_rows<true, true>(sm + ToLayout::wz, sm + ToLayout::wxz, 0, kPanelBytes, w_z, 0, 128, ln_out_w, ln_out_b, 1.0f, warp, warps,
                                  lane, 1);
-    for (int i = tid; i < 2 * 2 * 16 * 8; i += threads) {   // rows of ones behind both weights
-      const int panel = i >> 7, piece = i & 127;
-      const uint32_t one = ones16x2(panel >= 2 || kF16);     // panels 0, 1: gate weights, 2, 3: projection
-      *reinterpret_cast<uint4*>(sm + ToLayout::wg + panel * kToWPanel + 128 * 128 + piece * 16) = make_uint4(one, one, one, one);
-    }
-    for (int i = tid; i < 2 * 16 * 2; i += threads)          // ... which take no correction
-      *reinterpret_cast<uint4*>(sm + ToLayout::wxg + (i >> 5) * kToWExtra + 128 * 32 + (i & 31) * 16) = make_uint4(0u, 0u, 0u, 0u);
-    for (int i = 2 * (kToWBytes + kToWExtra) + tid * 16; i < kBytes; i += threads * 16)   // padding up to the tiles
-      *reinterpret_cast<uint4*>(sm + i) = make_uint4(0u, 0u, 0u, 0u);
   }
 };
 
 template <typename Tz, bool kBulk>
-__global__ void __launch_bounds__(kToThreads, 1)
+__global__ void __launch_bounds__(to_threads(sizeof(Tz) != 2), 1)
 trimul_out_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_constant__ CUtensorMap map_x,
                      const __grid_constant__ CUtensorMap map_out, const Tz* __restrict__ z_in, Tz* __restrict__ z_out,
                      const ToWeights<sizeof(Tz) != 2> weights, const unsigned char* __restrict__ folded,
                      int n_i, int n, int add_residual, float eps, int tiles_j, int n_tiles) {
   constexpr bool kTma = sizeof(Tz) == 2;               // bf16: residual from the z tile, output through TMA
   constexpr bool kF16 = !kTma;                           // operand format of the z side; the x side is always fp16
+  constexpr int kStats = to_stats_warps(kF16), kThreads = to_threads(kF16), kLoad = 16 + kStats;   // kLoad: the producer's warp
+  constexpr int kSets = kTma ? 2 : 1;                    // sets of accumulators (two made no difference to fp32 rows)
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* sm = smem_aligned(smem_raw);
   ToBars& bars = *reinterpret_cast<ToBars*>(sm + ToLayout::bars);
@@ -102,27 +98,29 @@ trimul_out_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_con
   if (threadIdx.x == 0) {
     for (int s = 0; s < kToStages; ++s) {
       mbar_init(&bars.raw_full[s], 1);
-      mbar_init(&bars.a_ready[s], 4);
-      mbar_init(&bars.a_empty[s], 4);                      // three issuing threads and the store of the output rows
+      mbar_init(&bars.a_ready[s], kStats);
+      mbar_init(&bars.a_empty[s], 1);                      // the epilogue, which waits for everything else that reads the stage
     }
     mbar_init(&bars.w_full, 1);
-    mbar_init(&bars.gram_full, 1);
-    mbar_init(&bars.gram_free, 4);
-    mbar_init(&bars.main_full, 2);
-    mbar_init(&bars.acc_full, 2);
-    mbar_init(&bars.acc_free, 16);
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(&bars.acc_full[b], 2);
+      mbar_init(&bars.acc_free[b], 16);
+    }
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
-  if (warp == 20) {
+  if (warp == kLoad) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(&bars.tmem_base)),
                  "r"(512u)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
   }
-  for (int i = threadIdx.x; i < kToStages * 128 * 2; i += kToThreads)  // tile-side panels start out finite
-    *reinterpret_cast<uint4*>(sm + ToLayout::ax + i * 16) = make_uint4(0u, 0u, 0u, 0u);
+  if (kF16)                                                // standardised rows: known statistics of the z side, (0, 1)
+    for (int i = threadIdx.x; i < kToSlots * 128; i += kThreads) {
+      if (i < kToStages * 128) write_correction_row(sm + ToLayout::ax + (i >> 7) * 128 * 32, i & 127, 0.f, 1.f, false, 0, false);
+      reinterpret_cast<float2*>(sm + ToLayout::scale)[i].x = 1.f;
+    }
   asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-  if (!cta_ready(skip, warp == 20, bars.tmem_base, 512u, [&] {
+  if (!cta_ready(skip, warp == kLoad, bars.tmem_base, 512u, [&] {
         if (folded && threadIdx.x == 0) folded_load(sm, folded, ToWeights<kF16>::kBytes, &bars.w_full);
       }))
     return;
@@ -130,13 +128,16 @@ trimul_out_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_con
   const uint32_t tmem_base = bars.tmem_base;
   const int first_tile = blockIdx.x, tile_step = gridDim.x;
 
-  if (warp >= 20) {
-    if (warp == 20) {
+  if (warp >= kLoad) {
+    if (warp == kLoad) {
       // ---------------------------------------------------------------- tile producer: z (bf16 rows) and x
       int k = 0;
       for (int tile = first_tile; tile < n_tiles; tile += tile_step, ++k) {
         const int s = k % kToStages, m = k / kToStages;
         if (!mbar_wait_warp(&bars.a_empty[s], (m & 1) ^ 1, 1u)) break;
+        // Where rows are added in L2, a tile is asked for once the one before has arrived and been measured: loads that queue
+        // further ahead delay the additions (asked for with the stage: 553 -> 568 us at N = 1536, 247 -> 256 at 1024; below 500 level).
+        if (kBulk && add_residual && k && !mbar_wait_warp(&bars.a_ready[(k - 1) % kToStages], ((k - 1) / kToStages) & 1, 1u)) break;
         if (elect_lane()) {
           const int i = tile / tiles_j, j0 = (tile % tiles_j) * 128;
           mbar_expect_tx(&bars.raw_full[s], 2 * kOperandBytes);
@@ -159,53 +160,19 @@ trimul_out_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_con
         }
         __syncwarp();
       }
-    } else if (warp == 23) {
-      // ---------------------------------------------------------------- statistics products: Z Z^T, then X^T X
-      constexpr uint32_t idesc_z = umma_idesc_16(128, 128, kF16, kF16), idesc_x = umma_idesc_f16(128, 128, true, true);
-      int k = 0;
-      for (int tile = first_tile; tile < n_tiles; tile += tile_step, ++k) {
-        const int s = k % kToStages, m = k / kToStages;
-        // bf16 rows: two phases of the statistics accumulator per tile (z, then x); standardised rows have known
-        // statistics, so only x is measured and the phases alternate from tile to tile
-        if (!mbar_wait_warp(&bars.raw_full[s], m & 1, 2u) || !mbar_wait_warp(&bars.gram_free, kF16 ? ((k & 1) ^ 1) : 1u, 2u)) break;
-        tc_fence_after();
-        const uint32_t z_addr = smem_u32(sm + ToLayout::zt + s * kOperandBytes), x_addr = smem_u32(sm + ToLayout::xt + s * kOperandBytes);
-        if (!kF16) {
-          if (elect_lane()) {
-#pragma unroll
-            for (int ks = 0; ks < 8; ++ks) {
-              const uint64_t d = umma_desc_sw128(z_addr + (ks >> 2) * kPanelBytes) + 2 * (ks & 3);
-              umma_bf16(tmem_base + kToColGram, d, d, idesc_z, ks ? 1u : 0u);
-            }
-            umma_commit(&bars.gram_full);
-          }
-          __syncwarp();
-          if (!mbar_wait_warp(&bars.gram_free, 0u, 2u)) break;
-          tc_fence_after();
-        }
-        if (elect_lane()) {
-#pragma unroll
-          for (int ks = 0; ks < 8; ++ks) {
-            const uint64_t d = umma_desc_mn_sw128(x_addr + ks * 2048, kPanelBytes, 1024);
-            umma_bf16(tmem_base + kToColGram, d, d, idesc_x, ks ? 1u : 0u);
-          }
-          umma_commit(&bars.gram_full);
-          umma_commit(&bars.a_empty[s]);
-        }
-        __syncwarp();
-      }
     } else {
-      // ---------------------------------------------------------------- gate (warp 21) / projection (warp 22) product
-      const bool proj = warp == 22;
-      const uint32_t idesc = proj ? umma_idesc_f16(128, 144, true, false) : umma_idesc_16(128, 144, kF16, kF16);
+      // ---------------------------------------------------------------- gate / projection product
+      const bool proj = warp == kLoad + 2;
+      const uint32_t idesc = proj ? umma_idesc_f16(128, 128, true, false) : umma_idesc_16(128, 128, kF16, kF16);
       const uint32_t d_tmem = tmem_base + (proj ? kToColP : kToColG);
       const uint32_t w_addr = smem_u32(sm + (proj ? ToLayout::wz : ToLayout::wg));
       const uint64_t wx_desc = umma_desc_sw32(smem_u32(sm + (proj ? ToLayout::wxz : ToLayout::wxg)));
       int k = 0;
       const bool have_w = mbar_wait_warp(&bars.w_full, 0, 4u);   // the resident weights
       for (int tile = first_tile; tile < n_tiles && have_w; tile += tile_step, ++k) {
-        const int s = k % kToStages, m = k / kToStages;
-        if (!mbar_wait_warp(&bars.raw_full[s], m & 1, 4u) || !mbar_wait_warp(&bars.acc_free, (k & 1) ^ 1, 8u)) break;
+        const int s = k % kToStages, m = k / kToStages, b = k % kSets;
+        const uint32_t d = d_tmem + b * kToColSet;
+        if (!mbar_wait_warp(&bars.raw_full[s], m & 1, 4u) || !mbar_wait_warp(&bars.acc_free[b], ((k / kSets) & 1) ^ 1, 8u)) break;
         tc_fence_after();
         if (elect_lane()) {
           const uint32_t a_addr = smem_u32(sm + (proj ? ToLayout::xt : ToLayout::zt) + s * kOperandBytes);
@@ -213,69 +180,70 @@ trimul_out_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_con
           for (int ks = 0; ks < 8; ++ks) {
             const uint64_t a_desc = proj ? umma_desc_mn_sw128(a_addr + ks * 2048, kPanelBytes, 1024)
                                          : umma_desc_sw128(a_addr + (ks >> 2) * kPanelBytes) + 2 * (ks & 3);
-            umma_bf16(d_tmem, a_desc, umma_desc_sw128(w_addr + (ks >> 2) * kToWPanel) + 2 * (ks & 3), idesc, ks ? 1u : 0u);
+            umma_bf16(d, a_desc, umma_desc_sw128(w_addr + (ks >> 2) * kPanelBytes) + 2 * (ks & 3), idesc, ks ? 1u : 0u);
           }
-          umma_commit(&bars.main_full);                      // the sums (columns 128..143) are there
         }
         __syncwarp();
         if (!mbar_wait_warp(&bars.a_ready[s], m & 1, 4u)) break;   // the correction step needs the statistics
         tc_fence_after();
         if (elect_lane()) {
-          umma_bf16(d_tmem, umma_desc_sw32(smem_u32(sm + ToLayout::ax + s * 128 * 32)), wx_desc,
-                    umma_idesc_bf16(128, 144, false, false), 1u);
-          umma_commit(&bars.acc_full);
-          umma_commit(&bars.a_empty[s]);
+          umma_bf16(d, umma_desc_sw32(smem_u32(sm + ToLayout::ax + s * 128 * 32)), wx_desc, umma_idesc_bf16(128, 128, false, false),
+                    1u);
+          umma_commit(&bars.acc_full[b]);
         }
         __syncwarp();
       }
     }
   } else if (warp >= 16) {
-    // ------------------------------------------------------------------ row statistics, one thread per row
-    const int qw = warp - 16, r = 32 * qw + lane;
-    const uint32_t lane_addr = tmem_base + ((uint32_t)(32 * qw) << 16);
-    float2* scale = reinterpret_cast<float2*>(sm + ToLayout::scale);
+    // ------------------------------------------------------------------ row statistics
+    // z: two lanes a row.  x, whose rows lie across the tile ([128 c][64 j] a panel): a lane sums two neighbouring j over the
+    // channels 8 i + 2 (lane / 8) and the one behind, so that a warp's load meets every bank once, and four lanes add up.
+    const int sw = warp - 16;
+    float* scale = reinterpret_cast<float*>(sm + ToLayout::scale);
     int k = 0;
-    bool ok = true;
     for (int tile = first_tile; tile < n_tiles; tile += tile_step, ++k) {
       const int s = k % kToStages;
-      float sumsq[2] = {0.f, 0.f};
-#pragma unroll
-      for (int which = kF16 ? 1 : 0; which < 2; ++which) {   // 0: z (bf16 rows only), 1: x
-        ok = mbar_wait(&bars.gram_full, kF16 ? (k & 1) : which, 16u);
-        ok = __all_sync(0xffffffffu, ok);
-        if (!ok) break;
-        tc_fence_after();
-        uint32_t diag[32];
-        tmem_ld32(lane_addr + kToColGram + 32 * qw, diag);
-        tmem_wait_ld();
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&bars.gram_free);
-        sumsq[which] = select_own(diag, lane);
-      }
-      if (!ok) break;
-      ok = mbar_wait(&bars.main_full, k & 1, 16u);
-      ok = __all_sync(0xffffffffu, ok);
-      if (!ok) break;
-      tc_fence_after();
-      uint32_t sz[16], sx[16];
-      tmem_ld16(lane_addr + kToColG + 128, sz);
-      tmem_ld16(lane_addr + kToColP + 128, sx);
-      tmem_wait_ld();
-      tc_fence_before();
-      float rstd[2];
-#pragma unroll
-      for (int which = 0; which < 2; ++which) {
-        float mean = __uint_as_float(which ? sx[0] : sz[0]) * (1.0f / kC);
-        const float var = fmaxf(sumsq[which] * (1.0f / kC) - mean * mean, 0.f);
-        const float e = which ? eps * (PX_TRIMUL_X_SCALE * PX_TRIMUL_X_SCALE) : eps;   // x arrives scaled
-        float std = sqrtf(var + e);
-        rstd[which] = rsqrtf(var + e);
-        if (kF16 && which == 0) mean = 0.f, std = 1.f, rstd[0] = 1.f;   // standardised rows: known statistics
+      if (!mbar_wait_warp(&bars.raw_full[s], (k / kToStages) & 1, 16u)) break;
+      unsigned char* ax = sm + ToLayout::ax + s * 128 * 32;
+      float* sc = scale + (k % kToSlots) * 256;
+      if (!kF16) {
+        const int r = 16 * sw + (lane >> 1), half = lane & 1;
+        float mean, var;
+        bf16_row_stats(sm + ToLayout::zt + s * kOperandBytes, r, half, mean, var);
         // rstd * (W'x - mean * s + std * t): the row side of the correction step holds (-mean, std)
-        write_correction_row(sm + ToLayout::ax + s * 128 * 32, r, -mean, std, false, which, false);
+        if (half == 0) {
+          write_correction_row(ax, r, -mean, sqrtf(var + eps), false, 0, false);
+          sc[2 * r] = rsqrtf(var + eps);
+        }
       }
-      scale[(k % kToSlots) * 128 + r] = make_float2(rstd[0], rstd[1]);
+#pragma unroll 1
+      for (int r0 = 16 * sw; r0 < 128; r0 += 16 * kStats) {
+        const unsigned char* x = sm + ToLayout::xt + s * kOperandBytes + (r0 >> 6) * kPanelBytes + (lane & 3) * 4;
+        const int piece = ((r0 & 63) >> 3) + ((lane >> 2) & 1), c0 = 2 * (lane >> 3);
+        const auto pair = [&](int c) { return unpack_f16x2(*reinterpret_cast<const uint32_t*>(x + c * 128 + ((piece ^ (c & 7)) << 4))); };
+        const float2 x0 = pair(0);                         // about one of its values, nothing cancels
+        float s0 = 0.f, s1 = 0.f, q0 = 0.f, q1 = 0.f;
+#pragma unroll
+        for (int i = 0; i < 32; ++i) {
+          float2 d = pair(8 * (i >> 1) + c0 + (i & 1));
+          add2(d.x, d.y, -x0.x, -x0.y);
+          add2(s0, s1, d.x, d.y);
+          fma2(q0, q1, d.x, d.y, d.x, d.y, q0, q1);
+        }
+#pragma unroll
+        for (int o = 8; o < 32; o *= 2) {
+          add2(s0, s1, __shfl_xor_sync(0xffffffffu, s0, o), __shfl_xor_sync(0xffffffffu, s1, o));
+          add2(q0, q1, __shfl_xor_sync(0xffffffffu, q0, o), __shfl_xor_sync(0xffffffffu, q1, o));
+        }
+        if (lane < 16) {
+          const bool odd = lane >= 8;
+          const int r = r0 + 2 * (lane & 7) + odd;
+          const float m = (odd ? s1 : s0) * (1.0f / kC), var = fmaxf((odd ? q1 : q0) * (1.0f / kC) - m * m, 0.f);
+          const float e = eps * (PX_TRIMUL_X_SCALE * PX_TRIMUL_X_SCALE);   // x arrives scaled
+          write_correction_row(ax, r, -((odd ? x0.y : x0.x) + m), sqrtf(var + e), false, 1, false);
+          sc[2 * r + 1] = rsqrtf(var + e);
+        }
+      }
       asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
       __syncwarp();
       if (lane == 0) mbar_arrive(&bars.a_ready[s]);
@@ -304,19 +272,20 @@ trimul_out_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_con
             asm volatile("prefetch.global.L2 [%0];\n" ::"l"(reinterpret_cast<const float*>(z_in) + ((size_t)i2 * n + j2) * kC + 32 * part));
         }
       }
-      ok = mbar_wait(&bars.acc_full, k & 1, 32u);
+      const int b = k % kSets;
+      ok = mbar_wait(&bars.acc_full[b], (k / kSets) & 1, 32u);
       ok = named_barrier_all(1, 512, ok);                  // all sixteen warps go on, or none
       if (!ok) break;
       tc_fence_after();
       const float2 sc = reinterpret_cast<const float2*>(sm + ToLayout::scale)[(k % kToSlots) * 128 + row];
       unsigned char* ztile = sm + ToLayout::zt + s * kOperandBytes;
       uint32_t g[32], p[32];
-      tmem_ld32(lane_addr + kToColG + 32 * part, g);
-      tmem_ld32(lane_addr + kToColP + 32 * part, p);
+      tmem_ld32(lane_addr + b * kToColSet + kToColG + 32 * part, g);
+      tmem_ld32(lane_addr + b * kToColSet + kToColP + 32 * part, p);
       tmem_wait_ld();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&bars.acc_free);          // this warp has read its part of the accumulators
+      if (lane == 0) mbar_arrive(&bars.acc_free[b]);          // this warp has read its part of the accumulators
       float v[32];
 #pragma unroll
       for (int e = 0; e < 32; ++e) {
@@ -373,7 +342,7 @@ trimul_out_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_con
 
   tc_fence_before();
   cta_teardown_sync();
-  if (warp == 20) {
+  if (warp == kLoad) {
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem_base), "r"(512u) : "memory");
   }
@@ -413,7 +382,7 @@ static int32_t launch_trimul_out(const px_f16* x, const void* z_in, const px_f16
   const int64_t tiles_j = (n + 127) / 128, n_tiles = tiles_j * n_i;
   if (n_tiles > 0x7fffffff) return PX_ERR_UNSUPPORTED;
   const int grid = even_grid(n_tiles, sm_count());
-  return launch_pdl(trimul_out_tc_kernel<Tz, kBulk>, dim3(grid), kToThreads, smem, st, mz, mx, mout, (const Tz*)z_in, (Tz*)z_out, weights,
+  return launch_pdl(trimul_out_tc_kernel<Tz, kBulk>, dim3(grid), to_threads(sizeof(Tz) != 2), smem, st, mz, mx, mout, (const Tz*)z_in, (Tz*)z_out, weights,
                     (const unsigned char*)folded, (int)n_i, (int)n, (int)add_residual, eps, (int)tiles_j, (int)n_tiles)
              ? PX_OK
              : PX_ERR_LAUNCH;
