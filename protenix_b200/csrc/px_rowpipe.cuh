@@ -278,8 +278,12 @@ __device__ __forceinline__ void bf16_row_stats(const unsigned char* tile, int r,
 // The statistics warps (`sw` = 0..3, or 0..7 for bf16 rows).  per_row(k, u, t, r, rstd) is called once per
 // tile and row with the row's 1/std, before a_ready is signalled.  `kStandardised`: the rows are a standardised copy
 // (mean 0, deviation 1 by construction), so the correction row is (0, 1), written once, and the factor is 1.
-template <typename Ctx, typename PerRow>
-__device__ __forceinline__ void tile_stats_loop(const Ctx& c, float eps, int sw, int lane, PerRow per_row) {
+// after(u, t) follows once the stage and the statistics have been handed over: for what nothing in the kernel waits for.
+struct TileNothingAfter {
+  __device__ __forceinline__ void operator()(int, int) const {}
+};
+template <typename Ctx, typename PerRow, typename After = TileNothingAfter>
+__device__ __forceinline__ void tile_stats_loop(const Ctx& c, float eps, int sw, int lane, PerRow per_row, After after = After()) {
   constexpr bool kStandardised = Ctx::kStandardised;
   const int r = kStandardised ? 32 * sw + lane : 16 * sw + (lane >> 1), half = lane & 1;
   int k = 0;
@@ -304,6 +308,7 @@ __device__ __forceinline__ void tile_stats_loop(const Ctx& c, float eps, int sw,
       mbar_arrive(&c.bars->a_ready[k % Ctx::kSlots]);
       mbar_arrive(&c.bars->a_empty[s]);                 // after the last use of what was read from the stage
     }
+    if (kStandardised || half == 0) after(u, t);
   }
 }
 

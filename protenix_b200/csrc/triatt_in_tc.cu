@@ -138,17 +138,22 @@ triatt_in_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_cons
                         umma_idesc_16(128, 80, kF16, kF16), &bars.w_full, bars.acc_full[1], bars.acc_free[1], 2, 256);
     }
   } else if (warp >= 16) {
-    // ------------------------------------------------------------------ row statistics, one thread per row
+    // ------------------------------------------------------------------ row statistics (tile_stats_loop) and mask bias
+    // The mask bias comes after the hand-over: its load of the mask, up to 2 us from memory, otherwise holds up both the products and
+    // the stage of every tile.  bf16, starting node: 40.0 -> 33.5 us at N = 384, 147 -> 120 at 768, 592 -> 465 at 1536; ending node
+    // (a sector of the mask serves eight u) 35.9 -> 33.8, 125 -> 123 and 494 -> 479; N = 128 9.4 -> 9.0.
     float2* scale = reinterpret_cast<float2*>(sm + AiLayout<kF16>::scale);
-    tile_stats_loop(ctx, eps, warp - 16, lane, [&](int k, int u, int t, int r, float rstd) {
-      scale[(k % Ctx::kSlots) * 128 + r] = make_float2(rstd, t < n ? rstd : 0.f);
-      if (hpair == 0 && t < ldm) {                       // mask bias, -inf in the pad columns [n, ldm)
-        float mv = -CUDART_INF_F;
-        if (t < n)
-          mv = mask ? (__ldg(mask + (swap ? ((size_t)t * n_u + u) : ((size_t)u * n + t))) - 1.0f) * inf * kLog2e : 0.f;
-        mb_out[(size_t)u * ldm + t] = mv;
-      }
-    });
+    tile_stats_loop(
+        ctx, eps, warp - 16, lane,
+        [&](int k, int, int t, int r, float rstd) { scale[(k % Ctx::kSlots) * 128 + r] = make_float2(rstd, t < n ? rstd : 0.f); },
+        [&](int u, int t) {
+          if (hpair == 0 && t < ldm) {                   // mask bias, -inf in the pad columns [n, ldm)
+            float mv = -CUDART_INF_F;
+            if (t < n)
+              mv = mask ? (__ldg(mask + (swap ? ((size_t)t * n_u + u) : ((size_t)u * n + t))) - 1.0f) * inf * kLog2e : 0.f;
+            mb_out[(size_t)u * ldm + t] = mv;
+          }
+        });
   } else if (warp < 8) {
     // ------------------------------------------------------------------ epilogue of q | k
     const int which = warp >> 2, qw = warp & 3;          // 0: q, 1: k
