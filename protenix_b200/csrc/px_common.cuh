@@ -148,6 +148,19 @@ static inline int sm_count() {
   return cached[dev];
 }
 
+// Size of the current device's L2 in bytes (cached per device ordinal).
+static inline int64_t l2_bytes() {
+  static int cached[64] = {};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 126 << 20;
+  if (!cached[dev]) {
+    int n = 0;
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrL2CacheSize, dev) != cudaSuccess || n <= 0) n = 126 << 20;
+    cached[dev] = n;
+  }
+  return cached[dev];
+}
+
 // CTAs (or pairs of them) of a persistent kernel that deals out `tiles` in turn: as few of the `room` that fit as end with the same
 // number of tiles each.  The others would only end a tile earlier, and they keep CTAs of another stream (the single branch) from
 // the SMs and ask L2 for more at once: pair path at N = 200 249 -> 246 us a block, with the single branch beside it 288 -> 285.

@@ -186,7 +186,8 @@ __device__ __forceinline__ void named_barrier(int id, int threads) {
 //     now hold a second set of accumulators for bf16 rows, too.
 // What bounds these kernels from N = 384 on is the way of a tile from memory, 2 us under load: three stages where they fit
 // (with the statistics as they are now; projections of the triangle multiplication, bf16 N = 768 132 -> 117 us, N = 437 55.3 -> 47.5;
-// fp16 N = 384 in a stack 36.4 -> 31.8; two stages and a second staging buffer 148 at N = 768 where three took 136).
+// fp16 N = 384 in a stack 36.4 -> 31.8; two stages and a second staging buffer 148 at N = 768 where three took 136).  The projections of
+// the triangle attention, which write three times what they read, take two from the size on where the rows exceed L2 (triatt_in_tc.cu).
 // ---------------------------------------------------------------------------------------------------------------
 constexpr int kTileBytes = kOperandBytes;
 constexpr int kTileExtra = 128 * 32;           // [128 rows][16 k] correction panel

@@ -26,19 +26,19 @@ constexpr int kAiH = 4, kAiD = 32;
 constexpr int kAiW1Panel = 80 * 128;           // [v 64 | bias 16][64 k]
 constexpr int kAiStageOut = 32 * 256;          // [32 d][128 t] fp16: one head
 constexpr int ai_threads(bool f16) { return 32 * (16 + tile_stats_warps(f16) + 3); }
-constexpr int ai_stages(bool f16) { return f16 ? 3 : 2; }     // what shared memory holds: standardised rows need one correction panel
+// Stages of the row-tile ring: two, or three where shared memory holds them, which is where the rows are standardised ones (they need
+// one correction panel).  Which: triatt_in_stages.
 // tensor memory: q|k (128) | v|bias (80) | -, twice
 
-template <bool kF16>
+template <int kStages>
 struct AiBars {
-  TileBars<ai_stages(kF16)> tile;
+  TileBars<kStages> tile;
   uint64_t acc_full[2][2], acc_free[2][2];   // [product][accumulator]
   uint64_t w_full;
   uint32_t tmem_base;
 };
-template <bool kF16>
+template <bool kF16, int kStages>
 struct AiLayout {
-  static constexpr int kStages = ai_stages(kF16);
   static constexpr int w0 = 0;                                  // [q 64 | k 64][128 k]
   static constexpr int w1 = w0 + kOperandBytes;                 // [v 64 | bias 16][128 k]
   static constexpr int wx0 = w1 + 2 * kAiW1Panel;               // correction panels
@@ -49,19 +49,19 @@ struct AiLayout {
   static constexpr int qk = out + 2 * kAiStageOut;              // q, k staging: 8 warps x 2 heads x [32 t][32] fp16
   static constexpr int scale = qk + 8 * 2 * 2048;               // float2 (rstd, rstd or 0 beyond n) per row and slot
   static constexpr int bars = scale + tile_slots(kStages) * 128 * 8;
-  static constexpr int total = bars + (int)sizeof(AiBars<kF16>);
+  static constexpr int total = bars + (int)sizeof(AiBars<kStages>);
 };
-static_assert(AiLayout<true>::total + 1024 <= 232448 && AiLayout<false>::total + 1024 <= 232448, "shared memory budget");
-static_assert(AiLayout<true>::a % 1024 == 0, "tile ring must keep the swizzle alignment");
+static_assert(AiLayout<true, 3>::total + 1024 <= 232448 && AiLayout<false, 2>::total + 1024 <= 232448, "shared memory budget");
+static_assert(AiLayout<true, 3>::a % 1024 == 0, "tile ring must keep the swizzle alignment");
 
 // The resident weights of a CTA (variant: which pair of heads): q carries the softmax scale, the bias rows log2(e).
 template <bool kF16>
 struct AiWeights {
   const float *ln_w, *ln_b;
   const bf16 *q, *k, *v, *bias;
-  static constexpr int kBytes = AiLayout<kF16>::a;
+  static constexpr int kBytes = AiLayout<kF16, 2>::a;          // the ring lies behind the weights, however many stages it has
   __device__ __forceinline__ void fold(unsigned char* sm, int hpair, int warp, int warps, int lane, int tid, int threads) const {
-    unsigned char *w0 = sm + AiLayout<kF16>::w0, *w1 = sm + AiLayout<kF16>::w1, *wx0 = sm + AiLayout<kF16>::wx0, *wx1 = sm + AiLayout<kF16>::wx1;
+    unsigned char *w0 = sm + AiLayout<kF16, 2>::w0, *w1 = sm + AiLayout<kF16, 2>::w1, *wx0 = sm + AiLayout<kF16, 2>::wx0, *wx1 = sm + AiLayout<kF16, 2>::wx1;
     const float qscale = kLog2e * rsqrtf((float)kAiD);
     fold_weight_rows<kF16, kF16>(w0, wx0, 0, kPanelBytes, q, 64 * hpair, 64, ln_w, ln_b, qscale, warp, warps, lane);
     fold_weight_rows<kF16, kF16>(w0, wx0, 64, kPanelBytes, k, 64 * hpair, 64, ln_w, ln_b, 1.0f, warp, warps, lane);
@@ -75,23 +75,24 @@ struct AiWeights {
 };
 
 // kF16: the rows are the standardised fp16 copy of an fp32 pair tensor (fp16 weights); otherwise bf16 rows of z.
-template <bool kF16>
+template <bool kF16, int kStages>
 __global__ void __launch_bounds__(ai_threads(kF16), 1)
 triatt_in_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_constant__ CUtensorMap map_v,
                     const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k, const float* __restrict__ mask,
                     const AiWeights<kF16> weights, const unsigned char* __restrict__ folded,
                     float* __restrict__ bias_out, float* __restrict__ mb_out, int n_u, int n,
                     int ldm, int swap, float eps, float inf, int tiles_t, int n_tiles) {
+  typedef AiLayout<kF16, kStages> Layout;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* sm = smem_aligned(smem_raw);
-  AiBars<kF16>& bars = *reinterpret_cast<AiBars<kF16>*>(sm + AiLayout<kF16>::bars);
+  AiBars<kStages>& bars = *reinterpret_cast<AiBars<kStages>*>(sm + Layout::bars);
   const int warp = warp_index(), lane = threadIdx.x & 31;
   const int hpair = blockIdx.x & 1;                      // this CTA's heads: 2*hpair, 2*hpair + 1
-  typedef TileCtx<ai_stages(kF16), kF16> Ctx;
+  typedef TileCtx<kStages, kF16> Ctx;
   constexpr int kCtl = 16 + tile_stats_warps(kF16);      // first control warp
   Ctx ctx;
-  ctx.tiles = sm + AiLayout<kF16>::a;
-  ctx.extras = sm + AiLayout<kF16>::ax;
+  ctx.tiles = sm + Layout::a;
+  ctx.extras = sm + Layout::ax;
   ctx.bars = &bars.tile;
   ctx.first_tile = blockIdx.x >> 1;
   ctx.tile_step = gridDim.x >> 1;
@@ -131,10 +132,10 @@ triatt_in_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_cons
     if (warp == kCtl) {
       tile_producer_loop(ctx, &map_z);
     } else if (warp == kCtl + 1) {
-      tile_product_loop(ctx, tmem_base, smem_u32(sm + AiLayout<kF16>::w0), kPanelBytes, smem_u32(sm + AiLayout<kF16>::wx0),
+      tile_product_loop(ctx, tmem_base, smem_u32(sm + Layout::w0), kPanelBytes, smem_u32(sm + Layout::wx0),
                         umma_idesc_16(128, 128, kF16, kF16), &bars.w_full, bars.acc_full[0], bars.acc_free[0], 2, 256);
     } else {
-      tile_product_loop(ctx, tmem_base + 128, smem_u32(sm + AiLayout<kF16>::w1), kAiW1Panel, smem_u32(sm + AiLayout<kF16>::wx1),
+      tile_product_loop(ctx, tmem_base + 128, smem_u32(sm + Layout::w1), kAiW1Panel, smem_u32(sm + Layout::wx1),
                         umma_idesc_16(128, 80, kF16, kF16), &bars.w_full, bars.acc_full[1], bars.acc_free[1], 2, 256);
     }
   } else if (warp >= 16) {
@@ -142,7 +143,7 @@ triatt_in_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_cons
     // The mask bias comes after the hand-over: its load of the mask, up to 2 us from memory, otherwise holds up both the products and
     // the stage of every tile.  bf16, starting node: 40.0 -> 33.5 us at N = 384, 147 -> 120 at 768, 592 -> 465 at 1536; ending node
     // (a sector of the mask serves eight u) 35.9 -> 33.8, 125 -> 123 and 494 -> 479; N = 128 9.4 -> 9.0.
-    float2* scale = reinterpret_cast<float2*>(sm + AiLayout<kF16>::scale);
+    float2* scale = reinterpret_cast<float2*>(sm + Layout::scale);
     tile_stats_loop(
         ctx, eps, warp - 16, lane,
         [&](int k, int, int t, int r, float rstd) { scale[(k % Ctx::kSlots) * 128 + r] = make_float2(rstd, t < n ? rstd : 0.f); },
@@ -159,7 +160,7 @@ triatt_in_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_cons
     const int which = warp >> 2, qw = warp & 3;          // 0: q, 1: k
     const int row = 32 * qw + lane;
     const uint32_t t_acc = tmem_base + ((uint32_t)(32 * qw) << 16) + 64 * which;
-    unsigned char* stage = sm + AiLayout<kF16>::qk + warp * 4096;
+    unsigned char* stage = sm + Layout::qk + warp * 4096;
     int k = 0;
     for (int tile = ctx.first_tile; tile < n_tiles; tile += ctx.tile_step, ++k) {
       const int u = tile / tiles_t, tw = (tile % tiles_t) * 128 + 32 * qw;   // the warp's first row
@@ -168,7 +169,7 @@ triatt_in_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_cons
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
       tc_fence_after();
-      const float rstd = reinterpret_cast<const float2*>(sm + AiLayout<kF16>::scale)[(k % Ctx::kSlots) * 128 + row].x;
+      const float rstd = reinterpret_cast<const float2*>(sm + Layout::scale)[(k % Ctx::kSlots) * 128 + row].x;
       uint32_t h0[32], h1[32];
       tmem_ld32(t_acc + 256 * ab, h0);
       tmem_ld32(t_acc + 256 * ab + 32, h1);
@@ -208,7 +209,7 @@ triatt_in_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_cons
     for (int tile = ctx.first_tile; tile < n_tiles && ok; tile += ctx.tile_step, ++k) {
       const int u = tile / tiles_t, t0 = (tile % tiles_t) * 128, t = t0 + row;
       const int ab = k & 1, an = k >> 1;
-      unsigned char* const area = sm + AiLayout<kF16>::out + half * kAiStageOut;
+      unsigned char* const area = sm + Layout::out + half * kAiStageOut;
       unsigned char* const stage = area + row * 2;
       ok = mbar_wait(&bars.acc_full[1][ab], an & 1, 64u);
       // the store that last read the staging area (one tile ago) must be through with it
@@ -216,7 +217,7 @@ triatt_in_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_cons
       ok = named_barrier_all(1 + half, 128, ok);           // all four warps go on, or none
       if (!ok) break;
       tc_fence_after();
-      const float2 sc = reinterpret_cast<const float2*>(sm + AiLayout<kF16>::scale)[(k % Ctx::kSlots) * 128 + row];
+      const float2 sc = reinterpret_cast<const float2*>(sm + Layout::scale)[(k % Ctx::kSlots) * 128 + row];
       uint32_t v[32], b[16];
       tmem_ld32(t_acc + 256 * ab, v);
       if (half == 0) tmem_ld16(tmem_base + ((uint32_t)(32 * qw) << 16) + 256 * ab + 128 + 64, b);
@@ -252,7 +253,7 @@ triatt_in_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_cons
 
 PX_DEFINE_FAMILY_HOOKS(triatt_in)
 
-template <bool kF16>
+template <bool kF16, int kStages>
 static int32_t launch_triatt_in(const void* z, const float* mask, const AiWeights<kF16>& weights, const void* folded,
                                 px_f16* q, px_f16* k, px_f16* v, float* bias, float* mask_bias, int64_t n_u,
                                 int64_t n, int64_t ldm, int32_t ending, float eps, float inf, cudaStream_t st) {
@@ -274,19 +275,28 @@ static int32_t launch_triatt_in(const void* z, const float* mask, const AiWeight
     if (!make_map_3d(i ? &mk : &mq, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, i ? k : q, kAiD, (uint64_t)n, (uint64_t)n_u * kAiH, kAiD * 2,
                      (uint64_t)n * kAiD * 2, kAiD, 32, CU_TENSOR_MAP_SWIZZLE_64B))
       return PX_ERR_LAUNCH;
-  const size_t smem = AiLayout<kF16>::total + 1024;
+  const size_t smem = AiLayout<kF16, kStages>::total + 1024;
   static SmemLimit limit;
-  if (!limit.set(triatt_in_tc_kernel<kF16>, smem)) return PX_ERR_LAUNCH;
+  if (!limit.set(triatt_in_tc_kernel<kF16, kStages>, smem)) return PX_ERR_LAUNCH;
   const int64_t tiles_t = (n + 127) / 128, n_tiles = tiles_t * n_u;   // 128-wide tiles cover the pad columns up to ldm
   if (n_tiles > 0x7fffffff) return PX_ERR_UNSUPPORTED;
   const int pairs = even_grid(n_tiles, sm_count() / 2);
-  return launch_pdl(triatt_in_tc_kernel<kF16>, dim3(2 * pairs), ai_threads(kF16), smem, st, mz, mv, mq, mk, mask, weights,
+  return launch_pdl(triatt_in_tc_kernel<kF16, kStages>, dim3(2 * pairs), ai_threads(kF16), smem, st, mz, mv, mq, mk, mask, weights,
                     (const unsigned char*)folded, bias, mask_bias, (int)n_u, (int)n, (int)ldm, (int)ending, eps, inf, (int)tiles_t,
                     (int)n_tiles)
              ? PX_OK
              : PX_ERR_LAUNCH;
 }
 
+// Stages for the standardised rows of an fp32 pair tensor.  Three let the two CTAs of a pair drift apart, and once the rows are larger than
+// L2 the second one finds its tile gone: N = 1024, starting node, 390 MB read from memory where two stages read 273.
+// Two | three, us: starting node N = 437 39.8 | 39.2, 576 64.3 | 63.7, 640 74.9 | 77.2, 704 95.5 | 95.7, 768 107 | 114, 1024 187 | 213,
+// 1536 425 | 512; ending node, whose tiles take 256 bytes from each of 128 places, 512 52.4 | 48.4, 704 103 | 89, 768 117 | 116,
+// 832 143 | 130, 896 156 | 162, 1024 207 | 224, 1536 468 | 568.  L2 holds the rows of 704 tokens, two thirds of those of 862.
+// (One instantiation each: a count known at run time only cost 0.1 us a launch.)
+static int triatt_in_stages(int64_t n_u, int64_t n, int32_t ending) {
+  return n_u * n * (2 * kC) > (ending ? l2_bytes() * 3 / 2 : l2_bytes()) ? 2 : 3;
+}
 static bool triatt_in_args_ok(const void* z, const void* q, const void* k, const void* v, const float* bias, const float* mask_bias,
                               int64_t n_u, int64_t n_t, int64_t ldm) {
   return z && q && k && v && bias && mask_bias && n_u > 0 && n_t > 0 && n_u <= 32768 && n_t <= 32768 && ldm == px_ld_mask(n_t) &&
@@ -325,9 +335,10 @@ extern "C" int32_t px_triatt_in_proj_folded(const void* z, int32_t z_dtype, cons
   if (!triatt_in_args_ok(z, q, k, v, bias, mask_bias, n_u, n_t, ldm) || !folded || ((uintptr_t)folded & 15)) return PX_ERR_BAD_ARG;
   cudaStream_t st = (cudaStream_t)stream;
   if (z_dtype == PX_F16)
-    return launch_triatt_in<true>(z, mask, AiWeights<true>{}, folded, q, k, v, bias, mask_bias, n_u, n_t, ldm, ending, eps, inf, st);
+    return (triatt_in_stages(n_u, n_t, ending) == 2 ? launch_triatt_in<true, 2> : launch_triatt_in<true, 3>)(
+        z, mask, AiWeights<true>{}, folded, q, k, v, bias, mask_bias, n_u, n_t, ldm, ending, eps, inf, st);
   if (z_dtype == PX_BF16)
-    return launch_triatt_in<false>(z, mask, AiWeights<false>{}, folded, q, k, v, bias, mask_bias, n_u, n_t, ldm, ending, eps, inf, st);
+    return launch_triatt_in<false, 2>(z, mask, AiWeights<false>{}, folded, q, k, v, bias, mask_bias, n_u, n_t, ldm, ending, eps, inf, st);
   return PX_ERR_UNSUPPORTED;
 }
 
@@ -340,10 +351,10 @@ extern "C" int32_t px_triatt_in_proj(const void* z, int32_t z_dtype, const float
     return PX_ERR_BAD_ARG;
   cudaStream_t st = (cudaStream_t)stream;
   if (z_dtype == PX_F16)   // standardised rows of an fp32 pair tensor (px_standardise_rows)
-    return launch_triatt_in<true>(z, mask, ai_weights<true>(ln_w, ln_b, w_q, w_k, w_v, w_bias), nullptr, q, k, v, bias, mask_bias, n_u,
-                                  n_t, ldm, ending, eps, inf, st);
+    return (triatt_in_stages(n_u, n_t, ending) == 2 ? launch_triatt_in<true, 2> : launch_triatt_in<true, 3>)(
+        z, mask, ai_weights<true>(ln_w, ln_b, w_q, w_k, w_v, w_bias), nullptr, q, k, v, bias, mask_bias, n_u, n_t, ldm, ending, eps, inf, st);
   if (z_dtype == PX_BF16)
-    return launch_triatt_in<false>(z, mask, ai_weights<false>(ln_w, ln_b, w_q, w_k, w_v, w_bias), nullptr, q, k, v, bias, mask_bias, n_u,
-                                   n_t, ldm, ending, eps, inf, st);
+    return launch_triatt_in<false, 2>(z, mask, ai_weights<false>(ln_w, ln_b, w_q, w_k, w_v, w_bias), nullptr, q, k, v, bias, mask_bias, n_u,
+                                      n_t, ldm, ending, eps, inf, st);
   return PX_ERR_UNSUPPORTED;
 }

@@ -44,3 +44,20 @@ def test_triatt_in(n_u, n_t, ending, dtype):
     # the mask bias is exact for masks of zeros and ones
     assert torch.equal(mb[:, :n_t], torch.where(m > 0, 0.0, torch.tensor(-1e9, device="cuda") * torch.tensor(LOG2E, device="cuda")))
     assert bool((mb[:, n_t:] == -math.inf).all()) and not bool(bias[..., n_t:].any()) and not bool(v[..., n_t:].any())
+
+
+@pytest.mark.parametrize("ending", [False, True])
+def test_rows_beyond_l2_equal_a_slab(ending):
+    """More rows than L2 holds are loaded with fewer tiles on their way; each u is computed by itself, so a slab of them gives the same
+    bits."""
+    l2 = torch.cuda.get_device_properties(0).L2_cache_size
+    n_t = 500
+    n_u = -(-(3 * l2 // 2) // (n_t * 256)) + 5
+    z, mask, w = inputs(n_u, n_t, torch.float32, ending)
+    whole = ops.triatt_in_proj(z, mask, *w, ending=ending)
+    for u0 in (0, n_u // 2, n_u - 3):
+        part = (slice(None), slice(u0, u0 + 3)) if ending else (slice(u0, u0 + 3),)
+        slab = ops.triatt_in_proj(z[part].contiguous(), mask[part].contiguous(), *w, ending=ending)
+        for name, a, b in zip("qkvbm", whole, slab):
+            assert torch.equal(a[:, u0:u0 + 3] if name == "b" else a[u0:u0 + 3], b), name
+    ops.device_error_flags()
