@@ -312,6 +312,8 @@ static int32_t launch_contract(const void* a, const void* b, void* x, int64_t ch
   const int64_t total = tiles_i * tiles_j * channels;
   if (total > 0x7fffffff) return PX_ERR_UNSUPPORTED;
   const int64_t room = sm_count() / kCtas;
+  const bool ragged = rows_a % (kTcBM * kCtas) || rows_b % kTcBN;
+  const int64_t period = !ragged ? 1 : channels > 1 ? tiles_i * tiles_j : tiles_j;
   const size_t smem = Shape::kBars + sizeof(TcBarriers) + 1024;
   static_assert(Shape::kBars + sizeof(TcBarriers) + 1024 <= 232448, "shared memory budget");
   static SmemLimit limit;
@@ -322,7 +324,7 @@ static int32_t launch_contract(const void* a, const void* b, void* x, int64_t ch
   at[1].id = cudaLaunchAttributeClusterDimension;
   at[1].val.clusterDim.x = kCtas, at[1].val.clusterDim.y = 1, at[1].val.clusterDim.z = 1;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(even_grid(total, room) * kCtas));
+  cfg.gridDim = dim3((unsigned)(even_grid(total, room, period) * kCtas));
   cfg.blockDim = dim3(192);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;

@@ -222,7 +222,7 @@ extern "C" int32_t px_msa_average(const px_bf16* w, const px_bf16* v, float* wv,
   if (n_tiles > 0x7fffffff) return PX_ERR_UNSUPPORTED;
   const size_t smem = MvLayout::total + 1024;
   static SmemLimit limit;
-  const int grid = even_grid(n_tiles, sm_count());
+  const int grid = even_grid(n_tiles, sm_count(), n % 128 ? tiles_m : 1);
   return limit.set(msa_average_tc_kernel, smem) &&
                  launch_pdl(msa_average_tc_kernel, dim3((unsigned)grid), kMvThreads, smem, (cudaStream_t)stream, mw, mv, wv, (int)n, (int)cols,
                             (int)tiles_m, (int)tiles_n, (int)n_tiles, (int)((n + 63) / 64))

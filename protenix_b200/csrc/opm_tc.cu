@@ -217,7 +217,7 @@ static int32_t launch_opm_out(const px_f16* x, const px_f16* w_out, const float*
   if (!limit.set(opm_out_tc_kernel<Tz>, smem)) return PX_ERR_LAUNCH;
   const int64_t tiles_j = (n + 127) / 128, total = tiles_j * n_i;
   if (total > 0x7fffffff) return PX_ERR_UNSUPPORTED;
-  const int grid = even_grid(total, sm_count());
+  const int grid = even_grid(total, sm_count(), n % 128 ? tiles_j : 1);
   return launch_pdl(opm_out_tc_kernel<Tz>, dim3(grid), 192, smem, st, mx, mw, bias, inv_norm, (const Tz*)z_in, (Tz*)z_out, (int)n,
                     (int)add_residual, tiles_j, total)
              ? PX_OK

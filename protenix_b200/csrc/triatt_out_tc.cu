@@ -386,7 +386,7 @@ static int32_t launch_triatt_out(const px_f16* o, const void* z_in, const px_f16
   if (!limit.set(triatt_out_tc_kernel<kMode>, smem)) return PX_ERR_LAUNCH;
   const int64_t tiles_t = (n + 127) / 128, n_tiles = tiles_t * n_u;
   if (n_tiles > 0x7fffffff) return PX_ERR_UNSUPPORTED;
-  const int grid = even_grid(n_tiles, sm_count());
+  const int grid = even_grid(n_tiles, sm_count(), n % 128 ? tiles_t : 1);
   return launch_pdl(triatt_out_tc_kernel<kMode>, dim3(grid), ao_threads(kMode != 0), smem, st, mz, mo, mout, z_in, z_out, weights,
                     (const unsigned char*)folded, (int)n_u, (int)n, (int)ending, (int)add_residual, eps, (int)tiles_t, (int)n_tiles)
              ? PX_OK

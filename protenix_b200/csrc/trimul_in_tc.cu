@@ -217,7 +217,7 @@ static int32_t launch_trimul_in(const void* z, const float* mask, const TiWeight
   if (!limit.set(trimul_in_tc_kernel<kF16>, smem)) return PX_ERR_LAUNCH;
   const int64_t tiles_t = (ld + 127) / 128, n_tiles = tiles_t * n_u;
   if (n_tiles > 0x7fffffff) return PX_ERR_UNSUPPORTED;
-  const int pairs = even_grid(n_tiles, sm_count() / 2);
+  const int pairs = even_grid(n_tiles, sm_count() / 2, ld % 128 ? tiles_t : 1);
   return launch_pdl(trimul_in_tc_kernel<kF16>, dim3(2 * pairs), ti_threads(kF16), smem, st, mz, ma, mb, mask, weights,
                     (const unsigned char*)folded, (int)n_u, (int)n_t, (int)incoming, eps, (int)tiles_t, (int)n_tiles)
              ? PX_OK

@@ -381,7 +381,7 @@ static int32_t launch_trimul_out(const px_f16* x, const void* z_in, const px_f16
   if (!limit.set(trimul_out_tc_kernel<Tz, kBulk>, smem)) return PX_ERR_LAUNCH;
   const int64_t tiles_j = (n + 127) / 128, n_tiles = tiles_j * n_i;
   if (n_tiles > 0x7fffffff) return PX_ERR_UNSUPPORTED;
-  const int grid = even_grid(n_tiles, sm_count());
+  const int grid = even_grid(n_tiles, sm_count(), n % 128 ? tiles_j : 1);
   return launch_pdl(trimul_out_tc_kernel<Tz, kBulk>, dim3(grid), to_threads(sizeof(Tz) != 2), smem, st, mz, mx, mout, (const Tz*)z_in, (Tz*)z_out, weights,
                     (const unsigned char*)folded, (int)n_i, (int)n, (int)add_residual, eps, (int)tiles_j, (int)n_tiles)
              ? PX_OK

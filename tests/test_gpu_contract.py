@@ -1,7 +1,8 @@
 """The contraction alone and paired (one or two CTAs to a tile) at the edges of its tiles, against fp64 of the same operands.
 
 Pairs take many tiles (two to an SM) of long contractions: with 128-byte lines from six row tiles and k = 448 on, with 32-byte sectors from k = 272,
-with rows that straddle sectors from four row tiles and k = 152."""
+with rows that straddle sectors from four row tiles and k = 152.  The last two sizes run in more CTAs than end evenly, so that each gets
+ragged and whole tiles."""
 import pytest
 import torch
 
@@ -16,7 +17,8 @@ def _close(got, want):
 
 
 @pytest.mark.parametrize("channels,n", [(3, 1), (5, 64), (150, 100), (3, 129), (2, 200), (80, 256), (2, 257), (2, 385), (1, 512), (2, 520), (1, 777),
-                                        (50, 384), (50, 390), (50, 400), (40, 520), (32, 640), (25, 641), (25, 777), (10, 1030)])
+                                        (50, 384), (50, 390), (50, 400), (40, 520), (32, 640), (25, 641), (25, 777), (10, 1030),
+                                        (128, 300), (128, 530)])
 def test_contract(channels, n):
     torch.manual_seed(n)
     ld = ops.ld(n)
