@@ -81,7 +81,7 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
 
 // 2^x for two arguments on the FMA pipe (the special-function unit delivers 16 ex2 per clock and SM and is the
 // busiest unit of this kernel): x = n + f with n = round(x) taken from the mantissa after adding 1.5 * 2^23,
-// 2^f by a cubic on [-0.5, 0.5] (relative error 7.5e-5, far below the bf16 rounding of P), 2^n added into the exponent
+// 2^f by a cubic on [-0.5, 0.5] (relative error 7.5e-5, below the fp16 rounding of P), 2^n added into the exponent
 // field.  Arguments below -126 (masked or padded keys) give 2^-126.
 constexpr int kFPolyEvery = 4;   // every fourth pair of exponentials takes this path
 __device__ __forceinline__ void exp2_poly2(float x0, float x1, float& p0, float& p1) {

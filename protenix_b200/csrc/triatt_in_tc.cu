@@ -11,7 +11,7 @@
 //   warps 0..7    epilogue of q | k: a thread owns one pair element and both heads of q (warps 0..3) or k (4..7):
 //                 a warp's 32 rows of a head, 2 KB, are staged (64-byte swizzle) and leave by TMA.  Written by their threads in
 //                 pieces of 16 bytes, half a sector each, they took the kernel from 32 to 42 us at N = 384 and from 119 to 144 at N = 768.
-//   warps 8..15   epilogue of v | bias: v goes through a [64 d][128 t] staging tile and a TMA store (the transpose),
+//   warps 8..15   epilogue of v | bias: v goes through a [32 d][128 t] staging tile per head and a TMA store (the transpose),
 //                 the two bias values of the row are written directly.
 //   warps 16..19  (bf16 rows 16..23) statistics, correction row, scale pair, mask bias.
 //   then          a TMA producer and the MMA issuers of the two products (N = 128 and N = 80), each into two accumulators in turn.

@@ -180,7 +180,7 @@ triatt_out_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_con
       }
     }
   } else if (warp >= 16) {
-    // ------------------------------------------------------------------ row statistics, one thread per row
+    // ------------------------------------------------------------------ row statistics (bf16 rows: two lanes a row)
     float* scale = reinterpret_cast<float*>(sm + AoLayout::scale);
     tile_stats_loop(ctx, eps, warp - 16, lane,
                         [&](int k, int u, int t, int r, float rstd) { scale[(k % Ctx::kSlots) * 128 + r] = rstd; });

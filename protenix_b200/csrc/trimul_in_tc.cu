@@ -125,7 +125,7 @@ trimul_in_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_cons
                         bars.acc_free[ph], 2, 256);
     }
   } else if (warp >= 16) {
-    // ------------------------------------------------------------------ row statistics, one thread per row
+    // ------------------------------------------------------------------ row statistics (bf16 rows: two lanes a row)
     float2* scale = reinterpret_cast<float2*>(sm + TiLayout::scale);
     tile_stats_loop(ctx, eps, warp - 16, lane, [&](int k, int u, int t, int r, float rstd) {
       float mk = 0.f;

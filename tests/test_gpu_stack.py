@@ -1,4 +1,5 @@
-"""The stack runs the single branch of a block beside the attention core of the next one; block by block, on one stream, the same bits."""
+"""The stack runs the single branch of a block beside the attention core of the next one, above 1280 tokens in order; block by block, on one
+stream, the same bits."""
 import pytest
 import torch
 
@@ -10,7 +11,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
-@pytest.mark.parametrize("n, blocks", [(1, 3), (40, 1), (40, 2), (130, 4), (257, 3), (769, 2)])
+@pytest.mark.parametrize("n, blocks", [(1, 3), (40, 1), (40, 2), (130, 4), (257, 3), (769, 2), (1281, 2)])
 def test_stack_equals_its_blocks(n, blocks, dtype):
     torch.manual_seed(n)
     stack = randomize_parameters_(px.PairformerStack(n_blocks=blocks), 3).cuda().eval()
