@@ -280,7 +280,9 @@ static int32_t launch_triatt_in(const void* z, const float* mask, const AiWeight
   if (!limit.set(triatt_in_tc_kernel<kF16, kStages>, smem)) return PX_ERR_LAUNCH;
   const int64_t tiles_t = (n + 127) / 128, n_tiles = tiles_t * n_u;   // 128-wide tiles cover the pad columns up to ldm
   if (n_tiles > 0x7fffffff) return PX_ERR_UNSUPPORTED;
-  const int pairs = even_grid(n_tiles, sm_count() / 2, n % 128 ? tiles_t : 1);
+  // Whole tiles of bf16 rows take little longer than ragged ones (their statistics are the same work), and an even number serves them 2 to 4 %
+  // better from 132 to 230 tokens (N = 160 13.5 us against 14.0), 1 to 2 % worse at 430 and 450; standardised rows gain 3 to 8 % there.
+  const int pairs = even_grid(n_tiles, sm_count() / 2, kF16 && n % 128 ? tiles_t : 1);
   return launch_pdl(triatt_in_tc_kernel<kF16, kStages>, dim3(2 * pairs), ai_threads(kF16), smem, st, mz, mv, mq, mk, mask, weights,
                     (const unsigned char*)folded, bias, mask_bias, (int)n_u, (int)n, (int)ldm, (int)ending, eps, inf, (int)tiles_t,
                     (int)n_tiles)
