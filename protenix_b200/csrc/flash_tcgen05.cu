@@ -19,9 +19,13 @@
 //   warp 15       loads the pair-bias tiles [128 q][64 k] fp32 (two 128-byte-swizzled boxes, 2-deep ring).
 // Tensor memory: S (3 x 64) | P (3 x 32, two fp16 per column) | O (6 x 32).
 //
-// What bounds it (per item of 128 queries x 64 keys, 800 cycles at N = 1536): nothing alone.  Tensor pipe 416 (a copy
-// of 8 columns takes 64 cycles, S 96, P V 64), special-function unit 384, issue slots 440, L2 29 bytes a cycle and SM at most
-// (with the arithmetic taken out 457 cycles are left, of L2 traffic).  Hence the bias split in halves: all 64 columns copied
+// What bounds it (per item of 128 queries x 64 keys, 770 cycles at N = 768): no unit alone, but the chain of a group's item.  Tensor
+// pipe 416 (a copy of 8 columns takes 64 cycles, S 96, P V 64), special-function unit 384, issue slots 440; without any load of K, V
+// and bias the time is the same.  So nothing waits on the chain that can wait beside it: the other half of the bias is fetched
+// before S is waited for, and the store of the zeros is waited for behind the tile maximum (N = 200 30.5 -> 29.8 us, 384 110.2 -> 106.7,
+// 768 677 -> 653, 1536 4.98 -> 4.80 ms; either alone less than 1 %).  Taken against the standing maximum before it is checked,
+// the logits need fewer steps on the chain, but 709 us at N = 768; P handed over behind the loads of the next S 685; bias held for both rows 662.
+// Hence, too, the bias split in halves: all 64 columns copied
 // make the tensor pipe 80 % busy and S late (N = 384 118.7 us against 110.4, N = 1536 level), none copied is 48 more
 // instructions of 400 per softmax thread (123.5, 5.61 ms against 5.06).  24 or 40 columns: as 32 within 1 %.  Writing the bias
 // into S from the softmax threads for the next item: 5.32 ms (a store and its wait are on the group's chain).  Four groups of
@@ -242,15 +246,15 @@ triatt_flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
       m_ref[r] = -CUDART_INF_F;
       l_sum[r] = 0.f;
     }
-    // the product adds to what S holds: the columns without the bias start from zero
+    // the product adds to what S holds: the columns without the bias start from zero (the store is waited for by the caller)
     auto clear_rest = [&] {
       uint32_t zero[kFKT - kFCopied];
 #pragma unroll
       for (int e = 0; e < kFKT - kFCopied; ++e) zero[e] = 0u;
       tmem_st32(t_s + kFCopied, zero);
-      tmem_wait_st();
     };
     clear_rest();
+    tmem_wait_st();
     tc_fence_before();
     __syncwarp();
     if (lane == 0) mbar_arrive(&bars.s_free[g]);
@@ -288,7 +292,15 @@ triatt_flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
       for (int r = 0; r < kFRpg; ++r) {
         const int i = kt * kFRpg + r;               // this group's work item
         // a wait that gave up is voted on once per item, below: what is computed till then goes nowhere
-        ok = mbar_wait(&bars.s_full[g], i & 1, 128u);
+        if (r == 0) ok = mbar_wait(&bars.bias_full[kt & 1], (kt >> 1) & 1, 64u);
+        // The pair bias of the columns that were not copied (128-byte rows, 16-byte pieces swizzled by row) is fetched before S is waited
+        // for, so that it is at hand when S comes.
+        float4 b4[(kFKT - kFCopied) / 4];
+        const float* brow = reinterpret_cast<const float*>(sm + FlashLayout::bias + (kt & 1) * kFBiasBytes) + row * 32;
+#pragma unroll
+        for (int c = kFCopied / 4; c < kFKT / 4; ++c)
+          b4[c - kFCopied / 4] = *reinterpret_cast<const float4*>(brow + (c >> 3) * (128 * 32) + (((c & 7) ^ (row & 7)) << 2));
+        ok = mbar_wait(&bars.s_full[g], i & 1, 128u) && ok;
         __syncwarp();
         tc_fence_after();
         float s[kFKT];
@@ -300,17 +312,10 @@ triatt_flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
           tmem_wait_ld();
           clear_rest();
         }
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&bars.s_free[g]);  // S is in registers: the next S may be computed
-        // + pair bias of the other columns: 128-byte rows, 16-byte pieces swizzled by row
-        if (r == 0) ok = mbar_wait(&bars.bias_full[kt & 1], (kt >> 1) & 1, 64u) && ok;
-        const float* brow = reinterpret_cast<const float*>(sm + FlashLayout::bias + (kt & 1) * kFBiasBytes) + row * 32;
 #pragma unroll
         for (int c = kFCopied / 4; c < kFKT / 4; ++c) {
-          const float4 b4 = *reinterpret_cast<const float4*>(brow + (c >> 3) * (128 * 32) + (((c & 7) ^ (row & 7)) << 2));
-          add2(s[4 * c + 0], s[4 * c + 1], b4.x, b4.y);
-          add2(s[4 * c + 2], s[4 * c + 3], b4.z, b4.w);
+          add2(s[4 * c + 0], s[4 * c + 1], b4[c - kFCopied / 4].x, b4[c - kFCopied / 4].y);
+          add2(s[4 * c + 2], s[4 * c + 3], b4[c - kFCopied / 4].z, b4[c - kFCopied / 4].w);
         }
         if ((flag_word[r] >> (kt & 63)) & 1ull) {     // warp-uniform
           const int u = (ug + r < n_u) ? ug + r : 0;
@@ -332,6 +337,12 @@ triatt_flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
           mq[c] = fmaxf(mq[c], s[16 * c + 15]);
         }
         const float mt = fmaxf(fmaxf(mq[0], mq[1]), fmaxf(mq[2], mq[3]));
+        // S is in registers and its columns are zero again: the next S may be computed.  Said only here, when the store of the zeros has long
+        // arrived, so that nobody waits for it; the next S has the time of the exponentials to come.
+        tmem_wait_st();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bars.s_free[g]);
         // Does the reference maximum have to move?  Rare after the first tiles.  The exponentials need only this thread's own answer;
         // the warp's (tensor memory is rescaled by whole warps) is asked for beside them.
         const bool up = mt > m_ref[r] + kRescaleGap;
