@@ -5,7 +5,7 @@
 // q, k, v and o are fp16 (projections of standardised rows and convex combinations of them: far inside its range;
 // fp16 keeps three more bits than bf16), the pair bias, the logits, the softmax and the accumulators fp32.
 //
-// One CTA = (head h, 128 queries, 6 attended rows u), 16 warps:
+// One CTA = (head h, 128 queries, 6 attended rows u; 3 for part of the last wave, then one row a group), 16 warps:
 //   warps 0..11   three softmax groups of four warps; group g owns rows u0+2g, u0+2g+1, each thread one query row and
 //                 the softmax denominator of it.  The pair bias does not depend on u: all six rows use the same tile.
 //   warps 12..14  one control warp per group, whose elected lane issues.  It loads the group's Q tiles once
@@ -36,6 +36,8 @@
 // Exponentials are fp32 (three pairs in four by ex2, the fourth by a cubic on the FMA pipe); P is their rounding to
 // fp16, the denominators sum the fp32 values.  Every mbarrier wait is bounded.
 #include <math_constants.h>
+
+#include <type_traits>
 
 #include "px_rowpipe.cuh"
 
@@ -106,17 +108,23 @@ __device__ __forceinline__ void exp2_poly2(float x0, float x1, float& p0, float&
   p1 = __int_as_float(__float_as_int(q1) + (__float_as_int(t1) << 23));
 }
 
+template <bool kHalves>
 __global__ void __launch_bounds__(kFThreads, 1)
 triatt_flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                        const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_b,
                        const __grid_constant__ CUtensorMap map_o, const float* __restrict__ mb,
-                       int n_u, int n, int ldm, int nkt) {
+                       int n_u, int n, int ldm, int nkt, int whole) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* sm = smem_aligned(smem_raw);
   FlashBars& bars = *reinterpret_cast<FlashBars*>(sm + FlashLayout::bars);
   const int warp = warp_index(), lane = threadIdx.x & 31;
-  // the last rows first: their q, k and v were written last and may still lie in L2
-  const int q0 = blockIdx.x * 128, h = blockIdx.y, u0 = (gridDim.z - 1 - blockIdx.z) * kFRows;
+  // The last rows first: their q, k and v were written last and may still lie in L2.
+  // kHalves: slices of the grid from `whole` on have one row per group, two of them share the rows of one (see px_triatt_flash).
+  const int q0 = blockIdx.x * 128, h = blockIdx.y, behind = kHalves ? (int)blockIdx.z - whole : -1;
+  const int halves = kHalves ? ((int)gridDim.z - whole) >> 1 : 0;
+  const int u0 = !kHalves ? (gridDim.z - 1 - blockIdx.z) * kFRows
+                 : behind < 0 ? (halves - 1 - behind) * kFRows : halves * kFRows - (behind + 1) * kFGroups;
+  if (kHalves && u0 >= n_u) return;      // the second half of the last rows, where they are three at most
 
   const bool skip = cta_begin();         // an earlier bounded wait gave up: do not start new work
   if (threadIdx.x == 32) prefetch_maps(map_q, map_k, map_v, map_b, map_o);
@@ -144,6 +152,8 @@ triatt_flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
   if (!cta_ready(skip, warp == 4 * kFGroups, bars.tmem_base, kFCols)) return;
   const uint32_t tmem_base = bars.tmem_base;
 
+  const auto rows = [&](auto per_group) {
+  constexpr int kRpg = decltype(per_group)::value;     // attended rows per group
   if (warp >= 4 * kFGroups) {
     // ------------------------------------------------------------------ control warp of group g
     asm volatile("setmaxnreg.dec.sync.aligned.u32 32;\n");   // registers go to the softmax warpgroups
@@ -165,20 +175,20 @@ triatt_flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
       }
     } else {
       constexpr uint32_t idesc_s = umma_idesc_f16(128, kFKT), idesc_o = umma_idesc_f16(128, kFON);
-      const int n_items = nkt * kFRpg;              // work item i = (key tile i / 2, row i % 2 of the group)
-      const uint32_t q_addr = smem_u32(sm + FlashLayout::q + g * kFRpg * kFQBytes);
+      const int n_items = nkt * kRpg;              // work item i = (key tile i / 2, row i % 2 of the group)
+      const uint32_t q_addr = smem_u32(sm + FlashLayout::q + g * kRpg * kFQBytes);
       const uint32_t ring = smem_u32(sm + FlashLayout::kv + g * kFStages * kFStageBytes);
       const uint32_t d_s = tmem_base + kFColS + kFKT * g, d_p = tmem_base + kFColP + (kFKT / 2) * g;
-      const uint32_t d_o = tmem_base + kFColO + kFON * kFRpg * g;
-      const int uh0 = (u0 + g * kFRpg) * kFH + h;   // rows past n_u: coordinate beyond the tensor -> zero fill
+      const uint32_t d_o = tmem_base + kFColO + kFON * kRpg * g;
+      const int uh0 = (u0 + g * kRpg) * kFH + h;   // rows past n_u: coordinate beyond the tensor -> zero fill
       auto load_kv = [&](int i) {                   // K and V tiles of item i into stage i % kFStages (one lane)
-        const int s = i % kFStages, kt = i / kFRpg, uh = uh0 + (i % kFRpg) * kFH;
+        const int s = i % kFStages, kt = i / kRpg, uh = uh0 + (i % kRpg) * kFH;
         mbar_expect_tx(&bars.kv_full[g][s], kFKBytes + kFVBox);
         tma_load_3d(ring + s * kFStageBytes, &map_k, &bars.kv_full[g][s], 0, kt * kFKT, uh);
         tma_load_3d(ring + s * kFStageBytes + kFKBytes, &map_v, &bars.kv_full[g][s], kt * kFKT, 0, uh);
       };
       auto issue_s = [&](int i) {                   // S(i) = bias + Q_r K^T
-        const int s = i % kFStages, kt = i / kFRpg, r = i % kFRpg;
+        const int s = i % kFStages, kt = i / kRpg, r = i % kRpg;
         if (r == 0 && !mbar_wait_warp(&bars.bias_full[kt & 1], (kt >> 1) & 1, 64u)) return false;
         if (!mbar_wait_warp(&bars.kv_full[g][s], (i / kFStages) & 1, 8u)) return false;
         tc_fence_after();
@@ -191,20 +201,20 @@ triatt_flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
           umma_bf16(d_s, dq, dk, idesc_s, 1u);
           umma_bf16(d_s, dq + 2, dk + 2, idesc_s, 1u);
           umma_commit(&bars.s_full[g]);
-          if (r == kFRpg - 1) umma_commit(&bars.bias_empty[kt & 1]);   // this group is done with the bias tile
+          if (r == kRpg - 1) umma_commit(&bars.bias_empty[kt & 1]);   // this group is done with the bias tile
         }
         __syncwarp();
         return true;
       };
       if (elect_lane()) {
-        mbar_expect_tx(&bars.q_full[g], kFRpg * kFQBytes);
-        for (int r = 0; r < kFRpg; ++r) tma_load_3d(q_addr + r * kFQBytes, &map_q, &bars.q_full[g], 0, q0, uh0 + r * kFH);
+        mbar_expect_tx(&bars.q_full[g], kRpg * kFQBytes);
+        for (int r = 0; r < kRpg; ++r) tma_load_3d(q_addr + r * kFQBytes, &map_q, &bars.q_full[g], 0, q0, uh0 + r * kFH);
         for (int i = 0; i < kFStages - 1 && i < n_items; ++i) load_kv(i);   // first use of these stages
       }
       __syncwarp();
       bool ok = mbar_wait_warp(&bars.q_full[g], 0, 4u) && mbar_wait_warp(&bars.s_free[g], 0, 2u) && issue_s(0);
       for (int i = 0; i < n_items && ok; ++i) {
-        const int kt = i / kFRpg, r = i % kFRpg;
+        const int kt = i / kRpg, r = i % kRpg;
         if (i + 1 < n_items) {                      // next S as soon as the group holds the current one in registers
           ok = mbar_wait_warp(&bars.s_free[g], (i + 1) & 1, 2u) && issue_s(i + 1);
           if (!ok) break;
@@ -236,12 +246,12 @@ triatt_flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     const uint32_t lane_addr = (uint32_t)(32 * qw) << 16;
     const uint32_t t_s = tmem_base + lane_addr + kFColS + kFKT * g;
     const uint32_t t_p = tmem_base + lane_addr + kFColP + (kFKT / 2) * g;
-    const uint32_t t_o = tmem_base + lane_addr + kFColO + kFON * kFRpg * g;
-    const int ug = u0 + kFRpg * g;                  // first row of this group
-    unsigned long long flag_word[kFRpg];            // bit kt & 63: some key of tile kt has a mask bias other than zero
-    float m_ref[kFRpg], l_sum[kFRpg];             // reference maximum and denominator of this thread's query per row
+    const uint32_t t_o = tmem_base + lane_addr + kFColO + kFON * kRpg * g;
+    const int ug = u0 + kRpg * g;                  // first row of this group
+    unsigned long long flag_word[kRpg];            // bit kt & 63: some key of tile kt has a mask bias other than zero
+    float m_ref[kRpg], l_sum[kRpg];             // reference maximum and denominator of this thread's query per row
 #pragma unroll
-    for (int r = 0; r < kFRpg; ++r) {
+    for (int r = 0; r < kRpg; ++r) {
       flag_word[r] = 0;
       m_ref[r] = -CUDART_INF_F;
       l_sum[r] = 0.f;
@@ -261,23 +271,23 @@ triatt_flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     bool ok = true;
     for (int kt = 0; kt < nkt && ok; ++kt) {
       if ((kt & 63) == 0) {
-        for (int r = 0; r < kFRpg; ++r) flag_word[r] = 0;
+        for (int r = 0; r < kRpg; ++r) flag_word[r] = 0;
         // A load covers two tiles (ldm is a multiple of 128), eight are in flight beside the first TMA loads and products (two
         // in flight: 6.17 ms at N = 1536, against 5.88).  As a kernel of its own this cost a launch: 16.6 us together at
         // N = 128 against 12.6, 143 against 136 at N = 384.
         const int left = min(nkt - kt, 64);
 #pragma unroll 1
         for (int t0 = 0; t0 < left; t0 += 8) {
-          float4 m4[kFRpg][4];
+          float4 m4[kRpg][4];
 #pragma unroll
-          for (int r = 0; r < kFRpg; ++r)
+          for (int r = 0; r < kRpg; ++r)
 #pragma unroll
             for (int j = 0; j < 4; ++j)
               m4[r][j] = t0 + 2 * j < left ? __ldg(reinterpret_cast<const float4*>(mb + (size_t)((ug + r < n_u) ? ug + r : 0) * ldm +
                                                                                    (kt + t0 + 2 * j) * kFKT) + lane)
                                            : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-          for (int r = 0; r < kFRpg; ++r) {
+          for (int r = 0; r < kRpg; ++r) {
             unsigned bits = 0;
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
@@ -289,10 +299,10 @@ triatt_flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         }
       }
 #pragma unroll
-      for (int r = 0; r < kFRpg; ++r) {
-        const int i = kt * kFRpg + r;               // this group's work item
+      for (int r = 0; r < kRpg; ++r) {
+        const int i = kt * kRpg + r;               // this group's work item
         // a wait that gave up is voted on once per item, below: what is computed till then goes nowhere
-        if (r == 0) ok = mbar_wait(&bars.bias_full[kt & 1], (kt >> 1) & 1, 64u);
+        ok = r == 0 ? mbar_wait(&bars.bias_full[kt & 1], (kt >> 1) & 1, 64u) : true;
         // The pair bias of the columns that were not copied (128-byte rows, 16-byte pieces swizzled by row) is fetched before S is waited
         // for, so that it is at hand when S comes.
         float4 b4[(kFKT - kFCopied) / 4];
@@ -399,12 +409,12 @@ triatt_flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
           mbar_arrive(&bars.p_ready[g]);
           // Done with the bias tile.  Only here, where every value read from it has been used: signalled right behind the loads, while
           // these were generic ones, the next tile now and then overtook them (one row in 10^8 wrong).
-          if (r == kFRpg - 1) mbar_arrive(&bars.bias_empty[kt & 1]);
+          if (r == kRpg - 1) mbar_arrive(&bars.bias_empty[kt & 1]);
         }
       }
     }
     // ---- epilogue: o = O / denominator for this group's rows
-    ok = ok && mbar_wait(&bars.pv_done[g], (nkt * kFRpg - 1) & 1, 512u);
+    ok = ok && mbar_wait(&bars.pv_done[g], (nkt * kRpg - 1) & 1, 512u);
     ok = __all_sync(0xffffffffu, ok);
     if (ok) {
       tc_fence_after();
@@ -412,11 +422,11 @@ triatt_flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
       // 2 KB there (64-byte swizzle).  Written by their threads, 16 bytes at 256-byte distances, they took 4 % of the kernel at
       // N = 384 (135 us against 129) and 1.6 % at N = 1536 (5.89 ms against 5.79).
 #pragma unroll
-      for (int r = 0; r < kFRpg; ++r) {
+      for (int r = 0; r < kRpg; ++r) {
         uint32_t a[32];
         tmem_ld32(t_o + kFON * r, a);
         tmem_wait_ld();
-        unsigned char* tile = sm + FlashLayout::q + (g * kFRpg + r) * kFQBytes;
+        unsigned char* tile = sm + FlashLayout::q + (g * kRpg + r) * kFQBytes;
         const float inv = 1.0f / l_sum[r];
 #pragma unroll
         for (int v = 0; v < 4; ++v) {
@@ -437,6 +447,11 @@ triatt_flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
       if (lane == 0) tma_store_wait_read<0>();
     }
   }
+  };
+  if (kHalves && behind >= 0)
+    rows(std::integral_constant<int, 1>{});
+  else
+    rows(std::integral_constant<int, kFRpg>{});
 
   tc_fence_before();
   cta_teardown_sync();
@@ -483,10 +498,17 @@ extern "C" int32_t px_triatt_flash(const px_f16* q, const px_f16* k, const px_f1
     return PX_ERR_LAUNCH;
   cudaStream_t st = (cudaStream_t)stream;
   const size_t smem = FlashLayout::total + 1024;
-  static SmemLimit limit;
-  if (!limit.set(triatt_flash_tc_kernel, smem)) return PX_ERR_LAUNCH;
-  dim3 grid((unsigned)((n + 127) / 128), kFH, (unsigned)((n_u + kFRows - 1) / kFRows));
-  return launch_pdl(triatt_flash_tc_kernel, grid, kFThreads, smem, st, mq, mk, mv, mbias, mo, mask_bias, (int)n_u, (int)n, (int)ldm, nkt)
+  // CTAs of six rows (two a group); where what is left of them for the last wave fits the SMs twice, that in CTAs of three (one a
+  // group; whole slices of the grid), so that the wave ends in little more than half the time: N = 100 10.2 -> 7.8 us, 160 23.9 -> 20.8,
+  // 256 41.5 -> 37.6, 300 76.5 -> 72, 384 106.4 -> 101.6, 512 218.5 -> 213.  CTAs of three only: 384 125, 768 805 against 653.  Each
+  // number of rows has its own code (as a run-time number, which leaves no parity known to the compiler, 15 % slower).
+  const int64_t per = (n + 127) / 128 * kFH, slices = (n_u + kFRows - 1) / kFRows, room = sm_count(), left = per * slices % room;
+  const int64_t halves = 2 * left <= room ? (left + per - 1) / per : 0, whole = slices - halves;
+  const auto kernel = halves ? triatt_flash_tc_kernel<true> : triatt_flash_tc_kernel<false>;
+  static SmemLimit limit[2];
+  if (!limit[halves > 0].set(kernel, smem)) return PX_ERR_LAUNCH;
+  return launch_pdl(kernel, dim3((unsigned)((n + 127) / 128), kFH, (unsigned)(whole + 2 * halves)), kFThreads, smem, st, mq, mk, mv, mbias,
+                    mo, mask_bias, (int)n_u, (int)n, (int)ldm, nkt, (int)whole)
              ? PX_OK
              : PX_ERR_LAUNCH;
 }

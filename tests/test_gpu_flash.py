@@ -49,3 +49,24 @@ def test_attention_core_is_the_same_every_time():
     first = ops.triatt_flash(q, k, v, bias, mb)
     differs = sum((ops.triatt_flash(q, k, v, bias, mb) != first).any() for _ in range(300))
     assert int(differs) == 0
+
+
+@pytest.mark.parametrize("n_u", [1, 3, 4, 9, 100, 111, 114, 130])
+def test_rows_do_not_depend_on_how_they_are_dealt_out(n_u):
+    """CTAs of six rows, of three in the last wave, none for rows beyond the last: a slab of rows gives the bits of the whole."""
+    n = 150
+    g = torch.Generator("cuda").manual_seed(n)
+    draw = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    q, k = (0.3 * draw(n, 4, n, 32)).half(), draw(n, 4, n, 32).half()
+    v = torch.zeros(n, 4, 32, ops.ld(n), dtype=torch.half, device="cuda")
+    v[..., :n] = draw(n, 4, 32, n).half()
+    ldm = (n + 127) // 128 * 128
+    bias, mb = torch.zeros(4, n, ldm, device="cuda"), torch.full((n, ldm), -float("inf"), device="cuda")
+    bias[..., :n] = 2 * draw(4, n, n)
+    mb[:, :n] = 0
+    whole = ops.triatt_flash(q, k, v, bias, mb)
+    for first in {0, (n - n_u) // 2, n - n_u}:
+        rows = slice(first, first + n_u)
+        part = ops.triatt_flash(q[rows].contiguous(), k[rows].contiguous(), v[rows].contiguous(), bias, mb[rows].contiguous())
+        assert torch.equal(part, whole[rows])
+    ops.device_error_flags()
