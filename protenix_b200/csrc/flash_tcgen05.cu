@@ -108,7 +108,8 @@ __device__ __forceinline__ void exp2_poly2(float x0, float x1, float& p0, float&
   p1 = __int_as_float(__float_as_int(q1) + (__float_as_int(t1) << 23));
 }
 
-template <bool kHalves>
+// kHalves: the grid ends with CTAs of one row per group.  kBrief: the last key tile has 32 keys at most, its other half is left out.
+template <bool kHalves, bool kBrief>
 __global__ void __launch_bounds__(kFThreads, 1)
 triatt_flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                        const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_b,
@@ -231,8 +232,10 @@ triatt_flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         if (elect_lane()) {
           const uint64_t dv = umma_desc_sw128(ring + (i % kFStages) * kFStageBytes + kFKBytes);
 #pragma unroll
-          for (int ks = 0; ks < kFKT / 16; ++ks)    // 16 keys per step: 8 TMEM columns of P, 32 bytes of the value rows
+          for (int ks = 0; ks < kFKT / 16; ++ks) {  // 16 keys per step: 8 TMEM columns of P, 32 bytes of the value rows
+            if (kBrief && ks == kFKT / 32 && kt == nkt - 1) break;
             umma_bf16_ts(d_o + kFON * r, d_p + 8 * ks, dv + 2 * ks, idesc_o, (kt | ks) ? 1u : 0u);
+          }
           umma_commit(&bars.pv_done[g]);
         }
         __syncwarp();
@@ -268,8 +271,7 @@ triatt_flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     tc_fence_before();
     __syncwarp();
     if (lane == 0) mbar_arrive(&bars.s_free[g]);
-    bool ok = true;
-    for (int kt = 0; kt < nkt && ok; ++kt) {
+    const auto mask_flags = [&](int kt) {
       if ((kt & 63) == 0) {
         for (int r = 0; r < kRpg; ++r) flag_word[r] = 0;
         // A load covers two tiles (ldm is a multiple of 128), eight are in flight beside the first TMA loads and products (two
@@ -298,32 +300,32 @@ triatt_flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
           }
         }
       }
+    };
+    // The items of key tile kt, of which the first `keys` exist: 64, or 32 where a last tile has no more.
+    const auto items = [&](int kt, auto keys) {
+      constexpr int kKeys = decltype(keys)::value;
 #pragma unroll
       for (int r = 0; r < kRpg; ++r) {
         const int i = kt * kRpg + r;               // this group's work item
         // a wait that gave up is voted on once per item, below: what is computed till then goes nowhere
-        ok = r == 0 ? mbar_wait(&bars.bias_full[kt & 1], (kt >> 1) & 1, 64u) : true;
+        bool ok = r == 0 ? mbar_wait(&bars.bias_full[kt & 1], (kt >> 1) & 1, 64u) : true;
         // The pair bias of the columns that were not copied (128-byte rows, 16-byte pieces swizzled by row) is fetched before S is waited
         // for, so that it is at hand when S comes.
         float4 b4[(kFKT - kFCopied) / 4];
         const float* brow = reinterpret_cast<const float*>(sm + FlashLayout::bias + (kt & 1) * kFBiasBytes) + row * 32;
 #pragma unroll
-        for (int c = kFCopied / 4; c < kFKT / 4; ++c)
+        for (int c = kFCopied / 4; c < kKeys / 4; ++c)
           b4[c - kFCopied / 4] = *reinterpret_cast<const float4*>(brow + (c >> 3) * (128 * 32) + (((c & 7) ^ (row & 7)) << 2));
         ok = mbar_wait(&bars.s_full[g], i & 1, 128u) && ok;
         __syncwarp();
         tc_fence_after();
-        float s[kFKT];
-        {
-          uint32_t(&t0)[32] = *reinterpret_cast<uint32_t(*)[32]>(&s[0]);
-          uint32_t(&t1)[32] = *reinterpret_cast<uint32_t(*)[32]>(&s[32]);
-          tmem_ld32(t_s, t0);
-          tmem_ld32(t_s + 32, t1);
-          tmem_wait_ld();
-          clear_rest();
-        }
+        float s[kKeys];
 #pragma unroll
-        for (int c = kFCopied / 4; c < kFKT / 4; ++c) {
+        for (int c = 0; c < kKeys; c += 32) tmem_ld32(t_s + c, *reinterpret_cast<uint32_t(*)[32]>(&s[c]));
+        tmem_wait_ld();
+        if (kKeys == kFKT) clear_rest();             // (a tile of 32 keys is the last)
+#pragma unroll
+        for (int c = kFCopied / 4; c < kKeys / 4; ++c) {
           add2(s[4 * c + 0], s[4 * c + 1], b4[c - kFCopied / 4].x, b4[c - kFCopied / 4].y);
           add2(s[4 * c + 2], s[4 * c + 3], b4[c - kFCopied / 4].z, b4[c - kFCopied / 4].w);
         }
@@ -331,25 +333,26 @@ triatt_flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
           const int u = (ug + r < n_u) ? ug + r : 0;
           const float4* mrow = reinterpret_cast<const float4*>(mb + (size_t)u * ldm + kt * kFKT);
 #pragma unroll
-          for (int c4 = 0; c4 < kFKT / 4; ++c4) {
+          for (int c4 = 0; c4 < kKeys / 4; ++c4) {
             const float4 m4 = __ldg(mrow + c4);
             add2(s[4 * c4 + 0], s[4 * c4 + 1], m4.x, m4.y);
             add2(s[4 * c4 + 2], s[4 * c4 + 3], m4.z, m4.w);
           }
         }
-        // tile maximum: four independent chains, so the reduction costs about 8 dependent steps
-        float mq[4];
+        // tile maximum: independent chains of 16, so the reduction costs about 8 dependent steps
+        float mq[kKeys / 16];
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
+        for (int c = 0; c < kKeys / 16; ++c) {
           mq[c] = max3(s[16 * c], s[16 * c + 1], s[16 * c + 2]);
 #pragma unroll
           for (int e = 3; e + 1 < 16; e += 2) mq[c] = max3(mq[c], s[16 * c + e], s[16 * c + e + 1]);
           mq[c] = fmaxf(mq[c], s[16 * c + 15]);
         }
-        const float mt = fmaxf(fmaxf(mq[0], mq[1]), fmaxf(mq[2], mq[3]));
+        float mt = fmaxf(mq[0], mq[1]);
+        if constexpr (kKeys == 64) mt = fmaxf(mt, fmaxf(mq[2], mq[3]));
         // S is in registers and its columns are zero again: the next S may be computed.  Said only here, when the store of the zeros has long
         // arrived, so that nobody waits for it; the next S has the time of the exponentials to come.
-        tmem_wait_st();
+        if (kKeys == kFKT) tmem_wait_st();
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(&bars.s_free[g]);
@@ -359,12 +362,12 @@ triatt_flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         const bool move = __any_sync(0xffffffffu, up) && kt > 0;     // first tile: the P.V product overwrites O
         const float m_old = m_ref[r];
         m_ref[r] = up ? mt : m_old;
-        uint32_t w[kFKT / 2];
+        uint32_t w[kKeys / 2];
         float l0 = 0.f, l1 = 0.f;
         {
           const float nm = -m_ref[r];
 #pragma unroll
-          for (int e = 0; e < kFKT / 2; ++e) {
+          for (int e = 0; e < kKeys / 2; ++e) {
             // fp32 exponentials; P is their rounding to nearest fp16 (one conversion per pair), which is unbiased,
             // so the denominator can sum the fp32 values themselves.
             add2(s[2 * e], s[2 * e + 1], nm, nm);
@@ -382,7 +385,7 @@ triatt_flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         // P.V of the previous item must be through before O is rescaled or the P buffer overwritten
         if (i >= 1) ok = mbar_wait(&bars.pv_done[g], (i - 1) & 1, 256u) && ok;
         ok = __all_sync(0xffffffffu, ok);
-        if (!ok) break;
+        if (!ok) return false;
         tc_fence_after();
         if (move) {
           const float alpha = fast_exp2(m_old - m_ref[r]);
@@ -398,10 +401,10 @@ triatt_flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
           }
         }
         l_sum[r] += l0 + l1;
-        {
-          uint32_t(&w0)[32] = *reinterpret_cast<uint32_t(*)[32]>(&w[0]);
-          tmem_st32(t_p, w0);
-        }
+        if constexpr (kKeys == 64)
+          tmem_st32(t_p, w);
+        else
+          tmem_st16(t_p, w);
         tmem_wait_st();
         tc_fence_before();
         __syncwarp();
@@ -412,6 +415,16 @@ triatt_flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
           if (r == kRpg - 1) mbar_arrive(&bars.bias_empty[kt & 1]);
         }
       }
+      return true;
+    };
+    bool ok = true;
+    for (int kt = 0; kt < nkt - (kBrief ? 1 : 0) && ok; ++kt) {
+      mask_flags(kt);
+      ok = items(kt, std::integral_constant<int, kFKT>{});
+    }
+    if (kBrief && ok) {
+      mask_flags(nkt - 1);
+      ok = items(nkt - 1, std::integral_constant<int, kFKT / 2>{});
     }
     // ---- epilogue: o = O / denominator for this group's rows
     ok = ok && mbar_wait(&bars.pv_done[g], (nkt * kRpg - 1) & 1, 512u);
@@ -504,9 +517,13 @@ extern "C" int32_t px_triatt_flash(const px_f16* q, const px_f16* k, const px_f1
   // number of rows has its own code (as a run-time number, which leaves no parity known to the compiler, 15 % slower).
   const int64_t per = (n + 127) / 128 * kFH, slices = (n_u + kFRows - 1) / kFRows, room = sm_count(), left = per * slices % room;
   const int64_t halves = 2 * left <= room ? (left + per - 1) / per : 0, whole = slices - halves;
-  const auto kernel = halves ? triatt_flash_tc_kernel<true> : triatt_flash_tc_kernel<false>;
-  static SmemLimit limit[2];
-  if (!limit[halves > 0].set(kernel, smem)) return PX_ERR_LAUNCH;
+  // A last key tile of 32 keys at most is worked off by its half, in kernels of their own (the branch costs the others 1 %): N = 150
+  // 20.6 -> 19.2 us, 200 29.8 -> 28.1, 224 36.1 -> 34.1, 528 298 -> 291, 1056 1824 -> 1812, 1300 level.
+  const bool brief = (n - 1) % kFKT < kFKT / 2;
+  const auto kernel = halves ? (brief ? triatt_flash_tc_kernel<true, true> : triatt_flash_tc_kernel<true, false>)
+                             : (brief ? triatt_flash_tc_kernel<false, true> : triatt_flash_tc_kernel<false, false>);
+  static SmemLimit limit[4];
+  if (!limit[2 * (halves > 0) + brief].set(kernel, smem)) return PX_ERR_LAUNCH;
   return launch_pdl(kernel, dim3((unsigned)((n + 127) / 128), kFH, (unsigned)(whole + 2 * halves)), kFThreads, smem, st, mq, mk, mv, mbias,
                     mo, mask_bias, (int)n_u, (int)n, (int)ldm, nkt, (int)whole)
              ? PX_OK
