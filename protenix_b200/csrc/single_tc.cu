@@ -15,8 +15,10 @@
 //   split_gemm RES    s2 = s1 + h W_out^T, the contraction split over a cluster of four CTAs
 // At N tokens each product has N/128 x (outputs/64) tiles: far too few to fill the chip at any N, so every launch is
 // bound by the latency of one tile (load, 16 MMAs per 64 inputs, epilogue); hence narrow 64-column tiles, no
-// persistence, and the split contraction where it is 1536 long.  Whole branch on an idle GPU: 64 us at N = 128 and 76 us at
-// N = 384, where library GEMMs and the composed attention took 290 us; 0.36 ms against 0.76 at N = 1536.
+// persistence, and the split contraction where it is 1536 long.  The epilogue is as long as the products (64 columns of a row, half
+// of them through expf and a division, six accumulators): sixteen warps, 16 columns a thread, and stores from shared memory.  Four
+// warps of 64 columns a thread, storing their rows, against that, each kernel alone at N = 384: QKVG 13.5 -> 9.3 us, SWIGLU 16.1 -> 10.5,
+// RES 9.9 -> 7.8 and 10.4 -> 9.9.
 #include <initializer_list>
 
 #include "px_split.cuh"
@@ -41,9 +43,10 @@ constexpr int kSgStages = 3;
 constexpr int kSgMain = 4;
 constexpr int kSgCorr = kSgBN * kSgMain;  // columns of the corrections: order 2^-8, then order 2^-16
 constexpr int kSgAcc = kSgMain + 2;
-constexpr int kSgEpilogue = 4;            // first of the epilogue's four warps
+constexpr int kSgEpilogue = 4;            // first of the epilogue's warps
+constexpr int kSgEpiWarps = 16;           // four for every 32 rows of the tile, 16 columns each
 constexpr uint32_t kSgCols = 512;
-constexpr int kSgThreads = 32 * (kSgEpilogue + 4);
+constexpr int kSgThreads = 32 * (kSgEpilogue + kSgEpiWarps);
 constexpr int kSgSplit = 4;               // CTAs of a cluster that share a contraction of 1536
 
 enum { kSgQkvg = 0, kSgRes = 1, kSgSwiglu = 2 };
@@ -104,7 +107,8 @@ __device__ __forceinline__ void cluster_sync() {
 }
 
 // One 128 x 64 tile of a split product per cluster (of gridDim.z CTAs, each with its share of the contraction).
-// Warp 0: TMA producer (three planes of A and of W per 64 inputs), warp 1: MMA issuer, warps 4..7: epilogue.
+// Warp 0: TMA producer (three planes of A and of W per 64 inputs), warp 1: MMA issuer, warps 4..19: epilogue, a thread 16 columns of a
+// row, which leave through shared memory so that the stores of a warp are runs of 64 to 256 bytes.
 template <int kMode, typename T>
 __global__ void __launch_bounds__(kSgThreads, 1)
 split_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w, const SgArgs g) {
@@ -144,7 +148,6 @@ split_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
   __syncwarp();
   pdl_wait();
   const uint32_t tmem_base = bars.tmem_base;
-  float v[kSgBN];                                // epilogue: this thread's row of the tile
   bool ok = !skip;
 
   if (warp == 0) {
@@ -187,62 +190,76 @@ split_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
       __syncwarp();
     }
   } else if (warp >= kSgEpilogue) {
-    const int q = warp & 3, r = 32 * q + lane;     // tensor-memory lane = row of the tile
+    // thread: row r of the tile (its tensor-memory lane), columns c0 .. c0 + 7 and c1 .. c1 + 7
+    const int q = warp & 3, r = 32 * q + lane, part = (warp - kSgEpilogue) >> 2, tid = threadIdx.x - 32 * kSgEpilogue;
+    const int c0 = kMode == kSgSwiglu ? 8 * part : 16 * part, c1 = kMode == kSgSwiglu ? kSgBN / 2 + 8 * part : c0 + 8;
     ok = ok && mbar_wait(&bars.acc_full, 0, 4u);
     ok = __all_sync(0xffffffffu, ok);
+    float v[16];
     if (ok) {
       tc_fence_after();
       const uint32_t t = tmem_base + ((uint32_t)(32 * q) << 16);
-      constexpr int kLast = (kSgAcc - 1) * kSgBN;  // corrections first
-      tmem_ld32(t + kLast, *reinterpret_cast<uint32_t(*)[32]>(&v[0]));
-      tmem_ld32(t + kLast + 32, *reinterpret_cast<uint32_t(*)[32]>(&v[32]));
+      uint32_t x[2][16];
 #pragma unroll
-      for (int p = 2 * (kSgAcc - 1) - 1; p >= 0; --p) {
-        uint32_t x[32];
-        tmem_ld32(t + (p >> 1) * kSgBN + 32 * (p & 1), x);
+      for (int p = kSgAcc - 1; p > 0; p -= 2) {    // corrections first
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          tmem_ld8(t + (p - i) * kSgBN + c0, x[i]);
+          tmem_ld8(t + (p - i) * kSgBN + c1, x[i] + 8);
+        }
         tmem_wait_ld();
 #pragma unroll
-        for (int e = 0; e < 32; ++e) v[32 * (p & 1) + e] += __uint_as_float(x[e]);
+        for (int e = 0; e < 16; ++e) {
+          v[e] = p == kSgAcc - 1 ? __uint_as_float(x[0][e]) : v[e] + __uint_as_float(x[0][e]);
+          v[e] += __uint_as_float(x[1][e]);
+        }
       }
-      const int row = m0 + r;
-      if (kMode == kSgQkvg) {
-        const int part = n0 / kSc;                 // q, k, v or g: a tile of 64 lies in one of them
-        if (part == 0) {
+      // the ring is idle: every product of this CTA is complete.  Rows of 16 pieces of 16 bytes, swizzled by row
+      uint4* const stg = reinterpret_cast<uint4*>(ring);
+      if (kMode == kSgSwiglu) {                    // columns 0..31: a, 32..63: b of hidden units n0/2 ..; pieces: plane, eight units
+        uint32_t w[4][3];
 #pragma unroll
-          for (int e = 0; e < kSgBN; ++e) v[e] = (v[e] + __ldg(g.bias + n0 + e)) * g.scale;
-        } else if (part == 3) {
-#pragma unroll
-          for (int e = 0; e < kSgBN; ++e) v[e] = 1.0f / (1.0f + expf(-v[e]));
+        for (int e = 0; e < 4; ++e) {
+          const float a0 = v[2 * e], a1 = v[2 * e + 1];
+          split3x2(a0 / (1.0f + expf(-a0)) * v[8 + 2 * e], a1 / (1.0f + expf(-a1)) * v[8 + 2 * e + 1], w[e]);
         }
-        if (row < g.rows) {
-          float4* dst = reinterpret_cast<float4*>(g.out_f + (size_t)row * kSf + n0);
 #pragma unroll
-          for (int e = 0; e < kSgBN / 4; ++e) dst[e] = make_float4(v[4 * e], v[4 * e + 1], v[4 * e + 2], v[4 * e + 3]);
-        }
-      } else if (kMode == kSgSwiglu) {
-        if (row < g.rows) {                        // columns 0..31: a, 32..63: b of hidden units n0/2 ..
+        for (int p = 0; p < 3; ++p) stg[r * 16 + ((4 * p + part) ^ (r & 15))] = make_uint4(w[0][p], w[1][p], w[2][p], w[3][p]);
+      } else {
+        if (kMode == kSgQkvg) {
+          const int kind = n0 / kSc;               // q, k, v or g: a tile of 64 lies in one of them
+          if (kind == 0) {
 #pragma unroll
-          for (int e = 0; e < 32; e += 8) {
-            uint32_t w[4][3];
+            for (int e = 0; e < 16; ++e) v[e] = (v[e] + __ldg(g.bias + n0 + c0 + e)) * g.scale;
+          } else if (kind == 3) {
 #pragma unroll
-            for (int p = 0; p < 4; ++p) {
-              const float a0 = v[e + 2 * p], a1 = v[e + 2 * p + 1];
-              const float h0 = a0 / (1.0f + expf(-a0)) * v[32 + e + 2 * p];
-              const float h1 = a1 / (1.0f + expf(-a1)) * v[32 + e + 2 * p + 1];
-              split3x2(h0, h1, w[p]);
-            }
-#pragma unroll
-            for (int p = 0; p < 3; ++p)
-              *reinterpret_cast<uint4*>(g.out_planes + ((size_t)p * g.rows + row) * kSf + n0 / 2 + e) =
-                  make_uint4(w[0][p], w[1][p], w[2][p], w[3][p]);
+            for (int e = 0; e < 16; ++e) v[e] = 1.0f / (1.0f + expf(-v[e]));
           }
         }
-      } else {
-        // partial sums to shared memory (the ring is idle: every product of this CTA is complete)
-        float4* stg = reinterpret_cast<float4*>(ring) + r * (kSgBN / 4);
 #pragma unroll
-        for (int e = 0; e < kSgBN / 4; ++e)
-          stg[e ^ (r & 15)] = make_float4(v[4 * e], v[4 * e + 1], v[4 * e + 2], v[4 * e + 3]);
+        for (int e = 0; e < 4; ++e)
+          stg[r * 16 + ((4 * part + e) ^ (r & 15))] = make_uint4(__float_as_uint(v[4 * e]), __float_as_uint(v[4 * e + 1]),
+                                                                 __float_as_uint(v[4 * e + 2]), __float_as_uint(v[4 * e + 3]));
+      }
+    }
+    if (kMode != kSgRes) {
+      ok = named_barrier_all(1, 32 * kSgEpiWarps, ok);
+      if (ok) {
+        const uint4* const stg = reinterpret_cast<const uint4*>(ring);
+        constexpr int kPieces = kMode == kSgSwiglu ? 12 : 16;
+#pragma unroll
+        for (int i = 0; i < 128 * kPieces; i += 32 * kSgEpiWarps) {
+          // SWIGLU: the planes one after the other, four pieces a row
+          const int at = i + tid, p = kMode == kSgSwiglu ? at >> 9 : 0;
+          const int rr = kMode == kSgSwiglu ? (at & 511) >> 2 : at >> 4, c = kMode == kSgSwiglu ? at & 3 : at & 15, row = m0 + rr;
+          if (row < g.rows) {
+            const uint4 o = stg[rr * 16 + ((4 * p + c) ^ (rr & 15))];
+            if (kMode == kSgSwiglu)
+              *reinterpret_cast<uint4*>(g.out_planes + ((size_t)p * g.rows + row) * kSf + n0 / 2 + 8 * c) = o;
+            else
+              *reinterpret_cast<uint4*>(g.out_f + (size_t)row * kSf + n0 + 4 * c) = o;
+          }
+        }
       }
     }
   }
@@ -252,7 +269,7 @@ split_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
     if (warp >= kSgEpilogue && ok) {
       // each CTA sums and writes its share of the rows; a thread takes 16 bytes of a row at a time
       const int split = gridDim.z, per = 128 / split, tid = threadIdx.x - 32 * kSgEpilogue;
-      for (int i = tid; i < per * (kSgBN / 4); i += 128) {
+      for (int i = tid; i < per * (kSgBN / 4); i += 32 * kSgEpiWarps) {
         const int r = blockIdx.z * per + i / (kSgBN / 4), c = i % (kSgBN / 4), row = m0 + r;
         const uint32_t src = smem_u32(ring) + (r * (kSgBN / 4) + (c ^ (r & 15))) * 16;
         float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
