@@ -79,7 +79,7 @@ pair_bias_tc_kernel(const __grid_constant__ CUtensorMap map_z, const PbWeights<k
   const bool skip = cta_begin();         // an earlier bounded wait gave up: do not start new work
   if (threadIdx.x == 32) prefetch_maps(map_z);
   if (threadIdx.x == 0) {
-    tile_bars_init(bars.tile, 1, kF16);
+    tile_bars_init(bars.tile, 1);
     mbar_init(&bars.w_full, 1);
     mbar_init(&bars.acc_full, 1);
     mbar_init(&bars.acc_free, 4);
@@ -108,7 +108,7 @@ pair_bias_tc_kernel(const __grid_constant__ CUtensorMap map_z, const PbWeights<k
   } else if (warp >= 4) {
     float* scale = reinterpret_cast<float*>(sm + PbLayout::scale);
     tile_stats_loop(ctx, eps, warp - 4, lane,
-                        [&](int k, int u, int t, int r, float rstd) { scale[(k % Ctx::kSlots) * 128 + r] = rstd; });
+                        [&](int k, int, int, int r, float rstd, float) { scale[(k % Ctx::kSlots) * 128 + r] = rstd; });
   } else {
     // ------------------------------------------------------------------ epilogue
     const int row = 32 * warp + lane;

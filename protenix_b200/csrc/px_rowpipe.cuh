@@ -201,16 +201,20 @@ constexpr int tile_slots(int stages) { return stages + 2; }
 // The correction rows of standardised rows are all alike: one panel serves every tile.
 constexpr int tile_extras(int stages, bool standardised) { return standardised ? 1 : tile_slots(stages); }
 
+// Barriers that say a tile has arrived: of every one, each set of statistics warps sees all phases or none (a wait on a parity tells a
+// phase from the one before only; tile k + 1 may arrive before tile k), so there is an even number of them.
+constexpr int tile_fulls(int stages) { return stages % 2 ? 2 * stages : stages; }
+
 template <int kStages>
 struct TileBars {
   // raw_full: tile in shared memory; a_ready: statistics, correction rows and scales written;
   // a_empty: every MMA that reads the stage is complete (one commit per issuing thread)
-  uint64_t raw_full[kStages], a_ready[tile_slots(kStages)], a_empty[kStages];
+  uint64_t raw_full[tile_fulls(kStages)], a_ready[tile_slots(kStages)], a_empty[kStages];
 };
 // kStandardised: the rows are a standardised fp16 copy (otherwise bf16 rows of z).
 template <int kStages_, bool kStandardised_>
 struct TileCtx {
-  static constexpr int kStages = kStages_, kSlots = tile_slots(kStages_);
+  static constexpr int kStages = kStages_, kSlots = tile_slots(kStages_), kFulls = tile_fulls(kStages_);
   static constexpr bool kStandardised = kStandardised_;
   unsigned char* tiles;     // kStages x kTileBytes
   unsigned char* extras;    // tile_extras() x kTileExtra (the correction step of a tile runs after its stage is freed)
@@ -219,17 +223,17 @@ struct TileCtx {
   __device__ __forceinline__ unsigned char* extra(int k) const { return extras + (kStandardised ? 0 : (k % kSlots) * kTileExtra); }
 };
 
-// Statistics warps: a thread per row where there is nothing to measure, two for bf16 rows.
-constexpr int tile_stats_warps(bool standardised) { return standardised ? 4 : 8; }
+// Statistics warps: four, a thread per row, where there is nothing to measure; for bf16 rows two sets of four that take the tiles in
+// turn, two threads a row.
+constexpr int kStatsSet = 4;
+constexpr int tile_stats_sets(bool standardised) { return standardised ? 1 : 2; }
+constexpr int tile_stats_warps(bool standardised) { return kStatsSet * tile_stats_sets(standardised); }
 // readers: how many arrivals free a stage besides those of the statistics warps.
 template <int kStages>
-__device__ __forceinline__ void tile_bars_init(TileBars<kStages>& b, int readers, bool standardised) {
-  const int warps = tile_stats_warps(standardised);
-  for (int s = 0; s < kStages; ++s) {
-    mbar_init(&b.raw_full[s], 1);
-    mbar_init(&b.a_empty[s], readers + warps);
-  }
-  for (int s = 0; s < tile_slots(kStages); ++s) mbar_init(&b.a_ready[s], warps);
+__device__ __forceinline__ void tile_bars_init(TileBars<kStages>& b, int readers) {
+  for (int s = 0; s < tile_fulls(kStages); ++s) mbar_init(&b.raw_full[s], 1);
+  for (int s = 0; s < kStages; ++s) mbar_init(&b.a_empty[s], readers + kStatsSet);
+  for (int s = 0; s < tile_slots(kStages); ++s) mbar_init(&b.a_ready[s], kStatsSet);
 }
 
 // One warp: TMA loads of the tiles.
@@ -241,10 +245,11 @@ __device__ __forceinline__ void tile_producer_loop(const Ctx& c, const CUtensorM
     if (!mbar_wait_warp(&c.bars->a_empty[s], (n & 1) ^ 1, 1u)) break;
     if (elect_lane()) {
       const int u = tile / c.tiles_t, t0 = (tile % c.tiles_t) * 128;
-      mbar_expect_tx(&c.bars->raw_full[s], kOperandBytes);
+      uint64_t* const full = &c.bars->raw_full[k % Ctx::kFulls];
+      mbar_expect_tx(full, kOperandBytes);
       const uint32_t dst = smem_u32(c.tiles + s * kTileBytes);
       for (int p = 0; p < 2; ++p)
-        tma_load_3d(dst + p * kPanelBytes, map_z, &c.bars->raw_full[s], 64 * p, c.swap ? u : t0, c.swap ? t0 : u);
+        tma_load_3d(dst + p * kPanelBytes, map_z, full, 64 * p, c.swap ? u : t0, c.swap ? t0 : u);
     }
     __syncwarp();
   }
@@ -276,40 +281,68 @@ __device__ __forceinline__ void bf16_row_stats(const unsigned char* tile, int r,
   mean = x0 + m;
 }
 
-// The statistics warps (`sw` = 0..3, or 0..7 for bf16 rows).  per_row(k, u, t, r, rstd) is called once per
+// The statistics warps (`sw` = 0..3, or 0..7 for bf16 rows).  per_row(k, u, t, r, rstd, fetched) is called once per
 // tile and row with the row's 1/std, before a_ready is signalled.  `kStandardised`: the rows are a standardised copy
 // (mean 0, deviation 1 by construction), so the correction row is (0, 1), written once, and the factor is 1.
-// after(u, t) follows once the stage and the statistics have been handed over: for what nothing in the kernel waits for.
+// fetched: what ahead(u, t) loaded from global memory a tile earlier, so that nothing waits for it between the arrival of a tile and the
+// hand-over.  after(u, t) follows once the stage and the statistics have been handed over: for what nothing in the kernel waits for.
+// A tile's statistics are a chain of 1.3 us (arrival, loads, sums, square roots, hand-over), about what a tile lasts: two sets of four
+// warps work on two tiles, each lane on two rows of its tile at once.  Eight warps on one tile, with the load of the mask on the chain,
+// against that (projections of the triangle multiplication, outgoing, us): bf16 N = 200 15.2 -> 14.5, 384 36.2 -> 31.0, 437 47.0 -> 42.8,
+// 768 118 -> 105.5, 1536 477 -> 424 (the mask alone 111 at 768; without any statistics 96); fp16 rows, which only had the mask
+// there, 384 28.9 -> 27.8, 768 98 -> 94.5, 1536 388 -> 377.
+struct TileNothingAhead {
+  __device__ __forceinline__ float operator()(int, int) const { return 0.f; }
+};
 struct TileNothingAfter {
   __device__ __forceinline__ void operator()(int, int) const {}
 };
-template <typename Ctx, typename PerRow, typename After = TileNothingAfter>
-__device__ __forceinline__ void tile_stats_loop(const Ctx& c, float eps, int sw, int lane, PerRow per_row, After after = After()) {
+template <typename Ctx, typename PerRow, typename Ahead = TileNothingAhead, typename After = TileNothingAfter>
+__device__ __forceinline__ void tile_stats_loop(const Ctx& c, float eps, int sw, int lane, PerRow per_row, Ahead ahead = Ahead(),
+                                                After after = After()) {
   constexpr bool kStandardised = Ctx::kStandardised;
-  const int r = kStandardised ? 32 * sw + lane : 16 * sw + (lane >> 1), half = lane & 1;
-  int k = 0;
-  for (int tile = c.first_tile; tile < c.n_tiles; tile += c.tile_step, ++k) {
+  constexpr int kSets = tile_stats_sets(kStandardised), kRows = kStandardised ? 1 : 2;
+  const int set = kStandardised ? 0 : sw >> 2, half = kStandardised ? 0 : lane & 1;
+  const int r0 = kStandardised ? 32 * sw + lane : 16 * (sw & 3) + (lane >> 1);            // and r0 + 64
+  float next[kRows];
+  const auto fetch = [&](int tile) {
+#pragma unroll
+    for (int j = 0; j < kRows; ++j)
+      next[j] = tile < c.n_tiles ? ahead(tile / c.tiles_t, (tile % c.tiles_t) * 128 + r0 + 64 * j) : 0.f;
+  };
+  fetch(c.first_tile + set * c.tile_step);
+  int k = set;
+  for (int tile = c.first_tile + set * c.tile_step; tile < c.n_tiles; tile += kSets * c.tile_step, k += kSets) {
     const int s = k % Ctx::kStages;
-    const int u = tile / c.tiles_t, t = (tile % c.tiles_t) * 128 + r;
-    float mean = 0.f, std = 1.f, rstd = 1.f;
+    const int u = tile / c.tiles_t, t0 = (tile % c.tiles_t) * 128 + r0;
+    float fetched[kRows], mean[kRows], var[kRows];
+#pragma unroll
+    for (int j = 0; j < kRows; ++j) fetched[j] = next[j];
+    fetch(tile + kSets * c.tile_step);
     // for standardised rows the arrival of the tile only paces this loop, so that the slots it writes are those of tiles in flight
-    if (!mbar_wait_warp(&c.bars->raw_full[s], (k / Ctx::kStages) & 1, 16u)) break;
-    if (!kStandardised) {
-      float var;
-      bf16_row_stats(c.tiles + s * kTileBytes, r, half, mean, var);
-      rstd = rsqrtf(var + eps);
-      std = sqrtf(var + eps);
+    if (!mbar_wait_warp(&c.bars->raw_full[k % Ctx::kFulls], (k / Ctx::kFulls) & 1, 16u)) break;
+    if constexpr (!kStandardised) {
+#pragma unroll
+      for (int j = 0; j < kRows; ++j) bf16_row_stats(c.tiles + s * kTileBytes, r0 + 64 * j, half, mean[j], var[j]);
     }
-    // rstd * (W'x - mean * s + std * t): the row side of the correction step holds (-mean, std)
-    if (kStandardised ? k == 0 : half == 0) write_correction_row(c.extra(k), r, -mean, std, false);
-    if (kStandardised || half == 0) per_row(k, u, t, r, rstd);
+#pragma unroll
+    for (int j = 0; j < kRows; ++j) {
+      const float rstd = kStandardised ? 1.f : rsqrtf(var[j] + eps);
+      // rstd * (W'x - mean * s + std * t): the row side of the correction step holds (-mean, std)
+      if (kStandardised ? k == 0 : half == 0)
+        write_correction_row(c.extra(k), r0 + 64 * j, kStandardised ? -0.f : -mean[j], kStandardised ? 1.f : sqrtf(var[j] + eps), false);
+      if (half == 0) per_row(k, u, t0 + 64 * j, r0 + 64 * j, rstd, fetched[j]);
+    }
     asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
     __syncwarp();
     if (lane == 0) {
       mbar_arrive(&c.bars->a_ready[k % Ctx::kSlots]);
       mbar_arrive(&c.bars->a_empty[s]);                 // after the last use of what was read from the stage
     }
-    if (kStandardised || half == 0) after(u, t);
+    if (half == 0) {
+#pragma unroll
+      for (int j = 0; j < kRows; ++j) after(u, t0 + 64 * j);
+    }
   }
 }
 
@@ -328,10 +361,10 @@ __device__ __forceinline__ void tile_product_loop(const Ctx& c, uint32_t d_tmem,
   const uint32_t idesc_corr = idesc | (1u << 7) | (1u << 10);
   int k = 0;
   for (int tile = c.first_tile; tile < c.n_tiles; tile += c.tile_step, ++k) {
-    const int s = k % Ctx::kStages, n = k / Ctx::kStages;
+    const int s = k % Ctx::kStages;
     const int ab = n_acc == 2 ? (k & 1) : 0, an = n_acc == 2 ? (k >> 1) : k;
     const uint32_t d = d_tmem + ab * acc_cols;
-    if (!mbar_wait_warp(&c.bars->raw_full[s], n & 1, 4u) || !mbar_wait_warp(&acc_free[ab], (an & 1) ^ 1, 8u)) break;
+    if (!mbar_wait_warp(&c.bars->raw_full[k % Ctx::kFulls], (k / Ctx::kFulls) & 1, 4u) || !mbar_wait_warp(&acc_free[ab], (an & 1) ^ 1, 8u)) break;
     tc_fence_after();
     if (elect_lane()) {
       const uint32_t a_addr = smem_u32(c.tiles + s * kTileBytes);

@@ -73,7 +73,7 @@ recycle_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_consta
     if (kTma) prefetch_maps(map_init, map_out);
   }
   if (threadIdx.x == 0) {
-    tile_bars_init(bars.tile, 1, kF16);
+    tile_bars_init(bars.tile, 1);
     mbar_init(&bars.w_full, 1);
     mbar_init(&bars.acc_full, 1);
     mbar_init(&bars.acc_free, 8);
@@ -128,7 +128,7 @@ recycle_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_consta
   } else if (warp >= 8) {
     float* scale = reinterpret_cast<float*>(sm + RcLayout::scale);
     tile_stats_loop(ctx, eps, warp - 8, lane,
-                        [&](int k, int u, int t, int r, float rstd) { scale[(k % Ctx::kSlots) * 128 + r] = rstd; });
+                        [&](int k, int, int, int r, float rstd, float) { scale[(k % Ctx::kSlots) * 128 + r] = rstd; });
   } else {
     // ------------------------------------------------------------------ output rows
     const int half = (warp >> 2) & 1, qw = warp & 3;

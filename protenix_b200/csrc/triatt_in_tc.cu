@@ -105,7 +105,7 @@ triatt_in_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_cons
   const bool skip = cta_begin();         // an earlier bounded wait gave up: do not start new work
   if (threadIdx.x == 32) prefetch_maps(map_z, map_v, map_q, map_k);
   if (threadIdx.x == 0) {
-    tile_bars_init(bars.tile, 2, kF16);
+    tile_bars_init(bars.tile, 2);
     mbar_init(&bars.w_full, 1);
     for (int b = 0; b < 4; ++b) {
       mbar_init(&bars.acc_full[b >> 1][b & 1], 1);
@@ -146,7 +146,8 @@ triatt_in_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_cons
     float2* scale = reinterpret_cast<float2*>(sm + Layout::scale);
     tile_stats_loop(
         ctx, eps, warp - 16, lane,
-        [&](int k, int, int t, int r, float rstd) { scale[(k % Ctx::kSlots) * 128 + r] = make_float2(rstd, t < n ? rstd : 0.f); },
+        [&](int k, int, int t, int r, float rstd, float) { scale[(k % Ctx::kSlots) * 128 + r] = make_float2(rstd, t < n ? rstd : 0.f); },
+        TileNothingAhead(),
         [&](int u, int t) {
           if (hpair == 0 && t < ldm) {                   // mask bias, -inf in the pad columns [n, ldm)
             float mv = -CUDART_INF_F;

@@ -101,7 +101,7 @@ triatt_out_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_con
   }
   if (threadIdx.x == 0) {
     // a stage is read by the gate product and the output warps
-    tile_bars_init(bars.tile, 2, kF16);
+    tile_bars_init(bars.tile, 2);
     mbar_init(&bars.w_full, 1);
     mbar_init(&bars.g_full, 1);
     mbar_init(&bars.g_free, 8);
@@ -183,7 +183,7 @@ triatt_out_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_con
     // ------------------------------------------------------------------ row statistics (bf16 rows: two lanes a row)
     float* scale = reinterpret_cast<float*>(sm + AoLayout::scale);
     tile_stats_loop(ctx, eps, warp - 16, lane,
-                        [&](int k, int u, int t, int r, float rstd) { scale[(k % Ctx::kSlots) * 128 + r] = rstd; });
+                        [&](int k, int, int, int r, float rstd, float) { scale[(k % Ctx::kSlots) * 128 + r] = rstd; });
   } else if (warp < 8) {
     // ------------------------------------------------------------------ gate: o * sigmoid(g) -> tensor memory
     const int half = warp >> 2, qw = warp & 3;

@@ -92,7 +92,7 @@ trimul_in_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_cons
   const bool skip = cta_begin();         // an earlier bounded wait gave up: do not start new work
   if (threadIdx.x == 32) prefetch_maps(map_z, map_a, map_b);
   if (threadIdx.x == 0) {
-    tile_bars_init(bars.tile, 2, kF16);
+    tile_bars_init(bars.tile, 2);
     mbar_init(&bars.w_full, 1);
     for (int b = 0; b < 4; ++b) {
       mbar_init(&bars.acc_full[b >> 1][b & 1], 1);
@@ -127,11 +127,12 @@ trimul_in_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_cons
   } else if (warp >= 16) {
     // ------------------------------------------------------------------ row statistics (bf16 rows: two lanes a row)
     float2* scale = reinterpret_cast<float2*>(sm + TiLayout::scale);
-    tile_stats_loop(ctx, eps, warp - 16, lane, [&](int k, int u, int t, int r, float rstd) {
-      float mk = 0.f;
-      if (t < n_t) mk = mask ? __ldg(mask + (swap ? ((size_t)t * n_u + u) : ((size_t)u * n_t + t))) : 1.f;
-      scale[(k % Ctx::kSlots) * 128 + r] = make_float2(rstd, 0.5f * rstd * mk);
-    });
+    tile_stats_loop(
+        ctx, eps, warp - 16, lane,
+        [&](int k, int, int, int r, float rstd, float mk) { scale[(k % Ctx::kSlots) * 128 + r] = make_float2(rstd, 0.5f * rstd * mk); },
+        [&](int u, int t) {
+          return t >= n_t ? 0.f : mask ? __ldg(mask + (swap ? ((size_t)t * n_u + u) : ((size_t)u * n_t + t))) : 1.f;
+        });
   } else {
     // ------------------------------------------------------------------ epilogue of output ph
     const int ph = warp >> 3, half = (warp >> 2) & 1, qw = warp & 3;
