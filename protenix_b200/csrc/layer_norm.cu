@@ -41,12 +41,20 @@ __device__ __forceinline__ float param(P v) { return Cvt<T>::to_f(Cvt<T>::from_f
 
 constexpr int kMaxIt = 8;
 
+// Launch of 256 threads a CTA that overlaps the end of the kernel before it (see pdl_wait): [384, 384] fp32 8.5 -> 7.9 us a call, forward
+// and backward of [768^2, 128] bf16 141.9 -> 136.8.
+template <typename... Params, typename... Args>
+static cudaError_t pdl(void (*kernel)(Params...), unsigned grid, size_t smem, cudaStream_t st, Args... args) {
+  return launch_pdl(kernel, dim3(grid), 256, smem, st, args...) ? cudaSuccess : cudaErrorLaunchFailure;
+}
+
 // Register-resident path: cols <= 32 * VEC * kMaxIt.
 template <typename T, int VEC, typename P>
 __global__ void __launch_bounds__(256) ln_fwd_cached(const T* __restrict__ x, const P* __restrict__ gamma,
                                                      const P* __restrict__ beta, T* __restrict__ y,
                                                      float* __restrict__ mean_out, float* __restrict__ invvar_out,
                                                      int64_t rows, int cols, float eps) {
+  pdl_wait();
   const int lane = threadIdx.x & 31;
   const int64_t warp0 = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int64_t nwarps = (int64_t)gridDim.x * (blockDim.x >> 5);
@@ -122,6 +130,7 @@ __global__ void __launch_bounds__(256, kLnFwdOcc) ln_fwd_rows16(const T* __restr
                                                                 const P* __restrict__ beta, T* __restrict__ y,
                                                                 float* __restrict__ mean_out, float* __restrict__ invvar_out,
                                                                 int64_t rows, float eps) {
+  pdl_wait();
   constexpr int VEC = 16 / (int)sizeof(T), kCols = VEC * LANES, kR = 32 / LANES, kB = kLnFwdGroups;
   const int lane = threadIdx.x & 31, sub = lane / LANES, li = lane % LANES;
   const int64_t warp0 = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -199,9 +208,7 @@ static cudaError_t launch_rows16(const void* x, const void* g, const void* b, vo
   int64_t ctas = (rows + rows_per_cta - 1) / rows_per_cta;
   const int64_t cap = 148 * kLnFwdOcc;
   if (ctas > cap) ctas = cap;
-  ln_fwd_rows16<T, LANES, P><<<(unsigned)ctas, 256, 0, st>>>((const T*)x, (const P*)g, (const P*)b, (T*)y, mean, invvar, rows,
-                                                          eps);
-  return cudaGetLastError();
+  return pdl(ln_fwd_rows16<T, LANES, P>, (unsigned)ctas, 0, st, (const T*)x, (const P*)g, (const P*)b, (T*)y, mean, invvar, rows, eps);
 }
 
 // Wide rows: three passes over the row (the second and third hit L1/L2).
@@ -246,9 +253,7 @@ static cudaError_t launch_cached(const void* x, const void* g, const void* b, vo
   int64_t ctas = (rows + warps_per_cta - 1) / warps_per_cta;
   const int64_t cap = 148 * 8 * 4;  // a few waves of resident CTAs; warps stride over the rows
   if (ctas > cap) ctas = cap;
-  ln_fwd_cached<T, VEC, P><<<(unsigned)ctas, 256, 0, st>>>((const T*)x, (const P*)g, (const P*)b, (T*)y, mean, invvar,
-                                                         rows, cols, eps);
-  return cudaGetLastError();
+  return pdl(ln_fwd_cached<T, VEC, P>, (unsigned)ctas, 0, st, (const T*)x, (const P*)g, (const P*)b, (T*)y, mean, invvar, rows, cols, eps);
 }
 
 template <typename T, typename P>
@@ -299,6 +304,7 @@ __global__ void __launch_bounds__(256, IT == 1 ? kLnBwdOcc : 1) ln_bwd_rows(cons
                                                    const float* __restrict__ mean, const float* __restrict__ invvar,
                                                    const P* __restrict__ gamma, T* __restrict__ dx,
                                                    float* __restrict__ scratch, long long rows, int cols) {
+  pdl_wait();
   constexpr int VEC = 16 / (int)sizeof(T), kR = 32 / LANES;
   constexpr int kB = ln_bwd_groups(IT, (int)sizeof(T));                  // row groups in flight per warp
   extern __shared__ float ln_bwd_sums[];                 // [8 warps][2][cols]
@@ -458,10 +464,18 @@ __global__ void __launch_bounds__(256) ln_bwd_wide(const T* __restrict__ dy, con
   }
 }
 
+// A kernel and not a memset: between kernels alone a launch overlaps the end of the kernel before it.
+__global__ void __launch_bounds__(256) ln_bwd_zero_kernel(float* __restrict__ scratch, int n) {
+  pdl_wait();
+  const int i = blockIdx.x * 256 + threadIdx.x;
+  if (i < n) scratch[i] = 0.f;
+}
+
 // The sums are rounded to the type of x, whatever the type of the gradients (fp32 parameters of a 16-bit x).
 template <typename T, typename P>
 __global__ void ln_bwd_finish_kernel(const float* __restrict__ scratch, P* __restrict__ dgamma, P* __restrict__ dbeta,
                                      int cols) {
+  pdl_wait();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= cols) return;
   if (dgamma) dgamma[c] = Cvt<P>::from_f(Cvt<T>::to_f(Cvt<T>::from_f(scratch[c])));
@@ -475,9 +489,8 @@ static cudaError_t launch_bwd_rows(const void* dy, const void* x, const float* m
   const size_t smem = scratch ? (size_t)16 * cols * sizeof(float) : 0;
   const long long want = (rows + kRows - 1) / kRows;
   const int grid = (int)(want < kLnBwdOcc * sms ? want : (long long)kLnBwdOcc * sms);   // resident CTAs: every extra one adds 2 * cols atomics
-  ln_bwd_rows<T, P, LANES, IT><<<grid, 256, smem, st>>>((const T*)dy, (const T*)x, mean, invvar, (const P*)gamma, (T*)dx, scratch,
-                                                        rows, cols);
-  return cudaGetLastError();
+  return pdl(ln_bwd_rows<T, P, LANES, IT>, (unsigned)grid, smem, st, (const T*)dy, (const T*)x, mean, invvar, (const P*)gamma, (T*)dx,
+             scratch, rows, cols);
 }
 
 template <typename T, typename P>
@@ -487,7 +500,7 @@ static cudaError_t dispatch_bwd(const void* dy, const void* x, const float* mean
   const bool sums = dgamma || dbeta;
   if (!sums) scratch = nullptr;
   if (sums) {
-    const cudaError_t e = cudaMemsetAsync(scratch, 0, (size_t)2 * cols * sizeof(float), st);
+    const cudaError_t e = pdl(ln_bwd_zero_kernel, (unsigned)((2 * cols + 255) / 256), 0, st, scratch, 2 * cols);
     if (e != cudaSuccess) return e;
   }
   int dev = 0, sms = 148;
@@ -516,8 +529,8 @@ static cudaError_t dispatch_bwd(const void* dy, const void* x, const float* mean
     if (e != cudaSuccess) return e;
   }
   if (sums)
-    ln_bwd_finish_kernel<T, P><<<(cols + 255) / 256, 256, 0, st>>>(scratch, (P*)dgamma, (P*)dbeta, cols);
-  return cudaGetLastError();
+    return pdl(ln_bwd_finish_kernel<T, P>, (unsigned)((cols + 255) / 256), 0, st, (const float*)scratch, (P*)dgamma, (P*)dbeta, cols);
+  return cudaSuccess;
 }
 
 // Calls f<T, P> for the type of x and of the parameters (that of x, or fp32).
