@@ -630,7 +630,9 @@ c10::cuda::CUDAStream side_stream(const Use& use) {
 // transition only beside the second core: 145 at N = 128, 276 against 278 at 200, 720 against 719 at 384.
 // One block alone: its projections of s, which need no bias, beside its own pair path (224 | 216 at N = 128, no difference from 200 on).
 // Everything is allocated on the caller's stream, which waits for the side stream before this returns.
-constexpr int64_t kBesideBelow = 1281, kProjectFirstUpTo = 256;
+// Where the main stream waits for the side stream before it writes a pair-bias buffer anew, the launch behind does not overlap the kernel
+// before.  Up to kManyBiasUpTo tokens there are eight buffers (together as large as an fp32 z) and one such wait in four blocks.
+constexpr int64_t kBesideBelow = 1281, kProjectFirstUpTo = 256, kManyBiasUpTo = 384;
 std::tuple<OptTensor, Tensor> stack_forward(const std::vector<std::shared_ptr<Block>>& blocks, const OptTensor& s_in,
                                             const Tensor& z, const OptTensor& mask, bool inplace) {
   bool batch;
@@ -671,12 +673,15 @@ std::tuple<OptTensor, Tensor> stack_forward(const std::vector<std::shared_ptr<Bl
   const bool first = n <= kProjectFirstUpTo;       // projections of s beside the pair path of the first block from its start on
   const bool aside = singles && (blocks.size() > 1 ? n < kBesideBelow : first);
   const auto side = aside ? side_stream(use) : main;
-  Tensor bias[2], sb[2], sws;
+  // update k of s has bias buffer k % (2 * per_wait); the main stream waits before every per_wait-th for those of the round before
+  const int64_t per_wait = n <= kManyBiasUpTo ? 4 : 1;
+  std::vector<Tensor> bias;
+  Tensor sb[2], sws;
   at::cuda::CUDAEvent gate, side_done[2];
-  int64_t waiting = -1;             // block whose bias is made and whose update is still to be issued
-  int waiting_turn = 0;
+  int64_t waiting = -1;             // block whose bias is made and whose update, number k - 1, is still to be issued
   if (singles) {
-    for (int i = 0; i < (blocks.size() > 1 ? 2 : 1); ++i) bias[i] = at::empty({kHeadsSingle, n, n}, zc.options().dtype(at::kFloat));
+    for (int64_t i = 0; i < std::min<int64_t>(blocks.size(), 2 * per_wait); ++i)
+      bias.push_back(at::empty({kHeadsSingle, n, n}, zc.options().dtype(at::kFloat)));
     for (int i = 0; i < (blocks.size() > 1 ? 2 : 1); ++i) sb[i] = at::empty_like(s);
     sws = bytes_like(zc, abi.px_single_workspace_bytes(n));
     if (aside) {
@@ -708,9 +713,10 @@ std::tuple<OptTensor, Tensor> stack_forward(const std::vector<std::shared_ptr<Bl
       gate.record(main);
       gate.block(side);
       if (waiting >= 0) {
-        single_finish(side, *ready[waiting].single, zf, s, sb[waiting_turn], bias[waiting_turn], sws);
-        side_done[waiting_turn].record(side);
-        s = sb[waiting_turn];
+        const int64_t done = k - 1;
+        single_finish(side, *ready[waiting].single, zf, s, sb[done & 1], bias[done % bias.size()], sws);
+        if (k % per_wait == 0) side_done[(k / per_wait) & 1].record(side);      // updates up to k - 1
+        s = sb[done & 1];
         waiting = -1;
       }
       if (r.single && !(first && b == 0)) single_project(side, *r.single, zf, s, sws);
@@ -719,17 +725,18 @@ std::tuple<OptTensor, Tensor> stack_forward(const std::vector<std::shared_ptr<Bl
     rows.valid = false;
     transition_rows(c.st, *r.transition, zf, c.dt, z, z, n * n, true);
     if (!r.single) continue;
-    const int turn = k & 1;
+    const Tensor& pair_bias = bias[k % bias.size()];
     // the copy for the pair bias also serves the next block's first update
     if (fp32) rows.need(c, z, r.pair_bias->scalars[0]);
-    if (aside && k >= 2) side_done[turn].block(main);       // the single branch two blocks ago has read this buffer
+    // the updates that read this and the next buffers last, up to number k - per_wait - 1, are through
+    if (aside && k >= 2 * per_wait && k % per_wait == 0) side_done[(k / per_wait - 1) & 1].block(main);
     const auto& p = r.pair_bias->p[zf];
     launch("px_pair_bias_proj", c.st, [&] {
-      return abi.px_pair_bias_proj_folded(fp32 ? rows.zn : z, fp32 ? PX_F16 : PX_BF16, p[0], (float*)bias[turn].data_ptr(), n * n, kHeadsSingle,
+      return abi.px_pair_bias_proj_folded(fp32 ? rows.zn : z, fp32 ? PX_F16 : PX_BF16, p[0], (float*)pair_bias.data_ptr(), n * n, kHeadsSingle,
                                           r.pair_bias->scalars[0], c.st);
     });
     if (aside && (int64_t)b != last) {
-      waiting = b, waiting_turn = turn;
+      waiting = b;
       ++k;
       continue;
     }
@@ -739,8 +746,8 @@ std::tuple<OptTensor, Tensor> stack_forward(const std::vector<std::shared_ptr<Bl
     } else if (!first) {
       single_project(main, *r.single, zf, s, sws);
     }
-    single_finish(main, *r.single, zf, s, sb[turn], bias[turn], sws);
-    s = sb[turn];
+    single_finish(main, *r.single, zf, s, sb[k & 1], pair_bias, sws);
+    s = sb[k & 1];
     ++k;
   }
   return {s.defined() ? OptTensor(s) : OptTensor(), batch ? zc.unsqueeze(0) : zc};
