@@ -236,6 +236,12 @@ __device__ __forceinline__ void tile_bars_init(TileBars<kStages>& b, int readers
   for (int s = 0; s < tile_slots(kStages); ++s) mbar_init(&b.a_ready[s], kStatsSet);
 }
 
+// Where consecutive rows of tiles lie behind one another in every tensor of a kernel (rows of z as they are, and no pad columns), the
+// tiles need not end with each row: one row of n_u * n_t elements has fewer of them unless n_t is a multiple of 128 (both output stages of
+// the triangle multiplication, its outgoing projection and the output stage of the starting node, us a block of a stack: 160 tokens
+// 205.3 -> 196.5, 200 260.5 -> 252.5, 400 914 -> 873; where fewer tiles leave SMs free, the single branch has them).
+static inline bool one_row_pays(int64_t n_u, int64_t n_t) { return n_u > 1 && n_t % 128 != 0; }
+
 // One warp: TMA loads of the tiles.
 template <typename Ctx>
 __device__ __forceinline__ void tile_producer_loop(const Ctx& c, const CUtensorMap* map_z) {

@@ -354,6 +354,7 @@ static int32_t launch_triatt_out(const px_f16* o, const void* z_in, const px_f16
                                  const AoWeights<kMode != 0>& weights, const void* folded, int64_t n_u, int64_t n, int32_t ending,
                                  int32_t add_residual, float eps, cudaStream_t st) {
   CUtensorMap mz, mo, mout;
+  if (!ending && one_row_pays(n_u, n)) n *= n_u, n_u = 1;
   // operand rows: bf16 z itself, or the standardised fp16 copy of an fp32 z; pair element (u, t) is row u*n + t, or
   // row t*n_u + u when the two indices are exchanged
   const CUtensorMapDataType zt = kMode == 0 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
@@ -386,7 +387,7 @@ static int32_t launch_triatt_out(const px_f16* o, const void* z_in, const px_f16
   if (!limit.set(triatt_out_tc_kernel<kMode>, smem)) return PX_ERR_LAUNCH;
   const int64_t tiles_t = (n + 127) / 128, n_tiles = tiles_t * n_u;
   if (n_tiles > 0x7fffffff) return PX_ERR_UNSUPPORTED;
-  const int grid = even_grid(n_tiles, sm_count(), n % 128 ? tiles_t : 1);
+  const int grid = even_grid(n_tiles, sm_count(), n % 128 && n_u > 1 ? tiles_t : 1);
   return launch_pdl(triatt_out_tc_kernel<kMode>, dim3(grid), ao_threads(kMode != 0), smem, st, mz, mo, mout, z_in, z_out, weights,
                     (const unsigned char*)folded, (int)n_u, (int)n, (int)ending, (int)add_residual, eps, (int)tiles_t, (int)n_tiles)
              ? PX_OK

@@ -200,6 +200,7 @@ template <bool kF16>
 static int32_t launch_trimul_in(const void* z, const float* mask, const TiWeights<kF16>& weights, const void* folded, px_f16* a,
                                 px_f16* b, int64_t n_u, int64_t n_t, int64_t ld, int32_t incoming, float eps, cudaStream_t st) {
   CUtensorMap mz, ma, mb;
+  if (!incoming && ld == n_t && one_row_pays(n_u, n_t)) n_t *= n_u, ld = n_t, n_u = 1;
   const CUtensorMapDataType zt = kF16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
   // pair element (u, t) is row u*n_t + t of z, or row t*n_u + u when the two indices are exchanged
   const bool ok = incoming ? make_map_3d(&mz, zt, z, 128, (uint64_t)n_u, (uint64_t)n_t, 256, (uint64_t)n_u * 256, 64, 1,
@@ -218,7 +219,7 @@ static int32_t launch_trimul_in(const void* z, const float* mask, const TiWeight
   if (!limit.set(trimul_in_tc_kernel<kF16>, smem)) return PX_ERR_LAUNCH;
   const int64_t tiles_t = (ld + 127) / 128, n_tiles = tiles_t * n_u;
   if (n_tiles > 0x7fffffff) return PX_ERR_UNSUPPORTED;
-  const int pairs = even_grid(n_tiles, sm_count() / 2, ld % 128 ? tiles_t : 1);
+  const int pairs = even_grid(n_tiles, sm_count() / 2, ld % 128 && n_u > 1 ? tiles_t : 1);
   return launch_pdl(trimul_in_tc_kernel<kF16>, dim3(2 * pairs), ti_threads(kF16), smem, st, mz, ma, mb, mask, weights,
                     (const unsigned char*)folded, (int)n_u, (int)n_t, (int)incoming, eps, (int)tiles_t, (int)n_tiles)
              ? PX_OK

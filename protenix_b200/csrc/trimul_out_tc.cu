@@ -356,6 +356,7 @@ static int32_t launch_trimul_out(const px_f16* x, const void* z_in, const px_f16
                                  const ToWeights<sizeof(Tz) != 2>& weights, const void* folded,
                                  int64_t n_i, int64_t n, int64_t ld, int32_t add_residual, float eps, cudaStream_t st) {
   CUtensorMap mz, mx, mout;
+  if (ld == n && one_row_pays(n_i, n)) n *= n_i, ld = n, n_i = 1;
   // operand rows: bf16 z itself, or the standardised fp16 copy of an fp32 z
   if (!make_map_3d(&mz, sizeof(Tz) == 2 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16,
                    sizeof(Tz) == 2 ? z_in : (const void*)zn, 128, (uint64_t)n, (uint64_t)n_i, 256, (uint64_t)n * 256, 64, 128,
@@ -381,7 +382,7 @@ static int32_t launch_trimul_out(const px_f16* x, const void* z_in, const px_f16
   if (!limit.set(trimul_out_tc_kernel<Tz, kBulk>, smem)) return PX_ERR_LAUNCH;
   const int64_t tiles_j = (n + 127) / 128, n_tiles = tiles_j * n_i;
   if (n_tiles > 0x7fffffff) return PX_ERR_UNSUPPORTED;
-  const int grid = even_grid(n_tiles, sm_count(), n % 128 ? tiles_j : 1);
+  const int grid = even_grid(n_tiles, sm_count(), n % 128 && n_i > 1 ? tiles_j : 1);
   return launch_pdl(trimul_out_tc_kernel<Tz, kBulk>, dim3(grid), to_threads(sizeof(Tz) != 2), smem, st, mz, mx, mout, (const Tz*)z_in, (Tz*)z_out, weights,
                     (const unsigned char*)folded, (int)n_i, (int)n, (int)add_residual, eps, (int)tiles_j, (int)n_tiles)
              ? PX_OK

@@ -49,3 +49,14 @@ def test_trimul_in_is_the_same_every_time(dtype):
         differs += int(not (torch.equal(again[0], first[0]) and torch.equal(again[1], first[1])))
     assert differs == 0
     ops.device_error_flags()
+
+
+@pytest.mark.parametrize("n", [8, 40, 136, 200])
+def test_tiles_across_rows_equal_a_slab_of_one(n):
+    """Without pad columns the tiles of the outgoing projection run on from row to row; a slab of one row has them by itself."""
+    z, mask, w = inputs(n, n, torch.float32, False)
+    a, b = ops.trimul_in_proj(z, mask, *w, False)
+    for u in (0, n // 2, n - 1):
+        pa, pb = ops.trimul_in_proj(z[u:u + 1].contiguous(), mask[u:u + 1].contiguous(), *w, False)
+        assert torch.equal(pa[:, 0], a[:, u]) and torch.equal(pb[:, 0], b[:, u])
+    ops.device_error_flags()
