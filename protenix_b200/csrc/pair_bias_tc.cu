@@ -71,7 +71,7 @@ pair_bias_tc_kernel(const __grid_constant__ CUtensorMap map_z, const PbWeights<k
   ctx.first_tile = blockIdx.x;
   ctx.tile_step = gridDim.x;
   ctx.n_tiles = n_tiles;
-  ctx.tiles_t = n_tiles;                                 // the rows are one long line of tiles: u = 0, t = row
+  ctx.runs_t = n_tiles;                                  // the rows are one long line of tiles: u = 0, t = row
   ctx.n_u = 1;
   ctx.n_t = (int)rows;
   ctx.swap = 0;

@@ -177,8 +177,8 @@ __device__ __forceinline__ void named_barrier(int id, int threads) {
 
 // ---------------------------------------------------------------------------------------------------------------
 // Row tiles: the part of the pipeline that is the same for every kernel that consumes LayerNorm'd pair rows.
-// A tile is 128 pair elements (one u, 128 consecutive t); element (u, t) is row u*n_t + t of z, or row t*n_u + u when
-// the two indices are exchanged (`swap`).  A stage of the ring holds the tile as two k panels of 128 rows.
+// A tile is 128 pair elements: 128 consecutive t of one u, or two runs of 64, each of one u; element (u, t) is row u*n_t + t of z, or row
+// t*n_u + u when the two indices are exchanged (`swap`).  A stage of the ring holds the tile as two k panels of 128 rows.
 //   * producer thread: TMA loads of the rows (bf16 rows of z, or the standardised fp16 copy of an fp32 z);
 //   * statistics threads: mean and variance of the row as it lies in the stage (bf16 rows), correction row (-mean, std),
 //     and whatever the kernel wants per row.  For standardised rows the statistics are known: (0, 1).  A product Z Z^T
@@ -212,14 +212,15 @@ struct TileBars {
   uint64_t raw_full[tile_fulls(kStages)], a_ready[tile_slots(kStages)], a_empty[kStages];
 };
 // kStandardised: the rows are a standardised fp16 copy (otherwise bf16 rows of z).
-template <int kStages_, bool kStandardised_>
+template <int kStages_, bool kStandardised_, int kRun_ = 128>
 struct TileCtx {
   static constexpr int kStages = kStages_, kSlots = tile_slots(kStages_), kFulls = tile_fulls(kStages_);
   static constexpr bool kStandardised = kStandardised_;
+  static constexpr int kRun = kRun_;          // elements of a run: 128 or 64
   unsigned char* tiles;     // kStages x kTileBytes
   unsigned char* extras;    // tile_extras() x kTileExtra (the correction step of a tile runs after its stage is freed)
   TileBars<kStages_>* bars;
-  int first_tile, tile_step, n_tiles, tiles_t, n_u, n_t, swap;
+  int first_tile, tile_step, n_tiles, runs_t, n_u, n_t, swap;   // runs_t: runs that cover the t of one u
   __device__ __forceinline__ unsigned char* extra(int k) const { return extras + (kStandardised ? 0 : (k % kSlots) * kTileExtra); }
 };
 
@@ -236,13 +237,38 @@ __device__ __forceinline__ void tile_bars_init(TileBars<kStages>& b, int readers
   for (int s = 0; s < tile_slots(kStages); ++s) mbar_init(&b.a_ready[s], kStatsSet);
 }
 
+// Run number `run`: which u, and its first t.  With runs of 64 tile k is made of the runs 2 k and 2 k + 1, which lie behind one another or are
+// the end of one u and the beginning of the next; the second run of the last tile may be none (u = n_u: loads give zeros, nothing is
+// stored).  In tiles of 128 t of one u a length just above a multiple of 128 pays for half a tile more.
+struct Run {
+  int u, t;
+};
+template <int kRun>
+__device__ __forceinline__ Run run_at(int run, int runs_t) {
+  const int u = run / runs_t;
+  return {u, (run - u * runs_t) * kRun};
+}
+static inline int64_t runs_of(int64_t n_t, int run) { return (n_t + run - 1) / run; }
+static inline int64_t tiles_of(int64_t n_u, int64_t n_t, int run) { return (n_u * runs_of(n_t, run) * run + 127) / 128; }
+// Tiles of unlike size (ragged runs) recur every so many (for even_grid).
+static inline int64_t tile_period(int64_t n_u, int64_t n_t, int run) {
+  const int64_t runs = runs_of(n_t, run);
+  return n_u == 1 || n_t % run == 0 ? 1 : run == 64 && runs % 2 == 0 ? runs / 2 : runs;
+}
+
 // Where consecutive rows of tiles lie behind one another in every tensor of a kernel (rows of z as they are, and no pad columns), the
-// tiles need not end with each row: one row of n_u * n_t elements has fewer of them unless n_t is a multiple of 128 (both output stages of
+// tiles need not end with each row: one row of n_u * n_t elements has fewer of them unless n_t is a multiple of 64 (both output stages of
 // the triangle multiplication, its outgoing projection and the output stage of the starting node, us a block of a stack: 160 tokens
 // 205.3 -> 196.5, 200 260.5 -> 252.5, 400 914 -> 873; where fewer tiles leave SMs free, the single branch has them).
-static inline bool one_row_pays(int64_t n_u, int64_t n_t) { return n_u > 1 && n_t % 128 != 0; }
+static inline bool one_row_pays(int64_t n_u, int64_t n_t) { return n_u > 1 && n_t % 64 != 0; }
 
-// One warp: TMA loads of the tiles.
+// Projections: tiles of two runs where that makes fewer of them.  They load and store twice as many pieces, which costs whole tiles 2 (fp16)
+// to 6 % (bf16), hence up to 1024.  Incoming projection of the triangle multiplication, us, one run of 128 | two of 64: bf16 N = 136
+// 11.4 | 10.3, 437 43.5 | 41.0, 700 97.3 | 95.2, whole tiles 384 31.7 | 33.3; fp16 437 40.2 | 38.7, 700 93.2 | 86.3, 768 95.9 | 98.0.
+// The output stages, which nothing but the loads tells of it, take runs of 64 always.
+static inline bool two_runs_pay(int64_t n_u, int64_t n_t) { return n_u > 1 && n_t < 1024 && (n_t - 1) % 128 < 64; }
+
+// One warp: TMA loads of the tiles (boxes of a run).
 template <typename Ctx>
 __device__ __forceinline__ void tile_producer_loop(const Ctx& c, const CUtensorMap* map_z) {
   int k = 0;
@@ -250,12 +276,15 @@ __device__ __forceinline__ void tile_producer_loop(const Ctx& c, const CUtensorM
     const int s = k % Ctx::kStages, n = k / Ctx::kStages;
     if (!mbar_wait_warp(&c.bars->a_empty[s], (n & 1) ^ 1, 1u)) break;
     if (elect_lane()) {
-      const int u = tile / c.tiles_t, t0 = (tile % c.tiles_t) * 128;
       uint64_t* const full = &c.bars->raw_full[k % Ctx::kFulls];
       mbar_expect_tx(full, kOperandBytes);
       const uint32_t dst = smem_u32(c.tiles + s * kTileBytes);
-      for (int p = 0; p < 2; ++p)
-        tma_load_3d(dst + p * kPanelBytes, map_z, full, 64 * p, c.swap ? u : t0, c.swap ? t0 : u);
+      constexpr int kPer = 128 / Ctx::kRun;
+      for (int h = 0; h < kPer; ++h) {
+        const Run r = run_at<Ctx::kRun>(kPer * tile + h, c.runs_t);
+        for (int p = 0; p < 2; ++p)
+          tma_load_3d(dst + p * kPanelBytes + h * (Ctx::kRun * 128), map_z, full, 64 * p, c.swap ? r.u : r.t, c.swap ? r.t : r.u);
+      }
     }
     __syncwarp();
   }
@@ -310,17 +339,25 @@ __device__ __forceinline__ void tile_stats_loop(const Ctx& c, float eps, int sw,
   constexpr int kSets = tile_stats_sets(kStandardised), kRows = kStandardised ? 1 : 2;
   const int set = kStandardised ? 0 : sw >> 2, half = kStandardised ? 0 : lane & 1;
   const int r0 = kStandardised ? 32 * sw + lane : 16 * (sw & 3) + (lane >> 1);            // and r0 + 64
+  const auto where = [&](int tile, int j) {           // (u, t) of row j of this lane
+    constexpr int kPer = 128 / Ctx::kRun;
+    const int row = r0 + 64 * j;
+    Run r = run_at<Ctx::kRun>(kPer * tile + (kPer == 2 ? row >> 6 : 0), c.runs_t);
+    r.t += row % Ctx::kRun;
+    return r;
+  };
   float next[kRows];
   const auto fetch = [&](int tile) {
 #pragma unroll
-    for (int j = 0; j < kRows; ++j)
-      next[j] = tile < c.n_tiles ? ahead(tile / c.tiles_t, (tile % c.tiles_t) * 128 + r0 + 64 * j) : 0.f;
+    for (int j = 0; j < kRows; ++j) {
+      const Run r = where(tile, j);
+      next[j] = tile < c.n_tiles ? ahead(r.u, r.t) : 0.f;
+    }
   };
   fetch(c.first_tile + set * c.tile_step);
   int k = set;
   for (int tile = c.first_tile + set * c.tile_step; tile < c.n_tiles; tile += kSets * c.tile_step, k += kSets) {
     const int s = k % Ctx::kStages;
-    const int u = tile / c.tiles_t, t0 = (tile % c.tiles_t) * 128 + r0;
     float fetched[kRows], mean[kRows], var[kRows];
 #pragma unroll
     for (int j = 0; j < kRows; ++j) fetched[j] = next[j];
@@ -337,7 +374,10 @@ __device__ __forceinline__ void tile_stats_loop(const Ctx& c, float eps, int sw,
       // rstd * (W'x - mean * s + std * t): the row side of the correction step holds (-mean, std)
       if (kStandardised ? k == 0 : half == 0)
         write_correction_row(c.extra(k), r0 + 64 * j, kStandardised ? -0.f : -mean[j], kStandardised ? 1.f : sqrtf(var[j] + eps), false);
-      if (half == 0) per_row(k, u, t0 + 64 * j, r0 + 64 * j, rstd, fetched[j]);
+      if (half == 0) {
+        const Run r = where(tile, j);
+        per_row(k, r.u, r.t, r0 + 64 * j, rstd, fetched[j]);
+      }
     }
     asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
     __syncwarp();
@@ -347,7 +387,10 @@ __device__ __forceinline__ void tile_stats_loop(const Ctx& c, float eps, int sw,
     }
     if (half == 0) {
 #pragma unroll
-      for (int j = 0; j < kRows; ++j) after(u, t0 + 64 * j);
+      for (int j = 0; j < kRows; ++j) {
+        const Run r = where(tile, j);
+        after(r.u, r.t);
+      }
     }
   }
 }

@@ -11,7 +11,7 @@
 //   warps 0..7    epilogue of q | k: a thread owns one pair element and both heads of q (warps 0..3) or k (4..7):
 //                 a warp's 32 rows of a head, 2 KB, are staged (64-byte swizzle) and leave by TMA.  Written by their threads in
 //                 pieces of 16 bytes, half a sector each, they took the kernel from 32 to 42 us at N = 384 and from 119 to 144 at N = 768.
-//   warps 8..15   epilogue of v | bias: v goes through a [32 d][128 t] staging tile per head and a TMA store (the transpose),
+//   warps 8..15   epilogue of v | bias: v goes through a [32 d][t] staging tile per head and run and a TMA store (the transpose),
 //                 the two bias values of the row are written directly.
 //   warps 16..19  (bf16 rows 16..23) statistics, correction row, scale pair, mask bias.
 //   then          a TMA producer and the MMA issuers of the two products (N = 128 and N = 80), each into two accumulators in turn.
@@ -24,7 +24,7 @@ namespace px {
 
 constexpr int kAiH = 4, kAiD = 32;
 constexpr int kAiW1Panel = 80 * 128;           // [v 64 | bias 16][64 k]
-constexpr int kAiStageOut = 32 * 256;          // [32 d][128 t] fp16: one head
+constexpr int kAiStageOut = 32 * 256;          // per run [32 d][t] fp16: one head
 constexpr int ai_threads(bool f16) { return 32 * (16 + tile_stats_warps(f16) + 3); }
 // Stages of the row-tile ring: two, or three where shared memory holds them, which is where the rows are standardised ones (they need
 // one correction panel).  Which: triatt_in_stages.
@@ -75,20 +75,21 @@ struct AiWeights {
 };
 
 // kF16: the rows are the standardised fp16 copy of an fp32 pair tensor (fp16 weights); otherwise bf16 rows of z.
-template <bool kF16, int kStages>
+template <bool kF16, int kStages, int kRun>
 __global__ void __launch_bounds__(ai_threads(kF16), 1)
 triatt_in_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_constant__ CUtensorMap map_v,
                     const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k, const float* __restrict__ mask,
                     const AiWeights<kF16> weights, const unsigned char* __restrict__ folded,
                     float* __restrict__ bias_out, float* __restrict__ mb_out, int n_u, int n,
-                    int ldm, int swap, float eps, float inf, int tiles_t, int n_tiles) {
+                    int ldm, int swap, float eps, float inf, int runs_t, int n_tiles) {
   typedef AiLayout<kF16, kStages> Layout;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* sm = smem_aligned(smem_raw);
   AiBars<kStages>& bars = *reinterpret_cast<AiBars<kStages>*>(sm + Layout::bars);
   const int warp = warp_index(), lane = threadIdx.x & 31;
   const int hpair = blockIdx.x & 1;                      // this CTA's heads: 2*hpair, 2*hpair + 1
-  typedef TileCtx<kStages, kF16> Ctx;
+  typedef TileCtx<kStages, kF16, kRun> Ctx;
+  constexpr int kPer = 128 / kRun;                       // runs of a tile
   constexpr int kCtl = 16 + tile_stats_warps(kF16);      // first control warp
   Ctx ctx;
   ctx.tiles = sm + Layout::a;
@@ -97,7 +98,7 @@ triatt_in_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_cons
   ctx.first_tile = blockIdx.x >> 1;
   ctx.tile_step = gridDim.x >> 1;
   ctx.n_tiles = n_tiles;
-  ctx.tiles_t = tiles_t;
+  ctx.runs_t = runs_t;
   ctx.n_u = n_u;
   ctx.n_t = n;
   ctx.swap = swap;
@@ -149,11 +150,13 @@ triatt_in_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_cons
         [&](int k, int, int t, int r, float rstd, float) { scale[(k % Ctx::kSlots) * 128 + r] = make_float2(rstd, t < n ? rstd : 0.f); },
         TileNothingAhead(),
         [&](int u, int t) {
-          if (hpair == 0 && t < ldm) {                   // mask bias, -inf in the pad columns [n, ldm)
+          if (hpair == 0 && u < n_u) {                   // mask bias, -inf in the pad columns [n, ldm)
             float mv = -CUDART_INF_F;
             if (t < n)
               mv = mask ? (__ldg(mask + (swap ? ((size_t)t * n_u + u) : ((size_t)u * n + t))) - 1.0f) * inf * kLog2e : 0.f;
             mb_out[(size_t)u * ldm + t] = mv;
+            // an odd number of runs of 64 leaves 64 columns of the padding to the last one
+            if (kRun == 64 && t >= 64 * (runs_t - 1) && t + 64 < ldm) mb_out[(size_t)u * ldm + t + 64] = -CUDART_INF_F;
           }
         });
   } else if (warp < 8) {
@@ -164,7 +167,8 @@ triatt_in_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_cons
     unsigned char* stage = sm + Layout::qk + warp * 4096;
     int k = 0;
     for (int tile = ctx.first_tile; tile < n_tiles; tile += ctx.tile_step, ++k) {
-      const int u = tile / tiles_t, tw = (tile % tiles_t) * 128 + 32 * qw;   // the warp's first row
+      const Run run = run_at<kRun>(kPer * tile + 32 * qw / kRun, runs_t);
+      const int u = run.u, tw = run.t + 32 * qw % kRun;   // the warp's first row
       const int ab = k & 1, an = k >> 1;
       bool ok = mbar_wait(&bars.acc_full[0][ab], an & 1, 32u);
       ok = __all_sync(0xffffffffu, ok);
@@ -192,7 +196,7 @@ triatt_in_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_cons
       }
       asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
       __syncwarp();
-      if (lane == 0 && tw < n) {
+      if (lane == 0 && tw < n && u < n_u) {
         for (int e = 0; e < 2; ++e)
           tma_store_3d(which ? &map_k : &map_q, smem_u32(stage + e * 2048), 0, tw, u * kAiH + 2 * hpair + e);
         tma_store_commit();
@@ -208,10 +212,11 @@ triatt_in_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_cons
     int k = 0;
     bool ok = true;
     for (int tile = ctx.first_tile; tile < n_tiles && ok; tile += ctx.tile_step, ++k) {
-      const int u = tile / tiles_t, t0 = (tile % tiles_t) * 128, t = t0 + row;
+      const Run run = run_at<kRun>(kPer * tile + 32 * qw / kRun, runs_t);
+      const int u = run.u, t = run.t + row % kRun;
       const int ab = k & 1, an = k >> 1;
       unsigned char* const area = sm + Layout::out + half * kAiStageOut;
-      unsigned char* const stage = area + row * 2;
+      unsigned char* const stage = area + row / kRun * (kAiStageOut / kPer) + row % kRun * 2;
       ok = mbar_wait(&bars.acc_full[1][ab], an & 1, 64u);
       // the store that last read the staging area (one tile ago) must be through with it
       if (leader) tma_store_wait_read<0>();
@@ -228,16 +233,22 @@ triatt_in_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_cons
       if (lane == 0) mbar_arrive(&bars.acc_free[1][ab]);  // this warp has read its part of the accumulator
 #pragma unroll
       for (int e = 0; e < 32; ++e)
-        *reinterpret_cast<__half*>(stage + e * 256) = __float2half_rn(sc.y * __uint_as_float(v[e]));
-      if (half == 0 && t < ldm) {                        // zero in the pad columns [n, ldm)
+        *reinterpret_cast<__half*>(stage + e * (2 * kRun)) = __float2half_rn(sc.y * __uint_as_float(v[e]));
+      if (half == 0 && u < n_u) {                        // zero in the pad columns [n, ldm)
 #pragma unroll
-        for (int e = 0; e < 2; ++e)
-          bias_out[((size_t)(2 * hpair + e) * n_u + u) * ldm + t] = sc.y * __uint_as_float(b[e]);
+        for (int e = 0; e < 2; ++e) {
+          float* const to = bias_out + ((size_t)(2 * hpair + e) * n_u + u) * ldm + t;
+          *to = sc.y * __uint_as_float(b[e]);
+          if (kRun == 64 && t >= 64 * (runs_t - 1) && t + 64 < ldm) to[64] = 0.f;     // an odd number of runs
+        }
       }
       asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
       named_barrier(1 + half, 128);
       if (leader) {
-        tma_store_3d(&map_v, smem_u32(area), t0, u * 128 + 64 * hpair + 32 * half, 0);
+        for (int h = 0; h < kPer; ++h) {
+          const Run r = run_at<kRun>(kPer * tile + h, runs_t);
+          if (r.u < n_u) tma_store_3d(&map_v, smem_u32(area) + h * (kAiStageOut / kPer), r.t, r.u * 128 + 64 * hpair + 32 * half, 0);
+        }
         tma_store_commit();
       }
     }
@@ -254,21 +265,21 @@ triatt_in_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_cons
 
 PX_DEFINE_FAMILY_HOOKS(triatt_in)
 
-template <bool kF16, int kStages>
-static int32_t launch_triatt_in(const void* z, const float* mask, const AiWeights<kF16>& weights, const void* folded,
+template <bool kF16, int kStages, int kRun>
+static int32_t launch_triatt_in_runs(const void* z, const float* mask, const AiWeights<kF16>& weights, const void* folded,
                                 px_f16* q, px_f16* k, px_f16* v, float* bias, float* mask_bias, int64_t n_u,
                                 int64_t n, int64_t ldm, int32_t ending, float eps, float inf, cudaStream_t st) {
   CUtensorMap mz, mv, mq, mk;
   const CUtensorMapDataType zt = kF16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
   // pair element (u, t) is row u*n + t of z, or row t*n_u + u when the two indices are exchanged
   const bool ok = ending ? make_map_3d(&mz, zt, z, 128, (uint64_t)n_u, (uint64_t)n, 256, (uint64_t)n_u * 256, 64, 1,
-                                       CU_TENSOR_MAP_SWIZZLE_128B, 128)
-                         : make_map_3d(&mz, zt, z, 128, (uint64_t)n, (uint64_t)n_u, 256, (uint64_t)n * 256, 64, 128,
+                                       CU_TENSOR_MAP_SWIZZLE_128B, kRun)
+                         : make_map_3d(&mz, zt, z, 128, (uint64_t)n, (uint64_t)n_u, 256, (uint64_t)n * 256, 64, kRun,
                                        CU_TENSOR_MAP_SWIZZLE_128B, 1);
   if (!ok) return PX_ERR_LAUNCH;
-  // v is [n_u * 128 rows (u, head, d)][ldt]: a store writes [32 rows][128 t]
+  // v is [n_u * 128 rows (u, head, d)][ldt]: a store writes [32 rows][a run]
   const uint64_t ldt = (uint64_t)px_ld(n);
-  if (!make_map_3d(&mv, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, v, ldt, (uint64_t)n_u * 128, 1, ldt * 2, ldt * 2 * n_u * 128, 128,
+  if (!make_map_3d(&mv, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, v, ldt, (uint64_t)n_u * 128, 1, ldt * 2, ldt * 2 * n_u * 128, kRun,
                    32, CU_TENSOR_MAP_SWIZZLE_NONE, 1))
     return PX_ERR_LAUNCH;
   // q, k: [n_u * 4][n][32], a store writes [32 t][32]
@@ -278,17 +289,25 @@ static int32_t launch_triatt_in(const void* z, const float* mask, const AiWeight
       return PX_ERR_LAUNCH;
   const size_t smem = AiLayout<kF16, kStages>::total + 1024;
   static SmemLimit limit;
-  if (!limit.set(triatt_in_tc_kernel<kF16, kStages>, smem)) return PX_ERR_LAUNCH;
-  const int64_t tiles_t = (n + 127) / 128, n_tiles = tiles_t * n_u;   // 128-wide tiles cover the pad columns up to ldm
+  if (!limit.set(triatt_in_tc_kernel<kF16, kStages, kRun>, smem)) return PX_ERR_LAUNCH;
+  const int64_t n_tiles = tiles_of(n_u, n, kRun);
   if (n_tiles > 0x7fffffff) return PX_ERR_UNSUPPORTED;
   // Whole tiles of bf16 rows take little longer than ragged ones (their statistics are the same work), and an even number serves them 2 to 4 %
   // better from 132 to 230 tokens (N = 160 13.5 us against 14.0), 1 to 2 % worse at 430 and 450; standardised rows gain 3 to 8 % there.
-  const int pairs = even_grid(n_tiles, sm_count() / 2, kF16 && n % 128 ? tiles_t : 1);
-  return launch_pdl(triatt_in_tc_kernel<kF16, kStages>, dim3(2 * pairs), ai_threads(kF16), smem, st, mz, mv, mq, mk, mask, weights,
-                    (const unsigned char*)folded, bias, mask_bias, (int)n_u, (int)n, (int)ldm, (int)ending, eps, inf, (int)tiles_t,
+  const int pairs = even_grid(n_tiles, sm_count() / 2, kF16 ? tile_period(n_u, n, kRun) : 1);
+  return launch_pdl(triatt_in_tc_kernel<kF16, kStages, kRun>, dim3(2 * pairs), ai_threads(kF16), smem, st, mz, mv, mq, mk, mask, weights,
+                    (const unsigned char*)folded, bias, mask_bias, (int)n_u, (int)n, (int)ldm, (int)ending, eps, inf, (int)runs_of(n, kRun),
                     (int)n_tiles)
              ? PX_OK
              : PX_ERR_LAUNCH;
+}
+
+template <bool kF16, int kStages>
+static int32_t launch_triatt_in(const void* z, const float* mask, const AiWeights<kF16>& weights, const void* folded,
+                                px_f16* q, px_f16* k, px_f16* v, float* bias, float* mask_bias, int64_t n_u,
+                                int64_t n, int64_t ldm, int32_t ending, float eps, float inf, cudaStream_t st) {
+  return (two_runs_pay(n_u, n) ? launch_triatt_in_runs<kF16, kStages, 64> : launch_triatt_in_runs<kF16, kStages, 128>)(
+      z, mask, weights, folded, q, k, v, bias, mask_bias, n_u, n, ldm, ending, eps, inf, st);
 }
 
 // Stages for the standardised rows of an fp32 pair tensor.  Three let the two CTAs of a pair drift apart, and once the rows are larger than

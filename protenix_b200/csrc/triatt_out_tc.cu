@@ -71,7 +71,7 @@ template <int kMode>
 __global__ void __launch_bounds__(ao_threads(kMode != 0), 1)
 triatt_out_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_constant__ CUtensorMap map_o,
                      const __grid_constant__ CUtensorMap map_out, const void* __restrict__ z_in, void* __restrict__ z_out,
-                     const AoWeights<kMode != 0> weights, const unsigned char* __restrict__ folded, int n_u, int n, int swap, int add_residual, float eps, int tiles_t,
+                     const AoWeights<kMode != 0> weights, const unsigned char* __restrict__ folded, int n_u, int n, int swap, int add_residual, float eps, int runs_t,
                      int n_tiles) {
   constexpr bool kTma = kMode == 0 || kMode == 2;        // 16-bit output: packed over the o tile, leaves through TMA
   constexpr bool kBulk = kMode == 3;                     // fp32 output: staged, stored or added by TMA
@@ -80,7 +80,7 @@ triatt_out_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_con
   unsigned char* sm = smem_aligned(smem_raw);
   AoBars& bars = *reinterpret_cast<AoBars*>(sm + AoLayout::bars);
   const int warp = warp_index(), lane = threadIdx.x & 31;
-  typedef TileCtx<kAoStages, kF16> Ctx;
+  typedef TileCtx<kAoStages, kF16, 64> Ctx;
   constexpr int kCtl = 16 + tile_stats_warps(kF16);      // first control warp
   Ctx ctx;
   ctx.tiles = sm + AoLayout::a;
@@ -89,7 +89,7 @@ triatt_out_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_con
   ctx.first_tile = blockIdx.x;
   ctx.tile_step = gridDim.x;
   ctx.n_tiles = n_tiles;
-  ctx.tiles_t = tiles_t;
+  ctx.runs_t = runs_t;
   ctx.n_u = n_u;
   ctx.n_t = n;
   ctx.swap = swap;
@@ -136,21 +136,26 @@ triatt_out_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_con
         // ahead delay the additions (starting node, fp32 N = 200 15.2 -> 14.2 us, 437 48.0 -> 45.0, 768 141 -> 139; level at 1536).
         if (kBulk && add_residual && k && !mbar_wait_warp(&bars.g_full, (k - 1) & 1, 1u)) break;
         if (elect_lane()) {
-          const int u = tile / tiles_t, t0 = (tile % tiles_t) * 128;
           mbar_expect_tx(&bars.tile.raw_full[s], 2 * kOperandBytes);
           const uint32_t zdst = smem_u32(ctx.tiles + s * kTileBytes), odst = smem_u32(sm + AoLayout::o + s * kOperandBytes);
-          for (int p = 0; p < 2; ++p) {
-            tma_load_3d(zdst + p * kPanelBytes, &map_z, &bars.tile.raw_full[s], 64 * p, swap ? u : t0, swap ? t0 : u);
-            tma_load_3d(odst + p * kPanelBytes, &map_o, &bars.tile.raw_full[s], 64 * p, t0, u);
+          for (int h = 0; h < 2; ++h) {
+            const Run r = run_at<64>(2 * tile + h, runs_t);
+            for (int p = 0; p < 2; ++p) {
+              const int at = p * kPanelBytes + h * (64 * 128);
+              tma_load_3d(zdst + at, &map_z, &bars.tile.raw_full[s], 64 * p, swap ? r.u : r.t, swap ? r.t : r.u);
+              tma_load_3d(odst + at, &map_o, &bars.tile.raw_full[s], 64 * p, r.t, r.u);
+            }
           }
           // The tile that takes this stage next is asked of L2 (a stage is held until its rows have left, so only two tiles are on
           // their way): bf16 N = 768 103 -> 93 us.  Not where rows are added in L2, which is then what is waited for: 562 -> 594 at N = 1536.
           const int next = tile + 2 * ctx.tile_step;
           if ((kTma || (kBulk && !add_residual)) && next < n_tiles) {
-            const int u2 = next / tiles_t, t2 = (next % tiles_t) * 128;
-            for (int p = 0; p < 2; ++p) {
-              tma_prefetch_3d(&map_z, 64 * p, swap ? u2 : t2, swap ? t2 : u2);
-              tma_prefetch_3d(&map_o, 64 * p, t2, u2);
+            for (int h = 0; h < 2; ++h) {
+              const Run r = run_at<64>(2 * next + h, runs_t);
+              for (int p = 0; p < 2; ++p) {
+                tma_prefetch_3d(&map_z, 64 * p, swap ? r.u : r.t, swap ? r.t : r.u);
+                tma_prefetch_3d(&map_o, 64 * p, r.t, r.u);
+              }
             }
           }
         }
@@ -238,12 +243,13 @@ triatt_out_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_con
     bool ok = true;
     for (int tile = ctx.first_tile; tile < n_tiles && ok; tile += ctx.tile_step, ++k) {
       const int s = k % kAoStages;
-      const int u = tile / tiles_t, t0 = (tile % tiles_t) * 128;
-      // fp32 rows: this warp's 32 rows (u, t0 + 32 qw + i) in units of 128-channel rows of z, and their residual
+      const Run run = run_at<64>(2 * tile + (qw >> 1), runs_t);
+      const int u = run.u, tw = run.t + 32 * (qw & 1);
+      // fp32 rows: this warp's 32 rows (u, tw + i) in units of 128-channel rows of z, and their residual
       // values for the first 32 channels, requested before the wait (the second block's lines are asked of L2)
-      const long long first_row = swap ? (long long)(t0 + 32 * qw) * n_u + u : (long long)u * n + t0 + 32 * qw;
+      const long long first_row = swap ? (long long)tw * n_u + u : (long long)u * n + tw;
       const long long row_stride = swap ? n_u : 1;
-      const int valid = n - (t0 + 32 * qw) < 32 ? (n - (t0 + 32 * qw) > 0 ? n - (t0 + 32 * qw) : 0) : 32;
+      const int valid = u >= n_u || tw >= n ? 0 : n - tw < 32 ? n - tw : 32;
       RowsOutReq rq;
       if (!kTma && !kBulk) {
         rows_out_request(rq, reinterpret_cast<const float*>(z_in), first_row, row_stride, valid, 64 * half, lane,
@@ -254,8 +260,9 @@ triatt_out_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_con
         // and both blocks of the next tile, so that its requests hit L2
         const int nt = tile + ctx.tile_step;
         if (add_residual && nt < n_tiles) {
-          const int u2 = nt / tiles_t, t2 = (nt % tiles_t) * 128 + 32 * qw + lane;
-          if (t2 < n) {
+          const Run r2 = run_at<64>(2 * nt + (qw >> 1), runs_t);
+          const int u2 = r2.u, t2 = r2.t + 32 * (qw & 1) + lane;
+          if (t2 < n && u2 < n_u) {
             const float* p2 = reinterpret_cast<const float*>(z_in) + (size_t)(swap ? (long long)t2 * n_u + u2 : (long long)u2 * n + t2) * kC + 64 * half;
             asm volatile("prefetch.global.L2 [%0];\n" ::"l"(p2));
             asm volatile("prefetch.global.L2 [%0];\n" ::"l"(p2 + 32));
@@ -305,8 +312,7 @@ triatt_out_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_con
 #pragma unroll
           for (int e = 0; e < 32; ++e) v[e] = __uint_as_float(acc[e]);
           unsigned char* stg = hh == 0 ? otile + (warp & 7) * 4096 : ctx.tiles + s * kTileBytes + half * kPanelBytes + qw * 4096;
-          const int tw = t0 + 32 * qw;
-          rows_bulk_out(stg, v, &map_out, add_residual != 0, 64 * half + 32 * hh, swap ? u : tw, swap ? tw : u, tw < n, lane);
+          rows_bulk_out(stg, v, &map_out, add_residual != 0, 64 * half + 32 * hh, swap ? u : tw, swap ? tw : u, valid > 0, lane);
         } else {
           // fp32 rows: coalesced through a warp-private staging area inside the o tile, which the gate warps and
           // the tensor core have finished reading (8 warps x 4 KB)
@@ -324,8 +330,11 @@ triatt_out_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_con
         asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
         named_barrier(1, 256);
         if (leader) {
-          for (int p = 0; p < 2; ++p)
-            tma_store_3d(&map_out, smem_u32(otile + p * kPanelBytes), 64 * p, swap ? u : t0, swap ? t0 : u);
+          for (int h = 0; h < 2; ++h) {
+            const Run r = run_at<64>(2 * tile + h, runs_t);
+            for (int p = 0; p < 2 && r.u < n_u; ++p)
+              tma_store_3d(&map_out, smem_u32(otile + p * kPanelBytes) + h * (64 * 128), 64 * p, swap ? r.u : r.t, swap ? r.t : r.u);
+          }
           tma_store_commit();
           tma_store_wait_read<0>();                        // the store has read the stage: hand it back
           mbar_arrive(&bars.tile.a_empty[s]);
@@ -360,8 +369,8 @@ static int32_t launch_triatt_out(const px_f16* o, const void* z_in, const px_f16
   const CUtensorMapDataType zt = kMode == 0 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
   const void* zrows = kMode == 1 || kMode == 3 ? (const void*)zn : z_in;
   if (!(ending ? make_map_3d(&mz, zt, zrows, 128, (uint64_t)n_u, (uint64_t)n, 256, (uint64_t)n_u * 256, 64, 1,
-                             CU_TENSOR_MAP_SWIZZLE_128B, 128)
-               : make_map_3d(&mz, zt, zrows, 128, (uint64_t)n, (uint64_t)n_u, 256, (uint64_t)n * 256, 64, 128,
+                             CU_TENSOR_MAP_SWIZZLE_128B, 64)
+               : make_map_3d(&mz, zt, zrows, 128, (uint64_t)n, (uint64_t)n_u, 256, (uint64_t)n * 256, 64, 64,
                              CU_TENSOR_MAP_SWIZZLE_128B, 1)))
     return PX_ERR_LAUNCH;
   if (kMode == 3) {
@@ -372,24 +381,24 @@ static int32_t launch_triatt_out(const px_f16* o, const void* z_in, const px_f16
       return PX_ERR_LAUNCH;
   } else if (kMode != 1) {
     if (!(ending ? make_map_3d(&mout, zt, z_out, 128, (uint64_t)n_u, (uint64_t)n, 256, (uint64_t)n_u * 256, 64, 1,
-                               CU_TENSOR_MAP_SWIZZLE_128B, 128)
-                 : make_map_3d(&mout, zt, z_out, 128, (uint64_t)n, (uint64_t)n_u, 256, (uint64_t)n * 256, 64, 128,
+                               CU_TENSOR_MAP_SWIZZLE_128B, 64)
+                 : make_map_3d(&mout, zt, z_out, 128, (uint64_t)n, (uint64_t)n_u, 256, (uint64_t)n * 256, 64, 64,
                                CU_TENSOR_MAP_SWIZZLE_128B, 1)))
       return PX_ERR_LAUNCH;
   } else {
     memset(&mout, 0, sizeof(mout));
   }
   if (!make_map_3d(&mo, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, o, 128, (uint64_t)n, (uint64_t)n_u, 256, (uint64_t)n * 256, 64,
-                   128, CU_TENSOR_MAP_SWIZZLE_128B, 1))
+                   64, CU_TENSOR_MAP_SWIZZLE_128B, 1))
     return PX_ERR_LAUNCH;
   const size_t smem = AoLayout::total + 1024;
   static SmemLimit limit;
   if (!limit.set(triatt_out_tc_kernel<kMode>, smem)) return PX_ERR_LAUNCH;
-  const int64_t tiles_t = (n + 127) / 128, n_tiles = tiles_t * n_u;
+  const int64_t n_tiles = tiles_of(n_u, n, 64);
   if (n_tiles > 0x7fffffff) return PX_ERR_UNSUPPORTED;
-  const int grid = even_grid(n_tiles, sm_count(), n % 128 && n_u > 1 ? tiles_t : 1);
+  const int grid = even_grid(n_tiles, sm_count(), tile_period(n_u, n, 64));
   return launch_pdl(triatt_out_tc_kernel<kMode>, dim3(grid), ao_threads(kMode != 0), smem, st, mz, mo, mout, z_in, z_out, weights,
-                    (const unsigned char*)folded, (int)n_u, (int)n, (int)ending, (int)add_residual, eps, (int)tiles_t, (int)n_tiles)
+                    (const unsigned char*)folded, (int)n_u, (int)n, (int)ending, (int)add_residual, eps, (int)runs_of(n, 64), (int)n_tiles)
              ? PX_OK
              : PX_ERR_LAUNCH;
 }

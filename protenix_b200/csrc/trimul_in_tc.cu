@@ -3,14 +3,14 @@
 //   stored channel-major in fp16 with the contraction index t contiguous.  (a and b are products of a bounded gate
 //   and a projection of a standardised row: far inside the fp16 range, and fp16 keeps three more bits than bf16.)
 //
-// Persistent kernel, one CTA per SM.  A tile is 128 pair elements (one u, 128 consecutive t); the CTAs work in
+// Persistent kernel, one CTA per SM.  A tile is 128 pair elements (128 t, or two runs of 64); the CTAs work in
 // pairs on the same sequence of tiles, each CTA producing 64 of the 128 channels of a and of b (the second read of
 // a tile comes from L2).  Halving the weights a CTA keeps resident leaves shared memory for output staging
 // (px_rowpipe.cuh has the parts shared with the other row kernels):
 //   * The weights stay in shared memory for the whole kernel with gamma and the 1/2 of the sigmoid folded in;
 //     LayerNorm's mean and beta terms enter the product as one extra K step (see px_rowpipe.cuh).
 //   * The gated outputs are staged as [channel][t] in shared memory (two-byte stores, conflict-free) and leave
-//     through TMA stores, 256-byte runs per channel.  Four warps share a staging area of 32 channels.
+//     through TMA stores, 256 or 128 bytes per channel.  Four warps share a staging area of 32 channels.
 //
 //   warps 0..7    epilogue of output a: a thread owns one pair element (accumulator lane) and 32 of the CTA's 64
 //                 channels; warps 8..15 do the same for output b, concurrently.
@@ -25,7 +25,7 @@ namespace px {
 
 constexpr int kTiStages = 3;
 constexpr int kTiWExtra = 128 * 32;            // [128 rows][16 k] weight-side correction panel
-constexpr int kTiStageOut = 32 * 256;          // [32 channels][128 t] fp16
+constexpr int kTiStageOut = 32 * 256;          // per run [32 channels][t] fp16
 constexpr int ti_threads(bool f16) { return 32 * (16 + tile_stats_warps(f16) + 3); }
 // tensor memory: out a | out b, twice
 
@@ -65,18 +65,19 @@ struct TiWeights {
 };
 
 // kF16: the rows are the standardised fp16 copy of an fp32 pair tensor (fp16 weights); otherwise bf16 rows of z.
-template <bool kF16>
+template <bool kF16, int kRun>
 __global__ void __launch_bounds__(ti_threads(kF16), 1)
 trimul_in_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_constant__ CUtensorMap map_a,
                     const __grid_constant__ CUtensorMap map_b, const float* __restrict__ mask,
-                    const TiWeights<kF16> weights, const unsigned char* __restrict__ folded, int n_u, int n_t, int swap, float eps, int tiles_t, int n_tiles) {
+                    const TiWeights<kF16> weights, const unsigned char* __restrict__ folded, int n_u, int n_t, int swap, float eps, int runs_t, int n_tiles) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* sm = smem_aligned(smem_raw);
   TiBars& bars = *reinterpret_cast<TiBars*>(sm + TiLayout::bars);
   const int warp = warp_index(), lane = threadIdx.x & 31;
   constexpr int kCtl = 16 + tile_stats_warps(kF16);      // first control warp
   const int chan0 = 64 * (blockIdx.x & 1);               // this CTA's channels of a and b
-  typedef TileCtx<kTiStages, kF16> Ctx;
+  typedef TileCtx<kTiStages, kF16, kRun> Ctx;
+  constexpr int kPer = 128 / kRun;                       // runs of a tile
   Ctx ctx;
   ctx.tiles = sm + TiLayout::a;
   ctx.extras = sm + TiLayout::ax;
@@ -84,7 +85,7 @@ trimul_in_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_cons
   ctx.first_tile = blockIdx.x >> 1;
   ctx.tile_step = gridDim.x >> 1;
   ctx.n_tiles = n_tiles;
-  ctx.tiles_t = tiles_t;
+  ctx.runs_t = runs_t;
   ctx.n_u = n_u;
   ctx.n_t = n_t;
   ctx.swap = swap;
@@ -131,7 +132,7 @@ trimul_in_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_cons
         ctx, eps, warp - 16, lane,
         [&](int k, int, int, int r, float rstd, float mk) { scale[(k % Ctx::kSlots) * 128 + r] = make_float2(rstd, 0.5f * rstd * mk); },
         [&](int u, int t) {
-          return t >= n_t ? 0.f : mask ? __ldg(mask + (swap ? ((size_t)t * n_u + u) : ((size_t)u * n_t + t))) : 1.f;
+          return t >= n_t || u >= n_u ? 0.f : mask ? __ldg(mask + (swap ? ((size_t)t * n_u + u) : ((size_t)u * n_t + t))) : 1.f;
         });
   } else {
     // ------------------------------------------------------------------ epilogue of output ph
@@ -144,11 +145,10 @@ trimul_in_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_cons
     int k = 0;
     bool ok = true;
     for (int tile = ctx.first_tile; tile < n_tiles && ok; tile += ctx.tile_step, ++k) {
-      const int u = tile / tiles_t, t0 = (tile % tiles_t) * 128;
       const int ab = k & 1;
       const uint32_t t_buf = t_acc + 256 * ab;
       unsigned char* const area = sm + TiLayout::out + group * kTiStageOut;
-      unsigned char* const stage = area + row * 2;
+      unsigned char* const stage = area + row / kRun * (kTiStageOut / kPer) + row % kRun * 2;
       ok = mbar_wait(&bars.acc_full[ph][ab], (k >> 1) & 1, 32u);
       // the store that last read the staging area (one tile ago) must be through with it
       if (leader) tma_store_wait_read<0>();
@@ -162,7 +162,7 @@ trimul_in_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_cons
         for (int e = 0; e < 16; ++e) {
           const float h = sc.y * __uint_as_float(p[e]);
           const float v = fmaf(h, tanh_fast(sc.x * __uint_as_float(g[e])), h);
-          *reinterpret_cast<__half*>(stage + (16 * hh + e) * 256) = __float2half_rn(v);
+          *reinterpret_cast<__half*>(stage + (16 * hh + e) * (2 * kRun)) = __float2half_rn(v);
         }
       };
       uint32_t p0[16], g0[16], p1[16], g1[16];
@@ -179,7 +179,10 @@ trimul_in_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_cons
       asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
       named_barrier(1 + group, 128);
       if (leader) {
-        tma_store_3d(map_out, smem_u32(area), t0, u, chan0 + 32 * half);
+        for (int h = 0; h < kPer; ++h) {
+          const Run r = run_at<kRun>(kPer * tile + h, runs_t);
+          if (r.u < n_u) tma_store_3d(map_out, smem_u32(area) + h * (kTiStageOut / kPer), r.t, r.u, chan0 + 32 * half);
+        }
         tma_store_commit();
       }
     }
@@ -196,34 +199,41 @@ trimul_in_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_cons
 
 PX_DEFINE_FAMILY_HOOKS(trimul_in)
 
-template <bool kF16>
-static int32_t launch_trimul_in(const void* z, const float* mask, const TiWeights<kF16>& weights, const void* folded, px_f16* a,
+template <bool kF16, int kRun>
+static int32_t launch_trimul_in_runs(const void* z, const float* mask, const TiWeights<kF16>& weights, const void* folded, px_f16* a,
                                 px_f16* b, int64_t n_u, int64_t n_t, int64_t ld, int32_t incoming, float eps, cudaStream_t st) {
   CUtensorMap mz, ma, mb;
-  if (!incoming && ld == n_t && one_row_pays(n_u, n_t)) n_t *= n_u, ld = n_t, n_u = 1;
   const CUtensorMapDataType zt = kF16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
   // pair element (u, t) is row u*n_t + t of z, or row t*n_u + u when the two indices are exchanged
   const bool ok = incoming ? make_map_3d(&mz, zt, z, 128, (uint64_t)n_u, (uint64_t)n_t, 256, (uint64_t)n_u * 256, 64, 1,
-                                         CU_TENSOR_MAP_SWIZZLE_128B, 128)
-                           : make_map_3d(&mz, zt, z, 128, (uint64_t)n_t, (uint64_t)n_u, 256, (uint64_t)n_t * 256, 64, 128,
+                                         CU_TENSOR_MAP_SWIZZLE_128B, kRun)
+                           : make_map_3d(&mz, zt, z, 128, (uint64_t)n_t, (uint64_t)n_u, 256, (uint64_t)n_t * 256, 64, kRun,
                                          CU_TENSOR_MAP_SWIZZLE_128B, 1);
   if (!ok) return PX_ERR_LAUNCH;
-  // outputs [128 channels][n_u][ld]: a store writes [32 channels][one u][128 t]
+  // outputs [128 channels][n_u][ld]: a store writes [32 channels][one u][a run]
   if (!make_map_3d(&ma, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, a, (uint64_t)ld, (uint64_t)n_u, 128, (uint64_t)ld * 2,
-                   (uint64_t)n_u * ld * 2, 128, 1, CU_TENSOR_MAP_SWIZZLE_NONE, 32) ||
+                   (uint64_t)n_u * ld * 2, kRun, 1, CU_TENSOR_MAP_SWIZZLE_NONE, 32) ||
       !make_map_3d(&mb, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, b, (uint64_t)ld, (uint64_t)n_u, 128, (uint64_t)ld * 2,
-                   (uint64_t)n_u * ld * 2, 128, 1, CU_TENSOR_MAP_SWIZZLE_NONE, 32))
+                   (uint64_t)n_u * ld * 2, kRun, 1, CU_TENSOR_MAP_SWIZZLE_NONE, 32))
     return PX_ERR_LAUNCH;
   const size_t smem = TiLayout::total + 1024;
   static SmemLimit limit;
-  if (!limit.set(trimul_in_tc_kernel<kF16>, smem)) return PX_ERR_LAUNCH;
-  const int64_t tiles_t = (ld + 127) / 128, n_tiles = tiles_t * n_u;
+  if (!limit.set(trimul_in_tc_kernel<kF16, kRun>, smem)) return PX_ERR_LAUNCH;
+  const int64_t n_tiles = tiles_of(n_u, n_t, kRun);     // (runs cover the pad columns)
   if (n_tiles > 0x7fffffff) return PX_ERR_UNSUPPORTED;
-  const int pairs = even_grid(n_tiles, sm_count() / 2, ld % 128 && n_u > 1 ? tiles_t : 1);
-  return launch_pdl(trimul_in_tc_kernel<kF16>, dim3(2 * pairs), ti_threads(kF16), smem, st, mz, ma, mb, mask, weights,
-                    (const unsigned char*)folded, (int)n_u, (int)n_t, (int)incoming, eps, (int)tiles_t, (int)n_tiles)
+  const int pairs = even_grid(n_tiles, sm_count() / 2, tile_period(n_u, n_t, kRun));
+  return launch_pdl(trimul_in_tc_kernel<kF16, kRun>, dim3(2 * pairs), ti_threads(kF16), smem, st, mz, ma, mb, mask, weights,
+                    (const unsigned char*)folded, (int)n_u, (int)n_t, (int)incoming, eps, (int)runs_of(n_t, kRun), (int)n_tiles)
              ? PX_OK
              : PX_ERR_LAUNCH;
+}
+
+template <bool kF16>
+static int32_t launch_trimul_in(const void* z, const float* mask, const TiWeights<kF16>& weights, const void* folded, px_f16* a,
+                                px_f16* b, int64_t n_u, int64_t n_t, int64_t ld, int32_t incoming, float eps, cudaStream_t st) {
+  if (!incoming && ld == n_t && one_row_pays(n_u, n_t)) n_t *= n_u, ld = n_t, n_u = 1;
+  return (two_runs_pay(n_u, n_t) ? launch_trimul_in_runs<kF16, 64> : launch_trimul_in_runs<kF16, 128>)(z, mask, weights, folded, a, b, n_u, n_t,
+                                                                                                ld, incoming, eps, st);
 }
 
 static bool trimul_in_shapes_ok(const void* z, const px_f16* a, const px_f16* b, int64_t n_u, int64_t n_t, int64_t ld) {

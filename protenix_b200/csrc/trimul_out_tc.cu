@@ -3,12 +3,12 @@
 //   x [128 channels][n_i][ld] fp16, channel-major and scaled by PX_TRIMUL_X_SCALE as the contraction leaves it
 //   (LN_out runs with eps * scale^2, which gives exactly LN_out of the unscaled x).
 //
-// Persistent kernel, one CTA per SM, 128 pair elements (one i, 128 consecutive j) per tile.  Both LayerNorms are
+// Persistent kernel, one CTA per SM, 128 pair elements (two runs of 64 consecutive j of one i) per tile.  Both LayerNorms are
 // folded into the resident weights plus one shared correction K step (px_rowpipe.cuh); nothing is normalised or
 // transposed on the way in:
 //   * the z tile arrives by TMA as a K-major operand (rows of 128 channels): the bf16 rows of z themselves, or, for an
 //     fp32 z, its standardised fp16 copy `zn` (px_standardise_rows), whose statistics are known;
-//   * the x tile arrives by TMA exactly as it lies in memory, [128 channels][128 j], and is used as an MN-major
+//   * the x tile arrives by TMA exactly as it lies in memory, [128 channels][64 j] a run, and is used as an MN-major
 //     operand: the tensor core reads it transposed;
 //   * the statistics of both are summed by threads from the tiles in shared memory (Gram products with the sums of squares on their
 //     diagonals and rows of ones behind the weights took 600 to 1200 cycles more of the tensor pipe a tile, and the statistics of a
@@ -80,7 +80,7 @@ __global__ void __launch_bounds__(to_threads(sizeof(Tz) != 2), 1)
 trimul_out_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_constant__ CUtensorMap map_x,
                      const __grid_constant__ CUtensorMap map_out, const Tz* __restrict__ z_in, Tz* __restrict__ z_out,
                      const ToWeights<sizeof(Tz) != 2> weights, const unsigned char* __restrict__ folded,
-                     int n_i, int n, int add_residual, float eps, int tiles_j, int n_tiles) {
+                     int n_i, int n, int add_residual, float eps, int runs_j, int n_tiles) {
   constexpr bool kTma = sizeof(Tz) == 2;               // bf16: residual from the z tile, output through TMA
   constexpr bool kF16 = !kTma;                           // operand format of the z side; the x side is always fp16
   constexpr int kStats = to_stats_warps(kF16), kThreads = to_threads(kF16), kLoad = 16 + kStats;   // kLoad: the producer's warp
@@ -139,22 +139,23 @@ trimul_out_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_con
         // further ahead delay the additions (asked for with the stage: 553 -> 568 us at N = 1536, 247 -> 256 at 1024; below 500 level).
         if (kBulk && add_residual && k && !mbar_wait_warp(&bars.a_ready[(k - 1) % kToStages], ((k - 1) / kToStages) & 1, 1u)) break;
         if (elect_lane()) {
-          const int i = tile / tiles_j, j0 = (tile % tiles_j) * 128;
           mbar_expect_tx(&bars.raw_full[s], 2 * kOperandBytes);
           const uint32_t zdst = smem_u32(sm + ToLayout::zt + s * kOperandBytes), xdst = smem_u32(sm + ToLayout::xt + s * kOperandBytes);
-          for (int p = 0; p < 2; ++p) {
-            tma_load_3d(zdst + p * kPanelBytes, &map_z, &bars.raw_full[s], 64 * p, j0, i);
-            tma_load_3d(xdst + p * kPanelBytes, &map_x, &bars.raw_full[s], j0 + 64 * p, i, 0);
+          for (int h = 0; h < 2; ++h) {
+            const Run r = run_at<64>(2 * tile + h, runs_j);
+            for (int p = 0; p < 2; ++p)
+              tma_load_3d(zdst + p * kPanelBytes + h * (64 * 128), &map_z, &bars.raw_full[s], 64 * p, r.t, r.u);
+            tma_load_3d(xdst + h * kPanelBytes, &map_x, &bars.raw_full[s], r.t, r.u, 0);
           }
           // The tile that takes this stage next is asked of L2 (a stage is held until its rows have left, so only two tiles are on
           // their way): bf16 N = 768 122 -> 107 us, fp32 without a residual N = 1024 230 -> 203.  Not where rows are added in L2,
           // which is then what is waited for: 552 -> 610 at N = 1536, 140 -> 151 at N = 768.
           const int next = tile + 2 * tile_step;
           if ((kTma || (kBulk && !add_residual)) && next < n_tiles) {
-            const int i2 = next / tiles_j, j2 = (next % tiles_j) * 128;
-            for (int p = 0; p < 2; ++p) {
-              tma_prefetch_3d(&map_z, 64 * p, j2, i2);
-              tma_prefetch_3d(&map_x, j2 + 64 * p, i2, 0);
+            for (int h = 0; h < 2; ++h) {
+              const Run r = run_at<64>(2 * next + h, runs_j);
+              for (int p = 0; p < 2; ++p) tma_prefetch_3d(&map_z, 64 * p, r.t, r.u);
+              tma_prefetch_3d(&map_x, r.t, r.u, 0);
             }
           }
         }
@@ -258,17 +259,18 @@ trimul_out_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_con
     bool ok = true;
     for (int tile = first_tile; tile < n_tiles && ok; tile += tile_step, ++k) {
       const int s = k % kToStages;
-      const int i = tile / tiles_j, j0 = (tile % tiles_j) * 128;
+      const Run run = run_at<64>(2 * tile + (qw >> 1), runs_j);
+      const int i = run.u, jw = run.t + 32 * (qw & 1);     // the warp's first element
+      const int valid = i >= n_i || jw >= n ? 0 : n - jw < 32 ? n - jw : 32;
       RowsOutReq rq;
       if (!kTma && !kBulk) {                               // the residual values are requested before the wait
-        const int valid = n - (j0 + 32 * qw) < 32 ? (n - (j0 + 32 * qw) > 0 ? n - (j0 + 32 * qw) : 0) : 32;
-        rows_out_request(rq, reinterpret_cast<const float*>(z_in), (long long)i * n + j0 + 32 * qw, 1, valid, 32 * part, lane,
-                         add_residual != 0);
+        rows_out_request(rq, reinterpret_cast<const float*>(z_in), (long long)i * n + jw, 1, valid, 32 * part, lane, add_residual != 0);
         // the residual lines of the next tile are asked of L2 now: a tile later they are a hit, not a trip to HBM
         const int nt = tile + tile_step;
         if (add_residual && nt < n_tiles) {
-          const int i2 = nt / tiles_j, j2 = (nt % tiles_j) * 128 + 32 * qw + lane;
-          if (j2 < n)
+          const Run r2 = run_at<64>(2 * nt + (qw >> 1), runs_j);
+          const int i2 = r2.u, j2 = r2.t + 32 * (qw & 1) + lane;
+          if (j2 < n && i2 < n_i)
             asm volatile("prefetch.global.L2 [%0];\n" ::"l"(reinterpret_cast<const float*>(z_in) + ((size_t)i2 * n + j2) * kC + 32 * part));
         }
       }
@@ -315,7 +317,11 @@ trimul_out_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_con
         asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
         named_barrier(1, 512);
         if (leader) {
-          for (int pnl = 0; pnl < 2; ++pnl) tma_store_3d(&map_out, smem_u32(ztile + pnl * kPanelBytes), 64 * pnl, j0, i);
+          for (int h = 0; h < 2; ++h) {
+            const Run r = run_at<64>(2 * tile + h, runs_j);
+            for (int pnl = 0; pnl < 2 && r.u < n_i; ++pnl)
+              tma_store_3d(&map_out, smem_u32(ztile + pnl * kPanelBytes) + h * (64 * 128), 64 * pnl, r.t, r.u);
+          }
           tma_store_commit();
           tma_store_wait_read<0>();                          // the store has read the stage: hand it back
           mbar_arrive(&bars.a_empty[s]);
@@ -323,7 +329,7 @@ trimul_out_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_con
       } else if (kBulk) {
         // fp32 rows: staged inside the stage's tiles, which the tensor core has finished reading (16 warps x 4 KB)
         unsigned char* stg = sm + (warp < 8 ? ToLayout::zt : ToLayout::xt) + s * kOperandBytes + (warp & 7) * 4096;
-        rows_bulk_out(stg, v, &map_out, add_residual != 0, 32 * part, j0 + 32 * qw, i, j0 + 32 * qw < n, lane);
+        rows_bulk_out(stg, v, &map_out, add_residual != 0, 32 * part, jw, i, valid > 0, lane);
         if (lane == 0) tma_store_wait_read<0>();
         named_barrier(1, 512);
         if (leader) mbar_arrive(&bars.a_empty[s]);
@@ -331,8 +337,7 @@ trimul_out_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_con
         // fp32 rows: coalesced through a warp-private staging area inside the stage's tiles, which the tensor core
         // has finished reading (16 warps x 4 KB = the z tile and the x tile)
         unsigned char* stg = sm + (warp < 8 ? ToLayout::zt : ToLayout::xt) + s * kOperandBytes + (warp & 7) * 4096;
-        const int valid = n - (j0 + 32 * qw) < 32 ? (n - (j0 + 32 * qw) > 0 ? n - (j0 + 32 * qw) : 0) : 32;
-        rows_out_store(stg, v, rq, reinterpret_cast<float*>(z_out), (long long)i * n + j0 + 32 * qw, 1, valid, 32 * part, lane);
+        rows_out_store(stg, v, rq, reinterpret_cast<float*>(z_out), (long long)i * n + jw, 1, valid, 32 * part, lane);
         named_barrier(1, 512);
         if (leader) mbar_arrive(&bars.a_empty[s]);
       }
@@ -359,12 +364,12 @@ static int32_t launch_trimul_out(const px_f16* x, const void* z_in, const px_f16
   if (ld == n && one_row_pays(n_i, n)) n *= n_i, ld = n, n_i = 1;
   // operand rows: bf16 z itself, or the standardised fp16 copy of an fp32 z
   if (!make_map_3d(&mz, sizeof(Tz) == 2 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16,
-                   sizeof(Tz) == 2 ? z_in : (const void*)zn, 128, (uint64_t)n, (uint64_t)n_i, 256, (uint64_t)n * 256, 64, 128,
+                   sizeof(Tz) == 2 ? z_in : (const void*)zn, 128, (uint64_t)n, (uint64_t)n_i, 256, (uint64_t)n * 256, 64, 64,
                    CU_TENSOR_MAP_SWIZZLE_128B, 1))
     return PX_ERR_LAUNCH;
   if (sizeof(Tz) == 2) {
     if (!make_map_3d(&mout, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, z_out, 128, (uint64_t)n, (uint64_t)n_i, 256, (uint64_t)n * 256,
-                     64, 128, CU_TENSOR_MAP_SWIZZLE_128B, 1))
+                     64, 64, CU_TENSOR_MAP_SWIZZLE_128B, 1))
       return PX_ERR_LAUNCH;
   } else if (kBulk) {
     if (!make_map_3d(&mout, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, z_out, 128, (uint64_t)n, (uint64_t)n_i, 512, (uint64_t)n * 512, 32, 32,
@@ -380,11 +385,11 @@ static int32_t launch_trimul_out(const px_f16* x, const void* z_in, const px_f16
   const size_t smem = ToLayout::total + 1024;
   static SmemLimit limit;
   if (!limit.set(trimul_out_tc_kernel<Tz, kBulk>, smem)) return PX_ERR_LAUNCH;
-  const int64_t tiles_j = (n + 127) / 128, n_tiles = tiles_j * n_i;
+  const int64_t n_tiles = tiles_of(n_i, n, 64);
   if (n_tiles > 0x7fffffff) return PX_ERR_UNSUPPORTED;
-  const int grid = even_grid(n_tiles, sm_count(), n % 128 && n_i > 1 ? tiles_j : 1);
+  const int grid = even_grid(n_tiles, sm_count(), tile_period(n_i, n, 64));
   return launch_pdl(trimul_out_tc_kernel<Tz, kBulk>, dim3(grid), to_threads(sizeof(Tz) != 2), smem, st, mz, mx, mout, (const Tz*)z_in, (Tz*)z_out, weights,
-                    (const unsigned char*)folded, (int)n_i, (int)n, (int)add_residual, eps, (int)tiles_j, (int)n_tiles)
+                    (const unsigned char*)folded, (int)n_i, (int)n, (int)add_residual, eps, (int)runs_of(n, 64), (int)n_tiles)
              ? PX_OK
              : PX_ERR_LAUNCH;
 }

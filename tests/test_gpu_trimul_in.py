@@ -60,3 +60,13 @@ def test_tiles_across_rows_equal_a_slab_of_one(n):
         pa, pb = ops.trimul_in_proj(z[u:u + 1].contiguous(), mask[u:u + 1].contiguous(), *w, False)
         assert torch.equal(pa[:, 0], a[:, u]) and torch.equal(pb[:, 0], b[:, u])
     ops.device_error_flags()
+
+
+@pytest.mark.parametrize("n_u", [1, 2, 3, 75])
+def test_ends_of_two_rows_share_a_tile(n_u):
+    """130 t: two whole runs of 64 and a ragged one; the ends of neighbouring rows meet in one tile, the last row's may stand alone."""
+    z, mask, w = inputs(76, 130, torch.bfloat16, False)
+    a, b = ops.trimul_in_proj(z, mask, *w, False)
+    pa, pb = ops.trimul_in_proj(z[:n_u].contiguous(), mask[:n_u].contiguous(), *w, False)
+    assert torch.equal(pa, a[:, :n_u]) and torch.equal(pb, b[:, :n_u])
+    ops.device_error_flags()
