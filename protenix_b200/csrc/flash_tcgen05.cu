@@ -474,6 +474,12 @@ triatt_flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
   }
 }
 
+}  // namespace px
+
+#include "px_flash_units.cuh"
+
+namespace px {
+
 PX_DEFINE_FAMILY_HOOKS(flash)
 
 }  // namespace px
@@ -520,6 +526,20 @@ extern "C" int32_t px_triatt_flash(const px_f16* q, const px_f16* k, const px_f1
   // A last key tile of 32 keys at most is worked off by its half, in kernels of their own (the branch costs the others 1 %): N = 150
   // 20.6 -> 19.2 us, 200 29.8 -> 28.1, 224 36.1 -> 34.1, 528 298 -> 291, 1056 1824 -> 1812, 1300 level.
   const bool brief = (n - 1) % kFKT < kFKT / 2;
+  // Up to forty units an SM (N = 1024) CTAs work on several; beyond, the beginnings and ends of CTAs are too few to pay for slower items.
+  const int64_t units = per * slices;
+  if (units > room && units <= 40 * room) {
+    const int64_t halved = 2 * left <= room ? left : 0;
+    const auto kernel = halved ? (brief ? triatt_flash_units_tc_kernel<true, true> : triatt_flash_units_tc_kernel<true, false>)
+                               : (brief ? triatt_flash_units_tc_kernel<false, true> : triatt_flash_units_tc_kernel<false, false>);
+    constexpr size_t bytes = FlashUnitLayout::total + 1024;
+    static SmemLimit limit[4];
+    if (!limit[2 * (halved > 0) + brief].set(kernel, bytes)) return PX_ERR_LAUNCH;
+    return launch_pdl(kernel, dim3((unsigned)room), kFThreads, bytes, st, mq, mk, mv, mbias, mo, mask_bias, (int)n_u, (int)n, (int)ldm, nkt,
+                      (int)(units - halved), (int)halved)
+               ? PX_OK
+               : PX_ERR_LAUNCH;
+  }
   const auto kernel = halves ? (brief ? triatt_flash_tc_kernel<true, true> : triatt_flash_tc_kernel<true, false>)
                              : (brief ? triatt_flash_tc_kernel<false, true> : triatt_flash_tc_kernel<false, false>);
   static SmemLimit limit[4];

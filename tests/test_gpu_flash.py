@@ -70,3 +70,21 @@ def test_rows_do_not_depend_on_how_they_are_dealt_out(n_u):
         part = ops.triatt_flash(q[rows].contiguous(), k[rows].contiguous(), v[rows].contiguous(), bias, mb[rows].contiguous())
         assert torch.equal(part, whole[rows])
     ops.device_error_flags()
+
+
+def test_many_units_a_cta_equal_one(n=130):
+    """Beyond forty units an SM a CTA has one unit, below it several; the rows are the same to the bit."""
+    n_u = 6 * (41 * torch.cuda.get_device_properties(0).multi_processor_count // 8)
+    g = torch.Generator("cuda").manual_seed(n)
+    draw = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    q, k = (0.3 * draw(n_u, 4, n, 32)).half(), draw(n_u, 4, n, 32).half()
+    v = torch.zeros(n_u, 4, 32, ops.ld(n), dtype=torch.half, device="cuda")
+    v[..., :n] = draw(n_u, 4, 32, n).half()
+    ldm = (n + 127) // 128 * 128
+    bias, mb = torch.zeros(4, n, ldm, device="cuda"), torch.full((n_u, ldm), -float("inf"), device="cuda")
+    bias[..., :n] = 2 * draw(4, n, n)
+    mb[:, :n] = 0
+    whole = ops.triatt_flash(q, k, v, bias, mb)
+    for rows in (slice(0, 700), slice(n_u - 401, n_u)):
+        assert torch.equal(ops.triatt_flash(q[rows], k[rows], v[rows], bias, mb[rows]), whole[rows])
+    ops.device_error_flags()
