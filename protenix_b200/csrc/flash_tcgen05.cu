@@ -321,9 +321,11 @@ triatt_flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         tc_fence_after();
         float s[kKeys];
 #pragma unroll
-        for (int c = 0; c < kKeys; c += 32) tmem_ld32(t_s + c, *reinterpret_cast<uint32_t(*)[32]>(&s[c]));
-        tmem_wait_ld();
-        if (kKeys == kFKT) clear_rest();             // (a tile of 32 keys is the last)
+        for (int c = kKeys - 32; c >= 0; c -= 32) {  // the zeros are stored while the first half is on its way
+          tmem_ld32(t_s + c, *reinterpret_cast<uint32_t(*)[32]>(&s[c]));
+          tmem_wait_ld();
+          if (kKeys == kFKT && c) clear_rest();      // (a tile of 32 keys is the last)
+        }
 #pragma unroll
         for (int c = kFCopied / 4; c < kKeys / 4; ++c) {
           add2(s[4 * c + 0], s[4 * c + 1], b4[c - kFCopied / 4].x, b4[c - kFCopied / 4].y);
