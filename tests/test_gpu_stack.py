@@ -25,3 +25,11 @@ def test_stack_equals_its_blocks(n, blocks, dtype):
             got = stack(s, z, mask)
             assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
     ops.device_error_flags()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("n, blocks", [(40, 9), (64, 20), (130, 13), (384, 17), (385, 4), (641, 5)])
+def test_pair_bias_buffers_are_written_anew_in_time(n, blocks, dtype):
+    """Up to 384 tokens eight pair-bias buffers take turns and the main stream waits for the side stream once in four blocks, from the ninth
+    block on; beyond there are two, and it waits from the third on.  A buffer written too early changes the update that still reads it."""
+    test_stack_equals_its_blocks(n, blocks, dtype)
