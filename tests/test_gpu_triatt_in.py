@@ -61,3 +61,27 @@ def test_rows_beyond_l2_equal_a_slab(ending):
         for name, a, b in zip("qkvbm", whole, slab):
             assert torch.equal(a[:, u0:u0 + 3] if name == "b" else a[u0:u0 + 3], b), name
     ops.device_error_flags()
+
+
+@pytest.mark.parametrize("ending", [False, True])
+def test_two_runs_a_tile_beyond_l2(ending, n_t=520):
+    """As above where tiles are made of two runs of 64, and the same rows against fp64."""
+    l2 = torch.cuda.get_device_properties(0).L2_cache_size
+    n_u = -(-(3 * l2 // 2) // (n_t * 256)) + 5
+    z, mask, w = inputs(n_u, n_t, torch.float32, ending)
+    q, k, v, bias, mb = whole = ops.triatt_in_proj(z, mask, *w, ending=ending)
+    for u0 in (0, n_u // 2, n_u - 3):
+        part = (slice(None), slice(u0, u0 + 3)) if ending else (slice(u0, u0 + 3),)
+        slab = ops.triatt_in_proj(z[part].contiguous(), mask[part].contiguous(), *w, ending=ending)
+        for name, a, b in zip("qkvbm", whole, slab):
+            assert torch.equal(a[:, u0:u0 + 3] if name == "b" else a[u0:u0 + 3], b), name
+        rows = z[part].double().transpose(0, 1) if ending else z[part].double()
+        d = [t.double() for t in w]
+        y = F.layer_norm(rows, (128,), d[0], d[1], 1e-5)
+        heads = lambda t: (y @ t.T).view(3, n_t, 4, 32).permute(0, 2, 1, 3)
+        want = (heads(d[3]) * LOG2E / math.sqrt(32), heads(d[4]), heads(d[5]).transpose(2, 3), (y @ d[2].T).permute(2, 0, 1) * LOG2E)
+        got = (q[u0:u0 + 3], k[u0:u0 + 3], v[u0:u0 + 3, ..., :n_t], bias[:, u0:u0 + 3, :n_t])
+        for name, a, b in zip("qkvb", got, want):      # the tolerance of test_triatt_in
+            assert float((a.double() - b).norm() / b.norm()) < 1e-3, name
+    assert bool((mb[:, n_t:] == -math.inf).all()) and not bool(bias[..., n_t:].any()) and not bool(v[..., n_t:].any())
+    ops.device_error_flags()

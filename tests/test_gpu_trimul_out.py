@@ -39,3 +39,12 @@ def test_trimul_out(n_i, n_j, dtype):
     for shift in (0.2, 30.0):
         rel = errors(n_i, n_j, dtype, shift)
         assert rel < tol, (rel, shift)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("n_i,n_j", [(1, 8), (2, 72), (3, 40), (75, 120), (149, 136)])
+def test_trimul_out_across_rows(n_i, n_j, dtype):
+    """Without pad columns the tiles run on from row to row (the tolerances are those of test_trimul_out)."""
+    for shift in (0.2, 30.0):
+        rel = errors(n_i, n_j, dtype, shift)
+        assert rel < (1e-3 if dtype == torch.float32 else 3e-3), (rel, shift)
