@@ -207,8 +207,8 @@ constexpr int tile_fulls(int stages) { return stages % 2 ? 2 * stages : stages; 
 
 template <int kStages>
 struct TileBars {
-  // raw_full: tile in shared memory; a_ready: statistics, correction rows and scales written;
-  // a_empty: every MMA that reads the stage is complete (one commit per issuing thread)
+  // raw_full: tile in shared memory (which of them is tile k's, for every load and every wait: TileCtx::full); a_ready: statistics,
+  // correction rows and scales written; a_empty: every MMA that reads the stage is complete (one commit per issuing thread)
   uint64_t raw_full[tile_fulls(kStages)], a_ready[tile_slots(kStages)], a_empty[kStages];
 };
 // kStandardised: the rows are a standardised fp16 copy (otherwise bf16 rows of z).
@@ -221,6 +221,8 @@ struct TileCtx {
   unsigned char* extras;    // tile_extras() x kTileExtra (the correction step of a tile runs after its stage is freed)
   TileBars<kStages_>* bars;
   int first_tile, tile_step, n_tiles, runs_t, n_u, n_t, swap;   // runs_t: runs that cover the t of one u
+  __device__ __forceinline__ uint64_t* full(int k) const { return &bars->raw_full[k % kFulls]; }
+  __device__ __forceinline__ uint32_t full_parity(int k) const { return (k / kFulls) & 1; }
   __device__ __forceinline__ unsigned char* extra(int k) const { return extras + (kStandardised ? 0 : (k % kSlots) * kTileExtra); }
 };
 
@@ -276,7 +278,7 @@ __device__ __forceinline__ void tile_producer_loop(const Ctx& c, const CUtensorM
     const int s = k % Ctx::kStages, n = k / Ctx::kStages;
     if (!mbar_wait_warp(&c.bars->a_empty[s], (n & 1) ^ 1, 1u)) break;
     if (elect_lane()) {
-      uint64_t* const full = &c.bars->raw_full[k % Ctx::kFulls];
+      uint64_t* const full = c.full(k);
       mbar_expect_tx(full, kOperandBytes);
       const uint32_t dst = smem_u32(c.tiles + s * kTileBytes);
       constexpr int kPer = 128 / Ctx::kRun;
@@ -363,7 +365,7 @@ __device__ __forceinline__ void tile_stats_loop(const Ctx& c, float eps, int sw,
     for (int j = 0; j < kRows; ++j) fetched[j] = next[j];
     fetch(tile + kSets * c.tile_step);
     // for standardised rows the arrival of the tile only paces this loop, so that the slots it writes are those of tiles in flight
-    if (!mbar_wait_warp(&c.bars->raw_full[k % Ctx::kFulls], (k / Ctx::kFulls) & 1, 16u)) break;
+    if (!mbar_wait_warp(c.full(k), c.full_parity(k), 16u)) break;
     if constexpr (!kStandardised) {
 #pragma unroll
       for (int j = 0; j < kRows; ++j) bf16_row_stats(c.tiles + s * kTileBytes, r0 + 64 * j, half, mean[j], var[j]);
@@ -413,7 +415,7 @@ __device__ __forceinline__ void tile_product_loop(const Ctx& c, uint32_t d_tmem,
     const int s = k % Ctx::kStages;
     const int ab = n_acc == 2 ? (k & 1) : 0, an = n_acc == 2 ? (k >> 1) : k;
     const uint32_t d = d_tmem + ab * acc_cols;
-    if (!mbar_wait_warp(&c.bars->raw_full[k % Ctx::kFulls], (k / Ctx::kFulls) & 1, 4u) || !mbar_wait_warp(&acc_free[ab], (an & 1) ^ 1, 8u)) break;
+    if (!mbar_wait_warp(c.full(k), c.full_parity(k), 4u) || !mbar_wait_warp(&acc_free[ab], (an & 1) ^ 1, 8u)) break;
     tc_fence_after();
     if (elect_lane()) {
       const uint32_t a_addr = smem_u32(c.tiles + s * kTileBytes);

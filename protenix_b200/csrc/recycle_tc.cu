@@ -106,9 +106,9 @@ recycle_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_consta
         const int s = k % kRcStages, n = k / kRcStages;
         if (!mbar_wait_warp(&bars.tile.a_empty[s], (n & 1) ^ 1, 1u)) break;
         if (elect_lane()) {
-          mbar_expect_tx(&bars.tile.raw_full[s], kOperandBytes);
+          mbar_expect_tx(ctx.full(k), kOperandBytes);
           const uint32_t dst = smem_u32(ctx.tiles + s * kTileBytes);
-          for (int p = 0; p < 2; ++p) tma_load_3d(dst + p * kPanelBytes, &map_z, &bars.tile.raw_full[s], 64 * p, tile * 128, 0);
+          for (int p = 0; p < 2; ++p) tma_load_3d(dst + p * kPanelBytes, &map_z, ctx.full(k), 64 * p, tile * 128, 0);
         }
         __syncwarp();
         if (kTma) {

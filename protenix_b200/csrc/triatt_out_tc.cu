@@ -136,14 +136,14 @@ triatt_out_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_con
         // ahead delay the additions (starting node, fp32 N = 200 15.2 -> 14.2 us, 437 48.0 -> 45.0, 768 141 -> 139; level at 1536).
         if (kBulk && add_residual && k && !mbar_wait_warp(&bars.g_full, (k - 1) & 1, 1u)) break;
         if (elect_lane()) {
-          mbar_expect_tx(&bars.tile.raw_full[s], 2 * kOperandBytes);
+          mbar_expect_tx(ctx.full(k), 2 * kOperandBytes);
           const uint32_t zdst = smem_u32(ctx.tiles + s * kTileBytes), odst = smem_u32(sm + AoLayout::o + s * kOperandBytes);
           for (int h = 0; h < 2; ++h) {
             const Run r = run_at<64>(2 * tile + h, runs_t);
             for (int p = 0; p < 2; ++p) {
               const int at = p * kPanelBytes + h * (64 * 128);
-              tma_load_3d(zdst + at, &map_z, &bars.tile.raw_full[s], 64 * p, swap ? r.u : r.t, swap ? r.t : r.u);
-              tma_load_3d(odst + at, &map_o, &bars.tile.raw_full[s], 64 * p, r.t, r.u);
+              tma_load_3d(zdst + at, &map_z, ctx.full(k), 64 * p, swap ? r.u : r.t, swap ? r.t : r.u);
+              tma_load_3d(odst + at, &map_o, ctx.full(k), 64 * p, r.t, r.u);
             }
           }
           // The tile that takes this stage next is asked of L2 (a stage is held until its rows have left, so only two tiles are on
