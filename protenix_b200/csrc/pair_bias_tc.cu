@@ -79,7 +79,7 @@ pair_bias_tc_kernel(const __grid_constant__ CUtensorMap map_z, const PbWeights<k
   const bool skip = cta_begin();         // an earlier bounded wait gave up: do not start new work
   if (threadIdx.x == 32) prefetch_maps(map_z);
   if (threadIdx.x == 0) {
-    tile_bars_init(bars.tile, 1);
+    tile_bars_init(ctx, 1);
     mbar_init(&bars.w_full, 1);
     mbar_init(&bars.acc_full, 1);
     mbar_init(&bars.acc_free, 4);

@@ -202,41 +202,41 @@ constexpr int tile_slots(int stages) { return stages + 2; }
 constexpr int tile_extras(int stages, bool standardised) { return standardised ? 1 : tile_slots(stages); }
 
 // Barriers that say a tile has arrived: of every one, each set of statistics warps sees all phases or none (a wait on a parity tells a
-// phase from the one before only; tile k + 1 may arrive before tile k), so there is an even number of them.
-constexpr int tile_fulls(int stages) { return stages % 2 ? 2 * stages : stages; }
+// phase from the one before only; tile k + 1 may arrive before tile k), so two sets need an even number of them.
+constexpr int tile_fulls(int stages, int sets) { return sets == 2 && stages % 2 ? 2 * stages : stages; }
 
-template <int kStages>
+template <int kStages, int kFulls = kStages>
 struct TileBars {
   // raw_full: tile in shared memory (which of them is tile k's, for every load and every wait: TileCtx::full); a_ready: statistics,
   // correction rows and scales written; a_empty: every MMA that reads the stage is complete (one commit per issuing thread)
-  uint64_t raw_full[tile_fulls(kStages)], a_ready[tile_slots(kStages)], a_empty[kStages];
+  uint64_t raw_full[kFulls], a_ready[tile_slots(kStages)], a_empty[kStages];
 };
-// kStandardised: the rows are a standardised fp16 copy (otherwise bf16 rows of z).
-template <int kStages_, bool kStandardised_, int kRun_ = 128>
+// kStandardised: the rows are a standardised fp16 copy (otherwise bf16 rows of z).  kSets: of statistics warps for bf16 rows
+// (tile_stats_loop).
+template <int kStages_, bool kStandardised_, int kRun_ = 128, int kSets_ = 1>
 struct TileCtx {
-  static constexpr int kStages = kStages_, kSlots = tile_slots(kStages_), kFulls = tile_fulls(kStages_);
+  static constexpr int kStages = kStages_, kSlots = tile_slots(kStages_), kSets = kStandardised_ ? 1 : kSets_;
+  static constexpr int kFulls = tile_fulls(kStages_, kSets_);
   static constexpr bool kStandardised = kStandardised_;
   static constexpr int kRun = kRun_;          // elements of a run: 128 or 64
   unsigned char* tiles;     // kStages x kTileBytes
   unsigned char* extras;    // tile_extras() x kTileExtra (the correction step of a tile runs after its stage is freed)
-  TileBars<kStages_>* bars;
+  TileBars<kStages_, kFulls>* bars;
   int first_tile, tile_step, n_tiles, runs_t, n_u, n_t, swap;   // runs_t: runs that cover the t of one u
   __device__ __forceinline__ uint64_t* full(int k) const { return &bars->raw_full[k % kFulls]; }
   __device__ __forceinline__ uint32_t full_parity(int k) const { return (k / kFulls) & 1; }
   __device__ __forceinline__ unsigned char* extra(int k) const { return extras + (kStandardised ? 0 : (k % kSlots) * kTileExtra); }
 };
 
-// Statistics warps: four, a thread per row, where there is nothing to measure; for bf16 rows two sets of four that take the tiles in
-// turn, two threads a row.
-constexpr int kStatsSet = 4;
-constexpr int tile_stats_sets(bool standardised) { return standardised ? 1 : 2; }
-constexpr int tile_stats_warps(bool standardised) { return kStatsSet * tile_stats_sets(standardised); }
+// Statistics warps: a thread per row where there is nothing to measure, two for bf16 rows.
+constexpr int tile_stats_warps(bool standardised) { return standardised ? 4 : 8; }
 // readers: how many arrivals free a stage besides those of the statistics warps.
-template <int kStages>
-__device__ __forceinline__ void tile_bars_init(TileBars<kStages>& b, int readers) {
-  for (int s = 0; s < tile_fulls(kStages); ++s) mbar_init(&b.raw_full[s], 1);
-  for (int s = 0; s < kStages; ++s) mbar_init(&b.a_empty[s], readers + kStatsSet);
-  for (int s = 0; s < tile_slots(kStages); ++s) mbar_init(&b.a_ready[s], kStatsSet);
+template <typename Ctx>
+__device__ __forceinline__ void tile_bars_init(const Ctx& c, int readers) {
+  constexpr int kWarps = tile_stats_warps(Ctx::kStandardised) / Ctx::kSets;       // of a set
+  for (int s = 0; s < Ctx::kFulls; ++s) mbar_init(&c.bars->raw_full[s], 1);
+  for (int s = 0; s < Ctx::kStages; ++s) mbar_init(&c.bars->a_empty[s], readers + kWarps);
+  for (int s = 0; s < Ctx::kSlots; ++s) mbar_init(&c.bars->a_ready[s], kWarps);
 }
 
 // Run number `run`: which u, and its first t.  With runs of 64 tile k is made of the runs 2 k and 2 k + 1, which lie behind one another or are
@@ -323,11 +323,14 @@ __device__ __forceinline__ void bf16_row_stats(const unsigned char* tile, int r,
 // (mean 0, deviation 1 by construction), so the correction row is (0, 1), written once, and the factor is 1.
 // fetched: what ahead(u, t) loaded from global memory a tile earlier, so that nothing waits for it between the arrival of a tile and the
 // hand-over.  after(u, t) follows once the stage and the statistics have been handed over: for what nothing in the kernel waits for.
-// A tile's statistics are a chain of 1.3 us (arrival, loads, sums, square roots, hand-over), about what a tile lasts: two sets of four
-// warps work on two tiles, each lane on two rows of its tile at once.  Eight warps on one tile, with the load of the mask on the chain,
-// against that (projections of the triangle multiplication, outgoing, us): bf16 N = 200 15.2 -> 14.5, 384 36.2 -> 31.0, 437 47.0 -> 42.8,
-// 768 118 -> 105.5, 1536 477 -> 424 (the mask alone 111 at 768; without any statistics 96); fp16 rows, which only had the mask
-// there, 384 28.9 -> 27.8, 768 98 -> 94.5, 1536 388 -> 377.
+// A tile's statistics are a chain of 1.3 us (arrival, loads, sums, square roots, hand-over).  In the projections of the triangle
+// multiplication a tile lasts about as long: two sets of four warps work on two tiles there, each lane on two rows of its tile at once.
+// Eight warps on one tile, with the load of the mask on the chain, against that (outgoing, us): bf16 N = 200 15.2 -> 14.5, 384 36.2 -> 31.0,
+// 437 47.0 -> 42.8, 768 118 -> 105.5, 1536 477 -> 424 (the mask alone 111 at 768; without any statistics 96); fp16 rows, which only had
+// the mask there, 384 28.9 -> 27.8, 768 98 -> 94.5, 1536 388 -> 377.  In the output stage of the triangle attention, whose tiles
+// last longer than their statistics, all eight work on one tile (two sets | one set: N = 128 11.5 | 11.1, 384 30.9 | 29.9, 768 108.7 | 105,
+// 1536 398 | 392), and so they do in the pair bias (128 5.5 | 5.3, 256 7.7 | 7.4, 1024 56 | 55) and the recycling update (level).
+// Projections of the triangle attention: by the number of tiles (triatt_in_tc.cu).
 struct TileNothingAhead {
   __device__ __forceinline__ float operator()(int, int) const { return 0.f; }
 };
@@ -338,9 +341,9 @@ template <typename Ctx, typename PerRow, typename Ahead = TileNothingAhead, type
 __device__ __forceinline__ void tile_stats_loop(const Ctx& c, float eps, int sw, int lane, PerRow per_row, Ahead ahead = Ahead(),
                                                 After after = After()) {
   constexpr bool kStandardised = Ctx::kStandardised;
-  constexpr int kSets = tile_stats_sets(kStandardised), kRows = kStandardised ? 1 : 2;
-  const int set = kStandardised ? 0 : sw >> 2, half = kStandardised ? 0 : lane & 1;
-  const int r0 = kStandardised ? 32 * sw + lane : 16 * (sw & 3) + (lane >> 1);            // and r0 + 64
+  constexpr int kSets = Ctx::kSets, kRows = kSets;
+  const int set = kSets == 2 ? sw >> 2 : 0, half = kStandardised ? 0 : lane & 1;
+  const int r0 = kStandardised ? 32 * sw + lane : 16 * (kSets == 2 ? sw & 3 : sw) + (lane >> 1);      // two sets: and r0 + 64
   const auto where = [&](int tile, int j) {           // (u, t) of row j of this lane
     constexpr int kPer = 128 / Ctx::kRun;
     const int row = r0 + 64 * j;

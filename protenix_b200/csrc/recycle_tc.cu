@@ -73,7 +73,7 @@ recycle_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_consta
     if (kTma) prefetch_maps(map_init, map_out);
   }
   if (threadIdx.x == 0) {
-    tile_bars_init(bars.tile, 1);
+    tile_bars_init(ctx, 1);
     mbar_init(&bars.w_full, 1);
     mbar_init(&bars.acc_full, 1);
     mbar_init(&bars.acc_free, 8);

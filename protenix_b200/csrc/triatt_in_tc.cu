@@ -75,7 +75,7 @@ struct AiWeights {
 };
 
 // kF16: the rows are the standardised fp16 copy of an fp32 pair tensor (fp16 weights); otherwise bf16 rows of z.
-template <bool kF16, int kStages, int kRun>
+template <bool kF16, int kStages, int kRun, int kSets>
 __global__ void __launch_bounds__(ai_threads(kF16), 1)
 triatt_in_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_constant__ CUtensorMap map_v,
                     const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k, const float* __restrict__ mask,
@@ -88,7 +88,7 @@ triatt_in_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_cons
   AiBars<kStages>& bars = *reinterpret_cast<AiBars<kStages>*>(sm + Layout::bars);
   const int warp = warp_index(), lane = threadIdx.x & 31;
   const int hpair = blockIdx.x & 1;                      // this CTA's heads: 2*hpair, 2*hpair + 1
-  typedef TileCtx<kStages, kF16, kRun> Ctx;
+  typedef TileCtx<kStages, kF16, kRun, kSets> Ctx;
   constexpr int kPer = 128 / kRun;                       // runs of a tile
   constexpr int kCtl = 16 + tile_stats_warps(kF16);      // first control warp
   Ctx ctx;
@@ -106,7 +106,7 @@ triatt_in_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_cons
   const bool skip = cta_begin();         // an earlier bounded wait gave up: do not start new work
   if (threadIdx.x == 32) prefetch_maps(map_z, map_v, map_q, map_k);
   if (threadIdx.x == 0) {
-    tile_bars_init(bars.tile, 2);
+    tile_bars_init(ctx, 2);
     mbar_init(&bars.w_full, 1);
     for (int b = 0; b < 4; ++b) {
       mbar_init(&bars.acc_full[b >> 1][b & 1], 1);
@@ -265,7 +265,7 @@ triatt_in_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_cons
 
 PX_DEFINE_FAMILY_HOOKS(triatt_in)
 
-template <bool kF16, int kStages, int kRun>
+template <bool kF16, int kStages, int kRun, int kSets>
 static int32_t launch_triatt_in_runs(const void* z, const float* mask, const AiWeights<kF16>& weights, const void* folded,
                                 px_f16* q, px_f16* k, px_f16* v, float* bias, float* mask_bias, int64_t n_u,
                                 int64_t n, int64_t ldm, int32_t ending, float eps, float inf, cudaStream_t st) {
@@ -289,13 +289,13 @@ static int32_t launch_triatt_in_runs(const void* z, const float* mask, const AiW
       return PX_ERR_LAUNCH;
   const size_t smem = AiLayout<kF16, kStages>::total + 1024;
   static SmemLimit limit;
-  if (!limit.set(triatt_in_tc_kernel<kF16, kStages, kRun>, smem)) return PX_ERR_LAUNCH;
+  if (!limit.set(triatt_in_tc_kernel<kF16, kStages, kRun, kSets>, smem)) return PX_ERR_LAUNCH;
   const int64_t n_tiles = tiles_of(n_u, n, kRun);
   if (n_tiles > 0x7fffffff) return PX_ERR_UNSUPPORTED;
   // Whole tiles of bf16 rows take little longer than ragged ones (their statistics are the same work), and an even number serves them 2 to 4 %
   // better from 132 to 230 tokens (N = 160 13.5 us against 14.0), 1 to 2 % worse at 430 and 450; standardised rows gain 3 to 8 % there.
   const int pairs = even_grid(n_tiles, sm_count() / 2, kF16 ? tile_period(n_u, n, kRun) : 1);
-  return launch_pdl(triatt_in_tc_kernel<kF16, kStages, kRun>, dim3(2 * pairs), ai_threads(kF16), smem, st, mz, mv, mq, mk, mask, weights,
+  return launch_pdl(triatt_in_tc_kernel<kF16, kStages, kRun, kSets>, dim3(2 * pairs), ai_threads(kF16), smem, st, mz, mv, mq, mk, mask, weights,
                     (const unsigned char*)folded, bias, mask_bias, (int)n_u, (int)n, (int)ldm, (int)ending, eps, inf, (int)runs_of(n, kRun),
                     (int)n_tiles)
              ? PX_OK
@@ -306,8 +306,17 @@ template <bool kF16, int kStages>
 static int32_t launch_triatt_in(const void* z, const float* mask, const AiWeights<kF16>& weights, const void* folded,
                                 px_f16* q, px_f16* k, px_f16* v, float* bias, float* mask_bias, int64_t n_u,
                                 int64_t n, int64_t ldm, int32_t ending, float eps, float inf, cudaStream_t st) {
-  return (two_runs_pay(n_u, n) ? launch_triatt_in_runs<kF16, kStages, 64> : launch_triatt_in_runs<kF16, kStages, 128>)(
-      z, mask, weights, folded, q, k, v, bias, mask_bias, n_u, n, ldm, ending, eps, inf, st);
+  const bool two_runs = two_runs_pay(n_u, n);
+  // Two sets of statistics warps for bf16 rows where a CTA has 2 to 12 tiles: a single tile is measured faster by eight warps than by four, and
+  // from more tiles on the time is that of the memory, which tiles measured ahead of their turn only crowd.  One set | two, us, starting node:
+  // N = 64 11.3 | 11.5, 100 12.8 | 12.5, 200 20.5 | 19.5, 300 32.3 | 31.5, 320 33.1 | 32.7, 360 40.1 | 40.1, 512 64.8 | 64.9, 768 139 | 141; ending
+  // node 64 11.2 | 11.6, 200 20.6 | 19.5, 300 32.4 | 31.9, 384 42.3 | 43.3, 768 138 | 146, 1024 231 | 245; 96 rows of 768 24.5 | 22.8, 192 41.8 | 41.8.
+  const int64_t room = sm_count() / 2, rounds = (tiles_of(n_u, n, two_runs ? 64 : 128) + room - 1) / room;
+  constexpr int kTwo = kF16 ? 1 : 2;
+  const auto run = rounds > 1 && rounds <= 12
+                       ? (two_runs ? launch_triatt_in_runs<kF16, kStages, 64, kTwo> : launch_triatt_in_runs<kF16, kStages, 128, kTwo>)
+                       : (two_runs ? launch_triatt_in_runs<kF16, kStages, 64, 1> : launch_triatt_in_runs<kF16, kStages, 128, 1>);
+  return run(z, mask, weights, folded, q, k, v, bias, mask_bias, n_u, n, ldm, ending, eps, inf, st);
 }
 
 // Stages for the standardised rows of an fp32 pair tensor.  Three let the two CTAs of a pair drift apart, and once the rows are larger than

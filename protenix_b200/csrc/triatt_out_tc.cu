@@ -101,7 +101,7 @@ triatt_out_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_con
   }
   if (threadIdx.x == 0) {
     // a stage is read by the gate product and the output warps
-    tile_bars_init(bars.tile, 2);
+    tile_bars_init(ctx, 2);
     mbar_init(&bars.w_full, 1);
     mbar_init(&bars.g_full, 1);
     mbar_init(&bars.g_free, 8);

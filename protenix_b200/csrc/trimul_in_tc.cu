@@ -23,14 +23,14 @@
 
 namespace px {
 
-constexpr int kTiStages = 3;
+constexpr int kTiStages = 3, kTiSets = 2;     // sets of statistics warps for bf16 rows
 constexpr int kTiWExtra = 128 * 32;            // [128 rows][16 k] weight-side correction panel
 constexpr int kTiStageOut = 32 * 256;          // per run [32 channels][t] fp16
 constexpr int ti_threads(bool f16) { return 32 * (16 + tile_stats_warps(f16) + 3); }
 // tensor memory: out a | out b, twice
 
 struct TiBars {
-  TileBars<kTiStages> tile;
+  TileBars<kTiStages, tile_fulls(kTiStages, kTiSets)> tile;
   uint64_t acc_full[2][2], acc_free[2][2];   // [output][accumulator]
   uint64_t w_full;
   uint32_t tmem_base;
@@ -76,7 +76,7 @@ trimul_in_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_cons
   const int warp = warp_index(), lane = threadIdx.x & 31;
   constexpr int kCtl = 16 + tile_stats_warps(kF16);      // first control warp
   const int chan0 = 64 * (blockIdx.x & 1);               // this CTA's channels of a and b
-  typedef TileCtx<kTiStages, kF16, kRun> Ctx;
+  typedef TileCtx<kTiStages, kF16, kRun, kTiSets> Ctx;
   constexpr int kPer = 128 / kRun;                       // runs of a tile
   Ctx ctx;
   ctx.tiles = sm + TiLayout::a;
@@ -93,7 +93,7 @@ trimul_in_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_cons
   const bool skip = cta_begin();         // an earlier bounded wait gave up: do not start new work
   if (threadIdx.x == 32) prefetch_maps(map_z, map_a, map_b);
   if (threadIdx.x == 0) {
-    tile_bars_init(bars.tile, 2);
+    tile_bars_init(ctx, 2);
     mbar_init(&bars.w_full, 1);
     for (int b = 0; b < 4; ++b) {
       mbar_init(&bars.acc_full[b >> 1][b & 1], 1);

@@ -85,3 +85,17 @@ def test_two_runs_a_tile_beyond_l2(ending, n_t=520):
             assert float((a.double() - b).norm() / b.norm()) < 1e-3, name
     assert bool((mb[:, n_t:] == -math.inf).all()) and not bool(bias[..., n_t:].any()) and not bool(v[..., n_t:].any())
     ops.device_error_flags()
+
+
+@pytest.mark.parametrize("ending", [False, True])
+@pytest.mark.parametrize("n_t", [384, 400])
+def test_any_number_of_tiles_a_cta_gives_the_same_bits(ending, n_t):
+    """bf16 rows are measured by one set of warps or by two, by the tiles of a CTA: many, some and one of them here."""
+    z, mask, w = inputs(n_t, n_t, torch.bfloat16, ending)
+    whole = ops.triatt_in_proj(z, mask, *w, ending=ending)
+    for n_u in (300, 100, 37, 10, 1):
+        part = (slice(None), slice(7, 7 + n_u)) if ending else (slice(7, 7 + n_u),)
+        slab = ops.triatt_in_proj(z[part].contiguous(), mask[part].contiguous(), *w, ending=ending)
+        for name, a, b in zip("qkvbm", whole, slab):
+            assert torch.equal(a[:, 7:7 + n_u] if name == "b" else a[7:7 + n_u], b), (name, n_u)
+    ops.device_error_flags()
