@@ -259,15 +259,30 @@ static inline int64_t tile_period(int64_t n_u, int64_t n_t, int run) {
 }
 
 // Where consecutive rows of tiles lie behind one another in every tensor of a kernel (rows of z as they are, and no pad columns), the
-// tiles need not end with each row: one row of n_u * n_t elements has fewer of them unless n_t is a multiple of 64 (both output stages of
+// tiles need not end with each row: one row of n_u * n_t elements has fewer of them unless n_t is a multiple of 128 (both output stages of
 // the triangle multiplication, its outgoing projection and the output stage of the starting node, us a block of a stack: 160 tokens
 // 205.3 -> 196.5, 200 260.5 -> 252.5, 400 914 -> 873; where fewer tiles leave SMs free, the single branch has them).
 static inline bool one_row_pays(int64_t n_u, int64_t n_t) { return n_u > 1 && n_t % 64 != 0; }
 
+// How an output stage cuts its tiles: each u by itself (kRows), runs of 64, or as one row where that is possible; whichever makes fewer tiles,
+// and runs of 64, with their twice as many loads and stores, only where one row does not.  us, rows | runs | one row: triangle multiplication
+// N = 150 bf16 17.1 | 14.4 | - (pad columns), 160 17.0 | 14.4 | 14.3, 400 39.7 | 37.2 | 34.7, 1096 219 | 219 | 212, fp32 264 25.8 | 23.3 | 21.1;
+// starting node 300 fp32 25.6 | 23.4 | 21.6, bf16 448 48.8 | 45.5 | 44.4, whole tiles (N = 768) 104 | 107.
+// fp32 rows are the exception at both ends.  Where most SMs are idle anyway, an SM's tile should be small: N = 24 11.1 | 11.4 | 11.8, 64 11.5 |
+// 11.9 | 11.9, 100 level, 120 12.7 | 12.8 | 12.4.  From `most` tiles an SM on the time is that of their memory traffic, which the same SMs
+// ask for in fewer places at once when all tiles are full: triangle attention 320 26.6 | 24.8 | 24.4, 400 47.7 | 47.9 | 49.0, 437 54.8 | 56.4 |
+// 56.9, 776 148 | 151 | 157, triangle multiplication 520 78.8 | 77.0 | 77.0, 680 120 | 120 | 122, 1000 241 | 241 | 246.  most = 0: none.
+enum class Cut { kRows, kRuns, kOneRow };
+static inline Cut output_cut(int64_t n_u, int64_t n_t, bool can_be_one_row, int64_t most) {
+  const int64_t rows = tiles_of(n_u, n_t, 128), room = sm_count();
+  if (most && (3 * rows <= 2 * room || rows > most * room)) return Cut::kRows;
+  if (can_be_one_row && tiles_of(1, n_u * n_t, 128) < rows) return Cut::kOneRow;
+  return rows > room && tiles_of(n_u, n_t, 64) < rows ? Cut::kRuns : Cut::kRows;
+}
+
 // Projections: tiles of two runs where that makes fewer of them.  They load and store twice as many pieces, which costs whole tiles 2 (fp16)
 // to 6 % (bf16), hence up to 1024.  Incoming projection of the triangle multiplication, us, one run of 128 | two of 64: bf16 N = 136
 // 11.4 | 10.3, 437 43.5 | 41.0, 700 97.3 | 95.2, whole tiles 384 31.7 | 33.3; fp16 437 40.2 | 38.7, 700 93.2 | 86.3, 768 95.9 | 98.0.
-// The output stages, which nothing but the loads tells of it, take runs of 64 always.
 static inline bool two_runs_pay(int64_t n_u, int64_t n_t) { return n_u > 1 && n_t < 1024 && (n_t - 1) % 128 < 64; }
 
 // One warp: TMA loads of the tiles (boxes of a run).

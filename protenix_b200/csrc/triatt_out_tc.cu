@@ -67,7 +67,7 @@ struct AoWeights {
   }
 };
 
-template <int kMode>
+template <int kMode, int kRun>
 __global__ void __launch_bounds__(ao_threads(kMode != 0), 1)
 triatt_out_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_constant__ CUtensorMap map_o,
                      const __grid_constant__ CUtensorMap map_out, const void* __restrict__ z_in, void* __restrict__ z_out,
@@ -80,7 +80,8 @@ triatt_out_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_con
   unsigned char* sm = smem_aligned(smem_raw);
   AoBars& bars = *reinterpret_cast<AoBars*>(sm + AoLayout::bars);
   const int warp = warp_index(), lane = threadIdx.x & 31;
-  typedef TileCtx<kAoStages, kF16, 64> Ctx;
+  typedef TileCtx<kAoStages, kF16, kRun> Ctx;
+  constexpr int kPer = 128 / kRun;                       // runs of a tile
   constexpr int kCtl = 16 + tile_stats_warps(kF16);      // first control warp
   Ctx ctx;
   ctx.tiles = sm + AoLayout::a;
@@ -138,10 +139,10 @@ triatt_out_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_con
         if (elect_lane()) {
           mbar_expect_tx(ctx.full(k), 2 * kOperandBytes);
           const uint32_t zdst = smem_u32(ctx.tiles + s * kTileBytes), odst = smem_u32(sm + AoLayout::o + s * kOperandBytes);
-          for (int h = 0; h < 2; ++h) {
-            const Run r = run_at<64>(2 * tile + h, runs_t);
+          for (int h = 0; h < kPer; ++h) {
+            const Run r = run_at<kRun>(kPer * tile + h, runs_t);
             for (int p = 0; p < 2; ++p) {
-              const int at = p * kPanelBytes + h * (64 * 128);
+              const int at = p * kPanelBytes + h * (kRun * 128);
               tma_load_3d(zdst + at, &map_z, ctx.full(k), 64 * p, swap ? r.u : r.t, swap ? r.t : r.u);
               tma_load_3d(odst + at, &map_o, ctx.full(k), 64 * p, r.t, r.u);
             }
@@ -150,8 +151,8 @@ triatt_out_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_con
           // their way): bf16 N = 768 103 -> 93 us.  Not where rows are added in L2, which is then what is waited for: 562 -> 594 at N = 1536.
           const int next = tile + 2 * ctx.tile_step;
           if ((kTma || (kBulk && !add_residual)) && next < n_tiles) {
-            for (int h = 0; h < 2; ++h) {
-              const Run r = run_at<64>(2 * next + h, runs_t);
+            for (int h = 0; h < kPer; ++h) {
+              const Run r = run_at<kRun>(kPer * next + h, runs_t);
               for (int p = 0; p < 2; ++p) {
                 tma_prefetch_3d(&map_z, 64 * p, swap ? r.u : r.t, swap ? r.t : r.u);
                 tma_prefetch_3d(&map_o, 64 * p, r.t, r.u);
@@ -243,8 +244,8 @@ triatt_out_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_con
     bool ok = true;
     for (int tile = ctx.first_tile; tile < n_tiles && ok; tile += ctx.tile_step, ++k) {
       const int s = k % kAoStages;
-      const Run run = run_at<64>(2 * tile + (qw >> 1), runs_t);
-      const int u = run.u, tw = run.t + 32 * (qw & 1);
+      const Run run = run_at<kRun>(kPer * tile + 32 * qw / kRun, runs_t);
+      const int u = run.u, tw = run.t + 32 * qw % kRun;
       // fp32 rows: this warp's 32 rows (u, tw + i) in units of 128-channel rows of z, and their residual
       // values for the first 32 channels, requested before the wait (the second block's lines are asked of L2)
       const long long first_row = swap ? (long long)tw * n_u + u : (long long)u * n + tw;
@@ -260,8 +261,8 @@ triatt_out_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_con
         // and both blocks of the next tile, so that its requests hit L2
         const int nt = tile + ctx.tile_step;
         if (add_residual && nt < n_tiles) {
-          const Run r2 = run_at<64>(2 * nt + (qw >> 1), runs_t);
-          const int u2 = r2.u, t2 = r2.t + 32 * (qw & 1) + lane;
+          const Run r2 = run_at<kRun>(kPer * nt + 32 * qw / kRun, runs_t);
+          const int u2 = r2.u, t2 = r2.t + 32 * qw % kRun + lane;
           if (t2 < n && u2 < n_u) {
             const float* p2 = reinterpret_cast<const float*>(z_in) + (size_t)(swap ? (long long)t2 * n_u + u2 : (long long)u2 * n + t2) * kC + 64 * half;
             asm volatile("prefetch.global.L2 [%0];\n" ::"l"(p2));
@@ -330,10 +331,10 @@ triatt_out_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_con
         asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
         named_barrier(1, 256);
         if (leader) {
-          for (int h = 0; h < 2; ++h) {
-            const Run r = run_at<64>(2 * tile + h, runs_t);
+          for (int h = 0; h < kPer; ++h) {
+            const Run r = run_at<kRun>(kPer * tile + h, runs_t);
             for (int p = 0; p < 2 && r.u < n_u; ++p)
-              tma_store_3d(&map_out, smem_u32(otile + p * kPanelBytes) + h * (64 * 128), 64 * p, swap ? r.u : r.t, swap ? r.t : r.u);
+              tma_store_3d(&map_out, smem_u32(otile + p * kPanelBytes) + h * (kRun * 128), 64 * p, swap ? r.u : r.t, swap ? r.t : r.u);
           }
           tma_store_commit();
           tma_store_wait_read<0>();                        // the store has read the stage: hand it back
@@ -358,19 +359,18 @@ triatt_out_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_con
 
 PX_DEFINE_FAMILY_HOOKS(triatt_out)
 
-template <int kMode>
-static int32_t launch_triatt_out(const px_f16* o, const void* z_in, const px_f16* zn, void* z_out,
+template <int kMode, int kRun>
+static int32_t launch_triatt_out_runs(const px_f16* o, const void* z_in, const px_f16* zn, void* z_out,
                                  const AoWeights<kMode != 0>& weights, const void* folded, int64_t n_u, int64_t n, int32_t ending,
                                  int32_t add_residual, float eps, cudaStream_t st) {
   CUtensorMap mz, mo, mout;
-  if (!ending && one_row_pays(n_u, n)) n *= n_u, n_u = 1;
   // operand rows: bf16 z itself, or the standardised fp16 copy of an fp32 z; pair element (u, t) is row u*n + t, or
   // row t*n_u + u when the two indices are exchanged
   const CUtensorMapDataType zt = kMode == 0 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
   const void* zrows = kMode == 1 || kMode == 3 ? (const void*)zn : z_in;
   if (!(ending ? make_map_3d(&mz, zt, zrows, 128, (uint64_t)n_u, (uint64_t)n, 256, (uint64_t)n_u * 256, 64, 1,
-                             CU_TENSOR_MAP_SWIZZLE_128B, 64)
-               : make_map_3d(&mz, zt, zrows, 128, (uint64_t)n, (uint64_t)n_u, 256, (uint64_t)n * 256, 64, 64,
+                             CU_TENSOR_MAP_SWIZZLE_128B, kRun)
+               : make_map_3d(&mz, zt, zrows, 128, (uint64_t)n, (uint64_t)n_u, 256, (uint64_t)n * 256, 64, kRun,
                              CU_TENSOR_MAP_SWIZZLE_128B, 1)))
     return PX_ERR_LAUNCH;
   if (kMode == 3) {
@@ -381,26 +381,36 @@ static int32_t launch_triatt_out(const px_f16* o, const void* z_in, const px_f16
       return PX_ERR_LAUNCH;
   } else if (kMode != 1) {
     if (!(ending ? make_map_3d(&mout, zt, z_out, 128, (uint64_t)n_u, (uint64_t)n, 256, (uint64_t)n_u * 256, 64, 1,
-                               CU_TENSOR_MAP_SWIZZLE_128B, 64)
-                 : make_map_3d(&mout, zt, z_out, 128, (uint64_t)n, (uint64_t)n_u, 256, (uint64_t)n * 256, 64, 64,
+                               CU_TENSOR_MAP_SWIZZLE_128B, kRun)
+                 : make_map_3d(&mout, zt, z_out, 128, (uint64_t)n, (uint64_t)n_u, 256, (uint64_t)n * 256, 64, kRun,
                                CU_TENSOR_MAP_SWIZZLE_128B, 1)))
       return PX_ERR_LAUNCH;
   } else {
     memset(&mout, 0, sizeof(mout));
   }
   if (!make_map_3d(&mo, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, o, 128, (uint64_t)n, (uint64_t)n_u, 256, (uint64_t)n * 256, 64,
-                   64, CU_TENSOR_MAP_SWIZZLE_128B, 1))
+                   kRun, CU_TENSOR_MAP_SWIZZLE_128B, 1))
     return PX_ERR_LAUNCH;
   const size_t smem = AoLayout::total + 1024;
   static SmemLimit limit;
-  if (!limit.set(triatt_out_tc_kernel<kMode>, smem)) return PX_ERR_LAUNCH;
-  const int64_t n_tiles = tiles_of(n_u, n, 64);
+  if (!limit.set(triatt_out_tc_kernel<kMode, kRun>, smem)) return PX_ERR_LAUNCH;
+  const int64_t n_tiles = tiles_of(n_u, n, kRun);
   if (n_tiles > 0x7fffffff) return PX_ERR_UNSUPPORTED;
-  const int grid = even_grid(n_tiles, sm_count(), tile_period(n_u, n, 64));
-  return launch_pdl(triatt_out_tc_kernel<kMode>, dim3(grid), ao_threads(kMode != 0), smem, st, mz, mo, mout, z_in, z_out, weights,
-                    (const unsigned char*)folded, (int)n_u, (int)n, (int)ending, (int)add_residual, eps, (int)runs_of(n, 64), (int)n_tiles)
+  const int grid = even_grid(n_tiles, sm_count(), tile_period(n_u, n, kRun));
+  return launch_pdl(triatt_out_tc_kernel<kMode, kRun>, dim3(grid), ao_threads(kMode != 0), smem, st, mz, mo, mout, z_in, z_out, weights,
+                    (const unsigned char*)folded, (int)n_u, (int)n, (int)ending, (int)add_residual, eps, (int)runs_of(n, kRun), (int)n_tiles)
              ? PX_OK
              : PX_ERR_LAUNCH;
+}
+
+template <int kMode>
+static int32_t launch_triatt_out(const px_f16* o, const void* z_in, const px_f16* zn, void* z_out,
+                                 const AoWeights<kMode != 0>& weights, const void* folded, int64_t n_u, int64_t n, int32_t ending,
+                                 int32_t add_residual, float eps, cudaStream_t st) {
+  const Cut cut = output_cut(n_u, n, !ending, kMode == 1 || kMode == 3 ? 8 : 0);
+  if (cut == Cut::kOneRow) n *= n_u, n_u = 1;
+  return (cut == Cut::kRuns ? launch_triatt_out_runs<kMode, 64> : launch_triatt_out_runs<kMode, 128>)(
+      o, z_in, zn, z_out, weights, folded, n_u, n, ending, add_residual, eps, st);
 }
 
 // The three forms by the type of z; w: the raw weights (ignored when they come folded).

@@ -75,12 +75,13 @@ struct ToWeights {
   }
 };
 
-template <typename Tz, bool kBulk>
+template <typename Tz, bool kBulk, int kRun>
 __global__ void __launch_bounds__(to_threads(sizeof(Tz) != 2), 1)
 trimul_out_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_constant__ CUtensorMap map_x,
                      const __grid_constant__ CUtensorMap map_out, const Tz* __restrict__ z_in, Tz* __restrict__ z_out,
                      const ToWeights<sizeof(Tz) != 2> weights, const unsigned char* __restrict__ folded,
                      int n_i, int n, int add_residual, float eps, int runs_j, int n_tiles) {
+  constexpr int kPer = 128 / kRun;                     // runs of a tile
   constexpr bool kTma = sizeof(Tz) == 2;               // bf16: residual from the z tile, output through TMA
   constexpr bool kF16 = !kTma;                           // operand format of the z side; the x side is always fp16
   constexpr int kStats = to_stats_warps(kF16), kThreads = to_threads(kF16), kLoad = 16 + kStats;   // kLoad: the producer's warp
@@ -141,21 +142,21 @@ trimul_out_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_con
         if (elect_lane()) {
           mbar_expect_tx(&bars.raw_full[s], 2 * kOperandBytes);
           const uint32_t zdst = smem_u32(sm + ToLayout::zt + s * kOperandBytes), xdst = smem_u32(sm + ToLayout::xt + s * kOperandBytes);
-          for (int h = 0; h < 2; ++h) {
-            const Run r = run_at<64>(2 * tile + h, runs_j);
+          for (int h = 0; h < kPer; ++h) {
+            const Run r = run_at<kRun>(kPer * tile + h, runs_j);
             for (int p = 0; p < 2; ++p)
-              tma_load_3d(zdst + p * kPanelBytes + h * (64 * 128), &map_z, &bars.raw_full[s], 64 * p, r.t, r.u);
-            tma_load_3d(xdst + h * kPanelBytes, &map_x, &bars.raw_full[s], r.t, r.u, 0);
+              tma_load_3d(zdst + p * kPanelBytes + h * (kRun * 128), &map_z, &bars.raw_full[s], 64 * p, r.t, r.u);
+            for (int p = 0; p < kRun / 64; ++p) tma_load_3d(xdst + (h + p) * kPanelBytes, &map_x, &bars.raw_full[s], r.t + 64 * p, r.u, 0);
           }
           // The tile that takes this stage next is asked of L2 (a stage is held until its rows have left, so only two tiles are on
           // their way): bf16 N = 768 122 -> 107 us, fp32 without a residual N = 1024 230 -> 203.  Not where rows are added in L2,
           // which is then what is waited for: 552 -> 610 at N = 1536, 140 -> 151 at N = 768.
           const int next = tile + 2 * tile_step;
           if ((kTma || (kBulk && !add_residual)) && next < n_tiles) {
-            for (int h = 0; h < 2; ++h) {
-              const Run r = run_at<64>(2 * next + h, runs_j);
+            for (int h = 0; h < kPer; ++h) {
+              const Run r = run_at<kRun>(kPer * next + h, runs_j);
               for (int p = 0; p < 2; ++p) tma_prefetch_3d(&map_z, 64 * p, r.t, r.u);
-              tma_prefetch_3d(&map_x, r.t, r.u, 0);
+              for (int p = 0; p < kRun / 64; ++p) tma_prefetch_3d(&map_x, r.t + 64 * p, r.u, 0);
             }
           }
         }
@@ -259,8 +260,8 @@ trimul_out_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_con
     bool ok = true;
     for (int tile = first_tile; tile < n_tiles && ok; tile += tile_step, ++k) {
       const int s = k % kToStages;
-      const Run run = run_at<64>(2 * tile + (qw >> 1), runs_j);
-      const int i = run.u, jw = run.t + 32 * (qw & 1);     // the warp's first element
+      const Run run = run_at<kRun>(kPer * tile + 32 * qw / kRun, runs_j);
+      const int i = run.u, jw = run.t + 32 * qw % kRun;     // the warp's first element
       const int valid = i >= n_i || jw >= n ? 0 : n - jw < 32 ? n - jw : 32;
       RowsOutReq rq;
       if (!kTma && !kBulk) {                               // the residual values are requested before the wait
@@ -268,8 +269,8 @@ trimul_out_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_con
         // the residual lines of the next tile are asked of L2 now: a tile later they are a hit, not a trip to HBM
         const int nt = tile + tile_step;
         if (add_residual && nt < n_tiles) {
-          const Run r2 = run_at<64>(2 * nt + (qw >> 1), runs_j);
-          const int i2 = r2.u, j2 = r2.t + 32 * (qw & 1) + lane;
+          const Run r2 = run_at<kRun>(kPer * nt + 32 * qw / kRun, runs_j);
+          const int i2 = r2.u, j2 = r2.t + 32 * qw % kRun + lane;
           if (j2 < n && i2 < n_i)
             asm volatile("prefetch.global.L2 [%0];\n" ::"l"(reinterpret_cast<const float*>(z_in) + ((size_t)i2 * n + j2) * kC + 32 * part));
         }
@@ -317,10 +318,10 @@ trimul_out_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_con
         asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
         named_barrier(1, 512);
         if (leader) {
-          for (int h = 0; h < 2; ++h) {
-            const Run r = run_at<64>(2 * tile + h, runs_j);
+          for (int h = 0; h < kPer; ++h) {
+            const Run r = run_at<kRun>(kPer * tile + h, runs_j);
             for (int pnl = 0; pnl < 2 && r.u < n_i; ++pnl)
-              tma_store_3d(&map_out, smem_u32(ztile + pnl * kPanelBytes) + h * (64 * 128), 64 * pnl, r.t, r.u);
+              tma_store_3d(&map_out, smem_u32(ztile + pnl * kPanelBytes) + h * (kRun * 128), 64 * pnl, r.t, r.u);
           }
           tma_store_commit();
           tma_store_wait_read<0>();                          // the store has read the stage: hand it back
@@ -356,20 +357,19 @@ trimul_out_tc_kernel(const __grid_constant__ CUtensorMap map_z, const __grid_con
 PX_DEFINE_FAMILY_HOOKS(trimul_out)
 
 // kBulk (fp32 z): the output goes through TMA, which covers everything but a residual from another tensor.
-template <typename Tz, bool kBulk>
-static int32_t launch_trimul_out(const px_f16* x, const void* z_in, const px_f16* zn, void* z_out,
+template <typename Tz, bool kBulk, int kRun>
+static int32_t launch_trimul_out_runs(const px_f16* x, const void* z_in, const px_f16* zn, void* z_out,
                                  const ToWeights<sizeof(Tz) != 2>& weights, const void* folded,
                                  int64_t n_i, int64_t n, int64_t ld, int32_t add_residual, float eps, cudaStream_t st) {
   CUtensorMap mz, mx, mout;
-  if (ld == n && one_row_pays(n_i, n)) n *= n_i, ld = n, n_i = 1;
   // operand rows: bf16 z itself, or the standardised fp16 copy of an fp32 z
   if (!make_map_3d(&mz, sizeof(Tz) == 2 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16,
-                   sizeof(Tz) == 2 ? z_in : (const void*)zn, 128, (uint64_t)n, (uint64_t)n_i, 256, (uint64_t)n * 256, 64, 64,
+                   sizeof(Tz) == 2 ? z_in : (const void*)zn, 128, (uint64_t)n, (uint64_t)n_i, 256, (uint64_t)n * 256, 64, kRun,
                    CU_TENSOR_MAP_SWIZZLE_128B, 1))
     return PX_ERR_LAUNCH;
   if (sizeof(Tz) == 2) {
     if (!make_map_3d(&mout, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, z_out, 128, (uint64_t)n, (uint64_t)n_i, 256, (uint64_t)n * 256,
-                     64, 64, CU_TENSOR_MAP_SWIZZLE_128B, 1))
+                     64, kRun, CU_TENSOR_MAP_SWIZZLE_128B, 1))
       return PX_ERR_LAUNCH;
   } else if (kBulk) {
     if (!make_map_3d(&mout, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, z_out, 128, (uint64_t)n, (uint64_t)n_i, 512, (uint64_t)n * 512, 32, 32,
@@ -384,14 +384,24 @@ static int32_t launch_trimul_out(const px_f16* x, const void* z_in, const px_f16
     return PX_ERR_LAUNCH;
   const size_t smem = ToLayout::total + 1024;
   static SmemLimit limit;
-  if (!limit.set(trimul_out_tc_kernel<Tz, kBulk>, smem)) return PX_ERR_LAUNCH;
-  const int64_t n_tiles = tiles_of(n_i, n, 64);
+  if (!limit.set(trimul_out_tc_kernel<Tz, kBulk, kRun>, smem)) return PX_ERR_LAUNCH;
+  const int64_t n_tiles = tiles_of(n_i, n, kRun);
   if (n_tiles > 0x7fffffff) return PX_ERR_UNSUPPORTED;
-  const int grid = even_grid(n_tiles, sm_count(), tile_period(n_i, n, 64));
-  return launch_pdl(trimul_out_tc_kernel<Tz, kBulk>, dim3(grid), to_threads(sizeof(Tz) != 2), smem, st, mz, mx, mout, (const Tz*)z_in, (Tz*)z_out, weights,
-                    (const unsigned char*)folded, (int)n_i, (int)n, (int)add_residual, eps, (int)runs_of(n, 64), (int)n_tiles)
+  const int grid = even_grid(n_tiles, sm_count(), tile_period(n_i, n, kRun));
+  return launch_pdl(trimul_out_tc_kernel<Tz, kBulk, kRun>, dim3(grid), to_threads(sizeof(Tz) != 2), smem, st, mz, mx, mout, (const Tz*)z_in, (Tz*)z_out, weights,
+                    (const unsigned char*)folded, (int)n_i, (int)n, (int)add_residual, eps, (int)runs_of(n, kRun), (int)n_tiles)
              ? PX_OK
              : PX_ERR_LAUNCH;
+}
+
+template <typename Tz, bool kBulk>
+static int32_t launch_trimul_out(const px_f16* x, const void* z_in, const px_f16* zn, void* z_out,
+                                 const ToWeights<sizeof(Tz) != 2>& weights, const void* folded,
+                                 int64_t n_i, int64_t n, int64_t ld, int32_t add_residual, float eps, cudaStream_t st) {
+  const Cut cut = output_cut(n_i, n, ld == n, sizeof(Tz) == 4 ? 18 : 0);
+  if (cut == Cut::kOneRow) n *= n_i, ld = n, n_i = 1;
+  return (cut == Cut::kRuns ? launch_trimul_out_runs<Tz, kBulk, 64> : launch_trimul_out_runs<Tz, kBulk, 128>)(
+      x, z_in, zn, z_out, weights, folded, n_i, n, ld, add_residual, eps, st);
 }
 
 static bool trimul_out_args_ok(const px_f16* x, const void* z_in, const px_f16* zn, const void* z_out, int32_t z_dtype, int64_t n_i,

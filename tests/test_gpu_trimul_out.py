@@ -48,3 +48,27 @@ def test_trimul_out_across_rows(n_i, n_j, dtype):
     for shift in (0.2, 30.0):
         rel = errors(n_i, n_j, dtype, shift)
         assert rel < (1e-3 if dtype == torch.float32 else 3e-3), (rel, shift)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("n", [64, 100, 136, 150, 200, 448, 520])
+def test_tiles_are_cut_in_three_ways_with_the_same_bits(n, dtype):
+    """Rows by themselves, runs of 64 and one row, by the number of tiles; a few rows of the whole are cut in another way or lie elsewhere in it."""
+    g = torch.Generator("cuda").manual_seed(n)
+    draw = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    z, x = draw(n, n, 128).to(dtype), torch.zeros(128, n, ops.ld(n), dtype=torch.half, device="cuda")
+    x[..., :n] = draw(128, n, n).half()
+    wt = torch.float16 if dtype == torch.float32 else dtype
+    vectors = [1 + 0.2 * draw(128), 0.2 * draw(128), 1 + 0.2 * draw(128), 0.2 * draw(128)]
+    o, w_z, w_g = draw(n, n, 128).half(), (0.09 * draw(128, 128)).half(), (0.09 * draw(128, 128)).to(wt)
+    mul = ops.trimul_out(x, z.clone(), *vectors, w_z, w_g)
+    start = ops.triatt_out(o, z.clone(), *vectors[:2], w_g, w_z)
+    end = ops.triatt_out(o, z.clone(), *vectors[:2], w_g, w_z, ending=True)
+    for n_u in (1, 7, 40, n - 3):
+        rows = slice(n - n_u, n)
+        part = z[rows].clone()
+        assert torch.equal(ops.trimul_out(x[:, rows].contiguous(), part.clone(), *vectors, w_z, w_g), mul[rows])
+        assert torch.equal(ops.triatt_out(o[rows], part, *vectors[:2], w_g, w_z), start[rows])
+        part = z[:, rows].contiguous()
+        assert torch.equal(ops.triatt_out(o[rows], part, *vectors[:2], w_g, w_z, ending=True), end[:, rows])
+    ops.device_error_flags()
