@@ -308,12 +308,13 @@ static int32_t launch_triatt_in(const void* z, const float* mask, const AiWeight
                                 int64_t n, int64_t ldm, int32_t ending, float eps, float inf, cudaStream_t st) {
   const bool two_runs = two_runs_pay(n_u, n);
   // Two sets of statistics warps for bf16 rows where a CTA has 2 to 12 tiles: a single tile is measured faster by eight warps than by four, and
-  // from more tiles on the time is that of the memory, which tiles measured ahead of their turn only crowd.  One set | two, us, starting node:
-  // N = 64 11.3 | 11.5, 100 12.8 | 12.5, 200 20.5 | 19.5, 300 32.3 | 31.5, 320 33.1 | 32.7, 360 40.1 | 40.1, 512 64.8 | 64.9, 768 139 | 141; ending
-  // node 64 11.2 | 11.6, 200 20.6 | 19.5, 300 32.4 | 31.9, 384 42.3 | 43.3, 768 138 | 146, 1024 231 | 245; 96 rows of 768 24.5 | 22.8, 192 41.8 | 41.8.
+  // from more tiles on the time is that of the memory, which tiles measured ahead of their turn only crowd.  The starting node keeps two
+  // with ragged tiles, which have less to write and the same to measure.  One set | two, us, starting node: N = 64 11.3 | 11.5, 100 12.8 | 12.5,
+  // 200 20.5 | 19.5, 300 32.3 | 31.5, 512 64.8 | 64.9, 768 139 | 141, ragged 437 53.1 | 52.3, 776 156 | 151, 1096 287 | 282; ending node 64
+  // 11.2 | 11.6, 200 20.6 | 19.5, 300 32.4 | 31.9, 384 42.3 | 43.3, 448 54.7 | 56.2, 768 138 | 146, 1024 231 | 245; 96 rows of 768 24.5 | 22.8.
   const int64_t room = sm_count() / 2, rounds = (tiles_of(n_u, n, two_runs ? 64 : 128) + room - 1) / room;
   constexpr int kTwo = kF16 ? 1 : 2;
-  const auto run = rounds > 1 && rounds <= 12
+  const auto run = rounds > 1 && (rounds <= 12 || (!ending && n % 64))
                        ? (two_runs ? launch_triatt_in_runs<kF16, kStages, 64, kTwo> : launch_triatt_in_runs<kF16, kStages, 128, kTwo>)
                        : (two_runs ? launch_triatt_in_runs<kF16, kStages, 64, 1> : launch_triatt_in_runs<kF16, kStages, 128, 1>);
   return run(z, mask, weights, folded, q, k, v, bias, mask_bias, n_u, n, ldm, ending, eps, inf, st);
