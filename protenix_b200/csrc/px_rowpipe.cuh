@@ -280,10 +280,15 @@ static inline Cut output_cut(int64_t n_u, int64_t n_t, bool can_be_one_row, int6
   return rows > room && tiles_of(n_u, n_t, 64) < rows ? Cut::kRuns : Cut::kRows;
 }
 
-// Projections: tiles of two runs where that makes fewer of them.  They load and store twice as many pieces, which costs whole tiles 2 (fp16)
-// to 6 % (bf16), hence up to 1024.  Incoming projection of the triangle multiplication, us, one run of 128 | two of 64: bf16 N = 136
-// 11.4 | 10.3, 437 43.5 | 41.0, 700 97.3 | 95.2, whole tiles 384 31.7 | 33.3; fp16 437 40.2 | 38.7, 700 93.2 | 86.3, 768 95.9 | 98.0.
-static inline bool two_runs_pay(int64_t n_u, int64_t n_t) { return n_u > 1 && n_t < 1024 && (n_t - 1) % 128 < 64; }
+// Projections (a pair of CTAs a tile): tiles of two runs where the last pair is through in fewer of them.  They load and store twice as many
+// pieces, which costs whole tiles 2 (fp16) to 6 % (bf16), hence up to 1024.  Incoming projection of the triangle multiplication, us, one run
+// of 128 | two of 64: bf16 N = 136 16.6 | 15.9, 264 28.0 | 25.9, 437 51.9 | 49.3, 700 119 | 118; fp16 192 17.9 | 16.2, 437 47.2 | 46.0, 700
+// 110 | 99; whole tiles 384 31.7 | 33.3; no fewer a pair: 55 rows of 437 bf16 15.6 | 16.0, fp16 14.7 | 15.2, 110 rows 19.8 | 20.4, 18.7 | 19.0.
+// With one tile a pair there is nothing in it but the fewer of them to start (N = 56 level, 64 12.4 | 11.9).
+static inline bool two_runs_pay(int64_t n_u, int64_t n_t) {
+  const int64_t rows = tiles_of(n_u, n_t, 128), runs = tiles_of(n_u, n_t, 64), room = sm_count() / 2;
+  return n_u > 1 && n_t < 1024 && runs < rows && (rows <= room || (runs + room - 1) / room < (rows + room - 1) / room);
+}
 
 // One warp: TMA loads of the tiles (boxes of a run).
 template <typename Ctx>
