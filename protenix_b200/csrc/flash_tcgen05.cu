@@ -520,17 +520,21 @@ extern "C" int32_t px_triatt_flash(const px_f16* q, const px_f16* k, const px_f1
   cudaStream_t st = (cudaStream_t)stream;
   const size_t smem = FlashLayout::total + 1024;
   // CTAs of six rows (two a group); where what is left of them for the last wave fits the SMs twice, that in CTAs of three (one a
-  // group; whole slices of the grid), so that the wave ends in little more than half the time: N = 100 10.2 -> 7.8 us, 160 23.9 -> 20.8,
-  // 256 41.5 -> 37.6, 300 76.5 -> 72, 384 106.4 -> 101.6, 512 218.5 -> 213.  CTAs of three only: 384 125, 768 805 against 653.  Each
+  // group; whole slices of the grid), so that the wave ends in little more than half the time: N = 100 10.2 -> 7.8 us and, one unit a CTA as
+  // well, 160 23.9 -> 20.8, 256 41.5 -> 37.6, 384 106.4 -> 101.6, 512 218.5 -> 213.  CTAs of three only: 384 125, 768 805 against 653.  Each
   // number of rows has its own code (as a run-time number, which leaves no parity known to the compiler, 15 % slower).
   const int64_t per = (n + 127) / 128 * kFH, slices = (n_u + kFRows - 1) / kFRows, room = sm_count(), left = per * slices % room;
   const int64_t halves = 2 * left <= room ? (left + per - 1) / per : 0, whole = slices - halves;
   // A last key tile of 32 keys at most is worked off by its half, in kernels of their own (the branch costs the others 1 %): N = 150
-  // 20.6 -> 19.2 us, 200 29.8 -> 28.1, 224 36.1 -> 34.1, 528 298 -> 291, 1056 1824 -> 1812, 1300 level.
+  // 20.6 -> 19.2 us, 200 29.8 -> 28.1, 224 36.1 -> 34.1, 528 298 -> 291 (one unit a CTA), 1056 1824 -> 1812, 1300 level.
   const bool brief = (n - 1) % kFKT < kFKT / 2;
-  // Up to forty units an SM (N = 1024) CTAs work on several; beyond, the beginnings and ends of CTAs are too few to pay for slower items.
+  // Up to 1024 keys CTAs work on several units; with more, a unit is so long that its beginning and end do not pay for the slower items.  How
+  // many units an SM gets makes no difference.  One unit a CTA | several, us, rows x keys: 160 x 160 19.1 | 17.1, 384 x 384 98.7 | 92.4, 2000 x 384
+  // 468 | 427, 7000 x 150 630 | 512, 768 x 768 631 | 628, 96 x 768 95.8 | 96.0, 3000 x 768 2564 | 2493, 1024 x 1024 1474 | 1460, 128 x 1024
+  // 207 | 207, 2000 x 1024 3010 | 2984; 1088 x 1088 1856 | 1889, 137 x 1100 264 | 273, 1100 x 1100 1931 | 1988, 1300 x 1300 3311 | 3418, 96 x 1536
+  // 318 | 326, 192 x 1536 614 | 615, 384 x 1536 1171 | 1195, 1536 x 1536 4824 | 5053, 256 x 2048 1467 | 1514, 512 x 2048 2973 | 3110.
   const int64_t units = per * slices;
-  if (units > room && units <= 40 * room) {
+  if (units > room && n <= 1024) {
     const int64_t halved = 2 * left <= room ? left : 0;
     const auto kernel = halved ? (brief ? triatt_flash_units_tc_kernel<true, true> : triatt_flash_units_tc_kernel<true, false>)
                                : (brief ? triatt_flash_units_tc_kernel<false, true> : triatt_flash_units_tc_kernel<false, false>);

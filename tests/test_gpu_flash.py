@@ -88,3 +88,22 @@ def test_many_units_a_cta_equal_one(n=130):
     for rows in (slice(0, 700), slice(n_u - 401, n_u)):
         assert torch.equal(ops.triatt_flash(q[rows], k[rows], v[rows], bias, mb[rows]), whole[rows])
     ops.device_error_flags()
+
+
+@pytest.mark.parametrize("n_u, n", [(2400, 130), (40, 1000), (36, 1024)])
+def test_several_units_a_cta_equal_one(n_u, n):
+    """Up to 1024 keys CTAs work on several units where there are more units than SMs; a few rows have a CTA for each of theirs.  Same bits."""
+    g = torch.Generator("cuda").manual_seed(n)
+    draw = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    q, k = (0.3 * draw(n_u, 4, n, 32)).half(), draw(n_u, 4, n, 32).half()
+    v = torch.zeros(n_u, 4, 32, ops.ld(n), dtype=torch.half, device="cuda")
+    v[..., :n] = draw(n_u, 4, 32, n).half()
+    ldm = (n + 127) // 128 * 128
+    bias, mb = torch.zeros(4, n, ldm, device="cuda"), torch.full((n_u, ldm), -float("inf"), device="cuda")
+    bias[..., :n] = 2 * draw(4, n, n)
+    mb[:, :n] = -1.4e9 * (torch.rand(n_u, n, generator=g, device="cuda") < 0.1)
+    whole = ops.triatt_flash(q, k, v, bias, mb)
+    for first in (0, n_u // 2, n_u - 12):
+        rows = slice(first, first + 12)
+        assert torch.equal(ops.triatt_flash(q[rows], k[rows], v[rows], bias, mb[rows]), whole[rows])
+    ops.device_error_flags()
