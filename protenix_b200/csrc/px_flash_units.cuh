@@ -6,9 +6,11 @@
 // and bias tiles while its last items are worked on, and the rows of O leave through a staging area of their own, one row a group; to make
 // room for it the K/V ring has three stages.  Groups go on to the next unit each by itself.
 // Alone, us, one unit a CTA | this: N = 160 19.3 | 17.3, 200 28.1 | 26.4, 256 37.3 | 34.0, 300 72.2 | 64.9, 384 101.5 | 93.3, 437 161 | 154,
-// 512 213 | 205, 768 650 | 631, 1024 1471 | 1466, 1536 4740 | 4907 (its items take 3 % longer: more state beside the logits; flags of 32
-// tiles at a time and coordinates worked out anew in place of kept ones gave 2 %).  Runs of neighbouring units per CTA in place of every
-// 148th: 693 at N = 768 (K and V are not shared in L2); rings of three K and four V tiles with barriers of their own: 655.
+// 512 213 | 205, 768 650 | 631, 1024 1471 | 1466; beyond, its items take 3 % longer (more state beside the logits) and the one with a unit a CTA
+// is launched (figures at the rule, px_triatt_flash).  Flags of 32 tiles at a time in place of 64 gave 1 to 2 % with the coordinates worked out
+// anew for the rows of O; kept instead, as they are now, 0.5 % (N = 437 154.3 -> 153.1, 512 208.4 -> 207.4).  Runs of neighbouring units per CTA
+// in place of every 148th: 693 at N = 768 (K and V are not shared in L2); rings of three K and four V tiles with barriers of their own: 655.
+// The control warps' first unit taken as a whole one, as it always is, in place of the test for it: 1.5 % slower at 96 rows of 768.
 #pragma once
 
 namespace px {
@@ -35,7 +37,8 @@ static_assert(FlashUnitLayout::total + 1024 <= 232448, "shared memory budget");
 struct FlashUnit {
   int q0, h, u0;
 };
-// kHalves: the last CTA-loads of work are of one row per group.  kBrief: the last key tile has 32 keys at most, its other half is left out.
+// Units 0 .. whole - 1 are worked on whole, at least one by every CTA (whole >= gridDim.x).  kHalves: `halves` more are shared by two CTAs each,
+// one row per group.  kBrief: the last key tile has 32 keys at most, its other half is left out.
 template <bool kHalves, bool kBrief>
 __global__ void __launch_bounds__(kFThreads, 1)
 triatt_flash_units_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
@@ -240,12 +243,11 @@ triatt_flash_units_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __
     if (lane == 0) mbar_arrive(&bars.s_free[g]);
     int tiles = 0;                                  // bias tiles before this unit (the items before it are an even number)
     const auto softmax = [&](auto per_group, int unit, int second) {
-    FlashUnit w = unit_at(unit, second);
+    const FlashUnit w = unit_at(unit, second);
     constexpr int kRpg = decltype(per_group)::value;     // attended rows per group
     const uint32_t t_o = tmem_base + lane_addr + kFColO + kFON * kFRpg * g;
     const int ug = w.u0 + kRpg * g;                 // first row of this group
-    unsigned flag_word[kRpg];
-                // bit kt & 63: some key of tile kt has a mask bias other than zero
+    unsigned flag_word[kRpg];                       // bit kt & 31: some key of tile kt has a mask bias other than zero
     float m_ref[kRpg], l_sum[kRpg];                 // reference maximum and denominator of this thread's query per row
 #pragma unroll
     for (int r = 0; r < kRpg; ++r) {
@@ -411,10 +413,6 @@ triatt_flash_units_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __
       mask_flags(nkt - 1);
       ok = items(nkt - 1, std::integral_constant<int, kFKT / 2>{});
     }
-    // worked out anew: held through the items, these few registers cost 1 % at N = 1536
-    asm volatile("" : "+r"(unit));
-    w = unit_at(unit, second);
-    const int first_u = w.u0 + kRpg * g;
     tiles += nkt;
     // ---- epilogue: o = O / denominator for this group's rows.  They leave by TMA, a row at a time through the group's staging area: a
     // warp's 32 queries are 2 KB there (64-byte swizzle).  Written by their threads, 16 bytes at 256-byte distances, they took 4 % of
@@ -445,7 +443,7 @@ triatt_flash_units_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __
       }
       asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
       __syncwarp();
-      if (lane == 0 && first_u + r < n_u && w.q0 + 32 * qw < n) {
+      if (lane == 0 && ug + r < n_u && w.q0 + 32 * qw < n) {
         tma_store_3d(&map_o, smem_u32(tile + 32 * qw * 64), w.h * kFD, w.q0 + 32 * qw, ug + r);
         tma_store_commit();
       }
