@@ -238,10 +238,11 @@ def kernel_algo(n: int, zbytes: int, n_msa: int = 1024) -> dict:
 
 
 # DRAM bytes per pair element (dram__bytes_read.sum + dram__bytes_write.sum of one launch / N^2) from the ncu
-# captures at N = 768 with an fp32 z summarised under profiles/ (<kernel>_N768.md).  For these kernels traffic grows
-# with N^2 (operands of the N^3 kernels are re-read from L2, not DRAM), so a launch at another N is scaled by N^2.
+# captures at N = 768 with an fp32 z summarised under profiles/ (<kernel>_N768.md; the attention core at N = 1100, where the kernel
+# of the default workload runs).  For these kernels traffic grows with N^2 (operands of the N^3 kernels are re-read from L2, not DRAM), so a
+# launch at another N is scaled by N^2.
 NCU_TRAFFIC_PER_PAIR = {
-    "px_triatt_flash": 601.0e6 / 768 ** 2,
+    "px_triatt_flash": 1283.2e6 / 1100 ** 2,
     "px_transition": 545.2e6 / 768 ** 2,
     "px_trimul_contract": 424.1e6 / 768 ** 2,
     "px_trimul_in_proj": 395.0e6 / 768 ** 2,
@@ -603,7 +604,7 @@ def main() -> None:
     roof = {"kernel": name, "bound": algo[0], "achieved": achieved, "peak": peak, "unit": runit,
             "frac": achieved / peak, "peak_source": pk["source"],
             "traffic": (NCU_TRAFFIC_PER_PAIR[name] * n * n / world) if name in NCU_TRAFFIC_PER_PAIR else None,
-            "traffic_note": "bytes per launch; ncu capture at N=768 (profiles/) scaled by N^2", "avg_launch_ms": avg_ms,
+            "traffic_note": "bytes per launch; ncu capture at N=768 or 1100 (profiles/) scaled by N^2", "avg_launch_ms": avg_ms,
             "launches": cnt,
             "stage_ms_per_step": {k: round(v[1] / args.steps, 3) for k, v in sorted(stages.items())},
             "stage_share": {k: round(v[1] / args.steps / step_total, 4) for k, v in sorted(stages.items())}}
