@@ -19,6 +19,9 @@
 //   warp 15       loads the pair-bias tiles [128 q][64 k] fp32 (two 128-byte-swizzled boxes, 2-deep ring).
 // Tensor memory: S (3 x 64) | P (3 x 32, two fp16 per column) | O (6 x 32).
 //
+// It runs beyond 1024 keys and where there are no more units (128 queries of a head x 6 rows) than SMs; in between, px_flash_units.cuh does the
+// same with several units a CTA.  Figures from 129 to 1024 tokens in this file are from when this kernel ran there, too.
+//
 // What bounds it (per item of 128 queries x 64 keys, 770 cycles at N = 768): no unit alone, but the chain of a group's item.  Tensor
 // pipe 416 (a copy of 8 columns takes 64 cycles, S 96, P V 64), special-function unit 384, issue slots 440; without any load of K, V
 // and bias the time is the same.  So nothing waits on the chain that can wait beside it: the other half of the bias is fetched

@@ -258,9 +258,7 @@ triatt_flash_units_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __
     const auto mask_flags = [&](int kt) {
       if ((kt & 31) == 0) {
         for (int r = 0; r < kRpg; ++r) flag_word[r] = 0;
-        // A load covers two tiles (ldm is a multiple of 128), eight are in flight beside the first TMA loads and products (two
-        // in flight: 6.17 ms at N = 1536, against 5.88).  As a kernel of its own this cost a launch: 16.6 us together at
-        // N = 128 against 12.6, 143 against 136 at N = 384.
+        // A load covers two tiles (ldm is a multiple of 128), eight are in flight (figures in flash_tcgen05.cu).
         const int left = min(nkt - kt, 32);
 #pragma unroll 1
         for (int t0 = 0; t0 < left; t0 += 8) {
@@ -415,8 +413,7 @@ triatt_flash_units_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __
     }
     tiles += nkt;
     // ---- epilogue: o = O / denominator for this group's rows.  They leave by TMA, a row at a time through the group's staging area: a
-    // warp's 32 queries are 2 KB there (64-byte swizzle).  Written by their threads, 16 bytes at 256-byte distances, they took 4 % of
-    // the kernel at N = 384 and 1.6 % at N = 1536.  The first of two rows has been complete since the last item's P was stored.
+    // warp's 32 queries are 2 KB there (64-byte swizzle).  The first of two rows has been complete since the last item's P was stored.
 #pragma unroll
     for (int r = 0; r < kRpg; ++r) {
       if (r == kRpg - 1) {

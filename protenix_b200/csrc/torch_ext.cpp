@@ -621,17 +621,22 @@ c10::cuda::CUDAStream side_stream(const Use& use) {
 }
 
 // The blocks one after the other.  The pair path never reads s, and the single branch takes nothing from z but the pair
-// bias of the block's final z: the branch of a block runs on a side stream beside the pair path of the next block (two
-// pair-bias buffers take turns).  It is let go when the next block comes to its first attention core, whose CTAs are dealt out
-// as SMs come free; beside the row kernels, whose tiles are dealt out in advance, each of its kernels held up the tile of some
-// SM, and with it the whole kernel.  24 blocks, us per block, in order | beside from the block's start on | beside the attention core:
-// N = 24: 161 | 113 | 111, 64: 168 | 120 | 114, 128: - | 155 | 142, 200: - | 296 | 284, 256: 388 | 348 | 334, 384: - | 741 | 728,
-// 437: 1064 | 1044 | 1028, 640: 2305 | 2273 | 2242, 768: 3442 | - | 3419, 1024: 6838 | - | 6805, 1280: 11999 | - | 11973.  Its
-// transition only beside the second core: 145 at N = 128, 276 against 278 at 200, 720 against 719 at 384.
+// bias of the block's final z: the branch of a block runs on a side stream beside the pair path of the next block, which writes another
+// pair-bias buffer.  It is let go when the next block comes to its first attention core.  Beside row kernels, whose tiles are dealt out in
+// advance, each of its kernels holds up the tile of some SM, and with it the whole kernel.  So it does beside the core, whose units are dealt
+// out in advance as well from 129 to 1024 tokens, but by a smaller part of its far longer time.  us per block, fp32 z, in order | beside from the
+// block's start on | from its first attention core | from its second: N = 64 155 | 115 | 112 | 113, 128 182 | 151 | 145 | 148, 150 234 | 202 | 195 |
+// 198, 200 292 | 260 | 254 | 260, 256 353 | 323 | 324 | 324, 300 510 | 482 | 479 | 477, 384 743 | 693 | 695 | 695, 437 1059 | 1023 | 1010 | 1005,
+// 512 1352 | 1332 | 1305 | 1312, 640 2251 | 2240 | 2210 | 2226, 768 3405 | 3397 | 3367 | 3358, 1024 6783 | 6838 | 6747 | 6697, 1280 level;
+// bf16 200 274 | 242 | 238 | 243, 384 648 | 609 | 600 | 609, 768 3017 | 3008 | 2939 | 2988 (from 384 tokens on the runs of one side differ by 1
+// to 3 %).  Its transition only beside the second core, while the core had a CTA for each unit: 145 at N = 128, 276 against 278 at 200, 720
+// against 719 at 384.
 // One block alone: its projections of s, which need no bias, beside its own pair path (224 | 216 at N = 128, no difference from 200 on).
 // Everything is allocated on the caller's stream, which waits for the side stream before this returns.
 // Where the main stream waits for the side stream before it writes a pair-bias buffer anew, the launch behind does not overlap the kernel
-// before.  Up to kManyBiasUpTo tokens there are eight buffers (together as large as an fp32 z) and one such wait in four blocks.
+// before.  Up to kManyBiasUpTo tokens there are eight buffers (together as large as an fp32 z) and one such wait in four blocks.  Two buffers |
+// eight, us per block: N = 24 105.3 | 103.9, 64 110.5 | 109.3, 128 146.3 | 144.8, 200 256.9 | 255.6, 300 478.5 | 474.4, 384 691.0 | 690.9, 437
+// 1002 | 1017, 512 1312 | 1310, 640 2197 | 2202; bf16 200 235.5 | 234.3, 384 598.6 | 596.1.
 constexpr int64_t kBesideBelow = 1281, kProjectFirstUpTo = 256, kManyBiasUpTo = 384;
 std::tuple<OptTensor, Tensor> stack_forward(const std::vector<std::shared_ptr<Block>>& blocks, const OptTensor& s_in,
                                             const Tensor& z, const OptTensor& mask, bool inplace) {
