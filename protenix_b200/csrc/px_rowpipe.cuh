@@ -259,9 +259,9 @@ static inline int64_t tile_period(int64_t n_u, int64_t n_t, int run) {
 }
 
 // Where consecutive rows of tiles lie behind one another in every tensor of a kernel (rows of z as they are, and no pad columns), the
-// tiles need not end with each row: one row of n_u * n_t elements has fewer of them unless n_t is a multiple of 128 (both output stages of
-// the triangle multiplication, its outgoing projection and the output stage of the starting node, us a block of a stack: 160 tokens
-// 205.3 -> 196.5, 200 260.5 -> 252.5, 400 914 -> 873; where fewer tiles leave SMs free, the single branch has them).
+// tiles need not end with each row (both output stages of the triangle multiplication, its outgoing projection and the output stage of the
+// starting node, us a block of a stack: 160 tokens 205.3 -> 196.5, 200 260.5 -> 252.5, 400 914 -> 873; where fewer tiles leave SMs free, the single
+// branch has them).  Outgoing projection: as one row unless n_t is a multiple of 64 (lengths of an odd number of 64 take two runs a tile, below).
 static inline bool one_row_pays(int64_t n_u, int64_t n_t) { return n_u > 1 && n_t % 64 != 0; }
 
 // How an output stage cuts its tiles: each u by itself (kRows), runs of 64, or as one row where that is possible; whichever makes fewer tiles,

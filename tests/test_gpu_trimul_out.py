@@ -72,3 +72,19 @@ def test_tiles_are_cut_in_three_ways_with_the_same_bits(n, dtype):
         part = z[:, rows].contiguous()
         assert torch.equal(ops.triatt_out(o[rows], part, *vectors[:2], w_g, w_z, ending=True), end[:, rows])
     ops.device_error_flags()
+
+
+@pytest.mark.parametrize("ending", [False, True])
+@pytest.mark.parametrize("n", [64, 150, 200, 520])
+def test_update_alone_is_what_is_added(n, ending):
+    """The form that writes the update in fp16 from standardised rows, in the cuts that it takes, against the one that adds it to an fp32 z."""
+    g = torch.Generator("cuda").manual_seed(n)
+    draw = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    z, o = draw(n, n, 128), draw(n, n, 128).half()
+    zn = ops.standardise_rows(z)
+    args = 1 + 0.2 * draw(128), 0.2 * draw(128), (0.09 * draw(128, 128)).half(), (0.09 * draw(128, 128)).half()
+    update = ops.triatt_out(o, zn, *args, ending=ending)
+    added = ops.triatt_out(o, z.clone(), *args, ending=ending, zn=zn).double() - z.double()
+    # rounding to fp16, 2^-11 / sqrt 3 at most on average; the sum's own rounding is far below
+    assert float((update.double() - added).norm() / added.norm()) < 4e-4
+    ops.device_error_flags()
